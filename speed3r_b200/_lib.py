@@ -11,6 +11,7 @@ import threading
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libspeed3r_b200.so")
+TORCH_LIB_PATH = os.path.join(_PKG, "libspeed3r_b200_torch.so")     # the torch.library operators over LIB_PATH
 
 _i, _i64, _f, _p, _sz = C.c_int, C.c_int64, C.c_float, C.c_void_p, C.c_size_t
 
@@ -60,7 +61,7 @@ def load() -> C.CDLL:
     with _lock:
         if _lib is not None:
             return _lib
-        if not os.path.exists(LIB_PATH):
+        if not (os.path.exists(LIB_PATH) and os.path.exists(TORCH_LIB_PATH)):
             from . import build as _build
             _build.build()
         lib = C.CDLL(LIB_PATH)

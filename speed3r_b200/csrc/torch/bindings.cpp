@@ -1,0 +1,421 @@
+// The torch.library operators of the package: argument checks, allocation and autograd wiring around the
+// C ABI of include/speed3r_b200.h.  Everything between Python and the launches is native, because a call
+// on a short sequence is bounded by host work: through torch.library.custom_op, Python autograd functions
+// and ctypes the whole op at 2048 tokens took 243 us, of which the GPU worked 114 us.
+//
+// Two layers of operators:
+//   base operators (pool_fwd, cmp_attn_topk_fwd, sel_attn_fwd, ...): one C-ABI call each, no autograd.
+//     Registered for CUDA, and for CPU only to say that there is no CPU path.  Their shape functions for
+//     torch.compile are registered from Python (ops.py).
+//   differentiable operators (pool_tokens, flash_attn_topk, ..., sparse_attention): composite functions that
+//     call the base operators through the dispatcher, inside a C++ autograd node when a gradient is needed.
+#include <ATen/ATen.h>
+#include <ATen/core/dispatch/Dispatcher.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/library.h>
+
+#include <cmath>
+#include <tuple>
+#include <vector>
+
+#include "../../../include/speed3r_b200.h"
+
+namespace {
+
+using at::Tensor;
+using c10::optional;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+void need(const Tensor& t, const char* name, at::ScalarType dtype = at::kBFloat16, bool contiguous = true) {
+  TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor: the speed3r_b200 kernels have no CPU path");
+  TORCH_CHECK(t.scalar_type() == dtype, name, " must be ", dtype, ", got ", t.scalar_type());
+  TORCH_CHECK(!contiguous || t.is_contiguous(), name, " must be contiguous");
+}
+
+void check(int rc, const char* what) {
+  if (rc == 0) return;
+  char msg[512];
+  s3r_last_error(msg, sizeof(msg));
+  TORCH_CHECK(false, what, " failed with code ", rc, ": ", msg);
+}
+
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+const int32_t* i32(const Tensor& t) { return static_cast<const int32_t*>(t.data_ptr()); }
+int32_t* i32m(const Tensor& t) { return static_cast<int32_t*>(t.data_ptr()); }
+float* f32(const Tensor& t) { return static_cast<float*>(t.data_ptr()); }
+Tensor fresh(at::IntArrayRef shape, const Tensor& like, at::ScalarType dtype) {
+  return at::empty(shape, like.options().dtype(dtype));
+}
+// contiguous, whatever the strides of `t` (at::empty_like would keep a permuted layout)
+Tensor fresh_like(const Tensor& t) { return at::empty(t.sizes(), t.options()); }
+Tensor none(const Tensor& like) { return at::empty({0}, like.options()); }
+
+// ------------------------------------------------------------------------------------------------
+// base operators
+// ------------------------------------------------------------------------------------------------
+Tensor pool_fwd(const Tensor& x, int64_t kernel, int64_t stride) {
+  need(x, "x", at::kBFloat16, false);
+  TORCH_CHECK(x.dim() == 4 && x.stride(3) == 1, "pool: x must be [B,H,T,d] and its channel dimension must have unit stride");
+  const int64_t B = x.size(0), H = x.size(1), T = x.size(2), d = x.size(3);
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = fresh({B, H, (T - kernel) / stride + 1, d}, x, at::kBFloat16);
+  check(s3r_pool_fwd(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2), out.data_ptr(), B, H, T, d, kernel, stride,
+                     stream()), "s3r_pool_fwd");
+  return out;
+}
+
+Tensor pool_bwd(const Tensor& d_out, int64_t T, int64_t kernel, int64_t stride) {
+  need(d_out, "d_out");
+  const int64_t B = d_out.size(0), H = d_out.size(1), d = d_out.size(3);
+  c10::cuda::CUDAGuard guard(d_out.device());
+  Tensor d_in = fresh({B, H, T, d}, d_out, at::kBFloat16);
+  check(s3r_pool_bwd(d_out.data_ptr(), d_in.data_ptr(), H * T * d, T * d, d, B, H, T, d, kernel, stride, 0, stream()),
+        "s3r_pool_bwd");
+  return d_in;
+}
+
+// group = 0: the table ranks columns; otherwise blocks of `group` columns by the mass of their first `take`
+std::tuple<Tensor, Tensor, Tensor> cmp_fwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c, int64_t topk,
+                                           double scale, int64_t group, int64_t take) {
+  need(q_c, "q_c");
+  need(k_c, "k_c");
+  need(v_c, "v_c");
+  const int64_t B = q_c.size(0), H = q_c.size(1), Nq = q_c.size(2), d = q_c.size(3), Nc = k_c.size(2);
+  const std::vector<int64_t> want = {B, H, Nc, d};
+  TORCH_CHECK(k_c.sizes() == want && v_c.sizes() == want, "k_c/v_c shape mismatch: ", k_c.sizes(), " ", v_c.sizes(),
+              " vs B=", B, " H=", H, " d=", d);
+  c10::cuda::CUDAGuard guard(q_c.device());
+  Tensor o = fresh({B, H, Nq, d}, q_c, at::kBFloat16), lse = fresh({B, H, Nq}, q_c, at::kFloat),
+         idx = fresh({B, H, Nq, topk}, q_c, at::kInt);
+  if (group == 0)
+    check(s3r_cmp_attn_topk_fwd(q_c.data_ptr(), k_c.data_ptr(), v_c.data_ptr(), o.data_ptr(), f32(lse), i32m(idx), B, H,
+                                Nq, Nc, d, topk, scale, stream()), "s3r_cmp_attn_topk_fwd");
+  else
+    check(s3r_cmp_attn_blocktopk_fwd(q_c.data_ptr(), k_c.data_ptr(), v_c.data_ptr(), o.data_ptr(), f32(lse), i32m(idx),
+                                     B, H, Nq, Nc, d, topk, scale, group, take, stream()), "s3r_cmp_attn_blocktopk_fwd");
+  return {o, lse, idx};
+}
+std::tuple<Tensor, Tensor, Tensor> cmp_attn_topk_fwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c,
+                                                     int64_t topk, double scale) {
+  return cmp_fwd(q_c, k_c, v_c, topk, scale, 0, 0);
+}
+std::tuple<Tensor, Tensor, Tensor> cmp_attn_blocktopk_fwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c,
+                                                          int64_t topk, double scale, int64_t group, int64_t take) {
+  TORCH_CHECK(group > 0, "s3r_cmp_attn_blocktopk_fwd: group must be positive");
+  return cmp_fwd(q_c, k_c, v_c, topk, scale, group, take);
+}
+
+std::tuple<Tensor, Tensor, Tensor> cmp_attn_bwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c,
+                                                const Tensor& o_c, const Tensor& lse, const Tensor& do_c, double scale) {
+  need(q_c, "q_c");
+  need(k_c, "k_c");
+  need(v_c, "v_c");
+  need(o_c, "o_c");
+  need(do_c, "do_c");
+  need(lse, "lse", at::kFloat);
+  const int64_t B = q_c.size(0), H = q_c.size(1), Nq = q_c.size(2), d = q_c.size(3), Nc = k_c.size(2);
+  c10::cuda::CUDAGuard guard(q_c.device());
+  Tensor dq = fresh_like(q_c), dk = fresh_like(k_c), dv = fresh_like(v_c), delta = fresh_like(lse);
+  check(s3r_cmp_attn_bwd(q_c.data_ptr(), k_c.data_ptr(), v_c.data_ptr(), o_c.data_ptr(), f32(lse), do_c.data_ptr(),
+                         f32(delta), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Nq, Nc, d, scale, stream()),
+        "s3r_cmp_attn_bwd");
+  return {dq, dk, dv};
+}
+
+void need_gate(const Tensor& gate) {
+  need(gate, "gate", at::kBFloat16, false);
+  TORCH_CHECK(gate.dim() == 4 && gate.stride(3) == 1, "gate: the last dimension (g0,g1) must have unit stride");
+}
+
+// Returns (o_s, lse_s, y); tensors not asked for come back with zero elements.
+std::tuple<Tensor, Tensor, Tensor> sel_attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                                const optional<Tensor>& gate, const optional<Tensor>& o_c, int64_t block,
+                                                double scale, bool want_o, bool want_lse, int64_t kv_chunks) {
+  need(q, "q");
+  need(k, "k");
+  need(v, "v");
+  need(idx, "topk_idx", at::kInt);
+  const int64_t B = q.size(0), H = q.size(1), Tq = q.size(2), d = q.size(3);
+  int64_t Tk, chunk_stride = 0;
+  if (kv_chunks == 1) {
+    Tk = k.size(2);
+    TORCH_CHECK(k.sizes() == std::vector<int64_t>({B, H, Tk, d}) && v.sizes() == k.sizes(), "k/v must be [B,H,Tk,d]");
+  } else {                               // [chunks, B, H, Tk/chunks, d] as an all-gather leaves it
+    TORCH_CHECK(k.dim() == 5 && k.size(0) == kv_chunks && v.sizes() == k.sizes(), "chunked k/v must be [chunks,B,H,Tk/chunks,d]");
+    Tk = k.size(3) * kv_chunks;
+    chunk_stride = k.stride(0);
+  }
+  const int64_t K = idx.size(-1), nqb = (Tq + block - 1) / block;
+  TORCH_CHECK(idx.sizes() == std::vector<int64_t>({B, H, nqb, K}), "topk_idx must be [B,H,ceil(Tq/block),K] = [", B, ", ", H,
+              ", ", nqb, ", ", K, "], got ", idx.sizes());
+  const bool merge = gate.has_value();
+  int64_t gs[3] = {0, 0, 0};
+  if (merge) {
+    need_gate(*gate);
+    TORCH_CHECK(o_c.has_value(), "gate and o_c come together");
+    need(*o_c, "o_c");
+    TORCH_CHECK(gate->sizes() == std::vector<int64_t>({B, H, Tq, 2}) && o_c->sizes() == std::vector<int64_t>({B, H, nqb, d}),
+                "gate must be [B,H,Tq,2] and o_c [B,H,ceil(Tq/block),d]");
+    for (int i = 0; i < 3; ++i) gs[i] = gate->stride(i);
+  }
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor o_s = want_o ? fresh({B, H, Tq, d}, q, at::kBFloat16) : none(q);
+  Tensor lse = fresh(want_lse ? std::vector<int64_t>{B, H, Tq} : std::vector<int64_t>{0}, q, at::kFloat);
+  Tensor y = merge ? fresh({B, Tq, H * d}, q, at::kBFloat16) : none(q);
+  check(s3r_sel_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), kv_chunks, chunk_stride, i32(idx),
+                         want_o ? o_s.data_ptr() : nullptr, want_lse ? f32(lse) : nullptr, merge ? gate->data_ptr() : nullptr,
+                         gs[0], gs[1], gs[2], merge ? o_c->data_ptr() : nullptr, merge ? y.data_ptr() : nullptr, B, H, Tq, Tk,
+                         d, block, K, scale, stream()), "s3r_sel_attn_fwd");
+  return {o_s, lse, y};
+}
+
+std::tuple<Tensor, Tensor> csr(const Tensor& idx, int64_t nkb, bool fill) {
+  need(idx, "topk_idx", at::kInt);
+  const int64_t B = idx.size(0), H = idx.size(1), Nq = idx.size(2), K = idx.size(3);
+  c10::cuda::CUDAGuard guard(idx.device());
+  Tensor offsets = fresh({B, H, nkb + 1}, idx, at::kInt), qids = fresh({B, H, Nq * K}, idx, at::kInt);
+  if (fill) qids.fill_(-1);
+  const size_t nbytes = s3r_csr_workspace_bytes(B, H, Nq, K, nkb);
+  Tensor ws = fresh({static_cast<int64_t>(nbytes)}, idx, at::kByte);
+  check(s3r_build_key_csr(i32(idx), i32m(offsets), i32m(qids), B, H, Nq, K, nkb, ws.data_ptr(), nbytes, stream()),
+        "s3r_build_key_csr");
+  return {offsets, qids};
+}
+// slots behind the entries of the table that were dropped hold -1
+std::tuple<Tensor, Tensor> build_key_csr(const Tensor& idx, int64_t num_key_blocks) { return csr(idx, num_key_blocks, true); }
+
+std::tuple<Tensor, Tensor, Tensor> sel_attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                                const Tensor& lse, const Tensor& delta, const Tensor& do_s, int64_t block,
+                                                double scale) {
+  need(q, "q");
+  need(k, "k");
+  need(v, "v");
+  need(do_s, "do_s");
+  const int64_t B = q.size(0), H = q.size(1), Tq = q.size(2), d = q.size(3), Tk = k.size(2), K = idx.size(-1);
+  c10::cuda::CUDAGuard guard(q.device());
+  auto [offsets, qids] = csr(idx, (Tk + block - 1) / block, false);
+  Tensor dq = fresh_like(q), dk = fresh_like(k), dv = fresh_like(v);
+  check(s3r_sel_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), i32(idx), i32(offsets), i32(qids), f32(lse), f32(delta),
+                         do_s.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Tq, Tk, d, block, K, scale,
+                         stream()), "s3r_sel_attn_bwd");
+  return {dq, dk, dv};
+}
+
+Tensor delta(const Tensor& o, const Tensor& d_o) {
+  need(o, "o");
+  need(d_o, "do");
+  c10::cuda::CUDAGuard guard(o.device());
+  Tensor out = fresh(o.sizes().slice(0, o.dim() - 1), o, at::kFloat);
+  check(s3r_delta(o.data_ptr(), d_o.data_ptr(), f32(out), out.numel(), o.size(-1), stream()), "s3r_delta");
+  return out;
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> merge_bwd(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
+                                                     const Tensor& o_s, int64_t block) {
+  need(dy, "dy");
+  need_gate(gate);
+  const int64_t B = o_s.size(0), H = o_s.size(1), Tq = o_s.size(2), d = o_s.size(3);
+  c10::cuda::CUDAGuard guard(dy.device());
+  Tensor do_s = fresh_like(o_s), dgate = fresh({B, H, Tq, 2}, dy, at::kFloat), do_c = fresh_like(o_c),
+         delta_s = fresh({B, H, Tq}, dy, at::kFloat);
+  check(s3r_merge_bwd(dy.data_ptr(), gate.data_ptr(), gate.stride(0), gate.stride(1), gate.stride(2), o_c.data_ptr(),
+                      o_s.data_ptr(), do_s.data_ptr(), f32(dgate), do_c.data_ptr(), f32(delta_s), B, H, Tq, d, block,
+                      stream()), "s3r_merge_bwd");
+  return {do_s, dgate, do_c, delta_s};
+}
+
+// ------------------------------------------------------------------------------------------------
+// the base operators as the differentiable ones call them: through the dispatcher, so that fake tensors,
+// functionalisation and dispatch modes see them
+// ------------------------------------------------------------------------------------------------
+#define S3R_DISPATCHED(fn)                                                                              \
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("speed3r_b200::" #fn, "").typed<decltype(fn)>(); \
+  return op.call
+
+Tensor call_pool_fwd(const Tensor& x, int64_t kernel, int64_t stride) { S3R_DISPATCHED(pool_fwd)(x, kernel, stride); }
+Tensor call_pool_bwd(const Tensor& g, int64_t T, int64_t kernel, int64_t stride) { S3R_DISPATCHED(pool_bwd)(g, T, kernel, stride); }
+std::tuple<Tensor, Tensor, Tensor> call_cmp_topk(const Tensor& q, const Tensor& k, const Tensor& v, int64_t topk, double scale) {
+  S3R_DISPATCHED(cmp_attn_topk_fwd)(q, k, v, topk, scale);
+}
+std::tuple<Tensor, Tensor, Tensor> call_cmp_blocktopk(const Tensor& q, const Tensor& k, const Tensor& v, int64_t topk,
+                                                      double scale, int64_t group, int64_t take) {
+  S3R_DISPATCHED(cmp_attn_blocktopk_fwd)(q, k, v, topk, scale, group, take);
+}
+std::tuple<Tensor, Tensor, Tensor> call_cmp(const Tensor& q, const Tensor& k, const Tensor& v, int64_t topk, double scale,
+                                            int64_t group, int64_t take) {
+  return group == 0 ? call_cmp_topk(q, k, v, topk, scale) : call_cmp_blocktopk(q, k, v, topk, scale, group, take);
+}
+std::tuple<Tensor, Tensor, Tensor> call_cmp_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
+                                                const Tensor& lse, const Tensor& d_o, double scale) {
+  S3R_DISPATCHED(cmp_attn_bwd)(q, k, v, o, lse, d_o, scale);
+}
+std::tuple<Tensor, Tensor, Tensor> call_sel(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                            const optional<Tensor>& gate, const optional<Tensor>& o_c, int64_t block,
+                                            double scale, bool want_o, bool want_lse, int64_t chunks) {
+  S3R_DISPATCHED(sel_attn_fwd)(q, k, v, idx, gate, o_c, block, scale, want_o, want_lse, chunks);
+}
+std::tuple<Tensor, Tensor, Tensor> call_sel_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                                const Tensor& lse, const Tensor& dlt, const Tensor& d_o, int64_t block,
+                                                double scale) {
+  S3R_DISPATCHED(sel_attn_bwd)(q, k, v, idx, lse, dlt, d_o, block, scale);
+}
+Tensor call_delta(const Tensor& o, const Tensor& d_o) { S3R_DISPATCHED(delta)(o, d_o); }
+std::tuple<Tensor, Tensor, Tensor, Tensor> call_merge_bwd(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
+                                                          const Tensor& o_s, int64_t block) {
+  S3R_DISPATCHED(merge_bwd)(dy, gate, o_c, o_s, block);
+}
+
+// ------------------------------------------------------------------------------------------------
+// differentiable operators
+// ------------------------------------------------------------------------------------------------
+template <typename... T>
+bool wants_grad(const T&... t) {
+  return at::GradMode::is_enabled() && (t.requires_grad() || ...);
+}
+
+struct PoolNode : torch::autograd::Function<PoolNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t kernel, int64_t stride) {
+    ctx->saved_data["T"] = x.size(2);
+    ctx->saved_data["kernel"] = kernel;
+    ctx->saved_data["stride"] = stride;
+    at::AutoDispatchBelowADInplaceOrView below;
+    return call_pool_fwd(x, kernel, stride);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return {call_pool_bwd(g[0].contiguous(), ctx->saved_data["T"].toInt(), ctx->saved_data["kernel"].toInt(),
+                          ctx->saved_data["stride"].toInt()), Tensor(), Tensor()};
+  }
+};
+Tensor pool_tokens(const Tensor& x, int64_t kernel, int64_t stride) {
+  return wants_grad(x) ? PoolNode::apply(x, kernel, stride) : call_pool_fwd(x, kernel, stride);
+}
+
+struct CmpNode : torch::autograd::Function<CmpNode> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, int64_t topk,
+                               double scale, int64_t group, int64_t take) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto [o, lse, idx] = call_cmp(q, k, v, topk, scale, group, take);
+    ctx->save_for_backward({q, k, v, o, lse});
+    ctx->saved_data["scale"] = scale;
+    ctx->mark_non_differentiable({idx});
+    return {o, idx};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    auto [dq, dk, dv] = call_cmp_bwd(s[0], s[1], s[2], s[3], s[4],
+                                     g[0].defined() ? g[0].contiguous() : at::zeros_like(s[3]), ctx->saved_data["scale"].toDouble());
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+std::tuple<Tensor, Tensor> flash_attn_topk(const Tensor& q_, const Tensor& k_, const Tensor& v_, int64_t topk, double scale,
+                                           int64_t group, int64_t take) {
+  const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
+  if (!wants_grad(q, k, v)) {
+    auto [o, lse, idx] = call_cmp(q, k, v, topk, scale, group, take);
+    return {o, idx};
+  }
+  const auto r = CmpNode::apply(q, k, v, topk, scale, group, take);
+  return {r[0], r[1]};
+}
+
+struct SelNode : torch::autograd::Function<SelNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                        int64_t block, double scale) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto [o, lse, y] = call_sel(q, k, v, idx, {}, {}, block, scale, true, true, 1);
+    ctx->save_for_backward({q, k, v, o, lse, idx});
+    ctx->saved_data["block"] = block;
+    ctx->saved_data["scale"] = scale;
+    return o;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor d_o = g[0].contiguous();
+    auto [dq, dk, dv] = call_sel_bwd(s[0], s[1], s[2], s[5], s[4], call_delta(s[3], d_o), d_o,
+                                     ctx->saved_data["block"].toInt(), ctx->saved_data["scale"].toDouble());
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
+  }
+};
+Tensor topk_blocksparse(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, int64_t block, double scale) {
+  if (wants_grad(q, k, v)) return SelNode::apply(q, k, v, idx, block, scale);
+  return std::get<0>(call_sel(q, k, v, idx, {}, {}, block, scale, true, false, 1));
+}
+
+struct SelMergeNode : torch::autograd::Function<SelMergeNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                        const Tensor& gate, const Tensor& o_c, int64_t block, double scale) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto [o_s, lse, y] = call_sel(q, k, v, idx, gate, o_c, block, scale, true, true, 1);
+    ctx->save_for_backward({q, k, v, idx, gate, o_c, o_s, lse});
+    ctx->saved_data["block"] = block;
+    ctx->saved_data["scale"] = scale;
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const int64_t block = ctx->saved_data["block"].toInt();
+    auto [do_s, dgate, do_c, dlt] = call_merge_bwd(g[0].contiguous(), s[4], s[5], s[6], block);
+    auto [dq, dk, dv] = call_sel_bwd(s[0], s[1], s[2], s[3], s[7], dlt, do_s, block, ctx->saved_data["scale"].toDouble());
+    return {dq, dk, dv, Tensor(), dgate.to(s[4].scalar_type()), do_c, Tensor(), Tensor()};
+  }
+};
+Tensor sel_merge(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx, const Tensor& gate, const Tensor& o_c,
+                 int64_t block, double scale) {
+  if (wants_grad(q, k, v, gate, o_c)) return SelMergeNode::apply(q, k, v, idx, gate, o_c, block, scale);
+  return std::get<2>(call_sel(q, k, v, idx, gate, o_c, block, scale, false, false, 1));
+}
+
+// The whole op.  group = 0 where compressed keys are the selection blocks.
+std::tuple<Tensor, Tensor> sparse_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gate,
+                                            int64_t block, int64_t topk, int64_t kernel, int64_t stride, double scale,
+                                            int64_t group, int64_t take) {
+  const Tensor q_c = pool_tokens(q, block, block), k_c = pool_tokens(k, kernel, stride), v_c = pool_tokens(v, kernel, stride);
+  auto [o_c, idx] = flash_attn_topk(q_c, k_c, v_c, topk, scale, group, take);
+  return {sel_merge(q, k, v, idx, gate, o_c, block, scale), idx};
+}
+
+}  // namespace
+
+TORCH_LIBRARY(speed3r_b200, m) {
+  m.def("pool_fwd(Tensor x, int kernel, int stride) -> Tensor");
+  m.def("pool_bwd(Tensor d_out, int T, int kernel, int stride) -> Tensor");
+  m.def("cmp_attn_topk_fwd(Tensor q_c, Tensor k_c, Tensor v_c, int topk, float scale) -> (Tensor, Tensor, Tensor)");
+  m.def("cmp_attn_blocktopk_fwd(Tensor q_c, Tensor k_c, Tensor v_c, int topk, float scale, int group, int take) -> "
+        "(Tensor, Tensor, Tensor)");
+  m.def("cmp_attn_bwd(Tensor q_c, Tensor k_c, Tensor v_c, Tensor o_c, Tensor lse, Tensor do_c, float scale) -> "
+        "(Tensor, Tensor, Tensor)");
+  m.def("sel_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor idx, Tensor? gate, Tensor? o_c, int block, float scale, "
+        "bool want_o, bool want_lse, int kv_chunks) -> (Tensor, Tensor, Tensor)");
+  m.def("build_key_csr(Tensor idx, int num_key_blocks) -> (Tensor, Tensor)");
+  m.def("sel_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor idx, Tensor lse, Tensor delta, Tensor do_s, int block, "
+        "float scale) -> (Tensor, Tensor, Tensor)");
+  m.def("delta(Tensor o, Tensor d_o) -> Tensor");
+  m.def("merge_bwd(Tensor dy, Tensor gate, Tensor o_c, Tensor o_s, int block) -> (Tensor, Tensor, Tensor, Tensor)");
+
+  m.def("pool_tokens(Tensor x, int kernel, int stride) -> Tensor", &pool_tokens);
+  m.def("flash_attn_topk(Tensor q, Tensor k, Tensor v, int topk, float scale, int group, int take) -> (Tensor, Tensor)",
+        &flash_attn_topk);
+  m.def("topk_blocksparse(Tensor q, Tensor k, Tensor v, Tensor idx, int block, float scale) -> Tensor", &topk_blocksparse);
+  m.def("sel_merge(Tensor q, Tensor k, Tensor v, Tensor idx, Tensor gate, Tensor o_c, int block, float scale) -> Tensor",
+        &sel_merge);
+  m.def("sparse_attention(Tensor q, Tensor k, Tensor v, Tensor gate, int block, int topk, int kernel, int stride, "
+        "float scale, int group, int take) -> (Tensor, Tensor)", &sparse_attention);
+}
+
+#define S3R_BASE_OPS(m)                                     \
+  m.impl("pool_fwd", &pool_fwd);                            \
+  m.impl("pool_bwd", &pool_bwd);                            \
+  m.impl("cmp_attn_topk_fwd", &cmp_attn_topk_fwd);          \
+  m.impl("cmp_attn_blocktopk_fwd", &cmp_attn_blocktopk_fwd); \
+  m.impl("cmp_attn_bwd", &cmp_attn_bwd);                    \
+  m.impl("sel_attn_fwd", &sel_attn_fwd);                    \
+  m.impl("build_key_csr", &build_key_csr);                  \
+  m.impl("sel_attn_bwd", &sel_attn_bwd);                    \
+  m.impl("delta", &delta);                                  \
+  m.impl("merge_bwd", &merge_bwd)
+
+TORCH_LIBRARY_IMPL(speed3r_b200, CUDA, m) { S3R_BASE_OPS(m); }
+TORCH_LIBRARY_IMPL(speed3r_b200, CPU, m) { S3R_BASE_OPS(m); }      // every one of them refuses CPU tensors
