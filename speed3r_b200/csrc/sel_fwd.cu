@@ -3,33 +3,15 @@
 //
 // Bound: gather bandwidth.  A query block of BS rows reads topk*BS key rows and value rows
 // (2*topk*BS*128 B) for 4*BS*topk*BS*64 flop, i.e. BS flop per byte (16 at the reference's block
-// size) against a machine balance of ~250 flop/B, so the kernel is organised around keeping many
-// independent TMA gathers in flight, not around tensor-core throughput:
-//   * one "group" of BS/16 warps owns one query block; a CTA holds 8 warps = 8/(BS/16) groups;
-//   * each group has its own ring of STAGES shared-memory stages; lane 0 of the group's first warp
-//     issues one TMA tiled copy per selected key block (K and V, 128-byte swizzle) and the copies
-//     complete on the stage's mbarrier;
-//   * each warp multiplies its 16 query rows with the stage's keys with mma.sync m16n8k16 (a
-//     16-row query block is exactly one MMA M tile), keeps the online softmax in registers and
-//     accumulates P*V;
-//   * the epilogue normalises, optionally applies  y = g0*o_c + g1*o_s  and writes 128-byte rows.
+// size) against a machine balance of ~250 flop/B, so the kernels are organised around keeping many
+// independent TMA gathers in flight, not around tensor-core throughput: mma.sync m16n8k16, whose M tile
+// is a 16-row query block, online softmax in registers, epilogue y = g0*o_c + g1*o_s in 128-byte rows.
+// Two kernels: sel16_fwd_kernel for blocks of 16 (one warp per query block, below), sel_fwd_kernel for 32
+// and 64 (BS/16 warps share a query block's ring of stages).
 // CTAs are ordered head-major so that the CTAs resident at one time gather from one head's K/V.
 #include "common.cuh"
 
 namespace s3r {
-
-// Block size 16 (the reference's): the loop of one warp is a chain of dependent instructions, so the
-// kernel runs faster with more warps per SM than with deeper rings: 12 warps with 2 stages of 32 keys
-// (216 KB of shared memory) beat 8 warps with 3 stages by 20 % on B200.
-#ifndef S3R_SEL16_WARPS
-#define S3R_SEL16_WARPS 12
-#endif
-#ifndef S3R_SEL16_STAGES
-#define S3R_SEL16_STAGES 2
-#endif
-#ifndef S3R_SEL16_STAGE_KEYS
-#define S3R_SEL16_STAGE_KEYS 32
-#endif
 
 // Larger blocks (32, 64 tokens: not the reference's setting): the same lesson - two CTAs of 8 warps per SM
 // (128 registers, 2-stage rings) run the 64-token kernel in 15.5 ms at 1000 views where one CTA with a 6-stage
@@ -43,14 +25,14 @@ namespace s3r {
 
 template <int BS>
 struct SelCfg {
-  static constexpr int kWarps = (BS == 16) ? S3R_SEL16_WARPS : 8;
+  static constexpr int kWarps = 8;
   static constexpr int kWpg = BS / 16;                    // warps per query block
   static constexpr int kGroups = kWarps / kWpg;           // query blocks per CTA
-  static constexpr int kStageKeys = BS < 32 ? S3R_SEL16_STAGE_KEYS : BS;    // keys per pipeline stage
+  static constexpr int kStageKeys = BS;                   // keys per pipeline stage
   static constexpr int kBlkPerStage = kStageKeys / BS;
   static constexpr int kStageBytes = kStageKeys * 128 * 2;  // K tile + V tile
-  static constexpr int kStages = (BS == 16) ? S3R_SEL16_STAGES : S3R_SELBIG_STAGES;
-  static constexpr int kMinCtas = (BS == 16) ? 1 : S3R_SELBIG_MIN_CTAS;
+  static constexpr int kStages = S3R_SELBIG_STAGES;
+  static constexpr int kMinCtas = S3R_SELBIG_MIN_CTAS;
   static constexpr int kQBytes = BS * 128;
   static constexpr int kMaxTopk = 64;
   static constexpr int kSmemBytes = kGroups * (kStages * kStageBytes + kQBytes) + 1024 /*alignment slack*/;
@@ -412,6 +394,280 @@ static int launch_sel_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CU
   return 0;
 }
 
+// ------------------------------------------------------------------------------------------------
+// Blocks of 16 tokens (the reference's setting)
+// ------------------------------------------------------------------------------------------------
+// One warp = one CTA owns one query block (16 rows = one m16n8k16 M tile) and takes its selected key blocks
+// two at a time from a ring of two 8 KB stages; one TMA copy brings a block's keys and values.
+//   * All fragments of a stage go from shared memory to registers before the first product, so that no product
+//     waits for a load (with loads and products alternating a warp spent 2700 cycles on a pair of blocks).
+//   * The exponent offset of a row is the maximum of its first pair and moves only when a pair's sum of P passes
+//     2^24 (P keeps its relative precision, O and l are fp32): no maximum, no shuffles in between.
+//   * CTAs of one warp: nothing is shared between query blocks, and a finished warp makes room at once.
+// Bound: a bare TMA gather of the same blocks runs at 20 TB/s while a head's K and V fit L2 and at 10.5 TB/s at
+// 1000 views (258 MB per head).  Measured (H = 16, top-32, uniformly random blocks): 64 views 822 -> 532 us =
+// 15.9 TB/s gathered, 2048 tokens 46 -> 27 us, 250 views 3.16 -> 2.22 ms, 1000 views 14.9 -> 13.8 ms (9.6 TB/s).
+// Gathering straight into fragments with 16-byte loads instead (no shared memory) ran at 8.7 TB/s: a fragment load
+// touches 8 rows, and L1 serves few lines per cycle.
+struct Sel16Params {
+  const __nv_bfloat16* q;
+  const int32_t* idx;
+  __nv_bfloat16* o_s;
+  float* lse_s;
+  const __nv_bfloat16* gate;
+  int64_t gsb, gsh, gst;
+  const __nv_bfloat16* o_c;
+  __nv_bfloat16* y;
+  int H, Tq, Tk, Tc, nqb, topk;
+  float scale_log2e;
+  int v_first;                   // the value tensor lies below the key tensor in memory
+  uint32_t pair_bytes;           // what the copies of a pair of blocks bring
+  uint32_t* status;
+};
+
+constexpr int kSel16StageBytes = 2 * 2 * 2048;                    // two blocks of keys, two of values
+constexpr int kSel16Smem = 2 * kSel16StageBytes + 1024;
+
+__global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant__ CUtensorMap map_kv, const Sel16Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) int32_t list[64];        // first token of each valid key block, table order
+  __shared__ uint64_t full[2];
+  __shared__ uint32_t abort_word;
+  const int lane = threadIdx.x, g = lane >> 2, c = lane & 3;
+  const int64_t task = blockIdx.x;
+  const int bh = static_cast<int>(task / p.nqb), qb = static_cast<int>(task - static_cast<int64_t>(bh) * p.nqb);
+  volatile uint32_t* abort_flag = &abort_word;
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  if (lane == 0) {
+    abort_word = 0;
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    mbar_fence_init();
+  }
+
+  int nvalid = 0;
+  {
+    const int32_t* row = p.idx + task * p.topk;
+    for (int r0 = 0; r0 < p.topk; r0 += 32) {
+      const int i = r0 + lane;
+      const int n = (i < p.topk) ? row[i] : -1;
+      const bool ok = (n >= 0) && (static_cast<int64_t>(n) * 16 < p.Tk);
+      const uint32_t m = __ballot_sync(0xffffffffu, ok);
+      if (ok) list[nvalid + __popc(m & ((1u << lane) - 1u))] = n * 16;
+      nvalid += __popc(m);
+    }
+    __syncwarp();
+  }
+  // an odd list ends with its last block twice; the second copy's scores are masked
+  if ((nvalid & 1) && lane == 0) list[nvalid] = list[nvalid - 1];
+  __syncwarp();
+  const bool chunked = p.Tc != p.Tk;
+  // one copy per block brings its keys and its values
+  auto issue = [&](int pair, int s) {
+    if (lane == 0) {
+      const int2 t = *reinterpret_cast<const int2*>(list + 2 * pair);
+      int t0 = t.x, t1 = t.y, c0 = 0, c1 = 0;
+      if (chunked) {
+        c0 = t0 / p.Tc; t0 -= c0 * p.Tc;
+        c1 = t1 / p.Tc; t1 -= c1 * p.Tc;
+      }
+      const uint32_t dst = ring + s * kSel16StageBytes;
+      mbar_expect_tx(&full[s], p.pair_bytes);
+      tma_load_5d(dst, &map_kv, &full[s], 0, t0, bh, c0, 0);
+      tma_load_5d(dst + 4096, &map_kv, &full[s], 0, t1, bh, c1, 0);
+    }
+  };
+  const int npairs = (nvalid + 1) >> 1;
+  if (npairs > 0) issue(0, 0);
+  if (npairs > 1) issue(1, 1);
+
+  uint32_t qf[4][4];
+  {
+    const uint32_t* q32 = reinterpret_cast<const uint32_t*>(p.q) + static_cast<int64_t>(bh) * p.Tq * 32;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t* src = q32 + static_cast<int64_t>(min(qb * 16 + g + 8 * r, p.Tq - 1)) * 32 + c;
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        qf[ks][r] = __ldg(src + ks * 8);
+        qf[ks][r + 2] = __ldg(src + ks * 8 + 4);
+      }
+    }
+  }
+  // shared-memory offsets of this lane's ldmatrix rows (128-byte swizzle), per k-step of Q K^T and per pair of d-tiles of P V
+  uint32_t off_k[4], off_v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    off_k[i] = swz128((lane & 7) + (lane >> 4) * 8, 2 * i + ((lane >> 3) & 1)) + (p.v_first ? 2048u : 0u);
+    off_v[i] = swz128((lane & 7) + ((lane >> 3) & 1) * 8, 2 * i + (lane >> 4)) + (p.v_first || p.pair_bytes < 8192u ? 0u : 2048u);
+  }
+
+  float o[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  float m_used[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};        // l: this lane's share
+  const float cs = p.scale_log2e;
+  const bool ragged = (p.Tk & 15) != 0;
+#pragma unroll 1
+  for (int it = 0; it < npairs; ++it) {
+    const int S = it & 1;
+    if (!mbar_wait_warp(&full[S], (it >> 1) & 1, abort_flag)) {
+      volatile uint32_t dummy = 0;               // a last bounded chance for the other stage's copies to land
+      if (it + 1 < npairs) mbar_wait(&full[S ^ 1], ((it + 1) >> 1) & 1, &dummy);
+      if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+      return;
+    }
+    const uint32_t st = ring + S * kSel16StageBytes;
+    // every fragment of the stage goes to registers first: the products below then wait for no load
+    uint32_t kf[2][4][4], vf[2][4][4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) ldsm_x4(kf[j][ks][0], kf[j][ks][1], kf[j][ks][2], kf[j][ks][3], st + off_k[ks] + j * 4096);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int dp = 0; dp < 4; ++dp) ldsm_x4_t(vf[j][dp][0], vf[j][dp][1], vf[j][dp][2], vf[j][dp][3], st + off_v[dp] + j * 4096);
+    float s[2][2][4];                            // [block][key n-tile]
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (ks == 0) mma_bf16_z(s[j][t], qf[ks], kf[j][ks][2 * t], kf[j][ks][2 * t + 1]);
+          else mma_bf16(s[j][t], qf[ks], kf[j][ks][2 * t], kf[j][ks][2 * t + 1]);
+        }
+    if (2 * it + 1 >= nvalid) {                  // the second block is the padding of an odd list
+#pragma unroll
+      for (int t = 0; t < 2; ++t) s[1][t][0] = s[1][t][1] = s[1][t][2] = s[1][t][3] = -INFINITY;
+    }
+    if (ragged) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int left = p.Tk - list[2 * it + j];
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (t * 8 + 2 * c + (e & 1) >= left) s[j][t][e] = -INFINITY;
+      }
+    }
+    uint32_t pk[2][4];
+    float ts[2];
+    auto exps = [&]() {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float2 nm = make_float2(-m_used[r], -m_used[r]), cs2 = make_float2(cs, cs);
+        float2 sum;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            float2 x = ffma2(make_float2(s[j][t][2 * r], s[j][t][2 * r + 1]), cs2, nm);
+            x.x = fast_exp2(x.x);
+            x.y = fast_exp2(x.y);
+            sum = (j | t) ? fadd2(sum, x) : x;
+            pk[j][2 * t + r] = pack_bf16(x.x, x.y);
+          }
+        ts[r] = sum.x + sum.y;
+      }
+    };
+    auto row_max = [&](int r) {
+      float m = fmax3(fmaxf(s[0][0][2 * r], s[0][0][2 * r + 1]), s[0][1][2 * r], s[0][1][2 * r + 1]);
+      m = fmax3(fmax3(m, s[1][0][2 * r], s[1][0][2 * r + 1]), s[1][1][2 * r], s[1][1][2 * r + 1]);
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      return fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2)) * cs;       // scale > 0 keeps the order
+    };
+    if (it == 0) { m_used[0] = row_max(0); m_used[1] = row_max(1); }
+    exps();
+    if (__any_sync(0xffffffffu, !(fmaxf(ts[0], ts[1]) <= 16777216.f))) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float mn = fmaxf(m_used[r], row_max(r)), alpha = fast_exp2(m_used[r] - mn);
+        m_used[r] = mn;
+        l[r] *= alpha;
+#pragma unroll
+        for (int dt = 0; dt < 8; ++dt) { o[dt][2 * r] *= alpha; o[dt][2 * r + 1] *= alpha; }
+      }
+      exps();
+    }
+    l[0] += ts[0];
+    l[1] += ts[1];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int dp = 0; dp < 4; ++dp) {
+        mma_bf16(o[2 * dp], pk[j], vf[j][dp][0], vf[j][dp][1]);
+        mma_bf16(o[2 * dp + 1], pk[j], vf[j][dp][2], vf[j][dp][3]);
+      }
+    __syncwarp();
+    if (it + 2 < npairs) issue(it + 2, S);       // every fragment of the stage has been consumed
+  }
+  // ---- epilogue -----------------------------------------------------------------------------
+  float inv[2];
+  const int t0 = qb * 16 + g;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    float ls = l[r];
+    ls += __shfl_xor_sync(0xffffffffu, ls, 1);
+    ls += __shfl_xor_sync(0xffffffffu, ls, 2);
+    inv[r] = (nvalid > 0) ? 1.0f / ls : 0.f;             // no valid key: o = 0, lse = -inf
+    if (p.lse_s && c == 0 && t0 + 8 * r < p.Tq)
+      p.lse_s[static_cast<int64_t>(bh) * p.Tq + t0 + 8 * r] =
+          (nvalid > 0) ? (m_used[r] + log2f(ls)) * 0.6931471805599453f : -INFINITY;
+  }
+  // rows of 128 bytes leave through the warp's first stage (its copies have landed and been read)
+  __syncwarp();
+  uint8_t* stage = smem_raw + (ring - smem_u32(smem_raw));
+  auto put = [&](const float (&a)[8][4], uint8_t* dst, int64_t row_bytes) {
+#pragma unroll
+    for (int dt = 0; dt < 8; ++dt) {
+      *reinterpret_cast<uint32_t*>(stage + swz128(g, dt) + 4 * c) = pack_bf16(a[dt][0], a[dt][1]);
+      *reinterpret_cast<uint32_t*>(stage + swz128(g + 8, dt) + 4 * c) = pack_bf16(a[dt][2], a[dt][3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = (lane >> 3) + 4 * i;
+      if (qb * 16 + r < p.Tq)
+        *reinterpret_cast<uint4*>(dst + r * row_bytes + (lane & 7) * 16) = *reinterpret_cast<const uint4*>(stage + swz128(r, lane & 7));
+    }
+    __syncwarp();
+  };
+#pragma unroll
+  for (int dt = 0; dt < 8; ++dt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[dt][e] *= inv[e >> 1];
+  if (p.o_s) put(o, reinterpret_cast<uint8_t*>(p.o_s + (static_cast<int64_t>(bh) * p.Tq + static_cast<int64_t>(qb) * 16) * 64), 128);
+  if (p.y) {
+    const int b = bh / p.H, h = bh - b * p.H;
+    float g0[2], g1[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t w = *reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + min(t0 + 8 * r, p.Tq - 1) * p.gst);
+      g0[r] = bf16_lo(w); g1[r] = bf16_hi(w);
+    }
+    const uint32_t* oc = reinterpret_cast<const uint32_t*>(p.o_c) + task * 32 + c;
+#pragma unroll
+    for (int dt = 0; dt < 8; ++dt) {
+      const uint32_t w = oc[dt * 4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[dt][e] = g0[e >> 1] * ((e & 1) ? bf16_hi(w) : bf16_lo(w)) + g1[e >> 1] * o[dt][e];
+    }
+    put(o, reinterpret_cast<uint8_t*>(p.y + ((static_cast<int64_t>(b) * p.Tq + static_cast<int64_t>(qb) * 16) * p.H + h) * 64),
+        static_cast<int64_t>(p.H) * 128);
+  }
+}
+
+static int launch_sel16_fwd(const CUtensorMap& mkv, const Sel16Params& p, int64_t ntasks, cudaStream_t st) {
+  S3R_REQUIRE(ntasks < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_fwd: grid of %lld CTAs is too large", (long long)ntasks);
+  S3R_CUDA(cudaFuncSetAttribute(sel16_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSel16Smem));
+  sel16_fwd_kernel<<<static_cast<unsigned>(ntasks), 32, kSel16Smem, st>>>(mkv, p);
+  S3R_CUDA(cudaGetLastError());
+  return 0;
+}
+
 }  // namespace s3r
 
 using namespace s3r;
@@ -446,6 +702,41 @@ extern "C" int s3r_sel_attn_fwd(const void* q, const void* k, const void* v, int
 
   const int BH = B * H;
   const int Tc = Tk / kv_chunks;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  uint32_t* status = device_status_ptr();
+  S3R_REQUIRE(status != nullptr, S3R_ERR_DRIVER, "s3r_sel_attn_fwd: could not resolve the device status word");
+  if (block == 16) {
+    Sel16Params p;
+    p.q = static_cast<const __nv_bfloat16*>(q);
+    p.idx = idx;
+    p.o_s = static_cast<__nv_bfloat16*>(o_s);
+    p.lse_s = lse_s;
+    p.gate = static_cast<const __nv_bfloat16*>(gate);
+    p.gsb = gate_stride_b; p.gsh = gate_stride_h; p.gst = gate_stride_t;
+    p.o_c = static_cast<const __nv_bfloat16*>(o_c);
+    p.y = static_cast<__nv_bfloat16*>(y);
+    p.H = H; p.Tq = Tq; p.Tk = Tk; p.Tc = Tc;
+    p.nqb = (Tq + 15) / 16;
+    p.topk = topk;
+    p.scale_log2e = scale * 1.4426950408889634f;
+    p.status = status;
+    // keys and values as ONE tensor whose outermost dimension of two steps from one to the other, so that one copy
+    // brings both tiles of a block
+    p.v_first = reinterpret_cast<uintptr_t>(v) < reinterpret_cast<uintptr_t>(k);
+    CUtensorMap mkv;
+    const bool same = k == v;                    // one tile serves as both
+    const uint64_t dims[5] = {64, static_cast<uint64_t>(Tc), static_cast<uint64_t>(BH), static_cast<uint64_t>(kv_chunks), same ? 1u : 2u};
+    const uint64_t apart = p.v_first ? reinterpret_cast<uintptr_t>(k) - reinterpret_cast<uintptr_t>(v)
+                                     : reinterpret_cast<uintptr_t>(v) - reinterpret_cast<uintptr_t>(k);
+    const uint64_t strides[4] = {128, static_cast<uint64_t>(Tc) * 128,
+                                 kv_chunks > 1 ? static_cast<uint64_t>(kv_chunk_stride) * 2 : static_cast<uint64_t>(Tc) * 128 * BH,
+                                 same ? 128 : apart};
+    const uint32_t box[5] = {64, 16, 1, 1, same ? 1u : 2u};
+    p.pair_bytes = same ? 4096 : 8192;
+    const int rc = make_tensor_map(&mkv, p.v_first ? v : k, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    return launch_sel16_fwd(mkv, p, static_cast<int64_t>(BH) * p.nqb, st);
+  }
   CUtensorMap mq, mk, mv;
   {
     uint64_t dims[4] = {64, static_cast<uint64_t>(Tq), static_cast<uint64_t>(BH), 1};
@@ -476,10 +767,7 @@ extern "C" int s3r_sel_attn_fwd(const void* q, const void* k, const void* v, int
   p.nqb = (Tq + block - 1) / block;
   p.topk = topk;
   p.scale_log2e = scale * 1.4426950408889634f;
-  p.status = device_status_ptr();
-  S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_sel_attn_fwd: could not resolve the device status word");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (block == 16) return launch_sel_fwd<16>(mq, mk, mv, p, BH, st);
+  p.status = status;
   if (block == 32) return launch_sel_fwd<32>(mq, mk, mv, p, BH, st);
   return launch_sel_fwd<64>(mq, mk, mv, p, BH, st);
 }

@@ -1,0 +1,59 @@
+"""Edges of single kernels: sizes and layouts at which a tile, a ring or a dispatch rule changes."""
+import pytest
+import torch
+
+from _util import assert_bf16_close, bf16_round
+from oracle import restatement as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def randn(seed, *shape):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed))
+
+
+def table(seed, B, H, nqb, nkb, K):
+    return torch.randint(0, nkb, (B, H, nqb, K), generator=torch.Generator().manual_seed(seed), dtype=torch.int32)
+
+
+# ------------------------------------------------------------------ selection, blocks of 16
+@pytest.mark.parametrize("K", [1, 2, 3, 33, 64])
+@pytest.mark.parametrize("layout", ["k below v", "v below k", "k is v"])
+def test_sel16_fwd_rings_and_layouts(K, layout):
+    """Lists of odd length (the last pair is half empty), one-entry lists, the longest list, a last block cut
+    short, and keys and values in either order in memory (one copy brings both) or the same tensor."""
+    from speed3r_b200 import ops
+    B, H, T = 1, 3, 16 * 21 + 5
+    nb = -(-T // 16)
+    q, k, v = bf16_round(randn(1, B, H, T, 64), randn(2, B, H, T, 64), randn(3, B, H, T, 64))
+    idx = table(4, B, H, nb, nb, K)
+    idx[:, :, 2] = -1                                          # a query block without any valid entry
+    idx[:, :, 3, 0] = nb - 1                                   # the short block
+    buf = torch.empty(2, B, H, T, 64, device=DEV, dtype=torch.bfloat16)
+    kd, vd = (buf[0], buf[1]) if layout == "k below v" else (buf[1], buf[0])
+    kd.copy_(k)
+    if layout == "k is v":
+        v, vd = k, kd
+    else:
+        vd.copy_(v)
+    o, lse, _ = ops._sel_fwd(q.to(DEV, torch.bfloat16), kd, vd, idx.to(DEV), None, None, 16, 0.125, True, True, 1)
+    ref, lse_ref = R.sel_attn(q, k, v, idx, 16)
+    rows = torch.ones(T, dtype=torch.bool)
+    rows[32:48] = False
+    assert_bf16_close(o[:, :, rows.to(DEV)], ref[:, :, rows], f"sel16 K={K} {layout}")
+    assert_bf16_close(lse[:, :, rows.to(DEV)], lse_ref[:, :, rows], "lse", max_abs=5e-3, mean_abs=1e-3, scale_with_ref=False)
+    assert (o[:, :, 32:48] == 0).all() and (lse[:, :, 32:48] == -float("inf")).all()
+
+
+def test_sel16_fwd_offset_follows_growing_scores():
+    """Scores that grow along the list past 2^24 times the first pair's move the exponent offset."""
+    from speed3r_b200 import ops
+    B, H, T, K = 1, 2, 512, 32
+    q, k, v = bf16_round(4 * randn(5, B, H, T, 64), randn(6, B, H, T, 64), randn(7, B, H, T, 64))
+    k, = bf16_round(k * torch.linspace(0.1, 4.0, T).view(1, 1, T, 1))
+    idx = torch.arange(32, dtype=torch.int32).expand(B, H, T // 16, K).contiguous()
+    o, lse, _ = ops._sel_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), idx.to(DEV), None, None, 16, 0.125, True, True, 1)
+    ref, lse_ref = R.sel_attn(q, k, v, idx, 16)
+    assert_bf16_close(o, ref, "growing scores")
+    assert ((lse.cpu() - lse_ref).abs() <= 1e-4 * lse_ref.abs() + 1e-3).all()
