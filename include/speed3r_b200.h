@@ -228,6 +228,18 @@ int s3r_sel_attn_bwd(const void* q, const void* k, const void* v, const int32_t*
                      void* dq, void* dk, void* dv, int B, int H, int Tq, int Tk, int d, int block, int topk,
                      float scale, void* stream);
 
+/* The same with the gradient of the pooled branch (what s3r_pool_bwd would add) folded into the stores, in fp32 and
+ * with one rounding:
+ *   dq[t] += sum over windows j containing t of dq_c[j] / q_kernel   (windows of q_kernel tokens every q_stride)
+ *   dk[t], dv[t] likewise from dk_c, dv_c with k_kernel, k_stride
+ * dq_c [B,H,(Tq-q_kernel)/q_stride+1,d], dk_c / dv_c [B,H,(Tk-k_kernel)/k_stride+1,d]; any of them may be NULL.
+ * Kernels and strides must be multiples of 16. */
+int s3r_sel_attn_bwd_pooled(const void* q, const void* k, const void* v, const int32_t* idx, const int32_t* offsets,
+                            const int32_t* qids, const float* lse_s, const float* delta_s, const void* do_s, void* dq,
+                            void* dk, void* dv, const void* dq_c, const void* dk_c, const void* dv_c, int q_kernel,
+                            int q_stride, int k_kernel, int k_stride, int B, int H, int Tq, int Tk, int d, int block,
+                            int topk, float scale, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Multi-GPU helper of the sequence-partitioned op (the reference is single-GPU: no counterpart).
  * Copies `nseg` (<= 16) segments src[s] -> dst[s] of bytes[s] bytes (multiples of 16, 16-byte aligned)

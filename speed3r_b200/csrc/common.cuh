@@ -41,6 +41,11 @@ int make_tensor_map(CUtensorMap* out, const void* base, int rank, const uint64_t
                     const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle,
                     CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
 
+// Two tensors of the same shape (`chunks` chunks of [BH, T / chunks, 64] bf16) as ONE tensor map whose outermost
+// dimension of two steps from one to the other: a copy of a 16-row box brings 2 KB of each (a's tile first, or
+// b's when *b_first).  a == b: the box has one tile, which serves as both (*b_first = -1).
+int make_pair_map(CUtensorMap* out, const void* a, const void* b, int T, int BH, int chunks, int64_t chunk_stride_bytes, int* b_first);
+
 int sm_count();
 
 #ifdef __CUDACC__
@@ -259,11 +264,10 @@ __device__ __forceinline__ void mma_bf16_z(float (&d)[4], const uint32_t (&a)[4]
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
-// 16 bytes of read-only global memory.  volatile: the load is issued where it is written, ahead of the
-// arithmetic it is meant to overlap.
-__device__ __forceinline__ uint4 ldg128(const uint8_t* p) {
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
   return v;
 }
 

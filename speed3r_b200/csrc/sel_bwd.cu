@@ -4,13 +4,9 @@
 //   dQ    : one warp per 16 query rows, looping over the key blocks its query block selected
 //   dK/dV : one warp per 16 key rows, looping over the query blocks that selected its key block
 //           (CSR lists, ascending query block => a fixed summation order, no atomics on floats)
-// Both stream 16-row tiles through a cp.async ring private to the warp (two stages for dQ, whose list
-// sits in shared memory; three for dK/dV, which also fetches its list and the rows' statistics ahead) and
-// use the mma.sync building blocks of bwd_common.cuh.  Both gather ~130 GB of 128-byte rows out of L2 at
-// 1000 views (16..64 flop per byte): dQ 16 ms, dK/dV 22 ms.
 #include <mutex>
 
-#include "bwd_common.cuh"
+#include "common.cuh"
 
 namespace s3r {
 
@@ -85,16 +81,43 @@ __global__ void csr_fill_kernel(const int32_t* __restrict__ idx, int32_t* __rest
 
 // The fill above leaves every segment complete but in arrival order; the gradient kernel needs ascending
 // query blocks (a fixed summation order).  Segments are sorted by length class:
-//   len <= 32      one warp ranks the segment with shuffles (the common case: the mean length is top-k)
+//   len <= 128     one warp ranks the segment with shuffles, up to four entries per lane (the mean length is top-k;
+//                  with 32 as the limit half of all segments went to the class below: 0.72 of 0.97 ms at 250 views)
 //   len <= 4096    one CTA, bitonic network in shared memory
 //   longer         ("sink" key blocks that most query blocks select) one CTA walks the (b,h) slice of the
 //                  table in order and compacts the matching query blocks: O(Nq*topk), no comparison sort
 // The first kernel handles the short class and queues every other segment for the second.
 constexpr int kCsrSmemSort = 4096;
+constexpr int kCsrWarpSort = 128;
+
+// Ranks len <= 32 * N entries; entry and position make one unsigned key, so that equal entries keep an order.
+template <int N>
+__device__ __forceinline__ void csr_rank_sort(const int32_t* src, int32_t* dst, int len, int lane) {
+  uint32_t key[N];
+  int rank[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int pos = lane + 32 * i;
+    key[i] = pos < len ? static_cast<uint32_t>(src[pos]) * kCsrWarpSort + pos : 0xffffffffu;
+    rank[i] = 0;
+  }
+#pragma unroll
+  for (int ch = 0; ch < N; ++ch) {
+    const int n = min(32, len - 32 * ch);
+    for (int t = 0; t < n; ++t) {
+      const uint32_t y = __shfl_sync(0xffffffffu, key[ch], t);
+#pragma unroll
+      for (int i = 0; i < N; ++i) rank[i] += y < key[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (lane + 32 * i < len) dst[rank[i]] = static_cast<int32_t>(key[i] / kCsrWarpSort);
+}
 
 __global__ void __launch_bounds__(256) csr_sort_small_kernel(const int32_t* __restrict__ offsets,
                                                              const int32_t* __restrict__ tmp, int32_t* __restrict__ qids,
-                                                             int64_t per_bh, int Nkb, int64_t nseg,
+                                                             int64_t per_bh, int Nkb, int64_t nseg, int warp_max,
                                                              int32_t* __restrict__ queue) {
   const int lane = threadIdx.x & 31;
   const int64_t seg = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
@@ -103,17 +126,17 @@ __global__ void __launch_bounds__(256) csr_sort_small_kernel(const int32_t* __re
   const int n = static_cast<int>(seg - bh * Nkb);
   const int32_t* off = offsets + bh * (Nkb + 1);
   const int beg = off[n], len = off[n + 1] - beg;
-  if (len > 32) {
+  const int32_t* src = tmp + bh * per_bh + beg;
+  int32_t* dst = qids + bh * per_bh + beg;
+  if (len > warp_max) {
     if (lane == 0) queue[1 + atomicAdd(&queue[0], 1)] = static_cast<int32_t>(seg);
-    return;
+  } else if (len <= 32) {
+    csr_rank_sort<1>(src, dst, len, lane);
+  } else if (len <= 64) {
+    csr_rank_sort<2>(src, dst, len, lane);
+  } else {
+    csr_rank_sort<4>(src, dst, len, lane);
   }
-  const int32_t x = (lane < len) ? tmp[bh * per_bh + beg + lane] : 0x7fffffff;
-  int rank = 0;
-  for (int t = 0; t < len; ++t) {
-    const int32_t yt = __shfl_sync(0xffffffffu, x, t);
-    rank += (yt < x) || (yt == x && t < lane);
-  }
-  if (lane < len) qids[bh * per_bh + beg + rank] = x;
 }
 
 __global__ void __launch_bounds__(256) csr_sort_long_kernel(const int32_t* __restrict__ idx,
@@ -190,6 +213,84 @@ __global__ void __launch_bounds__(256) csr_sort_long_kernel(const int32_t* __res
         __syncthreads();
         if (tid == 0) run_base += total;
         __syncthreads();
+      }
+    }
+  }
+}
+
+// Short tables: one CTA builds the whole index of a (b,h) in shared memory - one launch instead of two memsets and five
+// kernels (68 us at 384 query blocks, top-32, 32 heads, most of it launches and the long-segment kernel).  The line at
+// kCsrOneEntries entries per (b,h) is where a CTA's passes over its table begin to outlast them (few CTAs: one per b,h).
+constexpr int kCsrOneEntries = 24576, kCsrOneKeys = 8192;
+
+__global__ void __launch_bounds__(1024) csr_one_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ offsets,
+                                                       int32_t* __restrict__ qids, int per_bh, int Nkb, int topk) {
+  extern __shared__ int32_t one_smem[];
+  int32_t* cur = one_smem;                   // counts, then the fill's cursors (= end of each segment afterwards)
+  int32_t* ent = one_smem + Nkb;             // query blocks by segment, arrival order
+  __shared__ int32_t warp_sums[32];
+  __shared__ int32_t carry_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int32_t* tab = idx + static_cast<int64_t>(blockIdx.x) * per_bh;
+  int32_t* off = offsets + static_cast<int64_t>(blockIdx.x) * (Nkb + 1);
+  int32_t* out = qids + static_cast<int64_t>(blockIdx.x) * per_bh;
+  for (int i = tid; i < Nkb; i += 1024) cur[i] = 0;
+  if (tid == 0) carry_s = 0;
+  __syncthreads();
+  for (int i = tid; i < per_bh; i += 1024) {
+    const int n = tab[i];
+    if (n >= 0 && n < Nkb) atomicAdd(&cur[n], 1);
+  }
+  __syncthreads();
+  for (int base = 0; base < Nkb; base += 1024) {             // exclusive scan in place
+    const int i = base + tid;
+    const int32_t v = i < Nkb ? cur[i] : 0;
+    int32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      int32_t w = warp_sums[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int32_t y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+      }
+      warp_sums[lane] = w;
+    }
+    __syncthreads();
+    const int32_t carry = carry_s, excl = carry + (warp > 0 ? warp_sums[warp - 1] : 0) + x - v;
+    if (i < Nkb) {
+      cur[i] = excl;
+      off[i] = excl;
+    }
+    __syncthreads();
+    if (tid == 1023) carry_s = carry + warp_sums[31];
+    __syncthreads();
+  }
+  if (tid == 0) off[Nkb] = carry_s;
+  for (int i = tid; i < per_bh; i += 1024) {
+    const int n = tab[i];
+    if (n >= 0 && n < Nkb) ent[atomicAdd(&cur[n], 1)] = i / topk;
+  }
+  __syncthreads();
+  for (int n = warp; n < Nkb; n += 32) {
+    const int beg = n > 0 ? cur[n - 1] : 0, len = cur[n] - beg;
+    if (len == 0) continue;
+    if (len <= 32) csr_rank_sort<1>(ent + beg, out + beg, len, lane);
+    else if (len <= 64) csr_rank_sort<2>(ent + beg, out + beg, len, lane);
+    else if (len <= kCsrWarpSort) csr_rank_sort<4>(ent + beg, out + beg, len, lane);
+    else {                                                   // ordered compaction over the table
+      int at = beg;
+      for (int base = 0; base < per_bh; base += 32) {
+        const bool hit = base + lane < per_bh && tab[base + lane] == n;
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        if (hit) out[at + __popc(m & ((1u << lane) - 1u))] = (base + lane) / topk;
+        at += __popc(m);
       }
     }
   }
@@ -304,206 +405,374 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
 // ------------------------------------------------------------------------------------------------
 // sparse dQ and dK/dV
 // ------------------------------------------------------------------------------------------------
-constexpr int kBwdWarps = 4;
-constexpr int kTile = 16 * kPitch;            // one 16-row tile in shared memory
-
+// Both kernels: one warp = one CTA owns 16 rows (queries | keys) and meets tiles of 16 rows of the other side, two at
+// a time, out of a ring of two 8 KB stages; one TMA copy brings a tile of two tensors (K and V | Q and dO).
+// Fragments are loaded ahead of the products that use them.  Softmax scale: applied once, to the accumulators.
+// Bound: shared memory (a tile is written once and read as three | four 2 KB fragment sets: 10 | 12 KB of traffic per
+// 4 KB gathered, at 128 bytes per cycle) and, close behind, mma.sync (24 | 32 of 8 cycles per tile and sub-partition);
+// what is missing to either is latency that twelve warps per SM (registers, rings) do not cover.  In the dQ kernel the
+// second tile's loads run under the first tile's exponentials (919 -> 638 us at 64 views, H = 16, top-32); the same
+// order in the dK/dV kernel needs more registers than it gains: with the tiles one after the other 1161 -> 937 us, with
+// eight or nine warps and the tiles overlapped 1110 us.
 struct SelBwdParams {
   const __nv_bfloat16 *q, *k, *v, *d_o;
   const int32_t *idx, *offsets, *qids;
   const float *lse, *delta;
   __nv_bfloat16 *dq, *dk, *dv;
-  int B, H, Tq, Tk, block, topk, nqb, nkb;
+  // gradient of the pooled branch, added to dq | dk, dv (null: none): element t of dq gets dq_c[j] / kernel of every
+  // window j that contains it.  Kernel and stride are multiples of 16, so a warp's 16 rows share their windows.
+  const __nv_bfloat16 *dq_c, *dk_c, *dv_c;
+  int q_kernel, q_stride, q_windows, k_kernel, k_stride, k_windows;
+  int B, H, Tq, Tk, block, block_shift, topk, nqb, nkb;     // block = 16 << block_shift
+  int first_kv, first_qdo;       // order of the tiles a copy brings (make_pair_map)
   float cs, scale;
+  uint32_t* status;
 };
 
-// 16 rows x 128 B from global (row stride 64 elements) into a padded tile; rows >= nrows zero-filled
-__device__ __forceinline__ void load_tile16(uint32_t dst, const __nv_bfloat16* src, int nrows, int lane) {
+constexpr int kSbStageBytes = 8192;
+constexpr int kSbSmem = 2 * kSbStageBytes + 1024;
+
+// sum over the windows that contain rows row0..row0+15, this lane's columns (8 dt + 2c, +1)
+__device__ __forceinline__ void add_pooled(float (&acc)[8][4], const __nv_bfloat16* g_c, int bh, int row0, int kernel,
+                                           int stride, int windows, int c) {
+  if (g_c == nullptr) return;
+  const int hi = min(windows - 1, row0 / stride), lo = row0 + 16 <= kernel ? 0 : (row0 + 16 - kernel + stride - 1) / stride;
+  const float inv = 1.0f / static_cast<float>(kernel);
+  for (int j = lo; j <= hi; ++j) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(g_c + (static_cast<int64_t>(bh) * windows + j) * 64) + c;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int ch = lane + 32 * i, r = ch >> 3, c16 = ch & 7;
-    cp_async16(dst + r * kPitch + c16 * 16, src + static_cast<int64_t>(r) * 64 + c16 * 8, r < nrows);
+    for (int dt = 0; dt < 8; ++dt) {
+      const uint32_t w = __ldg(src + dt * 4);
+      const float a = bf16_lo(w) * inv, b = bf16_hi(w) * inv;
+      acc[dt][0] += a; acc[dt][1] += b; acc[dt][2] += a; acc[dt][3] += b;
+    }
   }
 }
+// 16 x 64 accumulators -> bf16 rows of 128 bytes, through 2 KB of shared memory of this warp
+__device__ __forceinline__ void store_rows16(const float (&acc)[8][4], uint32_t tile, uint8_t* dst, int nrows, int lane) {
+  const int g = lane >> 2, c = lane & 3;
+#pragma unroll
+  for (int dt = 0; dt < 8; ++dt) {
+    sts32(tile + swz128(g, dt) + 4 * c, pack_bf16(acc[dt][0], acc[dt][1]));
+    sts32(tile + swz128(g + 8, dt) + 4 * c, pack_bf16(acc[dt][2], acc[dt][3]));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = (lane >> 3) + 4 * i;
+    if (r < nrows) *reinterpret_cast<uint4*>(dst + r * 128 + (lane & 7) * 16) = lds128(tile + swz128(r, lane & 7));
+  }
+  __syncwarp();
+}
+// A-operand fragments of 16 rows straight from global memory (rows of 128 bytes; rows >= nrows repeat the last)
+__device__ __forceinline__ void ldg_a_frags(uint32_t (&f)[4][4], const __nv_bfloat16* rows, int nrows, int lane) {
+  const int g = lane >> 2, c = lane & 3;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(rows) + min(g + 8 * r, nrows - 1) * 32 + c;
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      f[ks][r] = __ldg(src + ks * 8);
+      f[ks][r + 2] = __ldg(src + ks * 8 + 4);
+    }
+  }
+}
+// B-operand fragments of a swizzled 16-row tile: rows as n (off_n) or, transposed, rows as k (off_k)
+__device__ __forceinline__ void frags_n(uint32_t (&f)[4][4], uint32_t tile, const uint32_t (&off)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) ldsm_x4(f[i][0], f[i][1], f[i][2], f[i][3], tile + off[i]);
+}
+__device__ __forceinline__ void frags_k(uint32_t (&f)[4][4], uint32_t tile, const uint32_t (&off)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) ldsm_x4_t(f[i][0], f[i][1], f[i][2], f[i][3], tile + off[i]);
+}
+// x = X Y^T, y = Z W^T for 16 x 16 tiles over 64 channels: four independent chains of four
+__device__ __forceinline__ void two_products(float (&x)[2][4], float (&y)[2][4], const uint32_t (&xa)[4][4],
+                                             const uint32_t (&xb)[4][4], const uint32_t (&ya)[4][4], const uint32_t (&yb)[4][4]) {
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (ks == 0) {
+        mma_bf16_z(x[t], xa[ks], xb[ks][2 * t], xb[ks][2 * t + 1]);
+        mma_bf16_z(y[t], ya[ks], yb[ks][2 * t], yb[ks][2 * t + 1]);
+      } else {
+        mma_bf16(x[t], xa[ks], xb[ks][2 * t], xb[ks][2 * t + 1]);
+        mma_bf16(y[t], ya[ks], yb[ks][2 * t], yb[ks][2 * t + 1]);
+      }
+    }
+}
+__device__ __forceinline__ void accumulate(float (&acc)[8][4], const uint32_t (&a)[4], const uint32_t (&b)[4][4]) {
+#pragma unroll
+  for (int dp = 0; dp < 4; ++dp) {
+    mma_bf16(acc[2 * dp], a, b[dp][0], b[dp][1]);
+    mma_bf16(acc[2 * dp + 1], a, b[dp][2], b[dp][3]);
+  }
+}
+struct SbLane {                    // this lane's ldmatrix offsets inside a swizzled tile
+  uint32_t off_n[4], off_k[4];
+  __device__ __forceinline__ explicit SbLane(int lane) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      off_n[i] = swz128((lane & 7) + (lane >> 4) * 8, 2 * i + ((lane >> 3) & 1));
+      off_k[i] = swz128((lane & 7) + ((lane >> 3) & 1) * 8, 2 * i + (lane >> 4));
+    }
+  }
+};
 
-#ifndef S3R_DQ_MIN_CTAS
-#define S3R_DQ_MIN_CTAS 1
-#endif
-__global__ void __launch_bounds__(kBwdWarps * 32, S3R_DQ_MIN_CTAS) sel_bwd_dq_kernel(const SelBwdParams p) {
-  __shared__ __align__(16) uint8_t smem[kBwdWarps][2][2 * kTile];
-  __shared__ int32_t lists[kBwdWarps][64];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2;
+__global__ void __launch_bounds__(32, 10) sel_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_kv, const SelBwdParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ int32_t list[64];                        // first token of each valid key block, table order
+  __shared__ uint64_t full[2];
+  __shared__ uint32_t abort_word;
+  const int lane = threadIdx.x, g = lane >> 2, c = lane & 3;
   const int nslices = (p.Tq + 15) / 16;
-  const int64_t task = static_cast<int64_t>(blockIdx.x) * kBwdWarps + warp;
-  if (task >= static_cast<int64_t>(p.B) * p.H * nslices) return;
-  const int bh = static_cast<int>(task / nslices);
-  const int row0 = static_cast<int>(task % nslices) * 16;
-  const int m = row0 / p.block;
-  const uint32_t sm0 = smem_u32(&smem[warp][0][0]), sm1 = smem_u32(&smem[warp][1][0]);
-
-  // valid entries of the query block's row of the table, table order
+  const int64_t task = blockIdx.x;
+  const int bh = static_cast<int>(task / nslices), row0 = static_cast<int>(task % nslices) * 16;
+  const int nrows = min(16, p.Tq - row0);
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  volatile uint32_t* abort_flag = &abort_word;
+  if (lane == 0) {
+    abort_word = 0;
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    mbar_fence_init();
+  }
   int nvalid = 0;
   {
-    const int32_t* row = p.idx + (static_cast<int64_t>(bh) * p.nqb + m) * p.topk;
+    const int32_t* row = p.idx + (static_cast<int64_t>(bh) * p.nqb + (row0 >> (4 + p.block_shift))) * p.topk;
     for (int r0 = 0; r0 < p.topk; r0 += 32) {
       const int i = r0 + lane;
       const int n = (i < p.topk) ? row[i] : -1;
       const bool ok = (n >= 0) && (static_cast<int64_t>(n) * p.block < p.Tk);
       const uint32_t bal = __ballot_sync(0xffffffffu, ok);
-      if (ok) lists[warp][nvalid + __popc(bal & ((1u << lane) - 1u))] = n;
+      if (ok) list[nvalid + __popc(bal & ((1u << lane) - 1u))] = n * p.block;
       nvalid += __popc(bal);
     }
     __syncwarp();
   }
-  const __nv_bfloat16* Kb = p.k + static_cast<int64_t>(bh) * p.Tk * 64;
-  const __nv_bfloat16* Vb = p.v + static_cast<int64_t>(bh) * p.Tk * 64;
+  const int ntiles = nvalid << p.block_shift, npairs = (ntiles + 1) >> 1, in_block = (1 << p.block_shift) - 1;
+  auto tok_of = [&](int t) { return list[t >> p.block_shift] + ((t & in_block) << 4); };
+  auto issue = [&](int pair, int s) {
+    if (lane == 0) {
+      const int t = 2 * pair;
+      mbar_expect_tx(&full[s], (t + 1 < ntiles ? 8192u : 4096u) >> (p.first_kv < 0));
+      tma_load_5d(ring + s * kSbStageBytes, &map_kv, &full[s], 0, tok_of(t), bh, 0, 0);
+      if (t + 1 < ntiles) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_kv, &full[s], 0, tok_of(t + 1), bh, 0, 0);
+    }
+  };
+  if (npairs > 0) issue(0, 0);
+  if (npairs > 1) issue(1, 1);
 
-  // Q and dO fragments (through stage 0)
   uint32_t qf[4][4], dof[4][4];
-  const int qrows = min(16, p.Tq - row0);
-  load_tile16(sm0, p.q + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, qrows, lane);
-  load_tile16(sm0 + kTile, p.d_o + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, qrows, lane);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncwarp();
-  load_a_frags(qf, sm0, lane);
-  load_a_frags(dof, sm0 + kTile, lane);
-  __syncwarp();
+  ldg_a_frags(qf, p.q + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, nrows, lane);
+  ldg_a_frags(dof, p.d_o + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, nrows, lane);
   float lse2[2], delta[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const int t = row0 + g + 8 * r;
-    float l = (t < p.Tq) ? p.lse[static_cast<int64_t>(bh) * p.Tq + t] : INFINITY;
-    if (l == -INFINITY) l = INFINITY;                 // row without any valid key: no gradient
-    lse2[r] = l * 1.4426950408889634f;
-    delta[r] = (t < p.Tq) ? p.delta[static_cast<int64_t>(bh) * p.Tq + t] : 0.f;
+    const int64_t t = static_cast<int64_t>(bh) * p.Tq + row0 + min(g + 8 * r, nrows - 1);
+    lse2[r] = p.lse[t] * 1.4426950408889634f;         // finite wherever the list is not empty
+    delta[r] = p.delta[t];
   }
-  float dq[8][4] = {};
+  const SbLane of(lane);
+  const uint32_t k_at = p.first_kv > 0 ? 2048u : 0u, v_at = p.first_kv == 0 ? 2048u : 0u;
+  const bool ragged = (p.Tk & 15) != 0 || (p.Tk & (p.block - 1)) != 0;
 
-  const int spb = p.block / 16;                       // 16-key tiles per key block
-  const int ntiles = nvalid * spb;
-  auto prefetch = [&](int it) {
-    const int tok0 = lists[warp][it / spb] * p.block + (it % spb) * 16;
-    const uint32_t dst = (it & 1) ? sm1 : sm0;
-    const int nrows = min(16, p.Tk - tok0);
-    load_tile16(dst, Kb + static_cast<int64_t>(tok0) * 64, nrows, lane);
-    load_tile16(dst + kTile, Vb + static_cast<int64_t>(tok0) * 64, nrows, lane);
-    cp_async_commit();
-  };
-  if (ntiles > 0) prefetch(0);
-  for (int it = 0; it < ntiles; ++it) {
-    if (it + 1 < ntiles) { prefetch(it + 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
+  float dq[8][4] = {};
+#pragma unroll 1
+  for (int it = 0; it < npairs; ++it) {
+    const int S = it & 1;
+    if (!mbar_wait_warp(&full[S], (it >> 1) & 1, abort_flag)) {
+      volatile uint32_t dummy = 0;                    // a last bounded chance for the other stage's copies to land
+      if (it + 1 < npairs) mbar_wait(&full[S ^ 1], ((it + 1) >> 1) & 1, &dummy);
+      if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+      return;
+    }
+    const uint32_t st = ring + S * kSbStageBytes;
+    const bool both = 2 * it + 1 < ntiles;
+    uint32_t kn0[4][4], kn1[4][4], vn0[4][4], vn1[4][4], kk0[4][4], kk1[4][4];
+    float s0[2][4], dp0[2][4], s1[2][4], dp1[2][4];
+    auto grad = [&](float (&s)[2][4], const float (&dp)[2][4], int t, uint32_t (&a)[4]) {
+      const int left = ragged ? p.Tk - tok_of(t) : 16;
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float pr = fast_exp2(fmaf(s[nt][e], p.cs, -lse2[e >> 1]));
+          if (ragged && nt * 8 + 2 * c + (e & 1) >= left) pr = 0.f;
+          s[nt][e] = pr * (dp[nt][e] - delta[e >> 1]);
+        }
+      a[0] = pack_bf16(s[0][0], s[0][1]); a[1] = pack_bf16(s[0][2], s[0][3]);
+      a[2] = pack_bf16(s[1][0], s[1][1]); a[3] = pack_bf16(s[1][2], s[1][3]);
+    };
+    uint32_t a0[4], a1[4];
+    frags_n(kn0, st + k_at, of.off_n);
+    frags_n(vn0, st + v_at, of.off_n);
+    two_products(s0, dp0, qf, kn0, dof, vn0);
+    frags_k(kk0, st + k_at, of.off_k);
+    if (both) {
+      frags_n(kn1, st + 4096 + k_at, of.off_n);
+      frags_n(vn1, st + 4096 + v_at, of.off_n);
+      grad(s0, dp0, 2 * it, a0);
+      two_products(s1, dp1, qf, kn1, dof, vn1);
+      accumulate(dq, a0, kk0);
+      frags_k(kk1, st + 4096 + k_at, of.off_k);
+      grad(s1, dp1, 2 * it + 1, a1);
+      accumulate(dq, a1, kk1);
+    } else {
+      grad(s0, dp0, 2 * it, a0);
+      accumulate(dq, a0, kk0);
+    }
     __syncwarp();
-    const int tok0 = lists[warp][it / spb] * p.block + (it % spb) * 16;
-    const uint32_t cur = (it & 1) ? sm1 : sm0;
-    pair_dq(qf, dof, lse2, delta, cur, cur + kTile, min(16, p.Tk - tok0), p.cs, p.scale, dq, lane);
-    __syncwarp();
+    if (it + 2 < npairs) issue(it + 2, S);            // every fragment of the stage has been consumed
   }
-  __nv_bfloat16* out = p.dq + (static_cast<int64_t>(bh) * p.Tq + row0) * 64;
-  store_acc_bf16(dq, [&](int r) { return (row0 + r < p.Tq) ? out + r * 64 : nullptr; }, lane);
+#pragma unroll
+  for (int dt = 0; dt < 8; ++dt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dq[dt][e] *= p.scale;
+  add_pooled(dq, p.dq_c, bh, row0, p.q_kernel, p.q_stride, p.q_windows, c);
+  __syncwarp();
+  store_rows16(dq, ring, reinterpret_cast<uint8_t*>(p.dq + (static_cast<int64_t>(bh) * p.Tq + row0) * 64), nrows, lane);
 }
 
-// The loop over the query blocks that selected this key block is a chain of dependent accesses (list
-// entry -> row addresses -> rows and their lse/delta), so everything is fetched ahead: the list 32 entries
-// at a time into a register per lane (read back with a shuffle), rows and statistics by cp.async into a
-// ring kDkdvStages deep.  Nothing in the loop waits for a load it has just issued.
-// One warp per CTA: the loop length of a warp is the number of query blocks that selected its key block,
-// which varies from warp to warp; warps sharing a CTA would hold its registers and shared memory until the
-// longest of them is done.
-#ifndef S3R_DKDV_WARPS
-#define S3R_DKDV_WARPS 1
-#endif
-#ifndef S3R_DKDV_MIN_CTAS
-#define S3R_DKDV_MIN_CTAS 16               // caps the kernel at 128 registers: 16 instead of 10 warps per SM
-#endif
-#ifndef S3R_DKDV_STAGES
-#define S3R_DKDV_STAGES 3
-#endif
-constexpr int kDkdvWarps = S3R_DKDV_WARPS;
-constexpr int kDkdvStages = S3R_DKDV_STAGES;
-constexpr int kDkdvStageBytes = 2 * kTile + 128;          // Q tile, dO tile, 16 x lse | 16 x delta
-constexpr int kDkdvSmemBytes = kDkdvWarps * kDkdvStages * kDkdvStageBytes;
-
-__global__ void __launch_bounds__(kDkdvWarps * 32, S3R_DKDV_MIN_CTAS) sel_bwd_dkdv_kernel(const SelBwdParams p) {
-  extern __shared__ __align__(16) uint8_t dkdv_smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// The list of query blocks that selected this warp's key block comes 32 entries at a time into a register per
+// lane, the statistics of a tile's rows one load ahead of their use.
+__global__ void __launch_bounds__(32, 10) sel_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_qdo, const SelBwdParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) float stats[2][32];         // [tile of the pair][lse2 x 16 | delta x 16]
+  __shared__ uint64_t full[2];
+  __shared__ uint32_t abort_word;
+  const int lane = threadIdx.x, c = lane & 3;
   const int nslices = (p.Tk + 15) / 16;
-  const int64_t task = static_cast<int64_t>(blockIdx.x) * kDkdvWarps + warp;
-  if (task >= static_cast<int64_t>(p.B) * p.H * nslices) return;
-  const int bh = static_cast<int>(task / nslices);
-  const int row0 = static_cast<int>(task % nslices) * 16;
-  const int n = row0 / p.block;
-  uint8_t* my = dkdv_smem + warp * kDkdvStages * kDkdvStageBytes;
-  const uint32_t sm0 = smem_u32(my);
-
-  uint32_t kf[4][4], vf[4][4];
-  const int krows = min(16, p.Tk - row0);
-  load_tile16(sm0, p.k + (static_cast<int64_t>(bh) * p.Tk + row0) * 64, krows, lane);
-  load_tile16(sm0 + kTile, p.v + (static_cast<int64_t>(bh) * p.Tk + row0) * 64, krows, lane);
-  cp_async_commit();
-  cp_async_wait<0>();
+  const int64_t task = blockIdx.x;
+  const int bh = static_cast<int>(task / nslices), row0 = static_cast<int>(task % nslices) * 16;
+  const int nrows = min(16, p.Tk - row0);
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  volatile uint32_t* abort_flag = &abort_word;
+  if (lane == 0) {
+    abort_word = 0;
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    mbar_fence_init();
+  }
   __syncwarp();
-  load_a_frags(kf, sm0, lane);
-  load_a_frags(vf, sm0 + kTile, lane);
-  __syncwarp();
-
-  const int32_t* off = p.offsets + static_cast<int64_t>(bh) * (p.nkb + 1);
-  const int beg = off[n], cnt = off[n + 1] - beg;
+  const int n = row0 >> (4 + p.block_shift);
+  const int32_t* off = p.offsets + static_cast<int64_t>(bh) * (p.nkb + 1) + n;
+  const int beg = off[0], cnt = off[1] - beg;
   const int32_t* ql = p.qids + static_cast<int64_t>(bh) * p.nqb * p.topk + beg;
-  const __nv_bfloat16* Qb = p.q + static_cast<int64_t>(bh) * p.Tq * 64;
-  const __nv_bfloat16* Db = p.d_o + static_cast<int64_t>(bh) * p.Tq * 64;
-  const float* Lb = p.lse + static_cast<int64_t>(bh) * p.Tq;
-  const float* Eb = p.delta + static_cast<int64_t>(bh) * p.Tq;
-
-  float dk[8][4] = {}, dv[8][4] = {};
-  const int spb = p.block / 16;
-  const int ntiles = cnt * spb;
-  // list entries of chunk c (32 of them) live in `q_cur`, those of chunk c+1 in `q_nxt`
+  const int ntiles = cnt << p.block_shift, npairs = (ntiles + 1) >> 1, in_block = (1 << p.block_shift) - 1;
+  // list entries of chunk c (32 of them) live in `q_cur`, those of chunk c+1 in `q_nxt`; called with growing t only
   int q_chunk = 0;
   int q_cur = (lane < cnt) ? ql[lane] : 0;
   int q_nxt = (32 + lane < cnt) ? ql[32 + lane] : 0;
-  auto prefetch = [&](int it) {
-    const int qb = it / spb;
-    if ((qb >> 5) != q_chunk) {                       // warp-uniform
-      q_chunk = qb >> 5;
+  auto tok_of = [&](int t) {
+    const int e = t >> p.block_shift;
+    if ((e >> 5) != q_chunk) {                         // warp-uniform
+      q_chunk = e >> 5;
       q_cur = q_nxt;
       const int j = (q_chunk + 1) * 32 + lane;
       q_nxt = (j < cnt) ? ql[j] : 0;
     }
-    const int tok0 = __shfl_sync(0xffffffffu, q_cur, qb & 31) * p.block + (it % spb) * 16;
-    const uint32_t dst = sm0 + (it % kDkdvStages) * kDkdvStageBytes;
-    const int nrows = max(0, min(16, p.Tq - tok0));
-    load_tile16(dst, Qb + static_cast<int64_t>(tok0) * 64, nrows, lane);
-    load_tile16(dst + kTile, Db + static_cast<int64_t>(tok0) * 64, nrows, lane);
-    // per-query statistics: lanes 0-15 lse, lanes 16-31 delta (a padding query gets 0 and 0: its Q and dO
-    // rows are zero as well, so P = 1 meets dO = 0 and dP - delta = 0)
-    const int t = tok0 + (lane & 15);
-    cp_async4(dst + 2 * kTile + lane * 4, (lane < 16 ? Lb : Eb) + min(t, p.Tq - 1), t < p.Tq);
-    cp_async_commit();
+    return (__shfl_sync(0xffffffffu, q_cur, e & 31) << (4 + p.block_shift)) + ((t & in_block) << 4);
   };
-#pragma unroll
-  for (int a = 0; a < kDkdvStages - 1; ++a) {
-    if (a < ntiles) prefetch(a); else cp_async_commit();
-  }
-  for (int it = 0; it < ntiles; ++it) {
-    if (it + kDkdvStages - 1 < ntiles) prefetch(it + kDkdvStages - 1); else cp_async_commit();
-    cp_async_wait<kDkdvStages - 1>();
-    __syncwarp();
-    uint8_t* st = my + (it % kDkdvStages) * kDkdvStageBytes;
-    float* stats = reinterpret_cast<float*>(st + 2 * kTile);
-    if (lane < 16) {                                  // lse -> lse * log2(e); a row without any valid key: no gradient
-      const float l = stats[lane];
-      stats[lane] = (l == -INFINITY) ? INFINITY : l * 1.4426950408889634f;
+  auto issue = [&](int t0, int t1, bool both, int s) {
+    if (lane == 0) {
+      mbar_expect_tx(&full[s], (both ? 8192u : 4096u) >> (p.first_qdo < 0));
+      tma_load_5d(ring + s * kSbStageBytes, &map_qdo, &full[s], 0, t0, bh, 0, 0);
+      if (both) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_qdo, &full[s], 0, t1, bh, 0, 0);
     }
-    __syncwarp();
-    const uint32_t cur = smem_u32(st);
-    pair_dkdv(kf, vf, cur, cur + kTile, stats, stats + 16, p.cs, p.scale, dk, dv, lane);
-    __syncwarp();
+  };
+  // lanes 0-15 fetch lse, lanes 16-31 delta of a tile's rows; a row past the end gets lse = +inf: P is exactly 0
+  const float* stat_src = (lane < 16 ? p.lse : p.delta) + static_cast<int64_t>(bh) * p.Tq;
+  auto stat = [&](int tok0) {
+    const int t = tok0 + (lane & 15);
+    const float x = __ldg(stat_src + min(t, p.Tq - 1));
+    return lane >= 16 ? x : (t < p.Tq ? x * 1.4426950408889634f : INFINITY);
+  };
+  // tokens of the next pair to be computed (their copies are under way) and its statistics
+  int na = 0, nb = 0;
+  float sa = 0.f, sb = 0.f;
+  int ta = 0, tb = 0;
+  if (npairs > 0) {
+    na = tok_of(0);
+    nb = 1 < ntiles ? tok_of(1) : na;
+    issue(na, nb, 1 < ntiles, 0);
+    sa = stat(na);
+    sb = stat(nb);
   }
-  __nv_bfloat16* okp = p.dk + (static_cast<int64_t>(bh) * p.Tk + row0) * 64;
-  __nv_bfloat16* ovp = p.dv + (static_cast<int64_t>(bh) * p.Tk + row0) * 64;
-  store_acc_bf16(dk, [&](int r) { return (row0 + r < p.Tk) ? okp + r * 64 : nullptr; }, lane);
-  store_acc_bf16(dv, [&](int r) { return (row0 + r < p.Tk) ? ovp + r * 64 : nullptr; }, lane);
+  if (npairs > 1) {
+    ta = tok_of(2);
+    tb = 3 < ntiles ? tok_of(3) : ta;
+    issue(ta, tb, 3 < ntiles, 1);
+  }
+  uint32_t kf[4][4], vf[4][4];
+  ldg_a_frags(kf, p.k + (static_cast<int64_t>(bh) * p.Tk + row0) * 64, nrows, lane);
+  ldg_a_frags(vf, p.v + (static_cast<int64_t>(bh) * p.Tk + row0) * 64, nrows, lane);
+  const SbLane of(lane);
+  const uint32_t q_at = p.first_qdo > 0 ? 2048u : 0u, do_at = p.first_qdo == 0 ? 2048u : 0u;
+
+  float dk[8][4] = {}, dv[8][4] = {};
+#pragma unroll 1
+  for (int it = 0; it < npairs; ++it) {
+    const int S = it & 1;
+    stats[0][lane] = sa;
+    stats[1][lane] = sb;
+    __syncwarp();
+    if (it + 1 < npairs) { sa = stat(ta); sb = stat(tb); }
+    if (!mbar_wait_warp(&full[S], (it >> 1) & 1, abort_flag)) {
+      volatile uint32_t dummy = 0;                    // a last bounded chance for the other stage's copies to land
+      if (it + 1 < npairs) mbar_wait(&full[S ^ 1], ((it + 1) >> 1) & 1, &dummy);
+      if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+      return;
+    }
+    const uint32_t st = ring + S * kSbStageBytes;
+    // P^T and dS^T of a tile, packed as A operands
+    auto grad = [&](float (&s)[2][4], const float (&dp)[2][4], int j, uint32_t (&pa)[4], uint32_t (&da)[4]) {
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const float2 l2 = *reinterpret_cast<const float2*>(&stats[j][nt * 8 + 2 * c]);
+        const float2 d2 = *reinterpret_cast<const float2*>(&stats[j][16 + nt * 8 + 2 * c]);
+        float ds[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[nt][e] = fast_exp2(fmaf(s[nt][e], p.cs, -((e & 1) ? l2.y : l2.x)));
+          ds[e] = s[nt][e] * (dp[nt][e] - ((e & 1) ? d2.y : d2.x));
+        }
+        pa[2 * nt] = pack_bf16(s[nt][0], s[nt][1]); pa[2 * nt + 1] = pack_bf16(s[nt][2], s[nt][3]);
+        da[2 * nt] = pack_bf16(ds[0], ds[1]); da[2 * nt + 1] = pack_bf16(ds[2], ds[3]);
+      }
+    };
+    auto tile = [&](int j) {
+      uint32_t qn[4][4], dn[4][4], qk[4][4], dkk[4][4], pa[4], da[4];
+      float s[2][4], dp[2][4];
+      frags_n(qn, st + j * 4096 + q_at, of.off_n);
+      frags_n(dn, st + j * 4096 + do_at, of.off_n);
+      two_products(s, dp, kf, qn, vf, dn);
+      frags_k(dkk, st + j * 4096 + do_at, of.off_k);
+      frags_k(qk, st + j * 4096 + q_at, of.off_k);
+      grad(s, dp, j, pa, da);
+      accumulate(dv, pa, dkk);
+      accumulate(dk, da, qk);
+    };
+    tile(0);
+    if (2 * it + 1 < ntiles) tile(1);
+    __syncwarp();
+    if (it + 2 < npairs) {                            // every fragment of the stage has been consumed
+      ta = tok_of(2 * it + 4);
+      tb = 2 * it + 5 < ntiles ? tok_of(2 * it + 5) : ta;
+      issue(ta, tb, 2 * it + 5 < ntiles, S);
+    }
+  }
+#pragma unroll
+  for (int dt = 0; dt < 8; ++dt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dk[dt][e] *= p.scale;
+  add_pooled(dk, p.dk_c, bh, row0, p.k_kernel, p.k_stride, p.k_windows, c);
+  add_pooled(dv, p.dv_c, bh, row0, p.k_kernel, p.k_stride, p.k_windows, c);
+  __syncwarp();
+  const int64_t at = (static_cast<int64_t>(bh) * p.Tk + row0) * 64;
+  store_rows16(dk, ring, reinterpret_cast<uint8_t*>(p.dk + at), nrows, lane);
+  store_rows16(dv, ring, reinterpret_cast<uint8_t*>(p.dv + at), nrows, lane);
 }
 
 static int grid_for(int64_t threads, int block) {
@@ -522,8 +791,8 @@ extern "C" size_t s3r_csr_workspace_bytes(int B, int H, int Nq, int topk, int Nk
   const size_t bh = static_cast<size_t>(B) * H;
   size_t cursor = (bh * Nkb * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
   size_t tmp = (bh * Nq * topk * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
-  // queue of the segments longer than a warp: at most one per 33 table entries, plus its counter
-  size_t queue = ((bh * Nq * topk / 33 + 2) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
+  // queue of the segments that one warp does not sort: at most one per non-empty segment, plus its counter
+  size_t queue = ((bh * (Nq > (1 << 25) ? static_cast<size_t>(Nkb) : static_cast<size_t>(Nq) * topk / (kCsrWarpSort + 1)) + 2) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
   return cursor + tmp + queue;
 }
 
@@ -544,15 +813,25 @@ extern "C" int s3r_build_key_csr(const int32_t* idx, int32_t* offsets, int32_t* 
                                             ((bh * Nkb * sizeof(int32_t) + 255) & ~static_cast<size_t>(255)));
   const int64_t nseg = bh * Nkb;
   S3R_REQUIRE(nseg < (1ll << 31) && total < (1ll << 40), S3R_ERR_TOO_LARGE, "s3r_build_key_csr: table too large");
+  if (per_bh <= kCsrOneEntries && Nkb <= kCsrOneKeys) {
+    const int smem = (Nkb + static_cast<int>(per_bh)) * static_cast<int>(sizeof(int32_t));
+    S3R_CUDA(cudaFuncSetAttribute(csr_one_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (kCsrOneEntries + kCsrOneKeys) * static_cast<int>(sizeof(int32_t))));
+    csr_one_kernel<<<static_cast<unsigned>(bh), 1024, smem, st>>>(idx, offsets, qids, static_cast<int>(per_bh), Nkb, topk);
+    S3R_CUDA(cudaGetLastError());
+    return 0;
+  }
   int32_t* queue = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(tmp) +
                                               ((bh * Nq * topk * sizeof(int32_t) + 255) & ~static_cast<size_t>(255)));
   S3R_CUDA(cudaMemsetAsync(offsets, 0, bh * (Nkb + 1) * sizeof(int32_t), st));
   S3R_CUDA(cudaMemsetAsync(queue, 0, sizeof(int32_t), st));
+  // a query block and its position in the segment share a 32-bit sort key
+  const int warp_max = Nq <= (1 << 25) ? kCsrWarpSort : 0;
   csr_count_kernel<<<grid_for(total, 256), 256, 0, st>>>(idx, offsets, per_bh, total, Nkb);
   csr_scan_kernel<<<static_cast<unsigned>(bh), 1024, 0, st>>>(offsets, cursor, Nkb);
   csr_fill_kernel<<<grid_for(total, 256), 256, 0, st>>>(idx, cursor, tmp, per_bh, total, Nkb, topk);
   csr_sort_small_kernel<<<static_cast<unsigned>((nseg * 32 + 255) / 256), 256, 0, st>>>(offsets, tmp, qids, per_bh, Nkb,
-                                                                                        nseg, queue);
+                                                                                        nseg, warp_max, queue);
   csr_sort_long_kernel<<<sm_count() * 4, 256, 0, st>>>(idx, offsets, tmp, qids, per_bh, Nkb, topk, queue);
   S3R_CUDA(cudaGetLastError());
   return 0;
@@ -638,18 +917,57 @@ extern "C" int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stri
   return 0;
 }
 
+static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
+  S3R_REQUIRE(p.q && p.k && p.v && p.idx && p.offsets && p.qids && p.lse && p.delta && p.d_o && p.dq && p.dk && p.dv, S3R_ERR_NULL,
+              "s3r_sel_attn_bwd: NULL pointer");
+  S3R_REQUIRE(p.B > 0 && p.H > 0 && p.Tq > 0 && p.Tk > 0 && p.topk > 0, S3R_ERR_SHAPE, "s3r_sel_attn_bwd: bad sizes");
+  S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_sel_attn_bwd: head_dim %d not supported (64 only)", d);
+  S3R_REQUIRE(p.block == 16 || p.block == 32 || p.block == 64, S3R_ERR_UNSUPPORTED,
+              "s3r_sel_attn_bwd: block %d not supported (16, 32, 64)", p.block);
+  S3R_REQUIRE(p.topk <= 64, S3R_ERR_UNSUPPORTED, "s3r_sel_attn_bwd: topk %d exceeds 64", p.topk);
+  const uintptr_t al = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v) |
+                       reinterpret_cast<uintptr_t>(p.d_o) | reinterpret_cast<uintptr_t>(p.dq) |
+                       reinterpret_cast<uintptr_t>(p.dk) | reinterpret_cast<uintptr_t>(p.dv);
+  S3R_REQUIRE((al & 15) == 0, S3R_ERR_ALIGNMENT, "s3r_sel_attn_bwd: tensors must be 16-byte aligned");
+  p.block_shift = p.block == 16 ? 0 : p.block == 32 ? 1 : 2;
+  p.nqb = (p.Tq + p.block - 1) / p.block;
+  p.nkb = (p.Tk + p.block - 1) / p.block;
+  p.status = device_status_ptr();
+  S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_sel_attn_bwd: could not resolve the device status word");
+  const int64_t bh = static_cast<int64_t>(p.B) * p.H;
+  const int64_t tq = bh * ((p.Tq + 15) / 16), tk = bh * ((p.Tk + 15) / 16);
+  S3R_REQUIRE(tq < (1ll << 31) && tk < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_bwd: grid too large");
+  CUtensorMap mkv, mqdo;
+  int rc = make_pair_map(&mkv, p.k, p.v, p.Tk, static_cast<int>(bh), 1, 0, &p.first_kv);
+  if (rc) return rc;
+  rc = make_pair_map(&mqdo, p.q, p.d_o, p.Tq, static_cast<int>(bh), 1, 0, &p.first_qdo);
+  if (rc) return rc;
+  S3R_CUDA(cudaFuncSetAttribute(sel_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
+  S3R_CUDA(cudaFuncSetAttribute(sel_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
+  sel_bwd_dkdv_kernel<<<static_cast<unsigned>(tk), 32, kSbSmem, st>>>(mqdo, p);
+  sel_bwd_dq_kernel<<<static_cast<unsigned>(tq), 32, kSbSmem, st>>>(mkv, p);
+  S3R_CUDA(cudaGetLastError());
+  return 0;
+}
+
 extern "C" int s3r_sel_attn_bwd(const void* q, const void* k, const void* v, const int32_t* idx,
                                 const int32_t* offsets, const int32_t* qids, const float* lse_s, const float* delta_s,
                                 const void* do_s, void* dq, void* dk, void* dv, int B, int H, int Tq, int Tk, int d,
                                 int block, int topk, float scale, void* stream) {
-  S3R_REQUIRE(q && k && v && idx && offsets && qids && lse_s && delta_s && do_s && dq && dk && dv, S3R_ERR_NULL,
-              "s3r_sel_attn_bwd: NULL pointer");
-  S3R_REQUIRE(B > 0 && H > 0 && Tq > 0 && Tk > 0 && topk > 0, S3R_ERR_SHAPE, "s3r_sel_attn_bwd: bad sizes");
-  S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_sel_attn_bwd: head_dim %d not supported (64 only)", d);
-  S3R_REQUIRE(block == 16 || block == 32 || block == 64, S3R_ERR_UNSUPPORTED,
-              "s3r_sel_attn_bwd: block %d not supported (16, 32, 64)", block);
-  S3R_REQUIRE(topk <= 64, S3R_ERR_UNSUPPORTED, "s3r_sel_attn_bwd: topk %d exceeds 64", topk);
-  SelBwdParams p;
+  return s3r_sel_attn_bwd_pooled(q, k, v, idx, offsets, qids, lse_s, delta_s, do_s, dq, dk, dv, nullptr, nullptr, nullptr, 16,
+                                 16, 16, 16, B, H, Tq, Tk, d, block, topk, scale, stream);
+}
+
+extern "C" int s3r_sel_attn_bwd_pooled(const void* q, const void* k, const void* v, const int32_t* idx,
+                                       const int32_t* offsets, const int32_t* qids, const float* lse_s,
+                                       const float* delta_s, const void* do_s, void* dq, void* dk, void* dv,
+                                       const void* dq_c, const void* dk_c, const void* dv_c, int q_kernel, int q_stride,
+                                       int k_kernel, int k_stride, int B, int H, int Tq, int Tk, int d, int block, int topk,
+                                       float scale, void* stream) {
+  S3R_REQUIRE(q_kernel > 0 && q_stride > 0 && k_kernel > 0 && k_stride > 0, S3R_ERR_SHAPE, "s3r_sel_attn_bwd_pooled: bad pooling sizes");
+  S3R_REQUIRE((q_kernel | q_stride | k_kernel | k_stride) % 16 == 0, S3R_ERR_UNSUPPORTED,
+              "s3r_sel_attn_bwd_pooled: pooling kernels and strides must be multiples of 16");
+  SelBwdParams p = {};
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k = static_cast<const __nv_bfloat16*>(k);
   p.v = static_cast<const __nv_bfloat16*>(v);
@@ -659,18 +977,13 @@ extern "C" int s3r_sel_attn_bwd(const void* q, const void* k, const void* v, con
   p.dq = static_cast<__nv_bfloat16*>(dq);
   p.dk = static_cast<__nv_bfloat16*>(dk);
   p.dv = static_cast<__nv_bfloat16*>(dv);
+  p.dq_c = static_cast<const __nv_bfloat16*>(dq_c);
+  p.dk_c = static_cast<const __nv_bfloat16*>(dk_c);
+  p.dv_c = static_cast<const __nv_bfloat16*>(dv_c);
+  p.q_kernel = q_kernel; p.q_stride = q_stride; p.q_windows = Tq >= q_kernel ? (Tq - q_kernel) / q_stride + 1 : 0;
+  p.k_kernel = k_kernel; p.k_stride = k_stride; p.k_windows = Tk >= k_kernel ? (Tk - k_kernel) / k_stride + 1 : 0;
   p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.block = block; p.topk = topk;
-  p.nqb = (Tq + block - 1) / block;
-  p.nkb = (Tk + block - 1) / block;
   p.cs = scale * 1.4426950408889634f;
   p.scale = scale;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t bh = static_cast<int64_t>(B) * H;
-  const int64_t tq = bh * ((Tq + 15) / 16), tk = bh * ((Tk + 15) / 16);
-  S3R_CUDA(cudaFuncSetAttribute(sel_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDkdvSmemBytes));
-  S3R_REQUIRE((tk + kDkdvWarps - 1) / kDkdvWarps < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_bwd: grid too large");
-  sel_bwd_dkdv_kernel<<<static_cast<unsigned>((tk + kDkdvWarps - 1) / kDkdvWarps), kDkdvWarps * 32, kDkdvSmemBytes, st>>>(p);
-  sel_bwd_dq_kernel<<<static_cast<unsigned>((tq + kBwdWarps - 1) / kBwdWarps), kBwdWarps * 32, 0, st>>>(p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch_sel_bwd(p, d, static_cast<cudaStream_t>(stream));
 }

@@ -420,8 +420,7 @@ struct Sel16Params {
   __nv_bfloat16* y;
   int H, Tq, Tk, Tc, nqb, topk;
   float scale_log2e;
-  int v_first;                   // the value tensor lies below the key tensor in memory
-  uint32_t pair_bytes;           // what the copies of a pair of blocks bring
+  int v_first;                   // order of the tiles a copy brings (make_pair_map)
   uint32_t* status;
 };
 
@@ -472,7 +471,7 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
         c1 = t1 / p.Tc; t1 -= c1 * p.Tc;
       }
       const uint32_t dst = ring + s * kSel16StageBytes;
-      mbar_expect_tx(&full[s], p.pair_bytes);
+      mbar_expect_tx(&full[s], p.v_first < 0 ? 4096u : 8192u);
       tma_load_5d(dst, &map_kv, &full[s], 0, t0, bh, c0, 0);
       tma_load_5d(dst + 4096, &map_kv, &full[s], 0, t1, bh, c1, 0);
     }
@@ -498,8 +497,8 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
   uint32_t off_k[4], off_v[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    off_k[i] = swz128((lane & 7) + (lane >> 4) * 8, 2 * i + ((lane >> 3) & 1)) + (p.v_first ? 2048u : 0u);
-    off_v[i] = swz128((lane & 7) + ((lane >> 3) & 1) * 8, 2 * i + (lane >> 4)) + (p.v_first || p.pair_bytes < 8192u ? 0u : 2048u);
+    off_k[i] = swz128((lane & 7) + (lane >> 4) * 8, 2 * i + ((lane >> 3) & 1)) + (p.v_first > 0 ? 2048u : 0u);
+    off_v[i] = swz128((lane & 7) + ((lane >> 3) & 1) * 8, 2 * i + (lane >> 4)) + (p.v_first == 0 ? 2048u : 0u);
   }
 
   float o[8][4];
@@ -720,20 +719,8 @@ extern "C" int s3r_sel_attn_fwd(const void* q, const void* k, const void* v, int
     p.topk = topk;
     p.scale_log2e = scale * 1.4426950408889634f;
     p.status = status;
-    // keys and values as ONE tensor whose outermost dimension of two steps from one to the other, so that one copy
-    // brings both tiles of a block
-    p.v_first = reinterpret_cast<uintptr_t>(v) < reinterpret_cast<uintptr_t>(k);
     CUtensorMap mkv;
-    const bool same = k == v;                    // one tile serves as both
-    const uint64_t dims[5] = {64, static_cast<uint64_t>(Tc), static_cast<uint64_t>(BH), static_cast<uint64_t>(kv_chunks), same ? 1u : 2u};
-    const uint64_t apart = p.v_first ? reinterpret_cast<uintptr_t>(k) - reinterpret_cast<uintptr_t>(v)
-                                     : reinterpret_cast<uintptr_t>(v) - reinterpret_cast<uintptr_t>(k);
-    const uint64_t strides[4] = {128, static_cast<uint64_t>(Tc) * 128,
-                                 kv_chunks > 1 ? static_cast<uint64_t>(kv_chunk_stride) * 2 : static_cast<uint64_t>(Tc) * 128 * BH,
-                                 same ? 128 : apart};
-    const uint32_t box[5] = {64, 16, 1, 1, same ? 1u : 2u};
-    p.pair_bytes = same ? 4096 : 8192;
-    const int rc = make_tensor_map(&mkv, p.v_first ? v : k, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    const int rc = make_pair_map(&mkv, k, v, Tk, BH, kv_chunks, kv_chunk_stride * 2, &p.v_first);
     if (rc) return rc;
     return launch_sel16_fwd(mkv, p, static_cast<int64_t>(BH) * p.nqb, st);
   }

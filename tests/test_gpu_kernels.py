@@ -57,3 +57,44 @@ def test_sel16_fwd_offset_follows_growing_scores():
     ref, lse_ref = R.sel_attn(q, k, v, idx, 16)
     assert_bf16_close(o, ref, "growing scores")
     assert ((lse.cpu() - lse_ref).abs() <= 1e-4 * lse_ref.abs() + 1e-3).all()
+
+
+# ------------------------------------------------------------------ key-centric index
+@pytest.mark.parametrize("Nq,Nkb,K", [(768, 700, 32), (769, 700, 32),           # one CTA per head | the five kernels
+                                      (100, 8192, 8), (100, 8193, 8), (3000, 40, 32)])
+@pytest.mark.parametrize("spread", ["even", "skewed", "one"])
+def test_key_csr_segment_classes(Nq, Nkb, K, spread):
+    """Segments of every length class on both sides of the one-kernel line, against a stable argsort."""
+    from speed3r_b200 import ops
+    B, H = 1, 2
+    g = torch.Generator().manual_seed(11)
+    u = torch.rand(B, H, Nq, K, generator=g)
+    idx = {"even": u * Nkb, "skewed": u ** 4 * Nkb, "one": torch.full_like(u, 3)}[spread].int()
+    idx[:, :, 1, 0], idx[:, :, 2, 1] = -1, Nkb                  # dropped entries
+    off, qids = (t.cpu() for t in ops.build_key_csr(idx.to(DEV), Nkb))
+    for h in range(H):
+        flat = idx[0, h].flatten().long()
+        keep = (flat >= 0) & (flat < Nkb)
+        key, q = flat[keep], torch.arange(Nq).repeat_interleave(K)[keep]
+        counts = torch.bincount(key, minlength=Nkb)
+        assert torch.equal(off[0, h].long(), torch.cat((torch.zeros(1, dtype=torch.long), counts.cumsum(0))))
+        order = torch.argsort(key, stable=True)
+        assert torch.equal(qids[0, h, :len(key)].long(), q[order])
+
+
+# ------------------------------------------------------------------ selection backward
+@pytest.mark.parametrize("block,K,T", [(16, 1, 16 * 5 + 3), (16, 7, 16 * 40), (32, 3, 32 * 6 + 17), (64, 2, 64 * 3 + 1), (64, 5, 64 * 9)])
+def test_sel_bwd_tiles(block, K, T):
+    """Odd numbers of tiles, blocks of several tiles, tiles that lie past the end of the sequence, unlisted blocks."""
+    from speed3r_b200 import ops
+    B, H = 1, 2
+    nb = -(-T // block)
+    q, k, v, do = bf16_round(*(randn(20 + i, B, H, T, 64) for i in range(4)))
+    idx = table(25, B, H, nb, max(1, nb - 1), K)
+    idx[:, :, 0, 0] = nb - 1
+    qg, kg, vg = (t.to(DEV, torch.bfloat16).requires_grad_(True) for t in (q, k, v))
+    ops.topk_blocksparse_attention(qg, kg, vg, idx.to(DEV), block).backward(do.to(DEV, torch.bfloat16))
+    qr, kr, vr = (t.clone().requires_grad_(True) for t in (q, k, v))
+    R.sel_attn(qr, kr, vr, idx, block)[0].backward(do)
+    for n, a, b in (("dq", qg, qr), ("dk", kg, kr), ("dv", vg, vr)):
+        assert_bf16_close(a.grad, b.grad, f"{n} block {block} K {K} T {T}")
