@@ -61,6 +61,11 @@ int s3r_device_status(uint32_t* status_host, int clear);
 int s3r_pool_fwd(const void* in, int64_t stride_b, int64_t stride_h, int64_t stride_t,
                  void* out, int B, int H, int T, int d, int kernel, int stride, void* stream);
 
+/* The same for `n` (1 to 3) tensors of one shape [B,H,T,d] in one launch, each with its own strides (3 per tensor: b, h,
+ * t), window and window stride.  The arrays are HOST arrays of device pointers and sizes. */
+int s3r_pool_multi_fwd(int n, const void* const* in, const int64_t* strides, void* const* out, const int* kernels,
+                       const int* pool_strides, int B, int H, int T, int d, void* stream);
+
 /* Backward of s3r_pool_fwd (autograd of F.avg_pool1d, same lines):
  *   d_out [B,H,Nc,d];  d_in element (b,h,t,c) at d_in + b*stride_b + h*stride_h + t*stride_t + c
  *   d_in[b,h,t,:] = sum over windows j containing t of d_out[b,h,j,:] / kernel.

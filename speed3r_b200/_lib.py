@@ -21,6 +21,7 @@ SIGNATURES = {
     "s3r_last_error": (_i, [C.c_char_p, _i]),
     "s3r_device_status": (_i, [C.POINTER(C.c_uint32), _i]),
     "s3r_pool_fwd": (_i, [_p, _i64, _i64, _i64, _p, _i, _i, _i, _i, _i, _i, _p]),
+    "s3r_pool_multi_fwd": (_i, [_i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "s3r_pool_bwd": (_i, [_p, _p, _i64, _i64, _i64, _i, _i, _i, _i, _i, _i, _i, _p]),
     "s3r_qkv_prologue_fwd": (_i, [_p, _p, _p, _p, _i, _p, _p, _p, _p, _f, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p]),
     "s3r_cmp_attn_topk_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _p]),

@@ -67,6 +67,34 @@ Tensor pool_fwd(const Tensor& x, int64_t kernel, int64_t stride) {
   return out;
 }
 
+// q pooled per block, k and v with kernel/stride, in one launch
+std::tuple<Tensor, Tensor, Tensor> pool_qkv_fwd(const Tensor& q, const Tensor& k, const Tensor& v, int64_t block,
+                                                int64_t kernel, int64_t stride) {
+  const Tensor* x[3] = {&q, &k, &v};
+  for (const Tensor* t : x) {
+    need(*t, "x", at::kBFloat16, false);
+    TORCH_CHECK(t->dim() == 4 && t->sizes() == q.sizes() && t->stride(3) == 1,
+                "pool: q, k, v must be [B,H,T,d] of one shape and their channel dimension must have unit stride");
+  }
+  const int64_t B = q.size(0), H = q.size(1), T = q.size(2), d = q.size(3);
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor out[3];
+  const void* in_p[3];
+  void* out_p[3];
+  int64_t st[9];
+  int kernels[3], strides[3];
+  for (int i = 0; i < 3; ++i) {
+    kernels[i] = static_cast<int>(i == 0 ? block : kernel);
+    strides[i] = static_cast<int>(i == 0 ? block : stride);
+    out[i] = fresh({B, H, (T - kernels[i]) / strides[i] + 1, d}, q, at::kBFloat16);
+    in_p[i] = x[i]->data_ptr();
+    out_p[i] = out[i].data_ptr();
+    for (int j = 0; j < 3; ++j) st[3 * i + j] = x[i]->stride(j);
+  }
+  check(s3r_pool_multi_fwd(3, in_p, st, out_p, kernels, strides, B, H, T, d, stream()), "s3r_pool_multi_fwd");
+  return {out[0], out[1], out[2]};
+}
+
 Tensor pool_bwd(const Tensor& d_out, int64_t T, int64_t kernel, int64_t stride) {
   need(d_out, "d_out");
   const int64_t B = d_out.size(0), H = d_out.size(1), d = d_out.size(3);
@@ -187,9 +215,12 @@ std::tuple<Tensor, Tensor> csr(const Tensor& idx, int64_t nkb, bool fill) {
 // slots behind the entries of the table that were dropped hold -1
 std::tuple<Tensor, Tensor> build_key_csr(const Tensor& idx, int64_t num_key_blocks) { return csr(idx, num_key_blocks, true); }
 
-std::tuple<Tensor, Tensor, Tensor> sel_attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
-                                                const Tensor& lse, const Tensor& delta, const Tensor& do_s, int64_t block,
-                                                double scale) {
+// The selection branch's gradients; with dq_c, dk_c, dv_c (gradients of q pooled per block and of k, v pooled with
+// kernel/stride) the pooled branch's share is added to them.
+std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                           const Tensor& lse, const Tensor& delta, const Tensor& do_s, const Tensor* dq_c,
+                                           const Tensor* dk_c, const Tensor* dv_c, int64_t block, int64_t kernel,
+                                           int64_t stride, double scale) {
   need(q, "q");
   need(k, "k");
   need(v, "v");
@@ -198,10 +229,32 @@ std::tuple<Tensor, Tensor, Tensor> sel_attn_bwd(const Tensor& q, const Tensor& k
   c10::cuda::CUDAGuard guard(q.device());
   auto [offsets, qids] = csr(idx, (Tk + block - 1) / block, false);
   Tensor dq = fresh_like(q), dk = fresh_like(k), dv = fresh_like(v);
-  check(s3r_sel_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), i32(idx), i32(offsets), i32(qids), f32(lse), f32(delta),
-                         do_s.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Tq, Tk, d, block, K, scale,
-                         stream()), "s3r_sel_attn_bwd");
+  const bool fused = dq_c != nullptr && block % 16 == 0 && kernel % 16 == 0 && stride % 16 == 0;
+  auto ptr = [&](const Tensor* t) -> const void* { return fused ? t->data_ptr() : nullptr; };
+  check(s3r_sel_attn_bwd_pooled(q.data_ptr(), k.data_ptr(), v.data_ptr(), i32(idx), i32(offsets), i32(qids), f32(lse), f32(delta),
+                                do_s.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ptr(dq_c), ptr(dk_c), ptr(dv_c),
+                                fused ? block : 16, fused ? block : 16, fused ? kernel : 16, fused ? stride : 16, B, H, Tq, Tk,
+                                d, block, K, scale, stream()), "s3r_sel_attn_bwd");
+  if (dq_c != nullptr && !fused) {
+    check(s3r_pool_bwd(dq_c->data_ptr(), dq.data_ptr(), H * Tq * d, Tq * d, d, B, H, Tq, d, block, block, 1, stream()), "s3r_pool_bwd");
+    check(s3r_pool_bwd(dk_c->data_ptr(), dk.data_ptr(), H * Tk * d, Tk * d, d, B, H, Tk, d, kernel, stride, 1, stream()), "s3r_pool_bwd");
+    check(s3r_pool_bwd(dv_c->data_ptr(), dv.data_ptr(), H * Tk * d, Tk * d, d, B, H, Tk, d, kernel, stride, 1, stream()), "s3r_pool_bwd");
+  }
   return {dq, dk, dv};
+}
+std::tuple<Tensor, Tensor, Tensor> sel_attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                                const Tensor& lse, const Tensor& delta, const Tensor& do_s, int64_t block,
+                                                double scale) {
+  return sel_bwd(q, k, v, idx, lse, delta, do_s, nullptr, nullptr, nullptr, block, 16, 16, scale);
+}
+std::tuple<Tensor, Tensor, Tensor> sel_attn_bwd_pooled(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                                       const Tensor& lse, const Tensor& delta, const Tensor& do_s,
+                                                       const Tensor& dq_c, const Tensor& dk_c, const Tensor& dv_c,
+                                                       int64_t block, int64_t kernel, int64_t stride, double scale) {
+  need(dq_c, "dq_c");
+  need(dk_c, "dk_c");
+  need(dv_c, "dv_c");
+  return sel_bwd(q, k, v, idx, lse, delta, do_s, &dq_c, &dk_c, &dv_c, block, kernel, stride, scale);
 }
 
 Tensor delta(const Tensor& o, const Tensor& d_o) {
@@ -261,6 +314,16 @@ std::tuple<Tensor, Tensor, Tensor> call_sel_bwd(const Tensor& q, const Tensor& k
                                                 const Tensor& lse, const Tensor& dlt, const Tensor& d_o, int64_t block,
                                                 double scale) {
   S3R_DISPATCHED(sel_attn_bwd)(q, k, v, idx, lse, dlt, d_o, block, scale);
+}
+std::tuple<Tensor, Tensor, Tensor> call_sel_bwd_pooled(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
+                                                       const Tensor& lse, const Tensor& dlt, const Tensor& d_o,
+                                                       const Tensor& dq_c, const Tensor& dk_c, const Tensor& dv_c,
+                                                       int64_t block, int64_t kernel, int64_t stride, double scale) {
+  S3R_DISPATCHED(sel_attn_bwd_pooled)(q, k, v, idx, lse, dlt, d_o, dq_c, dk_c, dv_c, block, kernel, stride, scale);
+}
+std::tuple<Tensor, Tensor, Tensor> call_pool_qkv(const Tensor& q, const Tensor& k, const Tensor& v, int64_t block,
+                                                 int64_t kernel, int64_t stride) {
+  S3R_DISPATCHED(pool_qkv_fwd)(q, k, v, block, kernel, stride);
 }
 Tensor call_delta(const Tensor& o, const Tensor& d_o) { S3R_DISPATCHED(delta)(o, d_o); }
 std::tuple<Tensor, Tensor, Tensor, Tensor> call_merge_bwd(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
@@ -368,13 +431,46 @@ Tensor sel_merge(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor
   return std::get<2>(call_sel(q, k, v, idx, gate, o_c, block, scale, false, false, 1));
 }
 
-// The whole op.  group = 0 where compressed keys are the selection blocks.
+// The whole op.  group = 0 where compressed keys are the selection blocks.  As one node its backward adds the
+// pooled branch's gradients inside the selection kernels' stores: separate nodes write them out as [B,H,T,d] and add
+// two bf16 tensors three times (1.5 of 19.4 ms at 250 views).
+struct SparseNode : torch::autograd::Function<SparseNode> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gate,
+                               int64_t block, int64_t topk, int64_t kernel, int64_t stride, double scale, int64_t group,
+                               int64_t take) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto [q_c, k_c, v_c] = call_pool_qkv(q, k, v, block, kernel, stride);
+    auto [o_c, lse_c, idx] = call_cmp(q_c, k_c, v_c, topk, scale, group, take);
+    auto [o_s, lse_s, y] = call_sel(q, k, v, idx, gate, o_c, block, scale, true, true, 1);
+    ctx->save_for_backward({q, k, v, gate, q_c, k_c, v_c, o_c, lse_c, idx, o_s, lse_s});
+    ctx->saved_data["block"] = block;
+    ctx->saved_data["kernel"] = kernel;
+    ctx->saved_data["stride"] = stride;
+    ctx->saved_data["scale"] = scale;
+    ctx->mark_non_differentiable({idx});
+    return {y, idx};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const int64_t block = ctx->saved_data["block"].toInt();
+    const double scale = ctx->saved_data["scale"].toDouble();
+    auto [do_s, dgate, do_c, dlt] = call_merge_bwd(g[0].contiguous(), s[3], s[7], s[10], block);
+    auto [dq_c, dk_c, dv_c] = call_cmp_bwd(s[4], s[5], s[6], s[7], s[8], do_c, scale);
+    auto [dq, dk, dv] = call_sel_bwd_pooled(s[0], s[1], s[2], s[9], s[11], dlt, do_s, dq_c, dk_c, dv_c, block,
+                                            ctx->saved_data["kernel"].toInt(), ctx->saved_data["stride"].toInt(), scale);
+    return {dq, dk, dv, dgate.to(s[3].scalar_type()), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
 std::tuple<Tensor, Tensor> sparse_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& gate,
                                             int64_t block, int64_t topk, int64_t kernel, int64_t stride, double scale,
                                             int64_t group, int64_t take) {
-  const Tensor q_c = pool_tokens(q, block, block), k_c = pool_tokens(k, kernel, stride), v_c = pool_tokens(v, kernel, stride);
-  auto [o_c, idx] = flash_attn_topk(q_c, k_c, v_c, topk, scale, group, take);
-  return {sel_merge(q, k, v, idx, gate, o_c, block, scale), idx};
+  if (wants_grad(q, k, v, gate)) {
+    const auto r = SparseNode::apply(q, k, v, gate, block, topk, kernel, stride, scale, group, take);
+    return {r[0], r[1]};
+  }
+  auto [q_c, k_c, v_c] = call_pool_qkv(q, k, v, block, kernel, stride);
+  auto [o_c, lse, idx] = call_cmp(q_c, k_c, v_c, topk, scale, group, take);
+  return {std::get<2>(call_sel(q, k, v, idx, gate, o_c, block, scale, false, false, 1)), idx};
 }
 
 }  // namespace
@@ -392,6 +488,9 @@ TORCH_LIBRARY(speed3r_b200, m) {
   m.def("build_key_csr(Tensor idx, int num_key_blocks) -> (Tensor, Tensor)");
   m.def("sel_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor idx, Tensor lse, Tensor delta, Tensor do_s, int block, "
         "float scale) -> (Tensor, Tensor, Tensor)");
+  m.def("sel_attn_bwd_pooled(Tensor q, Tensor k, Tensor v, Tensor idx, Tensor lse, Tensor delta, Tensor do_s, Tensor dq_c, "
+        "Tensor dk_c, Tensor dv_c, int block, int kernel, int stride, float scale) -> (Tensor, Tensor, Tensor)");
+  m.def("pool_qkv_fwd(Tensor q, Tensor k, Tensor v, int block, int kernel, int stride) -> (Tensor, Tensor, Tensor)");
   m.def("delta(Tensor o, Tensor d_o) -> Tensor");
   m.def("merge_bwd(Tensor dy, Tensor gate, Tensor o_c, Tensor o_s, int block) -> (Tensor, Tensor, Tensor, Tensor)");
 
@@ -414,6 +513,8 @@ TORCH_LIBRARY(speed3r_b200, m) {
   m.impl("sel_attn_fwd", &sel_attn_fwd);                    \
   m.impl("build_key_csr", &build_key_csr);                  \
   m.impl("sel_attn_bwd", &sel_attn_bwd);                    \
+  m.impl("sel_attn_bwd_pooled", &sel_attn_bwd_pooled);      \
+  m.impl("pool_qkv_fwd", &pool_qkv_fwd);                    \
   m.impl("delta", &delta);                                  \
   m.impl("merge_bwd", &merge_bwd)
 

@@ -74,6 +74,16 @@ def _register_fakes() -> None:
     def _(q, k, v, idx, lse, delta, do_s, block, scale):
         return tuple(t.new_empty(t.shape) for t in (q, k, v))
 
+    @fake("speed3r_b200::sel_attn_bwd_pooled")
+    def _(q, k, v, idx, lse, delta, do_s, dq_c, dk_c, dv_c, block, kernel, stride, scale):
+        return tuple(t.new_empty(t.shape) for t in (q, k, v))
+
+    @fake("speed3r_b200::pool_qkv_fwd")
+    def _(q, k, v, block, kernel, stride):
+        B, H, T, d = q.shape
+        nc = (T - kernel) // stride + 1
+        return tuple(q.new_empty(B, H, n, d) for n in ((T - block) // block + 1, nc, nc))
+
     @fake("speed3r_b200::delta")
     def _(o, d_o):
         return o.new_empty(o.shape[:-1], dtype=torch.float32)

@@ -98,3 +98,33 @@ def test_sel_bwd_tiles(block, K, T):
     R.sel_attn(qr, kr, vr, idx, block)[0].backward(do)
     for n, a, b in (("dq", qg, qr), ("dk", kg, kr), ("dv", vg, vr)):
         assert_bf16_close(a.grad, b.grad, f"{n} block {block} K {K} T {T}")
+
+
+# ------------------------------------------------------------------ the op as one autograd node
+@pytest.mark.parametrize("block,kernel,stride,topk", [(16, 16, 16, 8), (64, 32, 16, 4), (16, 8, 4, 8), (32, 32, 32, 4)])
+def test_op_node_gradients_match_separate_nodes(block, kernel, stride, topk):
+    """The pooled branch's gradients added inside the selection kernels (or, for windows that are not multiples of 16,
+    by the pooling kernel) against the chain of separate nodes, which rounds each share to bf16 before adding:
+    three roundings of 2^-9 relative to a share instead of one."""
+    from speed3r_b200 import ops
+    B, H, T = 2, 2, 64 * 9
+    x = [randn(30 + i, B, H, T, 64).to(DEV, torch.bfloat16) for i in range(3)]
+    gate = torch.sigmoid(randn(33, B, H, T, 2)).to(DEV, torch.bfloat16)
+    dy = randn(34, B, T, H * 64).to(DEV, torch.bfloat16)
+    leaves = lambda: [t.clone().requires_grad_(True) for t in (*x, gate)]
+    a = leaves()
+    y, idx = ops.sparse_attention_op(*a, block, topk, kernel, stride)
+    y.backward(dy)
+    b = leaves()
+    q_c, k_c, v_c = (ops.pool_tokens(b[0], block, block), ops.pool_tokens(b[1], kernel, stride), ops.pool_tokens(b[2], kernel, stride))
+    if kernel == block:
+        o_c, idx2 = ops.flash_attn_topk_func(q_c, k_c, v_c, topk)
+    else:
+        o_c, idx2 = ops.flash_attn_blocktopk_func(q_c, k_c, v_c, topk, block // stride, (block - kernel) // stride + 1)
+    y2 = ops.sel_attn_merge(b[0], b[1], b[2], idx2, b[3], o_c, block)
+    y2.backward(dy)
+    assert torch.equal(y, y2) and torch.equal(idx, idx2)
+    assert torch.equal(a[3].grad, b[3].grad)
+    for n, s, t in zip("qkv", a, b):
+        scale = t.grad.float().abs().max()
+        assert (s.grad.float() - t.grad.float()).abs().max() <= 3 * 2 ** -8 * scale, n
