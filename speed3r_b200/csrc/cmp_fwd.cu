@@ -37,6 +37,7 @@
 // Ties on the score keep the smaller column first: the heap orders (score, ~column) as one 64-bit word.
 // Slots start empty (key 0), which decodes to column Nc-1, the reference's padding.
 #include "common.cuh"
+#include "cmp_common.cuh"
 
 namespace s3r {
 
@@ -98,18 +99,6 @@ __device__ __forceinline__ int lowbit16_alu(uint32_t m) {
 __device__ __forceinline__ uint32_t small_int_of_float(float f) {
   const uint32_t b = __float_as_uint(f);
   return ((b & 0x7fffffu) | 0x800000u) >> (150u - (b >> 23));
-}
-
-// Threshold for the float pre-filter `score > thr`: a score can only enter a full list if its key
-// is strictly greater than the key in slot topk-1 (an equal key loses to the older, smaller
-// column), so rows full of equal scores stop producing hits once their list is full.  The one
-// place where float order and key order disagree is -0.0 < +0.0: a kept -0.0 yields a threshold
-// just below zero so that +0.0 still passes the pre-filter (the exact test is on the keys).
-__device__ __forceinline__ float key_to_float(uint32_t key) {
-  if (key == 0u) return -INFINITY;            // empty slot: every finite score qualifies
-  if (key == 0x7fffffffu) return __uint_as_float(0x80000001u);   // -0.0 -> largest negative subnormal
-  const uint32_t b = (key & 0x80000000u) ? (key ^ 0x80000000u) : ~key;
-  return __uint_as_float(b);
 }
 
 // A row's best entries live in a binary MIN-heap of `size` 64-bit words (key(score) << 32 | ~column) in
@@ -676,6 +665,15 @@ static int launch_cmp_fwd(const char* who, const void* q_c, const void* k_c, con
     rc = make_tensor_map(&mv, v_c, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
   }
+  if (rank_take == 0) {
+    uint32_t* status = device_status_ptr();
+    S3R_REQUIRE(status != nullptr, S3R_ERR_DRIVER, "%s: could not resolve the device status word", who);
+    const CmpMaps m = {mq, mk, mv};
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int rc = cmp_attn_fwd(m, o_c, lse, reinterpret_cast<float*>(idx), topk, BH, Nq, Nc, scale, status, st);
+    if (rc) return rc;
+    return cmp_topk_fwd(m, idx, topk, BH, Nq, Nc, status, st);
+  }
   CmpParams p;
   p.o = static_cast<__nv_bfloat16*>(o_c);
   p.lse = lse;
@@ -690,10 +688,7 @@ static int launch_cmp_fwd(const char* who, const void* q_c, const void* k_c, con
   const int64_t grid = static_cast<int64_t>(BH) * ((Nq + 255) / 256);
   S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "%s: grid too large", who);
   // per device and idempotent: setting it on every call keeps the entry points free of process-global state
-  if (rank_take == 0) {
-    S3R_CUDA(cudaFuncSetAttribute(cmp_fwd_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCmpSmemBytes));
-    cmp_fwd_kernel<0><<<static_cast<unsigned>(grid), kCmpThreads, kCmpSmemBytes, st>>>(mq, mk, mv, p);
-  } else {
+  {
     S3R_CUDA(cudaFuncSetAttribute(cmp_fwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCmpSmemBytes));
     cmp_fwd_kernel<1><<<static_cast<unsigned>(grid), kCmpThreads, kCmpSmemBytes, st>>>(mq, mk, mv, p);
   }

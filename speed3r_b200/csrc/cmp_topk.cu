@@ -1,0 +1,380 @@
+// Compression branch, forward, second of two kernels: the `topk` columns of every pooled query's largest RAW logits,
+// ordered by (logit descending, column ascending).
+//
+// The first kernel (cmp_attn.cu) leaves a lower bound of each row's 32nd largest logit, so this one repeats Q K^T on
+// the tensor cores and only collects the logits that reach the bound - about 44 per row with independent scores - into
+// lists of (logit, column) pairs in shared memory, [slot][lane] so that a thread's accesses never meet another's on a
+// bank.  A row has two threads (in two warpgroups that take turns at its key tiles) and a list for each.  A list that
+// fills up (structured scores can leave a loose bound; equal scores all reach it) is cut back to its best 32 there and
+// then, and goes on with the 32nd of those as its bound.  At the end every thread sorts its list in registers, and one of
+// the two merges them.
+//
+// Bound: instructions and their latency in the scan: a max tree and a vote per 16 columns of a warp, and for the chunks
+// with a hit (three in four at 250 views, one in three at 1000) a mask and a store.  The products take half of the time
+// that the tensor pipe alone would need.  S of a tile is two buffers of 64 columns, each taken into registers in one go, so
+// that the next products run while a half is scanned (16 columns at a time, S held for a whole tile: 1.05 instead of
+// 0.95 ms for 15750 x 15750, 16 heads).
+// Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-19 scan: two row tiles of
+// 128 queries, two warpgroups each.  Tensor memory: 2 row tiles x 2 tiles x 128 columns.
+#include "common.cuh"
+#include "cmp_common.cuh"
+
+namespace s3r {
+
+constexpr int kTkTile = 128 * 128;             // 128 rows x 64 bf16, bytes
+constexpr int kTkCap = 40;                     // pairs a list holds before it is cut back to 32
+constexpr int kTkRows = 256;                   // query rows per CTA
+constexpr int kTkStages = 2;
+constexpr int kTkOffK = 2 * kTkTile;
+constexpr int kTkOffBuf = kTkOffK + kTkStages * kTkTile;
+constexpr int kTkSmem = kTkOffBuf + 2 * kTkRows * kTkCap * 8 + 1024;
+constexpr int kTkThreads = 128 + 512;
+constexpr int kTkSplitTiles = 16;              // with fewer tiles the two scans of a row take halves of every tile, not turns
+
+struct TkCtl {
+  uint64_t q_full, drained;
+  uint64_t k_full[kTkStages], k_empty[kTkStages];
+  uint64_t s_full[2][2][2], s_empty[2][2][2];  // [row tile][tile parity][half of the tile]
+  uint32_t tmem_base;
+  uint32_t abort_flag;
+};
+
+struct TkParams {
+  int32_t* idx;
+  int Nq, Nc, topk;
+  int vec;                     // rows of idx can be written 16 bytes at a time
+  uint32_t* status;
+};
+
+__device__ __forceinline__ uint64_t tk_entry(uint2 raw) {          // larger = better: (key of the logit, ~column)
+  return (static_cast<uint64_t>(sortable_key(__uint_as_float(raw.x))) << 32) | static_cast<uint32_t>(~raw.y);
+}
+
+// Cuts this thread's list of `cnt` > 32 pairs back to its best 32 (in place, column order lost) and returns the bound
+// to go on with.  A binary min-heap over slots 0..31 whose root is replaced by every better pair of the rest.
+__device__ __noinline__ float tk_cut(uint2* buf, int cnt) {
+  auto ld = [&](int i) { return tk_entry(buf[i * 32]); };
+  auto sift = [&](int i, uint2 raw) {
+    const uint64_t v = tk_entry(raw);
+    while (true) {
+      int c = 2 * i + 1;
+      if (c >= 32) break;
+      uint64_t e = ld(c);
+      if (c + 1 < 32) {
+        const uint64_t e2 = ld(c + 1);
+        if (e2 < e) { e = e2; ++c; }
+      }
+      if (e >= v) break;
+      buf[i * 32] = buf[c * 32];
+      i = c;
+    }
+    buf[i * 32] = raw;
+  };
+  for (int i = 15; i >= 0; --i) sift(i, buf[i * 32]);
+  for (int i = 32; i < cnt; ++i) {
+    const uint2 raw = buf[i * 32];
+    if (tk_entry(raw) > ld(0)) sift(0, raw);
+  }
+  return key_to_float(sortable_key(__uint_as_float(buf[0].x)));
+}
+
+// The hits of a chunk one by one, for rows whose list may fill up: rare, and out of line so that the registers of the
+// scan are not laid out around the cuts.
+struct TkChunk {
+  uint32_t x[16];
+};
+__device__ __noinline__ void tk_append_checked(const TkChunk ch, uint2* buf, uint32_t col0, int& cnt, float& thr) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < 16; ++i) {
+    if (!(__uint_as_float(ch.x[i]) > thr)) continue;
+    if (cnt == kTkCap) {
+      thr = tk_cut(buf, cnt);
+      cnt = 32;
+      if (!(__uint_as_float(ch.x[i]) > thr)) continue;
+    }
+    buf[cnt * 32] = make_uint2(ch.x[i], col0 + i);
+    ++cnt;
+  }
+}
+
+// Descending bitonic sort in registers.
+__device__ __forceinline__ void tk_cmp(uint64_t& a, uint64_t& b, bool desc) {
+  const bool swap = desc ? a < b : b < a;
+  const uint64_t x = swap ? b : a, y = swap ? a : b;
+  a = x;
+  b = y;
+}
+template <int N>
+__device__ __forceinline__ void tk_sort(uint64_t (&v)[N]) {
+#pragma unroll
+  for (int k = 2; k <= N; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if ((i ^ j) > i) tk_cmp(v[i], v[i ^ j], (i & k) == 0);
+}
+// A bitonic sequence (what a[i] = max(a[i], b[31 - i]) of two descending lists leaves: the best 32 of both), sorted.
+__device__ __forceinline__ void tk_merge(uint64_t (&v)[32]) {
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1)
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if ((i ^ j) > i) tk_cmp(v[i], v[i ^ j], true);
+}
+
+__global__ void __launch_bounds__(kTkThreads, 1)
+cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const TkParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ TkCtl ctl;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_per_bh = (p.Nq + kTkRows - 1) / kTkRows;
+  const int bh = blockIdx.x / tiles_per_bh;
+  const int q0 = (blockIdx.x % tiles_per_bh) * kTkRows;
+  const int ntiles = (p.Nc + 127) / 128;
+  const bool split = ntiles < kTkSplitTiles;
+  const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+
+  if (threadIdx.x == 0) {
+    ctl.abort_flag = 0;
+    mbar_init(&ctl.q_full, 1);
+    mbar_init(&ctl.drained, 1);
+    for (int s = 0; s < kTkStages; ++s) {
+      mbar_init(&ctl.k_full[s], 1);
+      mbar_init(&ctl.k_empty[s], 1);
+    }
+    for (int i = 0; i < 8; ++i) {
+      mbar_init(&ctl.s_full[0][0][0] + i, 1);
+      mbar_init(&ctl.s_empty[0][0][0] + i, 4);
+    }
+    mbar_fence_init();
+  }
+  if (warp == 2) {
+    tmem_alloc(&ctl.tmem_base, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = ctl.tmem_base;
+  volatile uint32_t* abort_flag = &ctl.abort_flag;
+
+  // registers: the launch gives every thread 96, the utility warps hand most of theirs to the scan
+  // (640 x 96 = 61440 >= 512 x 104 + 128 x 40)
+  if (warp < 4) {
+    reg_dealloc<40>();
+    if (warp == 0) {
+      if (lane == 0) {
+        mbar_expect_tx(&ctl.q_full, 2 * kTkTile);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) tma_load_3d(sbase + t * kTkTile, &map_q, &ctl.q_full, 0, q0 + t * 128, bh);
+        int issued = 0;
+        for (int j = 0; j < ntiles; ++j) {
+          const int s = j % kTkStages;
+          if (!mbar_wait(&ctl.k_empty[s], ((j / kTkStages) & 1) ^ 1, abort_flag)) break;
+          mbar_expect_tx(&ctl.k_full[s], kTkTile);
+          tma_load_3d(sbase + kTkOffK + s * kTkTile, &map_k, &ctl.k_full[s], 0, j * 128, bh);
+          issued = j + 1;
+        }
+        if (*abort_flag) {
+          // give copies already in flight a bounded chance to land before the CTA's memory is released
+          for (int j = max(0, issued - kTkStages); j < issued; ++j) {
+            volatile uint32_t dummy = 0;
+            mbar_wait(&ctl.k_full[j % kTkStages], (j / kTkStages) & 1, &dummy);
+          }
+        }
+      }
+    } else if (warp == 1) {
+      const bool leader = elect_one_sync();
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 64, 0, 0);
+      const uint64_t desc_q = umma_desc_sw128(sbase), desc_k = umma_desc_sw128(sbase + kTkOffK);
+      bool ok = mbar_wait_warp(&ctl.q_full, 0, abort_flag);
+      int s = 0;
+      uint32_t ph = 0;
+#pragma unroll 1
+      for (int j = 0; j < ntiles && ok; ++j) {
+        const int b = j & 1;
+        ok = mbar_wait_warp(&ctl.k_full[s], ph, abort_flag);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = i & 1, h = i >> 1;
+          if (ok) ok = mbar_wait_warp(&ctl.s_empty[t][b][h], ((j >> 1) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (leader) {
+            umma_ss_k4<2, 2>(tmem + t * 256 + b * 128 + h * 64, desc_q + static_cast<uint64_t>(t * (kTkTile >> 4)),
+                             desc_k + static_cast<uint64_t>(s * (kTkTile >> 4) + h * (kTkTile >> 5)), idesc, 0u);
+            umma_commit(&ctl.s_full[t][b][h]);
+            if (i == 3) umma_commit(&ctl.k_empty[s]);
+          }
+          __syncwarp();
+        }
+        if (++s == kTkStages) { s = 0; ph ^= 1u; }
+      }
+      if (!ok) {
+        if (leader) umma_commit(&ctl.drained);
+        __syncwarp();
+        volatile uint32_t dummy = 0;
+        mbar_wait(&ctl.drained, 0, &dummy);      // let issued MMAs drain before tensor memory is freed
+      }
+    }
+  } else {
+    reg_alloc<104>();
+    const int t = (warp - 4) >> 3, par = ((warp - 4) >> 2) & 1, quarter = warp & 3;
+    const int row = q0 + t * 128 + quarter * 32 + lane;
+    const uint32_t t_s = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + t * 256;
+    uint2* lists = reinterpret_cast<uint2*>(smem_raw + (sbase - smem_u32(smem_raw)) + kTkOffBuf);
+    uint2* buf = lists + (warp - 4) * (kTkCap * 32) + lane;
+    int32_t* out = p.idx + (static_cast<int64_t>(bh) * p.Nq + row) * p.topk;
+    // `score > thr` for every score that reaches the bound (NaN and -inf never do); rows past the end collect nothing
+    float thr = INFINITY;
+    if (row < p.Nq) {
+      const float bound = fmaxf(__int_as_float(*out), -3.402823466e38f);
+      thr = bound == 0.f ? __uint_as_float(0x80000001u) : key_to_float(sortable_key(bound) - 1u);
+    }
+    const uint32_t first = smem_u32(buf), end = first + kTkCap * 256;
+    uint32_t at = first;                         // where the list's next pair goes
+    bool ok = true;
+
+    // 16 columns: a max tree and a vote pass over chunks in which no row of the warp has a hit
+    auto scan = [&](const uint32_t* x, int col0) {
+      auto f = [&](int i) { return __uint_as_float(x[i]); };
+      const float m = fmaxf(fmax3(fmax3(f(0), f(1), f(2)), fmax3(f(3), f(4), f(5)), fmax3(f(6), f(7), f(8))),
+                            fmax3(fmax3(f(9), f(10), f(11)), fmax3(f(12), f(13), f(14)), f(15)));
+      if (!__any_sync(0xffffffffu, m > thr)) return;
+      // bit 15 - i of the mask = sign of thr - x[i]; two chains of shifts
+      uint32_t m0 = 0, m1 = 0;
+      const float2 minus = make_float2(-1.f, -1.f), thr2 = make_float2(thr, thr);
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        const float2 d0 = ffma2(make_float2(f(i), f(i + 1)), minus, thr2), d1 = ffma2(make_float2(f(8 + i), f(9 + i)), minus, thr2);
+        m0 = __funnelshift_l(__float_as_uint(d0.y), __funnelshift_l(__float_as_uint(d0.x), m0, 1), 1);
+        m1 = __funnelshift_l(__float_as_uint(d1.y), __funnelshift_l(__float_as_uint(d1.x), m1, 1), 1);
+      }
+      const uint32_t mask = (m0 << 8) | m1;
+      // one hit per row at most, and room for it: it is the chunk's maximum
+      if (!__any_sync(0xffffffffu, (mask & (mask - 1)) != 0u || at == end)) {
+        if (mask) {
+          sts64(at, __float_as_uint(m), static_cast<uint32_t>(col0 - 16 + __clz(mask)));
+          at += 256;
+        }
+      } else if (!__any_sync(0xffffffffu, at + 256 * __popc(mask) > end)) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (mask & (0x8000u >> i)) {
+            sts64(at, x[i], static_cast<uint32_t>(col0 + i));
+            at += 256;
+          }
+        }
+      } else {
+        TkChunk ch;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) ch.x[i] = x[i];
+        int cnt = static_cast<int>(at - first) >> 8;
+        tk_append_checked(ch, buf, static_cast<uint32_t>(col0), cnt, thr);
+        at = first + cnt * 256;
+        __syncwarp();
+      }
+    };
+    // half h of tile j
+    auto half_tile = [&](int j, int h) -> bool {
+      const int b = j & 1;
+      if (!mbar_wait_warp(&ctl.s_full[t][b][h], (j >> 1) & 1, abort_flag)) return false;
+      tc_fence_after();
+      const uint32_t src = t_s + b * 128 + h * 64;
+      const int col0 = j * 128 + h * 64, left = p.Nc - col0;
+      auto release = [&]() {                     // all of this half of S is in registers: the next Q K^T may overwrite it
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.s_empty[t][b][h]);
+      };
+      uint32_t xa[32], xb[32];
+      tmem_ld32(src, xa);
+      tmem_ld32(src + 32, xb);
+      tmem_ld_wait();
+      release();
+      if (left < 64) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          if (i >= left) xa[i] = 0xff800000u;   // -inf
+          if (32 + i >= left) xb[i] = 0xff800000u;
+        }
+      }
+      scan(xa, col0);
+      scan(xa + 16, col0 + 16);
+      scan(xb, col0 + 32);
+      scan(xb + 16, col0 + 48);
+      return true;
+    };
+    if (split) {
+#pragma unroll 1
+      for (int j = 0; j < ntiles && ok; ++j) ok = half_tile(j, par);
+    } else {
+#pragma unroll 1
+      for (int u = 2 * par; u < 2 * ntiles && ok; u = (u & 1) ? u + 3 : u + 1) ok = half_tile(u >> 1, u & 1);
+    }
+
+    const int cnt = static_cast<int>(at - first) >> 8;
+    // each list sorted by its own thread, then the two lists of a row merged by one of them
+    uint64_t a[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) a[i] = i < cnt ? tk_entry(buf[i * 32]) : 0ull;
+    tk_sort<32>(a);
+    if (__any_sync(0xffffffffu, cnt > 32)) {
+      uint64_t e[kTkCap - 32];
+#pragma unroll
+      for (int i = 0; i < kTkCap - 32; ++i) e[i] = 32 + i < cnt ? tk_entry(buf[(32 + i) * 32]) : 0ull;
+      tk_sort<kTkCap - 32>(e);
+#pragma unroll
+      for (int i = 0; i < kTkCap - 32; ++i) a[31 - i] = a[31 - i] < e[i] ? e[i] : a[31 - i];
+      tk_merge(a);
+    }
+    if (par == 1) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) buf[i * 32] = make_uint2(static_cast<uint32_t>(a[i] >> 32), static_cast<uint32_t>(a[i]));
+    }
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory");      // every scan warp of the row tile comes here, whatever happened
+    if (ok && par == 0 && row < p.Nq) {
+      const uint2* other = buf + 4 * (kTkCap * 32);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const uint2 w = other[(31 - i) * 32];
+        const uint64_t e = (static_cast<uint64_t>(w.x) << 32) | w.y;
+        a[i] = a[i] < e ? e : a[i];
+      }
+      tk_merge(a);
+      // an empty slot decodes to column Nc-1, the reference's padding
+      auto column = [&](int i) { return a[i] >> 32 ? static_cast<int32_t>(~static_cast<uint32_t>(a[i])) : p.Nc - 1; };
+      if (p.vec) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+          if (i < p.topk) *reinterpret_cast<int4*>(out + i) = make_int4(column(i), column(i + 1), column(i + 2), column(i + 3));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i < p.topk) out[i] = column(i);
+      }
+    }
+    if (!ok && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2) tmem_dealloc(tmem, 512);
+}
+
+int cmp_topk_fwd(const CmpMaps& m, int32_t* idx, int topk, int BH, int Nq, int Nc, uint32_t* status, cudaStream_t st) {
+  TkParams p;
+  p.idx = idx;
+  p.Nq = Nq; p.Nc = Nc; p.topk = topk;
+  p.vec = (topk & 3) == 0 && (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
+  p.status = status;
+  const int64_t grid = static_cast<int64_t>(BH) * ((Nq + kTkRows - 1) / kTkRows);
+  S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
+  S3R_CUDA(cudaFuncSetAttribute(cmp_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
+  cmp_topk_kernel<<<static_cast<unsigned>(grid), kTkThreads, kTkSmem, st>>>(m.q, m.k, p);
+  S3R_CUDA(cudaGetLastError());
+  return 0;
+}
+
+}  // namespace s3r

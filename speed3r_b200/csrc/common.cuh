@@ -94,6 +94,26 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
   return d;
 }
 
+// 2^x of a pair on the FMA pipe, for kernels whose exponentials saturate their own unit (16 results per cycle and SM):
+// x = n + f with n the nearest integer (the 1.5 * 2^23 shift), 2^f by a polynomial of degree 5 on [-1/2, 1/2], n added
+// to the exponent field.  The coefficients are a least-squares fit of the relative error, reweighted until it levelled
+// out: 7.5e-8, 2.3e-7 with fp32 rounding (ex2.approx: 2.4e-7).  x < 127; below -126 the result is 2^-126.
+__device__ __forceinline__ float2 exp2_fma2(float2 x) {
+  x.x = fmaxf(x.x, -126.f);
+  x.y = fmaxf(x.y, -126.f);
+  const float2 shift = make_float2(12582912.f, 12582912.f), unshift = make_float2(-12582912.f, -12582912.f);
+  const float2 t = fadd2(x, shift), n = fadd2(t, unshift), f = fadd2(x, make_float2(-n.x, -n.y));
+  float2 r = make_float2(1.327647012e-3f, 1.327647012e-3f);
+  r = ffma2(r, f, make_float2(9.675541319e-3f, 9.675541319e-3f));
+  r = ffma2(r, f, make_float2(5.550713279e-2f, 5.550713279e-2f));
+  r = ffma2(r, f, make_float2(2.402211972e-1f, 2.402211972e-1f));
+  r = ffma2(r, f, make_float2(6.931469671e-1f, 6.931469671e-1f));
+  r = ffma2(r, f, make_float2(1.f, 1.f));
+  r.x = __uint_as_float((__float_as_uint(t.x) << 23) + __float_as_uint(r.x));
+  r.y = __uint_as_float((__float_as_uint(t.y) << 23) + __float_as_uint(r.y));
+  return r;
+}
+
 // max of three in one instruction (three-operand max of sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
@@ -265,6 +285,9 @@ __device__ __forceinline__ void mma_bf16_z(float (&d)[4], const uint32_t (&a)[4]
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");

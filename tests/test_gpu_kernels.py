@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from _util import assert_bf16_close, bf16_round
+from _util import assert_bf16_close, assert_idx_match, bf16_round
 from oracle import restatement as R
 
 pytestmark = pytest.mark.gpu
@@ -128,3 +128,65 @@ def test_op_node_gradients_match_separate_nodes(block, kernel, stride, topk):
     for n, s, t in zip("qkv", a, b):
         scale = t.grad.float().abs().max()
         assert (s.grad.float() - t.grad.float()).abs().max() <= 3 * 2 ** -8 * scale, n
+
+
+# ------------------------------------------------------------------ compression attention and its table
+@pytest.mark.parametrize("jump", [1.0, 40.0])
+def test_cmp_offset_of_the_first_tile(jump):
+    """Rows whose later scores outgrow those of the first 128 keys: within the range of a float (one pass) and far
+    beyond it (the CTA's second pass), next to rows that need neither."""
+    from speed3r_b200 import ops
+    B, H, Nq, Nc = 1, 2, 300, 700
+    q, k, v = randn(40, B, H, Nq, 64), randn(41, B, H, Nc, 64), randn(42, B, H, Nc, 64)
+    k[:, :, 500:] *= jump
+    q[:, :, ::3] *= 0.01
+    q, k, v = bf16_round(q, k, v)
+    o, lse, idx = ops._cmp_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), 32, 0.125)
+    ref, lse_ref, idx_ref = R.cmp_attn_topk(q, k, v, 32)
+    S = q @ k.transpose(-1, -2)
+    # fp32 sums of 64 products of that size in another order
+    assert_idx_match(idx, idx_ref, S, f"jump {jump}", eps=max(1e-3, 64 * 2 ** -24 * S.abs().max().item()))
+    assert_bf16_close(o, ref, f"o_c jump {jump}")
+    assert ((lse.cpu() - lse_ref).abs() <= 1e-5 * lse_ref.abs() + 1e-3).all()
+
+
+@pytest.mark.parametrize("Nc", [1, 31, 32, 40, 65, 127, 128, 129, 15 * 128, 15 * 128 + 1, 16 * 128 + 77])
+@pytest.mark.parametrize("topk", [1, 7, 32])
+def test_cmp_table_sizes(Nc, topk):
+    """Fewer keys than table entries, one tile and its neighbours, and both ways of sharing tiles between the two scans."""
+    from speed3r_b200 import ops
+    B, H, Nq = 1, 2, 257
+    q, k, v = bf16_round(randn(50, B, H, Nq, 64), randn(51, B, H, Nc, 64), randn(52, B, H, Nc, 64))
+    o, lse, idx = ops._cmp_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), topk, 0.125)
+    ref, _, idx_ref = R.cmp_attn_topk(q, k, v, topk)
+    assert_idx_match(idx, idx_ref, q @ k.transpose(-1, -2), f"Nc {Nc} topk {topk}")
+    assert_bf16_close(o, ref, f"o_c Nc {Nc}")
+
+
+@pytest.mark.parametrize("heads", [40, 80])
+def test_cmp_one_and_two_row_tiles(heads):
+    """Both sides of the line between one and two row tiles per CTA, with rows past the end in the second."""
+    from speed3r_b200 import ops
+    q, k, v = bf16_round(randn(55, 1, heads, 270, 64), randn(56, 1, heads, 200, 64), randn(57, 1, heads, 200, 64))
+    o, lse, idx = ops._cmp_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), 32, 0.125)
+    ref, _, idx_ref = R.cmp_attn_topk(q, k, v, 32)
+    assert_idx_match(idx, idx_ref, q @ k.transpose(-1, -2), f"{heads} heads")
+    assert_bf16_close(o, ref, f"o_c {heads} heads")
+
+
+@pytest.mark.parametrize("period", [1, 16, 64])
+def test_cmp_table_when_the_bound_is_loose(period):
+    """Keys that repeat with a period: the best logits fall into few of the 64 column groups, so that far more logits than
+    a list holds reach the bound and lists are cut; exact repeats are ties, which the smaller column wins."""
+    from speed3r_b200 import ops
+    B, H, Nq, Nc = 1, 2, 130, 3000
+    q, v = bf16_round(randn(60, B, H, Nq, 64), randn(61, B, H, Nc, 64))
+    base, = bf16_round(randn(62, B, H, period, 64))
+    k = base.repeat(1, 1, -(-Nc // period), 1)[:, :, :Nc].contiguous()
+    o, lse, idx = ops._cmp_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), 32, 0.125)
+    ref, _, idx_ref = R.cmp_attn_topk(q, k, v, 32)
+    assert_idx_match(idx, idx_ref, q @ k.transpose(-1, -2), f"period {period}")
+    # equal logits on the device: whole runs of a repeated key, in column order
+    first = idx[..., 0:1].cpu().long()
+    assert torch.equal(idx.cpu().long(), first + period * torch.arange(32))
+    assert_bf16_close(o, ref, "o_c")
