@@ -89,11 +89,23 @@ int s3r_pool_bwd(const void* d_out, void* d_in, int64_t stride_b, int64_t stride
  *   q_weight..k_bias: fp32 [d] LayerNorm affine parameters, or all NULL (Identity norms)
  *   q,k,v          : [B,H,N,d] bf16 out;  q_c,k_c,v_c : [B,H,N/block,d] bf16 out
  * N must be a multiple of `block`; d = 64; at most 42 heads.  Forward only: a caller that
- * needs gradients runs the separate steps (s3r_pool_fwd/bwd and its own LayerNorm and rotary code). */
+ * needs gradients calls s3r_qkv_prologue_bwd. */
 int s3r_qkv_prologue_fwd(const void* qkv, const int64_t* pos, const void* cos_tab, const void* sin_tab,
                          int tab_rows, const float* q_weight, const float* q_bias, const float* k_weight,
                          const float* k_bias, float eps, void* q, void* k, void* v, void* q_c, void* k_c,
                          void* v_c, int B, int H, int N, int d, int block, void* stream);
+
+/* Backward of s3r_qkv_prologue_fwd (autograd of the same lines): from the gradients of its six outputs the gradient of the
+ * packed projection and of the LayerNorm parameters.
+ *   dq,dk,dv [B,H,N,d], dq_c,dk_c,dv_c [B,H,N/block,d] bf16;  dqkv [B,N,3,H,d] bf16, overwritten
+ *   q_weight, k_weight as in the forward; dparams [4,64] fp32 = dq_weight, dq_bias, dk_weight, dk_bias (NULL without norms)
+ *   workspace: s3r_qkv_prologue_bwd_workspace_bytes(...) bytes (unused without norms); need not be initialised.
+ * Positions outside the tables are clamped as in the forward, which has reported them.  Deterministic. */
+size_t s3r_qkv_prologue_bwd_workspace_bytes(int B, int N, int block);
+int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const void* cos_tab, const void* sin_tab, int tab_rows,
+                         const float* q_weight, const float* k_weight, float eps, const void* dq, const void* dk,
+                         const void* dv, const void* dq_c, const void* dk_c, const void* dv_c, void* dqkv, float* dparams,
+                         void* workspace, size_t workspace_bytes, int B, int H, int N, int d, int block, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Compression attention with fused top-k block selection.
@@ -253,6 +265,11 @@ int s3r_sel_attn_bwd_pooled(const void* q, const void* k, const void* v, const i
  * SMs so that it can run beside a kernel that fills all the others.
  * ------------------------------------------------------------------------------------------ */
 int s3r_peer_pull(const void* const* src, void* const* dst, const int64_t* bytes, int nseg, int ctas, void* stream);
+
+/* fp32 -> bf16 (round to nearest even) of `n` (1 to 8) tensors in one launch; no counterpart in the reference, whose autocast
+ * casts the module's input and weights one by one.  The arrays are HOST arrays of device pointers and element counts;
+ * every tensor 16-byte aligned. */
+int s3r_cast_bf16(int n, const float* const* src, void* const* dst, const int64_t* counts, void* stream);
 
 /* Strided copy between host and device (rows of `width_bytes` at the two pitches) on `stream`:
  * cudaMemcpy2DAsync with the direction inferred from the pointers.  No counterpart in the reference;

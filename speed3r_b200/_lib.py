@@ -24,6 +24,8 @@ SIGNATURES = {
     "s3r_pool_multi_fwd": (_i, [_i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "s3r_pool_bwd": (_i, [_p, _p, _i64, _i64, _i64, _i, _i, _i, _i, _i, _i, _i, _p]),
     "s3r_qkv_prologue_fwd": (_i, [_p, _p, _p, _p, _i, _p, _p, _p, _p, _f, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p]),
+    "s3r_qkv_prologue_bwd_workspace_bytes": (_sz, [_i, _i, _i]),
+    "s3r_qkv_prologue_bwd": (_i, [_p, _p, _p, _p, _i, _p, _p, _f] + [_p] * 9 + [_sz, _i, _i, _i, _i, _i, _p]),
     "s3r_cmp_attn_topk_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_cmp_attn_blocktopk_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p]),
     "s3r_cmp_attn_bwd": (_i, [_p] * 10 + [_i, _i, _i, _i, _i, _f, _p]),
@@ -36,6 +38,7 @@ SIGNATURES = {
     "s3r_delta": (_i, [_p, _p, _p, _i64, _i, _p]),
     "s3r_sel_attn_bwd": (_i, [_p] * 12 + [_i, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_sel_attn_bwd_pooled": (_i, [_p] * 15 + [_i] * 11 + [_f, _p]),
+    "s3r_cast_bf16": (_i, [_i, _p, _p, _p, _p]),
     "s3r_copy2d_async": (_i, [_p, _sz, _p, _sz, _sz, _sz, _p]),
     "s3r_peer_pull": (_i, [_p, _p, _p, _i, _i, _p]),
     "s3r_ipc_export": (_i, [_p, _p, C.POINTER(C.c_int64)]),

@@ -280,6 +280,90 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> merge_bwd(const Tensor& dy, const Ten
   return {do_s, dgate, do_c, delta_s};
 }
 
+const void* ptr_or_null(const optional<Tensor>& t) { return t.has_value() ? t->data_ptr() : nullptr; }
+const float* f32_or_null(const optional<Tensor>& t) { return t.has_value() ? f32(*t) : nullptr; }
+
+// What the prologue's arguments have to be; returns the rows of the rotary tables (0: no rotary embedding)
+int64_t need_prologue(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos, const optional<Tensor>& cos,
+                      const optional<Tensor>& sin, std::initializer_list<const optional<Tensor>*> norms) {
+  need(qkv, "qkv");
+  TORCH_CHECK(qkv.dim() >= 3 && heads > 0 && block > 0, "qkv_prologue: qkv must be [B,N,3*H*d]");
+  const int64_t B = qkv.size(0), N = qkv.size(1), C3 = B * N > 0 ? qkv.numel() / (B * N) : 0, d = C3 / (3 * heads);
+  TORCH_CHECK(C3 == 3 * heads * d && N % block == 0, "qkv_prologue: qkv ", qkv.sizes(), " does not split into 3 x ", heads,
+              " heads, or N=", N, " is not a multiple of the block ", block);
+  for (const auto* w : norms) {
+    TORCH_CHECK(w->has_value() == (*norms.begin())->has_value(), "qkv_prologue: q_norm and k_norm come together or not at all");
+    if (w->has_value()) need(**w, "norm parameter", at::kFloat);
+  }
+  if (!pos.has_value()) return 0;
+  TORCH_CHECK(cos.has_value() && sin.has_value(), "qkv_prologue: positions need the cos/sin tables");
+  need(*cos, "cos");
+  need(*sin, "sin");
+  TORCH_CHECK(cos->sizes() == sin->sizes() && cos->dim() == 2 && cos->size(1) == d / 2, "qkv_prologue: cos/sin tables must be [rows,",
+              d / 2, "]");
+  TORCH_CHECK(pos->sizes() == std::vector<int64_t>({B, N, 2}) && pos->device() == qkv.device(),
+              "qkv_prologue: pos must be [B,N,2] = [", B, ", ", N, ", 2] on ", qkv.device());
+  need(*pos, "pos", at::kLong);
+  return cos->size(0);
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> prologue_fwd(
+    const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos, const optional<Tensor>& cos,
+    const optional<Tensor>& sin, const optional<Tensor>& qw, const optional<Tensor>& qb, const optional<Tensor>& kw,
+    const optional<Tensor>& kb, double eps) {
+  const int64_t rows = need_prologue(qkv, heads, block, pos, cos, sin, {&qw, &qb, &kw, &kb});
+  const int64_t B = qkv.size(0), N = qkv.size(1), d = qkv.numel() / (B * N) / (3 * heads);
+  c10::cuda::CUDAGuard guard(qkv.device());
+  Tensor t[6];
+  for (int i = 0; i < 6; ++i) t[i] = fresh({B, heads, i < 3 ? N : N / block, d}, qkv, at::kBFloat16);
+  const bool rope = pos.has_value();
+  check(s3r_qkv_prologue_fwd(qkv.data_ptr(), static_cast<const int64_t*>(ptr_or_null(pos)), rope ? ptr_or_null(cos) : nullptr,
+                             rope ? ptr_or_null(sin) : nullptr, rows, f32_or_null(qw), f32_or_null(qb), f32_or_null(kw),
+                             f32_or_null(kb), eps, t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(),
+                             t[4].data_ptr(), t[5].data_ptr(), B, heads, N, d, block, stream()), "s3r_qkv_prologue_fwd");
+  return {t[0], t[1], t[2], t[3], t[4], t[5]};
+}
+
+// (gradient of qkv, [4,64] gradients of q weight, q bias, k weight, k bias; no elements without norms)
+std::tuple<Tensor, Tensor> prologue_bwd(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos,
+                                        const optional<Tensor>& cos, const optional<Tensor>& sin, const optional<Tensor>& qw,
+                                        const optional<Tensor>& kw, double eps, const Tensor& dq, const Tensor& dk,
+                                        const Tensor& dv, const Tensor& dq_c, const Tensor& dk_c, const Tensor& dv_c) {
+  const int64_t rows = need_prologue(qkv, heads, block, pos, cos, sin, {&qw, &kw});
+  for (const Tensor* g : {&dq, &dk, &dv, &dq_c, &dk_c, &dv_c}) need(*g, "gradient");
+  const int64_t B = qkv.size(0), N = qkv.size(1), d = qkv.numel() / (B * N) / (3 * heads);
+  c10::cuda::CUDAGuard guard(qkv.device());
+  const bool norm = qw.has_value(), rope = pos.has_value();
+  const size_t nbytes = norm ? s3r_qkv_prologue_bwd_workspace_bytes(B, N, block) : 0;
+  Tensor dqkv = fresh_like(qkv), ws = fresh({static_cast<int64_t>(nbytes)}, qkv, at::kByte),
+         dparams = fresh(norm ? std::vector<int64_t>{4, d} : std::vector<int64_t>{0}, qkv, at::kFloat);
+  check(s3r_qkv_prologue_bwd(qkv.data_ptr(), static_cast<const int64_t*>(ptr_or_null(pos)), rope ? ptr_or_null(cos) : nullptr,
+                             rope ? ptr_or_null(sin) : nullptr, rows, f32_or_null(qw), f32_or_null(kw), eps, dq.data_ptr(),
+                             dk.data_ptr(), dv.data_ptr(), dq_c.data_ptr(), dk_c.data_ptr(), dv_c.data_ptr(), dqkv.data_ptr(),
+                             norm ? f32(dparams) : nullptr, norm ? ws.data_ptr() : nullptr, nbytes, B, heads, N, d, block,
+                             stream()), "s3r_qkv_prologue_bwd");
+  return {dqkv, dparams};
+}
+
+// bf16 copies of fp32 tensors, in one launch (up to eight)
+std::vector<Tensor> cast_bf16(at::TensorList xs) {
+  TORCH_CHECK(!xs.empty() && xs.size() <= 8, "cast_bf16: 1 to 8 tensors");
+  c10::cuda::CUDAGuard guard(xs[0].device());
+  std::vector<Tensor> out;
+  const float* src[8];
+  void* dst[8];
+  int64_t counts[8];
+  for (size_t i = 0; i < xs.size(); ++i) {
+    need(xs[i], "x", at::kFloat);
+    out.push_back(fresh(xs[i].sizes(), xs[i], at::kBFloat16));
+    src[i] = f32(xs[i]);
+    dst[i] = out[i].data_ptr();
+    counts[i] = xs[i].numel();
+  }
+  check(s3r_cast_bf16(static_cast<int>(xs.size()), src, dst, counts, stream()), "s3r_cast_bf16");
+  return out;
+}
+
 // ------------------------------------------------------------------------------------------------
 // the base operators as the differentiable ones call them: through the dispatcher, so that fake tensors,
 // functionalisation and dispatch modes see them
@@ -329,6 +413,19 @@ Tensor call_delta(const Tensor& o, const Tensor& d_o) { S3R_DISPATCHED(delta)(o,
 std::tuple<Tensor, Tensor, Tensor, Tensor> call_merge_bwd(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
                                                           const Tensor& o_s, int64_t block) {
   S3R_DISPATCHED(merge_bwd)(dy, gate, o_c, o_s, block);
+}
+
+using SixTensors = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor>;
+SixTensors call_prologue(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos, const optional<Tensor>& cos,
+                         const optional<Tensor>& sin, const optional<Tensor>& qw, const optional<Tensor>& qb,
+                         const optional<Tensor>& kw, const optional<Tensor>& kb, double eps) {
+  S3R_DISPATCHED(prologue_fwd)(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
+}
+std::tuple<Tensor, Tensor> call_prologue_bwd(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos,
+                                             const optional<Tensor>& cos, const optional<Tensor>& sin, const optional<Tensor>& qw,
+                                             const optional<Tensor>& kw, double eps, const Tensor& dq, const Tensor& dk,
+                                             const Tensor& dv, const Tensor& dq_c, const Tensor& dk_c, const Tensor& dv_c) {
+  S3R_DISPATCHED(prologue_bwd)(qkv, heads, block, pos, cos, sin, qw, kw, eps, dq, dk, dv, dq_c, dk_c, dv_c);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -431,6 +528,88 @@ Tensor sel_merge(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor
   return std::get<2>(call_sel(q, k, v, idx, gate, o_c, block, scale, false, false, 1));
 }
 
+// The prologue with its backward.  Norm parameters are fp32 here (prologue() casts them, differentiably).
+struct PrologueNode : torch::autograd::Function<PrologueNode> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos,
+                               const optional<Tensor>& cos, const optional<Tensor>& sin, const optional<Tensor>& qw,
+                               const optional<Tensor>& qb, const optional<Tensor>& kw, const optional<Tensor>& kb, double eps) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    auto [q, k, v, q_c, k_c, v_c] = call_prologue(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
+    auto or_none = [](const optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); };
+    ctx->save_for_backward({qkv, or_none(pos), or_none(cos), or_none(sin), or_none(qw), or_none(kw)});
+    ctx->saved_data["heads"] = heads;
+    ctx->saved_data["block"] = block;
+    ctx->saved_data["eps"] = eps;
+    return {q, k, v, q_c, k_c, v_c};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    auto opt = [](const Tensor& t) { return t.defined() ? optional<Tensor>(t) : optional<Tensor>(); };
+    auto [dqkv, dp] = call_prologue_bwd(s[0], ctx->saved_data["heads"].toInt(), ctx->saved_data["block"].toInt(), opt(s[1]), opt(s[2]),
+                                        opt(s[3]), opt(s[4]), opt(s[5]), ctx->saved_data["eps"].toDouble(), g[0].contiguous(),
+                                        g[1].contiguous(), g[2].contiguous(), g[3].contiguous(), g[4].contiguous(),
+                                        g[5].contiguous());
+    const bool norm = s[4].defined();
+    auto param = [&](int i) { return norm ? dp.select(0, i) : Tensor(); };
+    return {dqkv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), param(0), param(1), param(2), param(3), Tensor()};
+  }
+};
+SixTensors prologue(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos_, const optional<Tensor>& cos,
+                    const optional<Tensor>& sin, const optional<Tensor>& qw_, const optional<Tensor>& qb_,
+                    const optional<Tensor>& kw_, const optional<Tensor>& kb_, double eps) {
+  auto as = [&](const optional<Tensor>& t, at::ScalarType type) {
+    return t.has_value() ? optional<Tensor>(t->to(qkv.device(), type).contiguous()) : t;
+  };
+  TORCH_CHECK(!pos_.has_value() || pos_->device() == qkv.device(), "qkv_prologue: pos must be on ", qkv.device());
+  const auto pos = as(pos_, at::kLong), qw = as(qw_, at::kFloat), qb = as(qb_, at::kFloat), kw = as(kw_, at::kFloat), kb = as(kb_, at::kFloat);
+  auto grad = [](const optional<Tensor>& t) { return t.has_value() && t->requires_grad(); };
+  if (at::GradMode::is_enabled() && (qkv.requires_grad() || grad(qw) || grad(qb) || grad(kw) || grad(kb))) {
+    const auto r = PrologueNode::apply(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
+    return {r[0], r[1], r[2], r[3], r[4], r[5]};
+  }
+  return call_prologue(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
+}
+
+// The whole attention module without gradients: projections (cuBLAS), sigmoid of the gate, prologue, the two attentions,
+// output projection.  fp32 input and parameters are rounded to bf16 as under autocast, all in one launch.
+std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, const optional<Tensor>& b_qkv, const Tensor& w_gate,
+                                        const optional<Tensor>& b_gate, const Tensor& w_proj, const optional<Tensor>& b_proj,
+                                        const optional<Tensor>& pos, const optional<Tensor>& cos, const optional<Tensor>& sin,
+                                        const optional<Tensor>& qw, const optional<Tensor>& qb, const optional<Tensor>& kw,
+                                        const optional<Tensor>& kb, double eps, int64_t heads, int64_t block, int64_t topk,
+                                        double scale) {
+  at::NoGradGuard no_grad;
+  c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+  std::vector<Tensor> in = {x_, w_qkv, w_gate, w_proj};
+  const optional<Tensor>* biases[3] = {&b_qkv, &b_gate, &b_proj};
+  int at_bias[3] = {-1, -1, -1};
+  for (int i = 0; i < 3; ++i)
+    if (biases[i]->has_value()) {
+      at_bias[i] = static_cast<int>(in.size());
+      in.push_back(**biases[i]);
+    }
+  std::vector<Tensor> wide;
+  std::vector<size_t> where;
+  for (size_t i = 0; i < in.size(); ++i)
+    if (in[i].scalar_type() == at::kFloat) {
+      wide.push_back(in[i].contiguous());
+      where.push_back(i);
+    }
+  if (!wide.empty()) {
+    const auto narrow = cast_bf16(wide);
+    for (size_t i = 0; i < where.size(); ++i) in[where[i]] = narrow[i];
+  }
+  auto bias = [&](int i) { return at_bias[i] >= 0 ? optional<Tensor>(in[at_bias[i]]) : optional<Tensor>(); };
+  const Tensor& x = in[0];
+  const int64_t B = x.size(0), N = x.size(1);
+  const Tensor qkv = at::linear(x, in[1], bias(0));
+  const Tensor gate = at::linear(x, in[2], bias(1)).sigmoid_().view({B, N, heads, 2}).permute({0, 2, 1, 3});
+  auto [q, k, v, q_c, k_c, v_c] = prologue(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
+  auto [o_c, lse, idx] = call_cmp_topk(q_c, k_c, v_c, topk, scale);
+  const Tensor y = std::get<2>(call_sel(q, k, v, idx, gate, o_c, block, scale, false, false, 1));
+  return {at::linear(y, in[3], bias(2)), idx};
+}
+
 // The whole op.  group = 0 where compressed keys are the selection blocks.  As one node its backward adds the
 // pooled branch's gradients inside the selection kernels' stores: separate nodes write them out as [B,H,T,d] and add
 // two bf16 tensors three times (1.5 of 19.4 ms at 250 views).
@@ -493,7 +672,16 @@ TORCH_LIBRARY(speed3r_b200, m) {
   m.def("pool_qkv_fwd(Tensor q, Tensor k, Tensor v, int block, int kernel, int stride) -> (Tensor, Tensor, Tensor)");
   m.def("delta(Tensor o, Tensor d_o) -> Tensor");
   m.def("merge_bwd(Tensor dy, Tensor gate, Tensor o_c, Tensor o_s, int block) -> (Tensor, Tensor, Tensor, Tensor)");
+  m.def("prologue_fwd(Tensor qkv, int heads, int block, Tensor? pos, Tensor? cos, Tensor? sin, Tensor? qw, Tensor? qb, "
+        "Tensor? kw, Tensor? kb, float eps) -> (Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)");
+  m.def("prologue_bwd(Tensor qkv, int heads, int block, Tensor? pos, Tensor? cos, Tensor? sin, Tensor? qw, Tensor? kw, "
+        "float eps, Tensor dq, Tensor dk, Tensor dv, Tensor dq_c, Tensor dk_c, Tensor dv_c) -> (Tensor, Tensor)");
 
+  m.def("prologue(Tensor qkv, int heads, int block, Tensor? pos, Tensor? cos, Tensor? sin, Tensor? qw, Tensor? qb, "
+        "Tensor? kw, Tensor? kb, float eps) -> (Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)", &prologue);
+  m.def("module_infer(Tensor x, Tensor w_qkv, Tensor? b_qkv, Tensor w_gate, Tensor? b_gate, Tensor w_proj, Tensor? b_proj, "
+        "Tensor? pos, Tensor? cos, Tensor? sin, Tensor? qw, Tensor? qb, Tensor? kw, Tensor? kb, float eps, int heads, "
+        "int block, int topk, float scale) -> (Tensor, Tensor)", &module_infer);
   m.def("pool_tokens(Tensor x, int kernel, int stride) -> Tensor", &pool_tokens);
   m.def("flash_attn_topk(Tensor q, Tensor k, Tensor v, int topk, float scale, int group, int take) -> (Tensor, Tensor)",
         &flash_attn_topk);
@@ -515,6 +703,8 @@ TORCH_LIBRARY(speed3r_b200, m) {
   m.impl("sel_attn_bwd", &sel_attn_bwd);                    \
   m.impl("sel_attn_bwd_pooled", &sel_attn_bwd_pooled);      \
   m.impl("pool_qkv_fwd", &pool_qkv_fwd);                    \
+  m.impl("prologue_fwd", &prologue_fwd);                    \
+  m.impl("prologue_bwd", &prologue_bwd);                    \
   m.impl("delta", &delta);                                  \
   m.impl("merge_bwd", &merge_bwd)
 

@@ -84,6 +84,17 @@ def _register_fakes() -> None:
         nc = (T - kernel) // stride + 1
         return tuple(q.new_empty(B, H, n, d) for n in ((T - block) // block + 1, nc, nc))
 
+    @fake("speed3r_b200::prologue_fwd")
+    def _(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps):
+        B, N = qkv.shape[:2]
+        d = qkv.numel() // (B * N * 3 * heads)
+        return tuple(qkv.new_empty(B, heads, n, d) for n in (N, N, N, N // block, N // block, N // block))
+
+    @fake("speed3r_b200::prologue_bwd")
+    def _(qkv, heads, block, pos, cos, sin, qw, kw, eps, dq, dk, dv, dq_c, dk_c, dv_c):
+        return (qkv.new_empty(qkv.shape),
+                qkv.new_empty((0,) if qw is None else (4, dq.shape[-1]), dtype=torch.float32))
+
     @fake("speed3r_b200::delta")
     def _(o, d_o):
         return o.new_empty(o.shape[:-1], dtype=torch.float32)
@@ -108,10 +119,6 @@ def _ops():
     return _ns
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
 def _need(t: Tensor, name: str, dtype=_BF16, contiguous=True) -> None:
     if not t.is_cuda:
         raise RuntimeError(f"{name} must be a CUDA tensor: the speed3r_b200 kernels have no CPU path")
@@ -119,10 +126,6 @@ def _need(t: Tensor, name: str, dtype=_BF16, contiguous=True) -> None:
         raise RuntimeError(f"{name} must be {dtype}, got {t.dtype}")
     if contiguous and not t.is_contiguous():
         raise RuntimeError(f"{name} must be contiguous")
-
-
-def _ptr(t: Optional[Tensor]) -> int:
-    return 0 if t is None else t.data_ptr()
 
 
 def _scale(softmax_scale: Optional[float], q: Tensor) -> float:
@@ -160,42 +163,20 @@ def qkv_prologue(qkv: Tensor, num_heads: int, block: int, pos: Optional[Tensor] 
     block's truncated mean position."""
     _need(qkv, "qkv")
     if qkv.requires_grad and torch.is_grad_enabled():
-        raise RuntimeError("qkv_prologue is forward-only; run the separate steps when gradients are needed")
-    B, N, C3 = qkv.shape[0], qkv.shape[1], qkv.numel() // (qkv.shape[0] * qkv.shape[1])
-    d = C3 // (3 * num_heads)
-    if C3 != 3 * num_heads * d or N % block:
-        raise RuntimeError(f"qkv_prologue: qkv {tuple(qkv.shape)} does not split into 3 x {num_heads} heads, "
-                           f"or N={N} is not a multiple of the block {block}")
+        raise RuntimeError("qkv_prologue is forward-only; the module's training path uses its differentiable form")
+    with torch.no_grad():
+        return _prologue(qkv, num_heads, block, pos, cos, sin, q_norm, k_norm)
+
+
+def _prologue(qkv, num_heads, block, pos, cos, sin, q_norm, k_norm):
+    """``qkv_prologue`` with a backward."""
     if (q_norm is None) != (k_norm is None):
         raise RuntimeError("qkv_prologue: q_norm and k_norm come together or not at all")
-    dev = qkv.device
-    f32 = lambda t: t.detach().to(device=dev, dtype=torch.float32).contiguous()
-    qw = qb = kw = kb = None
-    eps = 1e-5
-    if q_norm is not None:
-        if abs(q_norm[2] - k_norm[2]) > 0:
-            raise RuntimeError("qkv_prologue: q_norm and k_norm must share eps")
-        qw, qb, kw, kb, eps = f32(q_norm[0]), f32(q_norm[1]), f32(k_norm[0]), f32(k_norm[1]), float(q_norm[2])
-    rows = 0
-    if pos is not None:
-        _need(cos, "cos")
-        _need(sin, "sin")
-        if cos.shape != sin.shape or cos.dim() != 2 or cos.shape[1] != d // 2:
-            raise RuntimeError(f"qkv_prologue: cos/sin tables must be [rows,{d // 2}]")
-        if tuple(pos.shape) != (B, N, 2) or pos.device != dev:
-            raise RuntimeError(f"qkv_prologue: pos must be [B,N,2] = {(B, N, 2)} on {dev}")
-        pos = pos.to(torch.int64).contiguous()
-        rows = cos.shape[0]
-    mk = lambda n: torch.empty(B, num_heads, n, d, device=dev, dtype=qkv.dtype)
-    q, k, v = mk(N), mk(N), mk(N)
-    q_c, k_c, v_c = mk(N // block), mk(N // block), mk(N // block)
-    with torch.cuda.device(dev):
-        _lib.check(_lib.load().s3r_qkv_prologue_fwd(
-            qkv.data_ptr(), _ptr(pos), _ptr(cos) if pos is not None else 0, _ptr(sin) if pos is not None else 0, rows,
-            _ptr(qw), _ptr(qb), _ptr(kw), _ptr(kb), eps, q.data_ptr(), k.data_ptr(), v.data_ptr(),
-            q_c.data_ptr(), k_c.data_ptr(), v_c.data_ptr(), B, num_heads, N, d, block, _stream()),
-            "s3r_qkv_prologue_fwd")
-    return q, k, v, q_c, k_c, v_c
+    if q_norm is not None and abs(q_norm[2] - k_norm[2]) > 0:
+        raise RuntimeError("qkv_prologue: q_norm and k_norm must share eps")
+    qw, qb, eps = q_norm if q_norm is not None else (None, None, 1e-5)
+    kw, kb, _ = k_norm if k_norm is not None else (None, None, 0.0)
+    return _ops().prologue.default(qkv, num_heads, block, pos, cos, sin, qw, qb, kw, kb, float(eps))
 
 
 # ------------------------------------------------------------------------------------------------

@@ -6,9 +6,9 @@ attn_bias=None, xpos=None)`` of pi3/models/layers/sparse_attention.py:60-141, so
 the reference loads unchanged and ``BlockRope(attn_class=SparseFlashAttentionRope)`` works
 (pi3/models/layers/block.py:282-312).  The projections stay PyTorch (cuBLAS) code; pooling, the compression attention with its top-k
 selection, the selection attention and the gated merge run in the CUDA library (speed3r_b200.ops).
-Without gradients the LayerNorms, the rotary embedding, the pooling and the q/k/v split run as one
-library kernel as well (``ops.qkv_prologue``); with gradients they stay PyTorch code around the
-differentiable ops.
+The LayerNorms, the rotary embedding, the pooling and the q/k/v split run as one library kernel as well
+(``ops.qkv_prologue``), with gradients as without; settings that kernel does not take stay PyTorch code around
+the differentiable ops.
 
 The reference's literals (pooling 16/16, top-k 32) are keyword arguments here with the same
 defaults.
@@ -51,6 +51,14 @@ class _TableRows:
         seen = self._seen
         self._seen[key] = (weakref.ref(base, lambda _r, k=key: seen.pop(k, None)), base._version)
         return self.rows
+
+
+_WIDE = (torch.float32, torch.bfloat16)
+
+
+def _global_hooks() -> bool:
+    m = nn.modules.module
+    return bool(m._global_forward_hooks or m._global_forward_pre_hooks)
 
 
 def rope_tables(rope, D: int, rows: int, device, dtype):
@@ -152,11 +160,14 @@ class SparseFlashAttentionRope(nn.Module):
         self.seq_parallel = None     # a seq_parallel.SequenceParallel: x holds this rank's slice of the views
 
     def _can_fuse_prologue(self, qkv, x, xpos, N, Bs, d) -> bool:
-        """Inference (nothing to differentiate), norms that are LayerNorm(d) with affine or Identity, a 2-D
-        rotary module (this package's or the reference's pure-PyTorch one) or none, whole blocks, head
-        counts the kernel takes."""
+        """Inference (nothing to differentiate) in a setting the one-pass prologue takes."""
         if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
             return False
+        return self._prologue_takes(xpos, N, Bs, d)
+
+    def _prologue_takes(self, xpos, N, Bs, d) -> bool:
+        """Norms that are LayerNorm(d) with affine or Identity, a 2-D rotary module (this package's or the
+        reference's pure-PyTorch one) or none, whole blocks, head counts the kernel takes."""
         norms = (self.q_norm, self.k_norm)
         ident = all(isinstance(m, nn.Identity) for m in norms)
         ln = all(isinstance(m, nn.LayerNorm) and m.elementwise_affine and m.bias is not None and
@@ -167,16 +178,60 @@ class SparseFlashAttentionRope(nn.Module):
             return False
         return d == 64 and N % Bs == 0 and self.num_heads <= 42
 
-    def _forward_fused(self, qkv, gate, xpos, B, N, H, d, Bs) -> Tensor:
-        cos = sin = None
+    def _can_run_native(self, x, xpos, N, Bs, d) -> bool:
+        """Inference in which the whole module is one native call: plain Linear projections that nobody watches, bf16
+        (by autocast or by dtype), no dropout, no sequence partition."""
+        lins = (self.qkv, self.gate[0], self.proj)
+        mods = lins + (self.gate, self.gate[1], self.q_norm, self.k_norm, self.proj_drop)
+        if (torch.is_grad_enabled() or self.seq_parallel is not None or not x.is_cuda or type(x) is not Tensor or
+                (self.training and self.proj_drop.p > 0) or type(self.gate) is not nn.Sequential or len(self.gate) != 2 or
+                type(self.gate[1]) is not nn.Sigmoid or any(type(m) is not nn.Linear for m in lins) or
+                any(m._forward_hooks or m._forward_pre_hooks for m in mods) or _global_hooks() or
+                torch.compiler.is_compiling()):
+            return False
+        params = [p for m in lins for p in (m.weight, m.bias) if p is not None]
+        if any(type(p) is not nn.Parameter or p.device != x.device for p in params):
+            return False
+        if torch.is_autocast_enabled("cuda"):
+            if torch.get_autocast_dtype("cuda") != torch.bfloat16 or x.dtype not in _WIDE or any(p.dtype not in _WIDE for p in params):
+                return False
+        elif x.dtype != torch.bfloat16 or any(p.dtype != torch.bfloat16 for p in params):
+            return False
+        return self._can_fuse_prologue(None, x, xpos, N, Bs, d)
+
+    def _rope_and_norms(self, xpos, d, device, dtype):
+        """(cos, sin, q_norm, k_norm) as the one-pass prologue takes them."""
+        cos = sin = qn = kn = None
         if xpos is not None:
             rows = self.rope._seq_len(xpos) if isinstance(self.rope, RoPE2D) else self._rows(xpos)
-            cos, sin = rope_tables(self.rope, d // 2, rows, qkv.device, qkv.dtype)
-        qn = kn = None
+            cos, sin = rope_tables(self.rope, d // 2, rows, device, dtype)
         if isinstance(self.q_norm, nn.LayerNorm):
             qn = (self.q_norm.weight, self.q_norm.bias, self.q_norm.eps)
             kn = (self.k_norm.weight, self.k_norm.bias, self.k_norm.eps)
-        q, k, v, q_c, k_c, v_c = ops.qkv_prologue(qkv.detach(), H, Bs, xpos, cos, sin, qn, kn)
+        return cos, sin, qn, kn
+
+    def _forward_native(self, x, xpos, H, d, Bs) -> Tensor:
+        cos, sin, qn, kn = self._rope_and_norms(xpos, d, x.device, torch.bfloat16)
+        qw, qb, eps = qn if qn is not None else (None, None, 1e-5)
+        kw, kb, _ = kn if kn is not None else (None, None, 0.0)
+        g = self.gate[0]
+        y, idx = ops._ops().module_infer.default(x, self.qkv.weight, self.qkv.bias, g.weight, g.bias, self.proj.weight,
+                                                 self.proj.bias, xpos, cos, sin, qw, qb, kw, kb, eps, H, Bs, self.topk,
+                                                 1.0 / d ** 0.5)
+        if self.record_idx:
+            self.last_idx = idx
+        return y
+
+    def _forward_fused(self, qkv, gate, xpos, B, N, H, d, Bs, train=False) -> Tensor:
+        cos, sin, qn, kn = self._rope_and_norms(xpos, d, qkv.device, qkv.dtype)
+        q, k, v, q_c, k_c, v_c = ops._prologue(qkv, H, Bs, xpos, cos, sin, qn, kn)
+        if self.seq_parallel is not None and train:
+            # this rank's queries against the whole sequence; the backward reduce-scatters dK and dV
+            y, idx = self.seq_parallel.attention_grad(q, k, v, q_c, k_c, v_c, gate, Bs, self.topk,
+                                                      ops.flash_attn_topk_func, ops.sel_attn_merge)
+            if self.record_idx:
+                self.last_idx = idx.detach()
+            return self.proj_drop(self.proj(y))
         if self.seq_parallel is not None:
             # this rank's query blocks against the whole sequence: pooled and token-level K/V are exchanged
             y, idx = self.seq_parallel.attention(q, k, v, q_c, k_c, v_c, gate, Bs, self.topk,
@@ -195,6 +250,8 @@ class SparseFlashAttentionRope(nn.Module):
         H = self.num_heads
         d = C // H
         Bs = self.block_size ** 2
+        if self._can_run_native(x, xpos, N, Bs, d):
+            return self._forward_native(x, xpos, H, d, Bs)
         qkv = self.qkv(x)
         gate = self.gate(x).view(B, N, H, 2).permute(0, 2, 1, 3)          # [B,H,N,2] view, no copy
         if qkv.dtype != torch.bfloat16:
@@ -202,7 +259,9 @@ class SparseFlashAttentionRope(nn.Module):
                                f"got {qkv.dtype}")
         gate = gate.to(qkv.dtype)
         if self._can_fuse_prologue(qkv, x, xpos, N, Bs, d):
-            return self._forward_fused(qkv, gate, xpos, B, N, H, d, Bs)
+            return self._forward_fused(qkv.detach(), gate, xpos, B, N, H, d, Bs)
+        if torch.is_grad_enabled() and self._prologue_takes(xpos, N, Bs, d):
+            return self._forward_fused(qkv, gate, xpos, B, N, H, d, Bs, train=True)
         if self.seq_parallel is not None and N % Bs != 0:
             raise RuntimeError("sequence-parallel attention needs whole 16-token blocks on every rank")
         qkv5 = qkv.view(B, N, 3, H, d)

@@ -190,3 +190,97 @@ def test_cmp_table_when_the_bound_is_loose(period):
     first = idx[..., 0:1].cpu().long()
     assert torch.equal(idx.cpu().long(), first + period * torch.arange(32))
     assert_bf16_close(o, ref, "o_c")
+
+
+# ------------------------------------------------------------------ prologue backward, module paths
+@pytest.mark.parametrize("B,H,Bs,blocks,norm,rope", [(1, 1, 16, 1, True, True), (2, 16, 16, 7, True, True),
+                                                     (1, 17, 16, 3, True, True), (2, 3, 4, 5, True, False),
+                                                     (1, 2, 9, 4, False, True), (2, 16, 16, 200, True, True)])
+def test_prologue_backward(B, H, Bs, blocks, norm, rope):
+    """Gradients of the packed projection and of the norms' parameters against autograd through the fp32 restatement: one
+    block, more blocks than CTAs, blocks of odd length, more heads than the small kernel takes, no norms, no rotary embedding."""
+    import speed3r_b200
+    from speed3r_b200 import ops
+    N, d = Bs * blocks, 64
+    qkv, = bf16_round(1.5 * randn(70, B, N, 3 * H * d) + 0.3)
+    pos = torch.randint(0, 37, (B, N, 2), generator=torch.Generator().manual_seed(71)) if rope else None
+    norms = [(1 + 0.2 * randn(72 + i, d), 0.1 * randn(74 + i, d)) for i in range(2)] if norm else None
+    shapes = [(B, H, N, d)] * 3 + [(B, H, blocks, d)] * 3
+    grads = bf16_round(*(randn(80 + i, *s) for i, s in enumerate(shapes)))
+    table = speed3r_b200.RoPE2D(100.0)
+    cos, sin = table._cos_sin(d // 2, 37, torch.device(DEV), torch.bfloat16) if rope else (None, None)
+    x = qkv.to(DEV, torch.bfloat16).requires_grad_(True)
+    leaves = [(w.to(DEV).requires_grad_(True), b.to(DEV).requires_grad_(True), 1e-5) for w, b in norms] if norm else [None, None]
+    out = ops._prologue(x, H, Bs, pos.to(DEV) if rope else None, cos, sin, *leaves)
+    torch.autograd.backward(out, [g.to(DEV, torch.bfloat16) for g in grads])
+    xr = qkv.clone().requires_grad_(True)
+    ref_leaves = [(w.clone().requires_grad_(True), b.clone().requires_grad_(True)) for w, b in norms] if norm else [None, None]
+    ref = _prologue_fp32(xr, H, Bs, pos, cos, sin, *ref_leaves)
+    torch.autograd.backward(ref, grads)
+    # one rounding to bf16 (2^-9 of the value), and the mean of the block in the restatement is not rounded to bf16
+    scale = xr.grad.abs().max().item()
+    assert (x.grad.float().cpu() - xr.grad).abs().max().item() <= 1e-2 * scale
+    if norm:
+        for (w, b, _), (wr, br) in zip(leaves, ref_leaves):
+            for a, r in ((w, wr), (b, br)):
+                assert (a.grad.cpu() - r.grad).abs().max() <= 2e-3 * max(1.0, r.grad.abs().max().item())
+
+
+def _prologue_fp32(qkv, H, Bs, pos, cos, sin, qn, kn):
+    """Split, LayerNorm, rotary embedding and pooling in fp32 with the given (bf16) rotary tables."""
+    B, N, d = qkv.shape[0], qkv.shape[1], 64
+    q, k, v = (qkv.view(B, N, 3, H, d)[:, :, i].permute(0, 2, 1, 3) for i in range(3))
+    pool = lambda t: t.reshape(B, H, N // Bs, Bs, d).mean(3)
+    ln = lambda t, p: t if p is None else torch.nn.functional.layer_norm(t, (d,), *p)
+    def rot(t, at):
+        if pos is None:
+            return t
+        halves = []
+        for i, h in enumerate(t.chunk(2, -1)):
+            c, s = (tab.float().cpu()[at[..., i]][:, None] for tab in (cos, sin))
+            a, b = h.chunk(2, -1)
+            halves.append(h * c + torch.cat((-b, a), -1) * s)
+        return torch.cat(halves, -1)
+    at_c = None if pos is None else pos.view(B, N // Bs, Bs, 2).float().mean(2).int().long()
+    return (rot(ln(q, qn), pos), rot(ln(k, kn), pos), v, rot(ln(pool(q), qn), at_c), rot(ln(pool(k), kn), at_c), pool(v))
+
+
+@pytest.mark.parametrize("params,x_dtype,autocast,bias", [(torch.float32, torch.float32, True, True),
+                                                          (torch.float32, torch.bfloat16, True, False),
+                                                          (torch.bfloat16, torch.bfloat16, False, True)])
+def test_module_native_inference_matches_separate_projections(params, x_dtype, autocast, bias):
+    """The module as one native call against the same module with a hook on a projection, which keeps the projections in
+    PyTorch: same roundings, so equal up to the GEMM's summation order."""
+    import speed3r_b200
+    torch.manual_seed(0)
+    m = speed3r_b200.SparseFlashAttentionRope(256, num_heads=4, qkv_bias=bias, proj_bias=bias, qk_norm=True,
+                                              rope=speed3r_b200.RoPE2D(100.0)).to(DEV, params).eval()
+    x = torch.randn(2, 512, 256, device=DEV, dtype=x_dtype)
+    tok = torch.arange(512, device=DEV) % 256
+    xpos = torch.stack((tok // 16, tok % 16), -1)[None].expand(2, -1, -1).contiguous()
+    m.record_idx = True
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16, enabled=autocast):
+        assert m._can_run_native(x, xpos, 512, 16, 64)
+        y = m(x, xpos=xpos)
+        idx = m.last_idx
+        h = m.proj.register_forward_hook(lambda *a: None)
+        assert not m._can_run_native(x, xpos, 512, 16, 64)
+        y2 = m(x, xpos=xpos)
+        h.remove()
+    assert y.dtype == y2.dtype and y.shape == y2.shape
+    assert (idx != m.last_idx).float().mean() < 2e-2
+    assert_bf16_close(y, y2.float(), "native module", max_abs=2e-2, mean_abs=1e-3)
+
+
+def test_cast_bf16_sizes():
+    """Every remainder of a thread's eight elements and of a block's, in one launch with other tensors."""
+    import ctypes as C
+    from speed3r_b200 import _lib
+    sizes = [1, 7, 8, 9, 8191, 8192, 8193, 100003]
+    xs = [torch.randn(n, device=DEV) for n in sizes]
+    ys = [torch.empty(n, device=DEV, dtype=torch.bfloat16) for n in sizes]
+    n = len(sizes)
+    _lib.check(_lib.load().s3r_cast_bf16(n, (C.c_void_p * n)(*(t.data_ptr() for t in xs)), (C.c_void_p * n)(*(t.data_ptr() for t in ys)),
+                                         (C.c_int64 * n)(*sizes), torch.cuda.current_stream().cuda_stream), "s3r_cast_bf16")
+    for x, y in zip(xs, ys):
+        assert torch.equal(y, x.bfloat16())
