@@ -1,0 +1,388 @@
+// Selection branch, forward, blocks of 32 and 64 tokens: on tcgen05.
+//
+// A row tile of 128 queries is G = 128 / BS query blocks, each with its own list of key blocks.  A step takes the next key
+// block of every list: a key tile of 128 rows, one BS x 64 copy per list.  S = Q K^T (M=128, N=128) holds G x G blocks, of
+// which the diagonal ones are wanted: block g's queries against its own key block.  The softmax threads read those alone; P
+// is written over the diagonal blocks of a zeroed tile, so that O += P V (K=128) adds the right keys to each row.  The
+// G - 1 unwanted blocks beside each wanted one are cheaper than mma.sync without them: 16 heads, top-16 blocks of 64 at 250
+// views 3.86 -> 2.40 ms, 64 views 1002 -> 555 us; top-32 blocks of 32, 60000 tokens 1073 -> 818 us.
+// Bound: shared memory (copies 32 KB, operands 48 KB per step and CTA, at 128 bytes per cycle) and the tensor pipe, both about
+// three quarters busy inside a row tile; its start and its end take a fifth of its time.  Two threads per row instead of one
+// changed nothing (576 us); leaving out the exponentials, the second product or the gather's cache misses alone 3 % each.
+// Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-7 softmax, thread = row.
+// Two CTAs per SM: their steps fill each other's waits.
+// The exponent offset of a row is the maximum of its first step; a CTA in which some row outgrew it by more than 2^64 takes
+// its keys a second time with the exact maxima (cmp_attn.cu).
+#include "sel_common.cuh"
+
+namespace s3r {
+
+constexpr int kSbgTile = 128 * 128;            // 128 rows x 64 bf16, bytes
+constexpr int kSbgStages = 3;
+constexpr int kSbgOffK = kSbgTile;
+constexpr int kSbgOffV = kSbgOffK + kSbgStages * kSbgTile;
+constexpr int kSbgOffCtl = kSbgOffV + kSbgStages * kSbgTile;
+constexpr int kSbgThreads = 256;
+constexpr uint32_t kSbgColO = 128, kSbgColP = 192;
+
+struct SbgCtl {
+  uint64_t q_full, o_full;
+  uint64_t k_full[kSbgStages], k_empty[kSbgStages], v_full[kSbgStages], v_empty[kSbgStages];
+  uint64_t s_full, s_free, p_full, pv_done;
+  uint32_t tmem_base, abort_flag, again;
+  int nvalid[4], steps;
+};
+constexpr int kSbgOffList = kSbgOffCtl + 256;  // [G][topk] int32: first token of each valid key block
+// two CTAs fit an SM up to 115712 bytes each: lists of up to 64 entries for blocks of 64, 48 for blocks of 32
+static_assert(sizeof(SbgCtl) <= 256, "control words");
+
+template <int BS>
+__global__ void __launch_bounds__(kSbgThreads, 2)
+sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+               const __grid_constant__ CUtensorMap map_v, const SelParams p) {
+  constexpr int G = 128 / BS;                  // query blocks per row tile
+  extern __shared__ __align__(1024) uint8_t smem[];
+  SbgCtl& ctl = *reinterpret_cast<SbgCtl*>(smem + kSbgOffCtl);
+  int32_t* lists = reinterpret_cast<int32_t*>(smem + kSbgOffList);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_per_bh = (p.nqb + G - 1) / G;
+  const int bh = blockIdx.x / tiles_per_bh, qb0 = (blockIdx.x % tiles_per_bh) * G;
+  const uint32_t sbase = smem_u32(smem);
+
+  if (threadIdx.x == 0) {
+    ctl.abort_flag = 0;
+    ctl.again = 0;
+    mbar_init(&ctl.q_full, 1);
+    mbar_init(&ctl.o_full, 1);
+    for (int s = 0; s < kSbgStages; ++s) {
+      mbar_init(&ctl.k_full[s], 1);
+      mbar_init(&ctl.k_empty[s], 1);
+      mbar_init(&ctl.v_full[s], 1);
+      mbar_init(&ctl.v_empty[s], 1);
+    }
+    mbar_init(&ctl.s_full, 1);
+    mbar_init(&ctl.s_free, 4);
+    mbar_init(&ctl.p_full, 4);
+    mbar_init(&ctl.pv_done, 1);
+    mbar_fence_init();
+  }
+  if (warp == 2) {
+    tmem_alloc(&ctl.tmem_base, 256);
+    tmem_relinquish();
+  }
+  if (warp >= 4 && warp < 4 + G) {
+    // valid entries of one query block's row of the table, table order
+    const int g = warp - 4, qb = qb0 + g;
+    int n = 0;
+    if (qb < p.nqb) {
+      const int32_t* row = p.idx + (static_cast<int64_t>(bh) * p.nqb + qb) * p.topk;
+      for (int r0 = 0; r0 < p.topk; r0 += 32) {
+        const int i = r0 + lane, e = i < p.topk ? row[i] : -1;
+        const bool ok = e >= 0 && static_cast<int64_t>(e) * BS < p.Tk;
+        const uint32_t m = __ballot_sync(0xffffffffu, ok);
+        if (ok) lists[g * p.topk + n + __popc(m & ((1u << lane) - 1u))] = e * BS;
+        n += __popc(m);
+      }
+    }
+    if (lane == 0) ctl.nvalid[g] = n;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = ctl.tmem_base;
+  volatile uint32_t* abort_flag = &ctl.abort_flag;
+  int steps = ctl.nvalid[0];
+#pragma unroll
+  for (int g = 1; g < G; ++g) steps = max(steps, ctl.nvalid[g]);
+  const bool aligned = (sbase & 1023u) == 0;   // the swizzled tiles need it; dynamic shared memory starts there
+  if (!aligned) steps = 0;
+
+  // Steps are counted through both passes (n = pass * steps + j), every role meets the others at the end of a pass.
+  auto another_pass = [&](int pass) {
+    __syncthreads();
+    return pass == 0 && *static_cast<volatile uint32_t*>(&ctl.again) != 0u && *abort_flag == 0u;
+  };
+  if (warp < 4) {
+    if (warp == 0) {
+      // ---------------------------------------------------------------- TMA producer
+      const bool chunked = p.Tc != p.Tk;
+      int pass = 0;
+      do {
+        // lane g copies for list g; a list that has ended repeats its last block (its scores are masked, its values are
+        // finite whenever the list's own are); an empty one takes the sequence's first block
+        int issued = pass * steps;
+        if (steps > 0 && pass == 0 && lane == 0) {
+          mbar_expect_tx(&ctl.q_full, kSbgTile);
+          tma_load_4d_u32(sbase, &map_q, &ctl.q_full, 0, qb0 * BS, bh, 0);
+        }
+        const int nv = lane < G ? ctl.nvalid[lane] : 0;
+        for (int j = 0; j < steps; ++j) {
+          const int n = pass * steps + j, s = n % kSbgStages;
+          const uint32_t ph = (n / kSbgStages) & 1;
+          int tok = 0, ch = 0;
+          if (lane < G && nv > 0) tok = lists[lane * p.topk + min(j, nv - 1)];
+          if (chunked) { ch = tok / p.Tc; tok -= ch * p.Tc; }
+          if (!mbar_wait_warp(&ctl.k_empty[s], ph ^ 1, abort_flag)) break;
+          if (lane == 0) mbar_expect_tx(&ctl.k_full[s], kSbgTile);
+          __syncwarp();
+          if (lane < G) tma_load_4d_u32(sbase + kSbgOffK + s * kSbgTile + lane * BS * 128, &map_k, &ctl.k_full[s], 0, tok, bh, ch);
+          issued = n + 1;                                                   // K of step n is in flight
+          if (!mbar_wait_warp(&ctl.v_empty[s], ph ^ 1, abort_flag)) break;
+          if (lane == 0) mbar_expect_tx(&ctl.v_full[s], kSbgTile);
+          __syncwarp();
+          if (lane < G) tma_load_4d_u32(sbase + kSbgOffV + s * kSbgTile + lane * BS * 128, &map_v, &ctl.v_full[s], 0, tok, bh, ch);
+        }
+        if (*abort_flag) {
+          // give copies already in flight a bounded chance to land before the CTA's memory is released
+          for (int n = max(0, issued - kSbgStages); n < issued; ++n) {
+            volatile uint32_t dummy = 0;
+            mbar_wait(&ctl.k_full[n % kSbgStages], (n / kSbgStages) & 1, &dummy);
+          }
+        }
+        __syncwarp();
+      } while (another_pass(pass++));
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- MMA issuer
+      const bool leader = elect_one_sync();
+      constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0);
+      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 64, 0, 1);         // V tile is [keys][d]: N contiguous
+      const uint64_t desc_q = umma_desc_sw128(sbase), desc_k = umma_desc_sw128(sbase + kSbgOffK),
+                     desc_v = umma_desc_sw128(sbase + kSbgOffV);
+      auto issue_qk = [&](int s) {
+        umma_ss_k4<2, 2>(tmem, desc_q, desc_k + static_cast<uint64_t>(s * (kSbgTile >> 4)), idesc_qk, 0u);
+        umma_commit(&ctl.s_full);
+        umma_commit(&ctl.k_empty[s]);
+      };
+      auto issue_pv = [&](int s, uint32_t acc) {
+        const uint64_t v = desc_v + static_cast<uint64_t>(s * (kSbgTile >> 4));
+        umma_ts_k4<128>(tmem + kSbgColO, tmem + kSbgColP, v, idesc_pv, acc);
+        umma_ts_k4<128>(tmem + kSbgColO, tmem + kSbgColP + 32, v + 4 * 128, idesc_pv, 1u);
+        umma_commit(&ctl.pv_done);
+        umma_commit(&ctl.v_empty[s]);
+      };
+      bool ok = steps == 0 || mbar_wait_warp(&ctl.q_full, 0, abort_flag);
+      int pass = 0, s = 0, n = 0;
+      uint32_t ph = 0;
+      do {
+        ok = ok && (steps == 0 || mbar_wait_warp(&ctl.k_full[s], ph, abort_flag));
+        if (ok && steps > 0) {
+          tc_fence_after();
+          if (leader) issue_qk(s);
+          __syncwarp();
+        }
+#pragma unroll 1
+        for (int j = 0; j < steps && ok; ++j, ++n) {
+          const bool nxt = j + 1 < steps;
+          const int sn = s + 1 == kSbgStages ? 0 : s + 1;
+          const uint32_t phn = sn == 0 ? ph ^ 1u : ph;
+          if (nxt) {
+            ok = mbar_wait_warp(&ctl.k_full[sn], phn, abort_flag) &&
+                 mbar_wait_warp(&ctl.s_free, n & 1, abort_flag);            // S of step n is in registers
+            if (!ok) break;
+            tc_fence_after();
+            if (leader) issue_qk(sn);
+            __syncwarp();
+          }
+          ok = mbar_wait_warp(&ctl.v_full[s], ph, abort_flag) && mbar_wait_warp(&ctl.p_full, n & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (leader) issue_pv(s, j > 0 ? 1u : 0u);
+          __syncwarp();
+          s = sn;
+          ph = phn;
+        }
+        if (leader) umma_commit(&ctl.o_full);
+        __syncwarp();
+        if (!ok) {
+          volatile uint32_t dummy = 0;
+          mbar_wait(&ctl.o_full, pass & 1, &dummy);       // let issued MMAs drain before tensor memory is freed
+        }
+      } while (another_pass(pass++));
+    } else {
+      int pass = 0;
+      while (another_pass(pass++)) {}
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax, thread = row
+    const int quarter = warp & 3, r = quarter * 32 + lane, g = (quarter * 32) / BS, row = qb0 * BS + r;
+    const uint32_t lane_base = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t t_s = lane_base + g * BS, t_o = lane_base + kSbgColO, t_p = lane_base + kSbgColP + g * (BS / 2);
+    const float cs = p.scale_log2e;
+    const int nv = ctl.nvalid[g];
+    const int32_t* list = lists + g * p.topk;
+    const bool ragged = p.Tk % BS != 0;
+    {
+      uint32_t z[32];                           // P outside the diagonal blocks is zero for good
+#pragma unroll
+      for (int i = 0; i < 32; ++i) z[i] = 0u;
+      tmem_st32(lane_base + kSbgColP, z);
+      tmem_st32(lane_base + kSbgColP + 32, z);
+      tmem_st_wait();
+    }
+    float m_used = 0.f, l = 0.f;
+    float gm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};       // running maxima, raw logits
+    auto row_max = [&]() { return fmaxf(fmaxf(gm[0], gm[1]), fmaxf(gm[2], gm[3])); };
+    auto offset = [&]() {
+      const float m = row_max();
+      return m == -INFINITY ? 0.f : m * cs;
+    };
+    bool ok = true;
+    auto step = [&](int n, int j) -> bool {
+      if (!mbar_wait_warp(&ctl.s_full, n & 1, abort_flag)) return false;
+      tc_fence_after();
+      uint32_t x[BS / 32][32];
+#pragma unroll
+      for (int c = 0; c < BS / 32; ++c) tmem_ld32(t_s + c * 32, x[c]);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.s_free);              // this row's part of S is in registers
+      const int left = j >= nv ? 0 : (ragged ? p.Tk - list[j] : BS);
+      if (left < BS) {                                      // scores that do not exist
+#pragma unroll
+        for (int c = 0; c < BS / 32; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i >= left) x[c][i] = 0xff800000u;  // -inf
+      }
+#pragma unroll
+      for (int c = 0; c < BS / 32; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; i += 2)
+          gm[(i >> 1) & 3] = fmax3(gm[(i >> 1) & 3], __uint_as_float(x[c][i]), __uint_as_float(x[c][i + 1]));
+      if (n == 0) m_used = offset();
+      const float2 nm = make_float2(-m_used, -m_used), cs2 = make_float2(cs, cs);
+      float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      uint32_t pk[BS / 32][16];
+#pragma unroll
+      for (int c = 0; c < BS / 32; ++c) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float2 v = ffma2(make_float2(__uint_as_float(x[c][2 * i]), __uint_as_float(x[c][2 * i + 1])), cs2, nm);
+          if ((i & 3) == 0) {
+            v = exp2_fma2(v);
+          } else {
+            v.x = fast_exp2(v.x);
+            v.y = fast_exp2(v.y);
+          }
+          sum[i & 1] = fadd2(sum[i & 1], v);
+          pk[c][i] = pack_bf16(v.x, v.y);
+        }
+      }
+      // P of the previous step must have been consumed: all of P waits in registers, so that its product has this long
+      if (j > 0 && !mbar_wait_warp(&ctl.pv_done, (n - 1) & 1, abort_flag)) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < BS / 32; ++c) tmem_st16(t_p + c * 16, pk[c]);
+      l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.p_full);
+      return true;
+    };
+    int pass = 0;
+    do {
+      if (pass == 1) {
+        l = 0.f;
+        m_used = offset();
+      }
+#pragma unroll 1
+      for (int j = 0; j < steps && ok; ++j) ok = step(pass * steps + j, j);
+      if (ok) ok = mbar_wait_warp(&ctl.o_full, pass & 1, abort_flag);
+      if (pass == 0 && nv > 0 && !(row_max() * cs <= m_used + 64.f)) ctl.again = 1u;
+    } while (another_pass(pass++));
+
+    if (ok && aligned) {
+      tc_fence_after();
+      const float inv = nv > 0 ? 1.f / l : 0.f;             // no valid key: o = 0, lse = -inf
+      const int b = bh / p.H, h = bh - b * p.H;
+      const bool live = row < p.Tq;
+      if (live && p.lse_s)
+        p.lse_s[static_cast<int64_t>(bh) * p.Tq + row] = nv > 0 ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+      float g0 = 0.f, g1 = 0.f;
+      if (live && p.y) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + row * p.gst);
+        g0 = bf16_lo(w);
+        g1 = bf16_hi(w);
+      }
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t o[32];
+        if (steps > 0) {
+          tmem_ld32(t_o + hf * 32, o);
+          tmem_ld_wait();
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = nv > 0 ? __float_as_uint(__uint_as_float(o[i]) * inv) : 0u;
+        if (!live) continue;
+        auto f = [&](int i) { return __uint_as_float(o[i]); };
+        if (p.o_s) {
+          uint4* dst = reinterpret_cast<uint4*>(p.o_s + (static_cast<int64_t>(bh) * p.Tq + row) * 64 + hf * 32);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            dst[i] = make_uint4(pack_bf16(f(8 * i), f(8 * i + 1)), pack_bf16(f(8 * i + 2), f(8 * i + 3)),
+                                pack_bf16(f(8 * i + 4), f(8 * i + 5)), pack_bf16(f(8 * i + 6), f(8 * i + 7)));
+        }
+        if (p.y) {
+          const uint4* oc = reinterpret_cast<const uint4*>(p.o_c + (static_cast<int64_t>(bh) * p.nqb + qb0 + g) * 64 + hf * 32);
+          uint4* dst = reinterpret_cast<uint4*>(p.y + ((static_cast<int64_t>(b) * p.Tq + row) * p.H + h) * 64 + hf * 32);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint4 c = __ldg(oc + i);
+            const uint32_t cw[4] = {c.x, c.y, c.z, c.w};
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              w[e] = pack_bf16(g0 * bf16_lo(cw[e]) + g1 * f(8 * i + 2 * e), g0 * bf16_hi(cw[e]) + g1 * f(8 * i + 2 * e + 1));
+            dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+    }
+    if ((!ok || !aligned) && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2) tmem_dealloc(tmem, 256);
+}
+
+template <int BS>
+static int launch_sel_big(const void* q, const void* k, const void* v, int kv_chunks, int64_t kv_chunk_stride, const SelParams& p,
+                          cudaStream_t st) {
+  constexpr int G = 128 / BS;
+  const int BH = p.B * p.H;
+  CUtensorMap mq, mk, mv;
+  const uint64_t bh = static_cast<uint64_t>(BH), tq = static_cast<uint64_t>(p.Tq), tc = static_cast<uint64_t>(p.Tc);
+  {
+    const uint64_t dims[4] = {64, tq, bh, 1}, strides[3] = {128, tq * 128, tq * 128 * bh};
+    const uint32_t box[4] = {64, 128, 1, 1};
+    const int rc = make_tensor_map(&mq, q, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+  }
+  {
+    const uint64_t dims[4] = {64, tc, bh, static_cast<uint64_t>(kv_chunks)};
+    const uint64_t strides[3] = {128, tc * 128, kv_chunks > 1 ? static_cast<uint64_t>(kv_chunk_stride) * 2 : tc * 128 * bh};
+    const uint32_t box[4] = {64, static_cast<uint32_t>(BS), 1, 1};
+    int rc = make_tensor_map(&mk, k, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    rc = make_tensor_map(&mv, v, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+  }
+  const int64_t grid = static_cast<int64_t>(BH) * ((p.nqb + G - 1) / G);
+  S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_fwd: grid of %lld CTAs is too large", (long long)grid);
+  const int smem = kSbgOffList + G * p.topk * static_cast<int>(sizeof(int32_t));
+  S3R_CUDA(cudaFuncSetAttribute(sel_big_kernel<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbgOffList + 1024));
+  sel_big_kernel<BS><<<static_cast<unsigned>(grid), kSbgThreads, smem, st>>>(mq, mk, mv, p);
+  S3R_CUDA(cudaGetLastError());
+  return 0;
+}
+
+int sel_big_fwd(const void* q, const void* k, const void* v, int kv_chunks, int64_t kv_chunk_stride, int block, const SelParams& p,
+                cudaStream_t st) {
+  return block == 32 ? launch_sel_big<32>(q, k, v, kv_chunks, kv_chunk_stride, p, st)
+                     : launch_sel_big<64>(q, k, v, kv_chunks, kv_chunk_stride, p, st);
+}
+
+}  // namespace s3r

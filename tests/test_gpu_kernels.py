@@ -284,3 +284,43 @@ def test_cast_bf16_sizes():
                                          (C.c_int64 * n)(*sizes), torch.cuda.current_stream().cuda_stream), "s3r_cast_bf16")
     for x, y in zip(xs, ys):
         assert torch.equal(y, x.bfloat16())
+
+
+# ------------------------------------------------------------------ selection, blocks of 32 and 64
+@pytest.mark.parametrize("block", [32, 64])
+@pytest.mark.parametrize("K", [1, 3, 16, 48, 64])
+def test_sel_big_fwd_lists(block, K):
+    """Row tiles whose lists differ in length (dropped entries), empty lists, a row tile that is not full, a short last
+    block, one entry, and lists too long for two CTAs per SM."""
+    from speed3r_b200 import ops
+    B, H, T = 1, 3, 64 * 7 + 37
+    nb = -(-T // block)
+    q, k, v = bf16_round(randn(90, B, H, T, 64), randn(91, B, H, T, 64), randn(92, B, H, T, 64))
+    idx = table(93, B, H, nb, nb, K)
+    idx[:, :, 2] = -1                                          # a query block without any valid entry
+    idx[:, :, 3, 0] = nb - 1                                   # the short block
+    idx[:, :, 4, K // 2:] = nb + 5                             # half a list dropped
+    idx[:, :, 4, 0] = 1
+    o, lse, _ = ops._sel_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), idx.to(DEV), None, None, block, 0.125, True, True, 1)
+    ref, lse_ref = R.sel_attn(q, k, v, idx, block)
+    rows = torch.ones(T, dtype=torch.bool)
+    rows[2 * block:3 * block] = False
+    assert_bf16_close(o[:, :, rows.to(DEV)], ref[:, :, rows], f"block {block} K {K}")
+    assert_bf16_close(lse[:, :, rows.to(DEV)], lse_ref[:, :, rows], "lse", max_abs=5e-3, mean_abs=1e-3, scale_with_ref=False)
+    assert (o[:, :, ~rows.to(DEV)] == 0).all() and (lse[:, :, ~rows.to(DEV)] == -float("inf")).all()
+
+
+@pytest.mark.parametrize("block", [32, 64])
+def test_sel_big_fwd_second_pass(block):
+    """Scores that outgrow the first key block's by more than 2^64 make a row tile take its keys twice, beside one that does not."""
+    from speed3r_b200 import ops
+    B, H, T, K = 1, 2, 512, 4
+    nb = T // block
+    q, k, v = bf16_round(6 * randn(95, B, H, T, 64), randn(96, B, H, T, 64), randn(97, B, H, T, 64))
+    k, = bf16_round(k * torch.linspace(0.05, 6.0, T).view(1, 1, T, 1))
+    idx = torch.stack([torch.tensor([0, nb // 3, nb // 2, nb - 1])] * nb).int().expand(B, H, nb, K).contiguous()
+    idx[:, :, :128 // block] = torch.tensor([nb - 1, 0, 1, 2]).int()
+    o, lse, _ = ops._sel_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), idx.to(DEV), None, None, block, 0.125, True, True, 1)
+    ref, lse_ref = R.sel_attn(q, k, v, idx, block)
+    assert_bf16_close(o, ref, "growing scores")
+    assert ((lse.cpu() - lse_ref).abs() <= 1e-5 * lse_ref.abs() + 1e-3).all()
