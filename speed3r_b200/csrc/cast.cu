@@ -17,6 +17,8 @@ struct CastParams {
 };
 
 __global__ void __launch_bounds__(256) cast_bf16_kernel(const __grid_constant__ CastParams p) {
+  griddep_wait();
+  griddep_launch();
   int i = 0;
   while (i + 1 < p.n && static_cast<int>(blockIdx.x) >= p.first_block[i + 1]) ++i;
   const float* src = p.src[i];
@@ -66,7 +68,5 @@ extern "C" int s3r_cast_bf16(int n, const float* const* src, void* const* dst, c
     S3R_REQUIRE(blocks < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cast_bf16: grid too large");
   }
   p.first_block[n] = static_cast<int>(blocks);
-  cast_bf16_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(cast_bf16_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream), p);
 }

@@ -112,6 +112,8 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_wait();
+  griddep_launch();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
@@ -348,7 +350,7 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
     // epilogue: the bound (32nd largest of the row's 64 maxima: with both threads' 32 sorted, the larger of a[i] and
     // b[31 - i] over all i are the upper 32), lse and O / l.  The K ring is free by now.
-    sort32_desc(gm);
+    sort_desc<32>(gm);
     float* other = reinterpret_cast<float*>(smem_raw + (sbase - smem_u32(smem_raw)) + C::kOffK) + t * (32 * 128) + r;     // [slot][row]
     if (half == 1) {
 #pragma unroll
@@ -394,9 +396,7 @@ static int launch_cmp_attn(const CmpMaps& m, const AtParams& p, int BH, cudaStre
   const int64_t grid = static_cast<int64_t>(BH) * ((p.Nq + R * 128 - 1) / (R * 128));
   S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
   S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
-  cmp_attn_kernel<R><<<static_cast<unsigned>(grid), C::kThreads, C::kSmem, st>>>(m.q, m.k, m.v, p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(cmp_attn_kernel<R>, static_cast<unsigned>(grid), C::kThreads, C::kSmem, st, m.q, m.k, m.v, p);
 }
 
 int cmp_attn_fwd(const CmpMaps& m, void* o_c, float* lse, float* bound, int64_t bound_stride, int BH, int Nq, int Nc, float scale,

@@ -99,6 +99,8 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_wait();
+  griddep_launch();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
@@ -440,12 +442,11 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
   const int64_t g0 = static_cast<int64_t>(BH) * ((Nc + kCbOwnRows - 1) / kCbOwnRows),
                 g1 = static_cast<int64_t>(BH) * ((Nq + kCbOwnRows - 1) / kCbOwnRows);
   S3R_REQUIRE(g0 < (1ll << 31) && g1 < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_bwd: grid too large");
-  cmp_bwd_kernel<0><<<static_cast<unsigned>(g0), kCbThreads, kCbSmemBytes, st>>>(mk128, mv128, mq64, mdo64, p);
+  rc = launch(cmp_bwd_kernel<0>, static_cast<unsigned>(g0), kCbThreads, kCbSmemBytes, st, mk128, mv128, mq64, mdo64, p);
+  if (rc) return rc;
   // dQ: own = Q, dO (Nq rows), streamed = K, V (Nc rows)
   p.out0 = nullptr;
   p.out1 = static_cast<__nv_bfloat16*>(dq_c);
   p.n_own = Nq; p.n_str = Nc;
-  cmp_bwd_kernel<1><<<static_cast<unsigned>(g1), kCbThreads, kCbSmemBytes, st>>>(mq128, mdo128, mk64, mv64, p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(cmp_bwd_kernel<1>, static_cast<unsigned>(g1), kCbThreads, kCbSmemBytes, st, mq128, mdo128, mk64, mv64, p);
 }

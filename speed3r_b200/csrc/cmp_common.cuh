@@ -24,22 +24,27 @@ __device__ __forceinline__ float key_to_float(uint32_t key) {
   return __uint_as_float(b);
 }
 
-// Descending bitonic sort of 32 values in registers.
-__device__ __forceinline__ void sort32_desc(float (&v)[32]) {
+template <typename T>
+__device__ __forceinline__ void order_desc(T& a, T& b) {           // larger first
+  const T x = a < b ? b : a, y = a < b ? a : b;
+  a = x;
+  b = y;
+}
+__device__ __forceinline__ void order_desc(float& a, float& b) {
+  const float x = fmaxf(a, b), y = fminf(a, b);
+  a = x;
+  b = y;
+}
+// Descending sort in registers: Batcher's odd-even merge sort (191 exchanges for 32).
+template <int N, typename T>
+__device__ __forceinline__ void sort_desc(T (&v)[N]) {
 #pragma unroll
-  for (int k = 2; k <= 32; k <<= 1)
+  for (int p = 1; p < N; p <<= 1)
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1)
+    for (int k = p; k > 0; k >>= 1)
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int l = i ^ j;
-        if (l > i) {
-          const float hi = fmaxf(v[i], v[l]), lo = fminf(v[i], v[l]);
-          const bool desc = (i & k) == 0;
-          v[i] = desc ? hi : lo;
-          v[l] = desc ? lo : hi;
-        }
-      }
+      for (int i = 0; i < N - k; ++i)
+        if (i >= k % p && ((i - k % p) / k) % 2 == 0 && i / (2 * p) == (i + k) / (2 * p)) order_desc(v[i], v[i + k]);
 }
 #endif
 

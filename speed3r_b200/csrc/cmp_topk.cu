@@ -7,7 +7,10 @@
 // bank.  A row has two threads (in two warpgroups that take turns at its key tiles) and a list for each.  A list that
 // fills up (structured scores can leave a loose bound; equal scores all reach it) is cut back to its best 32 there and
 // then, and goes on with the 32nd of those as its bound.  At the end every thread sorts its list in registers, and one of
-// the two merges them.
+// the two merges them.  What is sorted is one 32-bit word per pair - the logit's key above the bound's, cut to 25 bits where it
+// needs more, and the pair's place - with a minimum and a maximum per exchange (sorting (key, column) as 64-bit words: 12 us
+// per CTA, most of the kernel up to 384 keys and 15 % of it at 6300); rows in which two of the words' keys are equal are
+// sorted again with the columns.
 //
 // Bound: instructions and their latency in the scan: a max tree and a vote per 16 columns of a warp, and for the chunks
 // with a hit (three in four at 250 views, one in three at 1000) a mask and a store.  The products take half of the time
@@ -97,31 +100,39 @@ __device__ __noinline__ void tk_append_checked(const TkChunk ch, uint2* buf, uin
   }
 }
 
-// Descending bitonic sort in registers.
-__device__ __forceinline__ void tk_cmp(uint64_t& a, uint64_t& b, bool desc) {
-  const bool swap = desc ? a < b : b < a;
-  const uint64_t x = swap ? b : a, y = swap ? a : b;
-  a = x;
-  b = y;
-}
-template <int N>
-__device__ __forceinline__ void tk_sort(uint64_t (&v)[N]) {
-#pragma unroll
-  for (int k = 2; k <= N; k <<= 1)
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1)
-#pragma unroll
-      for (int i = 0; i < N; ++i)
-        if ((i ^ j) > i) tk_cmp(v[i], v[i ^ j], (i & k) == 0);
-}
 // A bitonic sequence (what a[i] = max(a[i], b[31 - i]) of two descending lists leaves: the best 32 of both), sorted.
-__device__ __forceinline__ void tk_merge(uint64_t (&v)[32]) {
+template <typename T>
+__device__ __forceinline__ void tk_merge(T (&v)[32]) {
 #pragma unroll
   for (int j = 16; j > 0; j >>= 1)
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if ((i ^ j) > i) tk_cmp(v[i], v[i ^ j], true);
+      if ((i ^ j) > i) order_desc(v[i], v[i ^ j]);
 }
+// The best 32 of a row's two lists with ties in column order: columns to out[i * 128], ~0 for an empty place.
+__device__ __noinline__ void tk_exact(const uint2* la, int na, const uint2* lb, int nb, uint32_t* out) {
+  uint64_t a[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) a[i] = i < na ? tk_entry(la[i * 32]) : 0ull;
+  sort_desc<32>(a);
+#pragma unroll 1
+  for (int part = 0; part < 6; ++part) {       // the rest in pieces of eight: 32.. of the first list, all of the second
+    uint64_t e[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int s = part == 0 ? 32 + i : (part - 1) * 8 + i;
+      const bool in = part == 0 ? s < na : s < nb;
+      e[i] = in ? tk_entry((part == 0 ? la : lb)[s * 32]) : 0ull;
+    }
+    sort_desc<8>(e);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[31 - i] = a[31 - i] < e[i] ? e[i] : a[31 - i];
+    tk_merge(a);
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) out[i * 128] = a[i] >> 32 ? ~static_cast<uint32_t>(a[i]) : ~0u;
+}
+static_assert(kTkCap == 40, "tk_exact takes lists of up to 40, the packed words a place below 80");
 
 __global__ void __launch_bounds__(kTkThreads, 1)
 cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const TkParams p) {
@@ -156,6 +167,8 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_wait();
+  griddep_launch();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
@@ -228,8 +241,10 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     int32_t* out = p.idx + (static_cast<int64_t>(bh) * p.Nq + row) * p.topk;
     // `score > thr` for every score that reaches the bound (NaN and -inf never do); rows past the end collect nothing
     float thr = INFINITY;
+    uint32_t base_key = 0;                       // every collected pair's key is at least this
     if (row < p.Nq) {
       const float bound = fmaxf(__int_as_float(*out), -3.402823466e38f);
+      base_key = sortable_key(bound == 0.f ? -0.f : bound);
       thr = bound == 0.f ? __uint_as_float(0x80000001u) : key_to_float(sortable_key(bound) - 1u);
     }
     const uint32_t first = smem_u32(buf), end = first + kTkCap * 256;
@@ -315,44 +330,88 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
 
     const int cnt = static_cast<int>(at - first) >> 8;
-    // each list sorted by its own thread, then the two lists of a row merged by one of them
-    uint64_t a[32];
+    const int r = quarter * 32 + lane;
+    // Q and the K ring are idle once every scan warp is here (whatever happened): per row tile 32 words per row for sorted
+    // words and columns, and two per row for what its threads tell each other
+    asm volatile("bar.sync 3, 512;" ::: "memory");
+    uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (sbase - smem_u32(smem_raw))) + t * (35 * 128) + r;   // [place][row]
+    uint32_t* tell = words + 32 * 128;         // [list][row] largest key, [2][row] the second list's length
+    auto meet = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory"); };
+    uint32_t a[32], e[kTkCap - 32];
+    uint32_t top = 0;
+    // keys above the bound's, plus one: an empty place is 0
+    auto word = [&](int i) {
+      const uint32_t d = i < cnt ? sortable_key(__uint_as_float(buf[i * 32].x)) - base_key + 1u : 0u;
+      top = max(top, d);
+      return d;
+    };
 #pragma unroll
-    for (int i = 0; i < 32; ++i) a[i] = i < cnt ? tk_entry(buf[i * 32]) : 0ull;
-    tk_sort<32>(a);
+    for (int i = 0; i < 32; ++i) a[i] = word(i);
+#pragma unroll
+    for (int i = 0; i < kTkCap - 32; ++i) e[i] = word(32 + i);
+    tell[par * 128] = top;
+    if (par == 1) tell[2 * 128] = static_cast<uint32_t>(cnt);
+    meet();
+    top = max(top, tell[(par ^ 1) * 128]);
+    const int shift = max(0, 7 - __clz(top | 1u));        // bits of the keys beyond 25
+    auto pack = [&](uint32_t& d, int i) { d = d ? ((d >> shift) << 7) | static_cast<uint32_t>(127 - par * kTkCap - i) : 0u; };
+#pragma unroll
+    for (int i = 0; i < 32; ++i) pack(a[i], i);
+    sort_desc<32>(a);
+    uint32_t lost = 0;                         // the largest word that is not among the row's 32
     if (__any_sync(0xffffffffu, cnt > 32)) {
-      uint64_t e[kTkCap - 32];
 #pragma unroll
-      for (int i = 0; i < kTkCap - 32; ++i) e[i] = 32 + i < cnt ? tk_entry(buf[(32 + i) * 32]) : 0ull;
-      tk_sort<kTkCap - 32>(e);
+      for (int i = 0; i < kTkCap - 32; ++i) pack(e[i], 32 + i);
+      sort_desc<kTkCap - 32>(e);
 #pragma unroll
-      for (int i = 0; i < kTkCap - 32; ++i) a[31 - i] = a[31 - i] < e[i] ? e[i] : a[31 - i];
+      for (int i = 0; i < kTkCap - 32; ++i) {
+        lost = max(lost, min(a[31 - i], e[i]));
+        a[31 - i] = max(a[31 - i], e[i]);
+      }
       tk_merge(a);
     }
     if (par == 1) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) buf[i * 32] = make_uint2(static_cast<uint32_t>(a[i] >> 32), static_cast<uint32_t>(a[i]));
+      for (int i = 0; i < 32; ++i) words[i * 128] = a[i];
+      tell[1 * 128] = lost;
     }
-    asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory");      // every scan warp of the row tile comes here, whatever happened
-    if (ok && par == 0 && row < p.Nq) {
-      const uint2* other = buf + 4 * (kTkCap * 32);
+    meet();
+    if (par == 0) {
+      lost = max(lost, tell[1 * 128]);
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const uint2 w = other[(31 - i) * 32];
-        const uint64_t e = (static_cast<uint64_t>(w.x) << 32) | w.y;
-        a[i] = a[i] < e ? e : a[i];
+        const uint32_t o = words[(31 - i) * 128];
+        lost = max(lost, min(a[i], o));
+        a[i] = max(a[i], o);
       }
       tk_merge(a);
-      // an empty slot decodes to column Nc-1, the reference's padding
-      auto column = [&](int i) { return a[i] >> 32 ? static_cast<int32_t>(~static_cast<uint32_t>(a[i])) : p.Nc - 1; };
-      if (p.vec) {
+      bool equal = lost != 0u && lost >> 7 >= a[31] >> 7;
 #pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          if (i < p.topk) *reinterpret_cast<int4*>(out + i) = make_int4(column(i), column(i + 1), column(i + 2), column(i + 3));
+      for (int i = 0; i < 31; ++i) equal |= a[i + 1] != 0u && a[i] >> 7 == a[i + 1] >> 7;
+      const uint2* other = buf + 4 * (kTkCap * 32);
+      if (__any_sync(0xffffffffu, equal)) {
+        tk_exact(buf, cnt, other, static_cast<int>(tell[2 * 128]), words);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) a[i] = words[i * 128];
       } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (i < p.topk) out[i] = column(i);
+        for (int i = 0; i < 32; ++i) {
+          const int place = 127 - static_cast<int>(a[i] & 127u);
+          a[i] = a[i] ? (place < kTkCap ? buf[place * 32].y : other[(place - kTkCap) * 32].y) : ~0u;
+        }
+      }
+      if (ok && row < p.Nq) {
+        // an empty place decodes to column Nc-1, the reference's padding
+        auto column = [&](int i) { return a[i] != ~0u ? static_cast<int32_t>(a[i]) : p.Nc - 1; };
+        if (p.vec) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            if (i < p.topk) *reinterpret_cast<int4*>(out + i) = make_int4(column(i), column(i + 1), column(i + 2), column(i + 3));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (i < p.topk) out[i] = column(i);
+        }
       }
     }
     if (!ok && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
@@ -372,9 +431,7 @@ int cmp_topk_fwd(const CmpMaps& m, int32_t* idx, int topk, int BH, int Nq, int N
   const int64_t grid = static_cast<int64_t>(BH) * ((Nq + kTkRows - 1) / kTkRows);
   S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
   S3R_CUDA(cudaFuncSetAttribute(cmp_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
-  cmp_topk_kernel<<<static_cast<unsigned>(grid), kTkThreads, kTkSmem, st>>>(m.q, m.k, p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(cmp_topk_kernel, static_cast<unsigned>(grid), kTkThreads, kTkSmem, st, m.q, m.k, p);
 }
 
 }  // namespace s3r

@@ -49,6 +49,29 @@ int make_pair_map(CUtensorMap* out, const void* a, const void* b, int T, int BH,
 int sm_count();
 
 #ifdef __CUDACC__
+// Launch of a kernel whose CTAs may start while the kernel before it in the stream is still finishing (programmatic
+// stream serialisation).  Every thread of such a kernel calls griddep_wait() before its first access to global memory;
+// what comes before - barriers, tensor memory, index arithmetic - then overlaps the other kernel's last CTAs.  On a short
+// sequence a call is a chain of kernels of 3 to 25 us, whose starts and ends are a good part of it.
+template <typename... P, typename... A>
+inline int launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(static_cast<unsigned>(threads));
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = a;
+  c.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...), "kernel launch");
+}
+// All of the kernels before this one have completed and what they wrote is visible.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel's CTAs may start where there is room (they wait for this kernel's end themselves).
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------------------------

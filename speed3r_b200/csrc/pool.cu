@@ -63,6 +63,8 @@ __device__ __forceinline__ void pool_tensor(const PoolTensor& p, int B, int H, i
   }
 }
 __global__ void __launch_bounds__(256) pool_fwd_kernel(const PoolParams p) {
+  griddep_wait();
+  griddep_launch();
   const PoolTensor& t = p.t[blockIdx.y];
   if (t.kernel == 16) pool_tensor<16>(t, p.B, p.H, p.d);
   else pool_tensor<0>(t, p.B, p.H, p.d);
@@ -149,9 +151,7 @@ extern "C" int s3r_pool_multi_fwd(int n, const void* const* in, const int64_t* s
     const int64_t total = static_cast<int64_t>(B) * t.Nc * H * (d / 8);
     most = total > most ? total : most;
   }
-  pool_fwd_kernel<<<dim3(pool_grid(most), n), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(pool_fwd_kernel, dim3(pool_grid(most), n), 256, 0, static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" int s3r_pool_fwd(const void* in, int64_t stride_b, int64_t stride_h, int64_t stride_t, void* out, int B,

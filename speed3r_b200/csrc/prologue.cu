@@ -91,6 +91,8 @@ __device__ __forceinline__ void rope_row(uint32_t (&xw)[4], const __nv_bfloat16*
 template <int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads, kMaxThreads <= 384 ? 2 : 1)
 prologue_fwd_kernel(const PrologueParams p) {
+  griddep_wait();
+  griddep_launch();
   const int l8 = threadIdx.x & 7;
   const int g = threadIdx.x >> 3;                  // row of the token: (q|k|v, head)
   const uint32_t gmask = 0xffu << (threadIdx.x & 24);
@@ -251,6 +253,8 @@ __device__ __forceinline__ void ln_row_bwd(const float (&x)[8], float (&dy)[8], 
 template <int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads, kMaxThreads <= 384 ? 2 : 1) prologue_bwd_kernel(const PrologueBwdParams p) {
   extern __shared__ float red[];                   // [2H rows][weight|bias][64]
+  griddep_wait();
+  griddep_launch();
   const int l8 = threadIdx.x & 7, g = threadIdx.x >> 3;
   const uint32_t gmask = 0xffu << (threadIdx.x & 24);
   const int which = g / p.H, h = g - which * p.H;
@@ -359,6 +363,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMaxThreads <= 384 ? 2 : 1) prolo
 
 // out[o] = sum over CTAs of partial[cta][o]; a warp per output
 __global__ void __launch_bounds__(256) prologue_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ out, int ctas) {
+  griddep_wait();
+  griddep_launch();
   const int o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   float s = 0.f;
   for (int c = lane; c < ctas; c += 32) s += partial[c * 256 + o];
@@ -414,12 +420,8 @@ extern "C" int s3r_qkv_prologue_fwd(const void* qkv, const int64_t* pos, const v
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_qkv_prologue_fwd: could not resolve the device status word");
-  if (3 * H * 8 <= 384)
-    prologue_fwd_kernel<384><<<static_cast<unsigned>(grid), 3 * H * 8, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  else
-    prologue_fwd_kernel<1024><<<static_cast<unsigned>(grid), 3 * H * 8, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(3 * H * 8 <= 384 ? prologue_fwd_kernel<384> : prologue_fwd_kernel<1024>, static_cast<unsigned>(grid), 3 * H * 8, 0,
+                static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" size_t s3r_qkv_prologue_bwd_workspace_bytes(int B, int N, int block) {
@@ -466,9 +468,8 @@ extern "C" int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const v
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
   const int ctas = prologue_bwd_ctas(B, Nc), smem = 2 * H * 128 * static_cast<int>(sizeof(float));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (3 * H * 8 <= 384) prologue_bwd_kernel<384><<<ctas, 3 * H * 8, smem, st>>>(p);
-  else prologue_bwd_kernel<1024><<<ctas, 3 * H * 8, smem, st>>>(p);
-  if (dparams) prologue_bwd_reduce_kernel<<<32, 256, 0, st>>>(p.partial, dparams, ctas);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  const int rc = launch(3 * H * 8 <= 384 ? prologue_bwd_kernel<384> : prologue_bwd_kernel<1024>, static_cast<unsigned>(ctas),
+                        3 * H * 8, smem, st, p);
+  if (rc || !dparams) return rc;
+  return launch(prologue_bwd_reduce_kernel, 32, 256, 0, st, p.partial, dparams, ctas);
 }

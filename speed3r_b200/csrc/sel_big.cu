@@ -70,6 +70,8 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     tmem_alloc(&ctl.tmem_base, 256);
     tmem_relinquish();
   }
+  griddep_wait();
+  griddep_launch();
   if (warp >= 4 && warp < 4 + G) {
     // valid entries of one query block's row of the table, table order
     const int g = warp - 4, qb = qb0 + g;
@@ -374,9 +376,7 @@ static int launch_sel_big(const void* q, const void* k, const void* v, int kv_ch
   S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_fwd: grid of %lld CTAs is too large", (long long)grid);
   const int smem = kSbgOffList + G * p.topk * static_cast<int>(sizeof(int32_t));
   S3R_CUDA(cudaFuncSetAttribute(sel_big_kernel<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbgOffList + 1024));
-  sel_big_kernel<BS><<<static_cast<unsigned>(grid), kSbgThreads, smem, st>>>(mq, mk, mv, p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(sel_big_kernel<BS>, static_cast<unsigned>(grid), kSbgThreads, smem, st, mq, mk, mv, p);
 }
 
 int sel_big_fwd(const void* q, const void* k, const void* v, int kv_chunks, int64_t kv_chunk_stride, int block, const SelParams& p,

@@ -226,6 +226,8 @@ constexpr int kCsrOneEntries = 24576, kCsrOneKeys = 8192;
 __global__ void __launch_bounds__(1024) csr_one_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ offsets,
                                                        int32_t* __restrict__ qids, int per_bh, int Nkb, int topk) {
   extern __shared__ int32_t one_smem[];
+  griddep_wait();
+  griddep_launch();
   int32_t* cur = one_smem;                   // counts, then the fill's cursors (= end of each segment afterwards)
   int32_t* ent = one_smem + Nkb;             // query blocks by segment, arrival order
   __shared__ int32_t warp_sums[32];
@@ -302,6 +304,8 @@ __global__ void __launch_bounds__(1024) csr_one_kernel(const int32_t* __restrict
 __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ o,
                                                     const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,
                                                     int64_t rows) {
+  griddep_wait();
+  griddep_launch();
   const int64_t gid = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   const int64_t row = gid >> 3;
   const int c8 = threadIdx.x & 7;
@@ -336,6 +340,8 @@ struct MergeBwdParams {
 };
 
 __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) {
+  griddep_wait();
+  griddep_launch();
   const int lane = threadIdx.x & 31;
   const int64_t wid = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   if (wid >= static_cast<int64_t>(p.B) * p.H * p.nqb) return;
@@ -538,6 +544,8 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_dq_kernel(const __grid_constan
     mbar_init(&full[1], 1);
     mbar_fence_init();
   }
+  griddep_wait();
+  griddep_launch();
   int nvalid = 0;
   {
     const int32_t* row = p.idx + (static_cast<int64_t>(bh) * p.nqb + (row0 >> (4 + p.block_shift))) * p.topk;
@@ -655,6 +663,8 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_dkdv_kernel(const __grid_const
     mbar_init(&full[1], 1);
     mbar_fence_init();
   }
+  griddep_wait();
+  griddep_launch();
   __syncwarp();
   const int n = row0 >> (4 + p.block_shift);
   const int32_t* off = p.offsets + static_cast<int64_t>(bh) * (p.nkb + 1) + n;
@@ -817,9 +827,7 @@ extern "C" int s3r_build_key_csr(const int32_t* idx, int32_t* offsets, int32_t* 
     const int smem = (Nkb + static_cast<int>(per_bh)) * static_cast<int>(sizeof(int32_t));
     S3R_CUDA(cudaFuncSetAttribute(csr_one_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (kCsrOneEntries + kCsrOneKeys) * static_cast<int>(sizeof(int32_t))));
-    csr_one_kernel<<<static_cast<unsigned>(bh), 1024, smem, st>>>(idx, offsets, qids, static_cast<int>(per_bh), Nkb, topk);
-    S3R_CUDA(cudaGetLastError());
-    return 0;
+    return launch(csr_one_kernel, static_cast<unsigned>(bh), 1024, smem, st, idx, offsets, qids, static_cast<int>(per_bh), Nkb, topk);
   }
   int32_t* queue = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(tmp) +
                                               ((bh * Nq * topk * sizeof(int32_t) + 255) & ~static_cast<size_t>(255)));
@@ -887,10 +895,8 @@ extern "C" int s3r_delta(const void* o, const void* d_o, float* delta, int64_t r
   S3R_REQUIRE(rows > 0, S3R_ERR_SHAPE, "s3r_delta: rows must be positive");
   S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_delta: head_dim %d not supported (64 only)", d);
   const int64_t blocks = (rows * 8 + 255) / 256;
-  delta_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, rows);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(delta_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
+                static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, rows);
 }
 
 extern "C" int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
@@ -912,9 +918,7 @@ extern "C" int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stri
   p.B = B; p.H = H; p.Tq = Tq; p.block = block;
   p.nqb = (Tq + block - 1) / block;
   const int64_t warps = static_cast<int64_t>(B) * H * p.nqb;
-  merge_bwd_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(merge_bwd_kernel, static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), p);
 }
 
 static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
@@ -944,10 +948,9 @@ static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
   if (rc) return rc;
   S3R_CUDA(cudaFuncSetAttribute(sel_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
   S3R_CUDA(cudaFuncSetAttribute(sel_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
-  sel_bwd_dkdv_kernel<<<static_cast<unsigned>(tk), 32, kSbSmem, st>>>(mqdo, p);
-  sel_bwd_dq_kernel<<<static_cast<unsigned>(tq), 32, kSbSmem, st>>>(mkv, p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  rc = launch(sel_bwd_dkdv_kernel, static_cast<unsigned>(tk), 32, kSbSmem, st, mqdo, p);
+  if (rc) return rc;
+  return launch(sel_bwd_dq_kernel, static_cast<unsigned>(tq), 32, kSbSmem, st, mkv, p);
 }
 
 extern "C" int s3r_sel_attn_bwd(const void* q, const void* k, const void* v, const int32_t* idx,

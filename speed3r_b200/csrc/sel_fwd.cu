@@ -61,6 +61,8 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
     mbar_init(&full[1], 1);
     mbar_fence_init();
   }
+  griddep_wait();
+  griddep_launch();
 
   int nvalid = 0;
   {
@@ -280,9 +282,7 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
 static int launch_sel16_fwd(const CUtensorMap& mkv, const Sel16Params& p, int64_t ntasks, cudaStream_t st) {
   S3R_REQUIRE(ntasks < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_fwd: grid of %lld CTAs is too large", (long long)ntasks);
   S3R_CUDA(cudaFuncSetAttribute(sel16_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSel16Smem));
-  sel16_fwd_kernel<<<static_cast<unsigned>(ntasks), 32, kSel16Smem, st>>>(mkv, p);
-  S3R_CUDA(cudaGetLastError());
-  return 0;
+  return launch(sel16_fwd_kernel, static_cast<unsigned>(ntasks), 32, kSel16Smem, st, mkv, p);
 }
 
 }  // namespace s3r
