@@ -95,17 +95,34 @@ int s3r_qkv_prologue_fwd(const void* qkv, const int64_t* pos, const void* cos_ta
                          const float* k_bias, float eps, void* q, void* k, void* v, void* q_c, void* k_c,
                          void* v_c, int B, int H, int N, int d, int block, void* stream);
 
+/* The same on a projection that carries the gate's logits as well (one GEMM for qkv and gate):
+ *   proj : [B,N,3*H*d + 2*H] bf16, a token's q, k, v as above and then its logits (h, 2)
+ *   gate : [B,H,N,2] bf16 out = sigmoid of the logits, computed in fp32 and rounded once
+ * H must be a multiple of 4 (16-byte rows). */
+int s3r_qkv_gate_prologue_fwd(const void* proj, const int64_t* pos, const void* cos_tab, const void* sin_tab,
+                              int tab_rows, const float* q_weight, const float* q_bias, const float* k_weight,
+                              const float* k_bias, float eps, void* q, void* k, void* v, void* q_c, void* k_c,
+                              void* v_c, void* gate, int B, int H, int N, int d, int block, void* stream);
+
 /* Backward of s3r_qkv_prologue_fwd (autograd of the same lines): from the gradients of its six outputs the gradient of the
  * packed projection and of the LayerNorm parameters.
  *   dq,dk,dv [B,H,N,d], dq_c,dk_c,dv_c [B,H,N/block,d] bf16;  dqkv [B,N,3,H,d] bf16, overwritten
  *   q_weight, k_weight as in the forward; dparams [4,64] fp32 = dq_weight, dq_bias, dk_weight, dk_bias (NULL without norms)
  *   workspace: s3r_qkv_prologue_bwd_workspace_bytes(...) bytes (unused without norms); need not be initialised.
  * Positions outside the tables are clamped as in the forward, which has reported them.  Deterministic. */
-size_t s3r_qkv_prologue_bwd_workspace_bytes(int B, int N, int block);
+size_t s3r_qkv_prologue_bwd_workspace_bytes(int B, int H, int N, int block);
 int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const void* cos_tab, const void* sin_tab, int tab_rows,
                          const float* q_weight, const float* k_weight, float eps, const void* dq, const void* dk,
                          const void* dv, const void* dq_c, const void* dk_c, const void* dv_c, void* dqkv, float* dparams,
                          void* workspace, size_t workspace_bytes, int B, int H, int N, int d, int block, void* stream);
+
+/* Backward of s3r_qkv_gate_prologue_fwd: dproj [B,N,3*H*d + 2*H] also gets the gradient of the gate's logits,
+ * dgate * gate * (1 - gate), from gate [B,H,N,2] bf16 and dgate [B,H,N,2] fp32 (what s3r_merge_bwd writes). */
+int s3r_qkv_gate_prologue_bwd(const void* proj, const int64_t* pos, const void* cos_tab, const void* sin_tab, int tab_rows,
+                              const float* q_weight, const float* k_weight, float eps, const void* dq, const void* dk,
+                              const void* dv, const void* dq_c, const void* dk_c, const void* dv_c, const void* gate,
+                              const float* dgate, void* dproj, float* dparams, void* workspace, size_t workspace_bytes, int B,
+                              int H, int N, int d, int block, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Compression attention with fused top-k block selection.

@@ -24,8 +24,10 @@ SIGNATURES = {
     "s3r_pool_multi_fwd": (_i, [_i, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "s3r_pool_bwd": (_i, [_p, _p, _i64, _i64, _i64, _i, _i, _i, _i, _i, _i, _i, _p]),
     "s3r_qkv_prologue_fwd": (_i, [_p, _p, _p, _p, _i, _p, _p, _p, _p, _f, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p]),
-    "s3r_qkv_prologue_bwd_workspace_bytes": (_sz, [_i, _i, _i]),
+    "s3r_qkv_gate_prologue_fwd": (_i, [_p, _p, _p, _p, _i, _p, _p, _p, _p, _f] + [_p] * 7 + [_i, _i, _i, _i, _i, _p]),
+    "s3r_qkv_prologue_bwd_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "s3r_qkv_prologue_bwd": (_i, [_p, _p, _p, _p, _i, _p, _p, _f] + [_p] * 9 + [_sz, _i, _i, _i, _i, _i, _p]),
+    "s3r_qkv_gate_prologue_bwd": (_i, [_p, _p, _p, _p, _i, _p, _p, _f] + [_p] * 11 + [_sz, _i, _i, _i, _i, _i, _p]),
     "s3r_cmp_attn_topk_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_cmp_attn_blocktopk_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p]),
     "s3r_cmp_attn_bwd": (_i, [_p] * 10 + [_i, _i, _i, _i, _i, _f, _p]),

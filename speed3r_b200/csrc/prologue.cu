@@ -7,7 +7,7 @@
 // (6 KB per token, contiguous) and each output written once, so the kernel is bounded by HBM:
 // 2 * 3*N*H*d*2 bytes plus the pooled tensors.
 //
-// One CTA owns one block of `block` tokens of one batch element; eight lanes own one (q|k|v, head) row
+// A CTA works on one block of `block` tokens of one batch element; eight lanes own one (q|k|v, head) row
 // of 64 channels (16 bytes per lane) and walk the block's tokens, so a block's mean never leaves
 // registers.  Rounding points follow the reference under bf16 autocast: LayerNorm in fp32 from bf16
 // input, rounded to bf16; the rotary products and their sum each rounded to bf16; the block mean
@@ -18,7 +18,10 @@
 namespace s3r {
 
 struct PrologueParams {
-  const __nv_bfloat16* qkv;          // [B,N,3,H,64]
+  const __nv_bfloat16* qkv;          // [B,N,(3,H,64)], tokens tok_stride elements apart
+  int64_t tok_stride;
+  const __nv_bfloat16* gate_in;      // logits (h,2) of a token, tokens tok_stride apart; null: none
+  uint32_t* gate;                    // [B,H,N] pairs: their sigmoid
   const int64_t* pos;                // [B,N,2] (y,x) or null: no rotary embedding
   const __nv_bfloat16* cos_tab;      // [tab_rows,32]
   const __nv_bfloat16* sin_tab;
@@ -37,27 +40,77 @@ struct alignas(16) Vec8 {
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
+__device__ __forceinline__ float sum8(float x, uint32_t gmask) {
+  x += __shfl_xor_sync(gmask, x, 1);
+  x += __shfl_xor_sync(gmask, x, 2);
+  return x + __shfl_xor_sync(gmask, x, 4);
+}
+__device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return ffma2(a, b, splat(-0.f)); }
+__device__ __forceinline__ void unpack8(float2 (&x)[4], const Vec8& v) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = make_float2(bf16_lo(v.w[i]), bf16_hi(v.w[i]));
+}
+__device__ __forceinline__ Vec8 pack8(const float2 (&x)[4]) {
+  Vec8 v;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v.w[i] = pack_bf16(x[i].x, x[i].y);
+  return v;
+}
+__device__ __forceinline__ Vec8 ldg_vec8(const __nv_bfloat16* p) {
+  const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+  return Vec8{{v.x, v.y, v.z, v.w}};
+}
+// Rows of the rotary tables for a block's tokens and, behind them, for its mean position: (y, x) pairs in this warp's shared
+// memory, clamped and checked once per warp instead of once per (q|k, head) row of every token.
+__device__ __forceinline__ void block_rows(int* r, const int64_t* pos, int block, int tab_rows, uint32_t* status, int lane) {
+  bool bad = false;
+  auto put = [&](int i, int64_t pv) {
+    const int row = static_cast<int>(min(max(pv, static_cast<int64_t>(0)), static_cast<int64_t>(tab_rows - 1)));
+    bad |= pv != row;
+    r[i] = row;
+  };
+  float sum = 0.f;                                    // of the coordinate lane % 2: whole numbers, any order is exact
+  for (int i = lane; i < 2 * block; i += 32) {
+    const int64_t pv = __ldg(pos + i);
+    put(i, pv);
+    sum += static_cast<float>(pv);
+  }
+#pragma unroll
+  for (int d = 2; d < 32; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+  // float mean, truncated: xpos.view(..).float().mean(dim=2).int()
+  if (lane < 2) put(2 * block + lane, static_cast<int64_t>(static_cast<int>(sum / static_cast<float>(block))));
+  if (bad && status) atomicOr(status, kStatusBadIndex);     // clamped: the result for this token is wrong
+  __syncwarp();
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ Vec8 lds_vec8(uint32_t a) {
+  const uint4 v = lds128(a);
+  return Vec8{{v.x, v.y, v.z, v.w}};
+}
+
 // LayerNorm over the 64 channels held by 8 lanes (8 each), fp32, two passes; the caller rounds to bf16.
 // `gmask` names the 8 lanes of the row: rows of one warp may belong to different tensors (q, k or v) and
 // take different paths, so every shuffle synchronises its own group only.
-__device__ __forceinline__ void ln_row(float (&x)[8], const float (&w)[8], const float (&b)[8], float eps,
-                                       uint32_t gmask) {
-  float s = 0.f;
+__device__ __forceinline__ void ln_row(float2 (&x)[4], const float2 (&w)[4], const float2 (&b)[4], float eps, uint32_t gmask) {
+  const float2 s = fadd2(fadd2(x[0], x[1]), fadd2(x[2], x[3]));
+  const float mean = sum8(s.x + s.y, gmask) * (1.f / 64.f);
+  float2 v = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) s += x[i];
-  s += __shfl_xor_sync(gmask, s, 1);
-  s += __shfl_xor_sync(gmask, s, 2);
-  s += __shfl_xor_sync(gmask, s, 4);
-  const float mean = s * (1.f / 64.f);
-  float v = 0.f;
+  for (int i = 0; i < 4; ++i) {
+    x[i] = fadd2(x[i], splat(-mean));
+    v = ffma2(x[i], x[i], v);
+  }
+  const float rstd = rsqrtf(sum8(v.x + v.y, gmask) * (1.f / 64.f) + eps);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) { const float dlt = x[i] - mean; v = fmaf(dlt, dlt, v); }
-  v += __shfl_xor_sync(gmask, v, 1);
-  v += __shfl_xor_sync(gmask, v, 2);
-  v += __shfl_xor_sync(gmask, v, 4);
-  const float rstd = rsqrtf(v * (1.f / 64.f) + eps);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) x[i] = fmaf((x[i] - mean) * rstd, w[i], b[i]);   // rounded to bf16 when packed
+  for (int i = 0; i < 4; ++i) x[i] = ffma2(fmul2(x[i], splat(rstd)), w[i], b[i]);   // rounded to bf16 when packed
 }
 
 // 2-D rotary embedding of a row held by 8 lanes, on packed bf16 pairs: lanes 0-3 hold the y half (32
@@ -73,11 +126,7 @@ __device__ __forceinline__ uint32_t bf2_add(uint32_t a, uint32_t b) {
   const __nv_bfloat162 r = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-__device__ __forceinline__ void rope_row(uint32_t (&xw)[4], const __nv_bfloat16* __restrict__ cos_tab,
-                                         const __nv_bfloat16* __restrict__ sin_tab, int row, int l8,
-                                         uint32_t gmask) {
-  const Vec8 c = *reinterpret_cast<const Vec8*>(cos_tab + static_cast<int64_t>(row) * 32 + (l8 & 3) * 8);
-  const Vec8 s = *reinterpret_cast<const Vec8*>(sin_tab + static_cast<int64_t>(row) * 32 + (l8 & 3) * 8);
+__device__ __forceinline__ void rope_row(uint32_t (&xw)[4], const Vec8& c, const Vec8& s, int l8, uint32_t gmask) {
   const uint32_t flip = (l8 & 2) == 0 ? 0x80008000u : 0u;
 #pragma unroll
   for (int wd = 0; wd < 4; ++wd) {
@@ -86,96 +135,108 @@ __device__ __forceinline__ void rope_row(uint32_t (&xw)[4], const __nv_bfloat16*
   }
 }
 
-// kMaxThreads = 384 covers up to 16 heads with 80 registers per thread at two CTAs per SM; more heads use
-// the 1024-thread form (64 registers).
-template <int kMaxThreads>
-__global__ void __launch_bounds__(kMaxThreads, kMaxThreads <= 384 ? 2 : 1)
-prologue_fwd_kernel(const PrologueParams p) {
+// A CTA has up to 16 of the block's 3H rows (8 lanes each: four warps, one per scheduler).  A thread's share of 16 tokens is on
+// its way at once, 16 bytes a token in slots of its own in shared memory (cp.async; nobody else reads them, so there is no
+// barrier): 32 KB per CTA and six CTAs per SM keep 192 KB in flight.  16 heads, 252000 tokens: 628 us, 0.78 of the copy rate
+// (24 KB in flight, the next tokens' loads in registers: 759; four tokens ahead and the tables' rows found by every row: 908);
+// 24 rows per CTA 656 us, eight CTAs of 64 registers 804.
+constexpr int kProRows = 16, kProThreads = kProRows * 8, kProChunk = 16, kProCtas = 6, kProBwdCtas = 4;
+constexpr int kProRingBytes = kProChunk * kProThreads * 16;
+
+__global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(const PrologueParams p) {
+  extern __shared__ __align__(16) uint8_t smem[];      // [token of the chunk][thread] 16 bytes; [warp] rows of the tables
   griddep_wait();
   griddep_launch();
-  const int l8 = threadIdx.x & 7;
-  const int g = threadIdx.x >> 3;                  // row of the token: (q|k|v, head)
+  const int lane = threadIdx.x & 31, l8 = threadIdx.x & 7;
+  const int g = blockIdx.y * kProRows + (threadIdx.x >> 3);           // row of the token: (q|k|v, head)
   const uint32_t gmask = 0xffu << (threadIdx.x & 24);
+  const bool live = g < 3 * p.H;
   const int which = g / p.H, h = g - which * p.H;
   const int b = blockIdx.x / p.Nc, j = blockIdx.x - b * p.Nc;
   const float* lw = which == 0 ? p.qw : p.kw;
   const float* lb = which == 0 ? p.qb : p.kb;
-  const bool norm = which < 2 && lw != nullptr;
-  const bool rope = which < 2 && p.pos != nullptr;
+  const bool norm = which < 2 && lw != nullptr, rope = which < 2 && p.pos != nullptr;
   __nv_bfloat16* out = which == 0 ? p.q : (which == 1 ? p.k : p.v);
   __nv_bfloat16* out_c = which == 0 ? p.q_c : (which == 1 ? p.k_c : p.v_c);
   const int64_t bh = static_cast<int64_t>(b) * p.H + h;
-
-  float wreg[8], breg[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    wreg[i] = norm ? __ldg(lw + l8 * 8 + i) : 1.f;
-    breg[i] = norm ? __ldg(lb + l8 * 8 + i) : 0.f;
-  }
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  float pos_sum = 0.f;                              // of this lane's coordinate (y for lanes 0-3, x for 4-7)
   const int n0 = j * p.block;
-  const __nv_bfloat16* src0 = p.qkv + ((static_cast<int64_t>(b) * p.N + n0) * 3 * p.H + g) * 64 + l8 * 8;
-  const int64_t tok_stride = static_cast<int64_t>(3) * p.H * 64;
-  auto load = [&](int t) { return *reinterpret_cast<const Vec8*>(src0 + t * tok_stride); };
-  // one token of this row: accumulate the raw block sum, normalise, rotate, store
-  auto token = [&](int n, const Vec8& raw) {
-    float x[8];
+  const int64_t tok0 = static_cast<int64_t>(b) * p.N + n0;
+  const __nv_bfloat16* src = p.qkv + tok0 * p.tok_stride + g * 64 + l8 * 8;
+  __nv_bfloat16* dst = out + (bh * p.N + n0) * 64 + l8 * 8;
+  const uint32_t slots = smem_u32(smem) + threadIdx.x * 16;
+  int* rows = reinterpret_cast<int*>(smem + kProRingBytes) + (threadIdx.x >> 5) * 2 * (p.block + 1);
+  // two groups of loads per chunk: the first half is worked on while the second arrives
+  auto fetch = [&](int t0) {
 #pragma unroll
-    for (int wd = 0; wd < 4; ++wd) { x[2 * wd] = bf16_lo(raw.w[wd]); x[2 * wd + 1] = bf16_hi(raw.w[wd]); }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] += x[i];
-    Vec8 o = raw;
-    if (which < 2) {
-      if (norm) {
-        ln_row(x, wreg, breg, p.eps, gmask);
-#pragma unroll
-        for (int wd = 0; wd < 4; ++wd) o.w[wd] = pack_bf16(x[2 * wd], x[2 * wd + 1]);
-      }
-      if (rope) {
-        const int64_t pv = p.pos[(static_cast<int64_t>(b) * p.N + n) * 2 + (l8 >> 2)];
-        pos_sum += static_cast<float>(pv);
-        const int row = min(max(static_cast<int>(pv), 0), p.tab_rows - 1);
-        if (pv != row) atomicOr(p.status, kStatusBadIndex);      // clamped: the result for this token is wrong
-        rope_row(o.w, p.cos_tab, p.sin_tab, row, l8, gmask);
-      }
+    for (int i = 0; i < kProChunk; ++i) {
+      if (live && t0 + i < p.block) cp_async16(slots + i * (kProThreads * 16), src + (t0 + i) * p.tok_stride);
+      if (i == kProChunk / 2 - 1) cp_async_commit();
     }
-    *reinterpret_cast<Vec8*>(out + (bh * p.N + n) * 64 + l8 * 8) = o;
+    cp_async_commit();
   };
-  // The kernel lives on bytes in flight: the loads of the next four tokens are issued before the current
-  // four are processed (their shuffle and rounding chains are long, the loads are independent of them).
-  Vec8 cur[4];
+  fetch(0);
+  if (p.pos != nullptr) block_rows(rows, p.pos + tok0 * 2, p.block, p.tab_rows, p.status, lane);
+  if (!live) return;
+  float2 w[4], bias[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (i < p.block) cur[i] = load(i);
-  for (int t0 = 0; t0 < p.block; t0 += 4) {
-    Vec8 nxt[4];
+  for (int i = 0; i < 4; ++i) {
+    w[i] = norm ? __ldg(reinterpret_cast<const float2*>(lw) + l8 * 4 + i) : splat(1.f);
+    bias[i] = norm ? __ldg(reinterpret_cast<const float2*>(lb) + l8 * 4 + i) : splat(0.f);
+  }
+  const int* my_row = rows + (l8 >> 2);                // y for lanes 0-3, x for 4-7
+  const __nv_bfloat16 *cos_l = p.cos_tab + (l8 & 3) * 8, *sin_l = p.sin_tab + (l8 & 3) * 8;
+
+  float2 acc[4] = {splat(0.f), splat(0.f), splat(0.f), splat(0.f)};
+  // one token of this row: accumulate the raw block sum, normalise, rotate, store
+  auto token = [&](int t, int slot) {
+    Vec8 c, s, o = lds_vec8(slots + slot * (kProThreads * 16));
+    if (rope) {
+      const int row = my_row[2 * t] * 32;
+      c = ldg_vec8(cos_l + row);
+      s = ldg_vec8(sin_l + row);
+    }
+    float2 x[4];
+    unpack8(x, o);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (t0 + 4 + i < p.block) nxt[i] = load(t0 + 4 + i);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (t0 + i < p.block) token(n0 + t0 + i, cur[i]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
+    for (int i = 0; i < 4; ++i) acc[i] = fadd2(acc[i], x[i]);
+    if (norm) {
+      ln_row(x, w, bias, p.eps, gmask);
+      o = pack8(x);
+    }
+    if (rope) rope_row(o.w, c, s, l8, gmask);
+    *reinterpret_cast<Vec8*>(dst + t * 64) = o;
+  };
+  for (int t0 = 0; t0 < p.block; t0 += kProChunk) {
+    const int n = min(kProChunk, p.block - t0);
+    cp_async_wait<1>();
+#pragma unroll 2
+    for (int i = 0; i < min(n, kProChunk / 2); ++i) token(t0 + i, i);
+    cp_async_wait<0>();
+#pragma unroll 2
+    for (int i = kProChunk / 2; i < n; ++i) token(t0 + i, i);
+    if (t0 + kProChunk < p.block) fetch(t0 + kProChunk);
   }
   // compression branch: mean of the raw rows, then the same norm and the rotary embedding at the block's
-  // mean position (float mean, truncated: xpos.view(..).float().mean(dim=2).int())
+  // mean position
   const float inv = 1.f / static_cast<float>(p.block);
-  float x[8];
+  float2 x[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) x[i] = bf16r(acc[i] * inv);
-  if (norm) ln_row(x, wreg, breg, p.eps, gmask);
-  Vec8 o;
-#pragma unroll
-  for (int wd = 0; wd < 4; ++wd) o.w[wd] = pack_bf16(x[2 * wd], x[2 * wd + 1]);
+  for (int i = 0; i < 4; ++i) x[i] = make_float2(bf16r(acc[i].x * inv), bf16r(acc[i].y * inv));
+  if (norm) ln_row(x, w, bias, p.eps, gmask);
+  Vec8 o = pack8(x);
   if (rope) {
-    const int pc = static_cast<int>(pos_sum / static_cast<float>(p.block));
-    const int row = min(max(pc, 0), p.tab_rows - 1);
-    if (pc != row) atomicOr(p.status, kStatusBadIndex);
-    rope_row(o.w, p.cos_tab, p.sin_tab, row, l8, gmask);
+    const int row = my_row[2 * p.block] * 32;
+    rope_row(o.w, ldg_vec8(cos_l + row), ldg_vec8(sin_l + row), l8, gmask);
   }
   *reinterpret_cast<Vec8*>(out_c + (bh * p.Nc + j) * 64 + l8 * 8) = o;
+  if (p.gate_in != nullptr && blockIdx.y == 0) {
+    for (int i = threadIdx.x; i < p.block * p.H; i += min(kProThreads, 3 * p.H * 8)) {
+      const int t = i % p.block, hd = i / p.block;
+      const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(p.gate_in + (tok0 + t) * p.tok_stride) + hd);
+      const float g0 = 1.f / (1.f + __expf(-bf16_lo(v))), g1 = 1.f / (1.f + __expf(-bf16_hi(v)));
+      p.gate[(static_cast<int64_t>(b) * p.H + hd) * p.N + n0 + t] = pack_bf16(g0, g1);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -189,6 +250,10 @@ prologue_fwd_kernel(const PrologueParams p) {
 // order.
 struct PrologueBwdParams {
   const __nv_bfloat16* qkv;
+  int64_t tok_stride;                // of qkv and dqkv
+  const uint32_t* gate;              // [B,H,N] pairs, sigmoid of the logits (null: no gate)
+  const float2* dgate;               // [B,H,N] gradient of those
+  __nv_bfloat16* dgate_in;           // gradient of the logits, inside dqkv's rows
   const int64_t* pos;
   const __nv_bfloat16* cos_tab;
   const __nv_bfloat16* sin_tab;
@@ -197,167 +262,181 @@ struct PrologueBwdParams {
   float eps;
   const __nv_bfloat16 *dq, *dk, *dv, *dq_c, *dk_c, *dv_c;
   __nv_bfloat16* dqkv;
-  float* partial;                    // [gridDim.x][q|k][weight|bias][64], null without norms
+  float* partial;                    // [CTA][q|k][weight|bias][64], null without norms
   int B, H, N, Nc, block;
 };
 
-__device__ __forceinline__ float sum8(float x, uint32_t gmask) {
-  x += __shfl_xor_sync(gmask, x, 1);
-  x += __shfl_xor_sync(gmask, x, 2);
-  return x + __shfl_xor_sync(gmask, x, 4);
-}
-__device__ __forceinline__ void unpack8(float (&x)[8], const Vec8& v) {
-#pragma unroll
-  for (int wd = 0; wd < 4; ++wd) { x[2 * wd] = bf16_lo(v.w[wd]); x[2 * wd + 1] = bf16_hi(v.w[wd]); }
-}
 // transposed rotary embedding: dt[j] = dy[j] cos[j] + dy[j+16] sin[j+16] for j < 16, dy[j] cos[j] - dy[j-16] sin[j-16] otherwise
-__device__ __forceinline__ void rope_row_t(float (&dy)[8], const __nv_bfloat16* __restrict__ cos_tab,
-                                           const __nv_bfloat16* __restrict__ sin_tab, int row, int l8, uint32_t gmask) {
-  float c[8], s[8];
-  unpack8(c, *reinterpret_cast<const Vec8*>(cos_tab + static_cast<int64_t>(row) * 32 + (l8 & 3) * 8));
-  unpack8(s, *reinterpret_cast<const Vec8*>(sin_tab + static_cast<int64_t>(row) * 32 + (l8 & 3) * 8));
-  const float sign = (l8 & 2) == 0 ? 1.f : -1.f;
+__device__ __forceinline__ void rope_row_t(float2 (&dy)[4], const Vec8& cw, const Vec8& sw, int l8, uint32_t gmask) {
+  float2 c[4], s[4];
+  unpack8(c, cw);
+  unpack8(s, sw);
+  const float2 sign = splat((l8 & 2) == 0 ? 1.f : -1.f);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float other = __shfl_xor_sync(gmask, dy[i] * s[i], 2);
-    dy[i] = fmaf(dy[i], c[i], sign * other);
+  for (int i = 0; i < 4; ++i) {
+    float2 o = fmul2(dy[i], s[i]);
+    o.x = __shfl_xor_sync(gmask, o.x, 2);
+    o.y = __shfl_xor_sync(gmask, o.y, 2);
+    dy[i] = ffma2(o, sign, fmul2(dy[i], c[i]));
   }
 }
 // dx of y = LayerNorm(x) w + b in place of dy; adds to the parameters' gradients
-__device__ __forceinline__ void ln_row_bwd(const float (&x)[8], float (&dy)[8], const float (&w)[8], float (&gw)[8],
-                                           float (&gb)[8], float eps, uint32_t gmask) {
-  float s = 0.f, sg = 0.f;
+__device__ __forceinline__ void ln_row_bwd(float2 (&x)[4], float2 (&dy)[4], const float2 (&w)[4], float2 (&gw)[4],
+                                           float2 (&gb)[4], float eps, uint32_t gmask) {
+  float2 s = fadd2(fadd2(x[0], x[1]), fadd2(x[2], x[3])), sg = splat(0.f), g[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    s += x[i];
-    sg = fmaf(dy[i], w[i], sg);
+  for (int i = 0; i < 4; ++i) {
+    g[i] = fmul2(dy[i], w[i]);
+    sg = fadd2(sg, g[i]);
   }
-  const float mean = sum8(s, gmask) * (1.f / 64.f), mg = sum8(sg, gmask) * (1.f / 64.f);
-  float v = 0.f, sx = 0.f, xh[8];
+  const float mean = sum8(s.x + s.y, gmask) * (1.f / 64.f), mg = sum8(sg.x + sg.y, gmask) * (1.f / 64.f);
+  float2 v = splat(0.f), sx = splat(0.f);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    xh[i] = x[i] - mean;
-    v = fmaf(xh[i], xh[i], v);
-    sx = fmaf(dy[i] * w[i], xh[i], sx);
+  for (int i = 0; i < 4; ++i) {
+    x[i] = fadd2(x[i], splat(-mean));
+    v = ffma2(x[i], x[i], v);
+    sx = ffma2(g[i], x[i], sx);
   }
-  const float rstd = rsqrtf(sum8(v, gmask) * (1.f / 64.f) + eps), mgx = sum8(sx, gmask) * (1.f / 64.f) * rstd;
+  const float rstd = rsqrtf(sum8(v.x + v.y, gmask) * (1.f / 64.f) + eps);
+  const float mgx = sum8(sx.x + sx.y, gmask) * (1.f / 64.f) * rstd;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    xh[i] *= rstd;
-    gw[i] = fmaf(dy[i], xh[i], gw[i]);
-    gb[i] += dy[i];
-    dy[i] = rstd * (fmaf(dy[i], w[i], -mg) - xh[i] * mgx);
+  for (int i = 0; i < 4; ++i) {
+    x[i] = fmul2(x[i], splat(rstd));
+    gw[i] = ffma2(dy[i], x[i], gw[i]);
+    gb[i] = fadd2(gb[i], dy[i]);
+    dy[i] = fmul2(splat(rstd), ffma2(x[i], splat(-mgx), fadd2(g[i], splat(-mg))));
   }
 }
 
-template <int kMaxThreads>
-__global__ void __launch_bounds__(kMaxThreads, kMaxThreads <= 384 ? 2 : 1) prologue_bwd_kernel(const PrologueBwdParams p) {
-  extern __shared__ float red[];                   // [2H rows][weight|bias][64]
+// Same rows per CTA and the same private slots: a block's 16 tokens of the projection stay in shared memory for both uses (its
+// mean, then its tokens; longer blocks are read again), the gradients come through eight slots.  252000 tokens: 1272 us
+// (registers instead of slots, everybody waiting for a block's rows: 1903), 64512: 338.
+constexpr int kProBwdAhead = 8;
+constexpr int kProBwdRingBytes = (kProChunk + kProBwdAhead) * kProThreads * 16;
+
+__global__ void __launch_bounds__(kProThreads, kProBwdCtas) prologue_bwd_kernel(const PrologueBwdParams p) {
+  extern __shared__ __align__(16) uint8_t smem[];      // [token][thread] 16 bytes: projection, gradients; [warp] rows of the tables
   griddep_wait();
   griddep_launch();
-  const int l8 = threadIdx.x & 7, g = threadIdx.x >> 3;
+  const int lane = threadIdx.x & 31, l8 = threadIdx.x & 7;
+  const int g = blockIdx.y * kProRows + (threadIdx.x >> 3);
   const uint32_t gmask = 0xffu << (threadIdx.x & 24);
+  const bool live = g < 3 * p.H;
   const int which = g / p.H, h = g - which * p.H;
   const float* lw = which == 0 ? p.qw : p.kw;
   const bool norm = which < 2 && lw != nullptr, rope = which < 2 && p.pos != nullptr;
   const __nv_bfloat16* dout = which == 0 ? p.dq : (which == 1 ? p.dk : p.dv);
   const __nv_bfloat16* dout_c = which == 0 ? p.dq_c : (which == 1 ? p.dk_c : p.dv_c);
-  float w[8], gw[8], gb[8];
+  float2 w[4], gw[4], gb[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    w[i] = norm ? __ldg(lw + l8 * 8 + i) : 1.f;
-    gw[i] = gb[i] = 0.f;
+  for (int i = 0; i < 4; ++i) {
+    w[i] = norm ? __ldg(reinterpret_cast<const float2*>(lw) + l8 * 4 + i) : splat(1.f);
+    gw[i] = gb[i] = splat(0.f);
   }
   const float inv = 1.f / static_cast<float>(p.block);
-  const int64_t tok_stride = static_cast<int64_t>(3) * p.H * 64;
+  const uint32_t xs = smem_u32(smem) + threadIdx.x * 16, ds = xs + kProChunk * (kProThreads * 16);
+  int* rows = reinterpret_cast<int*>(smem + kProBwdRingBytes) + (threadIdx.x >> 5) * 2 * (p.block + 1);
+  const int* my_row = rows + (l8 >> 2);                // y for lanes 0-3, x for 4-7
+  const __nv_bfloat16 *cos_l = p.cos_tab + (l8 & 3) * 8, *sin_l = p.sin_tab + (l8 & 3) * 8;
+  const bool resident = p.block <= kProChunk;
   const int nblocks = p.B * p.Nc;
   for (int blk = blockIdx.x; blk < nblocks; blk += gridDim.x) {
     const int b = blk / p.Nc, j = blk - b * p.Nc;
     const int64_t bh = static_cast<int64_t>(b) * p.H + h, tok0 = static_cast<int64_t>(b) * p.N + static_cast<int64_t>(j) * p.block;
-    const __nv_bfloat16* src = p.qkv + tok0 * tok_stride + g * 64 + l8 * 8;
+    const __nv_bfloat16* src = p.qkv + tok0 * p.tok_stride + g * 64 + l8 * 8;
     const __nv_bfloat16* dsrc = dout + (bh * p.N + static_cast<int64_t>(j) * p.block) * 64 + l8 * 8;
-    __nv_bfloat16* dst = p.dqkv + tok0 * tok_stride + g * 64 + l8 * 8;
-    auto load = [&](const __nv_bfloat16* q, int64_t stride, int t) { return *reinterpret_cast<const Vec8*>(q + t * stride); };
-    auto row_of = [&](int64_t pv) { return min(max(static_cast<int>(pv), 0), p.tab_rows - 1); };
-    const int64_t* pos = p.pos + tok0 * 2 + (l8 >> 2);
-
-    // the pooled branch's gradient of every token of the block
-    float dc[8];
-    unpack8(dc, *reinterpret_cast<const Vec8*>(dout_c + (bh * p.Nc + j) * 64 + l8 * 8));
-    if (rope) {
-      float pos_sum = 0.f;
-      for (int t = 0; t < p.block; ++t) pos_sum += static_cast<float>(pos[2 * t]);
-      rope_row_t(dc, p.cos_tab, p.sin_tab, row_of(static_cast<int64_t>(pos_sum / static_cast<float>(p.block))), l8, gmask);
-    }
-    if (norm) {
-      float xc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-      for (int t = 0; t < p.block; ++t) {
-        float x[8];
-        unpack8(x, load(src, tok_stride, t));
+    __nv_bfloat16* dst = p.dqkv + tok0 * p.tok_stride + g * 64 + l8 * 8;
+    Vec8 raw_c;
+    if (live) {
+      if (norm && resident)
+        for (int t = 0; t < p.block; ++t) cp_async16(xs + t * (kProThreads * 16), src + t * p.tok_stride);
+      cp_async_commit();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) xc[i] += x[i];
+      for (int t = 0; t < kProBwdAhead; ++t) {
+        if (t < p.block) cp_async16(ds + t * (kProThreads * 16), dsrc + t * 64);
+        cp_async_commit();
       }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) xc[i] = bf16r(xc[i] * inv);
-      ln_row_bwd(xc, dc, w, gw, gb, p.eps, gmask);
+      raw_c = ldg_vec8(dout_c + (bh * p.Nc + j) * 64 + l8 * 8);
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) dc[i] *= inv;
-
-    auto token = [&](int t, const Vec8& rawx, const Vec8& rawd) {
-      float dy[8];
-      unpack8(dy, rawd);
-      if (rope) rope_row_t(dy, p.cos_tab, p.sin_tab, row_of(pos[2 * t]), l8, gmask);
+    __syncwarp();                                      // the previous block's rows have been used
+    if (p.pos != nullptr) block_rows(rows, p.pos + tok0 * 2, p.block, p.tab_rows, nullptr, lane);
+    if (live) {
+      // the pooled branch's gradient of every token of the block
+      float2 dc[4];
+      unpack8(dc, raw_c);
+      if (rope) {
+        const int row = my_row[2 * p.block] * 32;
+        rope_row_t(dc, ldg_vec8(cos_l + row), ldg_vec8(sin_l + row), l8, gmask);
+      }
+      cp_async_wait<kProBwdAhead>();
       if (norm) {
-        float x[8];
-        unpack8(x, rawx);
-        ln_row_bwd(x, dy, w, gw, gb, p.eps, gmask);
-      }
-      Vec8 o;
+        float2 xc[4] = {splat(0.f), splat(0.f), splat(0.f), splat(0.f)};
+#pragma unroll 4
+        for (int t = 0; t < p.block; ++t) {
+          float2 x[4];
+          unpack8(x, resident ? lds_vec8(xs + t * (kProThreads * 16)) : ldg_vec8(src + t * p.tok_stride));
 #pragma unroll
-      for (int wd = 0; wd < 4; ++wd) o.w[wd] = pack_bf16(dy[2 * wd] + dc[2 * wd], dy[2 * wd + 1] + dc[2 * wd + 1]);
-      *reinterpret_cast<Vec8*>(dst + t * tok_stride) = o;
-    };
-    // two tokens' loads ahead of the two being worked on
-    Vec8 cx[2], cd[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (i < p.block) {
-        if (norm) cx[i] = load(src, tok_stride, i);
-        cd[i] = load(dsrc, 64, i);
-      }
-    for (int t0 = 0; t0 < p.block; t0 += 2) {
-      Vec8 nx[2], nd[2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        if (t0 + 2 + i < p.block) {
-          if (norm) nx[i] = load(src, tok_stride, t0 + 2 + i);
-          nd[i] = load(dsrc, 64, t0 + 2 + i);
+          for (int i = 0; i < 4; ++i) xc[i] = fadd2(xc[i], x[i]);
         }
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-        if (t0 + i < p.block) token(t0 + i, cx[i], cd[i]);
+        for (int i = 0; i < 4; ++i) xc[i] = make_float2(bf16r(xc[i].x * inv), bf16r(xc[i].y * inv));
+        ln_row_bwd(xc, dc, w, gw, gb, p.eps, gmask);
+      }
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        cx[i] = nx[i];
-        cd[i] = nd[i];
+      for (int i = 0; i < 4; ++i) dc[i] = fmul2(dc[i], splat(inv));
+
+#pragma unroll 2
+      for (int t = 0; t < p.block; ++t) {
+        Vec8 c, s;
+        if (rope) {
+          const int row = my_row[2 * t] * 32;
+          c = ldg_vec8(cos_l + row);
+          s = ldg_vec8(sin_l + row);
+        }
+        cp_async_wait<kProBwdAhead - 1>();
+        const uint32_t slot = ds + (t % kProBwdAhead) * (kProThreads * 16);
+        float2 dy[4];
+        unpack8(dy, lds_vec8(slot));
+        if (t + kProBwdAhead < p.block) cp_async16(slot, dsrc + (t + kProBwdAhead) * 64);
+        cp_async_commit();
+        if (rope) rope_row_t(dy, c, s, l8, gmask);
+        if (norm) {
+          float2 x[4];
+          unpack8(x, resident ? lds_vec8(xs + t * (kProThreads * 16)) : ldg_vec8(src + t * p.tok_stride));
+          ln_row_bwd(x, dy, w, gw, gb, p.eps, gmask);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dy[i] = fadd2(dy[i], dc[i]);
+        *reinterpret_cast<Vec8*>(dst + t * p.tok_stride) = pack8(dy);
+      }
+    }
+    if (p.gate != nullptr && blockIdx.y == 0) {
+      for (int i = threadIdx.x; i < p.block * p.H; i += kProThreads) {
+        const int t = i % p.block, hd = i / p.block;
+        const int64_t at = (static_cast<int64_t>(b) * p.H + hd) * p.N + static_cast<int64_t>(j) * p.block + t;
+        const uint32_t v = __ldg(p.gate + at);
+        const float2 d = __ldg(p.dgate + at);
+        const float g0 = bf16_lo(v), g1 = bf16_hi(v);
+        *(reinterpret_cast<uint32_t*>(p.dgate_in + (tok0 + t) * p.tok_stride) + hd) = pack_bf16(d.x * g0 * (1.f - g0), d.y * g1 * (1.f - g1));
       }
     }
   }
   if (p.partial == nullptr) return;
-  if (which < 2) {
+  cp_async_wait<0>();
+  __syncthreads();
+  float* red = reinterpret_cast<float*>(smem);         // [row][weight|bias][64]
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      red[g * 128 + l8 * 8 + i] = gw[i];
-      red[g * 128 + 64 + l8 * 8 + i] = gb[i];
-    }
+  for (int i = 0; i < 4; ++i) {
+    const int at = (threadIdx.x >> 3) * 128 + l8 * 8 + 2 * i;
+    *reinterpret_cast<float2*>(&red[at]) = gw[i];
+    *reinterpret_cast<float2*>(&red[at + 64]) = gb[i];
   }
   __syncthreads();
-  for (int o = threadIdx.x; o < 256; o += blockDim.x) {      // (q|k, weight|bias, channel)
+  for (int o = threadIdx.x; o < 256; o += kProThreads) {     // (q|k, weight|bias, channel)
     float s = 0.f;
-    for (int r = 0; r < p.H; ++r) s += red[((o >> 7) * p.H + r) * 128 + (o & 127)];
-    p.partial[blockIdx.x * 256 + o] = s;
+    for (int r = 0; r < kProRows; ++r)
+      if ((blockIdx.y * kProRows + r) / p.H == (o >> 7)) s += red[r * 128 + (o & 127)];
+    p.partial[(blockIdx.y * gridDim.x + blockIdx.x) * 256 + o] = s;
   }
 }
 
@@ -373,8 +452,10 @@ __global__ void __launch_bounds__(256) prologue_bwd_reduce_kernel(const float* _
   if (lane == 0) out[o] = s;
 }
 
-static int prologue_bwd_ctas(int B, int Nc) {
-  const int64_t n = static_cast<int64_t>(B) * Nc, cap = 2 * sm_count();
+static int prologue_parts(int H) { return (3 * H + kProRows - 1) / kProRows; }
+// CTAs along the blocks: four per SM over all parts
+static int prologue_bwd_ctas(int B, int Nc, int H) {
+  const int64_t n = static_cast<int64_t>(B) * Nc, parts = prologue_parts(H), cap = (kProBwdCtas * sm_count() + parts - 1) / parts;
   return static_cast<int>(n < cap ? n : cap);
 }
 
@@ -382,7 +463,7 @@ static int prologue_bwd_ctas(int B, int Nc) {
 
 using namespace s3r;
 
-extern "C" int s3r_qkv_prologue_fwd(const void* qkv, const int64_t* pos, const void* cos_tab, const void* sin_tab,
+static int prologue_fwd(const void* qkv, int64_t tok_stride, const void* gate_in, void* gate, const int64_t* pos, const void* cos_tab, const void* sin_tab,
                                     int tab_rows, const float* q_weight, const float* q_bias, const float* k_weight,
                                     const float* k_bias, float eps, void* q, void* k, void* v, void* q_c, void* k_c,
                                     void* v_c, int B, int H, int N, int d, int block, void* stream) {
@@ -408,6 +489,9 @@ extern "C" int s3r_qkv_prologue_fwd(const void* qkv, const int64_t* pos, const v
               (long long)grid);
   PrologueParams p;
   p.qkv = static_cast<const __nv_bfloat16*>(qkv);
+  p.tok_stride = tok_stride;
+  p.gate_in = static_cast<const __nv_bfloat16*>(gate_in);
+  p.gate = static_cast<uint32_t*>(gate);
   p.pos = pos;
   p.cos_tab = static_cast<const __nv_bfloat16*>(cos_tab);
   p.sin_tab = static_cast<const __nv_bfloat16*>(sin_tab);
@@ -420,16 +504,38 @@ extern "C" int s3r_qkv_prologue_fwd(const void* qkv, const int64_t* pos, const v
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_qkv_prologue_fwd: could not resolve the device status word");
-  return launch(3 * H * 8 <= 384 ? prologue_fwd_kernel<384> : prologue_fwd_kernel<1024>, static_cast<unsigned>(grid), 3 * H * 8, 0,
+  const int smem = kProRingBytes + (kProThreads / 32) * 2 * (block + 1) * static_cast<int>(sizeof(int));
+  S3R_REQUIRE(smem <= 227 * 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_fwd: block %d is too long", block);
+  S3R_CUDA(cudaFuncSetAttribute(prologue_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return launch(prologue_fwd_kernel, dim3(static_cast<unsigned>(grid), prologue_parts(H)), kProThreads, smem,
                 static_cast<cudaStream_t>(stream), p);
 }
 
-extern "C" size_t s3r_qkv_prologue_bwd_workspace_bytes(int B, int N, int block) {
-  if (B <= 0 || N <= 0 || block <= 0 || N < block) return 0;
-  return static_cast<size_t>(prologue_bwd_ctas(B, N / block)) * 256 * sizeof(float);
+extern "C" int s3r_qkv_prologue_fwd(const void* qkv, const int64_t* pos, const void* cos_tab, const void* sin_tab,
+                                    int tab_rows, const float* q_weight, const float* q_bias, const float* k_weight,
+                                    const float* k_bias, float eps, void* q, void* k, void* v, void* q_c, void* k_c,
+                                    void* v_c, int B, int H, int N, int d, int block, void* stream) {
+  return prologue_fwd(qkv, static_cast<int64_t>(3) * H * d, nullptr, nullptr, pos, cos_tab, sin_tab, tab_rows, q_weight, q_bias, k_weight,
+                      k_bias, eps, q, k, v, q_c, k_c, v_c, B, H, N, d, block, stream);
 }
 
-extern "C" int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const void* cos_tab, const void* sin_tab, int tab_rows,
+extern "C" int s3r_qkv_gate_prologue_fwd(const void* proj, const int64_t* pos, const void* cos_tab, const void* sin_tab,
+                                         int tab_rows, const float* q_weight, const float* q_bias, const float* k_weight,
+                                         const float* k_bias, float eps, void* q, void* k, void* v, void* q_c, void* k_c,
+                                         void* v_c, void* gate, int B, int H, int N, int d, int block, void* stream) {
+  S3R_REQUIRE(proj && gate, S3R_ERR_NULL, "s3r_qkv_gate_prologue_fwd: NULL tensor");
+  S3R_REQUIRE(H > 0 && H % 4 == 0, S3R_ERR_UNSUPPORTED, "s3r_qkv_gate_prologue_fwd: %d heads are not a multiple of 4", H);
+  const int64_t C3 = static_cast<int64_t>(3) * H * d;
+  return prologue_fwd(proj, C3 + 2 * H, static_cast<const __nv_bfloat16*>(proj) + C3, gate, pos, cos_tab, sin_tab, tab_rows, q_weight,
+                      q_bias, k_weight, k_bias, eps, q, k, v, q_c, k_c, v_c, B, H, N, d, block, stream);
+}
+
+extern "C" size_t s3r_qkv_prologue_bwd_workspace_bytes(int B, int H, int N, int block) {
+  if (B <= 0 || H <= 0 || N <= 0 || block <= 0 || N < block) return 0;
+  return static_cast<size_t>(prologue_bwd_ctas(B, N / block, H)) * prologue_parts(H) * 256 * sizeof(float);
+}
+
+static int prologue_bwd(const void* qkv, int64_t tok_stride, const void* gate, const float* dgate, void* dgate_in, const int64_t* pos, const void* cos_tab, const void* sin_tab, int tab_rows,
                                     const float* q_weight, const float* k_weight, float eps, const void* dq, const void* dk,
                                     const void* dv, const void* dq_c, const void* dk_c, const void* dv_c, void* dqkv,
                                     float* dparams, void* workspace, size_t workspace_bytes, int B, int H, int N, int d,
@@ -444,9 +550,9 @@ extern "C" int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const v
               "s3r_qkv_prologue_bwd: LayerNorm weights of q and k and their gradients come together or not at all");
   S3R_REQUIRE(pos == nullptr || (cos_tab && sin_tab && tab_rows > 0), S3R_ERR_NULL,
               "s3r_qkv_prologue_bwd: positions need the cos/sin tables");
-  S3R_REQUIRE(!dparams || (workspace && workspace_bytes >= s3r_qkv_prologue_bwd_workspace_bytes(B, N, block)), S3R_ERR_TOO_LARGE,
+  S3R_REQUIRE(!dparams || (workspace && workspace_bytes >= s3r_qkv_prologue_bwd_workspace_bytes(B, H, N, block)), S3R_ERR_TOO_LARGE,
               "s3r_qkv_prologue_bwd: workspace of %zu bytes is smaller than the %zu needed", workspace_bytes,
-              s3r_qkv_prologue_bwd_workspace_bytes(B, N, block));
+              s3r_qkv_prologue_bwd_workspace_bytes(B, H, N, block));
   uintptr_t al = reinterpret_cast<uintptr_t>(cos_tab) | reinterpret_cast<uintptr_t>(sin_tab) | reinterpret_cast<uintptr_t>(dqkv);
   for (const void* t : {qkv, dq, dk, dv, dq_c, dk_c, dv_c}) al |= reinterpret_cast<uintptr_t>(t);
   S3R_REQUIRE((al & 15) == 0, S3R_ERR_ALIGNMENT, "s3r_qkv_prologue_bwd: tensors must be 16-byte aligned");
@@ -454,6 +560,10 @@ extern "C" int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const v
   S3R_REQUIRE(static_cast<int64_t>(B) * Nc < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_qkv_prologue_bwd: too many blocks");
   PrologueBwdParams p;
   p.qkv = static_cast<const __nv_bfloat16*>(qkv);
+  p.tok_stride = tok_stride;
+  p.gate = static_cast<const uint32_t*>(gate);
+  p.dgate = reinterpret_cast<const float2*>(dgate);
+  p.dgate_in = static_cast<__nv_bfloat16*>(dgate_in);
   p.pos = pos;
   p.cos_tab = static_cast<const __nv_bfloat16*>(cos_tab);
   p.sin_tab = static_cast<const __nv_bfloat16*>(sin_tab);
@@ -466,10 +576,34 @@ extern "C" int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const v
   p.dqkv = static_cast<__nv_bfloat16*>(dqkv);
   p.partial = dparams ? static_cast<float*>(workspace) : nullptr;
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
-  const int ctas = prologue_bwd_ctas(B, Nc), smem = 2 * H * 128 * static_cast<int>(sizeof(float));
+  const int ctas = prologue_bwd_ctas(B, Nc, H), parts = prologue_parts(H);
+  const int smem = kProBwdRingBytes + (kProThreads / 32) * 2 * (block + 1) * static_cast<int>(sizeof(int));
+  S3R_REQUIRE(smem <= 227 * 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_bwd: block %d is too long", block);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int rc = launch(3 * H * 8 <= 384 ? prologue_bwd_kernel<384> : prologue_bwd_kernel<1024>, static_cast<unsigned>(ctas),
-                        3 * H * 8, smem, st, p);
+  S3R_CUDA(cudaFuncSetAttribute(prologue_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int rc = launch(prologue_bwd_kernel, dim3(static_cast<unsigned>(ctas), parts), kProThreads, smem, st, p);
   if (rc || !dparams) return rc;
-  return launch(prologue_bwd_reduce_kernel, 32, 256, 0, st, p.partial, dparams, ctas);
+  return launch(prologue_bwd_reduce_kernel, 32, 256, 0, st, p.partial, dparams, ctas * parts);
+}
+
+extern "C" int s3r_qkv_prologue_bwd(const void* qkv, const int64_t* pos, const void* cos_tab, const void* sin_tab, int tab_rows,
+                                    const float* q_weight, const float* k_weight, float eps, const void* dq, const void* dk,
+                                    const void* dv, const void* dq_c, const void* dk_c, const void* dv_c, void* dqkv,
+                                    float* dparams, void* workspace, size_t workspace_bytes, int B, int H, int N, int d,
+                                    int block, void* stream) {
+  return prologue_bwd(qkv, static_cast<int64_t>(3) * H * d, nullptr, nullptr, nullptr, pos, cos_tab, sin_tab, tab_rows, q_weight, k_weight,
+                      eps, dq, dk, dv, dq_c, dk_c, dv_c, dqkv, dparams, workspace, workspace_bytes, B, H, N, d, block, stream);
+}
+
+extern "C" int s3r_qkv_gate_prologue_bwd(const void* proj, const int64_t* pos, const void* cos_tab, const void* sin_tab,
+                                         int tab_rows, const float* q_weight, const float* k_weight, float eps, const void* dq,
+                                         const void* dk, const void* dv, const void* dq_c, const void* dk_c, const void* dv_c,
+                                         const void* gate, const float* dgate, void* dproj, float* dparams, void* workspace,
+                                         size_t workspace_bytes, int B, int H, int N, int d, int block, void* stream) {
+  S3R_REQUIRE(proj && gate && dgate && dproj, S3R_ERR_NULL, "s3r_qkv_gate_prologue_bwd: NULL tensor");
+  S3R_REQUIRE(H > 0 && H % 4 == 0, S3R_ERR_UNSUPPORTED, "s3r_qkv_gate_prologue_bwd: %d heads are not a multiple of 4", H);
+  const int64_t C3 = static_cast<int64_t>(3) * H * d;
+  return prologue_bwd(proj, C3 + 2 * H, gate, dgate, static_cast<__nv_bfloat16*>(dproj) + C3, pos, cos_tab, sin_tab, tab_rows, q_weight,
+                      k_weight, eps, dq, dk, dv, dq_c, dk_c, dv_c, dproj, dparams, workspace, workspace_bytes, B, H, N, d, block,
+                      stream);
 }

@@ -334,7 +334,7 @@ std::tuple<Tensor, Tensor> prologue_bwd(const Tensor& qkv, int64_t heads, int64_
   const int64_t B = qkv.size(0), N = qkv.size(1), d = qkv.numel() / (B * N) / (3 * heads);
   c10::cuda::CUDAGuard guard(qkv.device());
   const bool norm = qw.has_value(), rope = pos.has_value();
-  const size_t nbytes = norm ? s3r_qkv_prologue_bwd_workspace_bytes(B, N, block) : 0;
+  const size_t nbytes = norm ? s3r_qkv_prologue_bwd_workspace_bytes(B, heads, N, block) : 0;
   Tensor dqkv = fresh_like(qkv), ws = fresh({static_cast<int64_t>(nbytes)}, qkv, at::kByte),
          dparams = fresh(norm ? std::vector<int64_t>{4, d} : std::vector<int64_t>{0}, qkv, at::kFloat);
   check(s3r_qkv_prologue_bwd(qkv.data_ptr(), static_cast<const int64_t*>(ptr_or_null(pos)), rope ? ptr_or_null(cos) : nullptr,
@@ -343,25 +343,6 @@ std::tuple<Tensor, Tensor> prologue_bwd(const Tensor& qkv, int64_t heads, int64_
                              norm ? f32(dparams) : nullptr, norm ? ws.data_ptr() : nullptr, nbytes, B, heads, N, d, block,
                              stream()), "s3r_qkv_prologue_bwd");
   return {dqkv, dparams};
-}
-
-// bf16 copies of fp32 tensors, in one launch (up to eight)
-std::vector<Tensor> cast_bf16(at::TensorList xs) {
-  TORCH_CHECK(!xs.empty() && xs.size() <= 8, "cast_bf16: 1 to 8 tensors");
-  c10::cuda::CUDAGuard guard(xs[0].device());
-  std::vector<Tensor> out;
-  const float* src[8];
-  void* dst[8];
-  int64_t counts[8];
-  for (size_t i = 0; i < xs.size(); ++i) {
-    need(xs[i], "x", at::kFloat);
-    out.push_back(fresh(xs[i].sizes(), xs[i], at::kBFloat16));
-    src[i] = f32(xs[i]);
-    dst[i] = out[i].data_ptr();
-    counts[i] = xs[i].numel();
-  }
-  check(s3r_cast_bf16(static_cast<int>(xs.size()), src, dst, counts, stream()), "s3r_cast_bf16");
-  return out;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -570,44 +551,137 @@ SixTensors prologue(const Tensor& qkv, int64_t heads, int64_t block, const optio
   return call_prologue(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
 }
 
-// The whole attention module without gradients: projections (cuBLAS), sigmoid of the gate, prologue, the two attentions,
-// output projection.  fp32 input and parameters are rounded to bf16 as under autocast, all in one launch.
+// The whole attention module without gradients: projections (cuBLAS), prologue, the two attentions, output projection.
+// fp32 input and parameters are rounded to bf16 as under autocast, all in one launch, with the weights of qkv and gate side
+// by side so that one GEMM does both; everything between the GEMMs lives in one allocation and goes straight to the C ABI:
+// at 2048 tokens the call is bound by host work (388 us at first, 178 with an operator for every step, TIME_HOST so).
 std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, const optional<Tensor>& b_qkv, const Tensor& w_gate,
                                         const optional<Tensor>& b_gate, const Tensor& w_proj, const optional<Tensor>& b_proj,
-                                        const optional<Tensor>& pos, const optional<Tensor>& cos, const optional<Tensor>& sin,
-                                        const optional<Tensor>& qw, const optional<Tensor>& qb, const optional<Tensor>& kw,
-                                        const optional<Tensor>& kb, double eps, int64_t heads, int64_t block, int64_t topk,
+                                        const optional<Tensor>& pos_, const optional<Tensor>& cos, const optional<Tensor>& sin,
+                                        const optional<Tensor>& qw_, const optional<Tensor>& qb_, const optional<Tensor>& kw_,
+                                        const optional<Tensor>& kb_, double eps, int64_t heads, int64_t block, int64_t topk,
                                         double scale) {
-  at::NoGradGuard no_grad;
+  at::AutoDispatchBelowAutograd below;
   c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
-  std::vector<Tensor> in = {x_, w_qkv, w_gate, w_proj};
-  const optional<Tensor>* biases[3] = {&b_qkv, &b_gate, &b_proj};
-  int at_bias[3] = {-1, -1, -1};
-  for (int i = 0; i < 3; ++i)
-    if (biases[i]->has_value()) {
-      at_bias[i] = static_cast<int>(in.size());
-      in.push_back(**biases[i]);
+  TORCH_CHECK(x_.is_cuda() && x_.dim() == 3, "x must be a CUDA tensor [B,N,C]: the speed3r_b200 kernels have no CPU path");
+  c10::cuda::CUDAGuard guard(x_.device());
+  void* st = stream();
+  const int64_t B = x_.size(0), N = x_.size(1), C = x_.size(2), H = heads, d = C / heads, M = B * N, Nc = N / block;
+  auto as = [&](const optional<Tensor>& t, at::ScalarType type) {
+    return t.has_value() ? optional<Tensor>(t->to(x_.device(), type).contiguous()) : t;
+  };
+  const auto pos = as(pos_, at::kLong), qw = as(qw_, at::kFloat), qb = as(qb_, at::kFloat), kw = as(kw_, at::kFloat), kb = as(kb_, at::kFloat);
+
+  // one GEMM for qkv and gate when both weights have to be cast anyway
+  const bool merged = w_qkv.scalar_type() == at::kFloat && w_gate.scalar_type() == at::kFloat && H % 4 == 0 &&
+                      b_qkv.has_value() == b_gate.has_value();
+  const int64_t P = merged ? 3 * C + 2 * H : 3 * C;          // columns of the first projection
+  // the allocation, in elements of bf16, every part 256-byte aligned
+  int64_t used = 0;
+  auto part = [&](int64_t n) {
+    const int64_t at = used;
+    used += (n + 127) & ~static_cast<int64_t>(127);
+    return at;
+  };
+  struct Cast {
+    Tensor from;
+    int64_t at;
+  };
+  std::vector<Cast> casts;
+  const bool x_wide = x_.scalar_type() == at::kFloat;
+  const int64_t at_x = x_wide ? part(M * C) : 0;
+  if (x_wide) casts.push_back({x_.contiguous(), at_x});
+  int64_t at_w = 0, at_b = 0;
+  if (merged) {
+    at_w = part(P * C);
+    casts.push_back({w_qkv.contiguous(), at_w});
+    casts.push_back({w_gate.contiguous(), at_w + 3 * C * C});
+    if (b_qkv.has_value()) {
+      at_b = part(P);
+      casts.push_back({b_qkv->contiguous(), at_b});
+      casts.push_back({b_gate->contiguous(), at_b + 3 * C});
     }
-  std::vector<Tensor> wide;
-  std::vector<size_t> where;
-  for (size_t i = 0; i < in.size(); ++i)
-    if (in[i].scalar_type() == at::kFloat) {
-      wide.push_back(in[i].contiguous());
-      where.push_back(i);
-    }
-  if (!wide.empty()) {
-    const auto narrow = cast_bf16(wide);
-    for (size_t i = 0; i < where.size(); ++i) in[where[i]] = narrow[i];
   }
-  auto bias = [&](int i) { return at_bias[i] >= 0 ? optional<Tensor>(in[at_bias[i]]) : optional<Tensor>(); };
-  const Tensor& x = in[0];
-  const int64_t B = x.size(0), N = x.size(1);
-  const Tensor qkv = at::linear(x, in[1], bias(0));
-  const Tensor gate = at::linear(x, in[2], bias(1)).sigmoid_().view({B, N, heads, 2}).permute({0, 2, 1, 3});
-  auto [q, k, v, q_c, k_c, v_c] = prologue(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
-  auto [o_c, lse, idx] = call_cmp_topk(q_c, k_c, v_c, topk, scale);
-  const Tensor y = std::get<2>(call_sel(q, k, v, idx, gate, o_c, block, scale, false, false, 1));
-  return {at::linear(y, in[3], bias(2)), idx};
+  auto narrow = [&](const Tensor& t) {                       // place of a bf16 copy, -1 where t is bf16 already
+    if (t.scalar_type() != at::kFloat) return static_cast<int64_t>(-1);
+    const int64_t at = part(t.numel());
+    casts.push_back({t.contiguous(), at});
+    return at;
+  };
+  const int64_t at_wp = narrow(w_proj), at_bp = b_proj.has_value() ? narrow(*b_proj) : -1;
+  int64_t at_wq = -1, at_bq = -1, at_wg = -1, at_bg = -1;
+  if (!merged) {
+    at_wq = narrow(w_qkv);
+    at_wg = narrow(w_gate);
+    if (b_qkv.has_value()) at_bq = narrow(*b_qkv);
+    if (b_gate.has_value()) at_bg = narrow(*b_gate);
+  }
+  const int64_t at_p = part(M * P), at_gl = merged ? 0 : part(M * 2 * H), at_tok = part(0);
+  const int64_t tok = (M * C + 127) & ~static_cast<int64_t>(127), pooled = (B * H * Nc * d + 127) & ~static_cast<int64_t>(127);
+  part(3 * tok + 4 * pooled);                                // q, k, v, q_c, k_c, v_c, o_c
+  const int64_t at_gate = merged ? part(M * 2 * H) : 0, at_y = part(M * C), at_lse = part(2 * B * H * Nc);
+  const Tensor buf = at::empty({used}, x_.options().dtype(at::kBFloat16));
+  char* base = static_cast<char*>(buf.data_ptr());
+  auto ptr = [&](int64_t at) { return static_cast<void*>(base + 2 * at); };
+  auto view = [&](int64_t at, int64_t r, int64_t c) { return buf.as_strided({r, c}, {c, 1}, at); };
+  if (!casts.empty()) {
+    TORCH_CHECK(casts.size() <= 8, "too many tensors to cast");
+    const float* src[8];
+    void* dst[8];
+    int64_t counts[8];
+    for (size_t i = 0; i < casts.size(); ++i) {
+      src[i] = f32(casts[i].from);
+      dst[i] = ptr(casts[i].at);
+      counts[i] = casts[i].from.numel();
+    }
+    check(s3r_cast_bf16(static_cast<int>(casts.size()), src, dst, counts, st), "s3r_cast_bf16");
+  }
+  auto gemm = [&](Tensor& out, const Tensor& a, const Tensor& w, const optional<Tensor>& bias) {
+    if (bias.has_value()) at::addmm_out(out, *bias, a, w.t());
+    else at::mm_out(out, a, w.t());
+  };
+  auto weight = [&](int64_t at, const Tensor& t) { return at >= 0 ? view(at, t.size(0), t.size(1)) : t; };
+  auto bias = [&](int64_t at, const optional<Tensor>& t) {
+    return t.has_value() && at >= 0 ? optional<Tensor>(buf.as_strided({t->size(0)}, {1}, at)) : t;
+  };
+  const Tensor x = x_wide ? view(at_x, M, C) : x_.contiguous().view({M, C});
+  Tensor proj = view(at_p, M, P), gate_logits;
+  if (merged) {
+    gemm(proj, x, view(at_w, P, C), b_qkv.has_value() ? optional<Tensor>(buf.as_strided({P}, {1}, at_b)) : optional<Tensor>());
+  } else {
+    gemm(proj, x, weight(at_wq, w_qkv), bias(at_bq, b_qkv));
+    gate_logits = view(at_gl, M, 2 * H);
+    gemm(gate_logits, x, weight(at_wg, w_gate), bias(at_bg, b_gate));
+    gate_logits.sigmoid_();
+  }
+  int64_t rows = 0;
+  if (pos.has_value()) {
+    TORCH_CHECK(cos.has_value() && sin.has_value() && pos->sizes() == std::vector<int64_t>({B, N, 2}), "xpos must be [B,N,2]");
+    need(*cos, "cos");
+    need(*sin, "sin");
+    rows = cos->size(0);
+  }
+  const void *cp = pos.has_value() ? cos->data_ptr() : nullptr, *sp = pos.has_value() ? sin->data_ptr() : nullptr;
+  const int64_t* pp = static_cast<const int64_t*>(ptr_or_null(pos));
+  void* t[7];                                                // q, k, v, q_c, k_c, v_c, o_c
+  for (int i = 0; i < 7; ++i) t[i] = ptr(at_tok + (i < 3 ? i * tok : 3 * tok + (i - 3) * pooled));
+  if (merged)
+    check(s3r_qkv_gate_prologue_fwd(ptr(at_p), pp, cp, sp, rows, f32_or_null(qw), f32_or_null(qb), f32_or_null(kw), f32_or_null(kb),
+                                    eps, t[0], t[1], t[2], t[3], t[4], t[5], ptr(at_gate), B, H, N, d, block, st),
+          "s3r_qkv_gate_prologue_fwd");
+  else
+    check(s3r_qkv_prologue_fwd(ptr(at_p), pp, cp, sp, rows, f32_or_null(qw), f32_or_null(qb), f32_or_null(kw), f32_or_null(kb), eps,
+                               t[0], t[1], t[2], t[3], t[4], t[5], B, H, N, d, block, st), "s3r_qkv_prologue_fwd");
+  const Tensor idx = at::empty({B, H, Nc, topk}, x_.options().dtype(at::kInt));
+  check(s3r_cmp_attn_topk_fwd(t[3], t[4], t[5], t[6], static_cast<float*>(ptr(at_lse)), i32m(idx), B, H, Nc, Nc, d, topk, scale, st),
+        "s3r_cmp_attn_topk_fwd");
+  // gate [B,H,N,2] from the prologue, or a view of the [B,N,H,2] logits
+  check(s3r_sel_attn_fwd(t[0], t[1], t[2], 1, 0, i32(idx), nullptr, nullptr, merged ? ptr(at_gate) : ptr(at_gl),
+                         merged ? H * N * 2 : N * H * 2, merged ? N * 2 : 2, merged ? 2 : H * 2, t[6], ptr(at_y), B, H, N, N, d, block,
+                         topk, scale, st), "s3r_sel_attn_fwd");
+  Tensor out = at::empty({M, w_proj.size(0)}, x_.options().dtype(at::kBFloat16));
+  gemm(out, view(at_y, M, C), weight(at_wp, w_proj), bias(at_bp, b_proj));
+  return {out.view({B, N, w_proj.size(0)}), idx};
 }
 
 // The whole op.  group = 0 where compressed keys are the selection blocks.  As one node its backward adds the
