@@ -288,6 +288,11 @@ int s3r_peer_pull(const void* const* src, void* const* dst, const int64_t* bytes
  * every tensor 16-byte aligned. */
 int s3r_cast_bf16(int n, const float* const* src, void* const* dst, const int64_t* counts, void* stream);
 
+/* out[c] = sum over rows of x[rows, cols] (bf16, fp32 accumulation, fixed order): the bias gradient of a Linear whose output
+ * gradient is x.  cols a multiple of 8; workspace of s3r_colsum_workspace_bytes bytes. */
+size_t s3r_colsum_workspace_bytes(int64_t rows, int cols);
+int s3r_colsum(const void* x, float* out, int64_t rows, int cols, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Strided copy between host and device (rows of `width_bytes` at the two pitches) on `stream`:
  * cudaMemcpy2DAsync with the direction inferred from the pointers.  No counterpart in the reference;
  * the pinned-host pipeline uses it to place one head group's columns of y [B,T,H*d] in the caller's

@@ -41,6 +41,8 @@ SIGNATURES = {
     "s3r_sel_attn_bwd": (_i, [_p] * 12 + [_i, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_sel_attn_bwd_pooled": (_i, [_p] * 15 + [_i] * 11 + [_f, _p]),
     "s3r_cast_bf16": (_i, [_i, _p, _p, _p, _p]),
+    "s3r_colsum_workspace_bytes": (_sz, [_i64, _i]),
+    "s3r_colsum": (_i, [_p, _p, _i64, _i, _p, _sz, _p]),
     "s3r_copy2d_async": (_i, [_p, _sz, _p, _sz, _sz, _sz, _p]),
     "s3r_peer_pull": (_i, [_p, _p, _p, _i, _i, _p]),
     "s3r_ipc_export": (_i, [_p, _p, C.POINTER(C.c_int64)]),

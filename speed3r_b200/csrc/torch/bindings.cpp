@@ -554,7 +554,7 @@ SixTensors prologue(const Tensor& qkv, int64_t heads, int64_t block, const optio
 // The whole attention module without gradients: projections (cuBLAS), prologue, the two attentions, output projection.
 // fp32 input and parameters are rounded to bf16 as under autocast, all in one launch, with the weights of qkv and gate side
 // by side so that one GEMM does both; everything between the GEMMs lives in one allocation and goes straight to the C ABI:
-// at 2048 tokens the call is bound by host work (388 us at first, 178 with an operator for every step, TIME_HOST so).
+// at 2048 tokens the call is bound by host work (388 us at first, 178 with an operator for every step, 105 so).
 std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, const optional<Tensor>& b_qkv, const Tensor& w_gate,
                                         const optional<Tensor>& b_gate, const Tensor& w_proj, const optional<Tensor>& b_proj,
                                         const optional<Tensor>& pos_, const optional<Tensor>& cos, const optional<Tensor>& sin,
@@ -684,6 +684,217 @@ std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, c
   return {out.view({B, N, w_proj.size(0)}), idx};
 }
 
+// The module with gradients as one node, for fp32 parameters under bf16 autocast.  The forward is that of module_infer (one
+// cast, one GEMM for qkv and gate) and keeps its one allocation for the backward; the backward runs the GEMMs with fp32
+// results where a parameter or input is fp32 (nothing is rounded to bf16 and cast back) and everything between them
+// through the C ABI.  As separate nodes a step at 2 x 6144 tokens enqueued for 1.1 ms, as long as the GPU worked on it.
+struct ModulePlan {                                          // places in the forward's allocation, elements of bf16
+  int64_t B, N, C, H, d, M, P, Nc, topk, block, used = 0;
+  int64_t x, w, b, wp, bp, proj, tok, pooled, t0, gate, y, o_s, lse_c, lse_s;
+  int64_t part(int64_t n) {
+    const int64_t at = used;
+    used += (n + 127) & ~static_cast<int64_t>(127);
+    return at;
+  }
+  ModulePlan(at::IntArrayRef shape, int64_t heads, int64_t block_, int64_t topk_, bool x_wide, int64_t out_features)
+      : B(shape[0]), N(shape[1]), C(shape[2]), H(heads), d(shape[2] / heads), M(B * N), P(3 * C + 2 * H), Nc(N / block_), topk(topk_),
+        block(block_) {
+    x = x_wide ? part(M * C) : -1;
+    w = part(P * C);
+    b = part(P);
+    wp = part(out_features * C);
+    bp = part(out_features);
+    proj = part(M * P);
+    tok = (M * C + 127) & ~static_cast<int64_t>(127);
+    pooled = (B * H * Nc * d + 127) & ~static_cast<int64_t>(127);
+    t0 = part(3 * tok + 4 * pooled);                         // q, k, v, q_c, k_c, v_c, o_c
+    gate = part(M * 2 * H);
+    y = part(M * C);
+    o_s = part(M * C);
+    lse_c = part(2 * B * H * Nc);
+    lse_s = part(2 * M * H);
+  }
+  int64_t t(int i) const { return t0 + (i < 3 ? i * tok : 3 * tok + (i - 3) * pooled); }
+};
+
+struct ModuleNode : torch::autograd::Function<ModuleNode> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x_, const Tensor& w_qkv, const optional<Tensor>& b_qkv,
+                               const Tensor& w_gate, const optional<Tensor>& b_gate, const Tensor& w_proj,
+                               const optional<Tensor>& b_proj, const optional<Tensor>& pos, const optional<Tensor>& cos,
+                               const optional<Tensor>& sin, const optional<Tensor>& qw, const optional<Tensor>& qb,
+                               const optional<Tensor>& kw, const optional<Tensor>& kb, double eps, int64_t heads, int64_t block,
+                               int64_t topk, double scale) {
+    at::AutoDispatchBelowAutograd below;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    c10::cuda::CUDAGuard guard(x_.device());
+    void* st = stream();
+    const bool x_wide = x_.scalar_type() == at::kFloat;
+    const ModulePlan m(x_.sizes(), heads, block, topk, x_wide, w_proj.size(0));
+    const Tensor buf = at::empty({m.used}, x_.options().dtype(at::kBFloat16)), x = x_.contiguous();
+    char* base = static_cast<char*>(buf.data_ptr());
+    auto ptr = [&](int64_t at) { return static_cast<void*>(base + 2 * at); };
+    auto view = [&](int64_t at, int64_t r, int64_t c) { return buf.as_strided({r, c}, {c, 1}, at); };
+    std::vector<Tensor> keep;
+    const float* src[8];
+    void* dst[8];
+    int64_t counts[8];
+    int n = 0;
+    auto cast = [&](const Tensor& t, int64_t at) {
+      need(t, "parameter", at::kFloat, false);
+      keep.push_back(t.contiguous());
+      src[n] = f32(keep.back());
+      dst[n] = ptr(at);
+      counts[n++] = t.numel();
+    };
+    if (x_wide) cast(x, m.x);
+    cast(w_qkv, m.w);
+    cast(w_gate, m.w + 3 * m.C * m.C);
+    if (b_qkv.has_value()) {
+      cast(*b_qkv, m.b);
+      cast(*b_gate, m.b + 3 * m.C);
+    }
+    cast(w_proj, m.wp);
+    if (b_proj.has_value()) cast(*b_proj, m.bp);
+    check(s3r_cast_bf16(n, src, dst, counts, st), "s3r_cast_bf16");
+    auto gemm = [&](Tensor out, const Tensor& a, const Tensor& w, bool bias, int64_t at_bias) {
+      if (bias) at::addmm_out(out, buf.as_strided({w.size(0)}, {1}, at_bias), a, w.t());
+      else at::mm_out(out, a, w.t());
+    };
+    gemm(view(m.proj, m.M, m.P), x_wide ? view(m.x, m.M, m.C) : x.view({m.M, m.C}), view(m.w, m.P, m.C), b_qkv.has_value(), m.b);
+    const int64_t rows = pos.has_value() ? cos->size(0) : 0;
+    check(s3r_qkv_gate_prologue_fwd(ptr(m.proj), static_cast<const int64_t*>(ptr_or_null(pos)), pos.has_value() ? cos->data_ptr() : nullptr,
+                                    pos.has_value() ? sin->data_ptr() : nullptr, rows, f32_or_null(qw), f32_or_null(qb), f32_or_null(kw),
+                                    f32_or_null(kb), eps, ptr(m.t(0)), ptr(m.t(1)), ptr(m.t(2)), ptr(m.t(3)), ptr(m.t(4)), ptr(m.t(5)),
+                                    ptr(m.gate), m.B, m.H, m.N, m.d, block, st), "s3r_qkv_gate_prologue_fwd");
+    const Tensor idx = at::empty({m.B, m.H, m.Nc, topk}, x_.options().dtype(at::kInt));
+    check(s3r_cmp_attn_topk_fwd(ptr(m.t(3)), ptr(m.t(4)), ptr(m.t(5)), ptr(m.t(6)), static_cast<float*>(ptr(m.lse_c)), i32m(idx), m.B,
+                                m.H, m.Nc, m.Nc, m.d, topk, scale, st), "s3r_cmp_attn_topk_fwd");
+    check(s3r_sel_attn_fwd(ptr(m.t(0)), ptr(m.t(1)), ptr(m.t(2)), 1, 0, i32(idx), ptr(m.o_s), static_cast<float*>(ptr(m.lse_s)), ptr(m.gate),
+                           m.H * m.N * 2, m.N * 2, 2, ptr(m.t(6)), ptr(m.y), m.B, m.H, m.N, m.N, m.d, block, topk, scale, st),
+          "s3r_sel_attn_fwd");
+    Tensor out = at::empty({m.M, w_proj.size(0)}, x_.options().dtype(at::kBFloat16));
+    gemm(out, view(m.y, m.M, m.C), view(m.wp, w_proj.size(0), m.C), b_proj.has_value(), m.bp);
+
+    auto or_none = [](const optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); };
+    ctx->save_for_backward({buf, x_wide ? Tensor() : x, idx, or_none(pos), or_none(cos), or_none(sin), or_none(qw), or_none(kw)});
+    ctx->saved_data["shape"] = x_.sizes().vec();
+    ctx->saved_data["ints"] = std::vector<int64_t>{heads, block, topk, w_proj.size(0), b_qkv.has_value(), b_proj.has_value()};
+    ctx->saved_data["eps"] = eps;
+    ctx->saved_data["scale"] = scale;
+    ctx->mark_non_differentiable({idx});
+    return {out.view({m.B, m.N, w_proj.size(0)}), idx};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    const auto s = ctx->get_saved_variables();
+    const Tensor &buf = s[0], &idx = s[2];
+    const auto shape = ctx->saved_data["shape"].toIntVector(), ints = ctx->saved_data["ints"].toIntVector();
+    const double eps = ctx->saved_data["eps"].toDouble(), scale = ctx->saved_data["scale"].toDouble();
+    const int64_t out_features = ints[3];
+    const bool x_wide = !s[1].defined(), rope = s[3].defined(), norm = s[6].defined();
+    const ModulePlan m(shape, ints[0], ints[1], ints[2], x_wide, out_features);
+    const size_t e_gate = ints[4] ? 3 : 2, e_wp = e_gate + (ints[4] ? 2 : 1);      // edges: absent biases have none
+    c10::cuda::CUDAGuard guard(buf.device());
+    void* st = stream();
+    char* base = static_cast<char*>(buf.data_ptr());
+    auto ptr = [&](int64_t at) { return static_cast<void*>(base + 2 * at); };
+    auto view = [&](int64_t at, int64_t r, int64_t c) { return buf.as_strided({r, c}, {c, 1}, at); };
+    const Tensor dy = g[0].to(at::kBFloat16).contiguous().view({m.M, out_features});
+
+    // scratch of the backward, bytes
+    int64_t used = 0;
+    auto part = [&](int64_t bytes) {
+      const int64_t at = used;
+      used += (bytes + 255) & ~static_cast<int64_t>(255);
+      return at;
+    };
+    const int64_t BH = m.B * m.H, tok = 2 * m.M * m.C, pooled = 2 * BH * m.Nc * m.d;
+    const int64_t a_dy = part(tok), a_dos = part(tok), a_dq = part(tok), a_dk = part(tok), a_dv = part(tok), a_doc = part(pooled),
+                  a_dqc = part(pooled), a_dkc = part(pooled), a_dvc = part(pooled), a_delc = part(4 * BH * m.Nc), a_dgate = part(8 * m.M * m.H),
+                  a_dels = part(4 * m.M * m.H), a_dproj = part(2 * m.M * m.P), a_off = part(4 * BH * (m.Nc + 1)),
+                  a_qids = part(4 * BH * m.Nc * m.topk);
+    const size_t csr_bytes = s3r_csr_workspace_bytes(m.B, m.H, m.Nc, m.topk, m.Nc),
+                 pro_bytes = norm ? s3r_qkv_prologue_bwd_workspace_bytes(m.B, m.H, m.N, m.block) : 0,
+                 col_bytes = std::max(s3r_colsum_workspace_bytes(m.M, m.P), s3r_colsum_workspace_bytes(m.M, out_features));
+    const int64_t a_csr = part(csr_bytes), a_pro = part(pro_bytes), a_col = part(col_bytes);
+    const Tensor scratch = at::empty({used / 2}, buf.options());
+    char* sb = static_cast<char*>(scratch.data_ptr());
+    auto sp = [&](int64_t at) { return static_cast<void*>(sb + at); };
+    auto sf = [&](int64_t at) { return reinterpret_cast<float*>(sb + at); };
+    auto sview = [&](int64_t at, int64_t r, int64_t c) { return scratch.as_strided({r, c}, {c, 1}, at / 2); };
+
+    // output projection
+    Tensor dya = sview(a_dy, m.M, m.C);
+    at::mm_out(dya, dy, view(m.wp, out_features, m.C));
+    Tensor dwp, dbp;
+    if (ctx->needs_input_grad(e_wp)) dwp = at::mm(dy.t(), view(m.y, m.M, m.C), at::kFloat);
+    auto colsum = [&](const void* x, int64_t cols) {
+      Tensor o = at::empty({cols}, buf.options().dtype(at::kFloat));
+      check(s3r_colsum(x, f32(o), m.M, cols, sp(a_col), col_bytes, st), "s3r_colsum");
+      return o;
+    };
+    if (ints[5] && ctx->needs_input_grad(e_wp + 1)) dbp = colsum(dy.data_ptr(), out_features);
+    // merge, the two branches, prologue
+    check(s3r_merge_bwd(sp(a_dy), ptr(m.gate), m.H * m.N * 2, m.N * 2, 2, ptr(m.t(6)), ptr(m.o_s), sp(a_dos), sf(a_dgate), sp(a_doc),
+                        sf(a_dels), m.B, m.H, m.N, m.d, m.block, st), "s3r_merge_bwd");
+    check(s3r_cmp_attn_bwd(ptr(m.t(3)), ptr(m.t(4)), ptr(m.t(5)), ptr(m.t(6)), static_cast<float*>(ptr(m.lse_c)), sp(a_doc), sf(a_delc),
+                           sp(a_dqc), sp(a_dkc), sp(a_dvc), m.B, m.H, m.Nc, m.Nc, m.d, scale, st), "s3r_cmp_attn_bwd");
+    int32_t *off = static_cast<int32_t*>(sp(a_off)), *qids = static_cast<int32_t*>(sp(a_qids));
+    check(s3r_build_key_csr(i32(idx), off, qids, m.B, m.H, m.Nc, m.topk, m.Nc, sp(a_csr), csr_bytes, st), "s3r_build_key_csr");
+    check(s3r_sel_attn_bwd(ptr(m.t(0)), ptr(m.t(1)), ptr(m.t(2)), i32(idx), off, qids, static_cast<float*>(ptr(m.lse_s)), sf(a_dels),
+                           sp(a_dos), sp(a_dq), sp(a_dk), sp(a_dv), m.B, m.H, m.N, m.N, m.d, m.block, m.topk, scale, st),
+          "s3r_sel_attn_bwd");
+    const Tensor dparams = at::empty({norm ? 4 : 0, m.d}, buf.options().dtype(at::kFloat));
+    check(s3r_qkv_gate_prologue_bwd(ptr(m.proj), rope ? static_cast<const int64_t*>(s[3].data_ptr()) : nullptr,
+                                    rope ? s[4].data_ptr() : nullptr, rope ? s[5].data_ptr() : nullptr, rope ? s[4].size(0) : 0,
+                                    norm ? f32(s[6]) : nullptr, norm ? f32(s[7]) : nullptr, eps, sp(a_dq), sp(a_dk), sp(a_dv), sp(a_dqc),
+                                    sp(a_dkc), sp(a_dvc), ptr(m.gate), sf(a_dgate), sp(a_dproj), norm ? f32(dparams) : nullptr, sp(a_pro),
+                                    pro_bytes, m.B, m.H, m.N, m.d, m.block, st), "s3r_qkv_gate_prologue_bwd");
+    // first projection
+    const Tensor dproj = sview(a_dproj, m.M, m.P);
+    Tensor dx, dw_qkv, dw_gate, db_qkv, db_gate;
+    if (ctx->needs_input_grad(0)) {
+      const Tensor w = view(m.w, m.P, m.C);
+      dx = (x_wide ? at::mm(dproj, w, at::kFloat) : at::mm(dproj, w)).view(shape);
+    }
+    if (ctx->needs_input_grad(1) || ctx->needs_input_grad(e_gate)) {
+      const Tensor dw = at::mm(dproj.t(), x_wide ? view(m.x, m.M, m.C) : s[1].view({m.M, m.C}), at::kFloat);
+      dw_qkv = dw.narrow(0, 0, 3 * m.C);
+      dw_gate = dw.narrow(0, 3 * m.C, 2 * m.H);
+    }
+    if (ints[4] && (ctx->needs_input_grad(2) || ctx->needs_input_grad(e_gate + 1))) {
+      const Tensor db = colsum(sp(a_dproj), m.P);
+      db_qkv = db.narrow(0, 0, 3 * m.C);
+      db_gate = db.narrow(0, 3 * m.C, 2 * m.H);
+    }
+    auto param = [&](int i) { return norm ? dparams.select(0, i) : Tensor(); };
+    return {dx, dw_qkv, db_qkv, dw_gate, db_gate, dwp, dbp, Tensor(), Tensor(), Tensor(), param(0), param(1), param(2), param(3),
+            Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+std::tuple<Tensor, Tensor> module_train(const Tensor& x, const Tensor& w_qkv, const optional<Tensor>& b_qkv, const Tensor& w_gate,
+                                        const optional<Tensor>& b_gate, const Tensor& w_proj, const optional<Tensor>& b_proj,
+                                        const optional<Tensor>& pos_, const optional<Tensor>& cos, const optional<Tensor>& sin,
+                                        const optional<Tensor>& qw_, const optional<Tensor>& qb_, const optional<Tensor>& kw_,
+                                        const optional<Tensor>& kb_, double eps, int64_t heads, int64_t block, int64_t topk,
+                                        double scale) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 3, "x must be a CUDA tensor [B,N,C]: the speed3r_b200 kernels have no CPU path");
+  TORCH_CHECK(heads % 4 == 0 && b_qkv.has_value() == b_gate.has_value(), "module_train: heads in fours, and biases of qkv and gate together");
+  auto as = [&](const optional<Tensor>& t, at::ScalarType type) {
+    return t.has_value() ? optional<Tensor>(t->to(x.device(), type).contiguous()) : t;
+  };
+  const auto pos = as(pos_, at::kLong);
+  if (pos.has_value()) {
+    TORCH_CHECK(cos.has_value() && sin.has_value() && pos->sizes() == std::vector<int64_t>({x.size(0), x.size(1), 2}), "xpos must be [B,N,2]");
+    need(*cos, "cos");
+    need(*sin, "sin");
+  }
+  const auto r = ModuleNode::apply(x, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, pos, cos, sin, as(qw_, at::kFloat), as(qb_, at::kFloat),
+                                   as(kw_, at::kFloat), as(kb_, at::kFloat), eps, heads, block, topk, scale);
+  return {r[0], r[1]};
+}
+
 // The whole op.  group = 0 where compressed keys are the selection blocks.  As one node its backward adds the
 // pooled branch's gradients inside the selection kernels' stores: separate nodes write them out as [B,H,T,d] and add
 // two bf16 tensors three times (1.5 of 19.4 ms at 250 views).
@@ -756,6 +967,9 @@ TORCH_LIBRARY(speed3r_b200, m) {
   m.def("module_infer(Tensor x, Tensor w_qkv, Tensor? b_qkv, Tensor w_gate, Tensor? b_gate, Tensor w_proj, Tensor? b_proj, "
         "Tensor? pos, Tensor? cos, Tensor? sin, Tensor? qw, Tensor? qb, Tensor? kw, Tensor? kb, float eps, int heads, "
         "int block, int topk, float scale) -> (Tensor, Tensor)", &module_infer);
+  m.def("module_train(Tensor x, Tensor w_qkv, Tensor? b_qkv, Tensor w_gate, Tensor? b_gate, Tensor w_proj, Tensor? b_proj, "
+        "Tensor? pos, Tensor? cos, Tensor? sin, Tensor? qw, Tensor? qb, Tensor? kw, Tensor? kb, float eps, int heads, "
+        "int block, int topk, float scale) -> (Tensor, Tensor)", &module_train);
   m.def("pool_tokens(Tensor x, int kernel, int stride) -> Tensor", &pool_tokens);
   m.def("flash_attn_topk(Tensor q, Tensor k, Tensor v, int topk, float scale, int group, int take) -> (Tensor, Tensor)",
         &flash_attn_topk);

@@ -58,7 +58,7 @@ _WIDE = (torch.float32, torch.bfloat16)
 
 def _global_hooks() -> bool:
     m = nn.modules.module
-    return bool(m._global_forward_hooks or m._global_forward_pre_hooks)
+    return bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks)
 
 
 def rope_tables(rope, D: int, rows: int, device, dtype):
@@ -178,26 +178,31 @@ class SparseFlashAttentionRope(nn.Module):
             return False
         return d == 64 and N % Bs == 0 and self.num_heads <= 42
 
-    def _can_run_native(self, x, xpos, N, Bs, d) -> bool:
-        """Inference in which the whole module is one native call: plain Linear projections that nobody watches, bf16
-        (by autocast or by dtype), no dropout, no sequence partition."""
+    def _native_op(self, x, xpos, N, Bs, d):
+        """The native operator that runs the whole module, or None: plain Linear projections that nobody watches, bf16 (by
+        autocast or by dtype), no sequence partition; with gradients fp32 parameters under autocast."""
         lins = (self.qkv, self.gate[0], self.proj)
-        mods = lins + (self.gate, self.gate[1], self.q_norm, self.k_norm, self.proj_drop)
-        if (torch.is_grad_enabled() or self.seq_parallel is not None or not x.is_cuda or type(x) is not Tensor or
-                (self.training and self.proj_drop.p > 0) or type(self.gate) is not nn.Sequential or len(self.gate) != 2 or
-                type(self.gate[1]) is not nn.Sigmoid or any(type(m) is not nn.Linear for m in lins) or
-                any(m._forward_hooks or m._forward_pre_hooks for m in mods) or _global_hooks() or
-                torch.compiler.is_compiling()):
-            return False
+        mods = lins + (self.gate, self.gate[1], self.q_norm, self.k_norm)
+        if (self.seq_parallel is not None or not x.is_cuda or type(x) is not Tensor or type(self.gate) is not nn.Sequential or
+                len(self.gate) != 2 or type(self.gate[1]) is not nn.Sigmoid or any(type(m) is not nn.Linear for m in lins) or
+                any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in mods) or
+                _global_hooks() or torch.compiler.is_compiling()):
+            return None
         params = [p for m in lins for p in (m.weight, m.bias) if p is not None]
         if any(type(p) is not nn.Parameter or p.device != x.device for p in params):
-            return False
-        if torch.is_autocast_enabled("cuda"):
+            return None
+        autocast = torch.is_autocast_enabled("cuda")
+        if autocast:
             if torch.get_autocast_dtype("cuda") != torch.bfloat16 or x.dtype not in _WIDE or any(p.dtype not in _WIDE for p in params):
-                return False
+                return None
         elif x.dtype != torch.bfloat16 or any(p.dtype != torch.bfloat16 for p in params):
-            return False
-        return self._can_fuse_prologue(None, x, xpos, N, Bs, d)
+            return None
+        if self._can_fuse_prologue(None, x, xpos, N, Bs, d):
+            return ops._ops().module_infer.default
+        if (torch.is_grad_enabled() and autocast and self.num_heads % 4 == 0 and all(p.dtype == torch.float32 for p in params) and
+                (self.qkv.bias is None) == (self.gate[0].bias is None) and self._prologue_takes(xpos, N, Bs, d)):
+            return ops._ops().module_train.default
+        return None
 
     def _rope_and_norms(self, xpos, d, device, dtype):
         """(cos, sin, q_norm, k_norm) as the one-pass prologue takes them."""
@@ -210,17 +215,16 @@ class SparseFlashAttentionRope(nn.Module):
             kn = (self.k_norm.weight, self.k_norm.bias, self.k_norm.eps)
         return cos, sin, qn, kn
 
-    def _forward_native(self, x, xpos, H, d, Bs) -> Tensor:
+    def _forward_native(self, op, x, xpos, H, d, Bs) -> Tensor:
         cos, sin, qn, kn = self._rope_and_norms(xpos, d, x.device, torch.bfloat16)
         qw, qb, eps = qn if qn is not None else (None, None, 1e-5)
         kw, kb, _ = kn if kn is not None else (None, None, 0.0)
         g = self.gate[0]
-        y, idx = ops._ops().module_infer.default(x, self.qkv.weight, self.qkv.bias, g.weight, g.bias, self.proj.weight,
-                                                 self.proj.bias, xpos, cos, sin, qw, qb, kw, kb, eps, H, Bs, self.topk,
-                                                 1.0 / d ** 0.5)
+        y, idx = op(x, self.qkv.weight, self.qkv.bias, g.weight, g.bias, self.proj.weight, self.proj.bias, xpos, cos, sin,
+                    qw, qb, kw, kb, eps, H, Bs, self.topk, 1.0 / d ** 0.5)
         if self.record_idx:
             self.last_idx = idx
-        return y
+        return self.proj_drop(y)
 
     def _forward_fused(self, qkv, gate, xpos, B, N, H, d, Bs, train=False) -> Tensor:
         cos, sin, qn, kn = self._rope_and_norms(xpos, d, qkv.device, qkv.dtype)
@@ -250,8 +254,9 @@ class SparseFlashAttentionRope(nn.Module):
         H = self.num_heads
         d = C // H
         Bs = self.block_size ** 2
-        if self._can_run_native(x, xpos, N, Bs, d):
-            return self._forward_native(x, xpos, H, d, Bs)
+        op = self._native_op(x, xpos, N, Bs, d)
+        if op is not None:
+            return self._forward_native(op, x, xpos, H, d, Bs)
         qkv = self.qkv(x)
         gate = self.gate(x).view(B, N, H, 2).permute(0, 2, 1, 3)          # [B,H,N,2] view, no copy
         if qkv.dtype != torch.bfloat16:

@@ -260,11 +260,11 @@ def test_module_native_inference_matches_separate_projections(params, x_dtype, a
     xpos = torch.stack((tok // 16, tok % 16), -1)[None].expand(2, -1, -1).contiguous()
     m.record_idx = True
     with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16, enabled=autocast):
-        assert m._can_run_native(x, xpos, 512, 16, 64)
+        assert m._native_op(x, xpos, 512, 16, 64) is not None
         y = m(x, xpos=xpos)
         idx = m.last_idx
         h = m.proj.register_forward_hook(lambda *a: None)
-        assert not m._can_run_native(x, xpos, 512, 16, 64)
+        assert m._native_op(x, xpos, 512, 16, 64) is None
         y2 = m(x, xpos=xpos)
         h.remove()
     assert y.dtype == y2.dtype and y.shape == y2.shape
@@ -324,3 +324,61 @@ def test_sel_big_fwd_second_pass(block):
     ref, lse_ref = R.sel_attn(q, k, v, idx, block)
     assert_bf16_close(o, ref, "growing scores")
     assert ((lse.cpu() - lse_ref).abs() <= 1e-5 * lse_ref.abs() + 1e-3).all()
+
+
+@pytest.mark.parametrize("x_dtype,bias,norm,frozen", [(torch.float32, True, True, False), (torch.bfloat16, False, True, False),
+                                                      (torch.float32, True, False, True)])
+def test_module_native_training_matches_separate_nodes(x_dtype, bias, norm, frozen):
+    """The module as one autograd node against the same module with a hook on a projection, which keeps the projections and
+    their gradients in PyTorch (bf16 gradients cast to fp32, where the node keeps fp32)."""
+    import speed3r_b200
+    torch.manual_seed(1)
+    B, N, dim = 2, 512, 256
+    m = speed3r_b200.SparseFlashAttentionRope(dim, num_heads=4, qkv_bias=bias, proj_bias=bias, qk_norm=norm,
+                                              rope=speed3r_b200.RoPE2D(100.0)).to(DEV)
+    if not bias:
+        m.gate[0].bias = None
+    if frozen:
+        m.qkv.weight.requires_grad_(False)
+    x0 = torch.randn(B, N, dim, device=DEV, dtype=x_dtype)
+    dy = 0.1 * torch.randn(B, N, dim, device=DEV)
+    tok = torch.arange(N, device=DEV) % 256
+    xpos = torch.stack((tok // 16, tok % 16), -1)[None].expand(B, -1, -1).contiguous()
+    m.record_idx = True
+    res = []
+    for native in (True, False):
+        h = None if native else m.proj.register_forward_hook(lambda *a: None)
+        x = x0.clone().requires_grad_(True)
+        m.zero_grad(set_to_none=True)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            assert (m._native_op(x, xpos, N, 16, 64) is not None) == native
+            y = m(x, xpos=xpos)
+        y.backward(dy.to(y.dtype))
+        res.append((y.detach(), m.last_idx, x.grad, {k: p.grad for k, p in m.named_parameters()}))
+        if h:
+            h.remove()
+    (y, idx, gx, gp), (y2, idx2, gx2, gp2) = res
+    assert y.dtype == y2.dtype and gx.dtype == gx2.dtype
+    same = (idx == idx2).all(-1)
+    assert same.float().mean() > 0.98
+    assert_bf16_close(y, y2.float(), "y", max_abs=2e-2, mean_abs=1e-3)
+    rel = lambda a, b: ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-6)).item()
+    assert rel(gx, gx2) < 2e-2
+    for k in gp:
+        assert (gp[k] is None) == (gp2[k] is None), k
+        if gp[k] is not None:
+            assert gp[k].dtype == gp2[k].dtype and rel(gp[k], gp2[k]) < 2e-2, k
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (63, 264), (64, 256), (5000, 3104), (200000, 8)])
+def test_colsum(rows, cols):
+    """One row, slices with a remainder, a last group of columns that is not full."""
+    from speed3r_b200 import _lib
+    lib = _lib.load()
+    x = randn(99, rows, cols).to(DEV, torch.bfloat16)
+    out = torch.empty(cols, device=DEV)
+    n = lib.s3r_colsum_workspace_bytes(rows, cols)
+    ws = torch.empty(n, device=DEV, dtype=torch.uint8)
+    _lib.check(lib.s3r_colsum(x.data_ptr(), out.data_ptr(), rows, cols, ws.data_ptr(), n, torch.cuda.current_stream().cuda_stream), "s3r_colsum")
+    ref = x.double().sum(0)
+    assert ((out.double() - ref).abs() <= 2 ** -24 * rows * x.double().abs().sum(0) / rows * 64 + 1e-6).all()
