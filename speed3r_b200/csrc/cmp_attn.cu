@@ -1,6 +1,6 @@
 // Compression branch, forward, first of two kernels: dense attention of the pooled queries over the pooled keys, and
-// for every row a lower bound of its 32nd largest raw logit, from which the second kernel (cmp_topk.cu) picks the
-// row's best columns.
+// for every row a lower bound of its topk-th largest raw logit (RANK 0) or score of a block of four columns (RANK 1),
+// from which the second kernel (cmp_topk.cu) picks the row's best columns or blocks.
 //
 // The two jobs want different things.  Attention is bound by the exponentials (one per score, 16 per cycle and SM);
 // the top-k has to look at every score once but keeps 32 of tens of thousands, through branches that depend on the
@@ -9,10 +9,17 @@
 // Measured (16 heads, one kernel before -> this one + cmp_topk.cu): 384 x 384 99 -> 9 + 23 us, 6300 x 6300 1047 ->
 // 223 + 244 us (scores that cluster by view and patch: 1923 -> 222 + 315), 7875 x 63000 5.81 -> 2.45 + 1.69 ms.
 //
-// The bound: a row keeps the running maxima of 64 groups of columns (half of the tile of 128, piece of 16 in it and column
-// mod 8).  32 of the maxima are >= the 32nd largest of the maxima, so at least 32 logits are, and the 32nd largest logit
-// is.  About 64 ln 2 = 44 logits of a row with independent scores reach the bound, whatever the number of columns.  The
-// maxima cost half an instruction per score (three-input max) and no branch.
+// The bound: a row keeps the running maxima of 64 groups of columns (half of S, piece of 16 in it and column mod 8).  topk of
+// the maxima are >= the topk-th largest of the maxima, so at least topk logits are, and the topk-th largest logit is.  With
+// topk = 32 about 64 ln 2 = 44 logits of a row with independent scores reach the bound, whatever the number of columns.
+// The maxima cost half an instruction per score (three-input max) and no branch.
+// Large scores come in runs of keys (the patches of a view the query looks at), which one group must not hold two of: the
+// copies of whole tiles bring keys i and 64 + i to columns 16 (i / 8) + i mod 8 and 8 further, so that a group is the keys
+// equal mod 64.  With the keys in order, 63 instead of 48 logits of one row in a hundred reached the bound and one list in four
+// of the second kernel filled up (6300 x 6300, keys of a view alike: both kernels 1048 -> 425 us).
+// RANK 1: compressed keys are finer than selection blocks (windows of Lc tokens every Sc, blocks of Bs = 4 * Sc), and a block's
+// score is log2 of the sum of 2^(c * s) over its first rank_take columns.  The groups keep the largest sums of P instead,
+// 16 groups per thread for even tiles and 16 for odd ones, keys in order.
 //
 // Roles (R row tiles of 128 queries per CTA, R = 1 or 2):
 //   warp 0  TMA producer: Q tiles once, then K and V tiles of 128 keys into rings
@@ -64,17 +71,19 @@ struct AtCtl {
 struct AtParams {
   __nv_bfloat16* o;
   float* lse;
-  float* bound;                // row r's bound goes to bound[r * bound_stride]
-  int64_t bound_stride;
-  int Nq, Nc;
+  float* bound;                // row r's bound goes to bound[r * topk]
+  int Nq, Nc, topk;
+  int scattered;               // leading tiles whose keys the copies spread over the column groups (map_ks, map_vs)
+  int rank_take;               // RANK 1: columns of a block that count
   float c_scale;               // softmax scale * log2(e)
   uint32_t* status;
 };
 
-template <int R>
+template <int R, int RANK>
 __global__ void __launch_bounds__(AtCfg<R>::kThreads, 1)
 cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                const __grid_constant__ CUtensorMap map_v, const AtParams p) {
+                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_ks,
+                const __grid_constant__ CUtensorMap map_vs, const AtParams p) {
   using C = AtCfg<R>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ AtCtl ctl;
@@ -141,11 +150,15 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             const uint32_t ph = (n / C::kStages) & 1;
             if (!mbar_wait(&ctl.k_empty[s], ph ^ 1, abort_flag)) break;
             mbar_expect_tx(&ctl.k_full[s], kAtTile);
-            tma_load_3d(sbase + C::kOffK + s * kAtTile, &map_k, &ctl.k_full[s], 0, j * 128, bh);
+            const bool scattered = RANK == 0 && j < p.scattered;
+            const uint32_t dst_k = sbase + C::kOffK + s * kAtTile, dst_v = sbase + C::kOffV + s * kAtTile;
+            if (scattered) tma_load_5d(dst_k, &map_ks, &ctl.k_full[s], 0, 0, 0, j * 16, bh);
+            else tma_load_3d(dst_k, &map_k, &ctl.k_full[s], 0, j * 128, bh);
             issued = n + 1;                                                 // K of tile n is in flight
             if (!mbar_wait(&ctl.v_empty[s], ph ^ 1, abort_flag)) break;
             mbar_expect_tx(&ctl.v_full[s], kAtTile);
-            tma_load_3d(sbase + C::kOffV + s * kAtTile, &map_v, &ctl.v_full[s], 0, j * 128, bh);
+            if (scattered) tma_load_5d(dst_v, &map_vs, &ctl.v_full[s], 0, 0, 0, j * 16, bh);
+            else tma_load_3d(dst_v, &map_v, &ctl.v_full[s], 0, j * 128, bh);
           }
           if (*abort_flag) {
             // give copies already in flight a bounded chance to land before the CTA's memory is released
@@ -238,10 +251,12 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                    t_p = lane_base + C::kColP + t * 64 + half * 32;
     const float cs = p.c_scale;
     float m_used = 0.f, l = 0.f;
-    float gm[32];                               // running maxima of this half's 32 column groups, raw logits
+    float gm[32];                               // running maxima of this half's 32 groups: raw logits, or sums of P
 #pragma unroll
-    for (int i = 0; i < 32; ++i) gm[i] = -INFINITY;
+    for (int i = 0; i < 32; ++i) gm[i] = RANK ? 0.f : -INFINITY;
+    float raw = -INFINITY;                      // RANK 1: largest raw logit
     auto half_max = [&]() {
+      if (RANK) return raw;
       float m[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -266,11 +281,17 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     };
     auto take_maxima = [&](const uint32_t (&x)[16], int c) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) gm[c * 8 + i] = fmax3(gm[c * 8 + i], __uint_as_float(x[i]), __uint_as_float(x[8 + i]));
+      for (int i = 0; i < 8; ++i) {
+        if (RANK) raw = fmax3(raw, __uint_as_float(x[i]), __uint_as_float(x[8 + i]));
+        else gm[c * 8 + i] = fmax3(gm[c * 8 + i], __uint_as_float(x[i]), __uint_as_float(x[8 + i]));
+      }
     };
-    // one tile; TAIL: its columns from `left` on do not exist
-    auto tile = [&](int n, bool first, auto tail, int left) -> bool {
+    const float2 w01 = make_float2(1.f, p.rank_take > 1 ? 1.f : 0.f),
+                 w23 = make_float2(p.rank_take > 2 ? 1.f : 0.f, p.rank_take > 3 ? 1.f : 0.f);
+    // one tile; TAIL: its columns from `left` on do not exist; RANK 1: the sums go to the 16 groups of parity ODD
+    auto tile = [&](int n, bool first, auto tail, auto odd, int left) -> bool {
       constexpr bool TAIL = decltype(tail)::value;
+      constexpr int ODD = decltype(odd)::value;
       if (!mbar_wait_warp(&ctl.s_full[t], n & 1, abort_flag)) return false;
       tc_fence_after();
       uint32_t xa[16], xb[16];
@@ -284,6 +305,7 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         if (TAIL) mask(x, c, left);
         take_maxima(x, c);
         uint32_t pk[8];
+        float2 counted = make_float2(0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           float2 v = ffma2(make_float2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), cs2, nm);
@@ -294,6 +316,13 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             v.y = fast_exp2(v.y);
           }
           sum[i & 1] = fadd2(sum[i & 1], v);
+          if (RANK && (i & 1) == 0) counted = make_float2(v.x, v.y * w01.y);
+          if (RANK && (i & 1) == 1) {
+            counted = ffma2(v, w23, counted);
+            const bool exists = !TAIL || half * 64 + c * 16 + 2 * (i - 1) + p.rank_take <= left;
+            float& g = gm[ODD * 16 + c * 4 + i / 2];
+            g = fmaxf(g, exists ? counted.x + counted.y : 0.f);
+          }
           pk[i] = pack_bf16(v.x, v.y);
         }
         tmem_st8(t_p + c * 8, pk);
@@ -339,17 +368,27 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (pass == 1) {
         l = 0.f;
         m_used = both_max() * cs;
+        if (RANK) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) gm[i] = 0.f;
+        }
       }
       int n = pass * ntiles;
 #pragma unroll 1
-      for (int j = 0; j < whole && ok; ++j, ++n) ok = tile(n, j == 0, std::false_type(), 0);
-      if (ok && whole < ntiles) ok = tile(n, whole == 0, std::true_type(), p.Nc - whole * 128);
+      for (int j = 0; j < whole && ok; ++j, ++n) {
+        if (RANK && (j & 1)) ok = tile(n, false, std::false_type(), std::integral_constant<int, RANK>(), 0);
+        else ok = tile(n, j == 0, std::false_type(), std::integral_constant<int, 0>(), 0);
+      }
+      if (ok && whole < ntiles) {
+        if (RANK && (whole & 1)) ok = tile(n, false, std::true_type(), std::integral_constant<int, RANK>(), p.Nc - whole * 128);
+        else ok = tile(n, whole == 0, std::true_type(), std::integral_constant<int, 0>(), p.Nc - whole * 128);
+      }
       if (ok) ok = mbar_wait_warp(&ctl.o_full, pass & 1, abort_flag);
       if (pass == 0 && !(half_max() * cs <= m_used + 64.f)) ctl.again = 1u;
     } while (another_pass(pass++));
 
-    // epilogue: the bound (32nd largest of the row's 64 maxima: with both threads' 32 sorted, the larger of a[i] and
-    // b[31 - i] over all i are the upper 32), lse and O / l.  The K ring is free by now.
+    // epilogue: the bound (topk-th largest of the row's 64 maxima: with both threads' 32 sorted, the larger of a[i] and
+    // b[topk - 1 - i] over i < topk are the upper topk), lse and O / l.  The K ring is free by now.
     sort_desc<32>(gm);
     float* other = reinterpret_cast<float*>(smem_raw + (sbase - smem_u32(smem_raw)) + C::kOffK) + t * (32 * 128) + r;     // [slot][row]
     if (half == 1) {
@@ -362,8 +401,12 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (ok && half == 0 && row < p.Nq) {
       float bound = INFINITY;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) bound = fminf(bound, fmaxf(gm[i], other[(31 - i) * 128]));
-      p.bound[(static_cast<int64_t>(bh) * p.Nq + row) * p.bound_stride] = bound;
+      for (int i = 0; i < 32; ++i)
+        if (i < p.topk) bound = fminf(bound, fmaxf(gm[i], other[(p.topk - 1 - i) * 128]));
+      // a sum's logarithm, less what its exponentials and the second kernel's scores can differ by: 2^-20 from the
+      // exponentials, and roundings of the arguments, each below 2^-24 of their size
+      if (RANK) bound = m_used + log2f(bound) - (6.103515625e-5f + 9.5367431640625e-7f * fabsf(m_used));
+      p.bound[(static_cast<int64_t>(bh) * p.Nq + row) * p.topk] = bound;
       p.lse[static_cast<int64_t>(bh) * p.Nq + row] = (m_used + log2f(l)) * 0.6931471805599453f;
     }
     if (ok) {
@@ -390,29 +433,31 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (warp == 2) tmem_dealloc(tmem, C::kCols);
 }
 
-template <int R>
+template <int R, int RANK>
 static int launch_cmp_attn(const CmpMaps& m, const AtParams& p, int BH, cudaStream_t st) {
   using C = AtCfg<R>;
   const int64_t grid = static_cast<int64_t>(BH) * ((p.Nq + R * 128 - 1) / (R * 128));
   S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
-  S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
-  return launch(cmp_attn_kernel<R>, static_cast<unsigned>(grid), C::kThreads, C::kSmem, st, m.q, m.k, m.v, p);
+  S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<R, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
+  return launch(cmp_attn_kernel<R, RANK>, static_cast<unsigned>(grid), C::kThreads, C::kSmem, st, m.q, m.k, m.v, m.ks, m.vs, p);
 }
 
-int cmp_attn_fwd(const CmpMaps& m, void* o_c, float* lse, float* bound, int64_t bound_stride, int BH, int Nq, int Nc, float scale,
-                 uint32_t* status, cudaStream_t st) {
+int cmp_attn_fwd(const CmpMaps& m, void* o_c, float* lse, float* bound, const CmpSizes& n, float scale, uint32_t* status,
+                 cudaStream_t st) {
   AtParams p;
   p.o = static_cast<__nv_bfloat16*>(o_c);
   p.lse = lse;
   p.bound = bound;
-  p.bound_stride = bound_stride;
-  p.Nq = Nq; p.Nc = Nc;
+  p.Nq = n.Nq; p.Nc = n.Nc; p.topk = n.topk;
+  p.scattered = m.scattered;
+  p.rank_take = n.rank_take;
   p.c_scale = scale * 1.4426950408889634f;
   p.status = status;
   // One row tile per CTA while all of them fit the GPU at once (384 x 384, 16 heads: 8.7 instead of 12.2 us), two row
   // tiles sharing every K and V tile beyond that (1512 x 1512: 25 instead of 35 us).
-  if (static_cast<int64_t>(BH) * ((Nq + 127) / 128) <= sm_count()) return launch_cmp_attn<1>(m, p, BH, st);
-  return launch_cmp_attn<2>(m, p, BH, st);
+  const bool one = static_cast<int64_t>(n.BH) * ((n.Nq + 127) / 128) <= sm_count();
+  if (n.rank_take > 0) return one ? launch_cmp_attn<1, 1>(m, p, n.BH, st) : launch_cmp_attn<2, 1>(m, p, n.BH, st);
+  return one ? launch_cmp_attn<1, 0>(m, p, n.BH, st) : launch_cmp_attn<2, 0>(m, p, n.BH, st);
 }
 
 }  // namespace s3r

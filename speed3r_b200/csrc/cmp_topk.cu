@@ -1,7 +1,8 @@
-// Compression branch, forward, second of two kernels: the `topk` columns of every pooled query's largest RAW logits,
-// ordered by (logit descending, column ascending).
+// Compression branch, forward, second of two kernels: the `topk` columns of every pooled query's largest RAW logits
+// (RANK 0), ordered by (logit descending, column ascending), or the `topk` blocks of four columns (RANK 1) by
+// log2 of the sum of 2^(c * s) over a block's first rank_take columns, which needs no row normaliser.
 //
-// The first kernel (cmp_attn.cu) leaves a lower bound of each row's 32nd largest logit, so this one repeats Q K^T on
+// The first kernel (cmp_attn.cu) leaves a lower bound of each row's topk-th largest logit, so this one repeats Q K^T on
 // the tensor cores and only collects the logits that reach the bound - about 44 per row with independent scores - into
 // lists of (logit, column) pairs in shared memory, [slot][lane] so that a thread's accesses never meet another's on a
 // bank.  A row has two threads (in two warpgroups that take turns at its key tiles) and a list for each.  A list that
@@ -17,6 +18,8 @@
 // that the tensor pipe alone would need.  S of a tile is two buffers of 64 columns, each taken into registers in one go, so
 // that the next products run while a half is scanned (16 columns at a time, S held for a whole tile: 1.05 instead of
 // 0.95 ms for 15750 x 15750, 16 heads).
+// RANK 1 sums exponentials relative to the bound, three in four of them needed where a block counts three columns, and
+// only blocks that reach it get their logarithm: bound by the exponentials' unit.
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-19 scan: two row tiles of
 // 128 queries, two warpgroups each.  Tensor memory: 2 row tiles x 2 tiles x 128 columns.
 #include "common.cuh"
@@ -45,6 +48,9 @@ struct TkCtl {
 struct TkParams {
   int32_t* idx;
   int Nq, Nc, topk;
+  int pad;                     // what an empty place decodes to: the last column or block, the reference's padding
+  int n_rank, rank_take;       // RANK 1: blocks whose counted columns all exist, columns counted per block
+  float c_scale;               // RANK 1: softmax scale * log2(e)
   int vec;                     // rows of idx can be written 16 bytes at a time
   uint32_t* status;
 };
@@ -81,24 +87,35 @@ __device__ __noinline__ float tk_cut(uint2* buf, int cnt) {
   return key_to_float(sortable_key(__uint_as_float(buf[0].x)));
 }
 
-// The hits of a chunk one by one, for rows whose list may fill up: rare, and out of line so that the registers of the
-// scan are not laid out around the cuts.
+// The hits of a chunk where some list of the warp may fill up: eight columns at a time, all lists that could be cut at once
+// (one by one as each fills, a warp cut up to 32 times where neighbouring queries want the same keys).  Out of line, so that
+// the registers of the scan are not laid out around the cuts.
 struct TkChunk {
   uint32_t x[16];
 };
 __device__ __noinline__ void tk_append_checked(const TkChunk ch, uint2* buf, uint32_t col0, int& cnt, float& thr) {
 #pragma unroll 1
-  for (uint32_t i = 0; i < 16; ++i) {
-    if (!(__uint_as_float(ch.x[i]) > thr)) continue;
-    if (cnt == kTkCap) {
-      thr = tk_cut(buf, cnt);
-      cnt = 32;
-      if (!(__uint_as_float(ch.x[i]) > thr)) continue;
+  for (uint32_t h = 0; h < 16; h += 8) {
+    int n = cnt;
+#pragma unroll 1
+    for (uint32_t i = 0; i < 8; ++i) n += __uint_as_float(ch.x[h + i]) > thr;
+    if (__any_sync(0xffffffffu, n > kTkCap)) {
+      if (cnt > 32) {
+        thr = tk_cut(buf, cnt);
+        cnt = 32;
+      }
+      __syncwarp();
     }
-    buf[cnt * 32] = make_uint2(ch.x[i], col0 + i);
-    ++cnt;
+#pragma unroll 1
+    for (uint32_t i = 0; i < 8; ++i) {
+      if (__uint_as_float(ch.x[h + i]) > thr) {
+        buf[cnt * 32] = make_uint2(ch.x[h + i], col0 + h + i);
+        ++cnt;
+      }
+    }
   }
 }
+static_assert(kTkCap >= 40, "eight pairs fit into a list that has been cut");
 
 // A bitonic sequence (what a[i] = max(a[i], b[31 - i]) of two descending lists leaves: the best 32 of both), sorted.
 template <typename T>
@@ -134,6 +151,7 @@ __device__ __noinline__ void tk_exact(const uint2* la, int na, const uint2* lb, 
 }
 static_assert(kTkCap == 40, "tk_exact takes lists of up to 40, the packed words a place below 80");
 
+template <int RANK>
 __global__ void __launch_bounds__(kTkThreads, 1)
 cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const TkParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -291,6 +309,53 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         __syncwarp();
       }
     };
+    // 16 columns as four blocks
+    const float cs = p.c_scale;
+    float2 off01, off23;                         // minus the bound; columns that do not count: minus infinity
+    float cutoff;                                // roundings of the sums stay well below 1e-3 up to |bound| = 8192
+    auto set_offsets = [&](float bound) {
+      off01 = make_float2(-bound, p.rank_take > 1 ? -bound : -INFINITY);
+      off23 = make_float2(p.rank_take > 2 ? -bound : -INFINITY, p.rank_take > 3 ? -bound : -INFINITY);
+      cutoff = fabsf(bound) < 8192.f ? 0.999f : 0.f;
+    };
+    if (RANK) set_offsets(fmaxf(thr, -3.402823466e38f));
+    const bool four = p.rank_take > 3;
+    auto scan_blocks = [&](const uint32_t* x, int col0) {
+      auto f = [&](int i) { return __uint_as_float(x[i]); };
+      const float2 cs2 = make_float2(cs, cs);
+      float sum[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 a = ffma2(make_float2(f(4 * i), f(4 * i + 1)), cs2, off01), b = ffma2(make_float2(f(4 * i + 2), f(4 * i + 3)), cs2, off23);
+        sum[i] = fast_exp2(a.x) + fast_exp2(a.y) + fast_exp2(b.x);
+        if (four) sum[i] += fast_exp2(b.y);
+      }
+      if (!__any_sync(0xffffffffu, fmaxf(fmax3(sum[0], sum[1], sum[2]), sum[3]) >= cutoff)) return;
+      if (__any_sync(0xffffffffu, at + 4 * 256 > end)) {                    // cut every list that has something to lose
+        const int cnt = static_cast<int>(at - first) >> 8;
+        if (cnt > 32) {
+          thr = tk_cut(buf, cnt);
+          at = first + 32 * 256;
+          set_offsets(thr);
+        }
+        __syncwarp();
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (sum[i] >= cutoff) {
+          float a[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] = e < p.rank_take ? f(4 * i + e) * cs : -INFINITY;
+          const float m = fmaxf(fmax3(a[0], a[1], a[2]), a[3]);
+          const float r = m + fast_log2((fast_exp2(a[0] - m) + fast_exp2(a[1] - m)) + (fast_exp2(a[2] - m) + fast_exp2(a[3] - m)));
+          const int n = (col0 >> 2) + i;
+          if (n < p.n_rank && r > thr) {
+            sts64(at, __float_as_uint(r), static_cast<uint32_t>(n));
+            at += 256;
+          }
+        }
+      }
+    };
     // half h of tile j
     auto half_tile = [&](int j, int h) -> bool {
       const int b = j & 1;
@@ -315,10 +380,14 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           if (32 + i >= left) xb[i] = 0xff800000u;
         }
       }
-      scan(xa, col0);
-      scan(xa + 16, col0 + 16);
-      scan(xb, col0 + 32);
-      scan(xb + 16, col0 + 48);
+      auto go = [&](const uint32_t* x, int c) {
+        if (RANK) scan_blocks(x, c);
+        else scan(x, c);
+      };
+      go(xa, col0);
+      go(xa + 16, col0 + 16);
+      go(xb, col0 + 32);
+      go(xb + 16, col0 + 48);
       return true;
     };
     if (split) {
@@ -401,8 +470,7 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
       }
       if (ok && row < p.Nq) {
-        // an empty place decodes to column Nc-1, the reference's padding
-        auto column = [&](int i) { return a[i] != ~0u ? static_cast<int32_t>(a[i]) : p.Nc - 1; };
+        auto column = [&](int i) { return a[i] != ~0u ? static_cast<int32_t>(a[i]) : p.pad; };
         if (p.vec) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4)
@@ -422,16 +490,21 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (warp == 2) tmem_dealloc(tmem, 512);
 }
 
-int cmp_topk_fwd(const CmpMaps& m, int32_t* idx, int topk, int BH, int Nq, int Nc, uint32_t* status, cudaStream_t st) {
+int cmp_topk_fwd(const CmpMaps& m, int32_t* idx, const CmpSizes& n, float scale, uint32_t* status, cudaStream_t st) {
   TkParams p;
   p.idx = idx;
-  p.Nq = Nq; p.Nc = Nc; p.topk = topk;
-  p.vec = (topk & 3) == 0 && (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
+  p.Nq = n.Nq; p.Nc = n.Nc; p.topk = n.topk;
+  p.rank_take = n.rank_take;
+  p.n_rank = n.rank_take > 0 ? (n.Nc - n.rank_take) / 4 + 1 : 0;
+  p.pad = (n.rank_take > 0 ? p.n_rank : n.Nc) - 1;
+  p.c_scale = scale * 1.4426950408889634f;
+  p.vec = (n.topk & 3) == 0 && (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
   p.status = status;
-  const int64_t grid = static_cast<int64_t>(BH) * ((Nq + kTkRows - 1) / kTkRows);
+  const int64_t grid = static_cast<int64_t>(n.BH) * ((n.Nq + kTkRows - 1) / kTkRows);
   S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
-  S3R_CUDA(cudaFuncSetAttribute(cmp_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
-  return launch(cmp_topk_kernel, static_cast<unsigned>(grid), kTkThreads, kTkSmem, st, m.q, m.k, p);
+  auto kernel = n.rank_take > 0 ? cmp_topk_kernel<1> : cmp_topk_kernel<0>;
+  S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
+  return launch(kernel, static_cast<unsigned>(grid), kTkThreads, kTkSmem, st, m.q, m.k, p);
 }
 
 }  // namespace s3r
