@@ -327,7 +327,12 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float2 a = ffma2(make_float2(f(4 * i), f(4 * i + 1)), cs2, off01), b = ffma2(make_float2(f(4 * i + 2), f(4 * i + 3)), cs2, off23);
-        sum[i] = fast_exp2(a.x) + fast_exp2(a.y) + fast_exp2(b.x);
+        if (i) {
+          sum[i] = fast_exp2(a.x) + fast_exp2(a.y) + fast_exp2(b.x);
+        } else {
+          const float2 e = exp2_fma2(make_float2(fminf(a.x, 126.f), fminf(a.y, 126.f)));
+          sum[i] = e.x + e.y + fast_exp2(b.x);
+        }
         if (four) sum[i] += fast_exp2(b.y);
       }
       if (!__any_sync(0xffffffffu, fmaxf(fmax3(sum[0], sum[1], sum[2]), sum[3]) >= cutoff)) return;
