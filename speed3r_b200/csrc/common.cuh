@@ -246,6 +246,40 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// ---- cp.async --------------------------------------------------------------------------------
+__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+
+// ---- cluster launch control: a running CTA takes over the work of one that has not been launched yet ----
+// One thread asks; the answer (16 bytes) lands in shared memory and completes `bar`.  After an answer without a CTA none
+// may be asked for again.
+__device__ __forceinline__ void clc_request(uint4* answer, uint64_t* bar) {
+  mbar_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(smem_u32(answer)), "r"(smem_u32(bar)) : "memory");
+}
+// blockIdx.x of the CTA whose work was handed over, -1: none left
+__device__ __forceinline__ int clc_answer(const uint4* answer) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .pred p;\n\t.reg .b32 y, z, w;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, y, z, w}, r;\n\t}"
+      : "=r"(x) : "r"(smem_u32(answer)) : "memory");
+  return x;
+}
+
 // ---- TMA tiled loads (no multicast anywhere in this library) --------------------------------
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
   asm volatile(

@@ -83,14 +83,6 @@ __device__ __forceinline__ void block_rows(int* r, const int64_t* pos, int block
   if (bad && status) atomicOr(status, kStatusBadIndex);     // clamped: the result for this token is wrong
   __syncwarp();
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ Vec8 lds_vec8(uint32_t a) {
   const uint4 v = lds128(a);
   return Vec8{{v.x, v.y, v.z, v.w}};

@@ -526,26 +526,24 @@ struct SbLane {                    // this lane's ldmatrix offsets inside a swiz
   }
 };
 
-__global__ void __launch_bounds__(32, 10) sel_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_kv, const SelBwdParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ int32_t list[64];                        // first token of each valid key block, table order
-  __shared__ uint64_t full[2];
-  __shared__ uint32_t abort_word;
+struct SbShared {
+  uint4 handed;                  // the next task (cluster launch control)
+  uint64_t full[2], handed_bar;
+  float stats[2][32];            // dK/dV: [tile of the pair][lse2 x 16 | delta x 16]
+  int32_t next_off[2];           // dK/dV: ends and first entries of the next task's list
+  int32_t list[64];              // those entries; dQ: first token of each valid key block, table order
+  uint32_t abort_word;
+};
+
+// dQ of 16 rows.  `taken` pairs have gone through the ring before: a pair is its n-th, stage n & 1, phase (n >> 1) & 1.
+__device__ __forceinline__ void sel_bwd_dq(const CUtensorMap& map_kv, const SelBwdParams& p, SbShared& sh, uint32_t ring,
+                                           uint32_t task, uint32_t taken) {
   const int lane = threadIdx.x, g = lane >> 2, c = lane & 3;
-  const int nslices = (p.Tq + 15) / 16;
-  const int64_t task = blockIdx.x;
-  const int bh = static_cast<int>(task / nslices), row0 = static_cast<int>(task % nslices) * 16;
+  const uint32_t nslices = (p.Tq + 15) / 16;
+  const int bh = static_cast<int>(task / nslices), row0 = static_cast<int>(task - static_cast<uint32_t>(bh) * nslices) * 16;
   const int nrows = min(16, p.Tq - row0);
-  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  volatile uint32_t* abort_flag = &abort_word;
-  if (lane == 0) {
-    abort_word = 0;
-    mbar_init(&full[0], 1);
-    mbar_init(&full[1], 1);
-    mbar_fence_init();
-  }
-  griddep_wait();
-  griddep_launch();
+  volatile uint32_t* abort_flag = &sh.abort_word;
+  int32_t* list = sh.list;
   int nvalid = 0;
   {
     const int32_t* row = p.idx + (static_cast<int64_t>(bh) * p.nqb + (row0 >> (4 + p.block_shift))) * p.topk;
@@ -564,13 +562,13 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_dq_kernel(const __grid_constan
   auto issue = [&](int pair, int s) {
     if (lane == 0) {
       const int t = 2 * pair;
-      mbar_expect_tx(&full[s], (t + 1 < ntiles ? 8192u : 4096u) >> (p.first_kv < 0));
-      tma_load_5d(ring + s * kSbStageBytes, &map_kv, &full[s], 0, tok_of(t), bh, 0, 0);
-      if (t + 1 < ntiles) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_kv, &full[s], 0, tok_of(t + 1), bh, 0, 0);
+      mbar_expect_tx(&sh.full[s], (t + 1 < ntiles ? 8192u : 4096u) >> (p.first_kv < 0));
+      tma_load_5d(ring + s * kSbStageBytes, &map_kv, &sh.full[s], 0, tok_of(t), bh, 0, 0);
+      if (t + 1 < ntiles) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_kv, &sh.full[s], 0, tok_of(t + 1), bh, 0, 0);
     }
   };
-  if (npairs > 0) issue(0, 0);
-  if (npairs > 1) issue(1, 1);
+  if (npairs > 0) issue(0, taken & 1);
+  if (npairs > 1) issue(1, (taken + 1) & 1);
 
   uint32_t qf[4][4], dof[4][4];
   ldg_a_frags(qf, p.q + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, nrows, lane);
@@ -588,11 +586,11 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_dq_kernel(const __grid_constan
 
   float dq[8][4] = {};
 #pragma unroll 1
-  for (int it = 0; it < npairs; ++it) {
-    const int S = it & 1;
-    if (!mbar_wait_warp(&full[S], (it >> 1) & 1, abort_flag)) {
+  for (int it = 0; it < npairs; ++it, ++taken) {
+    const int S = taken & 1;
+    if (!mbar_wait_warp(&sh.full[S], (taken >> 1) & 1, abort_flag)) {
       volatile uint32_t dummy = 0;                    // a last bounded chance for the other stage's copies to land
-      if (it + 1 < npairs) mbar_wait(&full[S ^ 1], ((it + 1) >> 1) & 1, &dummy);
+      if (it + 1 < npairs) mbar_wait(&sh.full[S ^ 1], ((taken + 1) >> 1) & 1, &dummy);
       if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
       return;
     }
@@ -645,36 +643,41 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_dq_kernel(const __grid_constan
 
 // The list of query blocks that selected this warp's key block comes 32 entries at a time into a register per
 // lane, the statistics of a tile's rows one load ahead of their use.
-__global__ void __launch_bounds__(32, 10) sel_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap map_qdo, const SelBwdParams p) {
+// A warp that has finished its rows takes over the rows of a CTA that has not started (cluster launch control) and has asked
+// for them, their list and their first copies before it is done with its own: lists differ in length by a factor of
+// five, and CTAs that came and went left a fifth of the warps' places empty (9.6 of 12 per SM).
+// Tasks: first all of dK/dV, then all of dQ, whose lists are of one length; a warp that is handed one of those is done after it.
+// (As two kernels the second could not start before the longest lists of the first had been worked off.)
+__global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__ CUtensorMap map_qdo,
+                                                         const __grid_constant__ CUtensorMap map_kv, const SelBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) float stats[2][32];         // [tile of the pair][lse2 x 16 | delta x 16]
-  __shared__ uint64_t full[2];
-  __shared__ uint32_t abort_word;
+  __shared__ __align__(16) SbShared sh;
   const int lane = threadIdx.x, c = lane & 3;
-  const int nslices = (p.Tk + 15) / 16;
-  const int64_t task = blockIdx.x;
-  const int bh = static_cast<int>(task / nslices), row0 = static_cast<int>(task % nslices) * 16;
-  const int nrows = min(16, p.Tk - row0);
+  const uint32_t nslices = (p.Tk + 15) / 16, kv_tasks = nslices * static_cast<uint32_t>(p.B * p.H);
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  volatile uint32_t* abort_flag = &abort_word;
+  volatile uint32_t* abort_flag = &sh.abort_word;
   if (lane == 0) {
-    abort_word = 0;
-    mbar_init(&full[0], 1);
-    mbar_init(&full[1], 1);
+    sh.abort_word = 0;
+    mbar_init(&sh.full[0], 1);
+    mbar_init(&sh.full[1], 1);
+    mbar_init(&sh.handed_bar, 1);
     mbar_fence_init();
   }
   griddep_wait();
   griddep_launch();
   __syncwarp();
-  const int n = row0 >> (4 + p.block_shift);
-  const int32_t* off = p.offsets + static_cast<int64_t>(bh) * (p.nkb + 1) + n;
-  const int beg = off[0], cnt = off[1] - beg;
-  const int32_t* ql = p.qids + static_cast<int64_t>(bh) * p.nqb * p.topk + beg;
-  const int ntiles = cnt << p.block_shift, npairs = (ntiles + 1) >> 1, in_block = (1 << p.block_shift) - 1;
+  if (blockIdx.x >= kv_tasks) {
+    sel_bwd_dq(map_kv, p, sh, ring, blockIdx.x - kv_tasks, 0);
+    return;
+  }
+  const int in_block = (1 << p.block_shift) - 1;
+  const SbLane of(lane);
+  const uint32_t q_at = p.first_qdo > 0 ? 2048u : 0u, do_at = p.first_qdo == 0 ? 2048u : 0u;
+
+  int bh, row0, cnt, ntiles, npairs;
+  const int32_t* ql;
   // list entries of chunk c (32 of them) live in `q_cur`, those of chunk c+1 in `q_nxt`; called with growing t only
-  int q_chunk = 0;
-  int q_cur = (lane < cnt) ? ql[lane] : 0;
-  int q_nxt = (32 + lane < cnt) ? ql[32 + lane] : 0;
+  int q_chunk, q_cur, q_nxt;
   auto tok_of = [&](int t) {
     const int e = t >> p.block_shift;
     if ((e >> 5) != q_chunk) {                         // warp-uniform
@@ -687,102 +690,184 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_dkdv_kernel(const __grid_const
   };
   auto issue = [&](int t0, int t1, bool both, int s) {
     if (lane == 0) {
-      mbar_expect_tx(&full[s], (both ? 8192u : 4096u) >> (p.first_qdo < 0));
-      tma_load_5d(ring + s * kSbStageBytes, &map_qdo, &full[s], 0, t0, bh, 0, 0);
-      if (both) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_qdo, &full[s], 0, t1, bh, 0, 0);
+      mbar_expect_tx(&sh.full[s], (both ? 8192u : 4096u) >> (p.first_qdo < 0));
+      tma_load_5d(ring + s * kSbStageBytes, &map_qdo, &sh.full[s], 0, t0, bh, 0, 0);
+      if (both) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_qdo, &sh.full[s], 0, t1, bh, 0, 0);
     }
   };
   // lanes 0-15 fetch lse, lanes 16-31 delta of a tile's rows; a row past the end gets lse = +inf: P is exactly 0
-  const float* stat_src = (lane < 16 ? p.lse : p.delta) + static_cast<int64_t>(bh) * p.Tq;
   auto stat = [&](int tok0) {
     const int t = tok0 + (lane & 15);
-    const float x = __ldg(stat_src + min(t, p.Tq - 1));
+    const float x = __ldg((lane < 16 ? p.lse : p.delta) + static_cast<int64_t>(bh) * p.Tq + min(t, p.Tq - 1));
     return lane >= 16 ? x : (t < p.Tq ? x * 1.4426950408889634f : INFINITY);
   };
-  // tokens of the next pair to be computed (their copies are under way) and its statistics
-  int na = 0, nb = 0;
-  float sa = 0.f, sb = 0.f;
-  int ta = 0, tb = 0;
-  if (npairs > 0) {
-    na = tok_of(0);
-    nb = 1 < ntiles ? tok_of(1) : na;
-    issue(na, nb, 1 < ntiles, 0);
-    sa = stat(na);
-    sb = stat(nb);
-  }
-  if (npairs > 1) {
-    ta = tok_of(2);
-    tb = 3 < ntiles ? tok_of(3) : ta;
-    issue(ta, tb, 3 < ntiles, 1);
-  }
+  auto offsets_of = [&](uint32_t task) {
+    const uint32_t h = task / nslices, slice = task - h * nslices;
+    return p.offsets + static_cast<int64_t>(h) * (p.nkb + 1) + (slice >> p.block_shift);
+  };
+  // a pair is the ring's n-th: stage n & 1, phase (n >> 1) & 1
+  uint32_t taken = 0;
+  int na = 0, nb = 0;                                  // tokens of the next pair to be computed (its copies are under way)
+  float sa = 0.f, sb = 0.f;                            // and its statistics
   uint32_t kf[4][4], vf[4][4];
-  ldg_a_frags(kf, p.k + (static_cast<int64_t>(bh) * p.Tk + row0) * 64, nrows, lane);
-  ldg_a_frags(vf, p.v + (static_cast<int64_t>(bh) * p.Tk + row0) * 64, nrows, lane);
-  const SbLane of(lane);
-  const uint32_t q_at = p.first_qdo > 0 ? 2048u : 0u, do_at = p.first_qdo == 0 ? 2048u : 0u;
-
-  float dk[8][4] = {}, dv[8][4] = {};
+  // the task's sizes, first copies and fragments; its list's first entries are in q_cur and q_nxt
+  auto begin = [&](uint32_t task, int beg, int count) {
+    bh = static_cast<int>(task / nslices);
+    row0 = static_cast<int>(task - static_cast<uint32_t>(bh) * nslices) * 16;
+    cnt = count;
+    ql = p.qids + static_cast<int64_t>(bh) * p.nqb * p.topk + beg;
+    q_chunk = 0;
+    ntiles = cnt << p.block_shift;
+    npairs = (ntiles + 1) >> 1;
+    if (npairs > 0) {
+      na = tok_of(0);
+      nb = 1 < ntiles ? tok_of(1) : na;
+      issue(na, nb, 1 < ntiles, taken & 1);
+      sa = stat(na);
+      sb = stat(nb);
+    }
+    const int64_t at = (static_cast<int64_t>(bh) * p.Tk + row0) * 64;
+    const int nrows = min(16, p.Tk - row0);
+    ldg_a_frags(kf, p.k + at, nrows, lane);
+    ldg_a_frags(vf, p.v + at, nrows, lane);
+  };
+  {
+    const int32_t* off = offsets_of(blockIdx.x);
+    const int beg = off[0], count = off[1] - beg;
+    const int32_t* src = p.qids + static_cast<int64_t>(blockIdx.x / nslices) * p.nqb * p.topk + beg;
+    q_cur = (lane < count) ? src[lane] : 0;
+    q_nxt = (32 + lane < count) ? src[32 + lane] : 0;
+    begin(blockIdx.x, beg, count);
+  }
+  uint32_t asked = 0, answered = 0;                    // requests and answers so far
 #pragma unroll 1
-  for (int it = 0; it < npairs; ++it) {
-    const int S = it & 1;
-    stats[0][lane] = sa;
-    stats[1][lane] = sb;
-    __syncwarp();
-    if (it + 1 < npairs) { sa = stat(ta); sb = stat(tb); }
-    if (!mbar_wait_warp(&full[S], (it >> 1) & 1, abort_flag)) {
-      volatile uint32_t dummy = 0;                    // a last bounded chance for the other stage's copies to land
-      if (it + 1 < npairs) mbar_wait(&full[S ^ 1], ((it + 1) >> 1) & 1, &dummy);
+  while (true) {
+    auto request = [&]() {
+      if (lane == 0) clc_request(&sh.handed, &sh.handed_bar);
+      ++asked;
+    };
+    if (npairs <= 3) request();
+    int ta = 0, tb = 0;
+    if (npairs > 1) {
+      ta = tok_of(2);
+      tb = 3 < ntiles ? tok_of(3) : ta;
+      issue(ta, tb, 3 < ntiles, (taken + 1) & 1);
+    }
+    int next = -1;
+    bool ok = true;
+    // the next task, if there is one, and the ends of its list
+    auto learn = [&]() {
+      ok = mbar_wait_warp(&sh.handed_bar, answered++ & 1, abort_flag);
+      next = ok ? clc_answer(&sh.handed) : -1;
+      if (static_cast<uint32_t>(next) < kv_tasks && lane < 2) cp_async4(smem_u32(&sh.next_off[lane]), offsets_of(next) + lane);
+      cp_async_commit();
+    };
+    // a pair later: the first entries of its list
+    auto look = [&]() {
+      cp_async_wait<0>();
+      __syncwarp();
+      if (static_cast<uint32_t>(next) >= kv_tasks) return;          // none, or dQ
+      const int beg = sh.next_off[0], count = sh.next_off[1] - beg;
+      const int32_t* src = p.qids + static_cast<int64_t>(static_cast<uint32_t>(next) / nslices) * p.nqb * p.topk + beg;
+      if (lane < count) cp_async4(smem_u32(&sh.list[lane]), src + lane);
+      if (32 + lane < count) cp_async4(smem_u32(&sh.list[32 + lane]), src + 32 + lane);
+      cp_async_commit();
+    };
+    float dk[8][4] = {}, dv[8][4] = {};
+#pragma unroll 1
+    for (int it = 0; it < npairs; ++it, ++taken) {
+      const int S = taken & 1;
+      sh.stats[0][lane] = sa;
+      sh.stats[1][lane] = sb;
+      __syncwarp();
+      if (it + 1 < npairs) { sa = stat(ta); sb = stat(tb); }
+      ok = ok && mbar_wait_warp(&sh.full[S], (taken >> 1) & 1, abort_flag);
+      if (!ok) {
+        volatile uint32_t dummy = 0;                    // a last bounded chance for what is under way to land
+        if (it + 1 < npairs) mbar_wait(&sh.full[S ^ 1], ((taken + 1) >> 1) & 1, &dummy);
+        if (asked != answered) mbar_wait(&sh.handed_bar, answered & 1, &dummy);
+        if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+        return;
+      }
+      const uint32_t st = ring + S * kSbStageBytes;
+      // P^T and dS^T of a tile, packed as A operands
+      auto grad = [&](float (&s)[2][4], const float (&dp)[2][4], int j, uint32_t (&pa)[4], uint32_t (&da)[4]) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const float2 l2 = *reinterpret_cast<const float2*>(&sh.stats[j][nt * 8 + 2 * c]);
+          const float2 d2 = *reinterpret_cast<const float2*>(&sh.stats[j][16 + nt * 8 + 2 * c]);
+          float ds[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s[nt][e] = fast_exp2(fmaf(s[nt][e], p.cs, -((e & 1) ? l2.y : l2.x)));
+            ds[e] = s[nt][e] * (dp[nt][e] - ((e & 1) ? d2.y : d2.x));
+          }
+          pa[2 * nt] = pack_bf16(s[nt][0], s[nt][1]); pa[2 * nt + 1] = pack_bf16(s[nt][2], s[nt][3]);
+          da[2 * nt] = pack_bf16(ds[0], ds[1]); da[2 * nt + 1] = pack_bf16(ds[2], ds[3]);
+        }
+      };
+      auto tile = [&](int j) {
+        uint32_t qn[4][4], dn[4][4], qk[4][4], dkk[4][4], pa[4], da[4];
+        float s[2][4], dp[2][4];
+        frags_n(qn, st + j * 4096 + q_at, of.off_n);
+        frags_n(dn, st + j * 4096 + do_at, of.off_n);
+        two_products(s, dp, kf, qn, vf, dn);
+        frags_k(dkk, st + j * 4096 + do_at, of.off_k);
+        frags_k(qk, st + j * 4096 + q_at, of.off_k);
+        grad(s, dp, j, pa, da);
+        accumulate(dv, pa, dkk);
+        accumulate(dk, da, qk);
+      };
+      tile(0);
+      if (2 * it + 1 < ntiles) tile(1);
+      __syncwarp();
+      if (it + 2 < npairs) {                            // every fragment of the stage has been consumed
+        ta = tok_of(2 * it + 4);
+        tb = 2 * it + 5 < ntiles ? tok_of(2 * it + 5) : ta;
+        issue(ta, tb, 2 * it + 5 < ntiles, S);
+      }
+      // a request takes a task from those who could start it now, so it is made no sooner than its answer is needed
+      const int left = npairs - 1 - it;
+      if (left == 3) request();
+      else if (left == 2) learn();
+      else if (left == 1 && it > 0) look();
+    }
+    if (npairs < 3) {
+      learn();
+      look();
+    }
+    if (!ok) {
       if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
       return;
     }
-    const uint32_t st = ring + S * kSbStageBytes;
-    // P^T and dS^T of a tile, packed as A operands
-    auto grad = [&](float (&s)[2][4], const float (&dp)[2][4], int j, uint32_t (&pa)[4], uint32_t (&da)[4]) {
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        const float2 l2 = *reinterpret_cast<const float2*>(&stats[j][nt * 8 + 2 * c]);
-        const float2 d2 = *reinterpret_cast<const float2*>(&stats[j][16 + nt * 8 + 2 * c]);
-        float ds[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[nt][e] = fast_exp2(fmaf(s[nt][e], p.cs, -((e & 1) ? l2.y : l2.x)));
-          ds[e] = s[nt][e] * (dp[nt][e] - ((e & 1) ? d2.y : d2.x));
-        }
-        pa[2 * nt] = pack_bf16(s[nt][0], s[nt][1]); pa[2 * nt + 1] = pack_bf16(s[nt][2], s[nt][3]);
-        da[2 * nt] = pack_bf16(ds[0], ds[1]); da[2 * nt + 1] = pack_bf16(ds[2], ds[3]);
-      }
-    };
-    auto tile = [&](int j) {
-      uint32_t qn[4][4], dn[4][4], qk[4][4], dkk[4][4], pa[4], da[4];
-      float s[2][4], dp[2][4];
-      frags_n(qn, st + j * 4096 + q_at, of.off_n);
-      frags_n(dn, st + j * 4096 + do_at, of.off_n);
-      two_products(s, dp, kf, qn, vf, dn);
-      frags_k(dkk, st + j * 4096 + do_at, of.off_k);
-      frags_k(qk, st + j * 4096 + q_at, of.off_k);
-      grad(s, dp, j, pa, da);
-      accumulate(dv, pa, dkk);
-      accumulate(dk, da, qk);
-    };
-    tile(0);
-    if (2 * it + 1 < ntiles) tile(1);
+    const int bh_done = bh, row_done = row0;
+    cp_async_wait<0>();
     __syncwarp();
-    if (it + 2 < npairs) {                            // every fragment of the stage has been consumed
-      ta = tok_of(2 * it + 4);
-      tb = 2 * it + 5 < ntiles ? tok_of(2 * it + 5) : ta;
-      issue(ta, tb, 2 * it + 5 < ntiles, S);
+    if (static_cast<uint32_t>(next) < kv_tasks) {
+      q_cur = sh.list[lane];
+      q_nxt = sh.list[32 + lane];
+      begin(next, sh.next_off[0], sh.next_off[1] - sh.next_off[0]);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int dt = 0; dt < 8; ++dt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dk[dt][e] *= p.scale;
+    add_pooled(dk, p.dk_c, bh_done, row_done, p.k_kernel, p.k_stride, p.k_windows, c);
+    add_pooled(dv, p.dv_c, bh_done, row_done, p.k_kernel, p.k_stride, p.k_windows, c);
+    const int64_t at = (static_cast<int64_t>(bh_done) * p.Tk + row_done) * 64;
+    const int nrows = min(16, p.Tk - row_done);
+    const uint32_t tile = ring + ((taken + 1) & 1) * kSbStageBytes;       // the next task's first pair is in the other stage
+    store_rows16(dk, tile, reinterpret_cast<uint8_t*>(p.dk + at), nrows, lane);
+    store_rows16(dv, tile, reinterpret_cast<uint8_t*>(p.dv + at), nrows, lane);
+    if (next < 0) return;
+    fence_proxy_async_smem();                           // copies and the next answer come after these reads and writes
+    __syncwarp();
+    if (static_cast<uint32_t>(next) >= kv_tasks) {
+      sel_bwd_dq(map_kv, p, sh, ring, static_cast<uint32_t>(next) - kv_tasks, taken);
+      return;
     }
   }
-#pragma unroll
-  for (int dt = 0; dt < 8; ++dt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) dk[dt][e] *= p.scale;
-  add_pooled(dk, p.dk_c, bh, row0, p.k_kernel, p.k_stride, p.k_windows, c);
-  add_pooled(dv, p.dv_c, bh, row0, p.k_kernel, p.k_stride, p.k_windows, c);
-  __syncwarp();
-  const int64_t at = (static_cast<int64_t>(bh) * p.Tk + row0) * 64;
-  store_rows16(dk, ring, reinterpret_cast<uint8_t*>(p.dk + at), nrows, lane);
-  store_rows16(dv, ring, reinterpret_cast<uint8_t*>(p.dv + at), nrows, lane);
 }
 
 static int grid_for(int64_t threads, int block) {
@@ -940,17 +1025,14 @@ static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_sel_attn_bwd: could not resolve the device status word");
   const int64_t bh = static_cast<int64_t>(p.B) * p.H;
   const int64_t tq = bh * ((p.Tq + 15) / 16), tk = bh * ((p.Tk + 15) / 16);
-  S3R_REQUIRE(tq < (1ll << 31) && tk < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_bwd: grid too large");
+  S3R_REQUIRE(tq + tk < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_bwd: grid too large");
   CUtensorMap mkv, mqdo;
   int rc = make_pair_map(&mkv, p.k, p.v, p.Tk, static_cast<int>(bh), 1, 0, &p.first_kv);
   if (rc) return rc;
   rc = make_pair_map(&mqdo, p.q, p.d_o, p.Tq, static_cast<int>(bh), 1, 0, &p.first_qdo);
   if (rc) return rc;
-  S3R_CUDA(cudaFuncSetAttribute(sel_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
-  S3R_CUDA(cudaFuncSetAttribute(sel_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
-  rc = launch(sel_bwd_dkdv_kernel, static_cast<unsigned>(tk), 32, kSbSmem, st, mqdo, p);
-  if (rc) return rc;
-  return launch(sel_bwd_dq_kernel, static_cast<unsigned>(tq), 32, kSbSmem, st, mkv, p);
+  S3R_CUDA(cudaFuncSetAttribute(sel_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
+  return launch(sel_bwd_kernel, static_cast<unsigned>(tk + tq), 32, kSbSmem, st, mqdo, mkv, p);
 }
 
 extern "C" int s3r_sel_attn_bwd(const void* q, const void* k, const void* v, const int32_t* idx,
