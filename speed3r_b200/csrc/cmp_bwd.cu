@@ -18,18 +18,21 @@
 // kernels at 1000 views with 128 owned rows), so a CTA owns 256 rows - as many as tensor memory holds
 // accumulators for (2 row tiles x (dK, dV) x 64 columns = 256 columns; the other 256 hold S and dP).
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warp 3 loads the
-// streamed rows' lse/delta (dK/dV kernel), warps 4-7 and 8-11 one compute warpgroup per row tile.  P and dS
-// are written in place, over the low columns of S and dP (a thread's bf16 chunk c covers columns
-// 8c..8c+7, all of which it has already read as part of fp32 chunk c/2).  A tile goes through two
-// passes per warpgroup - P from S (kept in registers as fp32), then dS from dP - each with its own
-// pair of barriers, so that the next S is being multiplied while dS is computed and the next dP while the
-// next P is.  Measured at 1000 views (Nq = Nc = 63000, 16 heads): 60 ms for both kernels, against 41 ms
-// for the same MMA sequence with the arithmetic left out and 160 ms for the mma.sync kernels they replace.
+// streamed rows' lse/delta (dK/dV), warps 4-19 compute, two warpgroups per row tile: a row has two threads, each with 32
+// of a tile's columns.  P and dS are written in place, over
+// the low half of a thread's own columns of S and dP (its bf16 chunk c covers its columns 8c..8c+7, all of which it has
+// read by then).  A tile goes through two passes per warpgroup - P from S (kept in registers as fp32), then dS from
+// dP - each with its own pair of barriers, so that the next S is being multiplied while dS is computed and the next
+// dP while the next P is.
+// Both kinds of CTA are in one grid, dK/dV first: they do not depend on each other, and a small grid of one kind leaves
+// SMs idle.
 #include "common.cuh"
 
 namespace s3r {
 
-constexpr int kCbThreads = 384;
+constexpr int kCbThreads = 640;
+// registers: the launch gives every thread 96, the utility warps hand some of theirs over (640 x 96 = 61440 >= 512 x 104 + 128 x 56)
+constexpr int kCbComputeRegs = 104, kCbUtilityRegs = 56;
 constexpr int kCbStages = 6;
 constexpr int kCbOwnRows = 256;
 constexpr int kCbOwnBytes = 128 * 128;        // 128 rows x 64 bf16
@@ -38,7 +41,7 @@ constexpr int kCbOffX = 0;                                    // row tile t: X0 
 constexpr int kCbOffY = 4 * kCbOwnBytes;                      // ring of (Y0, Y1)
 constexpr int kCbOffStat = kCbOffY + kCbStages * 2 * kCbStrBytes;   // ring of 64 x (lse2, delta)
 constexpr int kCbSmemBytes = kCbOffStat + kCbStages * 128 * 4 + 1024;
-// tensor-memory columns: row tile t holds S at 128 t and dP at 128 t + 64 (P and dS in their first 32
+// tensor-memory columns: row tile t holds S at 128 t and dP at 128 t + 64 (P and dS in the first 16 of each 32
 // columns), its accumulators at 256 + 128 t (dV) and 256 + 128 t + 64 (dK | dQ)
 constexpr uint32_t kCbColBuf = 128, kCbColDP = 64, kCbColAcc = 256, kCbColAcc1 = 64;
 
@@ -59,17 +62,14 @@ struct CbParams {
   uint32_t* status;
 };
 
-// MODE 0: dK/dV (own = K, V; streamed = Q, dO).  MODE 1: dQ (own = Q, dO; streamed = K, V).
+// MODE 0: dK/dV (own = K, V; streamed = Q, dO).  MODE 1: dQ (own = Q, dO; streamed = K, V).  `cta`: which 256 own rows.
 template <int MODE>
-__global__ void __launch_bounds__(kCbThreads, 1)
-cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant__ CUtensorMap map_x1,
-               const __grid_constant__ CUtensorMap map_y0, const __grid_constant__ CUtensorMap map_y1, const CbParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ CbCtl ctl;
+__device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUtensorMap& map_x1, const CUtensorMap& map_y0,
+                                            const CUtensorMap& map_y1, const CbParams& p, CbCtl& ctl, uint8_t* smem_raw, int cta) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int own_tiles = (p.n_own + kCbOwnRows - 1) / kCbOwnRows;
-  const int bh = blockIdx.x / own_tiles;
-  const int r0 = (blockIdx.x % own_tiles) * kCbOwnRows;
+  const int bh = cta / own_tiles;
+  const int r0 = (cta % own_tiles) * kCbOwnRows;
   const int ntiles = (p.n_str + 63) / 64;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sptr = smem_raw + (sbase - smem_u32(smem_raw));
@@ -87,8 +87,8 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
     for (int t = 0; t < 2; ++t) {
       mbar_init(&ctl.s_full[t], 1);
       mbar_init(&ctl.dp_full[t], 1);
-      mbar_init(&ctl.p_full[t], 128);
-      mbar_init(&ctl.ds_full[t], 128);
+      mbar_init(&ctl.p_full[t], 8);
+      mbar_init(&ctl.ds_full[t], 8);
     }
     mbar_fence_init();
   }
@@ -104,6 +104,8 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
+  if (warp < 4) {
+  reg_dealloc<kCbUtilityRegs>();
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -163,7 +165,7 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
         if (!ok) break;
         tc_fence_after();
         if (leader) {
-          if (MODE == 0 && i >= 1) umma_ts_k4<128>(d0, b0, y1 + (kCbStrBytes >> 4), idesc_2, i > 1 ? 1u : 0u);
+          if (MODE == 0 && i >= 1) umma_ts_k4<128, 24>(d0, b0, y1 + (kCbStrBytes >> 4), idesc_2, i > 1 ? 1u : 0u);
           if (more) {
             umma_ss_k4<2, 2>(b0, x_t0, y0, idesc_1, 0u);
             umma_commit(&ctl.s_full[0]);
@@ -178,7 +180,7 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
           }
           tc_fence_after();
           if (leader) {
-            if (i >= 2) umma_ts_k4<128>(d1 + kCbColAcc1, b1 + kCbColDP, y2, idesc_2, i > 2 ? 1u : 0u);
+            if (i >= 2) umma_ts_k4<128, 24>(d1 + kCbColAcc1, b1 + kCbColDP, y2, idesc_2, i > 2 ? 1u : 0u);
             umma_ss_k4<2, 2>(b1 + kCbColDP, x_t1 + (kCbOwnBytes >> 4), y1 + (kCbStrBytes >> 4), idesc_1, 0u);
             umma_commit(&ctl.dp_full[1]);
             if (i >= 2) umma_commit(&ctl.y_empty[st2]);
@@ -192,7 +194,7 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
         }
         tc_fence_after();
         if (leader) {
-          if (i >= 1) umma_ts_k4<128>(d0 + kCbColAcc1, b0 + kCbColDP, y1, idesc_2, i > 1 ? 1u : 0u);
+          if (i >= 1) umma_ts_k4<128, 24>(d0 + kCbColAcc1, b0 + kCbColDP, y1, idesc_2, i > 1 ? 1u : 0u);
           if (more) {
             umma_ss_k4<2, 2>(b0 + kCbColDP, x_t0 + (kCbOwnBytes >> 4), y0 + (kCbStrBytes >> 4), idesc_1, 0u);
             umma_commit(&ctl.dp_full[0]);
@@ -206,7 +208,7 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
         }
         tc_fence_after();
         if (leader) {
-          if (MODE == 0 && i >= 1) umma_ts_k4<128>(d1, b1, y1 + (kCbStrBytes >> 4), idesc_2, i > 1 ? 1u : 0u);
+          if (MODE == 0 && i >= 1) umma_ts_k4<128, 24>(d1, b1, y1 + (kCbStrBytes >> 4), idesc_2, i > 1 ? 1u : 0u);
           if (more) {
             umma_ss_k4<2, 2>(b1, x_t1, y0, idesc_1, 0u);
             umma_commit(&ctl.s_full[1]);
@@ -222,7 +224,7 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
         ok = mbar_wait_warp(&ctl.ds_full[1], (ntiles - 1) & 1, abort_flag);
         if (ok) {
           tc_fence_after();
-          if (leader) umma_ts_k4<128>(d1 + kCbColAcc1, b1 + kCbColDP, ydesc(st2), idesc_2, ntiles > 1 ? 1u : 0u);
+          if (leader) umma_ts_k4<128, 24>(d1 + kCbColAcc1, b1 + kCbColDP, ydesc(st2), idesc_2, ntiles > 1 ? 1u : 0u);
           __syncwarp();
         }
       }
@@ -252,13 +254,15 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
         if (lane == 0) mbar_arrive(&ctl.st_full[s]);
       }
     }
-  } else if (warp >= 4) {
-    // ------------------------------------------------------------------ compute, thread = owned row
-    const int t = (warp - 4) >> 2;                  // row tile of this warpgroup
+  }
+  } else {
+    // ------------------------------------------------------------------ compute, two threads per owned row
+    reg_alloc<kCbComputeRegs>();
+    const int t = (warp - 4) >> 3, half = ((warp - 4) >> 2) & 1;       // row tile and column half of this warpgroup
     const int quarter = warp & 3;
     const int row = r0 + t * 128 + quarter * 32 + lane;
     const uint32_t lane_base = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t t_s = lane_base + t * kCbColBuf, t_dp = t_s + kCbColDP;
+    const uint32_t t_s = lane_base + t * kCbColBuf + half * 32, t_dp = t_s + kCbColDP;
     const float cs = p.cs;
     float my_lse2 = INFINITY, my_delta = 0.f;       // dQ kernel: this row's statistics
     if (MODE == 1 && row < p.n_own) {
@@ -266,15 +270,20 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
       my_delta = p.delta[static_cast<int64_t>(bh) * p.Nq + row];
     }
     bool ok = true;
-    float pf[64];                                   // P of this row against the tile's 64 streamed rows
+    float pf[32];                                   // P of this row against 32 of the tile's streamed rows
+    auto arrive = [&](uint64_t* bar) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
     for (int i = 0; i < ntiles; ++i) {
       const int s = i % kCbStages;
       if (!mbar_wait_warp(&ctl.s_full[t], i & 1, abort_flag)) { ok = false; break; }
       if (MODE == 0 && !mbar_wait_warp(&ctl.st_full[s], (i / kCbStages) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      const float4* st4 = reinterpret_cast<const float4*>(stats + s * 128);
-      // pass 1: P = exp2(S c - lse), kept in registers; dK/dV kernel: bf16 P written over the low columns of S
-      // (columns 8c..8c+7 were read with chunk c/2).  Tensor-memory loads run one chunk ahead.
+      const float4* st4 = reinterpret_cast<const float4*>(stats + s * 128) + half * 8;
+      // pass 1: P = exp2(S c - lse), kept in registers; dK/dV: bf16 P written over the low columns of S.  Tensor-memory
+      // loads run one chunk ahead.
       auto pass1 = [&](const uint32_t (&xs)[16], int c) {
         uint32_t pk[8];
 #pragma unroll
@@ -321,21 +330,11 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
       tmem_ld16(t_s + 16, xb);
       pass1(xa, 0);
       tmem_ld_wait();
-      tmem_ld16(t_s + 32, xa);
+      if (MODE == 1) arrive(&ctl.p_full[t]);          // S is in registers: the next S may overwrite it
       pass1(xb, 1);
-      tmem_ld_wait();
-      tmem_ld16(t_s + 48, xb);
-      pass1(xa, 2);
-      tmem_ld_wait();
-      if (MODE == 1) {                                // S is in registers: the next S may overwrite it
-        tc_fence_before();
-        mbar_arrive(&ctl.p_full[t]);
-      }
-      pass1(xb, 3);
       if (MODE == 0) {
         tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(&ctl.p_full[t]);
+        arrive(&ctl.p_full[t]);
       }
       if (!mbar_wait_warp(&ctl.dp_full[t], i & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
@@ -344,16 +343,9 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
       tmem_ld16(t_dp + 16, xb);
       pass2(xa, 0);
       tmem_ld_wait();
-      tmem_ld16(t_dp + 32, xa);
       pass2(xb, 1);
-      tmem_ld_wait();
-      tmem_ld16(t_dp + 48, xb);
-      pass2(xa, 2);
-      tmem_ld_wait();
-      pass2(xb, 3);
       tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&ctl.ds_full[t]);
+      arrive(&ctl.ds_full[t]);
     }
     // epilogue: this row tile's accumulators -> bf16 (dK and dQ carry the softmax scale)
     if (ok) ok = mbar_wait_warp(&ctl.o_full, 0, abort_flag);
@@ -363,13 +355,12 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
       for (int a = (MODE == 0 ? 0 : 1); a < 2; ++a) {
         const float f = (a == 0) ? 1.f : p.scale;
         __nv_bfloat16* out = (a == 0 ? p.out0 : p.out1) + (static_cast<int64_t>(bh) * p.n_own + row) * 64;
-#pragma unroll 1
-        for (int hf = 0; hf < 2; ++hf) {
+        {
           uint32_t o[32];
-          tmem_ld32(lane_base + kCbColAcc + t * 128 + a * kCbColAcc1 + hf * 32, o);
+          tmem_ld32(lane_base + kCbColAcc + t * 128 + a * kCbColAcc1 + half * 32, o);
           tmem_ld_wait();
           if (row < p.n_own) {
-            uint4* dst = reinterpret_cast<uint4*>(out + hf * 32);
+            uint4* dst = reinterpret_cast<uint4*>(out + half * 32);
 #pragma unroll
             for (int v = 0; v < 4; ++v)
               dst[v] = make_uint4(pack_bf16(__uint_as_float(o[8 * v]) * f, __uint_as_float(o[8 * v + 1]) * f),
@@ -391,6 +382,19 @@ cmp_bwd_kernel(const __grid_constant__ CUtensorMap map_x0, const __grid_constant
   if (warp == 2) tmem_dealloc(tmem, 512);
 }
 
+struct CbMaps {
+  CUtensorMap q128, do128, k128, v128, q64, do64, k64, v64;
+};
+__global__ void __launch_bounds__(kCbThreads, 1)
+cmp_bwd_kernel(const __grid_constant__ CbMaps m, const CbParams kv, const CbParams q, const int kv_ctas) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ CbCtl ctl;
+  if (static_cast<int>(blockIdx.x) < kv_ctas)
+    cmp_bwd_cta<0>(m.k128, m.v128, m.q64, m.do64, kv, ctl, smem_raw, blockIdx.x);
+  else
+    cmp_bwd_cta<1>(m.q128, m.do128, m.k64, m.v64, q, ctl, smem_raw, static_cast<int>(blockIdx.x) - kv_ctas);
+}
+
 }  // namespace s3r
 
 using namespace s3r;
@@ -410,7 +414,7 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
   int rc = s3r_delta(o_c, do_c, delta, static_cast<int64_t>(B) * H * Nq, d, stream);
   if (rc) return rc;
   const int BH = B * H;
-  CUtensorMap mq128, mdo128, mk128, mv128, mq64, mdo64, mk64, mv64;
+  CbMaps m;
   {
     uint32_t box128[3] = {64, 128, 1}, box64[3] = {64, 64, 1};
     uint64_t dq_[3] = {64, static_cast<uint64_t>(Nq), static_cast<uint64_t>(BH)};
@@ -418,9 +422,9 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
     uint64_t dk_[3] = {64, static_cast<uint64_t>(Nc), static_cast<uint64_t>(BH)};
     uint64_t sk_[2] = {128, static_cast<uint64_t>(Nc) * 128};
     struct { CUtensorMap* m; const void* ptr; uint64_t* dims; uint64_t* strides; uint32_t* box; } maps[8] = {
-        {&mq128, q_c, dq_, sq_, box128}, {&mdo128, do_c, dq_, sq_, box128}, {&mk128, k_c, dk_, sk_, box128},
-        {&mv128, v_c, dk_, sk_, box128}, {&mq64, q_c, dq_, sq_, box64},     {&mdo64, do_c, dq_, sq_, box64},
-        {&mk64, k_c, dk_, sk_, box64},   {&mv64, v_c, dk_, sk_, box64}};
+        {&m.q128, q_c, dq_, sq_, box128}, {&m.do128, do_c, dq_, sq_, box128}, {&m.k128, k_c, dk_, sk_, box128},
+        {&m.v128, v_c, dk_, sk_, box128}, {&m.q64, q_c, dq_, sq_, box64},     {&m.do64, do_c, dq_, sq_, box64},
+        {&m.k64, k_c, dk_, sk_, box64},   {&m.v64, v_c, dk_, sk_, box64}};
     for (auto& e : maps) {
       rc = make_tensor_map(e.m, e.ptr, 3, e.dims, e.strides, e.box, CU_TENSOR_MAP_SWIZZLE_128B);
       if (rc) return rc;
@@ -433,20 +437,17 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
   p.scale = scale;
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_cmp_attn_bwd: could not resolve the device status word");
-  S3R_CUDA(cudaFuncSetAttribute(cmp_bwd_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCbSmemBytes));
-  S3R_CUDA(cudaFuncSetAttribute(cmp_bwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCbSmemBytes));
-  // dK, dV: own = K, V (Nc rows), streamed = Q, dO (Nq rows)
-  p.out0 = static_cast<__nv_bfloat16*>(dv_c);
-  p.out1 = static_cast<__nv_bfloat16*>(dk_c);
-  p.n_own = Nc; p.n_str = Nq;
+  S3R_CUDA(cudaFuncSetAttribute(cmp_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCbSmemBytes));
+  // dK, dV: own = K, V (Nc rows), streamed = Q, dO (Nq rows); dQ: own = Q, dO (Nq rows), streamed = K, V (Nc rows)
+  CbParams kv = p, q = p;
+  kv.out0 = static_cast<__nv_bfloat16*>(dv_c);
+  kv.out1 = static_cast<__nv_bfloat16*>(dk_c);
+  kv.n_own = Nc; kv.n_str = Nq;
+  q.out0 = nullptr;
+  q.out1 = static_cast<__nv_bfloat16*>(dq_c);
+  q.n_own = Nq; q.n_str = Nc;
   const int64_t g0 = static_cast<int64_t>(BH) * ((Nc + kCbOwnRows - 1) / kCbOwnRows),
                 g1 = static_cast<int64_t>(BH) * ((Nq + kCbOwnRows - 1) / kCbOwnRows);
-  S3R_REQUIRE(g0 < (1ll << 31) && g1 < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_bwd: grid too large");
-  rc = launch(cmp_bwd_kernel<0>, static_cast<unsigned>(g0), kCbThreads, kCbSmemBytes, st, mk128, mv128, mq64, mdo64, p);
-  if (rc) return rc;
-  // dQ: own = Q, dO (Nq rows), streamed = K, V (Nc rows)
-  p.out0 = nullptr;
-  p.out1 = static_cast<__nv_bfloat16*>(dq_c);
-  p.n_own = Nq; p.n_str = Nc;
-  return launch(cmp_bwd_kernel<1>, static_cast<unsigned>(g1), kCbThreads, kCbSmemBytes, st, mq128, mdo128, mk64, mv64, p);
+  S3R_REQUIRE(g0 + g1 < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_bwd: grid too large");
+  return launch(cmp_bwd_kernel, static_cast<unsigned>(g0 + g1), kCbThreads, kCbSmemBytes, st, m, kv, q, static_cast<int>(g0));
 }

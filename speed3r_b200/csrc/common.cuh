@@ -441,8 +441,8 @@ __device__ __forceinline__ void umma_ss_k4(uint32_t d_tmem, uint64_t a_desc, uin
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accum), "n"(A_STEP), "n"(B_STEP)
       : "memory");
 }
-// Same with A in tensor memory (bf16 pairs: 8 columns per k-step).
-template <int B_STEP>
+// Same with A in tensor memory (bf16 pairs: 8 columns per k-step; the third k-step starts A_JUMP columns after the second).
+template <int B_STEP, int A_JUMP = 8>
 __device__ __forceinline__ void umma_ts_k4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
   asm volatile(
       "{\n\t.reg .pred p, pt;\n\t.reg .b64 b;\n\t.reg .b32 a;\n\t"
@@ -450,11 +450,11 @@ __device__ __forceinline__ void umma_ts_k4(uint32_t d_tmem, uint32_t a_tmem, uin
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "add.u32 a, %1, 8;\n\tadd.s64 b, %2, %5;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n\t"
-      "add.u32 a, a, 8;\n\tadd.s64 b, b, %5;\n\t"
+      "add.u32 a, a, %6;\n\tadd.s64 b, b, %5;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n\t"
       "add.u32 a, a, 8;\n\tadd.s64 b, b, %5;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "n"(B_STEP)
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "n"(B_STEP), "n"(A_JUMP)
       : "memory");
 }
 // Arrive on an mbarrier once every tcgen05 operation issued so far by this thread has completed.
