@@ -39,7 +39,7 @@ constexpr int kCbOwnBytes = 128 * 128;        // 128 rows x 64 bf16
 constexpr int kCbStrBytes = 64 * 128;         // 64 rows x 64 bf16
 constexpr int kCbOffX = 0;                                    // row tile t: X0 at t*2*kCbOwnBytes, X1 behind it
 constexpr int kCbOffY = 4 * kCbOwnBytes;                      // ring of (Y0, Y1)
-constexpr int kCbOffStat = kCbOffY + kCbStages * 2 * kCbStrBytes;   // ring of 64 x (lse2, delta)
+constexpr int kCbOffStat = kCbOffY + kCbStages * 2 * kCbStrBytes;   // ring of 64 x (-lse2, -delta)
 constexpr int kCbSmemBytes = kCbOffStat + kCbStages * 128 * 4 + 1024;
 // tensor-memory columns: row tile t holds S at 128 t and dP at 128 t + 64 (P and dS in the first 16 of each 32
 // columns), its accumulators at 256 + 128 t (dV) and 256 + 128 t + 64 (dK | dQ)
@@ -73,7 +73,7 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
   const int ntiles = (p.n_str + 63) / 64;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sptr = smem_raw + (sbase - smem_u32(smem_raw));
-  float* stats = reinterpret_cast<float*>(sptr + kCbOffStat);        // [stage][lse2 x64 | delta x64]
+  float* stats = reinterpret_cast<float*>(sptr + kCbOffStat);        // [stage][-lse2 x64 | -delta x64]
 
   if (threadIdx.x == 0) {
     ctl.abort_flag = 0;
@@ -247,8 +247,8 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
           const int q = i * 64 + h * 32 + lane;
           const bool in = q < p.n_str;
           // rows past the end: lse = +inf makes P exactly 0
-          dst[h * 32 + lane] = in ? p.lse[static_cast<int64_t>(bh) * p.Nq + q] * 1.4426950408889634f : INFINITY;
-          dst[64 + h * 32 + lane] = in ? p.delta[static_cast<int64_t>(bh) * p.Nq + q] : 0.f;
+          dst[h * 32 + lane] = in ? -(p.lse[static_cast<int64_t>(bh) * p.Nq + q] * 1.4426950408889634f) : -INFINITY;
+          dst[64 + h * 32 + lane] = in ? -p.delta[static_cast<int64_t>(bh) * p.Nq + q] : 0.f;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl.st_full[s]);
@@ -264,10 +264,10 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
     const uint32_t lane_base = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t t_s = lane_base + t * kCbColBuf + half * 32, t_dp = t_s + kCbColDP;
     const float cs = p.cs;
-    float my_lse2 = INFINITY, my_delta = 0.f;       // dQ kernel: this row's statistics
+    float my_lse2 = -INFINITY, my_delta = 0.f;      // dQ: this row's statistics, negated
     if (MODE == 1 && row < p.n_own) {
-      my_lse2 = p.lse[static_cast<int64_t>(bh) * p.Nq + row] * 1.4426950408889634f;
-      my_delta = p.delta[static_cast<int64_t>(bh) * p.Nq + row];
+      my_lse2 = -(p.lse[static_cast<int64_t>(bh) * p.Nq + row] * 1.4426950408889634f);
+      my_delta = -p.delta[static_cast<int64_t>(bh) * p.Nq + row];
     }
     bool ok = true;
     float pf[32];                                   // P of this row against 32 of the tile's streamed rows
@@ -296,7 +296,12 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
             l4[0] = l4[1] = l4[2] = l4[3] = my_lse2;
           }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) pf[16 * c + 4 * g4 + e] = fast_exp2(fmaf(__uint_as_float(xs[4 * g4 + e]), cs, -l4[e]));
+          for (int e = 0; e < 4; e += 2) {
+            const float2 x = ffma2(make_float2(__uint_as_float(xs[4 * g4 + e]), __uint_as_float(xs[4 * g4 + e + 1])), make_float2(cs, cs),
+                             make_float2(l4[e], l4[e + 1]));
+            pf[16 * c + 4 * g4 + e] = fast_exp2(x.x);
+            pf[16 * c + 4 * g4 + e + 1] = fast_exp2(x.y);
+          }
           if (MODE == 0) {
             pk[2 * g4] = pack_bf16(pf[16 * c + 4 * g4], pf[16 * c + 4 * g4 + 1]);
             pk[2 * g4 + 1] = pack_bf16(pf[16 * c + 4 * g4 + 2], pf[16 * c + 4 * g4 + 3]);
@@ -318,7 +323,13 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
           }
           float dv[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) dv[e] = pf[16 * c + 4 * g4 + e] * (__uint_as_float(xd[4 * g4 + e]) - d4[e]);
+          for (int e = 0; e < 4; e += 2) {
+            const float2 d = fadd2(make_float2(__uint_as_float(xd[4 * g4 + e]), __uint_as_float(xd[4 * g4 + e + 1])),
+                                   make_float2(d4[e], d4[e + 1]));
+            const float2 m = fmul2(make_float2(pf[16 * c + 4 * g4 + e], pf[16 * c + 4 * g4 + e + 1]), d);
+            dv[e] = m.x;
+            dv[e + 1] = m.y;
+          }
           dk[2 * g4] = pack_bf16(dv[0], dv[1]);
           dk[2 * g4 + 1] = pack_bf16(dv[2], dv[3]);
         }
@@ -326,11 +337,10 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
       };
       uint32_t xa[16], xb[16];
       tmem_ld16(t_s, xa);
-      tmem_ld_wait();
       tmem_ld16(t_s + 16, xb);
-      pass1(xa, 0);
       tmem_ld_wait();
-      if (MODE == 1) arrive(&ctl.p_full[t]);          // S is in registers: the next S may overwrite it
+      if (MODE == 1) arrive(&ctl.p_full[t]);
+      pass1(xa, 0);
       pass1(xb, 1);
       if (MODE == 0) {
         tmem_st_wait();
@@ -339,10 +349,9 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
       if (!mbar_wait_warp(&ctl.dp_full[t], i & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       tmem_ld16(t_dp, xa);
-      tmem_ld_wait();
       tmem_ld16(t_dp + 16, xb);
-      pass2(xa, 0);
       tmem_ld_wait();
+      pass2(xa, 0);
       pass2(xb, 1);
       tmem_st_wait();
       arrive(&ctl.ds_full[t]);

@@ -117,6 +117,14 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
   return d;
 }
 
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
 // 2^x of a pair on the FMA pipe, for kernels whose exponentials saturate their own unit (16 results per cycle and SM):
 // x = n + f with n the nearest integer (the 1.5 * 2^23 shift), 2^f by a polynomial of degree 5 on [-1/2, 1/2], n added
 // to the exponent field.  The coefficients are a least-squares fit of the relative error, reweighted until it levelled

@@ -46,7 +46,6 @@ __device__ __forceinline__ float sum8(float x, uint32_t gmask) {
   return x + __shfl_xor_sync(gmask, x, 4);
 }
 __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return ffma2(a, b, splat(-0.f)); }
 __device__ __forceinline__ void unpack8(float2 (&x)[4], const Vec8& v) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) x[i] = make_float2(bf16_lo(v.w[i]), bf16_hi(v.w[i]));
