@@ -11,7 +11,9 @@
 //     call the base operators through the dispatcher, inside a C++ autograd node when a gradient is needed.
 #include <ATen/ATen.h>
 #include <ATen/core/dispatch/Dispatcher.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
@@ -200,6 +202,31 @@ std::tuple<Tensor, Tensor, Tensor> sel_attn_fwd(const Tensor& q, const Tensor& k
   return {o_s, lse, y};
 }
 
+// The table's inverse on a stream of its own, from construction to join(): it needs nothing of the backward that precedes
+// the selection branch's (31 us at 2 x 6144 tokens, as long as the merge and the compression branch take).
+struct CsrBeside {
+  c10::cuda::CUDAStream main, side;
+  at::cuda::CUDAEvent done;
+  bool joined = false;
+  CsrBeside(const int32_t* idx, int32_t* offsets, int32_t* qids, int64_t B, int64_t H, int64_t Nq, int64_t K, int64_t nkb, void* ws,
+            size_t bytes)
+      : main(c10::cuda::getCurrentCUDAStream()), side(c10::cuda::getStreamFromPool()) {
+    at::cuda::CUDAEvent start;
+    start.record(main);
+    start.block(side);
+    const int rc = s3r_build_key_csr(idx, offsets, qids, B, H, Nq, K, nkb, ws, bytes, side.stream());
+    done.record(side);
+    if (rc != 0) join();
+    check(rc, "s3r_build_key_csr");
+  }
+  void join() {
+    if (!joined) done.block(main);
+    joined = true;
+  }
+  ~CsrBeside() {
+    try { join(); } catch (...) {}
+  }
+};
 std::tuple<Tensor, Tensor> csr(const Tensor& idx, int64_t nkb, bool fill) {
   need(idx, "topk_idx", at::kInt);
   const int64_t B = idx.size(0), H = idx.size(1), Nq = idx.size(2), K = idx.size(3);
@@ -220,14 +247,14 @@ std::tuple<Tensor, Tensor> build_key_csr(const Tensor& idx, int64_t num_key_bloc
 std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
                                            const Tensor& lse, const Tensor& delta, const Tensor& do_s, const Tensor* dq_c,
                                            const Tensor* dk_c, const Tensor* dv_c, int64_t block, int64_t kernel,
-                                           int64_t stride, double scale) {
+                                           int64_t stride, double scale, const std::tuple<Tensor, Tensor>* inverse = nullptr) {
   need(q, "q");
   need(k, "k");
   need(v, "v");
   need(do_s, "do_s");
   const int64_t B = q.size(0), H = q.size(1), Tq = q.size(2), d = q.size(3), Tk = k.size(2), K = idx.size(-1);
   c10::cuda::CUDAGuard guard(q.device());
-  auto [offsets, qids] = csr(idx, (Tk + block - 1) / block, false);
+  auto [offsets, qids] = inverse ? *inverse : csr(idx, (Tk + block - 1) / block, false);
   Tensor dq = fresh_like(q), dk = fresh_like(k), dv = fresh_like(v);
   const bool fused = dq_c != nullptr && block % 16 == 0 && kernel % 16 == 0 && stride % 16 == 0;
   auto ptr = [&](const Tensor* t) -> const void* { return fused ? t->data_ptr() : nullptr; };
@@ -824,6 +851,8 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     auto sf = [&](int64_t at) { return reinterpret_cast<float*>(sb + at); };
     auto sview = [&](int64_t at, int64_t r, int64_t c) { return scratch.as_strided({r, c}, {c, 1}, at / 2); };
 
+    int32_t *off = static_cast<int32_t*>(sp(a_off)), *qids = static_cast<int32_t*>(sp(a_qids));
+    CsrBeside beside(i32(idx), off, qids, m.B, m.H, m.Nc, m.topk, m.Nc, sp(a_csr), csr_bytes);
     // output projection
     Tensor dya = sview(a_dy, m.M, m.C);
     at::mm_out(dya, dy, view(m.wp, out_features, m.C));
@@ -840,8 +869,7 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
                         sf(a_dels), m.B, m.H, m.N, m.d, m.block, st), "s3r_merge_bwd");
     check(s3r_cmp_attn_bwd(ptr(m.t(3)), ptr(m.t(4)), ptr(m.t(5)), ptr(m.t(6)), static_cast<float*>(ptr(m.lse_c)), sp(a_doc), sf(a_delc),
                            sp(a_dqc), sp(a_dkc), sp(a_dvc), m.B, m.H, m.Nc, m.Nc, m.d, scale, st), "s3r_cmp_attn_bwd");
-    int32_t *off = static_cast<int32_t*>(sp(a_off)), *qids = static_cast<int32_t*>(sp(a_qids));
-    check(s3r_build_key_csr(i32(idx), off, qids, m.B, m.H, m.Nc, m.topk, m.Nc, sp(a_csr), csr_bytes, st), "s3r_build_key_csr");
+    beside.join();
     check(s3r_sel_attn_bwd(ptr(m.t(0)), ptr(m.t(1)), ptr(m.t(2)), i32(idx), off, qids, static_cast<float*>(ptr(m.lse_s)), sf(a_dels),
                            sp(a_dos), sp(a_dq), sp(a_dk), sp(a_dv), m.B, m.H, m.N, m.N, m.d, m.block, m.topk, scale, st),
           "s3r_sel_attn_bwd");
@@ -895,6 +923,12 @@ std::tuple<Tensor, Tensor> module_train(const Tensor& x, const Tensor& w_qkv, co
   return {r[0], r[1]};
 }
 
+// a tensor with memory, not one of those that a tracer runs the backward on
+bool plain(const Tensor& t) {
+  return t.is_cuda() && !t.key_set().has(c10::DispatchKey::Python) && !t.key_set().has(c10::DispatchKey::Functionalize) &&
+         !c10::impl::dispatch_mode_enabled();
+}
+
 // The whole op.  group = 0 where compressed keys are the selection blocks.  As one node its backward adds the
 // pooled branch's gradients inside the selection kernels' stores: separate nodes write them out as [B,H,T,d] and add
 // two bf16 tensors three times (1.5 of 19.4 ms at 250 views).
@@ -918,6 +952,21 @@ struct SparseNode : torch::autograd::Function<SparseNode> {
     const auto s = ctx->get_saved_variables();
     const int64_t block = ctx->saved_data["block"].toInt();
     const double scale = ctx->saved_data["scale"].toDouble();
+    if (plain(s[0]) && plain(g[0])) {
+      c10::cuda::CUDAGuard guard(s[0].device());
+      const Tensor& idx = s[9];
+      const int64_t B = idx.size(0), H = idx.size(1), Nq = idx.size(2), K = idx.size(3), nkb = (s[1].size(2) + block - 1) / block;
+      const size_t nbytes = s3r_csr_workspace_bytes(B, H, Nq, K, nkb);
+      const std::tuple<Tensor, Tensor> inverse(fresh({B, H, nkb + 1}, idx, at::kInt), fresh({B, H, Nq * K}, idx, at::kInt));
+      const Tensor ws = fresh({static_cast<int64_t>(nbytes)}, idx, at::kByte);
+      CsrBeside beside(i32(idx), i32m(std::get<0>(inverse)), i32m(std::get<1>(inverse)), B, H, Nq, K, nkb, ws.data_ptr(), nbytes);
+      auto [do_s, dgate, do_c, dlt] = merge_bwd(g[0].contiguous(), s[3], s[7], s[10], block);
+      auto [dq_c, dk_c, dv_c] = cmp_attn_bwd(s[4], s[5], s[6], s[7], s[8], do_c, scale);
+      beside.join();
+      auto [dq, dk, dv] = sel_bwd(s[0], s[1], s[2], idx, s[11], dlt, do_s, &dq_c, &dk_c, &dv_c, block,
+                                  ctx->saved_data["kernel"].toInt(), ctx->saved_data["stride"].toInt(), scale, &inverse);
+      return {dq, dk, dv, dgate.to(s[3].scalar_type()), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
     auto [do_s, dgate, do_c, dlt] = call_merge_bwd(g[0].contiguous(), s[3], s[7], s[10], block);
     auto [dq_c, dk_c, dv_c] = call_cmp_bwd(s[4], s[5], s[6], s[7], s[8], do_c, scale);
     auto [dq, dk, dv] = call_sel_bwd_pooled(s[0], s[1], s[2], s[9], s[11], dlt, do_s, dq_c, dk_c, dv_c, block,
