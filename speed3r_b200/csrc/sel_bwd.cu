@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(256) csr_sort_long_kernel(const int32_t* __res
 
 // Short tables: one CTA builds the whole index of a (b,h) in shared memory - one launch instead of two memsets and five
 // kernels (68 us at 384 query blocks, top-32, 32 heads, most of it launches and the long-segment kernel).  The line at
-// kCsrOneEntries entries per (b,h) is where a CTA's passes over its table begin to outlast them (few CTAs: one per b,h).
+// kCsrOneEntries entries per (b,h) is where a CTA's passes over its table begin to outlast them.  Where there are more SMs
+// than (b,h), several CTAs count all of a table and each fills and sorts a range of its keys (gridDim.y of them).
 constexpr int kCsrOneEntries = 24576, kCsrOneKeys = 8192;
 
 __global__ void __launch_bounds__(1024) csr_one_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ offsets,
@@ -268,20 +269,23 @@ __global__ void __launch_bounds__(1024) csr_one_kernel(const int32_t* __restrict
     const int32_t carry = carry_s, excl = carry + (warp > 0 ? warp_sums[warp - 1] : 0) + x - v;
     if (i < Nkb) {
       cur[i] = excl;
-      off[i] = excl;
+      if (blockIdx.y == 0) off[i] = excl;
     }
     __syncthreads();
     if (tid == 1023) carry_s = carry + warp_sums[31];
     __syncthreads();
   }
-  if (tid == 0) off[Nkb] = carry_s;
+  if (tid == 0 && blockIdx.y == 0) off[Nkb] = carry_s;
+  const int per_part = (Nkb + gridDim.y - 1) / gridDim.y, lo = blockIdx.y * per_part, hi = min(Nkb, lo + per_part);
+  const int before = lo > 0 && lo < Nkb ? cur[lo] : 0;       // entries of the keys in front of this range
+  __syncthreads();
   for (int i = tid; i < per_bh; i += 1024) {
     const int n = tab[i];
-    if (n >= 0 && n < Nkb) ent[atomicAdd(&cur[n], 1)] = i / topk;
+    if (n >= lo && n < hi) ent[atomicAdd(&cur[n], 1)] = i / topk;
   }
   __syncthreads();
-  for (int n = warp; n < Nkb; n += 32) {
-    const int beg = n > 0 ? cur[n - 1] : 0, len = cur[n] - beg;
+  for (int n = lo + warp; n < hi; n += 32) {
+    const int beg = n > lo ? cur[n - 1] : before, len = cur[n] - beg;
     if (len == 0) continue;
     if (len <= 32) csr_rank_sort<1>(ent + beg, out + beg, len, lane);
     else if (len <= 64) csr_rank_sort<2>(ent + beg, out + beg, len, lane);
@@ -912,7 +916,8 @@ extern "C" int s3r_build_key_csr(const int32_t* idx, int32_t* offsets, int32_t* 
     const int smem = (Nkb + static_cast<int>(per_bh)) * static_cast<int>(sizeof(int32_t));
     S3R_CUDA(cudaFuncSetAttribute(csr_one_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (kCsrOneEntries + kCsrOneKeys) * static_cast<int>(sizeof(int32_t))));
-    return launch(csr_one_kernel, static_cast<unsigned>(bh), 1024, smem, st, idx, offsets, qids, static_cast<int>(per_bh), Nkb, topk);
+    const int64_t parts = bh < sm_count() ? sm_count() / bh : 1;
+    return launch(csr_one_kernel, dim3(static_cast<unsigned>(bh), static_cast<unsigned>(parts < 8 ? parts : 8)), 1024, smem, st, idx, offsets, qids, static_cast<int>(per_bh), Nkb, topk);
   }
   int32_t* queue = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(tmp) +
                                               ((bh * Nq * topk * sizeof(int32_t) + 255) & ~static_cast<size_t>(255)));
