@@ -15,7 +15,9 @@ the two axes on which it is independent and running three streams:
   strided copy into the group's columns of the caller's `y [1,T,H*d]`.
 
 The query chunk is sized so that one compression-attention launch fills whole waves of the GPU
-(`Hg * ceil(rows/256)` CTAs a multiple of the SM count).  Results are bit-identical to the unchunked
+(`Hg * ceil(rows/256)` CTAs a multiple of the SM count).  The last group's chunks are a quarter of the sequence at most:
+what follows the last byte in is one chunk's kernels and its copy out, and nothing else hides them (64512 tokens, 16
+heads: 8.55 -> 8.03 ms, of which 7.7 for the copies in).  Results are bit-identical to the unchunked
 call: every query row sees the same keys in the same order.
 """
 from __future__ import annotations
@@ -30,6 +32,7 @@ from . import _lib, ops
 
 _ROWS_PER_CTA = 256          # pooled query rows one compression-attention CTA owns
 _Q_BUFFERS = 4
+_GROUP_BYTES = 10 << 20      # q, k and v of a head group: about as long on the bus as the host takes to enqueue the group
 
 
 def rows_per_chunk_for(num_heads: int, sm_count: int) -> int:
@@ -71,11 +74,18 @@ class HostPipeline:
             raise RuntimeError("HostPipeline needs a CUDA device")
         self.Nc = T // block_size
         hg = heads_per_group if heads_per_group is not None else heads_per_copy
-        self.hg = max(1, min(H, hg if hg is not None else 4))
-        if rows_per_chunk is None:
+        if hg is None:
+            hg = 4
+            while hg < H and hg * T * d * 6 < _GROUP_BYTES:
+                hg *= 2
+        self.hg = max(1, min(H, hg))
+        whole_waves = rows_per_chunk is None
+        if whole_waves:
             sms = torch.cuda.get_device_properties(self.dev).multi_processor_count
             rows_per_chunk = rows_per_chunk_for(self.hg, sms)
         self.rows = max(1, min(self.Nc, rows_per_chunk))
+        quarter = -(-self.Nc // (4 * _ROWS_PER_CTA)) * _ROWS_PER_CTA
+        self.rows_last = min(self.rows, quarter) if whole_waves else self.rows
         bf = dict(device=self.dev, dtype=torch.bfloat16)
         hg = self.hg
         # two sets of group buffers: group g+1 lands while group g computes
@@ -89,7 +99,7 @@ class HostPipeline:
         self.s_in, self.s_out = torch.cuda.Stream(self.dev), torch.cuda.Stream(self.dev)
 
     def chunks(self):
-        """[(first pooled row, last pooled row + 1)] of the query chunks (the same for every head group)."""
+        """[(first pooled row, last pooled row + 1)] of the query chunks of every head group but the last."""
         return query_chunks(self.Nc, self.rows)
 
     def groups(self):
@@ -108,8 +118,18 @@ class HostPipeline:
         s_in, s_out = self.s_in, self.s_out
         s_in.wait_stream(main)            # device buffers may still be read by an earlier call
         s_out.wait_stream(main)
-        lib = _lib.load()
+        copy2d, in_stream, out_stream = _lib.load().s3r_copy2d_async, s_in.cuda_stream, s_out.cuda_stream
         esz = hy.element_size()
+        tok = d * esz                     # bytes of a token of one head
+
+        def fetch(dst: Tensor, src: Tensor, first: int, rows: int, width: int, pitch: int) -> None:
+            """``rows`` spans of ``width`` bytes, ``pitch`` apart in host memory from byte ``first`` on, to ``dst``."""
+            _lib.check(copy2d(dst.data_ptr(), width, src.data_ptr() + first, pitch, width, rows, in_stream), "s3r_copy2d_async")
+
+        def mark(stream) -> torch.cuda.Event:
+            e = torch.cuda.Event()
+            e.record(stream)
+            return e
 
         grp_free = [None, None]           # compute of the group that last used buffer set i is finished
         q_free = [None] * _Q_BUFFERS      # compute of the chunk that last used qbuf[i] is finished
@@ -117,47 +137,36 @@ class HostPipeline:
         for gi, (h0, h1) in enumerate(self.groups()):
             b, n = gi & 1, h1 - h0
             k, v, gate = (buf[b][:, :n] for buf in (self.k, self.v, self.gate))
-            with torch.cuda.stream(s_in):
-                if grp_free[b] is not None:
-                    s_in.wait_event(grp_free[b])
-                k.copy_(hk[:, h0:h1], non_blocking=True)
-                k_in = torch.cuda.Event()
-                k_in.record(s_in)
-                v.copy_(hv[:, h0:h1], non_blocking=True)
-                gate.copy_(hgate[:, h0:h1], non_blocking=True)
-                v_in = torch.cuda.Event()
-                v_in.record(s_in)
+            if grp_free[b] is not None:
+                s_in.wait_event(grp_free[b])
+            fetch(k, hk, h0 * T * tok, n, T * tok, T * tok)
+            k_in = mark(s_in)
+            fetch(v, hv, h0 * T * tok, n, T * tok, T * tok)
+            fetch(gate, hgate, h0 * T * 2 * esz, n, T * 2 * esz, T * 2 * esz)
+            v_in = mark(s_in)
             main.wait_event(k_in)
             k_c = ops.pool_tokens(k, bs, bs)                      # pooled while V is still on the bus
             main.wait_event(v_in)
             v_c = ops.pool_tokens(v, bs, bs)
             done = None
-            for r0, r1 in self.chunks():
+            for r0, r1 in (self.chunks() if h1 < H else query_chunks(self.Nc, self.rows_last)):
                 i = step % _Q_BUFFERS
                 step += 1
                 t0, t1 = r0 * bs, r1 * bs
                 q_dev = self.qbuf[i].view(-1)[:n * (t1 - t0) * d].view(1, n, t1 - t0, d)
-                with torch.cuda.stream(s_in):
-                    if q_free[i] is not None:
-                        s_in.wait_event(q_free[i])
-                    for h in range(n):                            # per head: contiguous spans on both sides
-                        q_dev[0, h].copy_(hq[0, h0 + h, t0:t1], non_blocking=True)
-                    landed = torch.cuda.Event()
-                    landed.record(s_in)
-                main.wait_event(landed)
+                if q_free[i] is not None:
+                    s_in.wait_event(q_free[i])
+                fetch(q_dev, hq, (h0 * T + t0) * tok, n, (t1 - t0) * tok, T * tok)
+                main.wait_event(mark(s_in))
                 q_c = ops.pool_tokens(q_dev, bs, bs)
                 o_c, idx = ops.flash_attn_topk_func(q_c, k_c, v_c, self.topk)
                 y = ops.sel_attn_merge(q_dev, k, v, idx, gate[:, :, t0:t1], o_c, bs)      # [1, t1-t0, n*d]
-                done = torch.cuda.Event()
-                done.record(main)
-                q_free[i] = done
+                done = q_free[i] = mark(main)
                 y.record_stream(s_out)    # the allocator must not hand y out again before it has left
-                with torch.cuda.stream(s_out):
-                    s_out.wait_event(done)
-                    # this group's columns of the rows t0..t1 of hy [1,T,H*d]
-                    _lib.check(lib.s3r_copy2d_async(hy.data_ptr() + (t0 * H * d + h0 * d) * esz, H * d * esz,
-                                                    y.data_ptr(), n * d * esz, n * d * esz, t1 - t0,
-                                                    s_out.cuda_stream), "s3r_copy2d_async")
+                s_out.wait_event(done)
+                # this group's columns of the rows t0..t1 of hy [1,T,H*d]
+                _lib.check(copy2d(hy.data_ptr() + t0 * H * tok + h0 * tok, H * tok, y.data_ptr(), n * tok, n * tok, t1 - t0,
+                                  out_stream), "s3r_copy2d_async")
             grp_free[b] = done
         main.wait_stream(s_out)
         main.wait_stream(s_in)
