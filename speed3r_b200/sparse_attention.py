@@ -61,6 +61,11 @@ def _global_hooks() -> bool:
     return bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks)
 
 
+def _watched(m: nn.Module) -> bool:
+    """Somebody's hook wants to see this module called."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
 def rope_tables(rope, D: int, rows: int, device, dtype):
     """cos/sin tables ``[rows, 2*(D/2)]`` with the reference's arithmetic (pos_embed.py:119-129: the
     angle is rounded to ``dtype`` before cos/sin).  ``rope`` is this package's ``RoPE2D`` or the
@@ -168,39 +173,60 @@ class SparseFlashAttentionRope(nn.Module):
     def _prologue_takes(self, xpos, N, Bs, d) -> bool:
         """Norms that are LayerNorm(d) with affine or Identity, a 2-D rotary module (this package's or the
         reference's pure-PyTorch one) or none, whole blocks, head counts the kernel takes."""
-        norms = (self.q_norm, self.k_norm)
-        ident = all(isinstance(m, nn.Identity) for m in norms)
-        ln = all(isinstance(m, nn.LayerNorm) and m.elementwise_affine and m.bias is not None and
-                 tuple(m.normalized_shape) == (d,) for m in norms)
-        if not (ident or (ln and self.q_norm.eps == self.k_norm.eps)):
-            return False
+        qn, kn = self._modules["q_norm"], self._modules["k_norm"]
+        if not (isinstance(qn, nn.Identity) and isinstance(kn, nn.Identity)):
+            for m in (qn, kn):
+                if not (isinstance(m, nn.LayerNorm) and m.elementwise_affine and m._parameters.get("bias") is not None and
+                        tuple(m.normalized_shape) == (d,)):
+                    return False
+            if qn.eps != kn.eps:
+                return False
         if xpos is not None and not _is_rope2d(self.rope):
             return False
         return d == 64 and N % Bs == 0 and self.num_heads <= 42
 
     def _native_op(self, x, xpos, N, Bs, d):
         """The native operator that runs the whole module, or None: plain Linear projections that nobody watches, bf16 (by
-        autocast or by dtype), no sequence partition; with gradients fp32 parameters under autocast."""
-        lins = (self.qkv, self.gate[0], self.proj)
-        mods = lins + (self.gate, self.gate[1], self.q_norm, self.k_norm)
-        if (self.seq_parallel is not None or not x.is_cuda or type(x) is not Tensor or type(self.gate) is not nn.Sequential or
-                len(self.gate) != 2 or type(self.gate[1]) is not nn.Sigmoid or any(type(m) is not nn.Linear for m in lins) or
-                any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in mods) or
-                _global_hooks() or torch.compiler.is_compiling()):
+        autocast or by dtype), no sequence partition; with gradients fp32 parameters under autocast.  Sub-modules and
+        parameters are taken from their dictionaries: nn.Module's attribute look-up was half of the 12 us this took."""
+        mods = self._modules
+        qkv, gate, proj = mods["qkv"], mods["gate"], mods["proj"]
+        if (self.seq_parallel is not None or not x.is_cuda or type(x) is not Tensor or type(gate) is not nn.Sequential or
+                len(gate._modules) != 2 or _global_hooks() or torch.compiler.is_compiling()):
             return None
-        params = [p for m in lins for p in (m.weight, m.bias) if p is not None]
-        if any(type(p) is not nn.Parameter or p.device != x.device for p in params):
+        glin, act = gate._modules.values()
+        if type(act) is not nn.Sigmoid:
             return None
+        for m in (gate, act, mods["q_norm"], mods["k_norm"]):
+            if _watched(m):
+                return None
+        dev, narrow, full = x.get_device(), 0, 0
+        for m in (qkv, glin, proj):
+            if type(m) is not nn.Linear or _watched(m):
+                return None
+            for p in m._parameters.values():
+                if p is None:
+                    continue
+                if type(p) is not nn.Parameter or p.get_device() != dev:
+                    return None
+                if p.dtype == torch.float32:
+                    full += 1
+                elif p.dtype == torch.bfloat16:
+                    narrow += 1
+                else:
+                    return None
+            if m._parameters.get("weight") is None:
+                return None
         autocast = torch.is_autocast_enabled("cuda")
         if autocast:
-            if torch.get_autocast_dtype("cuda") != torch.bfloat16 or x.dtype not in _WIDE or any(p.dtype not in _WIDE for p in params):
+            if torch.get_autocast_dtype("cuda") != torch.bfloat16 or x.dtype not in _WIDE:
                 return None
-        elif x.dtype != torch.bfloat16 or any(p.dtype != torch.bfloat16 for p in params):
+        elif x.dtype != torch.bfloat16 or full:
             return None
         if self._can_fuse_prologue(None, x, xpos, N, Bs, d):
             return ops._ops().module_infer.default
-        if (torch.is_grad_enabled() and autocast and self.num_heads % 4 == 0 and all(p.dtype == torch.float32 for p in params) and
-                (self.qkv.bias is None) == (self.gate[0].bias is None) and self._prologue_takes(xpos, N, Bs, d)):
+        if (torch.is_grad_enabled() and autocast and self.num_heads % 4 == 0 and not narrow and
+                (qkv._parameters["bias"] is None) == (glin._parameters["bias"] is None) and self._prologue_takes(xpos, N, Bs, d)):
             return ops._ops().module_train.default
         return None
 
@@ -210,21 +236,26 @@ class SparseFlashAttentionRope(nn.Module):
         if xpos is not None:
             rows = self.rope._seq_len(xpos) if isinstance(self.rope, RoPE2D) else self._rows(xpos)
             cos, sin = rope_tables(self.rope, d // 2, rows, device, dtype)
-        if isinstance(self.q_norm, nn.LayerNorm):
-            qn = (self.q_norm.weight, self.q_norm.bias, self.q_norm.eps)
-            kn = (self.k_norm.weight, self.k_norm.bias, self.k_norm.eps)
+        q_norm, k_norm = self._modules["q_norm"], self._modules["k_norm"]
+        if isinstance(q_norm, nn.LayerNorm):
+            qn = (q_norm.weight, q_norm.bias, q_norm.eps)
+            kn = (k_norm.weight, k_norm.bias, k_norm.eps)
         return cos, sin, qn, kn
 
     def _forward_native(self, op, x, xpos, H, d, Bs) -> Tensor:
         cos, sin, qn, kn = self._rope_and_norms(xpos, d, x.device, torch.bfloat16)
         qw, qb, eps = qn if qn is not None else (None, None, 1e-5)
         kw, kb, _ = kn if kn is not None else (None, None, 0.0)
-        g = self.gate[0]
-        y, idx = op(x, self.qkv.weight, self.qkv.bias, g.weight, g.bias, self.proj.weight, self.proj.bias, xpos, cos, sin,
+        mods = self._modules
+        qkv, g, proj = mods["qkv"]._parameters, next(iter(mods["gate"]._modules.values()))._parameters, mods["proj"]._parameters
+        y, idx = op(x, qkv["weight"], qkv["bias"], g["weight"], g["bias"], proj["weight"], proj["bias"], xpos, cos, sin,
                     qw, qb, kw, kb, eps, H, Bs, self.topk, 1.0 / d ** 0.5)
         if self.record_idx:
             self.last_idx = idx
-        return self.proj_drop(y)
+        drop = mods["proj_drop"]
+        if type(drop) is nn.Dropout and not _watched(drop) and (drop.p == 0.0 or not drop.training):
+            return y
+        return drop(y)
 
     def _forward_fused(self, qkv, gate, xpos, B, N, H, d, Bs, train=False) -> Tensor:
         cos, sin, qn, kn = self._rope_and_norms(xpos, d, qkv.device, qkv.dtype)
