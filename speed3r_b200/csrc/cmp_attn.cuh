@@ -1,12 +1,12 @@
 // Compression branch, forward, first of two kernels: dense attention of the pooled queries over the pooled keys, and
 // for every row a lower bound of its topk-th largest raw logit (RANK 0) or score of a block of four columns (RANK 1),
-// from which the second kernel (cmp_topk.cu) picks the row's best columns or blocks.
+// from which the second kernel (cmp_topk.cuh) picks the row's best columns or blocks.
 //
 // The two jobs want different things.  Attention is bound by the exponentials (one per score, 16 per cycle and SM);
 // the top-k has to look at every score once but keeps 32 of tens of thousands, through branches that depend on the
 // data.  Side by side in one kernel (softmax warps and top-k warps reading the same scores) each waited for the other
 // tile by tile; the products, which the second kernel repeats, are cheap: the tensor pipe was a fifth busy.
-// Measured (16 heads, one kernel before -> this one + cmp_topk.cu): 384 x 384 99 -> 9 + 23 us, 6300 x 6300 1047 ->
+// Measured (16 heads, one kernel before -> this one + cmp_topk.cuh): 384 x 384 99 -> 9 + 23 us, 6300 x 6300 1047 ->
 // 223 + 244 us (scores that cluster by view and patch: 1923 -> 222 + 315), 7875 x 63000 5.81 -> 2.45 + 1.69 ms.
 //
 // The bound: a row keeps the running maxima of 64 groups of columns (half of S, piece of 16 in it and column mod 8).  topk of
@@ -37,6 +37,7 @@
 // scores outgrew its offset by more than 2^64 takes its keys a second time with the rows' exact maxima, which the group
 // maxima have found by then.  No maximum, vote or branch stands between one exponential and the next (a check per tile, with
 // the tile redone: 2.90 ms; a check per 32 columns, with P rescaled: 3.40 ms).
+#pragma once
 #include <type_traits>
 
 #include "common.cuh"
@@ -52,11 +53,12 @@ struct AtCfg {
   static constexpr int kStages = 3;
   static constexpr int kOffK = R * kAtTile;
   static constexpr int kOffV = kOffK + kStages * kAtTile;
-  static constexpr int kSmem = kOffV + kStages * kAtTile + 1024;
+  static constexpr int kOffXchg = kOffV + kStages * kAtTile;      // what the two threads of a row tell each other: R x 2 x 128 floats
+  static constexpr int kSmem = kOffXchg + R * 1024 + 1024;
   static constexpr uint32_t kColO = R * 128, kColP = R * 192, kCols = R * 256;
   // registers: the launch gives every thread the same number, for R = 2 the utility warps hand some of theirs over
-  // (640 x 96 at launch = 61440 >= 512 x 104 + 128 x 56)
-  static constexpr int kSoftmaxRegs = 104, kUtilityRegs = 56;
+  // (640 x 96 at launch = 61440 = 512 x 112 + 128 x 32)
+  static constexpr int kSoftmaxRegs = 112, kUtilityRegs = 32;
 };
 
 struct AtCtl {
@@ -79,21 +81,19 @@ struct AtParams {
   uint32_t* status;
 };
 
+// `cta`: which R * 128 rows
 template <int R, int RANK>
-__global__ void __launch_bounds__(AtCfg<R>::kThreads, 1)
-cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_ks,
-                const __grid_constant__ CUtensorMap map_vs, const AtParams p) {
+__device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
+                                             const CUtensorMap& map_ks, const CUtensorMap& map_vs, const AtParams& p, AtCtl& ctl,
+                                             uint8_t* smem_raw, int cta) {
   using C = AtCfg<R>;
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ AtCtl ctl;
-  __shared__ float xchg[R][2][128];            // what the two threads of a row tell each other
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_bh = (p.Nq + R * 128 - 1) / (R * 128);
-  const int bh = blockIdx.x / tiles_per_bh;
-  const int q0 = (blockIdx.x % tiles_per_bh) * R * 128;
+  const int bh = cta / tiles_per_bh;
+  const int q0 = (cta % tiles_per_bh) * R * 128;
   const int ntiles = (p.Nc + 127) / 128;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  float (*xchg)[2][128] = reinterpret_cast<float (*)[2][128]>(smem_raw + (sbase - smem_u32(smem_raw)) + C::kOffXchg);
 
   if (threadIdx.x == 0) {
     ctl.abort_flag = 0;
@@ -431,33 +431,6 @@ cmp_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (warp == 2) tmem_dealloc(tmem, C::kCols);
-}
-
-template <int R, int RANK>
-static int launch_cmp_attn(const CmpMaps& m, const AtParams& p, int BH, cudaStream_t st) {
-  using C = AtCfg<R>;
-  const int64_t grid = static_cast<int64_t>(BH) * ((p.Nq + R * 128 - 1) / (R * 128));
-  S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
-  S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<R, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
-  return launch(cmp_attn_kernel<R, RANK>, static_cast<unsigned>(grid), C::kThreads, C::kSmem, st, m.q, m.k, m.v, m.ks, m.vs, p);
-}
-
-int cmp_attn_fwd(const CmpMaps& m, void* o_c, float* lse, float* bound, const CmpSizes& n, float scale, uint32_t* status,
-                 cudaStream_t st) {
-  AtParams p;
-  p.o = static_cast<__nv_bfloat16*>(o_c);
-  p.lse = lse;
-  p.bound = bound;
-  p.Nq = n.Nq; p.Nc = n.Nc; p.topk = n.topk;
-  p.scattered = m.scattered;
-  p.rank_take = n.rank_take;
-  p.c_scale = scale * 1.4426950408889634f;
-  p.status = status;
-  // One row tile per CTA while all of them fit the GPU at once (384 x 384, 16 heads: 8.7 instead of 12.2 us), two row
-  // tiles sharing every K and V tile beyond that (1512 x 1512: 25 instead of 35 us).
-  const bool one = static_cast<int64_t>(n.BH) * ((n.Nq + 127) / 128) <= sm_count();
-  if (n.rank_take > 0) return one ? launch_cmp_attn<1, 1>(m, p, n.BH, st) : launch_cmp_attn<2, 1>(m, p, n.BH, st);
-  return one ? launch_cmp_attn<1, 0>(m, p, n.BH, st) : launch_cmp_attn<2, 0>(m, p, n.BH, st);
 }
 
 }  // namespace s3r

@@ -8,16 +8,6 @@ struct CmpMaps {
   CUtensorMap q, k, v, ks, vs;
   int scattered;               // leading key tiles for which the first kernel uses ks and vs
 };
-struct CmpSizes {
-  int BH, Nq, Nc, topk;
-  int rank_take;               // 0: columns by logit; else blocks of four columns by the sum over this many of them
-};
-// Dense attention; row r's lower bound of its topk-th largest logit or score goes to bound[r * topk].
-int cmp_attn_fwd(const CmpMaps& m, void* o_c, float* lse, float* bound, const CmpSizes& n, float scale, uint32_t* status,
-                 cudaStream_t st);
-// Best columns or blocks of every row; idx[row * topk] holds the row's bound on entry.
-int cmp_topk_fwd(const CmpMaps& m, int32_t* idx, const CmpSizes& n, float scale, uint32_t* status, cudaStream_t st);
-
 #ifdef __CUDACC__
 // Threshold for the float pre-filter `score > thr`: an equal score with a larger column loses to the entry whose key
 // this is.  The one place where float order and key order disagree is -0.0 < +0.0: a kept -0.0 yields a threshold

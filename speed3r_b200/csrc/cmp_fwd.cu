@@ -1,7 +1,72 @@
-// Compression branch, forward: tensor maps and the two launches, attention with every row's bound (cmp_attn.cu) and the
-// columns or blocks that reach it (cmp_topk.cu).
-#include "common.cuh"
-#include "cmp_common.cuh"
+// Compression branch, forward: tensor maps and launches of the attention with every row's bound (cmp_attn.cuh) and of the
+// collection of the columns or blocks that reach it (cmp_topk.cuh).
+#include "cmp_attn.cuh"
+#include "cmp_topk.cuh"
+
+namespace s3r {
+
+template <int R, int RANK>
+__global__ void __launch_bounds__(AtCfg<R>::kThreads, 1)
+cmp_attn_kernel(const __grid_constant__ CmpMaps m, const __grid_constant__ AtParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ AtCtl ctl;
+  cmp_attn_cta<R, RANK>(m.q, m.k, m.v, m.ks, m.vs, p, ctl, smem_raw, blockIdx.x);
+}
+template <int RANK>
+__global__ void __launch_bounds__(kTkThreads, 1)
+cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ TkParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ TkCtl ctl;
+  cmp_topk_cta<RANK, false>(map_q, map_k, p, ctl, smem_raw, blockIdx.x);
+}
+
+// Both in one grid, all of the attention's CTAs first.  With more row tiles than SMs the last wave of either leaves SMs idle
+// (496 tiles on 148 SMs: a sixth of both); so the second kind's CTAs fill the first kind's last wave.  They wait for rows
+// whose CTA has been running since before them and waits for nobody.
+// Measured (16 heads, two launches -> one): 2400 x 2400 154 -> 126 us, 5000 x 5000 373 -> 320, 7875 x 63000 4.11 -> 3.66 ms;
+// where the waves are full anyway the same: 6300 x 6300 449, 15750 x 15750 2155 -> 2145 us.
+template <int RANK>
+__global__ void __launch_bounds__(kTkThreads, 1)
+cmp_both_kernel(const __grid_constant__ CmpMaps m, const __grid_constant__ AtParams pa, const __grid_constant__ TkParams pt,
+                const int attn_ctas) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ union {
+    AtCtl attn;
+    TkCtl topk;
+  } ctl;
+  if (static_cast<int>(blockIdx.x) < attn_ctas)
+    cmp_attn_cta<2, RANK>(m.q, m.k, m.v, m.ks, m.vs, pa, ctl.attn, smem_raw, blockIdx.x);
+  else
+    cmp_topk_cta<RANK, true>(m.q, m.k, pt, ctl.topk, smem_raw, static_cast<int>(blockIdx.x) - attn_ctas);
+}
+static_assert(AtCfg<2>::kThreads == kTkThreads && AtCfg<2>::kSmem <= kTkSmem, "one launch shape for both kinds");
+
+template <int RANK>
+static int launch_cmp(const CmpMaps& m, AtParams a, TkParams t, int64_t BH, cudaStream_t st) {
+  const int64_t tiles1 = BH * ((t.Nq + 127) / 128), per_bh = (t.Nq + kTkRows - 1) / kTkRows, tiles2 = BH * per_bh;
+  S3R_REQUIRE(2 * tiles2 < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
+  if (tiles2 > sm_count()) {
+    // all of the table, not only the words that are waited for: a strided fill takes ten times as long
+    S3R_CUDA(cudaMemsetAsync(t.idx, 0xff, static_cast<size_t>(BH) * t.Nq * t.topk * sizeof(int32_t), st));
+    S3R_CUDA(cudaFuncSetAttribute(cmp_both_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
+    return launch(cmp_both_kernel<RANK>, static_cast<unsigned>(2 * tiles2), kTkThreads, kTkSmem, st, m, a, t, static_cast<int>(tiles2));
+  }
+  int rc;
+  // One row tile per CTA while all of them fit the GPU at once (384 x 384, 16 heads: 8.7 instead of 12.2 us), two row
+  // tiles sharing every K and V tile beyond that (1512 x 1512: 25 instead of 35 us).
+  if (tiles1 <= sm_count()) {
+    S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<1, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, AtCfg<1>::kSmem));
+    rc = launch(cmp_attn_kernel<1, RANK>, static_cast<unsigned>(tiles1), AtCfg<1>::kThreads, AtCfg<1>::kSmem, st, m, a);
+  } else {
+    S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<2, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, AtCfg<2>::kSmem));
+    rc = launch(cmp_attn_kernel<2, RANK>, static_cast<unsigned>(tiles2), AtCfg<2>::kThreads, AtCfg<2>::kSmem, st, m, a);
+  }
+  if (rc) return rc;
+  S3R_CUDA(cudaFuncSetAttribute(cmp_topk_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
+  return launch(cmp_topk_kernel<RANK>, static_cast<unsigned>(tiles2), kTkThreads, kTkSmem, st, m.q, m.k, t);
+}
+
+}  // namespace s3r
 
 using namespace s3r;
 
@@ -52,11 +117,26 @@ static int launch_cmp_fwd(const char* who, const void* q_c, const void* k_c, con
   }
   uint32_t* status = device_status_ptr();
   S3R_REQUIRE(status != nullptr, S3R_ERR_DRIVER, "%s: could not resolve the device status word", who);
-  const CmpSizes n = {BH, Nq, Nc, topk, rank_take};
+  AtParams a;
+  a.o = static_cast<__nv_bfloat16*>(o_c);
+  a.lse = lse;
+  a.bound = reinterpret_cast<float*>(idx);
+  a.Nq = Nq; a.Nc = Nc; a.topk = topk;
+  a.scattered = m.scattered;
+  a.rank_take = rank_take;
+  a.c_scale = scale * 1.4426950408889634f;
+  a.status = status;
+  TkParams t;
+  t.idx = idx;
+  t.Nq = Nq; t.Nc = Nc; t.topk = topk;
+  t.rank_take = rank_take;
+  t.n_rank = rank_take > 0 ? (Nc - rank_take) / 4 + 1 : 0;       // blocks of four columns with all counted columns present
+  t.pad = (rank_take > 0 ? t.n_rank : Nc) - 1;
+  t.c_scale = a.c_scale;
+  t.vec = (topk & 3) == 0 && (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
+  t.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int rc = cmp_attn_fwd(m, o_c, lse, reinterpret_cast<float*>(idx), n, scale, status, st);
-  if (rc) return rc;
-  return cmp_topk_fwd(m, idx, n, scale, status, st);
+  return rank_take > 0 ? launch_cmp<1>(m, a, t, BH, st) : launch_cmp<0>(m, a, t, BH, st);
 }
 
 extern "C" int s3r_cmp_attn_topk_fwd(const void* q_c, const void* k_c, const void* v_c, void* o_c, float* lse,

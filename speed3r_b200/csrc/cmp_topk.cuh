@@ -2,7 +2,7 @@
 // (RANK 0), ordered by (logit descending, column ascending), or the `topk` blocks of four columns (RANK 1) by
 // log2 of the sum of 2^(c * s) over a block's first rank_take columns, which needs no row normaliser.
 //
-// The first kernel (cmp_attn.cu) leaves a lower bound of each row's topk-th largest logit, so this one repeats Q K^T on
+// The first kernel (cmp_attn.cuh) leaves a lower bound of each row's topk-th largest logit, so this one repeats Q K^T on
 // the tensor cores and only collects the logits that reach the bound - about 44 per row with independent scores - into
 // lists of (logit, column) pairs in shared memory, [slot][lane] so that a thread's accesses never meet another's on a
 // bank.  A row has two threads (in two warpgroups that take turns at its key tiles) and a list for each.  A list that
@@ -22,6 +22,7 @@
 // only blocks that reach it get their logarithm: bound by the exponentials' unit.
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-19 scan: two row tiles of
 // 128 queries, two warpgroups each.  Tensor memory: 2 row tiles x 2 tiles x 128 columns.
+#pragma once
 #include "common.cuh"
 #include "cmp_common.cuh"
 
@@ -151,15 +152,31 @@ __device__ __noinline__ void tk_exact(const uint2* la, int na, const uint2* lb, 
 }
 static_assert(kTkCap == 40, "tk_exact takes lists of up to 40, the packed words a place below 80");
 
-template <int RANK>
-__global__ void __launch_bounds__(kTkThreads, 1)
-cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const TkParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ TkCtl ctl;
+// Both kinds of CTA in one grid: a row's bound is there when its word is no longer what it was filled with (all bits set: a NaN
+// that no arithmetic returns).  For at most a second; called by whole warps.
+__device__ __forceinline__ bool wait_bound(const int32_t* word, bool mine, uint32_t& v, volatile uint32_t* abort_flag) {
+  const uint64_t start = globaltimer_ns();
+  while (true) {
+    v = 0;
+    if (mine) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+    if (__all_sync(0xffffffffu, v != ~0u)) return true;
+    const bool over = *abort_flag != 0u || globaltimer_ns() - start > 1000000000ull;
+    if (__any_sync(0xffffffffu, over)) {
+      *abort_flag = 1u;
+      return false;
+    }
+    __nanosleep(200);
+  }
+}
+
+// `cta`: which 256 rows.  WAIT: in one grid with the CTAs that find the bounds.
+template <int RANK, bool WAIT>
+__device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUtensorMap& map_k, const TkParams& p, TkCtl& ctl,
+                                             uint8_t* smem_raw, int cta) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_bh = (p.Nq + kTkRows - 1) / kTkRows;
-  const int bh = blockIdx.x / tiles_per_bh;
-  const int q0 = (blockIdx.x % tiles_per_bh) * kTkRows;
+  const int bh = cta / tiles_per_bh;
+  const int q0 = (cta % tiles_per_bh) * kTkRows;
   const int ntiles = (p.Nc + 127) / 128;
   const bool split = ntiles < kTkSplitTiles;
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -191,9 +208,9 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
   // registers: the launch gives every thread 96, the utility warps hand most of theirs to the scan
-  // (640 x 96 = 61440 >= 512 x 104 + 128 x 40)
+  // (640 x 96 = 61440 = 512 x 112 + 128 x 32)
   if (warp < 4) {
-    reg_dealloc<40>();
+    reg_dealloc<32>();
     if (warp == 0) {
       if (lane == 0) {
         mbar_expect_tx(&ctl.q_full, 2 * kTkTile);
@@ -250,7 +267,7 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       }
     }
   } else {
-    reg_alloc<104>();
+    reg_alloc<112>();
     const int t = (warp - 4) >> 3, par = ((warp - 4) >> 2) & 1, quarter = warp & 3;
     const int row = q0 + t * 128 + quarter * 32 + lane;
     const uint32_t t_s = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + t * 256;
@@ -260,14 +277,17 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // `score > thr` for every score that reaches the bound (NaN and -inf never do); rows past the end collect nothing
     float thr = INFINITY;
     uint32_t base_key = 0;                       // every collected pair's key is at least this
-    if (row < p.Nq) {
-      const float bound = fmaxf(__int_as_float(*out), -3.402823466e38f);
+    bool ok = true;
+    uint32_t bound_word = 0;
+    if (WAIT) ok = wait_bound(out, row < p.Nq, bound_word, abort_flag);
+    else if (row < p.Nq) bound_word = static_cast<uint32_t>(*out);
+    if (ok && row < p.Nq) {
+      const float bound = fmaxf(__uint_as_float(bound_word), -3.402823466e38f);
       base_key = sortable_key(bound == 0.f ? -0.f : bound);
       thr = bound == 0.f ? __uint_as_float(0x80000001u) : key_to_float(sortable_key(bound) - 1u);
     }
     const uint32_t first = smem_u32(buf), end = first + kTkCap * 256;
     uint32_t at = first;                         // where the list's next pair goes
-    bool ok = true;
 
     // 16 columns: a max tree and a vote pass over chunks in which no row of the warp has a hit
     auto scan = [&](const uint32_t* x, int col0) {
@@ -493,23 +513,6 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   if (warp == 2) tmem_dealloc(tmem, 512);
-}
-
-int cmp_topk_fwd(const CmpMaps& m, int32_t* idx, const CmpSizes& n, float scale, uint32_t* status, cudaStream_t st) {
-  TkParams p;
-  p.idx = idx;
-  p.Nq = n.Nq; p.Nc = n.Nc; p.topk = n.topk;
-  p.rank_take = n.rank_take;
-  p.n_rank = n.rank_take > 0 ? (n.Nc - n.rank_take) / 4 + 1 : 0;
-  p.pad = (n.rank_take > 0 ? p.n_rank : n.Nc) - 1;
-  p.c_scale = scale * 1.4426950408889634f;
-  p.vec = (n.topk & 3) == 0 && (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
-  p.status = status;
-  const int64_t grid = static_cast<int64_t>(n.BH) * ((n.Nq + kTkRows - 1) / kTkRows);
-  S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
-  auto kernel = n.rank_take > 0 ? cmp_topk_kernel<1> : cmp_topk_kernel<0>;
-  S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
-  return launch(kernel, static_cast<unsigned>(grid), kTkThreads, kTkSmem, st, m.q, m.k, p);
 }
 
 }  // namespace s3r

@@ -12,7 +12,7 @@
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-7 softmax, thread = row.
 // Two CTAs per SM: their steps fill each other's waits.
 // The exponent offset of a row is the maximum of its first step; a CTA in which some row outgrew it by more than 2^64 takes
-// its keys a second time with the exact maxima (cmp_attn.cu).
+// its keys a second time with the exact maxima (cmp_attn.cuh).
 #include "sel_common.cuh"
 
 namespace s3r {
