@@ -23,8 +23,9 @@ struct PoolParams {
   int B, H, d;
 };
 
-// KERNEL: the window length when it is known at compile time (all loads of a window then leave together), 0 otherwise.
-template <int KERNEL>
+// BATCH: so many loads of a window leave together (its length is a multiple of BATCH; one at a time, windows of 32 tokens at
+// 252000 took 760 us instead of 263).
+template <int BATCH>
 __device__ __forceinline__ void pool_tensor(const PoolTensor& p, int B, int H, int d) {
   const int vec_per_row = d >> 3;
   const int64_t total = static_cast<int64_t>(B) * p.Nc * H * vec_per_row;
@@ -47,14 +48,13 @@ __device__ __forceinline__ void pool_tensor(const PoolTensor& p, int B, int H, i
         acc[2 * w + 1] += bf16_hi(v.w[w]);
       }
     };
-    if (KERNEL > 0) {
-      Bf16x8 v[KERNEL > 0 ? KERNEL : 1];
+#pragma unroll 1
+    for (int t0 = 0; t0 < p.kernel; t0 += BATCH) {
+      Bf16x8 v[BATCH];
 #pragma unroll
-      for (int t = 0; t < KERNEL; ++t) v[t] = *reinterpret_cast<const Bf16x8*>(src + t * p.st);
+      for (int t = 0; t < BATCH; ++t) v[t] = *reinterpret_cast<const Bf16x8*>(src + (t0 + t) * p.st);
 #pragma unroll
-      for (int t = 0; t < KERNEL; ++t) add(v[t]);
-    } else {
-      for (int t = 0; t < p.kernel; ++t) add(*reinterpret_cast<const Bf16x8*>(src + t * p.st));
+      for (int t = 0; t < BATCH; ++t) add(v[t]);
     }
     Bf16x8 o;
 #pragma unroll
@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(256) pool_fwd_kernel(const PoolParams p) {
   griddep_wait();
   griddep_launch();
   const PoolTensor& t = p.t[blockIdx.y];
-  if (t.kernel == 16) pool_tensor<16>(t, p.B, p.H, p.d);
-  else pool_tensor<0>(t, p.B, p.H, p.d);
+  if (t.kernel % 16 == 0) pool_tensor<16>(t, p.B, p.H, p.d);
+  else pool_tensor<1>(t, p.B, p.H, p.d);
 }
 
 __global__ void __launch_bounds__(256)
