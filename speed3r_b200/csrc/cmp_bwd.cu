@@ -17,6 +17,8 @@
 // Every CTA reads the whole streamed tensors from L2: bytes per score = 256 / owned rows (254 GB for both
 // kernels at 1000 views with 128 owned rows), so a CTA owns 256 rows - as many as tensor memory holds
 // accumulators for (2 row tiles x (dK, dV) x 64 columns = 256 columns; the other 256 hold S and dP).
+// dQ's own tiles live in tensor memory, where dK/dV has its second accumulators: an M=128 N=64 product with both operands in
+// shared memory reads 24 KB of it (192 cycles at 128 bytes), with one of them in tensor memory 8 KB for 128 cycles of math.
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warp 3 loads the
 // streamed rows' lse/delta (dK/dV), warps 4-19 compute, two warpgroups per row tile: a row has two threads, each with 32
 // of a tile's columns.  P and dS are written in place, over
@@ -54,6 +56,7 @@ struct CbCtl {
 };
 
 struct CbParams {
+  const __nv_bfloat16 *x0, *x1;  // dQ: q and dO
   const float *lse, *delta;      // [BH, Nq]
   __nv_bfloat16 *out0, *out1;    // dK/dV kernel: dV, dK [BH, Nc, 64];  dQ kernel: unused, dQ [BH, Nq, 64]
   int n_own, n_str;              // rows of the owned and of the streamed tensors (Nc, Nq | Nq, Nc)
@@ -77,7 +80,7 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
 
   if (threadIdx.x == 0) {
     ctl.abort_flag = 0;
-    mbar_init(&ctl.x_full, 1);
+    mbar_init(&ctl.x_full, MODE == 0 ? 1 : 16);
     mbar_init(&ctl.o_full, 1);
     for (int s = 0; s < kCbStages; ++s) {
       mbar_init(&ctl.y_full[s], 1);
@@ -109,9 +112,9 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      mbar_expect_tx(&ctl.x_full, 4 * kCbOwnBytes);
+      if (MODE == 0) mbar_expect_tx(&ctl.x_full, 4 * kCbOwnBytes);
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
+      for (int t = 0; t < 2 && MODE == 0; ++t) {
         tma_load_3d(sbase + kCbOffX + t * 2 * kCbOwnBytes, &map_x0, &ctl.x_full, 0, r0 + t * 128, bh);
         tma_load_3d(sbase + kCbOffX + t * 2 * kCbOwnBytes + kCbOwnBytes, &map_x1, &ctl.x_full, 0, r0 + t * 128, bh);
       }
@@ -155,6 +158,11 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
       const uint64_t x_t0 = desc_x, x_t1 = desc_x + static_cast<uint64_t>(2 * kCbOwnBytes >> 4);
       const uint32_t d0 = tmem + kCbColAcc, d1 = tmem + kCbColAcc + 128;
       const uint32_t b0 = tmem, b1 = tmem + kCbColBuf;
+      // S or dP of a row tile: its own operand from shared memory, or from tensor memory
+      auto first_product = [&](uint32_t d, uint64_t x_smem, uint32_t x_tmem, uint64_t y) {
+        if (MODE == 0) umma_ss_k4<2, 2>(d, x_smem, y, idesc_1, 0u);
+        else umma_ts_k4<2>(d, x_tmem, y, idesc_1, 0u);
+      };
 #pragma unroll 1
       for (int i = 0; i <= ntiles && ok; ++i) {
         const bool more = i < ntiles;
@@ -167,7 +175,7 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
         if (leader) {
           if (MODE == 0 && i >= 1) umma_ts_k4<128, 24>(d0, b0, y1 + (kCbStrBytes >> 4), idesc_2, i > 1 ? 1u : 0u);
           if (more) {
-            umma_ss_k4<2, 2>(b0, x_t0, y0, idesc_1, 0u);
+            first_product(b0, x_t0, d0, y0);
             umma_commit(&ctl.s_full[0]);
           }
         }
@@ -181,7 +189,7 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
           tc_fence_after();
           if (leader) {
             if (i >= 2) umma_ts_k4<128, 24>(d1 + kCbColAcc1, b1 + kCbColDP, y2, idesc_2, i > 2 ? 1u : 0u);
-            umma_ss_k4<2, 2>(b1 + kCbColDP, x_t1 + (kCbOwnBytes >> 4), y1 + (kCbStrBytes >> 4), idesc_1, 0u);
+            first_product(b1 + kCbColDP, x_t1 + (kCbOwnBytes >> 4), d1 + 32, y1 + (kCbStrBytes >> 4));
             umma_commit(&ctl.dp_full[1]);
             if (i >= 2) umma_commit(&ctl.y_empty[st2]);
           }
@@ -196,7 +204,7 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
         if (leader) {
           if (i >= 1) umma_ts_k4<128, 24>(d0 + kCbColAcc1, b0 + kCbColDP, y1, idesc_2, i > 1 ? 1u : 0u);
           if (more) {
-            umma_ss_k4<2, 2>(b0 + kCbColDP, x_t0 + (kCbOwnBytes >> 4), y0 + (kCbStrBytes >> 4), idesc_1, 0u);
+            first_product(b0 + kCbColDP, x_t0 + (kCbOwnBytes >> 4), d0 + 32, y0 + (kCbStrBytes >> 4));
             umma_commit(&ctl.dp_full[0]);
           }
         }
@@ -210,7 +218,7 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
         if (leader) {
           if (MODE == 0 && i >= 1) umma_ts_k4<128, 24>(d1, b1, y1 + (kCbStrBytes >> 4), idesc_2, i > 1 ? 1u : 0u);
           if (more) {
-            umma_ss_k4<2, 2>(b1, x_t1, y0, idesc_1, 0u);
+            first_product(b1, x_t1, d1, y0);
             umma_commit(&ctl.s_full[1]);
           }
         }
@@ -268,6 +276,21 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
     if (MODE == 1 && row < p.n_own) {
       my_lse2 = -(p.lse[static_cast<int64_t>(bh) * p.Nq + row] * 1.4426950408889634f);
       my_delta = -p.delta[static_cast<int64_t>(bh) * p.Nq + row];
+    }
+    if (MODE == 1) {
+      // this thread's half of the own operands, 64 channels of q or dO, to where the accumulators leave columns free
+      uint32_t x[32];
+      const uint4* src = reinterpret_cast<const uint4*>((half ? p.x1 : p.x0) + (static_cast<int64_t>(bh) * p.n_own + row) * 64);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint4 v = row < p.n_own ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+        x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+      }
+      tmem_st32(lane_base + kCbColAcc + t * 128 + half * 32, x);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.x_full);
     }
     bool ok = true;
     float pf[32];                                   // P of this row against 32 of the tile's streamed rows
@@ -440,6 +463,7 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
     }
   }
   CbParams p;
+  p.x0 = p.x1 = nullptr;
   p.lse = lse; p.delta = delta;
   p.Nq = Nq;
   p.cs = scale * 1.4426950408889634f;
@@ -452,6 +476,8 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
   kv.out0 = static_cast<__nv_bfloat16*>(dv_c);
   kv.out1 = static_cast<__nv_bfloat16*>(dk_c);
   kv.n_own = Nc; kv.n_str = Nq;
+  q.x0 = static_cast<const __nv_bfloat16*>(q_c);
+  q.x1 = static_cast<const __nv_bfloat16*>(do_c);
   q.out0 = nullptr;
   q.out1 = static_cast<__nv_bfloat16*>(dq_c);
   q.n_own = Nq; q.n_str = Nc;
