@@ -149,6 +149,7 @@ def cpu_sample(views, seconds_hint=20.0):
 
 def own_launches(nq, nc, bwd):
     """Kernels of this library in one step: nq query blocks of this rank against nc key blocks."""
+    import torch
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
     n = 3 + (1 if H * -(-nq // 256) > sms else 2) + 1
     return n + (1 + (1 if nq * TOPK <= 24576 and nc <= 8192 else 5) + 1 + 2 + 3 if bwd else 0)

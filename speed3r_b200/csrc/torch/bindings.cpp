@@ -469,6 +469,7 @@ struct CmpNode : torch::autograd::Function<CmpNode> {
     ctx->save_for_backward({q, k, v, o, lse});
     ctx->saved_data["scale"] = scale;
     ctx->mark_non_differentiable({idx});
+    ctx->set_materialize_grads(false);      // no zeros for the table
     return {o, idx};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -809,10 +810,12 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     ctx->saved_data["eps"] = eps;
     ctx->saved_data["scale"] = scale;
     ctx->mark_non_differentiable({idx});
+    ctx->set_materialize_grads(false);      // no zeros for the table
     return {out.view({m.B, m.N, w_proj.size(0)}), idx};
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    if (!g[0].defined()) return variable_list(19);
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const auto s = ctx->get_saved_variables();
     const Tensor &buf = s[0], &idx = s[2];
@@ -946,12 +949,14 @@ struct SparseNode : torch::autograd::Function<SparseNode> {
     ctx->saved_data["stride"] = stride;
     ctx->saved_data["scale"] = scale;
     ctx->mark_non_differentiable({idx});
+    ctx->set_materialize_grads(false);      // no zeros for the table
     return {y, idx};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto s = ctx->get_saved_variables();
     const int64_t block = ctx->saved_data["block"].toInt();
     const double scale = ctx->saved_data["scale"].toDouble();
+    if (!g[0].defined()) return variable_list(11);
     if (plain(s[0]) && plain(g[0])) {
       c10::cuda::CUDAGuard guard(s[0].device());
       const Tensor& idx = s[9];

@@ -192,6 +192,76 @@ def test_cmp_table_when_the_bound_is_loose(period):
     assert_bf16_close(o, ref, "o_c")
 
 
+@pytest.mark.parametrize("topk", [1, 6, 32])
+@pytest.mark.parametrize("Nc", [50, 130, 1030])
+def test_cmp_both_kinds_in_one_grid(topk, Nc):
+    """More row tiles than SMs: attention and collection share a grid, twice with the same buffers (the table is filled anew)."""
+    from speed3r_b200 import ops
+    B, H, Nq = 1, 170, 130
+    q, k, v = bf16_round(randn(65, B, H, Nq, 64), randn(66, B, H, Nc, 64), randn(67, B, H, Nc, 64))
+    g = [t.to(DEV, torch.bfloat16) for t in (q, k, v)]
+    for _ in range(2):
+        o, lse, idx = ops._cmp_fwd(*g, topk, 0.125)
+    ref, lse_ref, idx_ref = R.cmp_attn_topk(q, k, v, topk)
+    assert_idx_match(idx, idx_ref, q @ k.transpose(-1, -2), f"Nc {Nc} topk {topk}")
+    assert_bf16_close(o, ref, "o_c")
+    assert_bf16_close(lse, lse_ref, "lse", max_abs=5e-3, mean_abs=1e-3, scale_with_ref=False)
+
+
+@pytest.mark.parametrize("Nc,take,topk,heads", [(3, 3, 4, 2), (128 * 3 + 2, 3, 32, 2), (128 * 4, 1, 16, 2), (128 * 5 - 1, 4, 32, 2),
+                                                (128 * 20 + 5, 2, 7, 2), (128 * 3 + 127, 3, 16, 170)])
+def test_cmp_block_ranking_tiles(Nc, take, topk, heads):
+    """Odd and even numbers of key tiles (two sets of group maxima), a last block that counts only if its columns exist, all
+    numbers of counted columns, and both kinds of CTA in one grid."""
+    from speed3r_b200 import ops
+    B, Nq = 1, 70
+    q, k, v = bf16_round(randn(70, B, heads, Nq, 64), randn(71, B, heads, Nc, 64), randn(72, B, heads, Nc, 64))
+    o, idx = ops.flash_attn_blocktopk_func(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), topk, 4, take)
+    ref, _, idx_ref = R.cmp_attn_topk(q, k, v, topk, rank_group=(4, take))
+    scores = R.block_rank_scores(q @ k.transpose(-1, -2), 0.125, 4, take)
+    n = scores.shape[-1]
+    assert_idx_match(idx[..., :min(topk, n)], idx_ref[..., :min(topk, n)], scores, f"Nc {Nc} take {take}")
+    assert (idx[..., n:] == n - 1).all()
+    assert_bf16_close(o, ref, "o_c")
+
+
+# ------------------------------------------------------------------ selection backward
+@pytest.mark.parametrize("block,T,K", [(16, 16 * 500 + 9, 3), (16, 16 * 520, 9), (32, 32 * 270 - 1, 2), (64, 64 * 130 + 1, 5)])
+def test_sel_bwd_tasks_handed_over(block, T, K):
+    """More tasks than places on the GPU, so that warps take over others': lists of no entry, one, and several hundred (a key
+    block that every query block selects), an odd number of tiles, a short last block."""
+    from speed3r_b200 import ops
+    B, H, nb = 1, 4, -(-T // block)
+    q, k, v, do = bf16_round(*(randn(75 + i, B, H, T, 64) for i in range(4)))
+    idx = table(79, B, H, nb, nb, K)
+    idx[:, 1] = idx[:, 1] // 7 * 7                                       # six of seven blocks unselected
+    idx[:, 2, :, 0] = nb // 2                                            # selected by all
+    idx[:, 3] = torch.arange(nb, dtype=torch.int32)[:, None]             # every block once per entry
+    idx[:, 3, :, 1:] = -1
+    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    R.sel_attn(*ref, idx, block)[0].backward(do)
+    got = [t.to(DEV, torch.bfloat16).requires_grad_(True) for t in (q, k, v)]
+    ops.topk_blocksparse_attention(*got, idx.to(DEV), block).backward(do.to(DEV, torch.bfloat16))
+    for n, a, b in zip("qkv", got, ref):
+        assert_bf16_close(a.grad, b.grad, f"d{n}")
+
+
+def test_host_pipeline_default_chunks():
+    """The sizes a caller gets who names none: all heads in one group on a short sequence, the last group's queries in quarters."""
+    from speed3r_b200 import HostPipeline, ops
+    H, T = 6, 16 * 300
+    hq, hk, hv = (randn(85 + i, 1, H, T, 64).bfloat16().pin_memory() for i in range(3))
+    hgate = torch.sigmoid(randn(88, 1, H, T, 2)).bfloat16().pin_memory()
+    q, k, v, gate = (t.to(DEV) for t in (hq, hk, hv, hgate))
+    y, _ = ops.sparse_attention_op(q, k, v, gate)
+    pipe = HostPipeline(H, T, device=DEV)
+    assert pipe.hg == H and pipe.rows_last == 256
+    hy = torch.zeros(1, T, H * 64, dtype=torch.bfloat16).pin_memory()
+    pipe(hq, hk, hv, hgate, hy)
+    torch.cuda.synchronize()
+    assert torch.equal(hy, y.cpu())
+
+
 # ------------------------------------------------------------------ prologue backward, module paths
 @pytest.mark.parametrize("B,H,Bs,blocks,norm,rope", [(1, 1, 16, 1, True, True), (2, 16, 16, 7, True, True),
                                                      (1, 17, 16, 3, True, True), (2, 3, 4, 5, True, False),
