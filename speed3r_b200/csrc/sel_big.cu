@@ -6,9 +6,11 @@
 // is written over the diagonal blocks of a zeroed tile, so that O += P V (K=128) adds the right keys to each row.  The
 // G - 1 unwanted blocks beside each wanted one are cheaper than mma.sync without them: 16 heads, top-16 blocks of 64 at 250
 // views 3.86 -> 2.40 ms, 64 views 1002 -> 555 us; top-32 blocks of 32, 60000 tokens 1073 -> 818 us.
-// Bound: shared memory (copies 32 KB, operands 48 KB per step and CTA, at 128 bytes per cycle) and the tensor pipe, both about
-// three quarters busy inside a row tile; its start and its end take a fifth of its time.  Two threads per row instead of one
-// changed nothing (576 us); leaving out the exponentials, the second product or the gather's cache misses alone 3 % each.
+// Bound: latency, with no unit more than half busy.  Of a CTA's 18.5 us at 64500 tokens, top-16, 2.4 pass until its first S is
+// there, 13 in 16 steps (0.8 us each beside another CTA, 80 KB of shared-memory traffic) and 3 at its end; 2.5 more until
+// the next CTA runs in its place.  The merge's operands are loaded before the last product is waited for (1.6 us less at the
+// end, 2 to 4 % of the whole).  Two threads per row instead of one changed nothing; several row tiles per CTA without a barrier
+// between them cost more registers and instructions than the starts they saved (574 -> 670 us).
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-7 softmax, thread = row.
 // Two CTAs per SM: their steps fill each other's waits.
 // The exponent offset of a row is the maximum of its first step; a CTA in which some row outgrew it by more than 2^64 takes
@@ -283,6 +285,10 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       if (lane == 0) mbar_arrive(&ctl.p_full);
       return true;
     };
+    const int b = bh / p.H, h = bh - b * p.H;
+    const bool live = row < p.Tq;
+    uint32_t gate_word = 0;
+    uint4 merged[8];                            // the row's block of the other branch
     int pass = 0;
     do {
       if (pass == 1) {
@@ -291,6 +297,13 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
 #pragma unroll 1
       for (int j = 0; j < steps && ok; ++j) ok = step(pass * steps + j, j);
+      // what the merge needs, on its way while the last product runs
+      if (live && p.y) {
+        gate_word = __ldg(reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + row * p.gst));
+        const uint4* oc = reinterpret_cast<const uint4*>(p.o_c + (static_cast<int64_t>(bh) * p.nqb + qb0 + g) * 64);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) merged[i] = __ldg(oc + i);
+      }
       if (ok) ok = mbar_wait_warp(&ctl.o_full, pass & 1, abort_flag);
       if (pass == 0 && nv > 0 && !(row_max() * cs <= m_used + 64.f)) ctl.again = 1u;
     } while (another_pass(pass++));
@@ -298,17 +311,10 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     if (ok && aligned) {
       tc_fence_after();
       const float inv = nv > 0 ? 1.f / l : 0.f;             // no valid key: o = 0, lse = -inf
-      const int b = bh / p.H, h = bh - b * p.H;
-      const bool live = row < p.Tq;
       if (live && p.lse_s)
         p.lse_s[static_cast<int64_t>(bh) * p.Tq + row] = nv > 0 ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
-      float g0 = 0.f, g1 = 0.f;
-      if (live && p.y) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + row * p.gst);
-        g0 = bf16_lo(w);
-        g1 = bf16_hi(w);
-      }
-#pragma unroll 1
+      const float g0 = bf16_lo(gate_word), g1 = bf16_hi(gate_word);
+#pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t o[32];
         if (steps > 0) {
@@ -327,11 +333,10 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                                 pack_bf16(f(8 * i + 4), f(8 * i + 5)), pack_bf16(f(8 * i + 6), f(8 * i + 7)));
         }
         if (p.y) {
-          const uint4* oc = reinterpret_cast<const uint4*>(p.o_c + (static_cast<int64_t>(bh) * p.nqb + qb0 + g) * 64 + hf * 32);
           uint4* dst = reinterpret_cast<uint4*>(p.y + ((static_cast<int64_t>(b) * p.Tq + row) * p.H + h) * 64 + hf * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const uint4 c = __ldg(oc + i);
+            const uint4 c = merged[hf * 4 + i];
             const uint32_t cw[4] = {c.x, c.y, c.z, c.w};
             uint32_t w[4];
 #pragma unroll
