@@ -167,6 +167,10 @@ int s3r_cmp_attn_blocktopk_fwd(const void* q_c, const void* k_c, const void* v_c
 int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_c, const void* o_c, const float* lse,
                      const void* do_c, float* delta, void* dq_c, void* dk_c, void* dv_c, int B, int H, int Nq,
                      int Nc, int d, float scale, void* stream);
+/* Same with delta given (s3r_merge_bwd_deltas writes it). */
+int s3r_cmp_attn_bwd_delta(const void* q_c, const void* k_c, const void* v_c, const float* lse, const void* do_c,
+                           const float* delta, void* dq_c, void* dk_c, void* dv_c, int B, int H, int Nq, int Nc, int d,
+                           float scale, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Selection attention (block-sparse flash attention) with the gated merge fused in.
@@ -244,6 +248,10 @@ int s3r_build_key_csr_static(const int32_t* idx, int32_t* offsets, int32_t* qids
 int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
                   int64_t gate_stride_t, const void* o_c, const void* o_s, void* do_s, float* dgate,
                   void* do_c, float* delta_s, int B, int H, int Tq, int d, int block, void* stream);
+/* Same, and delta_c [B,H,ceil(Tq/block)] fp32 = sum_d o_c*do_c (NULL: not wanted). */
+int s3r_merge_bwd_deltas(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
+                         int64_t gate_stride_t, const void* o_c, const void* o_s, void* do_s, float* dgate, void* do_c,
+                         float* delta_s, float* delta_c, int B, int H, int Tq, int d, int block, void* stream);
 
 /* Row-wise delta = sum_d o*do for [rows,d] bf16 tensors (backward_sum_o_do,
  * topk_blocksparse_attention.py:132-170); used when the merge is not fused. */

@@ -31,12 +31,14 @@ SIGNATURES = {
     "s3r_cmp_attn_topk_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_cmp_attn_blocktopk_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p]),
     "s3r_cmp_attn_bwd": (_i, [_p] * 10 + [_i, _i, _i, _i, _i, _f, _p]),
+    "s3r_cmp_attn_bwd_delta": (_i, [_p] * 9 + [_i, _i, _i, _i, _i, _f, _p]),
     "s3r_sel_attn_fwd": (_i, [_p, _p, _p, _i, _i64, _p, _p, _p, _p, _i64, _i64, _i64, _p, _p,
                               _i, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_csr_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),
     "s3r_build_key_csr": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p, _sz, _p]),
     "s3r_build_key_csr_static": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p]),
     "s3r_merge_bwd": (_i, [_p, _p, _i64, _i64, _i64, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p]),
+    "s3r_merge_bwd_deltas": (_i, [_p, _p, _i64, _i64, _i64, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _p]),
     "s3r_delta": (_i, [_p, _p, _p, _i64, _i, _p]),
     "s3r_sel_attn_bwd": (_i, [_p] * 12 + [_i, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_sel_attn_bwd_pooled": (_i, [_p] * 15 + [_i] * 11 + [_f, _p]),

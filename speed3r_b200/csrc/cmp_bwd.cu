@@ -431,10 +431,10 @@ cmp_bwd_kernel(const __grid_constant__ CbMaps m, const CbParams kv, const CbPara
 
 using namespace s3r;
 
-extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_c, const void* o_c, const float* lse,
-                                const void* do_c, float* delta, void* dq_c, void* dk_c, void* dv_c, int B, int H,
-                                int Nq, int Nc, int d, float scale, void* stream) {
-  S3R_REQUIRE(q_c && k_c && v_c && o_c && lse && do_c && delta && dq_c && dk_c && dv_c, S3R_ERR_NULL,
+extern "C" int s3r_cmp_attn_bwd_delta(const void* q_c, const void* k_c, const void* v_c, const float* lse, const void* do_c,
+                                      const float* delta, void* dq_c, void* dk_c, void* dv_c, int B, int H, int Nq,
+                                      int Nc, int d, float scale, void* stream) {
+  S3R_REQUIRE(q_c && k_c && v_c && lse && do_c && delta && dq_c && dk_c && dv_c, S3R_ERR_NULL,
               "s3r_cmp_attn_bwd: NULL pointer");
   S3R_REQUIRE(B > 0 && H > 0 && Nq > 0 && Nc > 0, S3R_ERR_SHAPE, "s3r_cmp_attn_bwd: bad sizes");
   S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_cmp_attn_bwd: head_dim %d not supported (64 only)", d);
@@ -443,8 +443,7 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
                        reinterpret_cast<uintptr_t>(dk_c) | reinterpret_cast<uintptr_t>(dv_c);
   S3R_REQUIRE((al & 15) == 0, S3R_ERR_ALIGNMENT, "s3r_cmp_attn_bwd: tensors must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int rc = s3r_delta(o_c, do_c, delta, static_cast<int64_t>(B) * H * Nq, d, stream);
-  if (rc) return rc;
+  int rc = 0;
   const int BH = B * H;
   CbMaps m;
   {
@@ -485,4 +484,16 @@ extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_
                 g1 = static_cast<int64_t>(BH) * ((Nq + kCbOwnRows - 1) / kCbOwnRows);
   S3R_REQUIRE(g0 + g1 < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_bwd: grid too large");
   return launch(cmp_bwd_kernel, static_cast<unsigned>(g0 + g1), kCbThreads, kCbSmemBytes, st, m, kv, q, static_cast<int>(g0));
+}
+
+extern "C" int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_c, const void* o_c, const float* lse,
+                                const void* do_c, float* delta, void* dq_c, void* dk_c, void* dv_c, int B, int H,
+                                int Nq, int Nc, int d, float scale, void* stream) {
+  S3R_REQUIRE(q_c && k_c && v_c && o_c && lse && do_c && delta && dq_c && dk_c && dv_c, S3R_ERR_NULL,
+              "s3r_cmp_attn_bwd: NULL pointer");
+  S3R_REQUIRE(B > 0 && H > 0 && Nq > 0 && Nc > 0, S3R_ERR_SHAPE, "s3r_cmp_attn_bwd: bad sizes");
+  S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_cmp_attn_bwd: head_dim %d not supported (64 only)", d);
+  const int rc = s3r_delta(o_c, do_c, delta, static_cast<int64_t>(B) * H * Nq, d, stream);
+  if (rc) return rc;
+  return s3r_cmp_attn_bwd_delta(q_c, k_c, v_c, lse, do_c, delta, dq_c, dk_c, dv_c, B, H, Nq, Nc, d, scale, stream);
 }

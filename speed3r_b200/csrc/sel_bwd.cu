@@ -340,6 +340,7 @@ struct MergeBwdParams {
   float* dgate;
   __nv_bfloat16* do_c;
   float* delta_s;
+  float* delta_c;                // null: not wanted
   int B, H, Tq, block, nqb;
 };
 
@@ -404,11 +405,18 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
     acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 8);
     acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
   }
-  if (sub == 0) {
-    uint4 out;
-    out.x = pack_bf16(acc[0], acc[1]); out.y = pack_bf16(acc[2], acc[3]);
-    out.z = pack_bf16(acc[4], acc[5]); out.w = pack_bf16(acc[6], acc[7]);
-    *reinterpret_cast<uint4*>(p.do_c + (static_cast<int64_t>(bh) * p.nqb + m) * 64 + c8 * 8) = out;
+  uint4 out;
+  out.x = pack_bf16(acc[0], acc[1]); out.y = pack_bf16(acc[2], acc[3]);
+  out.z = pack_bf16(acc[4], acc[5]); out.w = pack_bf16(acc[6], acc[7]);
+  if (sub == 0) *reinterpret_cast<uint4*>(p.do_c + (static_cast<int64_t>(bh) * p.nqb + m) * 64 + c8 * 8) = out;
+  if (p.delta_c) {                                         // of the rounded gradient, as s3r_delta takes it
+    const uint32_t w[4] = {out.x, out.y, out.z, out.w};
+    float d = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d += oc[2 * i] * bf16_lo(w[i]) + oc[2 * i + 1] * bf16_hi(w[i]);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    if (lane == 0) p.delta_c[static_cast<int64_t>(bh) * p.nqb + m] = d;
   }
 }
 
@@ -989,9 +997,10 @@ extern "C" int s3r_delta(const void* o, const void* d_o, float* delta, int64_t r
                 static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, rows);
 }
 
-extern "C" int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
-                             int64_t gate_stride_t, const void* o_c, const void* o_s, void* do_s, float* dgate,
-                             void* do_c, float* delta_s, int B, int H, int Tq, int d, int block, void* stream) {
+extern "C" int s3r_merge_bwd_deltas(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
+                                    int64_t gate_stride_t, const void* o_c, const void* o_s, void* do_s, float* dgate,
+                                    void* do_c, float* delta_s, float* delta_c, int B, int H, int Tq, int d, int block,
+                                    void* stream) {
   S3R_REQUIRE(dy && gate && o_c && o_s && do_s && dgate && do_c && delta_s, S3R_ERR_NULL, "s3r_merge_bwd: NULL pointer");
   S3R_REQUIRE(B > 0 && H > 0 && Tq > 0 && block > 0, S3R_ERR_SHAPE, "s3r_merge_bwd: bad sizes");
   S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_merge_bwd: head_dim %d not supported (64 only)", d);
@@ -1005,10 +1014,18 @@ extern "C" int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stri
   p.dgate = dgate;
   p.do_c = static_cast<__nv_bfloat16*>(do_c);
   p.delta_s = delta_s;
+  p.delta_c = delta_c;
   p.B = B; p.H = H; p.Tq = Tq; p.block = block;
   p.nqb = (Tq + block - 1) / block;
   const int64_t warps = static_cast<int64_t>(B) * H * p.nqb;
   return launch(merge_bwd_kernel, static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), p);
+}
+
+extern "C" int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
+                             int64_t gate_stride_t, const void* o_c, const void* o_s, void* do_s, float* dgate,
+                             void* do_c, float* delta_s, int B, int H, int Tq, int d, int block, void* stream) {
+  return s3r_merge_bwd_deltas(dy, gate, gate_stride_b, gate_stride_h, gate_stride_t, o_c, o_s, do_s, dgate, do_c, delta_s, nullptr,
+                              B, H, Tq, d, block, stream);
 }
 
 static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {

@@ -138,8 +138,9 @@ std::tuple<Tensor, Tensor, Tensor> cmp_attn_blocktopk_fwd(const Tensor& q_c, con
   return cmp_fwd(q_c, k_c, v_c, topk, scale, group, take);
 }
 
-std::tuple<Tensor, Tensor, Tensor> cmp_attn_bwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c,
-                                                const Tensor& o_c, const Tensor& lse, const Tensor& do_c, double scale) {
+std::tuple<Tensor, Tensor, Tensor> cmp_bwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c,
+                                                const Tensor& o_c, const Tensor& lse, const Tensor& do_c, double scale,
+                                                const Tensor* have_delta) {
   need(q_c, "q_c");
   need(k_c, "k_c");
   need(v_c, "v_c");
@@ -148,11 +149,22 @@ std::tuple<Tensor, Tensor, Tensor> cmp_attn_bwd(const Tensor& q_c, const Tensor&
   need(lse, "lse", at::kFloat);
   const int64_t B = q_c.size(0), H = q_c.size(1), Nq = q_c.size(2), d = q_c.size(3), Nc = k_c.size(2);
   c10::cuda::CUDAGuard guard(q_c.device());
-  Tensor dq = fresh_like(q_c), dk = fresh_like(k_c), dv = fresh_like(v_c), delta = fresh_like(lse);
+  Tensor dq = fresh_like(q_c), dk = fresh_like(k_c), dv = fresh_like(v_c);
+  if (have_delta) {
+    check(s3r_cmp_attn_bwd_delta(q_c.data_ptr(), k_c.data_ptr(), v_c.data_ptr(), f32(lse), do_c.data_ptr(), f32(*have_delta),
+                                 dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Nq, Nc, d, scale, stream()),
+          "s3r_cmp_attn_bwd_delta");
+    return {dq, dk, dv};
+  }
+  Tensor delta = fresh_like(lse);
   check(s3r_cmp_attn_bwd(q_c.data_ptr(), k_c.data_ptr(), v_c.data_ptr(), o_c.data_ptr(), f32(lse), do_c.data_ptr(),
                          f32(delta), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Nq, Nc, d, scale, stream()),
         "s3r_cmp_attn_bwd");
   return {dq, dk, dv};
+}
+std::tuple<Tensor, Tensor, Tensor> cmp_attn_bwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c,
+                                                const Tensor& o_c, const Tensor& lse, const Tensor& do_c, double scale) {
+  return cmp_bwd(q_c, k_c, v_c, o_c, lse, do_c, scale, nullptr);
 }
 
 void need_gate(const Tensor& gate) {
@@ -293,18 +305,23 @@ Tensor delta(const Tensor& o, const Tensor& d_o) {
   return out;
 }
 
-std::tuple<Tensor, Tensor, Tensor, Tensor> merge_bwd(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
-                                                     const Tensor& o_s, int64_t block) {
+std::tuple<Tensor, Tensor, Tensor, Tensor> merge_bwd_deltas(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
+                                                            const Tensor& o_s, int64_t block, Tensor* delta_c) {
   need(dy, "dy");
   need_gate(gate);
   const int64_t B = o_s.size(0), H = o_s.size(1), Tq = o_s.size(2), d = o_s.size(3);
   c10::cuda::CUDAGuard guard(dy.device());
   Tensor do_s = fresh_like(o_s), dgate = fresh({B, H, Tq, 2}, dy, at::kFloat), do_c = fresh_like(o_c),
          delta_s = fresh({B, H, Tq}, dy, at::kFloat);
-  check(s3r_merge_bwd(dy.data_ptr(), gate.data_ptr(), gate.stride(0), gate.stride(1), gate.stride(2), o_c.data_ptr(),
-                      o_s.data_ptr(), do_s.data_ptr(), f32(dgate), do_c.data_ptr(), f32(delta_s), B, H, Tq, d, block,
-                      stream()), "s3r_merge_bwd");
+  if (delta_c) *delta_c = fresh({B, H, o_c.size(2)}, dy, at::kFloat);
+  check(s3r_merge_bwd_deltas(dy.data_ptr(), gate.data_ptr(), gate.stride(0), gate.stride(1), gate.stride(2), o_c.data_ptr(),
+                             o_s.data_ptr(), do_s.data_ptr(), f32(dgate), do_c.data_ptr(), f32(delta_s),
+                             delta_c ? f32(*delta_c) : nullptr, B, H, Tq, d, block, stream()), "s3r_merge_bwd");
   return {do_s, dgate, do_c, delta_s};
+}
+std::tuple<Tensor, Tensor, Tensor, Tensor> merge_bwd(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
+                                                     const Tensor& o_s, int64_t block) {
+  return merge_bwd_deltas(dy, gate, o_c, o_s, block, nullptr);
 }
 
 const void* ptr_or_null(const optional<Tensor>& t) { return t.has_value() ? t->data_ptr() : nullptr; }
@@ -868,10 +885,10 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     };
     if (ints[5] && ctx->needs_input_grad(e_wp + 1)) dbp = colsum(dy.data_ptr(), out_features);
     // merge, the two branches, prologue
-    check(s3r_merge_bwd(sp(a_dy), ptr(m.gate), m.H * m.N * 2, m.N * 2, 2, ptr(m.t(6)), ptr(m.o_s), sp(a_dos), sf(a_dgate), sp(a_doc),
-                        sf(a_dels), m.B, m.H, m.N, m.d, m.block, st), "s3r_merge_bwd");
-    check(s3r_cmp_attn_bwd(ptr(m.t(3)), ptr(m.t(4)), ptr(m.t(5)), ptr(m.t(6)), static_cast<float*>(ptr(m.lse_c)), sp(a_doc), sf(a_delc),
-                           sp(a_dqc), sp(a_dkc), sp(a_dvc), m.B, m.H, m.Nc, m.Nc, m.d, scale, st), "s3r_cmp_attn_bwd");
+    check(s3r_merge_bwd_deltas(sp(a_dy), ptr(m.gate), m.H * m.N * 2, m.N * 2, 2, ptr(m.t(6)), ptr(m.o_s), sp(a_dos), sf(a_dgate),
+                               sp(a_doc), sf(a_dels), sf(a_delc), m.B, m.H, m.N, m.d, m.block, st), "s3r_merge_bwd");
+    check(s3r_cmp_attn_bwd_delta(ptr(m.t(3)), ptr(m.t(4)), ptr(m.t(5)), static_cast<float*>(ptr(m.lse_c)), sp(a_doc), sf(a_delc),
+                                 sp(a_dqc), sp(a_dkc), sp(a_dvc), m.B, m.H, m.Nc, m.Nc, m.d, scale, st), "s3r_cmp_attn_bwd_delta");
     beside.join();
     check(s3r_sel_attn_bwd(ptr(m.t(0)), ptr(m.t(1)), ptr(m.t(2)), i32(idx), off, qids, static_cast<float*>(ptr(m.lse_s)), sf(a_dels),
                            sp(a_dos), sp(a_dq), sp(a_dk), sp(a_dv), m.B, m.H, m.N, m.N, m.d, m.block, m.topk, scale, st),
@@ -965,8 +982,9 @@ struct SparseNode : torch::autograd::Function<SparseNode> {
       const std::tuple<Tensor, Tensor> inverse(fresh({B, H, nkb + 1}, idx, at::kInt), fresh({B, H, Nq * K}, idx, at::kInt));
       const Tensor ws = fresh({static_cast<int64_t>(nbytes)}, idx, at::kByte);
       CsrBeside beside(i32(idx), i32m(std::get<0>(inverse)), i32m(std::get<1>(inverse)), B, H, Nq, K, nkb, ws.data_ptr(), nbytes);
-      auto [do_s, dgate, do_c, dlt] = merge_bwd(g[0].contiguous(), s[3], s[7], s[10], block);
-      auto [dq_c, dk_c, dv_c] = cmp_attn_bwd(s[4], s[5], s[6], s[7], s[8], do_c, scale);
+      Tensor dlt_c;
+      auto [do_s, dgate, do_c, dlt] = merge_bwd_deltas(g[0].contiguous(), s[3], s[7], s[10], block, &dlt_c);
+      auto [dq_c, dk_c, dv_c] = cmp_bwd(s[4], s[5], s[6], s[7], s[8], do_c, scale, &dlt_c);
       beside.join();
       auto [dq, dk, dv] = sel_bwd(s[0], s[1], s[2], idx, s[11], dlt, do_s, &dq_c, &dk_c, &dv_c, block,
                                   ctx->saved_data["kernel"].toInt(), ctx->saved_data["stride"].toInt(), scale, &inverse);
