@@ -12,12 +12,12 @@ cmp_attn_kernel(const __grid_constant__ CmpMaps m, const __grid_constant__ AtPar
   __shared__ AtCtl ctl;
   cmp_attn_cta<R, RANK>(m.q, m.k, m.v, m.ks, m.vs, p, ctl, smem_raw, blockIdx.x);
 }
-template <int RANK>
-__global__ void __launch_bounds__(kTkThreads, 1)
+template <int R, int RANK>
+__global__ void __launch_bounds__(TkCfg<R>::kThreads, 1)
 cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ TkParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ TkCtl ctl;
-  cmp_topk_cta<RANK, false>(map_q, map_k, p, ctl, smem_raw, blockIdx.x);
+  cmp_topk_cta<R, RANK, false>(map_q, map_k, p, ctl, smem_raw, blockIdx.x);
 }
 
 // Both in one grid, all of the attention's CTAs first.  With more row tiles than SMs the last wave of either leaves SMs idle
@@ -26,7 +26,7 @@ cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 // Measured (16 heads, two launches -> one): 2400 x 2400 154 -> 126 us, 5000 x 5000 373 -> 320, 7875 x 63000 4.11 -> 3.66 ms;
 // where the waves are full anyway the same: 6300 x 6300 449, 15750 x 15750 2155 -> 2145 us.
 template <int RANK>
-__global__ void __launch_bounds__(kTkThreads, 1)
+__global__ void __launch_bounds__(TkCfg<2>::kThreads, 1)
 cmp_both_kernel(const __grid_constant__ CmpMaps m, const __grid_constant__ AtParams pa, const __grid_constant__ TkParams pt,
                 const int attn_ctas) {
   extern __shared__ uint8_t smem_raw[];
@@ -37,33 +37,31 @@ cmp_both_kernel(const __grid_constant__ CmpMaps m, const __grid_constant__ AtPar
   if (static_cast<int>(blockIdx.x) < attn_ctas)
     cmp_attn_cta<2, RANK>(m.q, m.k, m.v, m.ks, m.vs, pa, ctl.attn, smem_raw, blockIdx.x);
   else
-    cmp_topk_cta<RANK, true>(m.q, m.k, pt, ctl.topk, smem_raw, static_cast<int>(blockIdx.x) - attn_ctas);
+    cmp_topk_cta<2, RANK, true>(m.q, m.k, pt, ctl.topk, smem_raw, static_cast<int>(blockIdx.x) - attn_ctas);
 }
-static_assert(AtCfg<2>::kThreads == kTkThreads && AtCfg<2>::kSmem <= kTkSmem, "one launch shape for both kinds");
+static_assert(AtCfg<2>::kThreads == TkCfg<2>::kThreads && AtCfg<2>::kSmem <= TkCfg<2>::kSmem, "one launch shape for both kinds");
 
+template <int R, int RANK>
+static int launch_cmp_apart(const CmpMaps& m, const AtParams& a, const TkParams& t, int64_t ctas, cudaStream_t st) {
+  S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<R, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, AtCfg<R>::kSmem));
+  const int rc = launch(cmp_attn_kernel<R, RANK>, static_cast<unsigned>(ctas), AtCfg<R>::kThreads, AtCfg<R>::kSmem, st, m, a);
+  if (rc) return rc;
+  S3R_CUDA(cudaFuncSetAttribute(cmp_topk_kernel<R, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, TkCfg<R>::kSmem));
+  return launch(cmp_topk_kernel<R, RANK>, static_cast<unsigned>(ctas), TkCfg<R>::kThreads, TkCfg<R>::kSmem, st, m.q, m.k, t);
+}
 template <int RANK>
 static int launch_cmp(const CmpMaps& m, AtParams a, TkParams t, int64_t BH, cudaStream_t st) {
-  const int64_t tiles1 = BH * ((t.Nq + 127) / 128), per_bh = (t.Nq + kTkRows - 1) / kTkRows, tiles2 = BH * per_bh;
+  const int64_t tiles1 = BH * ((t.Nq + 127) / 128), tiles2 = BH * ((t.Nq + 255) / 256);
   S3R_REQUIRE(2 * tiles2 < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_cmp_attn_topk_fwd: grid too large");
   if (tiles2 > sm_count()) {
     // all of the table, not only the words that are waited for: a strided fill takes ten times as long
     S3R_CUDA(cudaMemsetAsync(t.idx, 0xff, static_cast<size_t>(BH) * t.Nq * t.topk * sizeof(int32_t), st));
-    S3R_CUDA(cudaFuncSetAttribute(cmp_both_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
-    return launch(cmp_both_kernel<RANK>, static_cast<unsigned>(2 * tiles2), kTkThreads, kTkSmem, st, m, a, t, static_cast<int>(tiles2));
+    S3R_CUDA(cudaFuncSetAttribute(cmp_both_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, TkCfg<2>::kSmem));
+    return launch(cmp_both_kernel<RANK>, static_cast<unsigned>(2 * tiles2), TkCfg<2>::kThreads, TkCfg<2>::kSmem, st, m, a, t, static_cast<int>(tiles2));
   }
-  int rc;
-  // One row tile per CTA while all of them fit the GPU at once (384 x 384, 16 heads: 8.7 instead of 12.2 us), two row
-  // tiles sharing every K and V tile beyond that (1512 x 1512: 25 instead of 35 us).
-  if (tiles1 <= sm_count()) {
-    S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<1, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, AtCfg<1>::kSmem));
-    rc = launch(cmp_attn_kernel<1, RANK>, static_cast<unsigned>(tiles1), AtCfg<1>::kThreads, AtCfg<1>::kSmem, st, m, a);
-  } else {
-    S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<2, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, AtCfg<2>::kSmem));
-    rc = launch(cmp_attn_kernel<2, RANK>, static_cast<unsigned>(tiles2), AtCfg<2>::kThreads, AtCfg<2>::kSmem, st, m, a);
-  }
-  if (rc) return rc;
-  S3R_CUDA(cudaFuncSetAttribute(cmp_topk_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTkSmem));
-  return launch(cmp_topk_kernel<RANK>, static_cast<unsigned>(tiles2), kTkThreads, kTkSmem, st, m.q, m.k, t);
+  // One row tile per CTA while all of them fit the GPU at once, two row tiles sharing every key tile beyond that.  Attention
+  // alone: 384 x 384, 16 heads: 8.7 instead of 12.2 us; 1512 x 1512: 35 instead of 25 us.
+  return tiles1 <= sm_count() ? launch_cmp_apart<1, RANK>(m, a, t, tiles1, st) : launch_cmp_apart<2, RANK>(m, a, t, tiles2, st);
 }
 
 }  // namespace s3r

@@ -20,8 +20,10 @@
 // 0.95 ms for 15750 x 15750, 16 heads).
 // RANK 1 sums exponentials relative to the bound, three in four of them needed where a block counts three columns, and
 // only blocks that reach it get their logarithm: bound by the exponentials' unit.
-// Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-19 scan: two row tiles of
-// 128 queries, two warpgroups each.  Tensor memory: 2 row tiles x 2 tiles x 128 columns.
+// Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-19 scan: R = 2 row tiles of
+// 128 queries, two warpgroups each.  Tensor memory: R row tiles x 2 tiles x 128 columns.  R = 1 (warps 4-11) where that still
+// leaves one CTA per SM at most: the sorts share the issue slots of half as many warps.  Both kernels, 16 heads: 128 x 128
+// 16.1 -> 13.6 us, 384 x 384 (2 samples) 24.2 -> 19.6, 1152 x 1152 56.0 -> 49.5.
 #pragma once
 #include "common.cuh"
 #include "cmp_common.cuh"
@@ -30,12 +32,13 @@ namespace s3r {
 
 constexpr int kTkTile = 128 * 128;             // 128 rows x 64 bf16, bytes
 constexpr int kTkCap = 40;                     // pairs a list holds before it is cut back to 32
-constexpr int kTkRows = 256;                   // query rows per CTA
 constexpr int kTkStages = 2;
-constexpr int kTkOffK = 2 * kTkTile;
-constexpr int kTkOffBuf = kTkOffK + kTkStages * kTkTile;
-constexpr int kTkSmem = kTkOffBuf + 2 * kTkRows * kTkCap * 8 + 1024;
-constexpr int kTkThreads = 128 + 512;
+template <int R>
+struct TkCfg {
+  static constexpr int kRows = R * 128, kThreads = 128 + 256 * R;
+  static constexpr int kOffK = R * kTkTile, kOffBuf = kOffK + kTkStages * kTkTile;
+  static constexpr int kSmem = kOffBuf + 2 * kRows * kTkCap * 8 + 1024;
+};
 constexpr int kTkSplitTiles = 16;              // with fewer tiles the two scans of a row take halves of every tile, not turns
 
 struct TkCtl {
@@ -169,17 +172,17 @@ __device__ __forceinline__ bool wait_bound(const int32_t* word, bool mine, uint3
   }
 }
 
-// `cta`: which 256 rows.  WAIT: in one grid with the CTAs that find the bounds.
-template <int RANK, bool WAIT>
+// `cta`: which R * 128 rows.  WAIT: in one grid with the CTAs that find the bounds.
+template <int R, int RANK, bool WAIT>
 __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUtensorMap& map_k, const TkParams& p, TkCtl& ctl,
                                              uint8_t* smem_raw, int cta) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_per_bh = (p.Nq + kTkRows - 1) / kTkRows;
+  using C = TkCfg<R>;
+  const int tiles_per_bh = (p.Nq + C::kRows - 1) / C::kRows;
   const int bh = cta / tiles_per_bh;
-  const int q0 = (cta % tiles_per_bh) * kTkRows;
+  const int q0 = (cta % tiles_per_bh) * C::kRows;
   const int ntiles = (p.Nc + 127) / 128;
   const bool split = ntiles < kTkSplitTiles;
-  const int row_tiles = q0 + 128 < p.Nq ? 2 : 1;          // of 128 rows, of which the second may not exist
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
 
   if (threadIdx.x == 0) {
@@ -197,7 +200,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     mbar_fence_init();
   }
   if (warp == 2) {
-    tmem_alloc(&ctl.tmem_base, 512);
+    tmem_alloc(&ctl.tmem_base, R * 256);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -208,21 +211,21 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
-  // registers: the launch gives every thread 96, the utility warps hand most of theirs to the scan
+  // registers: for R = 2 the launch gives every thread 96, the utility warps hand most of theirs to the scan
   // (640 x 96 = 61440 = 512 x 112 + 128 x 32)
   if (warp < 4) {
-    reg_dealloc<32>();
+    if (R == 2) reg_dealloc<32>();
     if (warp == 0) {
       if (lane == 0) {
-        mbar_expect_tx(&ctl.q_full, 2 * kTkTile);
+        mbar_expect_tx(&ctl.q_full, R * kTkTile);
 #pragma unroll
-        for (int t = 0; t < 2; ++t) tma_load_3d(sbase + t * kTkTile, &map_q, &ctl.q_full, 0, q0 + t * 128, bh);
+        for (int t = 0; t < R; ++t) tma_load_3d(sbase + t * kTkTile, &map_q, &ctl.q_full, 0, q0 + t * 128, bh);
         int issued = 0;
         for (int j = 0; j < ntiles; ++j) {
           const int s = j % kTkStages;
           if (!mbar_wait(&ctl.k_empty[s], ((j / kTkStages) & 1) ^ 1, abort_flag)) break;
           mbar_expect_tx(&ctl.k_full[s], kTkTile);
-          tma_load_3d(sbase + kTkOffK + s * kTkTile, &map_k, &ctl.k_full[s], 0, j * 128, bh);
+          tma_load_3d(sbase + C::kOffK + s * kTkTile, &map_k, &ctl.k_full[s], 0, j * 128, bh);
           issued = j + 1;
         }
         if (*abort_flag) {
@@ -236,7 +239,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     } else if (warp == 1) {
       const bool leader = elect_one_sync();
       constexpr uint32_t idesc = umma_idesc_bf16(128, 64, 0, 0);
-      const uint64_t desc_q = umma_desc_sw128(sbase), desc_k = umma_desc_sw128(sbase + kTkOffK);
+      const uint64_t desc_q = umma_desc_sw128(sbase), desc_k = umma_desc_sw128(sbase + C::kOffK);
       bool ok = mbar_wait_warp(&ctl.q_full, 0, abort_flag);
       int s = 0;
       uint32_t ph = 0;
@@ -245,9 +248,8 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
         const int b = j & 1;
         ok = mbar_wait_warp(&ctl.k_full[s], ph, abort_flag);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int t = i & 1, h = i >> 1;
-          if (t >= row_tiles) continue;
+        for (int i = 0; i < 2 * R; ++i) {
+          const int t = i % R, h = i / R;
           if (ok) ok = mbar_wait_warp(&ctl.s_empty[t][b][h], ((j >> 1) & 1) ^ 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
@@ -255,7 +257,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
             umma_ss_k4<2, 2>(tmem + t * 256 + b * 128 + h * 64, desc_q + static_cast<uint64_t>(t * (kTkTile >> 4)),
                              desc_k + static_cast<uint64_t>(s * (kTkTile >> 4) + h * (kTkTile >> 5)), idesc, 0u);
             umma_commit(&ctl.s_full[t][b][h]);
-            if (h == 1 && t == row_tiles - 1) umma_commit(&ctl.k_empty[s]);
+            if (i == 2 * R - 1) umma_commit(&ctl.k_empty[s]);
           }
           __syncwarp();
         }
@@ -269,256 +271,252 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
       }
     }
   } else {
-    reg_alloc<112>();
+    if (R == 2) reg_alloc<112>();
     const int t = (warp - 4) >> 3, par = ((warp - 4) >> 2) & 1, quarter = warp & 3;
-    if (t >= row_tiles) {
-      asm volatile("bar.sync 3, 512;" ::: "memory");      // the scan's end, below
-    } else {
-      const int row = q0 + t * 128 + quarter * 32 + lane;
-      const uint32_t t_s = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + t * 256;
-      uint2* lists = reinterpret_cast<uint2*>(smem_raw + (sbase - smem_u32(smem_raw)) + kTkOffBuf);
-      uint2* buf = lists + (warp - 4) * (kTkCap * 32) + lane;
-      int32_t* out = p.idx + (static_cast<int64_t>(bh) * p.Nq + row) * p.topk;
-      // `score > thr` for every score that reaches the bound (NaN and -inf never do); rows past the end collect nothing
-      float thr = INFINITY;
-      uint32_t base_key = 0;                       // every collected pair's key is at least this
-      bool ok = true;
-      uint32_t bound_word = 0;
-      if (WAIT) ok = wait_bound(out, row < p.Nq, bound_word, abort_flag);
-      else if (row < p.Nq) bound_word = static_cast<uint32_t>(*out);
-      if (ok && row < p.Nq) {
-        const float bound = fmaxf(__uint_as_float(bound_word), -3.402823466e38f);
-        base_key = sortable_key(bound == 0.f ? -0.f : bound);
-        thr = bound == 0.f ? __uint_as_float(0x80000001u) : key_to_float(sortable_key(bound) - 1u);
-      }
-      const uint32_t first = smem_u32(buf), end = first + kTkCap * 256;
-      uint32_t at = first;                         // where the list's next pair goes
+    const int row = q0 + t * 128 + quarter * 32 + lane;
+    const uint32_t t_s = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + t * 256;
+    uint2* lists = reinterpret_cast<uint2*>(smem_raw + (sbase - smem_u32(smem_raw)) + C::kOffBuf);
+    uint2* buf = lists + (warp - 4) * (kTkCap * 32) + lane;
+    int32_t* out = p.idx + (static_cast<int64_t>(bh) * p.Nq + row) * p.topk;
+    // `score > thr` for every score that reaches the bound (NaN and -inf never do); rows past the end collect nothing
+    float thr = INFINITY;
+    uint32_t base_key = 0;                       // every collected pair's key is at least this
+    bool ok = true;
+    uint32_t bound_word = 0;
+    if (WAIT) ok = wait_bound(out, row < p.Nq, bound_word, abort_flag);
+    else if (row < p.Nq) bound_word = static_cast<uint32_t>(*out);
+    if (ok && row < p.Nq) {
+      const float bound = fmaxf(__uint_as_float(bound_word), -3.402823466e38f);
+      base_key = sortable_key(bound == 0.f ? -0.f : bound);
+      thr = bound == 0.f ? __uint_as_float(0x80000001u) : key_to_float(sortable_key(bound) - 1u);
+    }
+    const uint32_t first = smem_u32(buf), end = first + kTkCap * 256;
+    uint32_t at = first;                         // where the list's next pair goes
 
-      // 16 columns: a max tree and a vote pass over chunks in which no row of the warp has a hit
-      auto scan = [&](const uint32_t* x, int col0) {
-        auto f = [&](int i) { return __uint_as_float(x[i]); };
-        const float m = fmaxf(fmax3(fmax3(f(0), f(1), f(2)), fmax3(f(3), f(4), f(5)), fmax3(f(6), f(7), f(8))),
-                              fmax3(fmax3(f(9), f(10), f(11)), fmax3(f(12), f(13), f(14)), f(15)));
-        if (!__any_sync(0xffffffffu, m > thr)) return;
-        // bit 15 - i of the mask = sign of thr - x[i]; two chains of shifts
-        uint32_t m0 = 0, m1 = 0;
-        const float2 minus = make_float2(-1.f, -1.f), thr2 = make_float2(thr, thr);
+    // 16 columns: a max tree and a vote pass over chunks in which no row of the warp has a hit
+    auto scan = [&](const uint32_t* x, int col0) {
+      auto f = [&](int i) { return __uint_as_float(x[i]); };
+      const float m = fmaxf(fmax3(fmax3(f(0), f(1), f(2)), fmax3(f(3), f(4), f(5)), fmax3(f(6), f(7), f(8))),
+                            fmax3(fmax3(f(9), f(10), f(11)), fmax3(f(12), f(13), f(14)), f(15)));
+      if (!__any_sync(0xffffffffu, m > thr)) return;
+      // bit 15 - i of the mask = sign of thr - x[i]; two chains of shifts
+      uint32_t m0 = 0, m1 = 0;
+      const float2 minus = make_float2(-1.f, -1.f), thr2 = make_float2(thr, thr);
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-          const float2 d0 = ffma2(make_float2(f(i), f(i + 1)), minus, thr2), d1 = ffma2(make_float2(f(8 + i), f(9 + i)), minus, thr2);
-          m0 = __funnelshift_l(__float_as_uint(d0.y), __funnelshift_l(__float_as_uint(d0.x), m0, 1), 1);
-          m1 = __funnelshift_l(__float_as_uint(d1.y), __funnelshift_l(__float_as_uint(d1.x), m1, 1), 1);
+      for (int i = 0; i < 8; i += 2) {
+        const float2 d0 = ffma2(make_float2(f(i), f(i + 1)), minus, thr2), d1 = ffma2(make_float2(f(8 + i), f(9 + i)), minus, thr2);
+        m0 = __funnelshift_l(__float_as_uint(d0.y), __funnelshift_l(__float_as_uint(d0.x), m0, 1), 1);
+        m1 = __funnelshift_l(__float_as_uint(d1.y), __funnelshift_l(__float_as_uint(d1.x), m1, 1), 1);
+      }
+      const uint32_t mask = (m0 << 8) | m1;
+      // one hit per row at most, and room for it: it is the chunk's maximum
+      if (!__any_sync(0xffffffffu, (mask & (mask - 1)) != 0u || at == end)) {
+        if (mask) {
+          sts64(at, __float_as_uint(m), static_cast<uint32_t>(col0 - 16 + __clz(mask)));
+          at += 256;
         }
-        const uint32_t mask = (m0 << 8) | m1;
-        // one hit per row at most, and room for it: it is the chunk's maximum
-        if (!__any_sync(0xffffffffu, (mask & (mask - 1)) != 0u || at == end)) {
-          if (mask) {
-            sts64(at, __float_as_uint(m), static_cast<uint32_t>(col0 - 16 + __clz(mask)));
+      } else if (!__any_sync(0xffffffffu, at + 256 * __popc(mask) > end)) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (mask & (0x8000u >> i)) {
+            sts64(at, x[i], static_cast<uint32_t>(col0 + i));
             at += 256;
           }
-        } else if (!__any_sync(0xffffffffu, at + 256 * __popc(mask) > end)) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            if (mask & (0x8000u >> i)) {
-              sts64(at, x[i], static_cast<uint32_t>(col0 + i));
-              at += 256;
-            }
-          }
-        } else {
-          TkChunk ch;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) ch.x[i] = x[i];
-          int cnt = static_cast<int>(at - first) >> 8;
-          tk_append_checked(ch, buf, static_cast<uint32_t>(col0), cnt, thr);
-          at = first + cnt * 256;
-          __syncwarp();
         }
-      };
-      // 16 columns as four blocks
-      const float cs = p.c_scale;
-      float2 off01, off23;                         // minus the bound; columns that do not count: minus infinity
-      float cutoff;                                // roundings of the sums stay well below 1e-3 up to |bound| = 8192
-      auto set_offsets = [&](float bound) {
-        off01 = make_float2(-bound, p.rank_take > 1 ? -bound : -INFINITY);
-        off23 = make_float2(p.rank_take > 2 ? -bound : -INFINITY, p.rank_take > 3 ? -bound : -INFINITY);
-        cutoff = fabsf(bound) < 8192.f ? 0.999f : 0.f;
-      };
-      if (RANK) set_offsets(fmaxf(thr, -3.402823466e38f));
-      const bool four = p.rank_take > 3;
-      auto scan_blocks = [&](const uint32_t* x, int col0) {
-        auto f = [&](int i) { return __uint_as_float(x[i]); };
-        const float2 cs2 = make_float2(cs, cs);
-        float sum[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 a = ffma2(make_float2(f(4 * i), f(4 * i + 1)), cs2, off01), b = ffma2(make_float2(f(4 * i + 2), f(4 * i + 3)), cs2, off23);
-          if (i) {
-            sum[i] = fast_exp2(a.x) + fast_exp2(a.y) + fast_exp2(b.x);
-          } else {
-            const float2 e = exp2_fma2(make_float2(fminf(a.x, 126.f), fminf(a.y, 126.f)));
-            sum[i] = e.x + e.y + fast_exp2(b.x);
-          }
-          if (four) sum[i] += fast_exp2(b.y);
-        }
-        if (!__any_sync(0xffffffffu, fmaxf(fmax3(sum[0], sum[1], sum[2]), sum[3]) >= cutoff)) return;
-        if (__any_sync(0xffffffffu, at + 4 * 256 > end)) {                    // cut every list that has something to lose
-          const int cnt = static_cast<int>(at - first) >> 8;
-          if (cnt > 32) {
-            thr = tk_cut(buf, cnt);
-            at = first + 32 * 256;
-            set_offsets(thr);
-          }
-          __syncwarp();
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (sum[i] >= cutoff) {
-            float a[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) a[e] = e < p.rank_take ? f(4 * i + e) * cs : -INFINITY;
-            const float m = fmaxf(fmax3(a[0], a[1], a[2]), a[3]);
-            const float r = m + fast_log2((fast_exp2(a[0] - m) + fast_exp2(a[1] - m)) + (fast_exp2(a[2] - m) + fast_exp2(a[3] - m)));
-            const int n = (col0 >> 2) + i;
-            if (n < p.n_rank && r > thr) {
-              sts64(at, __float_as_uint(r), static_cast<uint32_t>(n));
-              at += 256;
-            }
-          }
-        }
-      };
-      // half h of tile j
-      auto half_tile = [&](int j, int h) -> bool {
-        const int b = j & 1;
-        if (!mbar_wait_warp(&ctl.s_full[t][b][h], (j >> 1) & 1, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t src = t_s + b * 128 + h * 64;
-        const int col0 = j * 128 + h * 64, left = p.Nc - col0;
-        auto release = [&]() {                     // all of this half of S is in registers: the next Q K^T may overwrite it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl.s_empty[t][b][h]);
-        };
-        uint32_t xa[32], xb[32];
-        tmem_ld32(src, xa);
-        tmem_ld32(src + 32, xb);
-        tmem_ld_wait();
-        release();
-        if (left < 64) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (i >= left) xa[i] = 0xff800000u;   // -inf
-            if (32 + i >= left) xb[i] = 0xff800000u;
-          }
-        }
-        auto go = [&](const uint32_t* x, int c) {
-          if (RANK) scan_blocks(x, c);
-          else scan(x, c);
-        };
-        go(xa, col0);
-        go(xa + 16, col0 + 16);
-        go(xb, col0 + 32);
-        go(xb + 16, col0 + 48);
-        return true;
-      };
-      if (split) {
-#pragma unroll 1
-        for (int j = 0; j < ntiles && ok; ++j) ok = half_tile(j, par);
       } else {
-#pragma unroll 1
-        for (int u = 2 * par; u < 2 * ntiles && ok; u = (u & 1) ? u + 3 : u + 1) ok = half_tile(u >> 1, u & 1);
+        TkChunk ch;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) ch.x[i] = x[i];
+        int cnt = static_cast<int>(at - first) >> 8;
+        tk_append_checked(ch, buf, static_cast<uint32_t>(col0), cnt, thr);
+        at = first + cnt * 256;
+        __syncwarp();
       }
-
-      const int cnt = static_cast<int>(at - first) >> 8;
-      const int r = quarter * 32 + lane;
-      // Q and the K ring are idle once every scan warp is here (whatever happened): per row tile 32 words per row for sorted
-      // words and columns, and two per row for what its threads tell each other
-      asm volatile("bar.sync 3, 512;" ::: "memory");
-      uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (sbase - smem_u32(smem_raw))) + t * (35 * 128) + r;   // [place][row]
-      uint32_t* tell = words + 32 * 128;         // [list][row] largest key, [2][row] the second list's length
-      auto meet = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory"); };
-      uint32_t a[32], e[kTkCap - 32];
-      uint32_t top = 0;
-      // keys above the bound's, plus one: an empty place is 0
-      auto word = [&](int i) {
-        const uint32_t d = i < cnt ? sortable_key(__uint_as_float(buf[i * 32].x)) - base_key + 1u : 0u;
-        top = max(top, d);
-        return d;
-      };
+    };
+    // 16 columns as four blocks
+    const float cs = p.c_scale;
+    float2 off01, off23;                         // minus the bound; columns that do not count: minus infinity
+    float cutoff;                                // roundings of the sums stay well below 1e-3 up to |bound| = 8192
+    auto set_offsets = [&](float bound) {
+      off01 = make_float2(-bound, p.rank_take > 1 ? -bound : -INFINITY);
+      off23 = make_float2(p.rank_take > 2 ? -bound : -INFINITY, p.rank_take > 3 ? -bound : -INFINITY);
+      cutoff = fabsf(bound) < 8192.f ? 0.999f : 0.f;
+    };
+    if (RANK) set_offsets(fmaxf(thr, -3.402823466e38f));
+    const bool four = p.rank_take > 3;
+    auto scan_blocks = [&](const uint32_t* x, int col0) {
+      auto f = [&](int i) { return __uint_as_float(x[i]); };
+      const float2 cs2 = make_float2(cs, cs);
+      float sum[4];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) a[i] = word(i);
-#pragma unroll
-      for (int i = 0; i < kTkCap - 32; ++i) e[i] = word(32 + i);
-      tell[par * 128] = top;
-      if (par == 1) tell[2 * 128] = static_cast<uint32_t>(cnt);
-      meet();
-      top = max(top, tell[(par ^ 1) * 128]);
-      const int shift = max(0, 7 - __clz(top | 1u));        // bits of the keys beyond 25
-      auto pack = [&](uint32_t& d, int i) { d = d ? ((d >> shift) << 7) | static_cast<uint32_t>(127 - par * kTkCap - i) : 0u; };
-#pragma unroll
-      for (int i = 0; i < 32; ++i) pack(a[i], i);
-      sort_desc<32>(a);
-      uint32_t lost = 0;                         // the largest word that is not among the row's 32
-      if (__any_sync(0xffffffffu, cnt > 32)) {
-#pragma unroll
-        for (int i = 0; i < kTkCap - 32; ++i) pack(e[i], 32 + i);
-        sort_desc<kTkCap - 32>(e);
-#pragma unroll
-        for (int i = 0; i < kTkCap - 32; ++i) {
-          lost = max(lost, min(a[31 - i], e[i]));
-          a[31 - i] = max(a[31 - i], e[i]);
+      for (int i = 0; i < 4; ++i) {
+        const float2 a = ffma2(make_float2(f(4 * i), f(4 * i + 1)), cs2, off01), b = ffma2(make_float2(f(4 * i + 2), f(4 * i + 3)), cs2, off23);
+        if (i) {
+          sum[i] = fast_exp2(a.x) + fast_exp2(a.y) + fast_exp2(b.x);
+        } else {
+          const float2 e = exp2_fma2(make_float2(fminf(a.x, 126.f), fminf(a.y, 126.f)));
+          sum[i] = e.x + e.y + fast_exp2(b.x);
         }
-        tk_merge(a);
+        if (four) sum[i] += fast_exp2(b.y);
       }
-      if (par == 1) {
+      if (!__any_sync(0xffffffffu, fmaxf(fmax3(sum[0], sum[1], sum[2]), sum[3]) >= cutoff)) return;
+      if (__any_sync(0xffffffffu, at + 4 * 256 > end)) {                    // cut every list that has something to lose
+        const int cnt = static_cast<int>(at - first) >> 8;
+        if (cnt > 32) {
+          thr = tk_cut(buf, cnt);
+          at = first + 32 * 256;
+          set_offsets(thr);
+        }
+        __syncwarp();
+      }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) words[i * 128] = a[i];
-        tell[1 * 128] = lost;
+      for (int i = 0; i < 4; ++i) {
+        if (sum[i] >= cutoff) {
+          float a[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] = e < p.rank_take ? f(4 * i + e) * cs : -INFINITY;
+          const float m = fmaxf(fmax3(a[0], a[1], a[2]), a[3]);
+          const float r = m + fast_log2((fast_exp2(a[0] - m) + fast_exp2(a[1] - m)) + (fast_exp2(a[2] - m) + fast_exp2(a[3] - m)));
+          const int n = (col0 >> 2) + i;
+          if (n < p.n_rank && r > thr) {
+            sts64(at, __float_as_uint(r), static_cast<uint32_t>(n));
+            at += 256;
+          }
+        }
       }
-      meet();
-      if (par == 0) {
-        lost = max(lost, tell[1 * 128]);
+    };
+    // half h of tile j
+    auto half_tile = [&](int j, int h) -> bool {
+      const int b = j & 1;
+      if (!mbar_wait_warp(&ctl.s_full[t][b][h], (j >> 1) & 1, abort_flag)) return false;
+      tc_fence_after();
+      const uint32_t src = t_s + b * 128 + h * 64;
+      const int col0 = j * 128 + h * 64, left = p.Nc - col0;
+      auto release = [&]() {                     // all of this half of S is in registers: the next Q K^T may overwrite it
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.s_empty[t][b][h]);
+      };
+      uint32_t xa[32], xb[32];
+      tmem_ld32(src, xa);
+      tmem_ld32(src + 32, xb);
+      tmem_ld_wait();
+      release();
+      if (left < 64) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const uint32_t o = words[(31 - i) * 128];
-          lost = max(lost, min(a[i], o));
-          a[i] = max(a[i], o);
-        }
-        tk_merge(a);
-        bool equal = lost != 0u && lost >> 7 >= a[31] >> 7;
-#pragma unroll
-        for (int i = 0; i < 31; ++i) equal |= a[i + 1] != 0u && a[i] >> 7 == a[i + 1] >> 7;
-        const uint2* other = buf + 4 * (kTkCap * 32);
-        if (__any_sync(0xffffffffu, equal)) {
-          tk_exact(buf, cnt, other, static_cast<int>(tell[2 * 128]), words);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) a[i] = words[i * 128];
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int place = 127 - static_cast<int>(a[i] & 127u);
-            a[i] = a[i] ? (place < kTkCap ? buf[place * 32].y : other[(place - kTkCap) * 32].y) : ~0u;
-          }
-        }
-        if (ok && row < p.Nq) {
-          auto column = [&](int i) { return a[i] != ~0u ? static_cast<int32_t>(a[i]) : p.pad; };
-          if (p.vec) {
-#pragma unroll
-            for (int i = 0; i < 32; i += 4)
-              if (i < p.topk) *reinterpret_cast<int4*>(out + i) = make_int4(column(i), column(i + 1), column(i + 2), column(i + 3));
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < p.topk) out[i] = column(i);
-          }
+          if (i >= left) xa[i] = 0xff800000u;   // -inf
+          if (32 + i >= left) xb[i] = 0xff800000u;
         }
       }
-      if (!ok && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+      auto go = [&](const uint32_t* x, int c) {
+        if (RANK) scan_blocks(x, c);
+        else scan(x, c);
+      };
+      go(xa, col0);
+      go(xa + 16, col0 + 16);
+      go(xb, col0 + 32);
+      go(xb + 16, col0 + 48);
+      return true;
+    };
+    if (split) {
+#pragma unroll 1
+      for (int j = 0; j < ntiles && ok; ++j) ok = half_tile(j, par);
+    } else {
+#pragma unroll 1
+      for (int u = 2 * par; u < 2 * ntiles && ok; u = (u & 1) ? u + 3 : u + 1) ok = half_tile(u >> 1, u & 1);
     }
+
+    const int cnt = static_cast<int>(at - first) >> 8;
+    const int r = quarter * 32 + lane;
+    // Q and the K ring are idle once every scan warp is here (whatever happened): per row tile 32 words per row for sorted
+    // words and columns, and two per row for what its threads tell each other
+    asm volatile("bar.sync 3, %0;" ::"n"(256 * R) : "memory");
+    uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (sbase - smem_u32(smem_raw))) + t * (35 * 128) + r;   // [place][row]
+    uint32_t* tell = words + 32 * 128;         // [list][row] largest key, [2][row] the second list's length
+    auto meet = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory"); };
+    uint32_t a[32], e[kTkCap - 32];
+    uint32_t top = 0;
+    // keys above the bound's, plus one: an empty place is 0
+    auto word = [&](int i) {
+      const uint32_t d = i < cnt ? sortable_key(__uint_as_float(buf[i * 32].x)) - base_key + 1u : 0u;
+      top = max(top, d);
+      return d;
+    };
+#pragma unroll
+    for (int i = 0; i < 32; ++i) a[i] = word(i);
+#pragma unroll
+    for (int i = 0; i < kTkCap - 32; ++i) e[i] = word(32 + i);
+    tell[par * 128] = top;
+    if (par == 1) tell[2 * 128] = static_cast<uint32_t>(cnt);
+    meet();
+    top = max(top, tell[(par ^ 1) * 128]);
+    const int shift = max(0, 7 - __clz(top | 1u));        // bits of the keys beyond 25
+    auto pack = [&](uint32_t& d, int i) { d = d ? ((d >> shift) << 7) | static_cast<uint32_t>(127 - par * kTkCap - i) : 0u; };
+#pragma unroll
+    for (int i = 0; i < 32; ++i) pack(a[i], i);
+    sort_desc<32>(a);
+    uint32_t lost = 0;                         // the largest word that is not among the row's 32
+    if (__any_sync(0xffffffffu, cnt > 32)) {
+#pragma unroll
+      for (int i = 0; i < kTkCap - 32; ++i) pack(e[i], 32 + i);
+      sort_desc<kTkCap - 32>(e);
+#pragma unroll
+      for (int i = 0; i < kTkCap - 32; ++i) {
+        lost = max(lost, min(a[31 - i], e[i]));
+        a[31 - i] = max(a[31 - i], e[i]);
+      }
+      tk_merge(a);
+    }
+    if (par == 1) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) words[i * 128] = a[i];
+      tell[1 * 128] = lost;
+    }
+    meet();
+    if (par == 0) {
+      lost = max(lost, tell[1 * 128]);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const uint32_t o = words[(31 - i) * 128];
+        lost = max(lost, min(a[i], o));
+        a[i] = max(a[i], o);
+      }
+      tk_merge(a);
+      bool equal = lost != 0u && lost >> 7 >= a[31] >> 7;
+#pragma unroll
+      for (int i = 0; i < 31; ++i) equal |= a[i + 1] != 0u && a[i] >> 7 == a[i + 1] >> 7;
+      const uint2* other = buf + 4 * (kTkCap * 32);
+      if (__any_sync(0xffffffffu, equal)) {
+        tk_exact(buf, cnt, other, static_cast<int>(tell[2 * 128]), words);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) a[i] = words[i * 128];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const int place = 127 - static_cast<int>(a[i] & 127u);
+          a[i] = a[i] ? (place < kTkCap ? buf[place * 32].y : other[(place - kTkCap) * 32].y) : ~0u;
+        }
+      }
+      if (ok && row < p.Nq) {
+        auto column = [&](int i) { return a[i] != ~0u ? static_cast<int32_t>(a[i]) : p.pad; };
+        if (p.vec) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            if (i < p.topk) *reinterpret_cast<int4*>(out + i) = make_int4(column(i), column(i + 1), column(i + 2), column(i + 3));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (i < p.topk) out[i] = column(i);
+        }
+      }
+    }
+    if (!ok && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 2) tmem_dealloc(tmem, 512);
+  if (warp == 2) tmem_dealloc(tmem, R * 256);
 }
 
 }  // namespace s3r
