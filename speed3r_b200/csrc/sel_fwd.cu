@@ -19,8 +19,10 @@ namespace s3r {
 // two at a time from a ring of two 8 KB stages; one TMA copy brings a block's keys and values.
 //   * All fragments of a stage go from shared memory to registers before the first product, so that no product
 //     waits for a load (with loads and products alternating a warp spent 2700 cycles on a pair of blocks).
-//   * The exponent offset of a row is the maximum of its first pair and moves only when a pair's sum of P passes
-//     2^24 (P keeps its relative precision, O and l are fp32): no maximum, no shuffles in between.
+//   * The exponent offset of a row is its running maximum, pair by pair: the row's largest weights are 1 and lose nothing
+//     when P is rounded to bf16.  An offset fixed by the first pair saved the maxima and their shuffles, but not the
+//     rounding: error against 64 bits 2.33e-3 instead of 2.20e-3 at unit-scale logits, 2.20e-3 instead of 1.62e-3 where a
+//     few keys hold a row's weight.
 //   * CTAs of one warp: nothing is shared between query blocks, and a finished warp makes room at once.
 // Bound: a bare TMA gather of the same blocks runs at 20 TB/s while a head's K and V fit L2 and at 10.5 TB/s at
 // 1000 views (258 MB per head).  Measured (H = 16, top-32, uniformly random blocks): 64 views 822 -> 532 us =
@@ -157,9 +159,11 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
           if (ks == 0) mma_bf16_z(s[j][t], qf[ks], kf[j][ks][2 * t], kf[j][ks][2 * t + 1]);
           else mma_bf16(s[j][t], qf[ks], kf[j][ks][2 * t], kf[j][ks][2 * t + 1]);
         }
-    if (2 * it + 1 >= nvalid) {                  // the second block is the padding of an odd list
+    if (2 * it + 1 >= nvalid) {                  // the second block is the padding of an odd list: no scores, no values
 #pragma unroll
       for (int t = 0; t < 2; ++t) s[1][t][0] = s[1][t][1] = s[1][t][2] = s[1][t][3] = -INFINITY;
+#pragma unroll
+      for (int dp = 0; dp < 4; ++dp) vf[1][dp][0] = vf[1][dp][1] = vf[1][dp][2] = vf[1][dp][3] = 0u;
     }
     if (ragged) {
 #pragma unroll
@@ -172,47 +176,44 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
             if (t * 8 + 2 * c + (e & 1) >= left) s[j][t][e] = -INFINITY;
       }
     }
-    uint32_t pk[2][4];
-    float ts[2];
-    auto exps = [&]() {
+    // the offsets follow the running maxima; O and l only when one of the warp's rows moved
+    float mn[2], neg[2];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const float2 nm = make_float2(-m_used[r], -m_used[r]), cs2 = make_float2(cs, cs);
-        float2 sum;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            float2 x = ffma2(make_float2(s[j][t][2 * r], s[j][t][2 * r + 1]), cs2, nm);
-            x.x = fast_exp2(x.x);
-            x.y = fast_exp2(x.y);
-            sum = (j | t) ? fadd2(sum, x) : x;
-            pk[j][2 * t + r] = pack_bf16(x.x, x.y);
-          }
-        ts[r] = sum.x + sum.y;
-      }
-    };
-    auto row_max = [&](int r) {
+    for (int r = 0; r < 2; ++r) {
       float m = fmax3(fmaxf(s[0][0][2 * r], s[0][0][2 * r + 1]), s[0][1][2 * r], s[0][1][2 * r + 1]);
       m = fmax3(fmax3(m, s[1][0][2 * r], s[1][0][2 * r + 1]), s[1][1][2 * r], s[1][1][2 * r + 1]);
       m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-      return fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2)) * cs;       // scale > 0 keeps the order
-    };
-    if (it == 0) { m_used[0] = row_max(0); m_used[1] = row_max(1); }
-    exps();
-    if (__any_sync(0xffffffffu, !(fmaxf(ts[0], ts[1]) <= 16777216.f))) {
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+      mn[r] = fmaxf(m_used[r], m * cs);                               // scale > 0 keeps the order
+      neg[r] = mn[r] == -INFINITY ? 0.f : -mn[r];                     // no finite score yet: P = 0
+    }
+    if (__any_sync(0xffffffffu, mn[0] != m_used[0] || mn[1] != m_used[1])) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const float mn = fmaxf(m_used[r], row_max(r)), alpha = fast_exp2(m_used[r] - mn);
-        m_used[r] = mn;
+        const float alpha = fast_exp2(m_used[r] + neg[r]);
+        m_used[r] = mn[r];
         l[r] *= alpha;
 #pragma unroll
         for (int dt = 0; dt < 8; ++dt) { o[dt][2 * r] *= alpha; o[dt][2 * r + 1] *= alpha; }
       }
-      exps();
     }
-    l[0] += ts[0];
-    l[1] += ts[1];
+    uint32_t pk[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float2 nm = make_float2(neg[r], neg[r]), cs2 = make_float2(cs, cs);
+      float2 sum;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          float2 x = ffma2(make_float2(s[j][t][2 * r], s[j][t][2 * r + 1]), cs2, nm);
+          x.x = fast_exp2(x.x);
+          x.y = fast_exp2(x.y);
+          sum = (j | t) ? fadd2(sum, x) : x;
+          pk[j][2 * t + r] = pack_bf16(x.x, x.y);
+        }
+      l[r] += sum.x + sum.y;
+    }
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -231,10 +232,10 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
     float ls = l[r];
     ls += __shfl_xor_sync(0xffffffffu, ls, 1);
     ls += __shfl_xor_sync(0xffffffffu, ls, 2);
-    inv[r] = (nvalid > 0) ? 1.0f / ls : 0.f;             // no valid key: o = 0, lse = -inf
+    const bool any = ls != 0.f;                          // no valid key, or none with a score above -inf: o = 0, lse = -inf
+    inv[r] = any ? 1.0f / ls : 0.f;
     if (p.lse_s && c == 0 && t0 + 8 * r < p.Tq)
-      p.lse_s[static_cast<int64_t>(bh) * p.Tq + t0 + 8 * r] =
-          (nvalid > 0) ? (m_used[r] + log2f(ls)) * 0.6931471805599453f : -INFINITY;
+      p.lse_s[static_cast<int64_t>(bh) * p.Tq + t0 + 8 * r] = any ? (m_used[r] + log2f(ls)) * 0.6931471805599453f : -INFINITY;
   }
   // rows of 128 bytes leave through the warp's first stage (its copies have landed and been read)
   __syncwarp();

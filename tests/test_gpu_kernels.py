@@ -59,6 +59,28 @@ def test_sel16_fwd_offset_follows_growing_scores():
     assert ((lse.cpu() - lse_ref).abs() <= 1e-4 * lse_ref.abs() + 1e-3).all()
 
 
+@pytest.mark.parametrize("block, K", [(16, 32)])
+@pytest.mark.parametrize("outgrow", [False, True])
+def test_sel_fwd_rounds_no_more_than_its_result(block, K, outgrow):
+    """Queries ten times the usual size, so that few keys hold a row's weight, and (outgrow) keys that grow along the list.
+    The largest weight has to be exactly 1 in bf16: what is left is the rounding of the result, 1.66e-3 of its 2-norm (rms of
+    rounding to 8 bits), and at most 5e-4 from the smaller weights.  Weights relative to an earlier maximum round by
+    another 1.55e-3: 2.2e-3 together."""
+    from speed3r_b200 import ops
+    B, H, T = 1, 2, 4096
+    nb = T // block
+    ln = lambda x: torch.nn.functional.layer_norm(x, (64,))
+    q, k, v = bf16_round(10 * ln(randn(1, B, H, T, 64)), ln(randn(2, B, H, T, 64)), ln(randn(3, B, H, T, 64)))
+    if outgrow:
+        k = bf16_round(k * torch.linspace(0.2, 1.5, T)[:, None])[0]
+    idx = torch.rand(B, H, nb, nb, generator=torch.Generator().manual_seed(4)).topk(K, -1).indices.sort(-1).values.int()
+    o, lse, _ = ops._sel_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), idx.to(DEV), None, None, block, 0.125, True, True, 1)
+    ref, lse_ref = R.sel_attn(q.double(), k.double(), v.double(), idx, block)
+    err = ((o.cpu().double() - ref).norm() / ref.norm()).item()
+    assert err <= 1.8e-3, f"blocks of {block}: {err:.3e}"
+    assert (lse.cpu() - lse_ref).abs().max() <= 2e-4
+
+
 # ------------------------------------------------------------------ key-centric index
 @pytest.mark.parametrize("Nq,Nkb,K", [(768, 700, 32), (769, 700, 32),           # one CTA per head | the five kernels
                                       (100, 8192, 8), (100, 8193, 8), (3000, 40, 32)])
