@@ -13,8 +13,10 @@
 // between them cost more registers and instructions than the starts they saved (574 -> 670 us).
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-7 softmax, thread = row.
 // Two CTAs per SM: their steps fill each other's waits.
-// The exponent offset of a row is the maximum of its first step; a CTA in which some row outgrew it by more than 2^64 takes
-// its keys a second time with the exact maxima (cmp_attn.cuh).
+// The exponent offset of a row is its running maximum, step by step (O is rescaled in tensor memory where a row of the warp
+// moved): the row's largest weights are 1 and lose nothing when P is rounded to bf16.  Offsets fixed by the first step saved
+// the rescaling but rounded those weights: error against 64 bits 2.33e-3 instead of 2.24e-3 at unit-scale logits, 2.28e-3
+// instead of 1.64e-3 where a few keys hold a row's weight.
 #include "sel_common.cuh"
 
 namespace s3r {
@@ -31,7 +33,7 @@ struct SbgCtl {
   uint64_t q_full, o_full;
   uint64_t k_full[kSbgStages], k_empty[kSbgStages], v_full[kSbgStages], v_empty[kSbgStages];
   uint64_t s_full, s_free, p_full, pv_done;
-  uint32_t tmem_base, abort_flag, again;
+  uint32_t tmem_base, abort_flag;
   int nvalid[4], steps;
 };
 constexpr int kSbgOffList = kSbgOffCtl + 256;  // [G][topk] int32: first token of each valid key block
@@ -53,7 +55,6 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 
   if (threadIdx.x == 0) {
     ctl.abort_flag = 0;
-    ctl.again = 0;
     mbar_init(&ctl.q_full, 1);
     mbar_init(&ctl.o_full, 1);
     for (int s = 0; s < kSbgStages; ++s) {
@@ -101,28 +102,22 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   const bool aligned = (sbase & 1023u) == 0;   // the swizzled tiles need it; dynamic shared memory starts there
   if (!aligned) steps = 0;
 
-  // Steps are counted through both passes (n = pass * steps + j), every role meets the others at the end of a pass.
-  auto another_pass = [&](int pass) {
-    __syncthreads();
-    return pass == 0 && *static_cast<volatile uint32_t*>(&ctl.again) != 0u && *abort_flag == 0u;
-  };
   if (warp < 4) {
     if (warp == 0) {
       // ---------------------------------------------------------------- TMA producer
       const bool chunked = p.Tc != p.Tk;
-      int pass = 0;
-      do {
+      {
         // lane g copies for list g; a list that has ended repeats its last block (its scores are masked, its values are
         // finite whenever the list's own are); an empty one takes the sequence's first block
-        int issued = pass * steps;
-        if (steps > 0 && pass == 0 && lane == 0) {
+        int issued = 0;
+        if (steps > 0 && lane == 0) {
           mbar_expect_tx(&ctl.q_full, kSbgTile);
           tma_load_4d_u32(sbase, &map_q, &ctl.q_full, 0, qb0 * BS, bh, 0);
         }
         const int nv = lane < G ? ctl.nvalid[lane] : 0;
         for (int j = 0; j < steps; ++j) {
-          const int n = pass * steps + j, s = n % kSbgStages;
-          const uint32_t ph = (n / kSbgStages) & 1;
+          const int s = j % kSbgStages;
+          const uint32_t ph = (j / kSbgStages) & 1;
           int tok = 0, ch = 0;
           if (lane < G && nv > 0) tok = lists[lane * p.topk + min(j, nv - 1)];
           if (chunked) { ch = tok / p.Tc; tok -= ch * p.Tc; }
@@ -130,7 +125,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           if (lane == 0) mbar_expect_tx(&ctl.k_full[s], kSbgTile);
           __syncwarp();
           if (lane < G) tma_load_4d_u32(sbase + kSbgOffK + s * kSbgTile + lane * BS * 128, &map_k, &ctl.k_full[s], 0, tok, bh, ch);
-          issued = n + 1;                                                   // K of step n is in flight
+          issued = j + 1;                                                   // K of step j is in flight
           if (!mbar_wait_warp(&ctl.v_empty[s], ph ^ 1, abort_flag)) break;
           if (lane == 0) mbar_expect_tx(&ctl.v_full[s], kSbgTile);
           __syncwarp();
@@ -144,7 +139,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           }
         }
         __syncwarp();
-      } while (another_pass(pass++));
+      }
     } else if (warp == 1) {
       // ---------------------------------------------------------------- MMA issuer
       const bool leader = elect_one_sync();
@@ -165,9 +160,9 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         umma_commit(&ctl.v_empty[s]);
       };
       bool ok = steps == 0 || mbar_wait_warp(&ctl.q_full, 0, abort_flag);
-      int pass = 0, s = 0, n = 0;
+      int s = 0;
       uint32_t ph = 0;
-      do {
+      {
         ok = ok && (steps == 0 || mbar_wait_warp(&ctl.k_full[s], ph, abort_flag));
         if (ok && steps > 0) {
           tc_fence_after();
@@ -175,19 +170,19 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           __syncwarp();
         }
 #pragma unroll 1
-        for (int j = 0; j < steps && ok; ++j, ++n) {
+        for (int j = 0; j < steps && ok; ++j) {
           const bool nxt = j + 1 < steps;
           const int sn = s + 1 == kSbgStages ? 0 : s + 1;
           const uint32_t phn = sn == 0 ? ph ^ 1u : ph;
           if (nxt) {
             ok = mbar_wait_warp(&ctl.k_full[sn], phn, abort_flag) &&
-                 mbar_wait_warp(&ctl.s_free, n & 1, abort_flag);            // S of step n is in registers
+                 mbar_wait_warp(&ctl.s_free, j & 1, abort_flag);            // S of step j is in registers
             if (!ok) break;
             tc_fence_after();
             if (leader) issue_qk(sn);
             __syncwarp();
           }
-          ok = mbar_wait_warp(&ctl.v_full[s], ph, abort_flag) && mbar_wait_warp(&ctl.p_full, n & 1, abort_flag);
+          ok = mbar_wait_warp(&ctl.v_full[s], ph, abort_flag) && mbar_wait_warp(&ctl.p_full, j & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           if (leader) issue_pv(s, j > 0 ? 1u : 0u);
@@ -199,12 +194,9 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         __syncwarp();
         if (!ok) {
           volatile uint32_t dummy = 0;
-          mbar_wait(&ctl.o_full, pass & 1, &dummy);       // let issued MMAs drain before tensor memory is freed
+          mbar_wait(&ctl.o_full, 0, &dummy);              // let issued MMAs drain before tensor memory is freed
         }
-      } while (another_pass(pass++));
-    } else {
-      int pass = 0;
-      while (another_pass(pass++)) {}
+      }
     }
   } else {
     // ------------------------------------------------------------------ softmax, thread = row
@@ -223,16 +215,10 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       tmem_st32(lane_base + kSbgColP + 32, z);
       tmem_st_wait();
     }
-    float m_used = 0.f, l = 0.f;
-    float gm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};       // running maxima, raw logits
-    auto row_max = [&]() { return fmaxf(fmaxf(gm[0], gm[1]), fmaxf(gm[2], gm[3])); };
-    auto offset = [&]() {
-      const float m = row_max();
-      return m == -INFINITY ? 0.f : m * cs;
-    };
+    float m_used = -INFINITY, l = 0.f;
     bool ok = true;
-    auto step = [&](int n, int j) -> bool {
-      if (!mbar_wait_warp(&ctl.s_full, n & 1, abort_flag)) return false;
+    auto step = [&](int j) -> bool {
+      if (!mbar_wait_warp(&ctl.s_full, j & 1, abort_flag)) return false;
       tc_fence_after();
       uint32_t x[BS / 32][32];
 #pragma unroll
@@ -249,13 +235,17 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           for (int i = 0; i < 32; ++i)
             if (c * 32 + i >= left) x[c][i] = 0xff800000u;  // -inf
       }
+      float gm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int c = 0; c < BS / 32; ++c)
 #pragma unroll
         for (int i = 0; i < 32; i += 2)
           gm[(i >> 1) & 3] = fmax3(gm[(i >> 1) & 3], __uint_as_float(x[c][i]), __uint_as_float(x[c][i + 1]));
-      if (n == 0) m_used = offset();
-      const float2 nm = make_float2(-m_used, -m_used), cs2 = make_float2(cs, cs);
+      const float mn = fmax3(m_used, fmaxf(gm[0], gm[1]) * cs, fmaxf(gm[2], gm[3]) * cs);       // scale > 0 keeps the order
+      const float neg = mn == -INFINITY ? 0.f : -mn, alpha = fast_exp2(m_used + neg);
+      const bool moved = mn != m_used;
+      m_used = mn;
+      const float2 nm = make_float2(neg, neg), cs2 = make_float2(cs, cs);
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t pk[BS / 32][16];
 #pragma unroll
@@ -274,11 +264,22 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
       }
       // P of the previous step must have been consumed: all of P waits in registers, so that its product has this long
-      if (j > 0 && !mbar_wait_warp(&ctl.pv_done, (n - 1) & 1, abort_flag)) return false;
+      if (j > 0 && !mbar_wait_warp(&ctl.pv_done, (j - 1) & 1, abort_flag)) return false;
       tc_fence_after();
+      if (j > 0 && __any_sync(0xffffffffu, moved)) {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t o[32];
+          tmem_ld32(t_o + hf * 32, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st32(t_o + hf * 32, o);
+        }
+      }
 #pragma unroll
       for (int c = 0; c < BS / 32; ++c) tmem_st16(t_p + c * 16, pk[c]);
-      l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+      l = l * alpha + ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y));
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -289,14 +290,9 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const bool live = row < p.Tq;
     uint32_t gate_word = 0;
     uint4 merged[8];                            // the row's block of the other branch
-    int pass = 0;
-    do {
-      if (pass == 1) {
-        l = 0.f;
-        m_used = offset();
-      }
+    {
 #pragma unroll 1
-      for (int j = 0; j < steps && ok; ++j) ok = step(pass * steps + j, j);
+      for (int j = 0; j < steps && ok; ++j) ok = step(j);
       // what the merge needs, on its way while the last product runs
       if (live && p.y) {
         gate_word = __ldg(reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + row * p.gst));
@@ -304,15 +300,15 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < 8; ++i) merged[i] = __ldg(oc + i);
       }
-      if (ok) ok = mbar_wait_warp(&ctl.o_full, pass & 1, abort_flag);
-      if (pass == 0 && nv > 0 && !(row_max() * cs <= m_used + 64.f)) ctl.again = 1u;
-    } while (another_pass(pass++));
+      if (ok) ok = mbar_wait_warp(&ctl.o_full, 0, abort_flag);
+    }
 
     if (ok && aligned) {
       tc_fence_after();
-      const float inv = nv > 0 ? 1.f / l : 0.f;             // no valid key: o = 0, lse = -inf
+      const bool any = m_used != -INFINITY || l != l;       // no valid key, or none with a score above -inf: o = 0, lse = -inf
+      const float inv = any ? 1.f / l : 0.f;
       if (live && p.lse_s)
-        p.lse_s[static_cast<int64_t>(bh) * p.Tq + row] = nv > 0 ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+        p.lse_s[static_cast<int64_t>(bh) * p.Tq + row] = any ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
       const float g0 = bf16_lo(gate_word), g1 = bf16_hi(gate_word);
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
@@ -322,7 +318,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           tmem_ld_wait();
         }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = nv > 0 ? __float_as_uint(__uint_as_float(o[i]) * inv) : 0u;
+        for (int i = 0; i < 32; ++i) o[i] = any ? __float_as_uint(__uint_as_float(o[i]) * inv) : 0u;
         if (!live) continue;
         auto f = [&](int i) { return __uint_as_float(o[i]); };
         if (p.o_s) {

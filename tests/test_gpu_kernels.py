@@ -59,7 +59,7 @@ def test_sel16_fwd_offset_follows_growing_scores():
     assert ((lse.cpu() - lse_ref).abs() <= 1e-4 * lse_ref.abs() + 1e-3).all()
 
 
-@pytest.mark.parametrize("block, K", [(16, 32)])
+@pytest.mark.parametrize("block, K", [(16, 32), (32, 32), (64, 16)])
 @pytest.mark.parametrize("outgrow", [False, True])
 def test_sel_fwd_rounds_no_more_than_its_result(block, K, outgrow):
     """Queries ten times the usual size, so that few keys hold a row's weight, and (outgrow) keys that grow along the list.
