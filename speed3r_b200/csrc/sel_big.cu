@@ -17,6 +17,10 @@
 // moved): the row's largest weights are 1 and lose nothing when P is rounded to bf16.  Offsets fixed by the first step saved
 // the rescaling but rounded those weights: error against 64 bits 2.33e-3 instead of 2.24e-3 at unit-scale logits, 2.28e-3
 // instead of 1.64e-3 where a few keys hold a row's weight.
+// Zero times a value that is not finite is NaN, so one such value among a query block's keys reaches every row of the tile
+// through O += P V.  A row with finite scores and an O that is not is therefore done again from its own keys alone, by its
+// thread and out of line: taking the tile's lists one by one with the tensor cores instead needed the row's state in
+// registers across the passes and cost every call a fifth (250 views 3.81 -> 4.64 ms).
 #include "sel_common.cuh"
 
 namespace s3r {
@@ -40,10 +44,53 @@ constexpr int kSbgOffList = kSbgOffCtl + 256;  // [G][topk] int32: first token o
 // two CTAs fit an SM up to 115712 bytes each: lists of up to 64 entries for blocks of 64, 48 for blocks of 32
 static_assert(sizeof(SbgCtl) <= 256, "control words");
 
+// O of one row, normalised, from the row's own keys: `list` of `nv` first tokens, weights 2^(cs q.k - m) / l.
+template <int BS>
+__device__ __noinline__ void sbg_row_alone(const SelParams& p, int bh, int row, const int32_t* list, int nv, float m, float l) {
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(p.q) + (static_cast<int64_t>(bh) * p.Tq + row) * 32;
+  const int64_t chunk = static_cast<int64_t>(p.kv_chunk_stride) / 2, in_chunk = static_cast<int64_t>(bh) * p.Tc;
+  float o[64];
+#pragma unroll
+  for (int i = 0; i < 64; ++i) o[i] = 0.f;
+#pragma unroll 1
+  for (int j = 0; j < nv; ++j) {
+    const int t0 = list[j], ch = t0 / p.Tc, n = min(BS, p.Tk - t0);
+    const int64_t at = ch * chunk + (in_chunk + t0 - ch * p.Tc) * 32;
+    const uint32_t *k = reinterpret_cast<const uint32_t*>(p.k) + at, *v = reinterpret_cast<const uint32_t*>(p.v) + at;
+#pragma unroll 1
+    for (int t = 0; t < n; ++t, k += 32, v += 32) {
+      float s = 0.f;
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) s += bf16_lo(q[i]) * bf16_lo(k[i]) + bf16_hi(q[i]) * bf16_hi(k[i]);
+      const float w = exp2f(s * p.scale_log2e - m);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        o[2 * i] += w * bf16_lo(v[i]);
+        o[2 * i + 1] += w * bf16_hi(v[i]);
+      }
+    }
+  }
+  const int b = bh / p.H, h = bh - b * p.H, qb = row / BS;
+  const float inv = 1.f / l;
+  if (p.o_s) {
+    uint32_t* dst = reinterpret_cast<uint32_t*>(p.o_s) + (static_cast<int64_t>(bh) * p.Tq + row) * 32;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) dst[i] = pack_bf16(o[2 * i] * inv, o[2 * i + 1] * inv);
+  }
+  if (p.y) {
+    const uint32_t gw = *reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + row * p.gst);
+    const uint32_t* oc = reinterpret_cast<const uint32_t*>(p.o_c) + (static_cast<int64_t>(bh) * p.nqb + qb) * 32;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(p.y) + ((static_cast<int64_t>(b) * p.Tq + row) * p.H + h) * 32;
+    const float g0 = bf16_lo(gw), g1 = bf16_hi(gw) * inv;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) dst[i] = pack_bf16(g0 * bf16_lo(oc[i]) + g1 * o[2 * i], g0 * bf16_hi(oc[i]) + g1 * o[2 * i + 1]);
+  }
+}
+
 template <int BS>
 __global__ void __launch_bounds__(kSbgThreads, 2)
 sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-               const __grid_constant__ CUtensorMap map_v, const SelParams p) {
+               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ SelParams p) {
   constexpr int G = 128 / BS;                  // query blocks per row tile
   extern __shared__ __align__(1024) uint8_t smem[];
   SbgCtl& ctl = *reinterpret_cast<SbgCtl*>(smem + kSbgOffCtl);
@@ -106,40 +153,39 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     if (warp == 0) {
       // ---------------------------------------------------------------- TMA producer
       const bool chunked = p.Tc != p.Tk;
-      {
-        // lane g copies for list g; a list that has ended repeats its last block (its scores are masked, its values are
-        // finite whenever the list's own are); an empty one takes the sequence's first block
-        int issued = 0;
-        if (steps > 0 && lane == 0) {
-          mbar_expect_tx(&ctl.q_full, kSbgTile);
-          tma_load_4d_u32(sbase, &map_q, &ctl.q_full, 0, qb0 * BS, bh, 0);
-        }
-        const int nv = lane < G ? ctl.nvalid[lane] : 0;
-        for (int j = 0; j < steps; ++j) {
-          const int s = j % kSbgStages;
-          const uint32_t ph = (j / kSbgStages) & 1;
-          int tok = 0, ch = 0;
-          if (lane < G && nv > 0) tok = lists[lane * p.topk + min(j, nv - 1)];
-          if (chunked) { ch = tok / p.Tc; tok -= ch * p.Tc; }
-          if (!mbar_wait_warp(&ctl.k_empty[s], ph ^ 1, abort_flag)) break;
-          if (lane == 0) mbar_expect_tx(&ctl.k_full[s], kSbgTile);
-          __syncwarp();
-          if (lane < G) tma_load_4d_u32(sbase + kSbgOffK + s * kSbgTile + lane * BS * 128, &map_k, &ctl.k_full[s], 0, tok, bh, ch);
-          issued = j + 1;                                                   // K of step j is in flight
-          if (!mbar_wait_warp(&ctl.v_empty[s], ph ^ 1, abort_flag)) break;
-          if (lane == 0) mbar_expect_tx(&ctl.v_full[s], kSbgTile);
-          __syncwarp();
-          if (lane < G) tma_load_4d_u32(sbase + kSbgOffV + s * kSbgTile + lane * BS * 128, &map_v, &ctl.v_full[s], 0, tok, bh, ch);
-        }
-        if (*abort_flag) {
-          // give copies already in flight a bounded chance to land before the CTA's memory is released
-          for (int n = max(0, issued - kSbgStages); n < issued; ++n) {
-            volatile uint32_t dummy = 0;
-            mbar_wait(&ctl.k_full[n % kSbgStages], (n / kSbgStages) & 1, &dummy);
-          }
-        }
-        __syncwarp();
+      // lane g copies for list g; a list that has ended, or is empty, gets zeros (rows past the end of the map)
+      int issued = 0;
+      if (steps > 0 && lane == 0) {
+        mbar_expect_tx(&ctl.q_full, kSbgTile);
+        tma_load_4d_u32(sbase, &map_q, &ctl.q_full, 0, qb0 * BS, bh, 0);
       }
+      const int nv = lane < G ? ctl.nvalid[lane] : 0;
+      for (int j = 0; j < steps; ++j) {
+        const int s = j % kSbgStages;
+        const uint32_t ph = (j / kSbgStages) & 1;
+        int tok = p.Tc, ch = 0;
+        if (j < nv) {
+          tok = lists[lane * p.topk + j];
+          if (chunked) { ch = tok / p.Tc; tok -= ch * p.Tc; }
+        }
+        if (!mbar_wait_warp(&ctl.k_empty[s], ph ^ 1, abort_flag)) break;
+        if (lane == 0) mbar_expect_tx(&ctl.k_full[s], kSbgTile);
+        __syncwarp();
+        if (lane < G) tma_load_4d_u32(sbase + kSbgOffK + s * kSbgTile + lane * BS * 128, &map_k, &ctl.k_full[s], 0, tok, bh, ch);
+        issued = j + 1;                                                   // K of step j is in flight
+        if (!mbar_wait_warp(&ctl.v_empty[s], ph ^ 1, abort_flag)) break;
+        if (lane == 0) mbar_expect_tx(&ctl.v_full[s], kSbgTile);
+        __syncwarp();
+        if (lane < G) tma_load_4d_u32(sbase + kSbgOffV + s * kSbgTile + lane * BS * 128, &map_v, &ctl.v_full[s], 0, tok, bh, ch);
+      }
+      if (*abort_flag) {
+        // give copies already in flight a bounded chance to land before the CTA's memory is released
+        for (int n = max(0, issued - kSbgStages); n < issued; ++n) {
+          volatile uint32_t dummy = 0;
+          mbar_wait(&ctl.k_full[n % kSbgStages], (n / kSbgStages) & 1, &dummy);
+        }
+      }
+      __syncwarp();
     } else if (warp == 1) {
       // ---------------------------------------------------------------- MMA issuer
       const bool leader = elect_one_sync();
@@ -162,40 +208,38 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       bool ok = steps == 0 || mbar_wait_warp(&ctl.q_full, 0, abort_flag);
       int s = 0;
       uint32_t ph = 0;
-      {
-        ok = ok && (steps == 0 || mbar_wait_warp(&ctl.k_full[s], ph, abort_flag));
-        if (ok && steps > 0) {
-          tc_fence_after();
-          if (leader) issue_qk(s);
-          __syncwarp();
-        }
+      ok = ok && (steps == 0 || mbar_wait_warp(&ctl.k_full[s], ph, abort_flag));
+      if (ok && steps > 0) {
+        tc_fence_after();
+        if (leader) issue_qk(s);
+        __syncwarp();
+      }
 #pragma unroll 1
-        for (int j = 0; j < steps && ok; ++j) {
-          const bool nxt = j + 1 < steps;
-          const int sn = s + 1 == kSbgStages ? 0 : s + 1;
-          const uint32_t phn = sn == 0 ? ph ^ 1u : ph;
-          if (nxt) {
-            ok = mbar_wait_warp(&ctl.k_full[sn], phn, abort_flag) &&
-                 mbar_wait_warp(&ctl.s_free, j & 1, abort_flag);            // S of step j is in registers
-            if (!ok) break;
-            tc_fence_after();
-            if (leader) issue_qk(sn);
-            __syncwarp();
-          }
-          ok = mbar_wait_warp(&ctl.v_full[s], ph, abort_flag) && mbar_wait_warp(&ctl.p_full, j & 1, abort_flag);
+      for (int j = 0; j < steps && ok; ++j) {
+        const bool nxt = j + 1 < steps;
+        const int sn = s + 1 == kSbgStages ? 0 : s + 1;
+        const uint32_t phn = sn == 0 ? ph ^ 1u : ph;
+        if (nxt) {
+          ok = mbar_wait_warp(&ctl.k_full[sn], phn, abort_flag) &&
+               mbar_wait_warp(&ctl.s_free, j & 1, abort_flag);            // S of step j is in registers
           if (!ok) break;
           tc_fence_after();
-          if (leader) issue_pv(s, j > 0 ? 1u : 0u);
+          if (leader) issue_qk(sn);
           __syncwarp();
-          s = sn;
-          ph = phn;
         }
-        if (leader) umma_commit(&ctl.o_full);
+        ok = mbar_wait_warp(&ctl.v_full[s], ph, abort_flag) && mbar_wait_warp(&ctl.p_full, j & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        if (leader) issue_pv(s, j > 0 ? 1u : 0u);
         __syncwarp();
-        if (!ok) {
-          volatile uint32_t dummy = 0;
-          mbar_wait(&ctl.o_full, 0, &dummy);              // let issued MMAs drain before tensor memory is freed
-        }
+        s = sn;
+        ph = phn;
+      }
+      if (leader) umma_commit(&ctl.o_full);
+      __syncwarp();
+      if (!ok) {
+        volatile uint32_t dummy = 0;
+        mbar_wait(&ctl.o_full, 0, &dummy);              // let issued MMAs drain before tensor memory is freed
       }
     }
   } else {
@@ -290,18 +334,16 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const bool live = row < p.Tq;
     uint32_t gate_word = 0;
     uint4 merged[8];                            // the row's block of the other branch
-    {
 #pragma unroll 1
-      for (int j = 0; j < steps && ok; ++j) ok = step(j);
-      // what the merge needs, on its way while the last product runs
-      if (live && p.y) {
-        gate_word = __ldg(reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + row * p.gst));
-        const uint4* oc = reinterpret_cast<const uint4*>(p.o_c + (static_cast<int64_t>(bh) * p.nqb + qb0 + g) * 64);
+    for (int j = 0; j < steps && ok; ++j) ok = step(j);
+    // what the merge needs, on its way while the last product runs
+    if (live && p.y) {
+      gate_word = __ldg(reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + row * p.gst));
+      const uint4* oc = reinterpret_cast<const uint4*>(p.o_c + (static_cast<int64_t>(bh) * p.nqb + qb0 + g) * 64);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) merged[i] = __ldg(oc + i);
-      }
-      if (ok) ok = mbar_wait_warp(&ctl.o_full, 0, abort_flag);
+      for (int i = 0; i < 8; ++i) merged[i] = __ldg(oc + i);
     }
+    if (ok) ok = mbar_wait_warp(&ctl.o_full, 0, abort_flag);
 
     if (ok && aligned) {
       tc_fence_after();
@@ -310,6 +352,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       if (live && p.lse_s)
         p.lse_s[static_cast<int64_t>(bh) * p.Tq + row] = any ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
       const float g0 = bf16_lo(gate_word), g1 = bf16_hi(gate_word);
+      float2 off = make_float2(0.f, 0.f);                   // NaN where some value of O is not finite
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t o[32];
@@ -319,16 +362,18 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
 #pragma unroll
         for (int i = 0; i < 32; ++i) o[i] = any ? __float_as_uint(__uint_as_float(o[i]) * inv) : 0u;
-        if (!live) continue;
+#pragma unroll
+        for (int i = 0; i < 32; i += 2)
+          off = ffma2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), make_float2(0.f, 0.f), off);
         auto f = [&](int i) { return __uint_as_float(o[i]); };
-        if (p.o_s) {
+        if (live && p.o_s) {
           uint4* dst = reinterpret_cast<uint4*>(p.o_s + (static_cast<int64_t>(bh) * p.Tq + row) * 64 + hf * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             dst[i] = make_uint4(pack_bf16(f(8 * i), f(8 * i + 1)), pack_bf16(f(8 * i + 2), f(8 * i + 3)),
                                 pack_bf16(f(8 * i + 4), f(8 * i + 5)), pack_bf16(f(8 * i + 6), f(8 * i + 7)));
         }
-        if (p.y) {
+        if (live && p.y) {
           uint4* dst = reinterpret_cast<uint4*>(p.y + ((static_cast<int64_t>(b) * p.Tq + row) * p.H + h) * 64 + hf * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -342,6 +387,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           }
         }
       }
+      if (live && any && l - l == 0.f && !(off.x + off.y == 0.f)) sbg_row_alone<BS>(p, bh, row, list, nv, m_used, l);
     }
     if ((!ok || !aligned) && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
   }
@@ -352,8 +398,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 }
 
 template <int BS>
-static int launch_sel_big(const void* q, const void* k, const void* v, int kv_chunks, int64_t kv_chunk_stride, const SelParams& p,
-                          cudaStream_t st) {
+static int launch_sel_big(int kv_chunks, const SelParams& p, cudaStream_t st) {
   constexpr int G = 128 / BS;
   const int BH = p.B * p.H;
   CUtensorMap mq, mk, mv;
@@ -361,16 +406,16 @@ static int launch_sel_big(const void* q, const void* k, const void* v, int kv_ch
   {
     const uint64_t dims[4] = {64, tq, bh, 1}, strides[3] = {128, tq * 128, tq * 128 * bh};
     const uint32_t box[4] = {64, 128, 1, 1};
-    const int rc = make_tensor_map(&mq, q, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    const int rc = make_tensor_map(&mq, p.q, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
   }
   {
     const uint64_t dims[4] = {64, tc, bh, static_cast<uint64_t>(kv_chunks)};
-    const uint64_t strides[3] = {128, tc * 128, kv_chunks > 1 ? static_cast<uint64_t>(kv_chunk_stride) * 2 : tc * 128 * bh};
+    const uint64_t strides[3] = {128, tc * 128, kv_chunks > 1 ? static_cast<uint64_t>(p.kv_chunk_stride) * 2 : tc * 128 * bh};
     const uint32_t box[4] = {64, static_cast<uint32_t>(BS), 1, 1};
-    int rc = make_tensor_map(&mk, k, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    int rc = make_tensor_map(&mk, p.k, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    rc = make_tensor_map(&mv, v, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    rc = make_tensor_map(&mv, p.v, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
   }
   const int64_t grid = static_cast<int64_t>(BH) * ((p.nqb + G - 1) / G);
@@ -380,10 +425,8 @@ static int launch_sel_big(const void* q, const void* k, const void* v, int kv_ch
   return launch(sel_big_kernel<BS>, static_cast<unsigned>(grid), kSbgThreads, smem, st, mq, mk, mv, p);
 }
 
-int sel_big_fwd(const void* q, const void* k, const void* v, int kv_chunks, int64_t kv_chunk_stride, int block, const SelParams& p,
-                cudaStream_t st) {
-  return block == 32 ? launch_sel_big<32>(q, k, v, kv_chunks, kv_chunk_stride, p, st)
-                     : launch_sel_big<64>(q, k, v, kv_chunks, kv_chunk_stride, p, st);
+int sel_big_fwd(int kv_chunks, int block, const SelParams& p, cudaStream_t st) {
+  return block == 32 ? launch_sel_big<32>(kv_chunks, p, st) : launch_sel_big<64>(kv_chunks, p, st);
 }
 
 }  // namespace s3r

@@ -5,6 +5,8 @@
 namespace s3r {
 
 struct SelParams {
+  const __nv_bfloat16 *q, *k, *v;
+  int64_t kv_chunk_stride;       // elements
   const int32_t* idx;
   __nv_bfloat16* o_s;
   float* lse_s;
@@ -16,8 +18,7 @@ struct SelParams {
   float scale_log2e;
   uint32_t* status;
 };
-// Blocks of 32 and 64 tokens; kv_chunk_stride in elements.
-int sel_big_fwd(const void* q, const void* k, const void* v, int kv_chunks, int64_t kv_chunk_stride, int block, const SelParams& p,
-                cudaStream_t st);
+// Blocks of 32 and 64 tokens.
+int sel_big_fwd(int kv_chunks, int block, const SelParams& p, cudaStream_t st);
 
 }  // namespace s3r

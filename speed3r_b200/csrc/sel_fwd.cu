@@ -344,6 +344,10 @@ extern "C" int s3r_sel_attn_fwd(const void* q, const void* k, const void* v, int
     return launch_sel16_fwd(mkv, p, static_cast<int64_t>(BH) * p.nqb, st);
   }
   SelParams p;
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.k = static_cast<const __nv_bfloat16*>(k);
+  p.v = static_cast<const __nv_bfloat16*>(v);
+  p.kv_chunk_stride = kv_chunk_stride;
   p.idx = idx;
   p.o_s = static_cast<__nv_bfloat16*>(o_s);
   p.lse_s = lse_s;
@@ -356,5 +360,5 @@ extern "C" int s3r_sel_attn_fwd(const void* q, const void* k, const void* v, int
   p.topk = topk;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.status = status;
-  return sel_big_fwd(q, k, v, kv_chunks, kv_chunk_stride, block, p, st);
+  return sel_big_fwd(kv_chunks, block, p, st);
 }

@@ -81,6 +81,41 @@ def test_sel_fwd_rounds_no_more_than_its_result(block, K, outgrow):
     assert (lse.cpu() - lse_ref).abs().max() <= 2e-4
 
 
+@pytest.mark.parametrize("block", [16, 32, 64])
+@pytest.mark.parametrize("chunks", [1, 2])
+def test_sel_fwd_keeps_non_finite_values_to_the_blocks_that_selected_them(block, chunks):
+    """Infinities and NaN in the values of single key blocks, among them the sequence's first, beside query blocks of the
+    same row tile with other lists, a shorter list and none at all: rows of the others are the oracle's, and outside those
+    row tiles bit for bit what they are without such values; rows of their own have infinities and NaN where the oracle has
+    them."""
+    from speed3r_b200 import ops
+    B, H, T, K = 1, 2, 1024, 4
+    nb = T // block
+    q, k, v = bf16_round(randn(1, B, H, T, 64), randn(2, B, H, T, 64), randn(3, B, H, T, 64))
+    idx = 4 + table(4, B, H, nb, nb - 4, K)                        # blocks 0 to 3 by hand
+    idx[:, :, 0, 1], idx[:, :, 5, 2], idx[:, :, 9, 0] = 0, 1, 2
+    idx[:, :, 1] = -1                                              # none
+    idx[:, :, 4, 1:] = -1                                          # one block
+    bad = v.clone()
+    bad[:, :, 3, 5], bad[:, :, block + 1, 7], bad[:, :, 2 * block + 2, 60] = float("inf"), float("nan"), float("-inf")
+    def run(x):
+        t = lambda a: a.to(DEV, torch.bfloat16)
+        part = lambda a: t(a).view(B, H, chunks, T // chunks, 64).permute(2, 0, 1, 3, 4).contiguous() if chunks > 1 else t(a)
+        return ops._sel_fwd(t(q), part(k), part(x), idx.to(DEV), None, None, block, 0.125, True, True, chunks)[:2]
+    (o, lse), (o_clean, lse_clean) = run(bad), run(v)
+    hit = torch.zeros(T, dtype=torch.bool)
+    for m in (0, 5, 9):
+        hit[m * block:(m + 1) * block] = True
+    assert torch.equal(lse, lse_clean) and torch.equal(o[:, :, 9 * block + 128:], o_clean[:, :, 9 * block + 128:])
+    ref, _ = R.sel_attn(q, k, bad, idx, block)
+    ref[:, :, block:2 * block] = 0                                 # the query block without a list
+    assert_bf16_close(o.cpu()[:, :, ~hit], ref[:, :, ~hit], f"blocks of {block}, the others")
+    got, want = o.cpu().float()[:, :, hit], ref[:, :, hit]
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+    fin = want.isfinite()
+    assert_bf16_close(got[fin], want[fin], f"blocks of {block}")
+
+
 # ------------------------------------------------------------------ key-centric index
 @pytest.mark.parametrize("Nq,Nkb,K", [(768, 700, 32), (769, 700, 32),           # one CTA per head | the five kernels
                                       (100, 8192, 8), (100, 8193, 8), (3000, 40, 32)])
