@@ -121,7 +121,6 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     tmem_relinquish();
   }
   griddep_wait();
-  griddep_launch();
   if (warp >= 4 && warp < 4 + G) {
     // valid entries of one query block's row of the table, table order
     const int g = warp - 4, qb = qb0 + g;
@@ -141,6 +140,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  griddep_launch();                            // not before this CTA has its tensor memory: a CTA of the next kernel could take it
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
   int steps = ctl.nvalid[0];
