@@ -255,8 +255,8 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
 #pragma unroll
     for (int i = 0; i < 32; ++i) gm[i] = RANK ? 0.f : -INFINITY;
     float raw = -INFINITY;                      // RANK 1: largest raw logit
-    auto half_max = [&]() {
-      if (RANK) return raw;
+    auto half_max = [&]() {                     // of what is not NaN
+      if (RANK) return fmaxf(raw, -INFINITY);
       float m[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -282,8 +282,8 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
     auto take_maxima = [&](const uint32_t (&x)[16], int c) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        if (RANK) raw = fmax3(raw, __uint_as_float(x[i]), __uint_as_float(x[8 + i]));
-        else gm[c * 8 + i] = fmax3(gm[c * 8 + i], __uint_as_float(x[i]), __uint_as_float(x[8 + i]));
+        if (RANK) raw = fmax3_nan(raw, __uint_as_float(x[i]), __uint_as_float(x[8 + i]));
+        else gm[c * 8 + i] = fmax3_nan(gm[c * 8 + i], __uint_as_float(x[i]), __uint_as_float(x[8 + i]));
       }
     };
     const float2 w01 = make_float2(1.f, p.rank_take > 1 ? 1.f : 0.f),
@@ -387,6 +387,17 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
       if (pass == 0 && !(half_max() * cs <= m_used + 64.f)) ctl.again = 1u;
     } while (another_pass(pass++));
 
+    // A row with a NaN or an infinite score is NaN throughout; the polynomial exponentials have made numbers of them.  A
+    // group with a NaN counts as empty: the bound stays one.
+    bool bad = RANK && !(raw < INFINITY);
+    if (!RANK) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        bad |= !(gm[i] < INFINITY);
+        gm[i] = fmaxf(gm[i], -INFINITY);
+      }
+    }
+    if (bad) l = __uint_as_float(0x7fffffffu);
     // epilogue: the bound (topk-th largest of the row's 64 maxima: with both threads' 32 sorted, the larger of a[i] and
     // b[topk - 1 - i] over i < topk are the upper topk), lse and O / l.  The K ring is free by now.
     sort_desc<32>(gm);

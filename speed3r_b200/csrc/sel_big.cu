@@ -284,9 +284,10 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       for (int c = 0; c < BS / 32; ++c)
 #pragma unroll
         for (int i = 0; i < 32; i += 2)
-          gm[(i >> 1) & 3] = fmax3(gm[(i >> 1) & 3], __uint_as_float(x[c][i]), __uint_as_float(x[c][i + 1]));
-      const float mn = fmax3(m_used, fmaxf(gm[0], gm[1]) * cs, fmaxf(gm[2], gm[3]) * cs);       // scale > 0 keeps the order
-      const float neg = mn == -INFINITY ? 0.f : -mn, alpha = fast_exp2(m_used + neg);
+          gm[(i >> 1) & 3] = fmax3_nan(gm[(i >> 1) & 3], __uint_as_float(x[c][i]), __uint_as_float(x[c][i + 1]));
+      // scale > 0 keeps the order; a NaN, or a score of +infinity (0 x inf), makes the offset and with it the row NaN
+      const float mn = fmax3_nan(m_used, fmax3_nan(gm[0], gm[1], gm[2]) * cs, gm[3] * cs);
+      const float neg = mn == -INFINITY ? 0.f : fmaf(mn, 0.f, -mn), alpha = fast_exp2(m_used + neg);
       const bool moved = mn != m_used;
       m_used = mn;
       const float2 nm = make_float2(neg, neg), cs2 = make_float2(cs, cs);

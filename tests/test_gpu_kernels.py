@@ -116,6 +116,34 @@ def test_sel_fwd_keeps_non_finite_values_to_the_blocks_that_selected_them(block,
     assert_bf16_close(got[fin], want[fin], f"blocks of {block}")
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("first", [0, 200])
+def test_nan_scores_are_not_lost(first, value):
+    """A NaN in one key (or an infinity, whose score is +infinity in half of the rows) makes the rows that see it NaN, wherever in a tile the key stands (head h: key first + h; some
+    exponentials are polynomials, whose clamp and exponent arithmetic could make a number of it), and is never ranked."""
+    from speed3r_b200 import ops
+    B, H, T = 1, 32, 512
+    q, k, v = bf16_round(randn(1, B, H, T, 64), randn(2, B, H, T, 64), randn(3, B, H, T, 64))
+    for h in range(H):
+        k[0, h, first + h, 3] = value
+    nan = torch.full((B, H, T), True) if value != value else q[..., 3] > 0        # -infinity: the key has no weight
+    t = [x.to(DEV, torch.bfloat16) for x in (q, k, v)]
+    o, lse, idx = ops._cmp_fwd(*t, 32, 0.125)
+    assert torch.equal(o.isnan().all(-1).cpu(), nan) and torch.equal(o.isnan().any(-1).cpu(), nan)
+    assert torch.equal(lse.isnan().cpu(), nan)
+    ranked = (idx.cpu() == (first + torch.arange(H))[None, :, None, None]).any(-1)
+    assert not ranked.any() if value != value else torch.equal(ranked, nan)
+    _, _, blocks = ops._ops().cmp_attn_blocktopk_fwd.default(*t, 16, 0.125, 4, 3)
+    if value != value:
+        assert (blocks.cpu() != ((first + torch.arange(H)) // 4)[None, :, None, None]).masked_fill(((first + torch.arange(H)) % 4 == 3)[None, :, None, None], True).all()
+    for block in (16, 32, 64):
+        nb = T // block
+        table = torch.arange(nb, dtype=torch.int32).expand(B, H, nb, nb).contiguous().to(DEV)
+        o, lse, _ = ops._sel_fwd(*t, table, None, None, block, 0.125, True, True, 1)
+        assert torch.equal(o.isnan().all(-1).cpu(), nan) and torch.equal(o.isnan().any(-1).cpu(), nan), f"blocks of {block}"
+        assert torch.equal(lse.isnan().cpu(), nan), f"blocks of {block}"
+
+
 # ------------------------------------------------------------------ key-centric index
 @pytest.mark.parametrize("Nq,Nkb,K", [(768, 700, 32), (769, 700, 32),           # one CTA per head | the five kernels
                                       (100, 8192, 8), (100, 8193, 8), (3000, 40, 32)])

@@ -36,3 +36,20 @@ def test_next_kernel_starts_after_tensor_memory_is_allocated(path, at):
     launch = body.find("griddep_launch()")
     barrier = body.find("__syncthreads()", at)
     assert 0 <= barrier < launch, "griddep_launch() before the barrier behind tcgen05.alloc"
+
+
+def test_polynomial_exponential_is_as_exact_as_stated():
+    """2^f on [-1/2, 1/2] with the coefficients of exp2_fma2, in 64 bits and with every step rounded to fp32."""
+    import numpy as np
+    src = open(os.path.join(CSRC, "common.cuh")).read()
+    body = src[src.index("float2 exp2_fma2(float2 x)"):]
+    body = body[:body.index("\n}")]
+    coeff = [np.float32(c) for c in re.findall(r"make_float2\(([0-9.e+-]+)f, \1f\)", body)][2:]      # behind the two shifts
+    assert len(coeff) == 6 and coeff[-1] == 1
+    f = np.linspace(-0.5, 0.5, 200001).astype(np.float32).astype(np.float64)
+    exact = r = np.zeros_like(f)
+    for c in coeff:
+        exact = exact * f + np.float64(c)
+        r = (r * f + np.float64(c)).astype(np.float32).astype(np.float64)
+    assert np.abs(exact / 2.0 ** f - 1).max() < 1.65e-7
+    assert np.abs(r / 2.0 ** f - 1).max() < 2.25e-7
