@@ -86,7 +86,7 @@ int s3r_pool_bwd(const void* d_out, void* d_in, int64_t stride_b, int64_t stride
  *   cos_tab/sin_tab: [tab_rows, d/2] bf16, row p = cos/sin of bf16(p * inv_freq) duplicated over the two
  *                    halves (what RoPE2D caches); a position outside the table is clamped and
  *                    raises S3R_STATUS_BAD_INDEX in the device status word
- *   q_weight..k_bias: fp32 [d] LayerNorm affine parameters, or all NULL (Identity norms)
+ *   q_weight..k_bias: fp32 [d] LayerNorm affine parameters, 8-byte aligned, or all NULL (Identity norms)
  *   q,k,v          : [B,H,N,d] bf16 out;  q_c,k_c,v_c : [B,H,N/block,d] bf16 out
  * N must be a multiple of `block`; d = 64; at most 42 heads.  Forward only: a caller that
  * needs gradients calls s3r_qkv_prologue_bwd. */

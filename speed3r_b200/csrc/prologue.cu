@@ -474,6 +474,9 @@ static int prologue_fwd(const void* qkv, int64_t tok_stride, const void* gate_in
                        reinterpret_cast<uintptr_t>(k_c) | reinterpret_cast<uintptr_t>(v_c) |
                        reinterpret_cast<uintptr_t>(cos_tab) | reinterpret_cast<uintptr_t>(sin_tab);
   S3R_REQUIRE((al & 15) == 0, S3R_ERR_ALIGNMENT, "s3r_qkv_prologue_fwd: tensors must be 16-byte aligned");
+  const uintptr_t al8 = reinterpret_cast<uintptr_t>(q_weight) | reinterpret_cast<uintptr_t>(q_bias) |
+                        reinterpret_cast<uintptr_t>(k_weight) | reinterpret_cast<uintptr_t>(k_bias);
+  S3R_REQUIRE((al8 & 7) == 0, S3R_ERR_ALIGNMENT, "s3r_qkv_prologue_fwd: LayerNorm parameters must be 8-byte aligned");
   const int Nc = N / block;
   const int64_t grid = static_cast<int64_t>(B) * Nc;
   S3R_REQUIRE(grid < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_qkv_prologue_fwd: grid of %lld CTAs is too large",
@@ -547,6 +550,8 @@ static int prologue_bwd(const void* qkv, int64_t tok_stride, const void* gate, c
   uintptr_t al = reinterpret_cast<uintptr_t>(cos_tab) | reinterpret_cast<uintptr_t>(sin_tab) | reinterpret_cast<uintptr_t>(dqkv);
   for (const void* t : {qkv, dq, dk, dv, dq_c, dk_c, dv_c}) al |= reinterpret_cast<uintptr_t>(t);
   S3R_REQUIRE((al & 15) == 0, S3R_ERR_ALIGNMENT, "s3r_qkv_prologue_bwd: tensors must be 16-byte aligned");
+  S3R_REQUIRE(((reinterpret_cast<uintptr_t>(q_weight) | reinterpret_cast<uintptr_t>(k_weight)) & 7) == 0, S3R_ERR_ALIGNMENT,
+              "s3r_qkv_prologue_bwd: LayerNorm parameters must be 8-byte aligned");
   const int Nc = N / block;
   S3R_REQUIRE(static_cast<int64_t>(B) * Nc < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_qkv_prologue_bwd: too many blocks");
   PrologueBwdParams p;

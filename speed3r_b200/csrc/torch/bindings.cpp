@@ -53,6 +53,10 @@ Tensor fresh(at::IntArrayRef shape, const Tensor& like, at::ScalarType dtype) {
 }
 // contiguous, whatever the strides of `t` (at::empty_like would keep a permuted layout)
 Tensor fresh_like(const Tensor& t) { return at::empty(t.sizes(), t.options()); }
+// The same values at a multiple of 16 bytes: a contiguous view may begin anywhere in its storage (a slice, a flattened
+// parameter buffer), and the kernels load vectors.
+Tensor aligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(); }
+optional<Tensor> aligned(const optional<Tensor>& t) { return t.has_value() ? optional<Tensor>(aligned(*t)) : t; }
 Tensor none(const Tensor& like) { return at::empty({0}, like.options()); }
 
 // ------------------------------------------------------------------------------------------------
@@ -353,11 +357,12 @@ int64_t need_prologue(const Tensor& qkv, int64_t heads, int64_t block, const opt
 
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> prologue_fwd(
     const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos, const optional<Tensor>& cos,
-    const optional<Tensor>& sin, const optional<Tensor>& qw, const optional<Tensor>& qb, const optional<Tensor>& kw,
-    const optional<Tensor>& kb, double eps) {
-  const int64_t rows = need_prologue(qkv, heads, block, pos, cos, sin, {&qw, &qb, &kw, &kb});
+    const optional<Tensor>& sin, const optional<Tensor>& qw_, const optional<Tensor>& qb_, const optional<Tensor>& kw_,
+    const optional<Tensor>& kb_, double eps) {
+  const int64_t rows = need_prologue(qkv, heads, block, pos, cos, sin, {&qw_, &qb_, &kw_, &kb_});
   const int64_t B = qkv.size(0), N = qkv.size(1), d = qkv.numel() / (B * N) / (3 * heads);
   c10::cuda::CUDAGuard guard(qkv.device());
+  const auto qw = aligned(qw_), qb = aligned(qb_), kw = aligned(kw_), kb = aligned(kb_);
   Tensor t[6];
   for (int i = 0; i < 6; ++i) t[i] = fresh({B, heads, i < 3 ? N : N / block, d}, qkv, at::kBFloat16);
   const bool rope = pos.has_value();
@@ -370,13 +375,14 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> prologue_fwd(
 
 // (gradient of qkv, [4,64] gradients of q weight, q bias, k weight, k bias; no elements without norms)
 std::tuple<Tensor, Tensor> prologue_bwd(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos,
-                                        const optional<Tensor>& cos, const optional<Tensor>& sin, const optional<Tensor>& qw,
-                                        const optional<Tensor>& kw, double eps, const Tensor& dq, const Tensor& dk,
+                                        const optional<Tensor>& cos, const optional<Tensor>& sin, const optional<Tensor>& qw_,
+                                        const optional<Tensor>& kw_, double eps, const Tensor& dq, const Tensor& dk,
                                         const Tensor& dv, const Tensor& dq_c, const Tensor& dk_c, const Tensor& dv_c) {
-  const int64_t rows = need_prologue(qkv, heads, block, pos, cos, sin, {&qw, &kw});
+  const int64_t rows = need_prologue(qkv, heads, block, pos, cos, sin, {&qw_, &kw_});
   for (const Tensor* g : {&dq, &dk, &dv, &dq_c, &dk_c, &dv_c}) need(*g, "gradient");
   const int64_t B = qkv.size(0), N = qkv.size(1), d = qkv.numel() / (B * N) / (3 * heads);
   c10::cuda::CUDAGuard guard(qkv.device());
+  const auto qw = aligned(qw_), kw = aligned(kw_);
   const bool norm = qw.has_value(), rope = pos.has_value();
   const size_t nbytes = norm ? s3r_qkv_prologue_bwd_workspace_bytes(B, heads, N, block) : 0;
   Tensor dqkv = fresh_like(qkv), ws = fresh({static_cast<int64_t>(nbytes)}, qkv, at::kByte),
@@ -615,7 +621,8 @@ std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, c
   auto as = [&](const optional<Tensor>& t, at::ScalarType type) {
     return t.has_value() ? optional<Tensor>(t->to(x_.device(), type).contiguous()) : t;
   };
-  const auto pos = as(pos_, at::kLong), qw = as(qw_, at::kFloat), qb = as(qb_, at::kFloat), kw = as(kw_, at::kFloat), kb = as(kb_, at::kFloat);
+  const auto pos = as(pos_, at::kLong), qw = aligned(as(qw_, at::kFloat)), qb = aligned(as(qb_, at::kFloat)),
+             kw = aligned(as(kw_, at::kFloat)), kb = aligned(as(kb_, at::kFloat));
 
   // one GEMM for qkv and gate when both weights have to be cast anyway
   const bool merged = w_qkv.scalar_type() == at::kFloat && w_gate.scalar_type() == at::kFloat && H % 4 == 0 &&
@@ -766,13 +773,14 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x_, const Tensor& w_qkv, const optional<Tensor>& b_qkv,
                                const Tensor& w_gate, const optional<Tensor>& b_gate, const Tensor& w_proj,
                                const optional<Tensor>& b_proj, const optional<Tensor>& pos, const optional<Tensor>& cos,
-                               const optional<Tensor>& sin, const optional<Tensor>& qw, const optional<Tensor>& qb,
-                               const optional<Tensor>& kw, const optional<Tensor>& kb, double eps, int64_t heads, int64_t block,
+                               const optional<Tensor>& sin, const optional<Tensor>& qw_, const optional<Tensor>& qb_,
+                               const optional<Tensor>& kw_, const optional<Tensor>& kb_, double eps, int64_t heads, int64_t block,
                                int64_t topk, double scale) {
     at::AutoDispatchBelowAutograd below;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     c10::cuda::CUDAGuard guard(x_.device());
     void* st = stream();
+    const auto qw = aligned(qw_), qb = aligned(qb_), kw = aligned(kw_), kb = aligned(kb_);
     const bool x_wide = x_.scalar_type() == at::kFloat;
     const ModulePlan m(x_.sizes(), heads, block, topk, x_wide, w_proj.size(0));
     const Tensor buf = at::empty({m.used}, x_.options().dtype(at::kBFloat16)), x = x_.contiguous();
@@ -821,7 +829,7 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     gemm(out, view(m.y, m.M, m.C), view(m.wp, w_proj.size(0), m.C), b_proj.has_value(), m.bp);
 
     auto or_none = [](const optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); };
-    ctx->save_for_backward({buf, x_wide ? Tensor() : x, idx, or_none(pos), or_none(cos), or_none(sin), or_none(qw), or_none(kw)});
+    ctx->save_for_backward({buf, x_wide ? Tensor() : x, idx, or_none(pos), or_none(cos), or_none(sin), or_none(qw_), or_none(kw_)});
     ctx->saved_data["shape"] = x_.sizes().vec();
     ctx->saved_data["ints"] = std::vector<int64_t>{heads, block, topk, w_proj.size(0), b_qkv.has_value(), b_proj.has_value()};
     ctx->saved_data["eps"] = eps;
@@ -840,6 +848,7 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     const double eps = ctx->saved_data["eps"].toDouble(), scale = ctx->saved_data["scale"].toDouble();
     const int64_t out_features = ints[3];
     const bool x_wide = !s[1].defined(), rope = s[3].defined(), norm = s[6].defined();
+    const Tensor qw = norm ? aligned(s[6]) : s[6], kw = norm ? aligned(s[7]) : s[7];
     const ModulePlan m(shape, ints[0], ints[1], ints[2], x_wide, out_features);
     const size_t e_gate = ints[4] ? 3 : 2, e_wp = e_gate + (ints[4] ? 2 : 1);      // edges: absent biases have none
     c10::cuda::CUDAGuard guard(buf.device());
@@ -896,7 +905,7 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     const Tensor dparams = at::empty({norm ? 4 : 0, m.d}, buf.options().dtype(at::kFloat));
     check(s3r_qkv_gate_prologue_bwd(ptr(m.proj), rope ? static_cast<const int64_t*>(s[3].data_ptr()) : nullptr,
                                     rope ? s[4].data_ptr() : nullptr, rope ? s[5].data_ptr() : nullptr, rope ? s[4].size(0) : 0,
-                                    norm ? f32(s[6]) : nullptr, norm ? f32(s[7]) : nullptr, eps, sp(a_dq), sp(a_dk), sp(a_dv), sp(a_dqc),
+                                    norm ? f32(qw) : nullptr, norm ? f32(kw) : nullptr, eps, sp(a_dq), sp(a_dk), sp(a_dv), sp(a_dqc),
                                     sp(a_dkc), sp(a_dvc), ptr(m.gate), sf(a_dgate), sp(a_dproj), norm ? f32(dparams) : nullptr, sp(a_pro),
                                     pro_bytes, m.B, m.H, m.N, m.d, m.block, st), "s3r_qkv_gate_prologue_bwd");
     // first projection

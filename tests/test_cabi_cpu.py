@@ -74,6 +74,13 @@ def test_argument_errors_are_reported_without_a_gpu(lib):
     assert pro(H=43) == -2 and "heads" in _lib.last_error()
     assert pro(qw=p) == -4
     assert pro(pos=p) == -4 and "tables" in _lib.last_error()
+    # LayerNorm parameters are loaded in pairs
+    for name in ("qw", "qb", "kw", "kb"):
+        assert pro(**{n: p + 4 * (n == name) for n in ("qw", "qb", "kw", "kb")}) == -3 and "8-byte" in _lib.last_error()
+    for off in ((4, 0), (0, 4)):
+        rc = lib.s3r_qkv_prologue_bwd(p, None, None, None, 0, p + off[0], p + off[1], 1e-5, p, p, p, p, p, p, p, p, p, 1 << 30,
+                                      1, 4, 32, 64, 16, None)
+        assert rc == -3 and "8-byte" in _lib.last_error()
     # merge arguments must come together
     rc = lib.s3r_sel_attn_fwd(p, p, p, 1, 0, p, p, None, p, 0, 0, 0, None, None, 1, 1, 64, 64, 64, 16, 8, 0.125, None)
     assert rc == -4

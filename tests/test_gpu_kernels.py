@@ -537,3 +537,48 @@ def test_colsum(rows, cols):
     _lib.check(lib.s3r_colsum(x.data_ptr(), out.data_ptr(), rows, cols, ws.data_ptr(), n, torch.cuda.current_stream().cuda_stream), "s3r_colsum")
     ref = x.double().sum(0)
     assert ((out.double() - ref).abs() <= 2 ** -24 * rows * x.double().abs().sum(0) / rows * 64 + 1e-6).all()
+
+
+# ------------------------------------------------------------------ the attention module
+def module_and_input(seed, B=1, N=512, H=4, dim=None, **kw):
+    import speed3r_b200
+    dim = H * 64 if dim is None else dim
+    torch.manual_seed(seed)
+    m = speed3r_b200.SparseFlashAttentionRope(dim, num_heads=H, qkv_bias=True, qk_norm=True, rope=speed3r_b200.RoPE2D(100.0), **kw)
+    with torch.no_grad():
+        for p in m.parameters():
+            p.add_(0.05 * torch.randn_like(p))
+    x = torch.randn(B, N, dim)
+    pos = torch.stack((torch.arange(N) % 256 // 16, torch.arange(N) % 16), -1)[None].expand(B, -1, -1).contiguous()
+    return m.to(DEV), x.to(DEV), pos.to(DEV)
+
+
+def module_step(m, x, pos, dy=None):
+    """(output, gradients) of a training step, or the output alone without gradients."""
+    with torch.autocast("cuda", dtype=torch.bfloat16), torch.set_grad_enabled(dy is not None):
+        y = m(x, xpos=pos)
+    return [y.detach()] + (list(torch.autograd.grad(y, [x] + list(m.parameters()), dy)) if dy is not None else [])
+
+
+def odd_view(t):
+    """The same values in a contiguous view that begins one element behind an aligned address."""
+    flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    view = flat[1:].view(t.shape)
+    view.copy_(t.detach())
+    assert view.is_contiguous() and view.data_ptr() % 16
+    return view
+
+
+@pytest.mark.parametrize("which", ["norms"])
+@pytest.mark.parametrize("train", [False, True])
+def test_module_takes_views_that_begin_anywhere(which, train):
+    """Parameters inside a flattened buffer, an input or a gradient that is a slice: as if they were aligned, bit for bit."""
+    m, x, pos = module_and_input(0)
+    x.requires_grad_(train)
+    dy = torch.randn(x.shape, device=DEV).bfloat16() if train else None
+    want = module_step(m, x, pos, dy)
+    if which == "norms":
+        for n in (m.q_norm, m.k_norm):
+            n.weight, n.bias = torch.nn.Parameter(odd_view(n.weight)), torch.nn.Parameter(odd_view(n.bias))
+    got = module_step(m, x, pos, dy)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
