@@ -293,7 +293,7 @@ int s3r_peer_pull(const void* const* src, void* const* dst, const int64_t* bytes
 
 /* fp32 -> bf16 (round to nearest even) of `n` (1 to 8) tensors in one launch; no counterpart in the reference, whose autocast
  * casts the module's input and weights one by one.  The arrays are HOST arrays of device pointers and element counts;
- * every tensor 16-byte aligned. */
+ * tensors that begin at a multiple of 16 bytes on both sides move in vectors, others element by element. */
 int s3r_cast_bf16(int n, const float* const* src, void* const* dst, const int64_t* counts, void* stream);
 
 /* out[c] = sum over rows of x[rows, cols] (bf16, fp32 accumulation, fixed order): the bias gradient of a Linear whose output

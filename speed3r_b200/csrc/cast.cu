@@ -13,6 +13,7 @@ struct CastParams {
   __nv_bfloat16* dst[kCastMax];
   int64_t count[kCastMax];
   int first_block[kCastMax + 1];
+  uint32_t wide;               // bit i: both sides of tensor i begin at a multiple of 16 bytes
   int n;
 };
 
@@ -24,6 +25,10 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const __grid_constant__ 
   const float* src = p.src[i];
   __nv_bfloat16* dst = p.dst[i];
   const int64_t base = static_cast<int64_t>(blockIdx.x - p.first_block[i]) * kCastPerBlock, left = p.count[i] - base;
+  if (!(p.wide >> i & 1u)) {                   // a view that begins anywhere: one element at a time
+    for (int64_t e = threadIdx.x; e < min(left, static_cast<int64_t>(kCastPerBlock)); e += 256) dst[base + e] = __float2bfloat16_rn(src[base + e]);
+    return;
+  }
   float4 v[kCastVecs][2];
 #pragma unroll
   for (int u = 0; u < kCastVecs; ++u) {
@@ -54,12 +59,14 @@ extern "C" int s3r_cast_bf16(int n, const float* const* src, void* const* dst, c
   S3R_REQUIRE(n >= 1 && n <= kCastMax, S3R_ERR_SHAPE, "s3r_cast_bf16: %d tensors (1 to %d)", n, kCastMax);
   CastParams p;
   p.n = n;
+  p.wide = 0;
   int64_t blocks = 0;
   for (int i = 0; i < n; ++i) {
     S3R_REQUIRE(src[i] && dst[i], S3R_ERR_NULL, "s3r_cast_bf16: NULL pointer");
     S3R_REQUIRE(counts[i] > 0, S3R_ERR_SHAPE, "s3r_cast_bf16: sizes must be positive");
-    S3R_REQUIRE(((reinterpret_cast<uintptr_t>(src[i]) | reinterpret_cast<uintptr_t>(dst[i])) & 15) == 0, S3R_ERR_ALIGNMENT,
-                "s3r_cast_bf16: tensors must be 16-byte aligned");
+    S3R_REQUIRE((reinterpret_cast<uintptr_t>(src[i]) & 3) == 0 && (reinterpret_cast<uintptr_t>(dst[i]) & 1) == 0, S3R_ERR_ALIGNMENT,
+                "s3r_cast_bf16: elements must be aligned");
+    if (((reinterpret_cast<uintptr_t>(src[i]) | reinterpret_cast<uintptr_t>(dst[i])) & 15) == 0) p.wide |= 1u << i;
     p.src[i] = src[i];
     p.dst[i] = static_cast<__nv_bfloat16*>(dst[i]);
     p.count[i] = counts[i];

@@ -569,7 +569,7 @@ def odd_view(t):
     return view
 
 
-@pytest.mark.parametrize("which", ["norms"])
+@pytest.mark.parametrize("which", ["norms", "projections", "input"])
 @pytest.mark.parametrize("train", [False, True])
 def test_module_takes_views_that_begin_anywhere(which, train):
     """Parameters inside a flattened buffer, an input or a gradient that is a slice: as if they were aligned, bit for bit."""
@@ -580,5 +580,10 @@ def test_module_takes_views_that_begin_anywhere(which, train):
     if which == "norms":
         for n in (m.q_norm, m.k_norm):
             n.weight, n.bias = torch.nn.Parameter(odd_view(n.weight)), torch.nn.Parameter(odd_view(n.bias))
+    elif which == "projections":
+        for lin in (m.qkv, m.proj, m.gate[0]):
+            lin.weight, lin.bias = torch.nn.Parameter(odd_view(lin.weight)), torch.nn.Parameter(odd_view(lin.bias))
+    else:
+        x = odd_view(x).requires_grad_(train)
     got = module_step(m, x, pos, dy)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
