@@ -992,6 +992,8 @@ extern "C" int s3r_delta(const void* o, const void* d_o, float* delta, int64_t r
   S3R_REQUIRE(o && d_o && delta, S3R_ERR_NULL, "s3r_delta: NULL pointer");
   S3R_REQUIRE(rows > 0, S3R_ERR_SHAPE, "s3r_delta: rows must be positive");
   S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_delta: head_dim %d not supported (64 only)", d);
+  S3R_REQUIRE(((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o)) & 15) == 0, S3R_ERR_ALIGNMENT,
+              "s3r_delta: tensors must be 16-byte aligned");
   const int64_t blocks = (rows * 8 + 255) / 256;
   return launch(delta_kernel, static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream),
                 static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, rows);
@@ -1004,6 +1006,12 @@ extern "C" int s3r_merge_bwd_deltas(const void* dy, const void* gate, int64_t ga
   S3R_REQUIRE(dy && gate && o_c && o_s && do_s && dgate && do_c && delta_s, S3R_ERR_NULL, "s3r_merge_bwd: NULL pointer");
   S3R_REQUIRE(B > 0 && H > 0 && Tq > 0 && block > 0, S3R_ERR_SHAPE, "s3r_merge_bwd: bad sizes");
   S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_merge_bwd: head_dim %d not supported (64 only)", d);
+  uintptr_t al = 0;
+  for (const void* t : {dy, o_c, o_s, static_cast<const void*>(do_s), static_cast<const void*>(do_c)}) al |= reinterpret_cast<uintptr_t>(t);
+  S3R_REQUIRE((al & 15) == 0 && (reinterpret_cast<uintptr_t>(dgate) & 7) == 0, S3R_ERR_ALIGNMENT,
+              "s3r_merge_bwd: tensors must be 16-byte aligned, dgate 8-byte");
+  S3R_REQUIRE((reinterpret_cast<uintptr_t>(gate) & 3) == 0 && gate_stride_b % 2 == 0 && gate_stride_h % 2 == 0 && gate_stride_t % 2 == 0,
+              S3R_ERR_ALIGNMENT, "s3r_merge_bwd: gate pairs must be 4-byte aligned");
   MergeBwdParams p;
   p.dy = static_cast<const __nv_bfloat16*>(dy);
   p.gate = static_cast<const __nv_bfloat16*>(gate);

@@ -101,10 +101,11 @@ std::tuple<Tensor, Tensor, Tensor> pool_qkv_fwd(const Tensor& q, const Tensor& k
   return {out[0], out[1], out[2]};
 }
 
-Tensor pool_bwd(const Tensor& d_out, int64_t T, int64_t kernel, int64_t stride) {
-  need(d_out, "d_out");
-  const int64_t B = d_out.size(0), H = d_out.size(1), d = d_out.size(3);
-  c10::cuda::CUDAGuard guard(d_out.device());
+Tensor pool_bwd(const Tensor& d_out_, int64_t T, int64_t kernel, int64_t stride) {
+  need(d_out_, "d_out");
+  const int64_t B = d_out_.size(0), H = d_out_.size(1), d = d_out_.size(3);
+  c10::cuda::CUDAGuard guard(d_out_.device());
+  const Tensor d_out = aligned(d_out_);
   Tensor d_in = fresh({B, H, T, d}, d_out, at::kBFloat16);
   check(s3r_pool_bwd(d_out.data_ptr(), d_in.data_ptr(), H * T * d, T * d, d, B, H, T, d, kernel, stride, 0, stream()),
         "s3r_pool_bwd");
@@ -143,16 +144,17 @@ std::tuple<Tensor, Tensor, Tensor> cmp_attn_blocktopk_fwd(const Tensor& q_c, con
 }
 
 std::tuple<Tensor, Tensor, Tensor> cmp_bwd(const Tensor& q_c, const Tensor& k_c, const Tensor& v_c,
-                                                const Tensor& o_c, const Tensor& lse, const Tensor& do_c, double scale,
+                                                const Tensor& o_c, const Tensor& lse, const Tensor& do_c_, double scale,
                                                 const Tensor* have_delta) {
   need(q_c, "q_c");
   need(k_c, "k_c");
   need(v_c, "v_c");
   need(o_c, "o_c");
-  need(do_c, "do_c");
+  need(do_c_, "do_c");
   need(lse, "lse", at::kFloat);
   const int64_t B = q_c.size(0), H = q_c.size(1), Nq = q_c.size(2), d = q_c.size(3), Nc = k_c.size(2);
   c10::cuda::CUDAGuard guard(q_c.device());
+  const Tensor do_c = aligned(do_c_);
   Tensor dq = fresh_like(q_c), dk = fresh_like(k_c), dv = fresh_like(v_c);
   if (have_delta) {
     check(s3r_cmp_attn_bwd_delta(q_c.data_ptr(), k_c.data_ptr(), v_c.data_ptr(), f32(lse), do_c.data_ptr(), f32(*have_delta),
@@ -261,15 +263,16 @@ std::tuple<Tensor, Tensor> build_key_csr(const Tensor& idx, int64_t num_key_bloc
 // The selection branch's gradients; with dq_c, dk_c, dv_c (gradients of q pooled per block and of k, v pooled with
 // kernel/stride) the pooled branch's share is added to them.
 std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
-                                           const Tensor& lse, const Tensor& delta, const Tensor& do_s, const Tensor* dq_c,
+                                           const Tensor& lse, const Tensor& delta, const Tensor& do_s_, const Tensor* dq_c,
                                            const Tensor* dk_c, const Tensor* dv_c, int64_t block, int64_t kernel,
                                            int64_t stride, double scale, const std::tuple<Tensor, Tensor>* inverse = nullptr) {
   need(q, "q");
   need(k, "k");
   need(v, "v");
-  need(do_s, "do_s");
+  need(do_s_, "do_s");
   const int64_t B = q.size(0), H = q.size(1), Tq = q.size(2), d = q.size(3), Tk = k.size(2), K = idx.size(-1);
   c10::cuda::CUDAGuard guard(q.device());
+  const Tensor do_s = aligned(do_s_);
   auto [offsets, qids] = inverse ? *inverse : csr(idx, (Tk + block - 1) / block, false);
   Tensor dq = fresh_like(q), dk = fresh_like(k), dv = fresh_like(v);
   const bool fused = dq_c != nullptr && block % 16 == 0 && kernel % 16 == 0 && stride % 16 == 0;
@@ -300,21 +303,23 @@ std::tuple<Tensor, Tensor, Tensor> sel_attn_bwd_pooled(const Tensor& q, const Te
   return sel_bwd(q, k, v, idx, lse, delta, do_s, &dq_c, &dk_c, &dv_c, block, kernel, stride, scale);
 }
 
-Tensor delta(const Tensor& o, const Tensor& d_o) {
-  need(o, "o");
-  need(d_o, "do");
-  c10::cuda::CUDAGuard guard(o.device());
+Tensor delta(const Tensor& o_, const Tensor& d_o_) {
+  need(o_, "o");
+  need(d_o_, "do");
+  c10::cuda::CUDAGuard guard(o_.device());
+  const Tensor o = aligned(o_), d_o = aligned(d_o_);
   Tensor out = fresh(o.sizes().slice(0, o.dim() - 1), o, at::kFloat);
   check(s3r_delta(o.data_ptr(), d_o.data_ptr(), f32(out), out.numel(), o.size(-1), stream()), "s3r_delta");
   return out;
 }
 
-std::tuple<Tensor, Tensor, Tensor, Tensor> merge_bwd_deltas(const Tensor& dy, const Tensor& gate, const Tensor& o_c,
+std::tuple<Tensor, Tensor, Tensor, Tensor> merge_bwd_deltas(const Tensor& dy_, const Tensor& gate, const Tensor& o_c,
                                                             const Tensor& o_s, int64_t block, Tensor* delta_c) {
-  need(dy, "dy");
+  need(dy_, "dy");
   need_gate(gate);
   const int64_t B = o_s.size(0), H = o_s.size(1), Tq = o_s.size(2), d = o_s.size(3);
-  c10::cuda::CUDAGuard guard(dy.device());
+  c10::cuda::CUDAGuard guard(dy_.device());
+  const Tensor dy = aligned(dy_);
   Tensor do_s = fresh_like(o_s), dgate = fresh({B, H, Tq, 2}, dy, at::kFloat), do_c = fresh_like(o_c),
          delta_s = fresh({B, H, Tq}, dy, at::kFloat);
   if (delta_c) *delta_c = fresh({B, H, o_c.size(2)}, dy, at::kFloat);
@@ -376,13 +381,14 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> prologue_fwd(
 // (gradient of qkv, [4,64] gradients of q weight, q bias, k weight, k bias; no elements without norms)
 std::tuple<Tensor, Tensor> prologue_bwd(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos,
                                         const optional<Tensor>& cos, const optional<Tensor>& sin, const optional<Tensor>& qw_,
-                                        const optional<Tensor>& kw_, double eps, const Tensor& dq, const Tensor& dk,
-                                        const Tensor& dv, const Tensor& dq_c, const Tensor& dk_c, const Tensor& dv_c) {
+                                        const optional<Tensor>& kw_, double eps, const Tensor& dq_, const Tensor& dk_,
+                                        const Tensor& dv_, const Tensor& dq_c_, const Tensor& dk_c_, const Tensor& dv_c_) {
   const int64_t rows = need_prologue(qkv, heads, block, pos, cos, sin, {&qw_, &kw_});
-  for (const Tensor* g : {&dq, &dk, &dv, &dq_c, &dk_c, &dv_c}) need(*g, "gradient");
+  for (const Tensor* g : {&dq_, &dk_, &dv_, &dq_c_, &dk_c_, &dv_c_}) need(*g, "gradient");
   const int64_t B = qkv.size(0), N = qkv.size(1), d = qkv.numel() / (B * N) / (3 * heads);
   c10::cuda::CUDAGuard guard(qkv.device());
   const auto qw = aligned(qw_), kw = aligned(kw_);
+  const Tensor dq = aligned(dq_), dk = aligned(dk_), dv = aligned(dv_), dq_c = aligned(dq_c_), dk_c = aligned(dk_c_), dv_c = aligned(dv_c_);
   const bool norm = qw.has_value(), rope = pos.has_value();
   const size_t nbytes = norm ? s3r_qkv_prologue_bwd_workspace_bytes(B, heads, N, block) : 0;
   Tensor dqkv = fresh_like(qkv), ws = fresh({static_cast<int64_t>(nbytes)}, qkv, at::kByte),
@@ -856,7 +862,7 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     char* base = static_cast<char*>(buf.data_ptr());
     auto ptr = [&](int64_t at) { return static_cast<void*>(base + 2 * at); };
     auto view = [&](int64_t at, int64_t r, int64_t c) { return buf.as_strided({r, c}, {c, 1}, at); };
-    const Tensor dy = g[0].to(at::kBFloat16).contiguous().view({m.M, out_features});
+    const Tensor dy = aligned(g[0].to(at::kBFloat16).contiguous()).view({m.M, out_features});
 
     // scratch of the backward, bytes
     int64_t used = 0;
@@ -892,7 +898,8 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
       check(s3r_colsum(x, f32(o), m.M, cols, sp(a_col), col_bytes, st), "s3r_colsum");
       return o;
     };
-    if (ints[5] && ctx->needs_input_grad(e_wp + 1)) dbp = colsum(dy.data_ptr(), out_features);
+    if (ints[5] && ctx->needs_input_grad(e_wp + 1))          // the kernel reads rows of whole vectors
+      dbp = out_features % 8 == 0 ? colsum(dy.data_ptr(), out_features) : dy.sum(0, false, at::kFloat);
     // merge, the two branches, prologue
     check(s3r_merge_bwd_deltas(sp(a_dy), ptr(m.gate), m.H * m.N * 2, m.N * 2, 2, ptr(m.t(6)), ptr(m.o_s), sp(a_dos), sf(a_dgate),
                                sp(a_doc), sf(a_dels), sf(a_delc), m.B, m.H, m.N, m.d, m.block, st), "s3r_merge_bwd");

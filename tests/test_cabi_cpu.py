@@ -81,6 +81,12 @@ def test_argument_errors_are_reported_without_a_gpu(lib):
         rc = lib.s3r_qkv_prologue_bwd(p, None, None, None, 0, p + off[0], p + off[1], 1e-5, p, p, p, p, p, p, p, p, p, 1 << 30,
                                       1, 4, 32, 64, 16, None)
         assert rc == -3 and "8-byte" in _lib.last_error()
+    # 16-byte loads of what a caller hands to a backward
+    assert lib.s3r_delta(p, p + 2, p, 16, 64, None) == -3 and lib.s3r_delta(p + 8, p, p, 16, 64, None) == -3
+    for i in range(6):
+        a = [p + 2 * (i == j) for j in range(6)]                   # dy, gate, o_c, o_s, do_s, do_c
+        rc = lib.s3r_merge_bwd(a[0], a[1], 64, 32, 2, a[2], a[3], a[4], p, a[5], p, 1, 1, 16, 64, 16, None)
+        assert rc == -3 and "aligned" in _lib.last_error()
     # merge arguments must come together
     rc = lib.s3r_sel_attn_fwd(p, p, p, 1, 0, p, p, None, p, 0, 0, 0, None, None, 1, 1, 64, 64, 64, 16, 8, 0.125, None)
     assert rc == -4

@@ -569,7 +569,7 @@ def odd_view(t):
     return view
 
 
-@pytest.mark.parametrize("which", ["norms", "projections", "input"])
+@pytest.mark.parametrize("which", ["norms", "projections", "input", "gradient"])
 @pytest.mark.parametrize("train", [False, True])
 def test_module_takes_views_that_begin_anywhere(which, train):
     """Parameters inside a flattened buffer, an input or a gradient that is a slice: as if they were aligned, bit for bit."""
@@ -583,7 +583,38 @@ def test_module_takes_views_that_begin_anywhere(which, train):
     elif which == "projections":
         for lin in (m.qkv, m.proj, m.gate[0]):
             lin.weight, lin.bias = torch.nn.Parameter(odd_view(lin.weight)), torch.nn.Parameter(odd_view(lin.bias))
-    else:
+    elif which == "input":
         x = odd_view(x).requires_grad_(train)
+    elif train:
+        dy = odd_view(dy)
     got = module_step(m, x, pos, dy)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_ops_take_gradients_that_begin_anywhere():
+    from speed3r_b200 import ops
+    B, H, T = 1, 2, 512
+    q, k, v = (randn(s, B, H, T, 64).to(DEV, torch.bfloat16).requires_grad_(True) for s in (1, 2, 3))
+    gate = torch.sigmoid(randn(4, B, H, T, 2)).to(DEV, torch.bfloat16).requires_grad_(True)
+    idx = table(5, B, H, T // 16, T // 16, 8).to(DEV)
+    o_c = randn(6, B, H, T // 16, 64).to(DEV, torch.bfloat16).requires_grad_(True)
+    for what, out, wrt in (
+            ("pool", ops.pool_tokens(q), (q,)),
+            ("compression", ops.flash_attn_topk_func(q, k, v, 8)[0], (q, k, v)),
+            ("selection", ops.topk_blocksparse_attention(q, k, v, idx, 16), (q, k, v)),
+            ("merge", ops.sel_attn_merge(q, k, v, idx, gate, o_c, 16), (q, k, v, gate, o_c)),
+            ("op", ops.sparse_attention_op(q, k, v, gate)[0], (q, k, v, gate))):
+        g = torch.randn(out.shape, device=DEV).bfloat16()
+        want = torch.autograd.grad(out, wrt, g, retain_graph=True)
+        got = torch.autograd.grad(out, wrt, odd_view(g))
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), what
+
+
+def test_module_with_an_output_that_is_not_whole_vectors():
+    """A projection to 100 channels: the sum of its bias gradient's rows cannot be read in vectors of eight."""
+    m, x, pos = module_and_input(0)
+    m.proj = torch.nn.Linear(x.shape[-1], 100).to(DEV)
+    x.requires_grad_(True)
+    dy = torch.randn(1, x.shape[1], 100, device=DEV).bfloat16()
+    grads = dict(zip(["x"] + [n for n, _ in m.named_parameters()], module_step(m, x, pos, dy)[1:]))
+    assert_bf16_close(grads["proj.bias"], dy.float().sum((0, 1)), "bias")
