@@ -608,6 +608,43 @@ SixTensors prologue(const Tensor& qkv, int64_t heads, int64_t block, const optio
   return call_prologue(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps);
 }
 
+// What the module's arguments have to be: the native forms copy by these sizes into one allocation.  Shapes come before
+// devices, so that they can be checked without a GPU.
+void need_module(const Tensor& x, const Tensor& w_qkv, const optional<Tensor>& b_qkv, const Tensor& w_gate, const optional<Tensor>& b_gate,
+                 const Tensor& w_proj, const optional<Tensor>& b_proj, const optional<Tensor>& pos, const optional<Tensor>& cos,
+                 const optional<Tensor>& sin, std::initializer_list<const optional<Tensor>*> norms, int64_t heads, int64_t block) {
+  TORCH_CHECK(x.dim() == 3 && heads > 0 && block > 0, "attention module: x must be [B,N,C]");
+  const int64_t B = x.size(0), N = x.size(1), C = x.size(2), d = C / heads;
+  TORCH_CHECK(C == heads * d && N % block == 0, "attention module: x ", x.sizes(), " does not split into ", heads, " heads and blocks of ", block);
+  auto shape = [&](const Tensor& t, at::IntArrayRef want, const char* name) {
+    TORCH_CHECK(t.sizes() == want, "attention module: the shape of ", name, " must be ", want, ", got ", t.sizes());
+  };
+  auto linear = [&](const Tensor& w, const optional<Tensor>& b, int64_t out, const char* name) {
+    shape(w, {out, C}, name);
+    if (b.has_value()) shape(*b, {out}, name);
+  };
+  linear(w_qkv, b_qkv, 3 * C, "qkv");
+  linear(w_gate, b_gate, 2 * heads, "gate");
+  TORCH_CHECK(w_proj.dim() == 2, "attention module: the shape of proj must be [out,C]");
+  linear(w_proj, b_proj, w_proj.size(0), "proj");
+  for (const auto* w : norms) {
+    TORCH_CHECK(w->has_value() == (*norms.begin())->has_value(), "attention module: q_norm and k_norm come together or not at all");
+    if (w->has_value()) shape(**w, {d}, "norm parameter");
+  }
+  if (pos.has_value()) {
+    shape(*pos, {B, N, 2}, "xpos");
+    TORCH_CHECK(cos.has_value() && sin.has_value() && cos->dim() == 2, "attention module: positions need the cos/sin tables");
+    shape(*cos, {cos->size(0), d / 2}, "cos");
+    shape(*sin, cos->sizes(), "sin");
+  }
+  TORCH_CHECK(x.is_cuda(), "x must be a CUDA tensor: the speed3r_b200 kernels have no CPU path");
+  TORCH_CHECK(!pos.has_value() || pos->device() == x.device(), "xpos must be on ", x.device());
+  if (pos.has_value()) {
+    need(*cos, "cos");
+    need(*sin, "sin");
+  }
+}
+
 // The whole attention module without gradients: projections (cuBLAS), prologue, the two attentions, output projection.
 // fp32 input and parameters are rounded to bf16 as under autocast, all in one launch, with the weights of qkv and gate side
 // by side so that one GEMM does both; everything between the GEMMs lives in one allocation and goes straight to the C ABI:
@@ -620,7 +657,7 @@ std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, c
                                         double scale) {
   at::AutoDispatchBelowAutograd below;
   c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
-  TORCH_CHECK(x_.is_cuda() && x_.dim() == 3, "x must be a CUDA tensor [B,N,C]: the speed3r_b200 kernels have no CPU path");
+  need_module(x_, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, pos_, cos, sin, {&qw_, &qb_, &kw_, &kb_}, heads, block);
   c10::cuda::CUDAGuard guard(x_.device());
   void* st = stream();
   const int64_t B = x_.size(0), N = x_.size(1), C = x_.size(2), H = heads, d = C / heads, M = B * N, Nc = N / block;
@@ -712,13 +749,7 @@ std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, c
     gemm(gate_logits, x, weight(at_wg, w_gate), bias(at_bg, b_gate));
     gate_logits.sigmoid_();
   }
-  int64_t rows = 0;
-  if (pos.has_value()) {
-    TORCH_CHECK(cos.has_value() && sin.has_value() && pos->sizes() == std::vector<int64_t>({B, N, 2}), "xpos must be [B,N,2]");
-    need(*cos, "cos");
-    need(*sin, "sin");
-    rows = cos->size(0);
-  }
+  const int64_t rows = pos.has_value() ? cos->size(0) : 0;
   const void *cp = pos.has_value() ? cos->data_ptr() : nullptr, *sp = pos.has_value() ? sin->data_ptr() : nullptr;
   const int64_t* pp = static_cast<const int64_t*>(ptr_or_null(pos));
   void* t[7];                                                // q, k, v, q_c, k_c, v_c, o_c
@@ -943,17 +974,12 @@ std::tuple<Tensor, Tensor> module_train(const Tensor& x, const Tensor& w_qkv, co
                                         const optional<Tensor>& qw_, const optional<Tensor>& qb_, const optional<Tensor>& kw_,
                                         const optional<Tensor>& kb_, double eps, int64_t heads, int64_t block, int64_t topk,
                                         double scale) {
-  TORCH_CHECK(x.is_cuda() && x.dim() == 3, "x must be a CUDA tensor [B,N,C]: the speed3r_b200 kernels have no CPU path");
+  need_module(x, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, pos_, cos, sin, {&qw_, &qb_, &kw_, &kb_}, heads, block);
   TORCH_CHECK(heads % 4 == 0 && b_qkv.has_value() == b_gate.has_value(), "module_train: heads in fours, and biases of qkv and gate together");
   auto as = [&](const optional<Tensor>& t, at::ScalarType type) {
     return t.has_value() ? optional<Tensor>(t->to(x.device(), type).contiguous()) : t;
   };
   const auto pos = as(pos_, at::kLong);
-  if (pos.has_value()) {
-    TORCH_CHECK(cos.has_value() && sin.has_value() && pos->sizes() == std::vector<int64_t>({x.size(0), x.size(1), 2}), "xpos must be [B,N,2]");
-    need(*cos, "cos");
-    need(*sin, "sin");
-  }
   const auto r = ModuleNode::apply(x, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, pos, cos, sin, as(qw_, at::kFloat), as(qb_, at::kFloat),
                                    as(kw_, at::kFloat), as(kb_, at::kFloat), eps, heads, block, topk, scale);
   return {r[0], r[1]};

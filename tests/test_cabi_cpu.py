@@ -110,6 +110,30 @@ def test_python_layer_has_no_cpu_fallback():
         m(torch.randn(1, 64, 128))
 
 
+@pytest.mark.parametrize("op", ["module_infer", "module_train"])
+def test_native_module_refuses_shapes_that_do_not_fit(op):
+    """The native forms of the module copy its input and weights by size into one allocation: every shape is looked at first
+    (before the device, so that this needs no GPU)."""
+    from speed3r_b200 import ops
+    H, d, N = 4, 64, 32
+    C = H * d
+    good = dict(x=(1, N, C), w_qkv=(3 * C, C), b_qkv=(3 * C,), w_gate=(2 * H, C), b_gate=(2 * H,), w_proj=(C, C), b_proj=(C,),
+                pos=(1, N, 2), cos=(64, d // 2), sin=(64, d // 2), qw=(d,), qb=(d,), kw=(d,), kb=(d,))
+    def call(**shapes):
+        t = [torch.zeros(s, dtype=torch.int64 if n == "pos" else torch.float32) for n, s in {**good, **shapes}.items()]
+        getattr(ops._ops(), op).default(*t, 1e-5, H, 16, 32, 0.125)
+    with pytest.raises(RuntimeError, match="CUDA"):                # the shapes fit
+        call()
+    for name, shape in dict(x=(1, N, C + 1), w_qkv=(3 * C + 8, C), b_qkv=(3 * C + 1,), w_gate=(2 * H + 8, C), b_gate=(2 * H + 8,),
+                            w_proj=(C, C + 1), b_proj=(C + 1,), pos=(2, N, 2), cos=(64, d), sin=(63, d // 2), qw=(d - 1,), kb=(1,)).items():
+        with pytest.raises(RuntimeError, match="attention module"):
+            call(**{name: shape})
+    with pytest.raises(RuntimeError, match="attention module"):    # an input of another width than the weights
+        call(x=(1, N, 2 * C))
+    with pytest.raises(RuntimeError, match="blocks"):
+        call(x=(1, N + 1, C), pos=(1, N + 1, 2))
+
+
 def test_module_keeps_reference_state_dict_keys_and_init():
     """Keys and gate initialisation of pi3/models/layers/sparse_attention.py:62-86."""
     import speed3r_b200
