@@ -4,7 +4,8 @@
  *   - plain SIMT restatements of the two forward attentions (one thread per query row, fp32
  *     arithmetic), so that the tensor-core kernels can be cross-checked ON THE DEVICE at sizes a
  *     CPU check cannot reach;
- *   - a probe of the bounded device-side wait every kernel of the product library uses.
+ *   - a probe of the bounded device-side wait every kernel of the product library uses;
+ *   - the rule by which two tensors' tiles travel together.
  * Conventions (return codes, s3r_last_error, explicit stream) are those of speed3r_b200.h; the
  * library carries its own copy of the per-device status word, read with its own s3r_device_status.
  */
@@ -34,6 +35,10 @@ int s3r_check_sel_attn_fwd(const void* q, const void* k, const void* v, const in
  * (which has no device-side waits); it exists so that the give-up path is exercised without
  * leaving anything waiting on the GPU. */
 int s3r_check_wait_gives_up(uint64_t limit_ns, uint64_t* waited_ns, void* stream);
+
+/* How the selection kernels would copy the tiles of two tensors at device addresses `a` and `b` (host arithmetic, nothing is
+ * read): bit 0 b's tile in front of a's, bit 1 one tile serves as both, bit 2 two copies. */
+int s3r_check_pair_order(uint64_t a, uint64_t b);
 
 /* This library's copies of the two helpers of speed3r_b200.h. */
 int s3r_last_error(char* buf, int n);

@@ -94,16 +94,29 @@ int make_tensor_map(CUtensorMap* out, const void* base, int rank, const uint64_t
   return 0;
 }
 
-int make_pair_map(CUtensorMap* out, const void* a, const void* b, int T, int BH, int chunks, int64_t chunk_stride_bytes, int* b_first) {
-  const uintptr_t pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
-  const bool same = pa == pb, below = pb < pa;
+PairOrder pair_order(uint64_t a, uint64_t b) {
+  if (a == b) return {-1, 0};
+  if ((a < b ? b - a : a - b) >= (1ull << 40)) return {0, 1};
+  return {b < a, 0};
+}
+
+int make_pair_map(PairMap* out, const void* a, const void* b, int T, int BH, int chunks, int64_t chunk_stride_bytes) {
+  const uint64_t pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
+  const PairOrder o = pair_order(pa, pb);
+  const bool one = o.b_first < 0 || o.apart;                 // tiles a copy brings
   const uint64_t tc = static_cast<uint64_t>(T / chunks), bh = static_cast<uint64_t>(BH);
-  const uint64_t dims[5] = {64, tc, bh, static_cast<uint64_t>(chunks), same ? 1u : 2u};
+  const uint64_t dims[5] = {64, tc, bh, static_cast<uint64_t>(chunks), one ? 1u : 2u};
   const uint64_t strides[4] = {128, tc * 128, chunks > 1 ? static_cast<uint64_t>(chunk_stride_bytes) : tc * 128 * bh,
-                               same ? 128 : (below ? pa - pb : pb - pa)};
-  const uint32_t box[5] = {64, 16, 1, 1, same ? 1u : 2u};
-  *b_first = same ? -1 : (below ? 1 : 0);
-  return make_tensor_map(out, below ? b : a, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+                               one ? 128 : (o.b_first ? pa - pb : pb - pa)};
+  const uint32_t box[5] = {64, 16, 1, 1, one ? 1u : 2u};
+  out->b_first = o.b_first;
+  out->apart = o.apart;
+  const int rc = make_tensor_map(&out->both, o.b_first > 0 ? b : a, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc || !o.apart) {
+    out->second = out->both;
+    return rc;
+  }
+  return make_tensor_map(&out->second, b, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 }  // namespace s3r

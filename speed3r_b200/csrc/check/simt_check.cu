@@ -169,3 +169,8 @@ extern "C" int s3r_check_sel_attn_fwd(const void* q, const void* k, const void* 
   S3R_CUDA(cudaGetLastError());
   return 0;
 }
+
+extern "C" int s3r_check_pair_order(uint64_t a, uint64_t b) {
+  const PairOrder o = pair_order(a, b);
+  return (o.b_first > 0 ? 1 : 0) | (o.b_first < 0 ? 2 : 0) | (o.apart ? 4 : 0);
+}

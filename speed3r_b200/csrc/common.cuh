@@ -41,10 +41,21 @@ int make_tensor_map(CUtensorMap* out, const void* base, int rank, const uint64_t
                     const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle,
                     CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
 
-// Two tensors of the same shape (`chunks` chunks of [BH, T / chunks, 64] bf16) as ONE tensor map whose outermost
-// dimension of two steps from one to the other: a copy of a 16-row box brings 2 KB of each (a's tile first, or
-// b's when *b_first).  a == b: the box has one tile, which serves as both (*b_first = -1).
-int make_pair_map(CUtensorMap* out, const void* a, const void* b, int T, int BH, int chunks, int64_t chunk_stride_bytes, int* b_first);
+// Two tensors of the same shape (`chunks` chunks of [BH, T / chunks, 64] bf16) whose 16-row tiles travel together, 2 KB of
+// each: where the distance between them fits a tensor map's stride, as ONE map whose outermost dimension of two steps from
+// one to the other, so that one copy brings both.
+struct PairMap {
+  CUtensorMap both, second;      // second: b's own map, where they are apart
+  int b_first;                   // b's tile lies in front of a's; -1: a == b, one tile serves as both
+  int apart;                     // two copies
+};
+// (b_first, apart) of two addresses: strides are below 2^40 bytes, and device memory of different origin (virtual-memory
+// reservations, peers' and symmetric buffers) can be further apart.
+struct PairOrder {
+  int b_first, apart;
+};
+PairOrder pair_order(uint64_t a, uint64_t b);
+int make_pair_map(PairMap* out, const void* a, const void* b, int T, int BH, int chunks, int64_t chunk_stride_bytes);
 
 int sm_count();
 
@@ -328,6 +339,13 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst_smem, const CUtensorMap
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
       ::"r"(dst_smem), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
       : "memory");
+}
+// the tiles of 16 rows from `tok` on of both tensors, 2 KB each (one of them serves as both: 2 KB)
+// APART: kernels are compiled for both, so that the usual form does not ask
+template <bool APART>
+__device__ __forceinline__ void tma_load_pair(uint32_t dst_smem, const PairMap& m, uint64_t* bar, int tok, int bh, int chunk) {
+  tma_load_5d(dst_smem, &m.both, bar, 0, tok, bh, chunk, 0);
+  if (APART && m.apart) tma_load_5d(dst_smem + 2048, &m.second, bar, 0, tok, bh, chunk, 0);
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

@@ -442,7 +442,6 @@ struct SelBwdParams {
   const __nv_bfloat16 *dq_c, *dk_c, *dv_c;
   int q_kernel, q_stride, q_windows, k_kernel, k_stride, k_windows;
   int B, H, Tq, Tk, block, block_shift, topk, nqb, nkb;     // block = 16 << block_shift
-  int first_kv, first_qdo;       // order of the tiles a copy brings (make_pair_map)
   float cs, scale;
   uint32_t* status;
 };
@@ -548,7 +547,8 @@ struct SbShared {
 };
 
 // dQ of 16 rows.  `taken` pairs have gone through the ring before: a pair is its n-th, stage n & 1, phase (n >> 1) & 1.
-__device__ __forceinline__ void sel_bwd_dq(const CUtensorMap& map_kv, const SelBwdParams& p, SbShared& sh, uint32_t ring,
+template <bool APART>
+__device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdParams& p, SbShared& sh, uint32_t ring,
                                            uint32_t task, uint32_t taken) {
   const int lane = threadIdx.x, g = lane >> 2, c = lane & 3;
   const uint32_t nslices = (p.Tq + 15) / 16;
@@ -574,9 +574,9 @@ __device__ __forceinline__ void sel_bwd_dq(const CUtensorMap& map_kv, const SelB
   auto issue = [&](int pair, int s) {
     if (lane == 0) {
       const int t = 2 * pair;
-      mbar_expect_tx(&sh.full[s], (t + 1 < ntiles ? 8192u : 4096u) >> (p.first_kv < 0));
-      tma_load_5d(ring + s * kSbStageBytes, &map_kv, &sh.full[s], 0, tok_of(t), bh, 0, 0);
-      if (t + 1 < ntiles) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_kv, &sh.full[s], 0, tok_of(t + 1), bh, 0, 0);
+      mbar_expect_tx(&sh.full[s], (t + 1 < ntiles ? 8192u : 4096u) >> (map_kv.b_first < 0));
+      tma_load_pair<APART>(ring + s * kSbStageBytes, map_kv, &sh.full[s], tok_of(t), bh, 0);
+      if (t + 1 < ntiles) tma_load_pair<APART>(ring + s * kSbStageBytes + 4096, map_kv, &sh.full[s], tok_of(t + 1), bh, 0);
     }
   };
   if (npairs > 0) issue(0, taken & 1);
@@ -593,7 +593,7 @@ __device__ __forceinline__ void sel_bwd_dq(const CUtensorMap& map_kv, const SelB
     delta[r] = p.delta[t];
   }
   const SbLane of(lane);
-  const uint32_t k_at = p.first_kv > 0 ? 2048u : 0u, v_at = p.first_kv == 0 ? 2048u : 0u;
+  const uint32_t k_at = map_kv.b_first > 0 ? 2048u : 0u, v_at = map_kv.b_first == 0 ? 2048u : 0u;
   const bool ragged = (p.Tk & 15) != 0 || (p.Tk & (p.block - 1)) != 0;
 
   float dq[8][4] = {};
@@ -660,8 +660,9 @@ __device__ __forceinline__ void sel_bwd_dq(const CUtensorMap& map_kv, const SelB
 // five, and CTAs that came and went left a fifth of the warps' places empty (9.6 of 12 per SM).
 // Tasks: first all of dK/dV, then all of dQ, whose lists are of one length; a warp that is handed one of those is done after it.
 // (As two kernels the second could not start before the longest lists of the first had been worked off.)
-__global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__ CUtensorMap map_qdo,
-                                                         const __grid_constant__ CUtensorMap map_kv, const SelBwdParams p) {
+template <bool APART>
+__global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__ PairMap map_qdo,
+                                                         const __grid_constant__ PairMap map_kv, const SelBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(16) SbShared sh;
   const int lane = threadIdx.x, c = lane & 3;
@@ -679,12 +680,12 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
   griddep_launch();
   __syncwarp();
   if (blockIdx.x >= kv_tasks) {
-    sel_bwd_dq(map_kv, p, sh, ring, blockIdx.x - kv_tasks, 0);
+    sel_bwd_dq<APART>(map_kv, p, sh, ring, blockIdx.x - kv_tasks, 0);
     return;
   }
   const int in_block = (1 << p.block_shift) - 1;
   const SbLane of(lane);
-  const uint32_t q_at = p.first_qdo > 0 ? 2048u : 0u, do_at = p.first_qdo == 0 ? 2048u : 0u;
+  const uint32_t q_at = map_qdo.b_first > 0 ? 2048u : 0u, do_at = map_qdo.b_first == 0 ? 2048u : 0u;
 
   int bh, row0, cnt, ntiles, npairs;
   const int32_t* ql;
@@ -702,9 +703,9 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
   };
   auto issue = [&](int t0, int t1, bool both, int s) {
     if (lane == 0) {
-      mbar_expect_tx(&sh.full[s], (both ? 8192u : 4096u) >> (p.first_qdo < 0));
-      tma_load_5d(ring + s * kSbStageBytes, &map_qdo, &sh.full[s], 0, t0, bh, 0, 0);
-      if (both) tma_load_5d(ring + s * kSbStageBytes + 4096, &map_qdo, &sh.full[s], 0, t1, bh, 0, 0);
+      mbar_expect_tx(&sh.full[s], (both ? 8192u : 4096u) >> (map_qdo.b_first < 0));
+      tma_load_pair<APART>(ring + s * kSbStageBytes, map_qdo, &sh.full[s], t0, bh, 0);
+      if (both) tma_load_pair<APART>(ring + s * kSbStageBytes + 4096, map_qdo, &sh.full[s], t1, bh, 0);
     }
   };
   // lanes 0-15 fetch lse, lanes 16-31 delta of a tile's rows; a row past the end gets lse = +inf: P is exactly 0
@@ -876,7 +877,7 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
     fence_proxy_async_smem();                           // copies and the next answer come after these reads and writes
     __syncwarp();
     if (static_cast<uint32_t>(next) >= kv_tasks) {
-      sel_bwd_dq(map_kv, p, sh, ring, static_cast<uint32_t>(next) - kv_tasks, taken);
+      sel_bwd_dq<APART>(map_kv, p, sh, ring, static_cast<uint32_t>(next) - kv_tasks, taken);
       return;
     }
   }
@@ -1056,13 +1057,14 @@ static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
   const int64_t bh = static_cast<int64_t>(p.B) * p.H;
   const int64_t tq = bh * ((p.Tq + 15) / 16), tk = bh * ((p.Tk + 15) / 16);
   S3R_REQUIRE(tq + tk < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_bwd: grid too large");
-  CUtensorMap mkv, mqdo;
-  int rc = make_pair_map(&mkv, p.k, p.v, p.Tk, static_cast<int>(bh), 1, 0, &p.first_kv);
+  PairMap mkv, mqdo;
+  int rc = make_pair_map(&mkv, p.k, p.v, p.Tk, static_cast<int>(bh), 1, 0);
   if (rc) return rc;
-  rc = make_pair_map(&mqdo, p.q, p.d_o, p.Tq, static_cast<int>(bh), 1, 0, &p.first_qdo);
+  rc = make_pair_map(&mqdo, p.q, p.d_o, p.Tq, static_cast<int>(bh), 1, 0);
   if (rc) return rc;
-  S3R_CUDA(cudaFuncSetAttribute(sel_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
-  return launch(sel_bwd_kernel, static_cast<unsigned>(tk + tq), 32, kSbSmem, st, mqdo, mkv, p);
+  auto* kernel = mkv.apart || mqdo.apart ? sel_bwd_kernel<true> : sel_bwd_kernel<false>;
+  S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSbSmem));
+  return launch(kernel, static_cast<unsigned>(tk + tq), 32, kSbSmem, st, mqdo, mkv, p);
 }
 
 extern "C" int s3r_sel_attn_bwd(const void* q, const void* k, const void* v, const int32_t* idx,

@@ -40,14 +40,14 @@ struct Sel16Params {
   __nv_bfloat16* y;
   int H, Tq, Tk, Tc, nqb, topk;
   float scale_log2e;
-  int v_first;                   // order of the tiles a copy brings (make_pair_map)
   uint32_t* status;
 };
 
 constexpr int kSel16StageBytes = 2 * 2 * 2048;                    // two blocks of keys, two of values
 constexpr int kSel16Smem = 2 * kSel16StageBytes + 1024;
 
-__global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant__ CUtensorMap map_kv, const Sel16Params p) {
+template <bool APART>
+__global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant__ PairMap map_kv, const Sel16Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) int32_t list[64];        // first token of each valid key block, table order
   __shared__ uint64_t full[2];
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
   if ((nvalid & 1) && lane == 0) list[nvalid] = list[nvalid - 1];
   __syncwarp();
   const bool chunked = p.Tc != p.Tk;
-  // one copy per block brings its keys and its values
+  // a block's keys and its values together
   auto issue = [&](int pair, int s) {
     if (lane == 0) {
       const int2 t = *reinterpret_cast<const int2*>(list + 2 * pair);
@@ -93,9 +93,9 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
         c1 = t1 / p.Tc; t1 -= c1 * p.Tc;
       }
       const uint32_t dst = ring + s * kSel16StageBytes;
-      mbar_expect_tx(&full[s], p.v_first < 0 ? 4096u : 8192u);
-      tma_load_5d(dst, &map_kv, &full[s], 0, t0, bh, c0, 0);
-      tma_load_5d(dst + 4096, &map_kv, &full[s], 0, t1, bh, c1, 0);
+      mbar_expect_tx(&full[s], map_kv.b_first < 0 ? 4096u : 8192u);
+      tma_load_pair<APART>(dst, map_kv, &full[s], t0, bh, c0);
+      tma_load_pair<APART>(dst + 4096, map_kv, &full[s], t1, bh, c1);
     }
   };
   const int npairs = (nvalid + 1) >> 1;
@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
   uint32_t off_k[4], off_v[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    off_k[i] = swz128((lane & 7) + (lane >> 4) * 8, 2 * i + ((lane >> 3) & 1)) + (p.v_first > 0 ? 2048u : 0u);
-    off_v[i] = swz128((lane & 7) + ((lane >> 3) & 1) * 8, 2 * i + (lane >> 4)) + (p.v_first == 0 ? 2048u : 0u);
+    off_k[i] = swz128((lane & 7) + (lane >> 4) * 8, 2 * i + ((lane >> 3) & 1)) + (map_kv.b_first > 0 ? 2048u : 0u);
+    off_v[i] = swz128((lane & 7) + ((lane >> 3) & 1) * 8, 2 * i + (lane >> 4)) + (map_kv.b_first == 0 ? 2048u : 0u);
   }
 
   float o[8][4];
@@ -280,10 +280,11 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
   }
 }
 
-static int launch_sel16_fwd(const CUtensorMap& mkv, const Sel16Params& p, int64_t ntasks, cudaStream_t st) {
+static int launch_sel16_fwd(const PairMap& mkv, const Sel16Params& p, int64_t ntasks, cudaStream_t st) {
   S3R_REQUIRE(ntasks < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_fwd: grid of %lld CTAs is too large", (long long)ntasks);
-  S3R_CUDA(cudaFuncSetAttribute(sel16_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSel16Smem));
-  return launch(sel16_fwd_kernel, static_cast<unsigned>(ntasks), 32, kSel16Smem, st, mkv, p);
+  auto* kernel = mkv.apart ? sel16_fwd_kernel<true> : sel16_fwd_kernel<false>;
+  S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSel16Smem));
+  return launch(kernel, static_cast<unsigned>(ntasks), 32, kSel16Smem, st, mkv, p);
 }
 
 }  // namespace s3r
@@ -338,8 +339,8 @@ extern "C" int s3r_sel_attn_fwd(const void* q, const void* k, const void* v, int
     p.topk = topk;
     p.scale_log2e = scale * 1.4426950408889634f;
     p.status = status;
-    CUtensorMap mkv;
-    const int rc = make_pair_map(&mkv, k, v, Tk, BH, kv_chunks, kv_chunk_stride * 2, &p.v_first);
+    PairMap mkv;
+    const int rc = make_pair_map(&mkv, k, v, Tk, BH, kv_chunks, kv_chunk_stride * 2);
     if (rc) return rc;
     return launch_sel16_fwd(mkv, p, static_cast<int64_t>(BH) * p.nqb, st);
   }

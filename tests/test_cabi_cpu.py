@@ -41,6 +41,17 @@ def test_check_library_exports_every_declared_symbol():
     assert chk.s3r_check_wait_gives_up(0, None, None) == -4          # argument errors need no GPU
 
 
+def test_tiles_of_tensors_far_apart_are_copied_one_by_one():
+    """A tensor map's strides are below 2^40 bytes; a distance beyond that takes a map and a copy for each tensor."""
+    from speed3r_b200 import _lib
+    order, base = _lib.load_check().s3r_check_pair_order, 0x7F0000000000
+    assert order(base, base) == 2
+    for gap in (16, 1 << 30, (1 << 40) - 16):
+        assert order(base, base + gap) == 0 and order(base + gap, base) == 1
+    for gap in (1 << 40, (1 << 40) + 16, 1 << 45):
+        assert order(base, base + gap) == 4 and order(base + gap, base) == 4
+
+
 def test_argument_errors_are_reported_without_a_gpu(lib):
     from speed3r_b200 import _lib
     # NULL pointers

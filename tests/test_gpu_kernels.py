@@ -59,6 +59,68 @@ def test_sel16_fwd_offset_follows_growing_scores():
     assert ((lse.cpu() - lse_ref).abs() <= 1e-4 * lse_ref.abs() + 1e-3).all()
 
 
+class FarMemory:
+    """Device memory at addresses at least 2^40 bytes from `near`, as a virtual-memory reservation can have."""
+
+    def __init__(self, near, nbytes):
+        from cuda.bindings import driver as cu
+        self.cu = cu
+        self.prop = cu.CUmemAllocationProp()
+        self.prop.type = cu.CUmemAllocationType.CU_MEM_ALLOCATION_TYPE_PINNED
+        self.prop.location.type = cu.CUmemLocationType.CU_MEM_LOCATION_TYPE_DEVICE
+        self.prop.location.id = torch.cuda.current_device()
+        grain = self.ok(cu.cuMemGetAllocationGranularity(self.prop, cu.CUmemAllocationGranularity_flags.CU_MEM_ALLOC_GRANULARITY_MINIMUM))
+        self.size = -(-nbytes // grain) * grain
+        self.handle = self.ok(cu.cuMemCreate(self.size, self.prop, 0))
+        self.span = (1 << 42) + self.size                          # addresses only: one of its ends is far enough away
+        self.start = self.ok(cu.cuMemAddressReserve(self.span, 0, 0, 0))
+        ends = (int(self.start), int(self.start) + (1 << 42))
+        self.ptr = max(ends, key=lambda e: abs(e - near))
+        self.ok(cu.cuMemMap(self.ptr, self.size, 0, self.handle, 0))
+        access = cu.CUmemAccessDesc()
+        access.location = self.prop.location
+        access.flags = cu.CUmemAccess_flags.CU_MEM_ACCESS_FLAGS_PROT_READWRITE
+        self.ok(cu.cuMemSetAccess(self.ptr, self.size, [access], 1))
+        assert abs(self.ptr - near) >= 1 << 40
+        self.__cuda_array_interface__ = dict(shape=(nbytes // 2,), typestr="<i2", data=(self.ptr, False), version=3)
+
+    def ok(self, r):
+        assert int(r[0]) == 0, r[0]
+        return r[1] if len(r) > 1 else None
+
+    def free(self):
+        torch.cuda.synchronize()
+        self.ok(self.cu.cuMemUnmap(self.ptr, self.size))
+        self.ok(self.cu.cuMemRelease(self.handle))
+        self.ok(self.cu.cuMemAddressFree(self.start, self.span))
+
+
+@pytest.mark.parametrize("block", [16, 32])
+def test_selection_on_tensors_more_than_a_tensor_map_reaches_apart(block):
+    """Values and output gradients 2^41 bytes or more from keys and queries: forward and backward as with tensors side by side."""
+    from speed3r_b200 import ops
+    B, H, T, K = 1, 2, 16 * 21 + 5, 5
+    nb = -(-T // block)
+    q, k, v, do = (randn(s, B, H, T, 64).to(DEV, torch.bfloat16) for s in (1, 2, 3, 4))
+    idx = table(5, B, H, nb, nb, K).to(DEV)
+    def run(v, do):
+        o, lse, _ = ops._sel_fwd(q, k, v, idx, None, None, block, 0.125, True, True, 1)
+        dlt = ops._ops().delta.default(o, do)
+        return (o, lse) + tuple(ops._ops().sel_attn_bwd.default(q, k, v, idx, lse, dlt, do, block, 0.125))
+    want = run(v, do)
+    far = FarMemory(k.data_ptr(), 2 * v.numel() * 2)
+    try:
+        both = torch.as_tensor(far, device=DEV).view(torch.bfloat16).view(2, B, H, T, 64)
+        both[0].copy_(v)
+        both[1].copy_(do)
+        got = run(both[0], both[1])
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        del both
+    finally:
+        far.free()
+
+
 @pytest.mark.parametrize("block, K", [(16, 32), (32, 32), (64, 16)])
 @pytest.mark.parametrize("outgrow", [False, True])
 def test_sel_fwd_rounds_no_more_than_its_result(block, K, outgrow):
