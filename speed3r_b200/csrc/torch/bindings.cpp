@@ -12,6 +12,7 @@
 #include <ATen/ATen.h>
 #include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/CachingHostAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
@@ -985,6 +986,14 @@ std::tuple<Tensor, Tensor> module_train(const Tensor& x, const Tensor& w_qkv, co
   return {r[0], r[1]};
 }
 
+// Tells the pinned-memory allocator that the current stream of `device` works on `host`: what Tensor.copy_ does, and a copy on
+// raw pointers does not.  The memory is not handed out again before the work enqueued so far is done.
+void host_in_use(const Tensor& host, at::Device device) {
+  TORCH_CHECK(host.device().is_cpu() && device.is_cuda(), "host_in_use: a host tensor and a CUDA device");
+  c10::cuda::CUDAGuard guard(device);
+  at::cuda::CachingHostAllocator_recordEvent(host.data_ptr(), host.storage().data_ptr().get_context(), c10::cuda::getCurrentCUDAStream(device.index()));
+}
+
 // a tensor with memory, not one of those that a tracer runs the backward on
 bool plain(const Tensor& t) {
   return t.is_cuda() && !t.key_set().has(c10::DispatchKey::Python) && !t.key_set().has(c10::DispatchKey::Functionalize) &&
@@ -1084,6 +1093,7 @@ TORCH_LIBRARY(speed3r_b200, m) {
   m.def("module_train(Tensor x, Tensor w_qkv, Tensor? b_qkv, Tensor w_gate, Tensor? b_gate, Tensor w_proj, Tensor? b_proj, "
         "Tensor? pos, Tensor? cos, Tensor? sin, Tensor? qw, Tensor? qb, Tensor? kw, Tensor? kb, float eps, int heads, "
         "int block, int topk, float scale) -> (Tensor, Tensor)", &module_train);
+  m.def("host_in_use(Tensor host, Device device) -> ()", &host_in_use);
   m.def("pool_tokens(Tensor x, int kernel, int stride) -> Tensor", &pool_tokens);
   m.def("flash_attn_topk(Tensor q, Tensor k, Tensor v, int topk, float scale, int group, int take) -> (Tensor, Tensor)",
         &flash_attn_topk);

@@ -108,7 +108,7 @@ class HostPipeline:
 
     @torch.no_grad()
     def __call__(self, hq: Tensor, hk: Tensor, hv: Tensor, hgate: Tensor, hy: Tensor) -> None:
-        H, T, d, bs = self.H, self.T, self.d, self.block
+        H, T, d = self.H, self.T, self.d
         for n, t, shape in (("hq", hq, (1, H, T, d)), ("hk", hk, (1, H, T, d)), ("hv", hv, (1, H, T, d)),
                             ("hgate", hgate, (1, H, T, 2)), ("hy", hy, (1, T, H * d))):
             _pinned(t, n)
@@ -118,6 +118,22 @@ class HostPipeline:
         s_in, s_out = self.s_in, self.s_out
         s_in.wait_stream(main)            # device buffers may still be read by an earlier call
         s_out.wait_stream(main)
+        try:
+            self._enqueue(main, hq, hk, hv, hgate, hy)
+        finally:
+            # the caller may drop its tensors at once: their memory is not to be handed out before the copies are done
+            in_use = ops._ops().host_in_use.default
+            with torch.cuda.stream(s_in):
+                for t in (hq, hk, hv, hgate):
+                    in_use(t, self.dev)
+            with torch.cuda.stream(s_out):
+                in_use(hy, self.dev)
+            main.wait_stream(s_out)
+            main.wait_stream(s_in)
+
+    def _enqueue(self, main, hq: Tensor, hk: Tensor, hv: Tensor, hgate: Tensor, hy: Tensor) -> None:
+        H, T, d, bs = self.H, self.T, self.d, self.block
+        s_in, s_out = self.s_in, self.s_out
         copy2d, in_stream, out_stream = _lib.load().s3r_copy2d_async, s_in.cuda_stream, s_out.cuda_stream
         esz = hy.element_size()
         tok = d * esz                     # bytes of a token of one head
@@ -168,5 +184,3 @@ class HostPipeline:
                 _lib.check(copy2d(hy.data_ptr() + t0 * H * tok + h0 * tok, H * tok, y.data_ptr(), n * tok, n * tok, t1 - t0,
                                   out_stream), "s3r_copy2d_async")
             grp_free[b] = done
-        main.wait_stream(s_out)
-        main.wait_stream(s_in)

@@ -680,3 +680,23 @@ def test_module_with_an_output_that_is_not_whole_vectors():
     dy = torch.randn(1, x.shape[1], 100, device=DEV).bfloat16()
     grads = dict(zip(["x"] + [n for n, _ in m.named_parameters()], module_step(m, x, pos, dy)[1:]))
     assert_bf16_close(grads["proj.bias"], dy.float().sum((0, 1)), "bias")
+
+
+# ------------------------------------------------------------------ host pipeline
+def test_host_pipeline_keeps_dropped_tensors_until_they_are_copied():
+    """Pinned memory that the caller gives back while the copies are still enqueued is not handed out again."""
+    from speed3r_b200 import HostPipeline
+    H, T = 4, 512
+    pipe = HostPipeline(H, T, device=torch.device(DEV))
+    shapes = [(1, H, T, 64)] * 3 + [(1, H, T, 2), (1, T, H * 64)]
+    pinned = lambda: [torch.ones(s, dtype=torch.bfloat16, pin_memory=True) for s in shapes]
+    pipe(*pinned())                                                # the pools are filled, the kernels loaded
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)                                 # a tenth of a second in front of every copy
+    tensors = pinned()
+    before = {t.data_ptr() for t in tensors}
+    pipe(*tensors)
+    del tensors
+    after = {t.data_ptr() for t in pinned()}
+    assert not torch.cuda.current_stream().query(), "the copies were not waiting"
+    assert not before & after
