@@ -365,6 +365,15 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
       if (MODE == 1) arrive(&ctl.p_full[t]);
       pass1(xa, 0);
       pass1(xb, 1);
+      // dQ: keys past the end have S = 0, whose P overflows where all of a row's logits are far below zero
+      if (MODE == 1 && i == ntiles - 1) {
+        const int left = p.n_str - i * 64 - half * 32;
+        if (left < 32) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (e >= left) pf[e] = 0.f;
+        }
+      }
       if (MODE == 0) {
         tmem_st_wait();
         arrive(&ctl.p_full[t]);

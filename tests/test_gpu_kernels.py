@@ -601,6 +601,21 @@ def test_colsum(rows, cols):
     assert ((out.double() - ref).abs() <= 2 ** -24 * rows * x.double().abs().sum(0) / rows * 64 + 1e-6).all()
 
 
+@pytest.mark.parametrize("Nc", [65, 96, 127])
+def test_cmp_backward_with_all_logits_far_below_zero(Nc):
+    """Logits near -120: a key past the end, whose score is 0, would weigh e^116."""
+    from speed3r_b200 import ops
+    B, H, Nq = 1, 2, 70
+    q, k, v, do = bf16_round(3.875 + 0.1 * randn(1, B, H, Nq, 64), -3.875 + 0.1 * randn(2, B, H, Nc, 64), randn(3, B, H, Nc, 64),
+                             randn(4, B, H, Nq, 64))
+    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    torch.softmax(ref[0] @ ref[1].transpose(-1, -2) * 0.125, -1).matmul(ref[2]).backward(do)
+    t = [x.to(DEV, torch.bfloat16).requires_grad_(True) for x in (q, k, v)]
+    ops.flash_attn_topk_func(*t, 8)[0].backward(do.to(DEV, torch.bfloat16))
+    for name, a, b in zip(("dq", "dk", "dv"), t, ref):
+        assert_bf16_close(a.grad, b.grad, name)
+
+
 # ------------------------------------------------------------------ the attention module
 def module_and_input(seed, B=1, N=512, H=4, dim=None, **kw):
     import speed3r_b200
