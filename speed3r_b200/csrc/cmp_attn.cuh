@@ -415,8 +415,10 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
       for (int i = 0; i < 32; ++i)
         if (i < p.topk) bound = fminf(bound, fmaxf(gm[i], other[(p.topk - 1 - i) * 128]));
       // a sum's logarithm, less what its exponentials and the second kernel's scores can differ by: 2^-20 from the
-      // exponentials, and roundings of the arguments, each below 2^-24 of their size
-      if (RANK) bound = m_used + log2f(bound) - (6.103515625e-5f + 9.5367431640625e-7f * fabsf(m_used));
+      // exponentials, and roundings of the arguments, each below 2^-24 of their size.  The polynomial exponentials are 2^-126
+      // for anything smaller: a sum in which two of those are more than 2^-21 bounds nothing.
+      if (RANK) bound = bound < 4.930380657631324e-32f /* 2^-104 */ ? -INFINITY
+                                  : m_used + log2f(bound) - (6.103515625e-5f + 9.5367431640625e-7f * fabsf(m_used));
       p.bound[(static_cast<int64_t>(bh) * p.Nq + row) * p.topk] = bound;
       p.lse[static_cast<int64_t>(bh) * p.Nq + row] = (m_used + log2f(l)) * 0.6931471805599453f;
     }

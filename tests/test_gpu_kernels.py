@@ -601,6 +601,27 @@ def test_colsum(rows, cols):
     assert ((out.double() - ref).abs() <= 2 ** -24 * rows * x.double().abs().sum(0) / rows * 64 + 1e-6).all()
 
 
+@pytest.mark.parametrize("take", [1, 3, 4])
+@pytest.mark.parametrize("size, grow", [(30, 1), (60, 1), (100, 1), (10, 8)])
+def test_block_ranking_with_large_logits(take, size, grow):
+    """Rows in which fewer than top-k of the column groups lie within the exponentials' range of the row's largest score, and
+    (grow) rows whose later keys outgrow the first tile's by more than 2^64, so that the keys are taken a second time."""
+    from speed3r_b200 import ops
+    B, H, Nq, Nc, K = 1, 2, 200, 1024, 16
+    ln = lambda x: torch.nn.functional.layer_norm(x, (64,))
+    k = ln(randn(2, B, H, Nc, 64)) * torch.linspace(1, grow, Nc)[:, None]
+    q, k, v = bf16_round(size * ln(randn(1, B, H, Nq, 64)), k, ln(randn(3, B, H, Nc, 64)))
+    o_ref, _, idx_ref = R.cmp_attn_topk(q, k, v, K, rank_group=(4, take))
+    o, idx = ops.flash_attn_blocktopk_func(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), K, 4, take)
+    assert_bf16_close(o, o_ref, "o_c")
+    scores = R.block_rank_scores(q @ k.transpose(-1, -2), 0.125, 4, take)
+    idx, idx_ref = idx.cpu().long(), idx_ref.long()
+    assert (idx.sort(-1).values.diff(dim=-1) > 0).all(), "a block listed twice"
+    gap = (torch.gather(scores, -1, idx) - torch.gather(scores, -1, idx_ref)).abs()
+    # rounding of scores of this size: a few units of 2^-24 of the largest in both
+    assert gap.max() <= 1e-3 + 1e-6 * scores.abs().max(), f"{gap.max():.4g}"
+
+
 @pytest.mark.parametrize("Nc", [65, 96, 127])
 def test_cmp_backward_with_all_logits_far_below_zero(Nc):
     """Logits near -120: a key past the end, whose score is 0, would weigh e^116."""
