@@ -340,7 +340,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     auto set_offsets = [&](float bound) {
       off01 = make_float2(-bound, p.rank_take > 1 ? -bound : -INFINITY);
       off23 = make_float2(p.rank_take > 2 ? -bound : -INFINITY, p.rank_take > 3 ? -bound : -INFINITY);
-      cutoff = fabsf(bound) < 8192.f ? 0.999f : 0.f;
+      cutoff = bound == INFINITY ? INFINITY : fabsf(bound) < 8192.f ? 0.999f : 0.f;      // +inf: a row past the end takes nothing
     };
     if (RANK) set_offsets(fmaxf(thr, -3.402823466e38f));
     const bool four = p.rank_take > 3;
