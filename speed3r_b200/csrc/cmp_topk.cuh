@@ -2,6 +2,11 @@
 // (RANK 0), ordered by (logit descending, column ascending), or the `topk` blocks of four columns (RANK 1) by
 // log2 of the sum of 2^(c * s) over a block's first rank_take columns, which needs no row normaliser.
 //
+// RANK 0 compares its logits exactly with a bound that the first kernel took from products of another shape (N = 128 instead of
+// 64) with the keys in another order.  An element of S is the sum over its own row and column alone, in the same k-steps of
+// 16 channels of the same instruction, so neither its neighbours nor N should matter; nothing documents it, and one unit's
+// difference would lose the entries at the bound.  test_cmp_topk_keeps_logits_at_the_bound has the bound on single logits.
+//
 // The first kernel (cmp_attn.cuh) leaves a lower bound of each row's topk-th largest logit, so this one repeats Q K^T on
 // the tensor cores and only collects the logits that reach the bound - about 44 per row with independent scores - into
 // lists of (logit, column) pairs in shared memory, [slot][lane] so that a thread's accesses never meet another's on a

@@ -601,6 +601,22 @@ def test_colsum(rows, cols):
     assert ((out.double() - ref).abs() <= 2 ** -24 * rows * x.double().abs().sum(0) / rows * 64 + 1e-6).all()
 
 
+@pytest.mark.parametrize("Nq, Nc, topk", [(700, 64, 1), (700, 64, 5), (700, 64, 32), (300, 40, 32), (1000, 1024, 1), (1000, 2001, 1), (2500, 8000, 1)])
+def test_cmp_topk_keeps_logits_at_the_bound(Nq, Nc, topk):
+    """With one entry per row, or one column per group, the bound is itself the last entry's logit: the collection's products
+    have to reproduce it bit for bit, or the entry is missing (and the last column in its place)."""
+    from speed3r_b200 import ops
+    B, H = 1, 16
+    ln = lambda x: torch.nn.functional.layer_norm(x, (64,)).to(DEV, torch.bfloat16)
+    q, k, v = ln(randn(1, B, H, Nq, 64)), ln(randn(2, B, H, Nc, 64)), ln(randn(3, B, H, Nc, 64))
+    _, _, idx = ops._cmp_fwd(q, k, v, topk, 0.125)
+    S = q.double() @ k.double().transpose(-1, -2)
+    want = S.topk(topk, dim=-1).values
+    got = torch.gather(S, -1, idx.long())
+    assert (idx.sort(-1).values.diff(dim=-1) > 0).all(), "padding, or a column twice"
+    assert (got - want).abs().max() <= 1e-4                        # fp32 sums of 64 products of size 1 to 10
+
+
 @pytest.mark.parametrize("take", [1, 3, 4])
 @pytest.mark.parametrize("size, grow", [(30, 1), (60, 1), (100, 1), (10, 8)])
 def test_block_ranking_with_large_logits(take, size, grow):
