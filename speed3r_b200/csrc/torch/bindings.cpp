@@ -74,15 +74,16 @@ Tensor pool_fwd(const Tensor& x, int64_t kernel, int64_t stride) {
   return out;
 }
 
-// q pooled per block, k and v with kernel/stride, in one launch
+// q pooled per block, k and v with kernel/stride, in one launch where they are of one length
 std::tuple<Tensor, Tensor, Tensor> pool_qkv_fwd(const Tensor& q, const Tensor& k, const Tensor& v, int64_t block,
                                                 int64_t kernel, int64_t stride) {
   const Tensor* x[3] = {&q, &k, &v};
   for (const Tensor* t : x) {
     need(*t, "x", at::kBFloat16, false);
-    TORCH_CHECK(t->dim() == 4 && t->sizes() == q.sizes() && t->stride(3) == 1,
-                "pool: q, k, v must be [B,H,T,d] of one shape and their channel dimension must have unit stride");
+    TORCH_CHECK(t->dim() == 4 && t->stride(3) == 1, "pool: q, k, v must be [B,H,T,d] and their channel dimension must have unit stride");
   }
+  if (q.sizes() != k.sizes() || k.sizes() != v.sizes())            // queries against another sequence
+    return {pool_fwd(q, block, block), pool_fwd(k, kernel, stride), pool_fwd(v, kernel, stride)};
   const int64_t B = q.size(0), H = q.size(1), T = q.size(2), d = q.size(3);
   c10::cuda::CUDAGuard guard(q.device());
   Tensor out[3];

@@ -80,9 +80,8 @@ def _register_fakes() -> None:
 
     @fake("speed3r_b200::pool_qkv_fwd")
     def _(q, k, v, block, kernel, stride):
-        B, H, T, d = q.shape
-        nc = (T - kernel) // stride + 1
-        return tuple(q.new_empty(B, H, n, d) for n in ((T - block) // block + 1, nc, nc))
+        window = lambda x, kernel, stride: x.new_empty(*x.shape[:2], (x.shape[2] - kernel) // stride + 1, x.shape[3])
+        return window(q, block, block), window(k, kernel, stride), window(v, kernel, stride)
 
     @fake("speed3r_b200::prologue_fwd")
     def _(qkv, heads, block, pos, cos, sin, qw, qb, kw, kb, eps):

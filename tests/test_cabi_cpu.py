@@ -145,6 +145,17 @@ def test_native_module_refuses_shapes_that_do_not_fit(op):
         call(x=(1, N + 1, C), pos=(1, N + 1, 2))
 
 
+def test_op_shapes_for_queries_and_keys_of_different_lengths():
+    """Shape functions alone (meta tensors): the table and the output follow the queries."""
+    from speed3r_b200 import ops
+    q = torch.empty(1, 2, 256, 64, dtype=torch.bfloat16, device="meta")
+    k, gate = q.new_empty(1, 2, 512, 64), q.new_empty(1, 2, 256, 2)
+    for a, b in ((q, k), (q.requires_grad_(True), k)):
+        y, idx = ops.sparse_attention_op(a, b, b, gate, 16, 8)
+        assert y.shape == (1, 256, 128) and idx.shape == (1, 2, 16, 8)
+    assert [tuple(t.shape) for t in ops._ops().pool_qkv_fwd.default(q, k, k, 16, 16, 16)] == [(1, 2, 16, 64), (1, 2, 32, 64), (1, 2, 32, 64)]
+
+
 def test_module_keeps_reference_state_dict_keys_and_init():
     """Keys and gate initialisation of pi3/models/layers/sparse_attention.py:62-86."""
     import speed3r_b200

@@ -653,6 +653,30 @@ def test_cmp_backward_with_all_logits_far_below_zero(Nc):
         assert_bf16_close(a.grad, b.grad, name)
 
 
+@pytest.mark.parametrize("Tq, Tk, setting", [(512, 1024, (16, 32, 16, 16)), (1040, 336, (16, 8, 16, 16)), (256, 1024, (64, 4, 32, 16))])
+def test_op_on_queries_and_keys_of_different_lengths(Tq, Tk, setting):
+    """The whole op, forward and backward, where queries attend to another sequence."""
+    from speed3r_b200 import ops
+    B, H = 1, 2
+    block, topk, kernel, stride = setting
+    q, k, v = bf16_round(randn(1, B, H, Tq, 64), randn(2, B, H, Tk, 64), randn(3, B, H, Tk, 64))
+    gate, = bf16_round(torch.sigmoid(randn(4, B, H, Tq, 2)))
+    dy, = bf16_round(randn(5, B, Tq, H * 64))
+    t = [x.to(DEV, torch.bfloat16).requires_grad_(True) for x in (q, k, v, gate)]
+    y, idx = ops.sparse_attention_op(*t, *setting)
+    y.backward(dy.to(DEV, torch.bfloat16))
+    with torch.no_grad():
+        assert torch.equal(ops.sparse_attention_op(*t, *setting)[0], y)
+    r = [x.clone().requires_grad_(True) for x in (q, k, v, gate)]
+    pooled = R.pool_tokens(r[0], block, block), R.pool_tokens(r[1], kernel, stride), R.pool_tokens(r[2], kernel, stride)
+    o_c = torch.softmax(pooled[0] @ pooled[1].transpose(-1, -2) * 0.125, -1) @ pooled[2]
+    y_ref = R.gated_merge(r[3], o_c, R.sel_attn(r[0], r[1], r[2], idx.cpu(), block)[0], block)
+    y_ref.backward(dy)
+    assert_bf16_close(y, y_ref, "y")
+    for name, a, b in zip(("dq", "dk", "dv", "dgate"), t, r):
+        assert_bf16_close(a.grad, b.grad, name)
+
+
 # ------------------------------------------------------------------ the attention module
 def module_and_input(seed, B=1, N=512, H=4, dim=None, **kw):
     import speed3r_b200
