@@ -38,6 +38,12 @@ void need(const Tensor& t, const char* name, at::ScalarType dtype = at::kBFloat1
   TORCH_CHECK(!contiguous || t.is_contiguous(), name, " must be contiguous");
 }
 
+// Sizes that are divided by: a division by zero ends the process in C++, where Python raised.
+template <typename... N>
+void need_positive(const char* what, N... n) {
+  TORCH_CHECK(((n > 0) && ...), what, ": block, window and stride must be positive");
+}
+
 void check(int rc, const char* what) {
   if (rc == 0) return;
   char msg[512];
@@ -64,6 +70,7 @@ Tensor none(const Tensor& like) { return at::empty({0}, like.options()); }
 // base operators
 // ------------------------------------------------------------------------------------------------
 Tensor pool_fwd(const Tensor& x, int64_t kernel, int64_t stride) {
+  need_positive("pool", kernel, stride);
   need(x, "x", at::kBFloat16, false);
   TORCH_CHECK(x.dim() == 4 && x.stride(3) == 1, "pool: x must be [B,H,T,d] and its channel dimension must have unit stride");
   const int64_t B = x.size(0), H = x.size(1), T = x.size(2), d = x.size(3);
@@ -77,6 +84,7 @@ Tensor pool_fwd(const Tensor& x, int64_t kernel, int64_t stride) {
 // q pooled per block, k and v with kernel/stride, in one launch where they are of one length
 std::tuple<Tensor, Tensor, Tensor> pool_qkv_fwd(const Tensor& q, const Tensor& k, const Tensor& v, int64_t block,
                                                 int64_t kernel, int64_t stride) {
+  need_positive("pool", block, kernel, stride);
   const Tensor* x[3] = {&q, &k, &v};
   for (const Tensor* t : x) {
     need(*t, "x", at::kBFloat16, false);
@@ -184,6 +192,7 @@ void need_gate(const Tensor& gate) {
 std::tuple<Tensor, Tensor, Tensor> sel_attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& idx,
                                                 const optional<Tensor>& gate, const optional<Tensor>& o_c, int64_t block,
                                                 double scale, bool want_o, bool want_lse, int64_t kv_chunks) {
+  need_positive("selection attention", block);
   need(q, "q");
   need(k, "k");
   need(v, "v");
@@ -268,6 +277,7 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q, const Tensor& k, con
                                            const Tensor& lse, const Tensor& delta, const Tensor& do_s_, const Tensor* dq_c,
                                            const Tensor* dk_c, const Tensor* dv_c, int64_t block, int64_t kernel,
                                            int64_t stride, double scale, const std::tuple<Tensor, Tensor>* inverse = nullptr) {
+  need_positive("selection attention", block, kernel, stride);
   need(q, "q");
   need(k, "k");
   need(v, "v");
@@ -341,9 +351,9 @@ const float* f32_or_null(const optional<Tensor>& t) { return t.has_value() ? f32
 // What the prologue's arguments have to be; returns the rows of the rotary tables (0: no rotary embedding)
 int64_t need_prologue(const Tensor& qkv, int64_t heads, int64_t block, const optional<Tensor>& pos, const optional<Tensor>& cos,
                       const optional<Tensor>& sin, std::initializer_list<const optional<Tensor>*> norms) {
+  TORCH_CHECK(qkv.dim() >= 3 && heads > 0 && block > 0 && qkv.numel() > 0, "qkv_prologue: qkv must be [B,N,3*H*d] and not empty");
   need(qkv, "qkv");
-  TORCH_CHECK(qkv.dim() >= 3 && heads > 0 && block > 0, "qkv_prologue: qkv must be [B,N,3*H*d]");
-  const int64_t B = qkv.size(0), N = qkv.size(1), C3 = B * N > 0 ? qkv.numel() / (B * N) : 0, d = C3 / (3 * heads);
+  const int64_t B = qkv.size(0), N = qkv.size(1), C3 = qkv.numel() / (B * N), d = C3 / (3 * heads);
   TORCH_CHECK(C3 == 3 * heads * d && N % block == 0, "qkv_prologue: qkv ", qkv.sizes(), " does not split into 3 x ", heads,
               " heads, or N=", N, " is not a multiple of the block ", block);
   for (const auto* w : norms) {

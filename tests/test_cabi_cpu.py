@@ -145,6 +145,27 @@ def test_native_module_refuses_shapes_that_do_not_fit(op):
         call(x=(1, N + 1, C), pos=(1, N + 1, 2))
 
 
+def test_sizes_that_are_divided_by_are_looked_at_first():
+    """Zero blocks, windows and strides and empty projections raise (before the device is looked at, so that this needs no
+    GPU): divided by in native code, they would end the process."""
+    from speed3r_b200 import ops
+    o = ops._ops()
+    x, f = torch.zeros(1, 2, 64, 64, dtype=torch.bfloat16), torch.zeros(1, 2, 64)
+    idx = torch.zeros(1, 2, 4, 8, dtype=torch.int32)
+    for call in (lambda: o.pool_fwd.default(x, 0, 16), lambda: o.pool_fwd.default(x, 16, 0), lambda: ops.pool_tokens(x, 16, 0),
+                 lambda: o.pool_qkv_fwd.default(x, x, x, 0, 16, 16), lambda: o.pool_qkv_fwd.default(x, x, x, 16, 16, 0),
+                 lambda: ops.topk_blocksparse_attention(x, x, x, idx, 0), lambda: ops.sel_attn_merge(x, x, x, idx, x, x, 0),
+                 lambda: ops.sel_attn_merge_chunked(x, x[None], x[None], idx, x, x, 0),
+                 lambda: o.sel_attn_bwd.default(x, x, x, idx, f, f, x, 0, 0.125),
+                 lambda: o.sel_attn_bwd_pooled.default(x, x, x, idx, f, f, x, x, x, x, 16, 16, 0, 0.125),
+                 lambda: ops.sparse_attention_op(x, x, x, x, 0, 8, 0, 0)):
+        with pytest.raises(RuntimeError, match="must be positive"):
+            call()
+    for shape in ((0, 16, 384), (1, 0, 384), (1, 16, 0)):
+        with pytest.raises(RuntimeError, match="not empty"):
+            o.prologue_fwd.default(torch.zeros(shape, dtype=torch.bfloat16), 2, 16, None, None, None, None, None, None, None, 1e-5)
+
+
 def test_op_shapes_for_queries_and_keys_of_different_lengths():
     """Shape functions alone (meta tensors): the table and the output follow the queries."""
     from speed3r_b200 import ops
