@@ -309,6 +309,7 @@ std::tuple<Tensor, Tensor, Tensor> sel_attn_bwd_pooled(const Tensor& q, const Te
                                                        const Tensor& lse, const Tensor& delta, const Tensor& do_s,
                                                        const Tensor& dq_c, const Tensor& dk_c, const Tensor& dv_c,
                                                        int64_t block, int64_t kernel, int64_t stride, double scale) {
+  need_positive("selection attention", block, kernel, stride);
   need(dq_c, "dq_c");
   need(dk_c, "dk_c");
   need(dv_c, "dv_c");
