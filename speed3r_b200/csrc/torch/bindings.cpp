@@ -481,8 +481,17 @@ std::tuple<Tensor, Tensor> call_prologue_bwd(const Tensor& qkv, int64_t heads, i
 // ------------------------------------------------------------------------------------------------
 // differentiable operators
 // ------------------------------------------------------------------------------------------------
+// Forward-mode derivatives are refused, in every operator and whether a gradient is wanted or not: past the nodes, the base
+// operators would drop a tangent without a word.
+bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); }
+bool has_tangent(const optional<Tensor>& t) { return t.has_value() && has_tangent(*t); }
+template <typename... T>
+void no_tangents(const T&... t) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!(has_tangent(t) || ...), "speed3r_b200: forward mode AD is not implemented for the operators of this package");
+}
 template <typename... T>
 bool wants_grad(const T&... t) {
+  no_tangents(t...);
   return at::GradMode::is_enabled() && (t.requires_grad() || ...);
 }
 
@@ -611,6 +620,7 @@ SixTensors prologue(const Tensor& qkv, int64_t heads, int64_t block, const optio
   auto as = [&](const optional<Tensor>& t, at::ScalarType type) {
     return t.has_value() ? optional<Tensor>(t->to(qkv.device(), type).contiguous()) : t;
   };
+  no_tangents(qkv, qw_, qb_, kw_, kb_);
   TORCH_CHECK(!pos_.has_value() || pos_->device() == qkv.device(), "qkv_prologue: pos must be on ", qkv.device());
   const auto pos = as(pos_, at::kLong), qw = as(qw_, at::kFloat), qb = as(qb_, at::kFloat), kw = as(kw_, at::kFloat), kb = as(kb_, at::kFloat);
   auto grad = [](const optional<Tensor>& t) { return t.has_value() && t->requires_grad(); };
@@ -668,6 +678,7 @@ std::tuple<Tensor, Tensor> module_infer(const Tensor& x_, const Tensor& w_qkv, c
                                         const optional<Tensor>& qw_, const optional<Tensor>& qb_, const optional<Tensor>& kw_,
                                         const optional<Tensor>& kb_, double eps, int64_t heads, int64_t block, int64_t topk,
                                         double scale) {
+  no_tangents(x_, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, qw_, qb_, kw_, kb_);
   at::AutoDispatchBelowAutograd below;
   c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
   need_module(x_, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, pos_, cos, sin, {&qw_, &qb_, &kw_, &kb_}, heads, block);
@@ -987,6 +998,7 @@ std::tuple<Tensor, Tensor> module_train(const Tensor& x, const Tensor& w_qkv, co
                                         const optional<Tensor>& qw_, const optional<Tensor>& qb_, const optional<Tensor>& kw_,
                                         const optional<Tensor>& kb_, double eps, int64_t heads, int64_t block, int64_t topk,
                                         double scale) {
+  no_tangents(x, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, qw_, qb_, kw_, kb_);
   need_module(x, w_qkv, b_qkv, w_gate, b_gate, w_proj, b_proj, pos_, cos, sin, {&qw_, &qb_, &kw_, &kb_}, heads, block);
   TORCH_CHECK(heads % 4 == 0 && b_qkv.has_value() == b_gate.has_value(), "module_train: heads in fours, and biases of qkv and gate together");
   auto as = [&](const optional<Tensor>& t, at::ScalarType type) {

@@ -166,6 +166,33 @@ def test_sizes_that_are_divided_by_are_looked_at_first():
             o.prologue_fwd.default(torch.zeros(shape, dtype=torch.bfloat16), 2, 16, None, None, None, None, None, None, None, 1e-5)
 
 
+def differentiable_calls(t, gate):
+    from speed3r_b200 import ops
+    idx = torch.zeros(1, 2, 4, 2, dtype=torch.int32, device=t.device)
+    return {"pool": lambda: ops.pool_tokens(t), "compression": lambda: ops.flash_attn_topk_func(t, t, t, 2)[0],
+            "blocks": lambda: ops.flash_attn_blocktopk_func(t, t, t, 2, 4, 3)[0],
+            "selection": lambda: ops.topk_blocksparse_attention(t, t, t, idx, 16),
+            "merge": lambda: ops.sel_attn_merge(t, t, t, idx, gate, t[:, :, :4].contiguous(), 16),
+            "op": lambda: ops.sparse_attention_op(t, t, t, gate, 16, 2)[0],
+            "prologue": lambda: ops._prologue(t.transpose(1, 2).reshape(1, 64, 128).repeat(1, 1, 3), 2, 16, None, None, None, None, None)[0]}
+
+
+def meta_inputs():
+    return (torch.empty(s, dtype=torch.bfloat16, device="meta") for s in ((1, 2, 64, 64), (1, 2, 64, 2)))
+
+
+@pytest.mark.parametrize("name", ["pool", "compression", "blocks", "selection", "merge", "op", "prologue"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_forward_mode_is_refused(name, grad):
+    """A tangent is not dropped without a word, with reverse-mode gradients or without (meta tensors: no kernel runs)."""
+    import torch.autograd.forward_ad as fa
+    x, gate = meta_inputs()
+    with fa.dual_level():
+        t = fa.make_dual(x.requires_grad_(grad), torch.empty_like(x))
+        with pytest.raises((NotImplementedError, RuntimeError), match="not implemented"):
+            differentiable_calls(t, gate)[name]()
+
+
 def test_op_shapes_for_queries_and_keys_of_different_lengths():
     """Shape functions alone (meta tensors): the table and the output follow the queries."""
     from speed3r_b200 import ops
