@@ -17,6 +17,8 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/library.h>
 
 #include <cmath>
@@ -495,6 +497,30 @@ bool wants_grad(const T&... t) {
   return at::GradMode::is_enabled() && (t.requires_grad() || ...);
 }
 
+// A backward of a node.  It runs without recording; where its result is to be differentiated again (create_graph), the result
+// raises when that is tried: no operator here has a second derivative, and without this one would be missing silently.
+template <typename F>
+variable_list once(const variable_list& incoming, F&& backward) {
+  const bool again = at::GradMode::is_enabled();
+  variable_list g;
+  {
+    at::NoGradGuard no_grad;
+    g = backward();
+  }
+  if (!again) return g;
+  // the error stands between the result and all it depends on: the node's own inputs and the incoming gradients
+  torch::autograd::edge_list edges = torch::autograd::collect_next_edges(incoming);
+  if (const auto node = torch::autograd::get_current_node()) edges.insert(edges.end(), node->next_edges().begin(), node->next_edges().end());
+  const auto error = std::make_shared<torch::autograd::Error>("the backward of speed3r_b200 operators cannot be differentiated again",
+                                                              std::move(edges));
+  for (Tensor& t : g)
+    if (t.defined()) {
+      t = t.detach();
+      torch::autograd::set_history(t, error);
+    }
+  return g;
+}
+
 struct PoolNode : torch::autograd::Function<PoolNode> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t kernel, int64_t stride) {
     ctx->saved_data["T"] = x.size(2);
@@ -504,6 +530,9 @@ struct PoolNode : torch::autograd::Function<PoolNode> {
     return call_pool_fwd(x, kernel, stride);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return once(g, [&] { return gradients(ctx, g); });
+  }
+  static variable_list gradients(AutogradContext* ctx, const variable_list& g) {
     return {call_pool_bwd(g[0].contiguous(), ctx->saved_data["T"].toInt(), ctx->saved_data["kernel"].toInt(),
                           ctx->saved_data["stride"].toInt()), Tensor(), Tensor()};
   }
@@ -524,6 +553,9 @@ struct CmpNode : torch::autograd::Function<CmpNode> {
     return {o, idx};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return once(g, [&] { return gradients(ctx, g); });
+  }
+  static variable_list gradients(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
     auto [dq, dk, dv] = call_cmp_bwd(s[0], s[1], s[2], s[3], s[4],
                                      g[0].defined() ? g[0].contiguous() : at::zeros_like(s[3]), ctx->saved_data["scale"].toDouble());
@@ -552,6 +584,9 @@ struct SelNode : torch::autograd::Function<SelNode> {
     return o;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return once(g, [&] { return gradients(ctx, g); });
+  }
+  static variable_list gradients(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
     const Tensor d_o = g[0].contiguous();
     auto [dq, dk, dv] = call_sel_bwd(s[0], s[1], s[2], s[5], s[4], call_delta(s[3], d_o), d_o,
@@ -575,6 +610,9 @@ struct SelMergeNode : torch::autograd::Function<SelMergeNode> {
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return once(g, [&] { return gradients(ctx, g); });
+  }
+  static variable_list gradients(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
     const int64_t block = ctx->saved_data["block"].toInt();
     auto [do_s, dgate, do_c, dlt] = call_merge_bwd(g[0].contiguous(), s[4], s[5], s[6], block);
@@ -603,6 +641,9 @@ struct PrologueNode : torch::autograd::Function<PrologueNode> {
     return {q, k, v, q_c, k_c, v_c};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return once(g, [&] { return gradients(ctx, g); });
+  }
+  static variable_list gradients(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
     auto opt = [](const Tensor& t) { return t.defined() ? optional<Tensor>(t) : optional<Tensor>(); };
     auto [dqkv, dp] = call_prologue_bwd(s[0], ctx->saved_data["heads"].toInt(), ctx->saved_data["block"].toInt(), opt(s[1]), opt(s[2]),
@@ -901,6 +942,9 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return once(g, [&] { return gradients(ctx, g); });
+  }
+  static variable_list gradients(AutogradContext* ctx, const variable_list& g) {
     if (!g[0].defined()) return variable_list(19);
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const auto s = ctx->get_saved_variables();
@@ -1015,7 +1059,7 @@ std::tuple<Tensor, Tensor> module_train(const Tensor& x, const Tensor& w_qkv, co
 void host_in_use(const Tensor& host, at::Device device) {
   TORCH_CHECK(host.device().is_cpu() && device.is_cuda(), "host_in_use: a host tensor and a CUDA device");
   c10::cuda::CUDAGuard guard(device);
-  at::cuda::CachingHostAllocator_recordEvent(host.data_ptr(), host.storage().data_ptr().get_context(), c10::cuda::getCurrentCUDAStream(device.index()));
+  at::getHostAllocator(at::kCUDA)->record_event(host.data_ptr(), host.storage().data_ptr().get_context(), c10::cuda::getCurrentCUDAStream(device.index()));
 }
 
 // a tensor with memory, not one of those that a tracer runs the backward on
@@ -1045,6 +1089,9 @@ struct SparseNode : torch::autograd::Function<SparseNode> {
     return {y, idx};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    return once(g, [&] { return gradients(ctx, g); });
+  }
+  static variable_list gradients(AutogradContext* ctx, const variable_list& g) {
     const auto s = ctx->get_saved_variables();
     const int64_t block = ctx->saved_data["block"].toInt();
     const double scale = ctx->saved_data["scale"].toDouble();

@@ -193,6 +193,18 @@ def test_forward_mode_is_refused(name, grad):
             differentiable_calls(t, gate)[name]()
 
 
+@pytest.mark.parametrize("name", ["pool", "compression", "blocks", "selection", "merge", "op", "prologue"])
+def test_second_derivatives_are_refused(name):
+    """A gradient taken with create_graph is there; differentiating it raises instead of leaving these operators out."""
+    x, gate = meta_inputs()
+    x.requires_grad_(True)
+    y = differentiable_calls(x, gate)[name]()
+    first, = torch.autograd.grad((y.float() * y.float()).sum(), x, create_graph=True)
+    assert first.requires_grad
+    with pytest.raises(RuntimeError, match="cannot be differentiated again"):
+        torch.autograd.grad(first.sum(), x)
+
+
 def test_op_shapes_for_queries_and_keys_of_different_lengths():
     """Shape functions alone (meta tensors): the table and the output follow the queries."""
     from speed3r_b200 import ops

@@ -758,6 +758,20 @@ def test_module_with_an_output_that_is_not_whole_vectors():
     assert_bf16_close(grads["proj.bias"], dy.float().sum((0, 1)), "bias")
 
 
+def test_module_gradients_with_a_graph_are_the_same_and_final():
+    m, x, pos = module_and_input(0)
+    x.requires_grad_(True)
+    dy = torch.randn(x.shape, device=DEV).bfloat16()
+    want = module_step(m, x, pos, dy)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = m(x, xpos=pos)
+    got = torch.autograd.grad(y, [x] + list(m.parameters()), dy, create_graph=True)
+    assert all(torch.equal(a, b) and a.requires_grad for a, b in zip(got, want[1:]))
+    for g in got:
+        with pytest.raises(RuntimeError, match="cannot be differentiated again"):
+            torch.autograd.grad(g.sum(), x, retain_graph=True)
+
+
 # ------------------------------------------------------------------ host pipeline
 def test_host_pipeline_keeps_dropped_tensors_until_they_are_copied():
     """Pinned memory that the caller gives back while the copies are still enqueued is not handed out again."""
