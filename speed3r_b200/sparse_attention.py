@@ -62,8 +62,14 @@ def _global_hooks() -> bool:
 
 
 def _watched(m: nn.Module) -> bool:
-    """Somebody's hook wants to see this module called."""
-    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+    """Somebody wants to see this module called: a hook, or a ``forward`` of its own on the instance (as offloading and
+    quantisation wrappers put there)."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__)
+
+
+def _plain_rope(rope) -> bool:
+    """A rotary module whose ``forward`` is the table look-up that the prologue does itself."""
+    return rope is None or not (_watched(rope) or (isinstance(rope, RoPE2D) and type(rope).forward is not RoPE2D.forward))
 
 
 def rope_tables(rope, D: int, rows: int, device, dtype):
@@ -185,14 +191,22 @@ class SparseFlashAttentionRope(nn.Module):
             return False
         return d == 64 and N % Bs == 0 and self.num_heads <= 42
 
+    def _trains_through_prologue(self, xpos, N, Bs, d) -> bool:
+        """``_prologue_takes``, and the norms and the rotary module are what they look like: with gradients they are called
+        unless they are."""
+        mods = self._modules
+        return (all(type(m) in (nn.LayerNorm, nn.Identity) and not _watched(m) for m in (mods["q_norm"], mods["k_norm"])) and
+                not _global_hooks() and (xpos is None or _plain_rope(self.rope)) and self._prologue_takes(xpos, N, Bs, d))
+
     def _native_op(self, x, xpos, N, Bs, d):
         """The native operator that runs the whole module, or None: plain Linear projections that nobody watches, bf16 (by
-        autocast or by dtype), no sequence partition; with gradients fp32 parameters under autocast.  Sub-modules and
+        autocast or by dtype), no sequence partition; with gradients fp32 parameters under autocast.  A dispatch mode (a
+        tracer, a counter) sees no kernel of a native call, so under one the steps are taken apart.  Sub-modules and
         parameters are taken from their dictionaries: nn.Module's attribute look-up was half of the 12 us this took."""
         mods = self._modules
         qkv, gate, proj = mods["qkv"], mods["gate"], mods["proj"]
         if (self.seq_parallel is not None or not x.is_cuda or type(x) is not Tensor or type(gate) is not nn.Sequential or
-                len(gate._modules) != 2 or _global_hooks() or torch.compiler.is_compiling()):
+                len(gate._modules) != 2 or _global_hooks() or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack()):
             return None
         glin, act = gate._modules.values()
         if type(act) is not nn.Sigmoid:
@@ -226,7 +240,7 @@ class SparseFlashAttentionRope(nn.Module):
         if self._can_fuse_prologue(None, x, xpos, N, Bs, d):
             return ops._ops().module_infer.default
         if (torch.is_grad_enabled() and autocast and self.num_heads % 4 == 0 and not narrow and
-                (qkv._parameters["bias"] is None) == (glin._parameters["bias"] is None) and self._prologue_takes(xpos, N, Bs, d)):
+                (qkv._parameters["bias"] is None) == (glin._parameters["bias"] is None) and self._trains_through_prologue(xpos, N, Bs, d)):
             return ops._ops().module_train.default
         return None
 
@@ -296,7 +310,7 @@ class SparseFlashAttentionRope(nn.Module):
         gate = gate.to(qkv.dtype)
         if self._can_fuse_prologue(qkv, x, xpos, N, Bs, d):
             return self._forward_fused(qkv.detach(), gate, xpos, B, N, H, d, Bs)
-        if torch.is_grad_enabled() and self._prologue_takes(xpos, N, Bs, d):
+        if torch.is_grad_enabled() and self._trains_through_prologue(xpos, N, Bs, d):
             return self._forward_fused(qkv, gate, xpos, B, N, H, d, Bs, train=True)
         if self.seq_parallel is not None and N % Bs != 0:
             raise RuntimeError("sequence-parallel attention needs whole 16-token blocks on every rank")
