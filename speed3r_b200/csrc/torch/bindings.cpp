@@ -963,6 +963,35 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
     auto view = [&](int64_t at, int64_t r, int64_t c) { return buf.as_strided({r, c}, {c, 1}, at); };
     const Tensor dy = aligned(g[0].to(at::kBFloat16).contiguous()).view({m.M, out_features});
 
+    // the output projection's own gradients; is anything before it wanted?
+    auto colsum = [&](const void* x, int64_t cols, void* ws, size_t bytes) {
+      Tensor o = at::empty({cols}, buf.options().dtype(at::kFloat));
+      check(s3r_colsum(x, f32(o), m.M, cols, ws, bytes, st), "s3r_colsum");
+      return o;
+    };
+    Tensor dwp, dbp;
+    auto output_projection = [&]() {
+      if (ctx->needs_input_grad(e_wp)) dwp = at::mm(dy.t(), view(m.y, m.M, m.C), at::kFloat);
+      if (!ints[5] || !ctx->needs_input_grad(e_wp + 1)) return;
+      if (out_features % 8 == 0) {
+        const Tensor ws = fresh({static_cast<int64_t>(s3r_colsum_workspace_bytes(m.M, out_features))}, buf, at::kByte);
+        dbp = colsum(dy.data_ptr(), out_features, ws.data_ptr(), ws.numel());
+      } else {
+        dbp = dy.sum(0, false, at::kFloat);                  // the kernel reads rows of whole vectors
+      }
+    };
+    const size_t e_norm = e_wp + (ints[5] ? 2 : 1) + (rope ? 3 : 0);
+    bool before = false;
+    for (size_t e = 0; e < e_wp; ++e) before |= ctx->needs_input_grad(e);
+    for (size_t e = e_norm; norm && e < e_norm + 4; ++e) before |= ctx->needs_input_grad(e);
+    if (!before) {
+      output_projection();
+      variable_list out(19);
+      out[5] = dwp;
+      out[6] = dbp;
+      return out;
+    }
+
     // scratch of the backward, bytes
     int64_t used = 0;
     auto part = [&](int64_t bytes) {
@@ -977,7 +1006,7 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
                   a_qids = part(4 * BH * m.Nc * m.topk);
     const size_t csr_bytes = s3r_csr_workspace_bytes(m.B, m.H, m.Nc, m.topk, m.Nc),
                  pro_bytes = norm ? s3r_qkv_prologue_bwd_workspace_bytes(m.B, m.H, m.N, m.block) : 0,
-                 col_bytes = std::max(s3r_colsum_workspace_bytes(m.M, m.P), s3r_colsum_workspace_bytes(m.M, out_features));
+                 col_bytes = s3r_colsum_workspace_bytes(m.M, m.P);
     const int64_t a_csr = part(csr_bytes), a_pro = part(pro_bytes), a_col = part(col_bytes);
     const Tensor scratch = at::empty({used / 2}, buf.options());
     char* sb = static_cast<char*>(scratch.data_ptr());
@@ -987,18 +1016,9 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
 
     int32_t *off = static_cast<int32_t*>(sp(a_off)), *qids = static_cast<int32_t*>(sp(a_qids));
     CsrBeside beside(i32(idx), off, qids, m.B, m.H, m.Nc, m.topk, m.Nc, sp(a_csr), csr_bytes);
-    // output projection
     Tensor dya = sview(a_dy, m.M, m.C);
     at::mm_out(dya, dy, view(m.wp, out_features, m.C));
-    Tensor dwp, dbp;
-    if (ctx->needs_input_grad(e_wp)) dwp = at::mm(dy.t(), view(m.y, m.M, m.C), at::kFloat);
-    auto colsum = [&](const void* x, int64_t cols) {
-      Tensor o = at::empty({cols}, buf.options().dtype(at::kFloat));
-      check(s3r_colsum(x, f32(o), m.M, cols, sp(a_col), col_bytes, st), "s3r_colsum");
-      return o;
-    };
-    if (ints[5] && ctx->needs_input_grad(e_wp + 1))          // the kernel reads rows of whole vectors
-      dbp = out_features % 8 == 0 ? colsum(dy.data_ptr(), out_features) : dy.sum(0, false, at::kFloat);
+    output_projection();
     // merge, the two branches, prologue
     check(s3r_merge_bwd_deltas(sp(a_dy), ptr(m.gate), m.H * m.N * 2, m.N * 2, 2, ptr(m.t(6)), ptr(m.o_s), sp(a_dos), sf(a_dgate),
                                sp(a_doc), sf(a_dels), sf(a_delc), m.B, m.H, m.N, m.d, m.block, st), "s3r_merge_bwd");
@@ -1027,7 +1047,7 @@ struct ModuleNode : torch::autograd::Function<ModuleNode> {
       dw_gate = dw.narrow(0, 3 * m.C, 2 * m.H);
     }
     if (ints[4] && (ctx->needs_input_grad(2) || ctx->needs_input_grad(e_gate + 1))) {
-      const Tensor db = colsum(sp(a_dproj), m.P);
+      const Tensor db = colsum(sp(a_dproj), m.P, sp(a_col), col_bytes);
       db_qkv = db.narrow(0, 0, 3 * m.C);
       db_gate = db.narrow(0, 3 * m.C, 2 * m.H);
     }
@@ -1096,6 +1116,11 @@ struct SparseNode : torch::autograd::Function<SparseNode> {
     const int64_t block = ctx->saved_data["block"].toInt();
     const double scale = ctx->saved_data["scale"].toDouble();
     if (!g[0].defined()) return variable_list(11);
+    if (!ctx->needs_input_grad(0) && !ctx->needs_input_grad(1) && !ctx->needs_input_grad(2)) {          // the gate alone
+      variable_list out(11);
+      out[3] = std::get<1>(call_merge_bwd(g[0].contiguous(), s[3], s[7], s[10], block)).to(s[3].scalar_type());
+      return out;
+    }
     if (plain(s[0]) && plain(g[0])) {
       c10::cuda::CUDAGuard guard(s[0].device());
       const Tensor& idx = s[9];

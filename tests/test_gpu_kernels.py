@@ -772,6 +772,40 @@ def test_module_gradients_with_a_graph_are_the_same_and_final():
             torch.autograd.grad(g.sum(), x, retain_graph=True)
 
 
+@pytest.mark.parametrize("wanted", [["proj.weight", "proj.bias"], ["proj.bias"], ["gate.0.bias"], ["k_norm.bias"], ["qkv.weight", "proj.weight"]])
+def test_module_backward_of_some_parameters(wanted):
+    """The gradients of single parameters are what they are among all; without one before the output projection, none of the
+    attention's backward runs (nor is its memory taken)."""
+    m, x, pos = module_and_input(0, N=4096)
+    dy = torch.randn(x.shape, device=DEV).bfloat16()
+    every = dict(zip(["x"] + [n for n, _ in m.named_parameters()], module_step(m, x.requires_grad_(True), pos, dy)[1:]))
+    x.requires_grad_(False)
+    for n, p in m.named_parameters():
+        p.requires_grad_(n in wanted)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = m(x, xpos=pos)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    got = torch.autograd.grad(y, [m.get_parameter(n) for n in wanted], dy)
+    peak = torch.cuda.max_memory_allocated() - held
+    assert all(torch.equal(a, every[n]) for n, a in zip(wanted, got))
+    tokens = x.numel() * 2                                         # bytes of one bf16 tensor of the sequence
+    assert (peak < 2 * tokens) == all(n.startswith("proj") for n in wanted), f"{peak / tokens:.1f} tensors of the sequence"
+
+
+def test_op_backward_of_the_gate_alone():
+    from speed3r_b200 import ops
+    B, H, T = 1, 2, 1024
+    q, k, v = (randn(s, B, H, T, 64).to(DEV, torch.bfloat16).requires_grad_(True) for s in (1, 2, 3))
+    gate = torch.sigmoid(randn(4, B, H, T, 2)).to(DEV, torch.bfloat16).requires_grad_(True)
+    y, _ = ops.sparse_attention_op(q, k, v, gate)
+    dy = torch.randn(y.shape, device=DEV).bfloat16()
+    want = torch.autograd.grad(y, gate, dy)[0]
+    y, _ = ops.sparse_attention_op(q.detach(), k.detach(), v.detach(), gate)
+    assert torch.equal(torch.autograd.grad(y, gate, dy)[0], want)
+
+
 # ------------------------------------------------------------------ host pipeline
 def test_host_pipeline_keeps_dropped_tensors_until_they_are_copied():
     """Pinned memory that the caller gives back while the copies are still enqueued is not handed out again."""
