@@ -443,6 +443,10 @@ __global__ void __launch_bounds__(256) prologue_bwd_reduce_kernel(const float* _
   if (lane == 0) out[o] = s;
 }
 
+// The kernels' limit of dynamic shared memory is set to the most a CTA can have, the same in every call: set to a call's own
+// need, two threads with blocks of different lengths could lower it for one another between setting and launching.
+constexpr int kProMaxSmem = 227 * 1024;
+
 static int prologue_parts(int H) { return (3 * H + kProRows - 1) / kProRows; }
 // CTAs along the blocks: four per SM over all parts
 static int prologue_bwd_ctas(int B, int Nc, int H) {
@@ -499,8 +503,8 @@ static int prologue_fwd(const void* qkv, int64_t tok_stride, const void* gate_in
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_qkv_prologue_fwd: could not resolve the device status word");
   const int smem = kProRingBytes + (kProThreads / 32) * 2 * (block + 1) * static_cast<int>(sizeof(int));
-  S3R_REQUIRE(smem <= 227 * 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_fwd: block %d is too long", block);
-  S3R_CUDA(cudaFuncSetAttribute(prologue_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  S3R_REQUIRE(smem <= kProMaxSmem, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_fwd: block %d is too long", block);
+  S3R_CUDA(cudaFuncSetAttribute(prologue_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
   return launch(prologue_fwd_kernel, dim3(static_cast<unsigned>(grid), prologue_parts(H)), kProThreads, smem,
                 static_cast<cudaStream_t>(stream), p);
 }
@@ -574,9 +578,9 @@ static int prologue_bwd(const void* qkv, int64_t tok_stride, const void* gate, c
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
   const int ctas = prologue_bwd_ctas(B, Nc, H), parts = prologue_parts(H);
   const int smem = kProBwdRingBytes + (kProThreads / 32) * 2 * (block + 1) * static_cast<int>(sizeof(int));
-  S3R_REQUIRE(smem <= 227 * 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_bwd: block %d is too long", block);
+  S3R_REQUIRE(smem <= kProMaxSmem, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_bwd: block %d is too long", block);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  S3R_CUDA(cudaFuncSetAttribute(prologue_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  S3R_CUDA(cudaFuncSetAttribute(prologue_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
   const int rc = launch(prologue_bwd_kernel, dim3(static_cast<unsigned>(ctas), parts), kProThreads, smem, st, p);
   if (rc || !dparams) return rc;
   return launch(prologue_bwd_reduce_kernel, 32, 256, 0, st, p.partial, dparams, ctas * parts);

@@ -53,3 +53,11 @@ def test_polynomial_exponential_is_as_exact_as_stated():
         r = (r * f + np.float64(c)).astype(np.float32).astype(np.float64)
     assert np.abs(exact / 2.0 ** f - 1).max() < 1.65e-7
     assert np.abs(r / 2.0 ** f - 1).max() < 2.25e-7
+
+
+def test_shared_memory_limits_do_not_depend_on_the_call():
+    """cudaFuncSetAttribute changes a kernel for every thread of the process: the limit is a constant, or the largest of all."""
+    for path in SOURCES:
+        for limit in re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*?)\)\)?;", code(path), flags=re.S):
+            names = set(re.findall(r"[A-Za-z_]\w*", limit)) - {"static_cast", "int", "sizeof", "int32_t"}
+            assert all(re.match(r"k[A-Z]|C$|AtCfg|TkCfg|R$", n) for n in names), f"{os.path.basename(path)}: {limit}"
