@@ -13,6 +13,7 @@
 #include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CachingHostAllocator.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
@@ -239,9 +240,22 @@ struct CsrBeside {
   c10::cuda::CUDAStream main, side;
   at::cuda::CUDAEvent done;
   bool joined = false;
+  // A stream of PyTorch's pool, which callers' streams come from as well: one that is in a capture which this work is not part
+  // of is left alone, and the work goes where it would without a second stream.
+  static c10::cuda::CUDAStream beside(const c10::cuda::CUDAStream& main) {
+    const auto side = c10::cuda::getStreamFromPool();
+    auto capture = [](const c10::cuda::CUDAStream& s) {      // 0: none
+      cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+      unsigned long long id = 0;
+      C10_CUDA_CHECK(cudaStreamGetCaptureInfo(s.stream(), &status, &id));
+      return status == cudaStreamCaptureStatusNone ? 0ull : id;
+    };
+    const auto theirs = capture(side);
+    return theirs != 0 && theirs != capture(main) ? main : side;
+  }
   CsrBeside(const int32_t* idx, int32_t* offsets, int32_t* qids, int64_t B, int64_t H, int64_t Nq, int64_t K, int64_t nkb, void* ws,
             size_t bytes)
-      : main(c10::cuda::getCurrentCUDAStream()), side(c10::cuda::getStreamFromPool()) {
+      : main(c10::cuda::getCurrentCUDAStream()), side(beside(main)) {
     at::cuda::CUDAEvent start;
     start.record(main);
     start.block(side);

@@ -677,6 +677,71 @@ def test_op_on_queries_and_keys_of_different_lengths(Tq, Tk, setting):
         assert_bf16_close(a.grad, b.grad, name)
 
 
+def test_backward_beside_a_capture_of_another_thread():
+    """The table's inverse runs on a stream of PyTorch's pool; a capture that another thread has going on one of those is neither
+    joined nor broken by it."""
+    import threading
+    from speed3r_b200 import ops
+    B, H, T = 1, 2, 512
+    q, k, v = (randn(s, B, H, T, 64).to(DEV, torch.bfloat16).requires_grad_(True) for s in (1, 2, 3))
+    gate = torch.sigmoid(randn(4, B, H, T, 2)).to(DEV, torch.bfloat16)
+    grads = lambda: torch.autograd.grad(ops.sparse_attention_op(q, k, v, gate)[0].float().sum(), (q, k, v))
+    want = grads()
+    torch.cuda.synchronize()
+    started, finish, failed = threading.Event(), threading.Event(), []
+    a = torch.ones(1024, device=DEV)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+
+    def capture():
+        try:
+            with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+                b = a + 1
+                started.set()
+                assert finish.wait(60)
+                b.add_(1)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert (b == 3).all()
+        except Exception as e:
+            failed.append(e)
+            started.set()
+
+    t = threading.Thread(target=capture)
+    t.start()
+    assert started.wait(60)
+    try:
+        got = [grads() for _ in range(40)]                         # the pool's 32 streams and more
+    finally:
+        finish.set()
+        t.join()
+    assert not failed, failed
+    assert all(torch.equal(x, y) for g in got for x, y in zip(g, want))
+
+
+def test_forward_and_backward_in_a_graph():
+    """A captured step of the op, with the second stream inside the capture, replayed on new inputs."""
+    from speed3r_b200 import ops
+    B, H, T = 2, 2, 1024
+    q, k, v = (randn(s, B, H, T, 64).to(DEV, torch.bfloat16).requires_grad_(True) for s in (1, 2, 3))
+    gate = torch.sigmoid(randn(4, B, H, T, 2)).to(DEV, torch.bfloat16).requires_grad_(True)
+    def step():
+        y, idx = ops.sparse_attention_op(q, k, v, gate)
+        return (y, idx) + torch.autograd.grad(y, (q, k, v, gate), torch.ones_like(y))
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step()
+    with torch.no_grad():
+        q.copy_(randn(5, B, H, T, 64))
+        k.copy_(randn(6, B, H, T, 64))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(out, step()))
+
+
 # ------------------------------------------------------------------ the attention module
 def module_and_input(seed, B=1, N=512, H=4, dim=None, **kw):
     import speed3r_b200
