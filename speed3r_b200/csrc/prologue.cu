@@ -60,25 +60,30 @@ __device__ __forceinline__ Vec8 ldg_vec8(const __nv_bfloat16* p) {
   const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
   return Vec8{{v.x, v.y, v.z, v.w}};
 }
-// Rows of the rotary tables for a block's tokens and, behind them, for its mean position: (y, x) pairs in this warp's shared
-// memory, clamped and checked once per warp instead of once per (q|k, head) row of every token.
+__device__ __forceinline__ int table_row(int64_t pv, int tab_rows) {
+  return static_cast<int>(min(max(pv, static_cast<int64_t>(0)), static_cast<int64_t>(tab_rows - 1)));
+}
+// Rows of the rotary tables for a block's mean position and, behind it, for its tokens: (y, x) pairs in this warp's shared
+// memory, clamped and checked once per warp instead of once per (q|k, head) row of every token.  LONG: a block whose rows do
+// not fit there; its tokens' rows are found where they are used.
+template <bool LONG>
 __device__ __forceinline__ void block_rows(int* r, const int64_t* pos, int block, int tab_rows, uint32_t* status, int lane) {
   bool bad = false;
   auto put = [&](int i, int64_t pv) {
-    const int row = static_cast<int>(min(max(pv, static_cast<int64_t>(0)), static_cast<int64_t>(tab_rows - 1)));
+    const int row = table_row(pv, tab_rows);
     bad |= pv != row;
-    r[i] = row;
+    if (!LONG || i < 2) r[i] = row;
   };
   float sum = 0.f;                                    // of the coordinate lane % 2: whole numbers, any order is exact
   for (int i = lane; i < 2 * block; i += 32) {
     const int64_t pv = __ldg(pos + i);
-    put(i, pv);
+    put(2 + i, pv);
     sum += static_cast<float>(pv);
   }
 #pragma unroll
   for (int d = 2; d < 32; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
   // float mean, truncated: xpos.view(..).float().mean(dim=2).int()
-  if (lane < 2) put(2 * block + lane, static_cast<int64_t>(static_cast<int>(sum / static_cast<float>(block))));
+  if (lane < 2) put(lane, static_cast<int64_t>(static_cast<int>(sum / static_cast<float>(block))));
   if (bad && status) atomicOr(status, kStatusBadIndex);     // clamped: the result for this token is wrong
   __syncwarp();
 }
@@ -134,6 +139,7 @@ __device__ __forceinline__ void rope_row(uint32_t (&xw)[4], const Vec8& c, const
 constexpr int kProRows = 16, kProThreads = kProRows * 8, kProChunk = 16, kProCtas = 6, kProBwdCtas = 4;
 constexpr int kProRingBytes = kProChunk * kProThreads * 16;
 
+template <bool LONG>
 __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(const PrologueParams p) {
   extern __shared__ __align__(16) uint8_t smem[];      // [token of the chunk][thread] 16 bytes; [warp] rows of the tables
   griddep_wait();
@@ -155,7 +161,7 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   const __nv_bfloat16* src = p.qkv + tok0 * p.tok_stride + g * 64 + l8 * 8;
   __nv_bfloat16* dst = out + (bh * p.N + n0) * 64 + l8 * 8;
   const uint32_t slots = smem_u32(smem) + threadIdx.x * 16;
-  int* rows = reinterpret_cast<int*>(smem + kProRingBytes) + (threadIdx.x >> 5) * 2 * (p.block + 1);
+  int* rows = reinterpret_cast<int*>(smem + kProRingBytes) + (threadIdx.x >> 5) * 2 * (LONG ? 1 : p.block + 1);
   // two groups of loads per chunk: the first half is worked on while the second arrives
   auto fetch = [&](int t0) {
 #pragma unroll
@@ -166,7 +172,7 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
     cp_async_commit();
   };
   fetch(0);
-  if (p.pos != nullptr) block_rows(rows, p.pos + tok0 * 2, p.block, p.tab_rows, p.status, lane);
+  if (p.pos != nullptr) block_rows<LONG>(rows, p.pos + tok0 * 2, p.block, p.tab_rows, p.status, lane);
   if (!live) return;
   float2 w[4], bias[4];
 #pragma unroll
@@ -176,13 +182,14 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   }
   const int* my_row = rows + (l8 >> 2);                // y for lanes 0-3, x for 4-7
   const __nv_bfloat16 *cos_l = p.cos_tab + (l8 & 3) * 8, *sin_l = p.sin_tab + (l8 & 3) * 8;
+  auto row_of = [&](int t) { return LONG ? table_row(__ldg(p.pos + (tok0 + t) * 2 + (l8 >> 2)), p.tab_rows) : my_row[2 + 2 * t]; };
 
   float2 acc[4] = {splat(0.f), splat(0.f), splat(0.f), splat(0.f)};
   // one token of this row: accumulate the raw block sum, normalise, rotate, store
   auto token = [&](int t, int slot) {
     Vec8 c, s, o = lds_vec8(slots + slot * (kProThreads * 16));
     if (rope) {
-      const int row = my_row[2 * t] * 32;
+      const int row = row_of(t) * 32;
       c = ldg_vec8(cos_l + row);
       s = ldg_vec8(sin_l + row);
     }
@@ -216,7 +223,7 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   if (norm) ln_row(x, w, bias, p.eps, gmask);
   Vec8 o = pack8(x);
   if (rope) {
-    const int row = my_row[2 * p.block] * 32;
+    const int row = my_row[0] * 32;
     rope_row(o.w, ldg_vec8(cos_l + row), ldg_vec8(sin_l + row), l8, gmask);
   }
   *reinterpret_cast<Vec8*>(out_c + (bh * p.Nc + j) * 64 + l8 * 8) = o;
@@ -305,6 +312,7 @@ __device__ __forceinline__ void ln_row_bwd(float2 (&x)[4], float2 (&dy)[4], cons
 constexpr int kProBwdAhead = 8;
 constexpr int kProBwdRingBytes = (kProChunk + kProBwdAhead) * kProThreads * 16;
 
+template <bool LONG>
 __global__ void __launch_bounds__(kProThreads, kProBwdCtas) prologue_bwd_kernel(const PrologueBwdParams p) {
   extern __shared__ __align__(16) uint8_t smem[];      // [token][thread] 16 bytes: projection, gradients; [warp] rows of the tables
   griddep_wait();
@@ -326,7 +334,7 @@ __global__ void __launch_bounds__(kProThreads, kProBwdCtas) prologue_bwd_kernel(
   }
   const float inv = 1.f / static_cast<float>(p.block);
   const uint32_t xs = smem_u32(smem) + threadIdx.x * 16, ds = xs + kProChunk * (kProThreads * 16);
-  int* rows = reinterpret_cast<int*>(smem + kProBwdRingBytes) + (threadIdx.x >> 5) * 2 * (p.block + 1);
+  int* rows = reinterpret_cast<int*>(smem + kProBwdRingBytes) + (threadIdx.x >> 5) * 2 * (LONG ? 1 : p.block + 1);
   const int* my_row = rows + (l8 >> 2);                // y for lanes 0-3, x for 4-7
   const __nv_bfloat16 *cos_l = p.cos_tab + (l8 & 3) * 8, *sin_l = p.sin_tab + (l8 & 3) * 8;
   const bool resident = p.block <= kProChunk;
@@ -350,13 +358,13 @@ __global__ void __launch_bounds__(kProThreads, kProBwdCtas) prologue_bwd_kernel(
       raw_c = ldg_vec8(dout_c + (bh * p.Nc + j) * 64 + l8 * 8);
     }
     __syncwarp();                                      // the previous block's rows have been used
-    if (p.pos != nullptr) block_rows(rows, p.pos + tok0 * 2, p.block, p.tab_rows, nullptr, lane);
+    if (p.pos != nullptr) block_rows<LONG>(rows, p.pos + tok0 * 2, p.block, p.tab_rows, nullptr, lane);
     if (live) {
       // the pooled branch's gradient of every token of the block
       float2 dc[4];
       unpack8(dc, raw_c);
       if (rope) {
-        const int row = my_row[2 * p.block] * 32;
+        const int row = my_row[0] * 32;
         rope_row_t(dc, ldg_vec8(cos_l + row), ldg_vec8(sin_l + row), l8, gmask);
       }
       cp_async_wait<kProBwdAhead>();
@@ -380,7 +388,7 @@ __global__ void __launch_bounds__(kProThreads, kProBwdCtas) prologue_bwd_kernel(
       for (int t = 0; t < p.block; ++t) {
         Vec8 c, s;
         if (rope) {
-          const int row = my_row[2 * t] * 32;
+          const int row = (LONG ? table_row(__ldg(p.pos + (tok0 + t) * 2 + (l8 >> 2)), p.tab_rows) : my_row[2 + 2 * t]) * 32;
           c = ldg_vec8(cos_l + row);
           s = ldg_vec8(sin_l + row);
         }
@@ -447,6 +455,13 @@ __global__ void __launch_bounds__(256) prologue_bwd_reduce_kernel(const float* _
 // need, two threads with blocks of different lengths could lower it for one another between setting and launching.
 constexpr int kProMaxSmem = 227 * 1024;
 
+// Shared memory of a CTA; `lengthy`: not even the rows of a block of that many tokens fit beside the slots (more than 5000: no
+// setting of the model, but the kernel takes any).
+static int prologue_smem(int ring, int block, bool* lengthy) {
+  const int64_t warps = kProThreads / 32, all = ring + warps * 2 * (static_cast<int64_t>(block) + 1) * static_cast<int64_t>(sizeof(int));
+  *lengthy = all > kProMaxSmem;
+  return *lengthy ? ring + static_cast<int>(warps * 2 * sizeof(int)) : static_cast<int>(all);
+}
 static int prologue_parts(int H) { return (3 * H + kProRows - 1) / kProRows; }
 // CTAs along the blocks: four per SM over all parts
 static int prologue_bwd_ctas(int B, int Nc, int H) {
@@ -502,10 +517,11 @@ static int prologue_fwd(const void* qkv, int64_t tok_stride, const void* gate_in
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_qkv_prologue_fwd: could not resolve the device status word");
-  const int smem = kProRingBytes + (kProThreads / 32) * 2 * (block + 1) * static_cast<int>(sizeof(int));
-  S3R_REQUIRE(smem <= kProMaxSmem, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_fwd: block %d is too long", block);
-  S3R_CUDA(cudaFuncSetAttribute(prologue_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
-  return launch(prologue_fwd_kernel, dim3(static_cast<unsigned>(grid), prologue_parts(H)), kProThreads, smem,
+  bool lengthy;
+  const int smem = prologue_smem(kProRingBytes, block, &lengthy);
+  auto* kernel = lengthy ? prologue_fwd_kernel<true> : prologue_fwd_kernel<false>;
+  S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
+  return launch(kernel, dim3(static_cast<unsigned>(grid), prologue_parts(H)), kProThreads, smem,
                 static_cast<cudaStream_t>(stream), p);
 }
 
@@ -577,11 +593,12 @@ static int prologue_bwd(const void* qkv, int64_t tok_stride, const void* gate, c
   p.partial = dparams ? static_cast<float*>(workspace) : nullptr;
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
   const int ctas = prologue_bwd_ctas(B, Nc, H), parts = prologue_parts(H);
-  const int smem = kProBwdRingBytes + (kProThreads / 32) * 2 * (block + 1) * static_cast<int>(sizeof(int));
-  S3R_REQUIRE(smem <= kProMaxSmem, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_bwd: block %d is too long", block);
+  bool lengthy;
+  const int smem = prologue_smem(kProBwdRingBytes, block, &lengthy);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  S3R_CUDA(cudaFuncSetAttribute(prologue_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
-  const int rc = launch(prologue_bwd_kernel, dim3(static_cast<unsigned>(ctas), parts), kProThreads, smem, st, p);
+  auto* kernel = lengthy ? prologue_bwd_kernel<true> : prologue_bwd_kernel<false>;
+  S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
+  const int rc = launch(kernel, dim3(static_cast<unsigned>(ctas), parts), kProThreads, smem, st, p);
   if (rc || !dparams) return rc;
   return launch(prologue_bwd_reduce_kernel, 32, 256, 0, st, p.partial, dparams, ctas * parts);
 }

@@ -653,6 +653,22 @@ def test_cmp_backward_with_all_logits_far_below_zero(Nc):
         assert_bf16_close(a.grad, b.grad, name)
 
 
+def test_prologue_of_blocks_whose_table_rows_do_not_fit_shared_memory():
+    """Blocks of 6400 tokens: token rows as with blocks of 16, bit for bit, means as in fp32, and the backward."""
+    import speed3r_b200
+    from speed3r_b200 import ops
+    B, H, N, Bs = 1, 2, 12800, 6400
+    qkv = (1.5 * randn(1, B, N, 3 * H * 64) + 0.3).to(DEV, torch.bfloat16)
+    pos = torch.randint(0, 37, (B, N, 2), generator=torch.Generator().manual_seed(2)).to(DEV)
+    cos, sin = speed3r_b200.RoPE2D(100.0)._cos_sin(32, 37, torch.device(DEV), torch.bfloat16)
+    norm = [(1 + 0.2 * randn(3 + i, 64).to(DEV), 0.1 * randn(5 + i, 64).to(DEV), 1e-5) for i in range(2)]
+    long, short = (ops.qkv_prologue(qkv, H, b, pos, cos, sin, *norm) for b in (Bs, 16))
+    assert all(torch.equal(a, b) for a, b in zip(long[:3], short[:3]))
+    mean = qkv.view(B, N // Bs, Bs, 3, H, 64).float().mean(2).permute(2, 0, 3, 1, 4)
+    assert_bf16_close(long[5], mean[2], "v_c")
+    test_prologue_backward(B, H, Bs, N // Bs, True, True)
+
+
 @pytest.mark.parametrize("Tq, Tk, setting", [(512, 1024, (16, 32, 16, 16)), (1040, 336, (16, 8, 16, 16)), (256, 1024, (64, 4, 32, 16))])
 def test_op_on_queries_and_keys_of_different_lengths(Tq, Tk, setting):
     """The whole op, forward and backward, where queries attend to another sequence."""
