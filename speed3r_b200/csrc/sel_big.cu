@@ -157,7 +157,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       int issued = 0;
       if (steps > 0 && lane == 0) {
         mbar_expect_tx(&ctl.q_full, kSbgTile);
-        tma_load_4d_u32(sbase, &map_q, &ctl.q_full, 0, qb0 * BS, bh, 0);
+        tma_load_4d(sbase, &map_q, &ctl.q_full, 0, qb0 * BS, bh, 0);
       }
       const int nv = lane < G ? ctl.nvalid[lane] : 0;
       for (int j = 0; j < steps; ++j) {
@@ -171,12 +171,12 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (!mbar_wait_warp(&ctl.k_empty[s], ph ^ 1, abort_flag)) break;
         if (lane == 0) mbar_expect_tx(&ctl.k_full[s], kSbgTile);
         __syncwarp();
-        if (lane < G) tma_load_4d_u32(sbase + kSbgOffK + s * kSbgTile + lane * BS * 128, &map_k, &ctl.k_full[s], 0, tok, bh, ch);
+        if (lane < G) tma_load_4d(sbase + kSbgOffK + s * kSbgTile + lane * BS * 128, &map_k, &ctl.k_full[s], 0, tok, bh, ch);
         issued = j + 1;                                                   // K of step j is in flight
         if (!mbar_wait_warp(&ctl.v_empty[s], ph ^ 1, abort_flag)) break;
         if (lane == 0) mbar_expect_tx(&ctl.v_full[s], kSbgTile);
         __syncwarp();
-        if (lane < G) tma_load_4d_u32(sbase + kSbgOffV + s * kSbgTile + lane * BS * 128, &map_v, &ctl.v_full[s], 0, tok, bh, ch);
+        if (lane < G) tma_load_4d(sbase + kSbgOffV + s * kSbgTile + lane * BS * 128, &map_v, &ctl.v_full[s], 0, tok, bh, ch);
       }
       if (*abort_flag) {
         // give copies already in flight a bounded chance to land before the CTA's memory is released
