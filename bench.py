@@ -757,21 +757,10 @@ def main():
                 "pool_gbs": pool_bytes / t_pool / 1e6, "pool_frac_hbm": pool_bytes / t_pool / 1e6 / peaks["hbm_gbs"],
                 "cmp_tflops": f_cmp / t_cmp / 1e9, "sel_gather_gbs": sel_bytes / t_sel / 1e6,
                 "sel_tflops": f_sel / t_sel / 1e9}
-        # the gather figure counts every selected block as if it came from DRAM; L2 serves part of it.  DRAM
-        # traffic of this kernel measured with ncu on this workload (one-pass capture of one launch):
-        # 64.21 GB read + 2.07 GB written per launch at 1000 views (not proportional to views: L2 hit rate changes)
-        if args.views == 1000:
-            kern["sel_dram_gbs"] = 66.27e9 / t_sel / 1e6
-            kern["sel_frac_hbm"] = kern["sel_dram_gbs"] / peaks["hbm_gbs"]
+        # the gather figure counts every selected block as if it came from DRAM; L2 serves part of it
         ach = f_cmp / t_cmp / 1e9
-        # DRAM traffic of one launch: an ncu capture of a one-pass version of the kernel on this workload
-        # (1000 views: dram__bytes_read.sum 392.4 MB + dram__bytes_write.sum 235.1 MB).  It equals the
-        # algorithmic bytes (pooled q,k,v read once: 387 MB; o_c, lse and the table written once: 262 MB) and
-        # grows with views.  The collection of the columns reads q and k once more, mostly from L2.
-        traffic = 627.5e6 * (args.views / 1000.0)
         roof = {"kernel": "cmp_both_kernel (compression attention + top-k)", "bound": "tensor", "achieved": ach,
-                "peak": peaks["tflops"], "unit": "TFLOP/s", "frac": ach / peaks["tflops"], "traffic": traffic,
-                "traffic_unit": "bytes/launch (ncu dram read+write of a 1000-view capture, = the algorithmic bytes, scaled by views)",
+                "peak": peaks["tflops"], "unit": "TFLOP/s", "frac": ach / peaks["tflops"], "traffic": None,
                 "peak_source": f"{peaks['src']} sustained bf16 (kernel timed inside a long step)"}
 
     # end to end through the public op functions with HOST buffers (pinned), copies inside the timing

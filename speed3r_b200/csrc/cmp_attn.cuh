@@ -35,7 +35,8 @@
 // The exponent offset of a row is the maximum of its first tile and does not move: P, O and l are floats, which keep their
 // relative precision however far later scores outgrow the first tile's, up to their range.  A CTA in which some row's
 // scores outgrew its offset by more than 2^64 takes its keys a second time with the rows' exact maxima, which the group
-// maxima have found by then.  No maximum, vote or branch stands between one exponential and the next (a check per tile, with
+// maxima have found by then (rows beside such a row are then rounded from other offsets than in a launch that groups rows
+// otherwise: results do not depend on the grouping only while no row is).  No maximum, vote or branch stands between one exponential and the next (a check per tile, with
 // the tile redone: 2.90 ms; a check per 32 columns, with P rescaled: 3.40 ms).
 #pragma once
 #include <type_traits>

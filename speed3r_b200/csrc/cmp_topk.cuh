@@ -44,7 +44,11 @@ struct TkCfg {
   static constexpr int kOffK = R * kTkTile, kOffBuf = kOffK + kTkStages * kTkTile;
   static constexpr int kSmem = kOffBuf + 2 * kRows * kTkCap * 8 + 1024;
 };
-constexpr int kTkSplitTiles = 16;              // with fewer tiles the two scans of a row take halves of every tile, not turns
+// With fewer tiles the two scans of a row take halves of every tile, not turns: with an odd or small number of tiles one of
+// them would have more.  Both kernels, 16 heads, halves against turns: 384 x 896 (7 tiles) 43.6 and 45.0 us, 4096 x 1900 (15)
+// 143.5 and 146.2, 1512 x 1512 (12) 70.4 and 70.9; beyond the line 4096 x 4096 (32) 218.8 and 221.4, 6300 x 6300 (50) 445.3 and
+// 451.5, so that the line could lie higher; longer ones were not measured.
+constexpr int kTkSplitTiles = 16;
 
 struct TkCtl {
   uint64_t q_full, drained;

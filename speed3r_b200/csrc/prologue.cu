@@ -482,7 +482,7 @@ static int prologue_fwd(const void* qkv, int64_t tok_stride, const void* gate_in
               "s3r_qkv_prologue_fwd: sizes must be positive (B=%d H=%d N=%d block=%d)", B, H, N, block);
   S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_fwd: head_dim %d not supported (64 only)", d);
   S3R_REQUIRE(N % block == 0, S3R_ERR_SHAPE, "s3r_qkv_prologue_fwd: N=%d is not a multiple of the block %d", N, block);
-  S3R_REQUIRE(3 * H * 8 <= 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_fwd: %d heads exceed one CTA (42 at most)", H);
+  S3R_REQUIRE(3 * H * 8 <= 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_fwd: %d heads not supported (42 at most)", H);
   S3R_REQUIRE((q_weight != nullptr) == (q_bias != nullptr) && (k_weight != nullptr) == (k_bias != nullptr) &&
                   (q_weight != nullptr) == (k_weight != nullptr),
               S3R_ERR_NULL, "s3r_qkv_prologue_fwd: LayerNorm weights and biases of q and k come together or not at all");
@@ -559,7 +559,7 @@ static int prologue_bwd(const void* qkv, int64_t tok_stride, const void* gate, c
               "s3r_qkv_prologue_bwd: sizes must be positive (B=%d H=%d N=%d block=%d)", B, H, N, block);
   S3R_REQUIRE(d == 64, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_bwd: head_dim %d not supported (64 only)", d);
   S3R_REQUIRE(N % block == 0, S3R_ERR_SHAPE, "s3r_qkv_prologue_bwd: N=%d is not a multiple of the block %d", N, block);
-  S3R_REQUIRE(3 * H * 8 <= 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_bwd: %d heads exceed one CTA (42 at most)", H);
+  S3R_REQUIRE(3 * H * 8 <= 1024, S3R_ERR_UNSUPPORTED, "s3r_qkv_prologue_bwd: %d heads not supported (42 at most)", H);
   S3R_REQUIRE((q_weight != nullptr) == (k_weight != nullptr) && (q_weight != nullptr) == (dparams != nullptr), S3R_ERR_NULL,
               "s3r_qkv_prologue_bwd: LayerNorm weights of q and k and their gradients come together or not at all");
   S3R_REQUIRE(pos == nullptr || (cos_tab && sin_tab && tab_rows > 0), S3R_ERR_NULL,

@@ -5,8 +5,9 @@
 // which the diagonal ones are wanted: block g's queries against its own key block.  The softmax threads read those alone; P
 // is written over the diagonal blocks of a zeroed tile, so that O += P V (K=128) adds the right keys to each row.  The
 // G - 1 unwanted blocks beside each wanted one are cheaper than mma.sync without them: 16 heads, top-16 blocks of 64 at 250
-// views 3.86 -> 2.40 ms, 64 views 1002 -> 555 us; top-32 blocks of 32, 60000 tokens 1073 -> 818 us.
-// Bound: latency, with no unit more than half busy.  Of a CTA's 18.5 us at 64500 tokens, top-16, 2.4 pass until its first S is
+// views 3.86 -> 2.51 ms, 64 views 1002 -> 585 us; top-32 blocks of 32, 60000 tokens 1073 -> 964 us.
+// Bound: latency, with no unit more than half busy.  Of a CTA's 18.5 us at 64500 tokens, top-16 (with fixed offsets, below), 2.4
+// pass until its first S is
 // there, 13 in 16 steps (0.8 us each beside another CTA, 80 KB of shared-memory traffic) and 3 at its end; 2.5 more until
 // the next CTA runs in its place.  The merge's operands are loaded before the last product is waited for (1.6 us less at the
 // end, 2 to 4 % of the whole).  Two threads per row instead of one changed nothing; several row tiles per CTA without a barrier
@@ -15,8 +16,8 @@
 // Two CTAs per SM: their steps fill each other's waits.
 // The exponent offset of a row is its running maximum, step by step (O is rescaled in tensor memory where a row of the warp
 // moved): the row's largest weights are 1 and lose nothing when P is rounded to bf16.  Offsets fixed by the first step saved
-// the rescaling but rounded those weights: error against 64 bits 2.33e-3 instead of 2.24e-3 at unit-scale logits, 2.28e-3
-// instead of 1.64e-3 where a few keys hold a row's weight.
+// the rescaling (64 views 544 instead of 585 us, 250 views 2.42 instead of 2.51 ms) but rounded those weights: error against
+// 64 bits 2.33e-3 instead of 2.24e-3 at unit-scale logits, 2.28e-3 instead of 1.64e-3 where a few keys hold a row's weight.
 // Zero times a value that is not finite is NaN, so one such value among a query block's keys reaches every row of the tile
 // through O += P V.  A row with finite scores and an O that is not is therefore done again from its own keys alone, by its
 // thread and out of line: taking the tile's lists one by one with the tensor cores instead needed the row's state in

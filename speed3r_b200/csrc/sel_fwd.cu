@@ -24,9 +24,12 @@ namespace s3r {
 //     rounding: error against 64 bits 2.33e-3 instead of 2.20e-3 at unit-scale logits, 2.20e-3 instead of 1.62e-3 where a
 //     few keys hold a row's weight.
 //   * CTAs of one warp: nothing is shared between query blocks, and a finished warp makes room at once.
-// Bound: a bare TMA gather of the same blocks runs at 20 TB/s while a head's K and V fit L2 and at 10.5 TB/s at
-// 1000 views (258 MB per head).  Measured (H = 16, top-32, uniformly random blocks): 64 views 822 -> 532 us =
-// 15.9 TB/s gathered, 2048 tokens 46 -> 27 us, 250 views 3.16 -> 2.22 ms, 1000 views 14.9 -> 13.8 ms (9.6 TB/s).
+// Bound: the gather, and the latency of a pair's chain of products, maxima and exponentials that twelve warps per SM do not
+// cover.  H = 16, top-32, uniformly random blocks; this kernel without its arithmetic in brackets: 2048 tokens 28.9 us (21.5),
+// 64 views 548 us = 15.4 TB/s gathered (415, 20.4 TB/s), 100 views 852 (648), 250 views 2.16 ms (1.66), 1000 views, where a
+// head's 258 MB of keys and values miss L2, 14.5 ms = 9.1 TB/s (13.6, 9.7 TB/s).  The op's own tables favour some blocks (with
+// independent inputs a tenth of them has a third of the picks): at 1000 views 12.4 ms = 10.7 TB/s (10.4, 12.7 TB/s).  Offsets
+// fixed by the first pair: 26.2 us, 492 us, 765 us, 1.96 ms, 14.4 ms.
 // Gathering straight into fragments with 16-byte loads instead (no shared memory) ran at 8.7 TB/s: a fragment load
 // touches 8 rows, and L1 serves few lines per cycle.
 struct Sel16Params {

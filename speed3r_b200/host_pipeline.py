@@ -18,7 +18,9 @@ The query chunk is sized so that one compression-attention launch fills whole wa
 (`Hg * ceil(rows/256)` CTAs a multiple of the SM count).  The last group's chunks are a quarter of the sequence at most:
 what follows the last byte in is one chunk's kernels and its copy out, and nothing else hides them (64512 tokens, 16
 heads: 8.55 -> 8.03 ms, of which 7.7 for the copies in).  Results are bit-identical to the unchunked
-call: every query row sees the same keys in the same order.
+call: every query row sees the same keys in the same order.  One thing couples rows: where some row's compressed logits
+outgrow its first 128 keys' by more than 2^64, all rows of its 128 or 256 take their exact maxima as exponent offsets, and
+chunks group rows differently; such rows, which normalised queries and keys do not have, may round differently.
 """
 from __future__ import annotations
 
