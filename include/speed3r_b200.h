@@ -244,7 +244,8 @@ int s3r_build_key_csr_static(const int32_t* idx, int32_t* offsets, int32_t* qids
  *   do_s  [B,H,Tq,d] bf16 = g1 * dy
  *   dgate [B,H,Tq,2] fp32 : dg0 = sum_d dy*o_c[t/block], dg1 = sum_d dy*o_s
  *   do_c  [B,H,ceil(Tq/block),d] bf16 = sum over the block's tokens of g0 * dy
- *   delta_s [B,H,Tq] fp32 = sum_d o_s*do_s = g1*dg1 */
+ *   delta_s [B,H,Tq] fp32 = sum_d o_s*do_s = g1*dg1
+ * dy, o_c, o_s, do_s and do_c 16-byte aligned, gate pairs 4-byte, dgate 8-byte. */
 int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
                   int64_t gate_stride_t, const void* o_c, const void* o_s, void* do_s, float* dgate,
                   void* do_c, float* delta_s, int B, int H, int Tq, int d, int block, void* stream);
@@ -254,7 +255,7 @@ int s3r_merge_bwd_deltas(const void* dy, const void* gate, int64_t gate_stride_b
                          float* delta_s, float* delta_c, int B, int H, int Tq, int d, int block, void* stream);
 
 /* Row-wise delta = sum_d o*do for [rows,d] bf16 tensors (backward_sum_o_do,
- * topk_blocksparse_attention.py:132-170); used when the merge is not fused. */
+ * topk_blocksparse_attention.py:132-170); used when the merge is not fused.  o and d_o 16-byte aligned. */
 int s3r_delta(const void* o, const void* d_o, float* delta, int64_t rows, int d, void* stream);
 
 /* Backward of the selection attention.  Replaces TopkBlockSparseAttention.backward /

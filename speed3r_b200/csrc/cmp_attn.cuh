@@ -6,8 +6,9 @@
 // the top-k has to look at every score once but keeps 32 of tens of thousands, through branches that depend on the
 // data.  Side by side in one kernel (softmax warps and top-k warps reading the same scores) each waited for the other
 // tile by tile; the products, which the second kernel repeats, are cheap: the tensor pipe was a fifth busy.
-// Measured (16 heads, one kernel before -> this one + cmp_topk.cuh): 384 x 384 99 -> 9 + 23 us, 6300 x 6300 1047 ->
-// 223 + 244 us (scores that cluster by view and patch: 1923 -> 222 + 315), 7875 x 63000 5.81 -> 2.45 + 1.69 ms.
+// Measured (16 heads, one kernel before -> this one + cmp_topk.cuh): 6300 x 6300 1047 ->
+// 223 + 244 us (scores that cluster by view and patch: 1923 -> 222 + 315), 7875 x 63000 5.81 -> 2.45 + 1.69 ms; both kernels
+// 384 x 384 99 -> 19 to 34 us, depending on the inputs.
 //
 // The bound: a row keeps the running maxima of 64 groups of columns (half of S, piece of 16 in it and column mod 8).  topk of
 // the maxima are >= the topk-th largest of the maxima, so at least topk logits are, and the topk-th largest logit is.  With
