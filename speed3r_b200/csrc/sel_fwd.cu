@@ -23,13 +23,19 @@ namespace s3r {
 //     when P is rounded to bf16.  An offset fixed by the first pair saved the maxima and their shuffles, but not the
 //     rounding: error against 64 bits 2.33e-3 instead of 2.20e-3 at unit-scale logits, 2.20e-3 instead of 1.62e-3 where a
 //     few keys hold a row's weight.
+//   * O and l are rescaled with every pair, whether a row moved or not: among 16 rows one nearly always does (two in three
+//     warps still do at the last pair), and the vote and the branch stood in the chain (64 views 536 -> 510 us).
+//   * The thread that asks for copies is elected, so that the compiler knows it is one and coordinates need no loop over lanes
+//     (548 -> 533 us); the list's entries are read where they are used (read a pair ahead 548 -> 568 us).
 //   * CTAs of one warp: nothing is shared between query blocks, and a finished warp makes room at once.
-// Bound: the gather, and the latency of a pair's chain of products, maxima and exponentials that twelve warps per SM do not
-// cover.  H = 16, top-32, uniformly random blocks; this kernel without its arithmetic in brackets: 2048 tokens 28.9 us (21.5),
-// 64 views 548 us = 15.4 TB/s gathered (415, 20.4 TB/s), 100 views 852 (648), 250 views 2.16 ms (1.66), 1000 views, where a
-// head's 258 MB of keys and values miss L2, 14.5 ms = 9.1 TB/s (13.6, 9.7 TB/s).  The op's own tables favour some blocks (with
-// independent inputs a tenth of them has a third of the picks): at 1000 views 12.4 ms = 10.7 TB/s (10.4, 12.7 TB/s).  Offsets
-// fixed by the first pair: 26.2 us, 492 us, 765 us, 1.96 ms, 14.4 ms.
+// Bound: the gather and shared memory (4 KB of a pair of blocks written and read again: 64 of 68 cycles per SM).  H = 16, top-32,
+// uniformly random blocks; before the last two points, and this kernel without its arithmetic, in brackets: 2048 tokens 26.2 us
+// (28.1, 21.5), 64 views 509 us = 16.6 TB/s gathered (548; 415, 20.4 TB/s), 100 views 791 (852, 648), 250 views 2.07 ms (2.16,
+// 1.66), 1000 views, where a head's 258 MB of keys and values miss L2, 13.9 ms = 9.5 TB/s (14.0; 13.6, 9.7 TB/s).  The op's own
+// tables favour some blocks (with independent inputs a tenth of them has a third of the picks): at 1000 views 11.2 ms.
+// Slots of single blocks in a ring of three, which let 15 warps instead of 12 onto an SM, lost more to a second wait per pair
+// (64 views 592 us; 2048 tokens 25.2); refilling a slot before the products instead of after them changed nothing (lop3 of the
+// fragments or a proxy fence in front: 600 and 612 us).
 // Gathering straight into fragments with 16-byte loads instead (no shared memory) ran at 8.7 TB/s: a fragment load
 // touches 8 rows, and L1 serves few lines per cycle.
 struct Sel16Params {
@@ -85,10 +91,10 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
   // an odd list ends with its last block twice; the second copy's scores are masked
   if ((nvalid & 1) && lane == 0) list[nvalid] = list[nvalid - 1];
   __syncwarp();
-  const bool chunked = p.Tc != p.Tk;
+  const bool chunked = p.Tc != p.Tk, leader = elect_one_sync();
   // a block's keys and its values together
   auto issue = [&](int pair, int s) {
-    if (lane == 0) {
+    if (leader) {
       const int2 t = *reinterpret_cast<const int2*>(list + 2 * pair);
       int t0 = t.x, t1 = t.y, c0 = 0, c1 = 0;
       if (chunked) {
@@ -135,7 +141,7 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
 #pragma unroll 1
   for (int it = 0; it < npairs; ++it) {
     const int S = it & 1;
-    if (!mbar_wait_warp(&full[S], (it >> 1) & 1, abort_flag)) {
+    if (!__all_sync(0xffffffffu, mbar_try_wait(&full[S], (it >> 1) & 1)) && !mbar_wait_warp(&full[S], (it >> 1) & 1, abort_flag)) {
       volatile uint32_t dummy = 0;               // a last bounded chance for the other stage's copies to land
       if (it + 1 < npairs) mbar_wait(&full[S ^ 1], ((it + 1) >> 1) & 1, &dummy);
       if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
@@ -179,7 +185,7 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
             if (t * 8 + 2 * c + (e & 1) >= left) s[j][t][e] = -INFINITY;
       }
     }
-    // the offsets follow the running maxima; O and l only when one of the warp's rows moved
+    // the offsets follow the running maxima
     float mn[2], neg[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -190,14 +196,16 @@ __global__ void __launch_bounds__(32, 12) sel16_fwd_kernel(const __grid_constant
       mn[r] = fmaxf(m_used[r], m * cs);                               // scale > 0 keeps the order
       neg[r] = mn[r] == -INFINITY ? 0.f : -mn[r];                     // no finite score yet: P = 0
     }
-    if (__any_sync(0xffffffffu, mn[0] != m_used[0] || mn[1] != m_used[1])) {
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const float alpha = fast_exp2(m_used[r] + neg[r]);
-        m_used[r] = mn[r];
-        l[r] *= alpha;
+    for (int r = 0; r < 2; ++r) {
+      const float alpha = fast_exp2(m_used[r] + neg[r]);               // 1 where the row did not move
+      m_used[r] = mn[r];
+      l[r] *= alpha;
 #pragma unroll
-        for (int dt = 0; dt < 8; ++dt) { o[dt][2 * r] *= alpha; o[dt][2 * r + 1] *= alpha; }
+      for (int dt = 0; dt < 8; ++dt) {
+        const float2 x = fmul2(make_float2(o[dt][2 * r], o[dt][2 * r + 1]), make_float2(alpha, alpha));
+        o[dt][2 * r] = x.x;
+        o[dt][2 * r + 1] = x.y;
       }
     }
     uint32_t pk[2][4];
