@@ -432,6 +432,9 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
 // second tile's loads run under the first tile's exponentials (919 -> 638 us at 64 views, H = 16, top-32); the same
 // order in the dK/dV kernel needs more registers than it gains: with the tiles one after the other 1161 -> 937 us, with
 // eight or nine warps and the tiles overlapped 1110 us.
+// Packed pairs in the exponentials' arithmetic, an elected thread that asks for copies and a wait whose usual outcome is one vote:
+// both parts 1650 -> 1621 us at 64 views, 6350 -> 6255 at 250.  Turning fragments in registers (movmatrix) instead of reading
+// them a second time: dQ the same (1627), dK/dV slower (1697), so that shared memory is not what is missing.
 struct SelBwdParams {
   const __nv_bfloat16 *q, *k, *v, *d_o;
   const int32_t *idx, *offsets, *qids;
@@ -571,8 +574,9 @@ __device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdPa
   }
   const int ntiles = nvalid << p.block_shift, npairs = (ntiles + 1) >> 1, in_block = (1 << p.block_shift) - 1;
   auto tok_of = [&](int t) { return list[t >> p.block_shift] + ((t & in_block) << 4); };
+  const bool leader = elect_one_sync();
   auto issue = [&](int pair, int s) {
-    if (lane == 0) {
+    if (leader) {
       const int t = 2 * pair;
       mbar_expect_tx(&sh.full[s], (t + 1 < ntiles ? 8192u : 4096u) >> (map_kv.b_first < 0));
       tma_load_pair<APART>(ring + s * kSbStageBytes, map_kv, &sh.full[s], tok_of(t), bh, 0);
@@ -585,12 +589,13 @@ __device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdPa
   uint32_t qf[4][4], dof[4][4];
   ldg_a_frags(qf, p.q + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, nrows, lane);
   ldg_a_frags(dof, p.d_o + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, nrows, lane);
-  float lse2[2], delta[2];
+  float neg_lse2[2], neg_delta[2];
+  const float2 cs2 = make_float2(p.cs, p.cs);
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int64_t t = static_cast<int64_t>(bh) * p.Tq + row0 + min(g + 8 * r, nrows - 1);
-    lse2[r] = p.lse[t] * 1.4426950408889634f;         // finite wherever the list is not empty
-    delta[r] = p.delta[t];
+    neg_lse2[r] = p.lse[t] * -1.4426950408889634f;         // finite wherever the list is not empty
+    neg_delta[r] = -p.delta[t];
   }
   const SbLane of(lane);
   const uint32_t k_at = map_kv.b_first > 0 ? 2048u : 0u, v_at = map_kv.b_first == 0 ? 2048u : 0u;
@@ -600,7 +605,7 @@ __device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdPa
 #pragma unroll 1
   for (int it = 0; it < npairs; ++it, ++taken) {
     const int S = taken & 1;
-    if (!mbar_wait_warp(&sh.full[S], (taken >> 1) & 1, abort_flag)) {
+    if (!__all_sync(0xffffffffu, mbar_try_wait(&sh.full[S], (taken >> 1) & 1)) && !mbar_wait_warp(&sh.full[S], (taken >> 1) & 1, abort_flag)) {
       volatile uint32_t dummy = 0;                    // a last bounded chance for the other stage's copies to land
       if (it + 1 < npairs) mbar_wait(&sh.full[S ^ 1], ((taken + 1) >> 1) & 1, &dummy);
       if (lane == 0) atomicOr(p.status, kStatusWaitTimeout);
@@ -615,10 +620,15 @@ __device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdPa
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float pr = fast_exp2(fmaf(s[nt][e], p.cs, -lse2[e >> 1]));
-          if (ragged && nt * 8 + 2 * c + (e & 1) >= left) pr = 0.f;
-          s[nt][e] = pr * (dp[nt][e] - delta[e >> 1]);
+        for (int r = 0; r < 2; ++r) {
+          float2 pr = ffma2(make_float2(s[nt][2 * r], s[nt][2 * r + 1]), cs2, make_float2(neg_lse2[r], neg_lse2[r]));
+          pr.x = fast_exp2(pr.x);
+          pr.y = fast_exp2(pr.y);
+          if (ragged && nt * 8 + 2 * c >= left) pr.x = 0.f;
+          if (ragged && nt * 8 + 2 * c + 1 >= left) pr.y = 0.f;
+          const float2 ds = fmul2(pr, fadd2(make_float2(dp[nt][2 * r], dp[nt][2 * r + 1]), make_float2(neg_delta[r], neg_delta[r])));
+          s[nt][2 * r] = ds.x;
+          s[nt][2 * r + 1] = ds.y;
         }
       a[0] = pack_bf16(s[0][0], s[0][1]); a[1] = pack_bf16(s[0][2], s[0][3]);
       a[2] = pack_bf16(s[1][0], s[1][1]); a[3] = pack_bf16(s[1][2], s[1][3]);
@@ -701,8 +711,9 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
     }
     return (__shfl_sync(0xffffffffu, q_cur, e & 31) << (4 + p.block_shift)) + ((t & in_block) << 4);
   };
+  const bool leader = elect_one_sync();
   auto issue = [&](int t0, int t1, bool both, int s) {
-    if (lane == 0) {
+    if (leader) {
       mbar_expect_tx(&sh.full[s], (both ? 8192u : 4096u) >> (map_qdo.b_first < 0));
       tma_load_pair<APART>(ring + s * kSbStageBytes, map_qdo, &sh.full[s], t0, bh, 0);
       if (both) tma_load_pair<APART>(ring + s * kSbStageBytes + 4096, map_qdo, &sh.full[s], t1, bh, 0);
@@ -712,7 +723,7 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
   auto stat = [&](int tok0) {
     const int t = tok0 + (lane & 15);
     const float x = __ldg((lane < 16 ? p.lse : p.delta) + static_cast<int64_t>(bh) * p.Tq + min(t, p.Tq - 1));
-    return lane >= 16 ? x : (t < p.Tq ? x * 1.4426950408889634f : INFINITY);
+    return lane >= 16 ? -x : (t < p.Tq ? x * -1.4426950408889634f : -INFINITY);
   };
   auto offsets_of = [&](uint32_t task) {
     const uint32_t h = task / nslices, slice = task - h * nslices;
@@ -794,7 +805,7 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
       sh.stats[1][lane] = sb;
       __syncwarp();
       if (it + 1 < npairs) { sa = stat(ta); sb = stat(tb); }
-      ok = ok && mbar_wait_warp(&sh.full[S], (taken >> 1) & 1, abort_flag);
+      ok = ok && (__all_sync(0xffffffffu, mbar_try_wait(&sh.full[S], (taken >> 1) & 1)) || mbar_wait_warp(&sh.full[S], (taken >> 1) & 1, abort_flag));
       if (!ok) {
         volatile uint32_t dummy = 0;                    // a last bounded chance for what is under way to land
         if (it + 1 < npairs) mbar_wait(&sh.full[S ^ 1], ((taken + 1) >> 1) & 1, &dummy);
@@ -804,19 +815,20 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
       }
       const uint32_t st = ring + S * kSbStageBytes;
       // P^T and dS^T of a tile, packed as A operands
-      auto grad = [&](float (&s)[2][4], const float (&dp)[2][4], int j, uint32_t (&pa)[4], uint32_t (&da)[4]) {
+      auto grad = [&](const float (&s)[2][4], const float (&dp)[2][4], int j, uint32_t (&pa)[4], uint32_t (&da)[4]) {
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float2 l2 = *reinterpret_cast<const float2*>(&sh.stats[j][nt * 8 + 2 * c]);
           const float2 d2 = *reinterpret_cast<const float2*>(&sh.stats[j][16 + nt * 8 + 2 * c]);
-          float ds[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s[nt][e] = fast_exp2(fmaf(s[nt][e], p.cs, -((e & 1) ? l2.y : l2.x)));
-            ds[e] = s[nt][e] * (dp[nt][e] - ((e & 1) ? d2.y : d2.x));
+          for (int r = 0; r < 2; ++r) {
+            float2 pr = ffma2(make_float2(s[nt][2 * r], s[nt][2 * r + 1]), make_float2(p.cs, p.cs), l2);
+            pr.x = fast_exp2(pr.x);
+            pr.y = fast_exp2(pr.y);
+            const float2 ds = fmul2(pr, fadd2(make_float2(dp[nt][2 * r], dp[nt][2 * r + 1]), d2));
+            pa[2 * nt + r] = pack_bf16(pr.x, pr.y);
+            da[2 * nt + r] = pack_bf16(ds.x, ds.y);
           }
-          pa[2 * nt] = pack_bf16(s[nt][0], s[nt][1]); pa[2 * nt + 1] = pack_bf16(s[nt][2], s[nt][3]);
-          da[2 * nt] = pack_bf16(ds[0], ds[1]); da[2 * nt + 1] = pack_bf16(ds[2], ds[3]);
         }
       };
       auto tile = [&](int j) {
