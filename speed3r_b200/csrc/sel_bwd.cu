@@ -6,7 +6,7 @@
 //           (CSR lists, ascending query block => a fixed summation order, no atomics on floats)
 #include <mutex>
 
-#include "common.cuh"
+#include "sel_common.cuh"
 
 namespace s3r {
 
@@ -435,20 +435,6 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
 // Packed pairs in the exponentials' arithmetic, an elected thread that asks for copies and a wait whose usual outcome is one vote:
 // both parts 1650 -> 1621 us at 64 views, 6350 -> 6255 at 250.  Turning fragments in registers (movmatrix) instead of reading
 // them a second time: dQ the same (1627), dK/dV slower (1697), so that shared memory is not what is missing.
-struct SelBwdParams {
-  const __nv_bfloat16 *q, *k, *v, *d_o;
-  const int32_t *idx, *offsets, *qids;
-  const float *lse, *delta;
-  __nv_bfloat16 *dq, *dk, *dv;
-  // gradient of the pooled branch, added to dq | dk, dv (null: none): element t of dq gets dq_c[j] / kernel of every
-  // window j that contains it.  Kernel and stride are multiples of 16, so a warp's 16 rows share their windows.
-  const __nv_bfloat16 *dq_c, *dk_c, *dv_c;
-  int q_kernel, q_stride, q_windows, k_kernel, k_stride, k_windows;
-  int B, H, Tq, Tk, block, block_shift, topk, nqb, nkb;     // block = 16 << block_shift
-  float cs, scale;
-  uint32_t* status;
-};
-
 constexpr int kSbStageBytes = 8192;
 constexpr int kSbSmem = 2 * kSbStageBytes + 1024;
 
@@ -1066,6 +1052,7 @@ static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
   p.nkb = (p.Tk + p.block - 1) / p.block;
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_sel_attn_bwd: could not resolve the device status word");
+  if (p.block == 64) return sel_bwd64(p, st);          // 1.8 times as fast there; blocks of 32: see sel_bwd64.cu
   const int64_t bh = static_cast<int64_t>(p.B) * p.H;
   const int64_t tq = bh * ((p.Tq + 15) / 16), tk = bh * ((p.Tk + 15) / 16);
   S3R_REQUIRE(tq + tk < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_bwd: grid too large");

@@ -250,6 +250,42 @@ def test_sel_bwd_tiles(block, K, T):
         assert_bf16_close(a.grad, b.grad, f"{n} block {block} K {K} T {T}")
 
 
+@pytest.mark.parametrize("Tq,Tk,K", [(64, 64, 1), (64 * 3 + 1, 64 * 5 + 63, 3), (64 * 7, 64 * 2 + 17, 4), (64 * 40 - 1, 64 * 3, 33), (64 * 2, 64 * 70, 64)])
+def test_sel_bwd64_lists(Tq, Tk, K):
+    """Blocks of 64: lists of odd and even length, of none and of more entries than a lane holds at once, repeated and skipped
+    entries, first, last and cut-short blocks, as many queries as keys or not; values that are not finite stay with the rows
+    that use them."""
+    from speed3r_b200 import ops
+    B, H = 2, 2
+    nq, nk = -(-Tq // 64), -(-Tk // 64)
+    q, do = bf16_round(randn(90, B, H, Tq, 64), randn(91, B, H, Tq, 64))
+    k, v = bf16_round(randn(92, B, H, Tk, 64), randn(93, B, H, Tk, 64))
+    idx = table(94, B, H, nq, nk, K)
+    idx[:, 1, :, K // 2:] = -1                                           # skipped entries behind the first half
+    idx[:, :, 0, 0] = nk - 1                                             # the short block, and no list is empty
+    idx[1, 1, :, 0] = 0
+    if nk > 2:
+        idx[0, 0][idx[0, 0] == 1] = 0                                    # a block nobody selects
+    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    R.sel_attn(*ref, idx, 64)[0].backward(do)
+    got = [t.to(DEV, torch.bfloat16).requires_grad_(True) for t in (q, k, v)]
+    o = ops.topk_blocksparse_attention(*got, idx.to(DEV), 64)
+    grads = torch.autograd.grad(o, got, do.to(DEV, torch.bfloat16), retain_graph=True)
+    for n, a, b in zip("qkv", grads, ref):
+        assert_bf16_close(a, b.grad, f"d{n} {Tq} {Tk} {K}")
+    if nk > 2 and nq > 1:
+        bad = do.clone()
+        bad[0, 0, 0] = float("nan")                                      # of query block 0: its own keys and its own row
+        wrong = torch.autograd.grad(o, got, bad.to(DEV, torch.bfloat16))
+        used = torch.zeros(nk, dtype=torch.bool)
+        used[idx[0, 0, 0][idx[0, 0, 0] >= 0].long()] = True
+        rows = used.repeat_interleave(64)[:Tk]
+        for n, a, b in zip("kv", wrong[1:], grads[1:]):
+            assert torch.equal(a[0, 0][~rows.to(DEV)], b[0, 0][~rows.to(DEV)]) and torch.equal(a[1], b[1]), n
+        assert a[0, 0][rows.to(DEV)].isnan().any(-1).all()
+        assert wrong[0][0, 0, 0].isnan().all() and torch.equal(wrong[0][0, 0, 1:], grads[0][0, 0, 1:])
+
+
 # ------------------------------------------------------------------ the op as one autograd node
 @pytest.mark.parametrize("block,kernel,stride,topk", [(16, 16, 16, 8), (64, 32, 16, 4), (16, 8, 4, 8), (32, 32, 32, 4)])
 def test_op_node_gradients_match_separate_nodes(block, kernel, stride, topk):
