@@ -14,10 +14,15 @@
 // between them cost more registers and instructions than the starts they saved (574 -> 670 us).
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-7 softmax, thread = row.
 // Two CTAs per SM: their steps fill each other's waits.
-// The exponent offset of a row is its running maximum, step by step (O is rescaled in tensor memory where a row of the warp
-// moved): the row's largest weights are 1 and lose nothing when P is rounded to bf16.  Offsets fixed by the first step saved
-// the rescaling (64 views 544 instead of 585 us, 250 views 2.42 instead of 2.51 ms) but rounded those weights: error against
-// 64 bits 2.33e-3 instead of 2.24e-3 at unit-scale logits, 2.28e-3 instead of 1.64e-3 where a few keys hold a row's weight.
+// The exponent offset of a row is its running maximum, step by step (O is rescaled in tensor memory with every step: among a
+// warp's 32 rows one nearly always moves): the row's largest weights are 1 and lose nothing when P is rounded to bf16.  Offsets fixed
+// by the first step saved the rescaling (64 views 544 instead of 585 us, 250 views 2.42 instead of 2.51 ms) but rounded those weights:
+// error against 64 bits 2.33e-3 instead of 2.24e-3 at unit-scale logits, 2.28e-3 instead of 1.64e-3 where a few keys hold a row's
+// weight.  All exponentials on their own unit, packed rescaling and no vote in front of it: blocks of 64 at 64 views 551 -> 538 us, at
+// 250 views 2206 -> 2148 us (a quarter as polynomials, which this kernel's unit at half load does not need, 12 us of it).
+// Of a step's 1750 cycles (beside another CTA) 110 pass until the scores are in registers, 1000 from there to P, 170 until the
+// product before is known to be done, 330 for the rescaling and P's store.  Fetching the next step's scores before the
+// rescaling needed 192 registers and lost (614 us).
 // Zero times a value that is not finite is NaN, so one such value among a query block's keys reaches every row of the tile
 // through O += P V.  A row with finite scores and an O that is not is therefore done again from its own keys alone, by its
 // thread and out of line: taking the tile's lists one by one with the tensor cores instead needed the row's state in
@@ -289,7 +294,6 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // scale > 0 keeps the order; a NaN, or a score of +infinity (0 x inf), makes the offset and with it the row NaN
       const float mn = fmax3_nan(m_used, fmax3_nan(gm[0], gm[1], gm[2]) * cs, gm[3] * cs);
       const float neg = mn == -INFINITY ? 0.f : fmaf(mn, 0.f, -mn), alpha = fast_exp2(m_used + neg);
-      const bool moved = mn != m_used;
       m_used = mn;
       const float2 nm = make_float2(neg, neg), cs2 = make_float2(cs, cs);
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -299,12 +303,8 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float2 v = ffma2(make_float2(__uint_as_float(x[c][2 * i]), __uint_as_float(x[c][2 * i + 1])), cs2, nm);
-          if ((i & 3) == 0) {
-            v = exp2_fma2(v);
-          } else {
-            v.x = fast_exp2(v.x);
-            v.y = fast_exp2(v.y);
-          }
+          v.x = fast_exp2(v.x);
+          v.y = fast_exp2(v.y);
           sum[i & 1] = fadd2(sum[i & 1], v);
           pk[c][i] = pack_bf16(v.x, v.y);
         }
@@ -312,14 +312,18 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // P of the previous step must have been consumed: all of P waits in registers, so that its product has this long
       if (j > 0 && !mbar_wait_warp(&ctl.pv_done, (j - 1) & 1, abort_flag)) return false;
       tc_fence_after();
-      if (j > 0 && __any_sync(0xffffffffu, moved)) {
+      if (j > 0) {
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t o[32];
           tmem_ld32(t_o + hf * 32, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          for (int i = 0; i < 32; i += 2) {
+            const float2 x = fmul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), make_float2(alpha, alpha));
+            o[i] = __float_as_uint(x.x);
+            o[i + 1] = __float_as_uint(x.y);
+          }
           tmem_st32(t_o + hf * 32, o);
         }
       }
