@@ -411,6 +411,27 @@ def test_cmp_block_ranking_tiles(Nc, take, topk, heads):
     assert_bf16_close(o, ref, "o_c")
 
 
+@pytest.mark.parametrize("copies", [2, 3])
+@pytest.mark.parametrize("Nc", [48, 96, 384, 1536, 3264])
+def test_cmp_topk_orders_equal_logits(copies, Nc):
+    """Every key there two or three times, so that each logit is: both lists of a row hold some of the equal ones, for 48 keys the
+    bound is negative and its keys are cut.  Two copies end with the 32nd place, of three copies one is lost: equal logits stand in
+    the order of their columns either way."""
+    from speed3r_b200 import ops
+    B, H, Nq, n = 2, 2, 200, Nc // copies
+    q, k = bf16_round(randn(95, B, H, Nq, 64), randn(96, B, H, n, 64) / 4)
+    k = k.repeat(1, 1, copies, 1)
+    v, = bf16_round(randn(97, B, H, Nc, 64))
+    idx = ops._cmp_fwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v)), 32, 0.125)[2].cpu()
+    S = q.double() @ k[:, :, :n].double().transpose(-1, -2)
+    best, cols = S.topk(32 // copies + 1, dim=-1)
+    # rows whose different keys are further apart than fp32 sums of 64 products can differ
+    clear = ((best[..., :-1] - best[..., 1:]) > 64 * 2 ** -24 * S.abs().max()).all(-1)
+    assert clear.float().mean() > 0.5
+    want = (cols[..., None] + torch.arange(copies) * n).flatten(-2)[..., :32]
+    assert torch.equal(idx[clear].long(), want[clear])
+
+
 # ------------------------------------------------------------------ selection backward
 @pytest.mark.parametrize("block,T,K", [(16, 16 * 500 + 9, 3), (16, 16 * 520, 9), (32, 32 * 270 - 1, 2), (64, 64 * 130 + 1, 5)])
 def test_sel_bwd_tasks_handed_over(block, T, K):
