@@ -433,7 +433,8 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
 // order in the dK/dV kernel needs more registers than it gains: with the tiles one after the other 1161 -> 937 us, with
 // eight or nine warps and the tiles overlapped 1110 us.
 // Packed pairs in the exponentials' arithmetic, an elected thread that asks for copies and a wait whose usual outcome is one vote:
-// both parts 1650 -> 1621 us at 64 views, 6350 -> 6255 at 250.  Turning fragments in registers (movmatrix) instead of reading
+// both parts 1650 -> 1621 us at 64 views, 6350 -> 6255 at 250.  What an iteration asks for next - tokens of its copies, statistics -
+// is found at its start and nothing waits there for a load: 1621 -> 1596 and 6255 -> 6160.  Turning fragments in registers (movmatrix) instead of reading
 // them a second time: dQ the same (1627), dK/dV slower (1697), so that shared memory is not what is missing.
 constexpr int kSbStageBytes = 8192;
 constexpr int kSbSmem = 2 * kSbStageBytes + 1024;
@@ -561,16 +562,15 @@ __device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdPa
   const int ntiles = nvalid << p.block_shift, npairs = (ntiles + 1) >> 1, in_block = (1 << p.block_shift) - 1;
   auto tok_of = [&](int t) { return list[t >> p.block_shift] + ((t & in_block) << 4); };
   const bool leader = elect_one_sync();
-  auto issue = [&](int pair, int s) {
+  auto issue = [&](int t0, int t1, bool two, int s) {
     if (leader) {
-      const int t = 2 * pair;
-      mbar_expect_tx(&sh.full[s], (t + 1 < ntiles ? 8192u : 4096u) >> (map_kv.b_first < 0));
-      tma_load_pair<APART>(ring + s * kSbStageBytes, map_kv, &sh.full[s], tok_of(t), bh, 0);
-      if (t + 1 < ntiles) tma_load_pair<APART>(ring + s * kSbStageBytes + 4096, map_kv, &sh.full[s], tok_of(t + 1), bh, 0);
+      mbar_expect_tx(&sh.full[s], (two ? 8192u : 4096u) >> (map_kv.b_first < 0));
+      tma_load_pair<APART>(ring + s * kSbStageBytes, map_kv, &sh.full[s], t0, bh, 0);
+      if (two) tma_load_pair<APART>(ring + s * kSbStageBytes + 4096, map_kv, &sh.full[s], t1, bh, 0);
     }
   };
-  if (npairs > 0) issue(0, taken & 1);
-  if (npairs > 1) issue(1, (taken + 1) & 1);
+  if (npairs > 0) issue(tok_of(0), tok_of(min(1, ntiles - 1)), 1 < ntiles, taken & 1);
+  if (npairs > 1) issue(tok_of(2), tok_of(min(3, ntiles - 1)), 3 < ntiles, (taken + 1) & 1);
 
   uint32_t qf[4][4], dof[4][4];
   ldg_a_frags(qf, p.q + (static_cast<int64_t>(bh) * p.Tq + row0) * 64, nrows, lane);
@@ -624,6 +624,7 @@ __device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdPa
     frags_n(vn0, st + v_at, of.off_n);
     two_products(s0, dp0, qf, kn0, dof, vn0);
     frags_k(kk0, st + k_at, of.off_k);
+    const int t0 = tok_of(min(2 * it + 4, ntiles - 1)), t1 = tok_of(min(2 * it + 5, ntiles - 1));      // of the copies asked for below
     if (both) {
       frags_n(kn1, st + 4096 + k_at, of.off_n);
       frags_n(vn1, st + 4096 + v_at, of.off_n);
@@ -638,7 +639,7 @@ __device__ __forceinline__ void sel_bwd_dq(const PairMap& map_kv, const SelBwdPa
       accumulate(dq, a0, kk0);
     }
     __syncwarp();
-    if (it + 2 < npairs) issue(it + 2, S);            // every fragment of the stage has been consumed
+    if (it + 2 < npairs) issue(t0, t1, 2 * it + 5 < ntiles, S);            // every fragment of the stage has been consumed
   }
 #pragma unroll
   for (int dt = 0; dt < 8; ++dt)
@@ -705,12 +706,13 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
       if (both) tma_load_pair<APART>(ring + s * kSbStageBytes + 4096, map_qdo, &sh.full[s], t1, bh, 0);
     }
   };
-  // lanes 0-15 fetch lse, lanes 16-31 delta of a tile's rows; a row past the end gets lse = +inf: P is exactly 0
+  // lanes 0-15 fetch lse, lanes 16-31 delta of a tile's rows, as they are: nothing here waits for the load
   auto stat = [&](int tok0) {
-    const int t = tok0 + (lane & 15);
-    const float x = __ldg((lane < 16 ? p.lse : p.delta) + static_cast<int64_t>(bh) * p.Tq + min(t, p.Tq - 1));
-    return lane >= 16 ? -x : (t < p.Tq ? x * -1.4426950408889634f : -INFINITY);
+    return __ldg((lane < 16 ? p.lse : p.delta) + static_cast<int64_t>(bh) * p.Tq + min(tok0 + (lane & 15), p.Tq - 1));
   };
+  // -lse2 and -delta; a row past the end gets lse = +inf: P is exactly 0
+  const float stat_scale = lane < 16 ? -1.4426950408889634f : -1.f;
+  auto stat_value = [&](float x, int tok0) { return lane < 16 && tok0 + lane >= p.Tq ? -INFINITY : x * stat_scale; };
   auto offsets_of = [&](uint32_t task) {
     const uint32_t h = task / nslices, slice = task - h * nslices;
     return p.offsets + static_cast<int64_t>(h) * (p.nkb + 1) + (slice >> p.block_shift);
@@ -787,10 +789,10 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
 #pragma unroll 1
     for (int it = 0; it < npairs; ++it, ++taken) {
       const int S = taken & 1;
-      sh.stats[0][lane] = sa;
-      sh.stats[1][lane] = sb;
+      sh.stats[0][lane] = stat_value(sa, na);
+      sh.stats[1][lane] = stat_value(sb, nb);
       __syncwarp();
-      if (it + 1 < npairs) { sa = stat(ta); sb = stat(tb); }
+      if (it + 1 < npairs) { sa = stat(ta); sb = stat(tb); na = ta; nb = tb; }
       ok = ok && (__all_sync(0xffffffffu, mbar_try_wait(&sh.full[S], (taken >> 1) & 1)) || mbar_wait_warp(&sh.full[S], (taken >> 1) & 1, abort_flag));
       if (!ok) {
         volatile uint32_t dummy = 0;                    // a last bounded chance for what is under way to land
@@ -829,14 +831,14 @@ __global__ void __launch_bounds__(32, 10) sel_bwd_kernel(const __grid_constant__
         accumulate(dv, pa, dkk);
         accumulate(dk, da, qk);
       };
+      if (it + 2 < npairs) {                            // found here, where nothing waits for them
+        ta = tok_of(2 * it + 4);
+        tb = 2 * it + 5 < ntiles ? tok_of(2 * it + 5) : ta;
+      }
       tile(0);
       if (2 * it + 1 < ntiles) tile(1);
       __syncwarp();
-      if (it + 2 < npairs) {                            // every fragment of the stage has been consumed
-        ta = tok_of(2 * it + 4);
-        tb = 2 * it + 5 < ntiles ? tok_of(2 * it + 5) : ta;
-        issue(ta, tb, 2 * it + 5 < ntiles, S);
-      }
+      if (it + 2 < npairs) issue(ta, tb, 2 * it + 5 < ntiles, S);        // every fragment of the stage has been consumed
       // a request takes a task from those who could start it now, so it is made no sooner than its answer is needed
       const int left = npairs - 1 - it;
       if (left == 3) request();
