@@ -31,8 +31,9 @@
 // 2.45 ms for 7875 x 63000).
 // S of a tile is released as soon as its last columns are in registers, before their exponentials, so that the next
 // Q K^T runs under the rest of the softmax; P has tensor memory of its own.  Tensor memory: R x (S 128, O 64, P 64) columns.
-// A quarter of the exponentials are polynomials on the FMA pipe: with none the exponentials' unit saturates (2.63 ms), with
-// half of them the issue slots do (2.95 ms).
+// An eighth of the exponentials (ranking blocks: a sixteenth) are polynomials on the FMA pipe: they relieve the exponentials' unit and
+// cost issue slots, of which the running maxima and roundings leave few.  Both kernels, 15750 x 15750, 16 heads: none 2130 us, 1/16
+// 2085, 1/8 2062, 1/4 2098, 5/16 2160; 7875 x 63000: 3763, 3653, 3610, 3688, 3742; ranking blocks, 3937 x 15747: 808, 810, 846, 848.
 // The exponent offset of a row is the maximum of its first tile and does not move: P, O and l are floats, which keep their
 // relative precision however far later scores outgrow the first tile's, up to their range.  A CTA in which some row's
 // scores outgrew its offset by more than 2^64 takes its keys a second time with the rows' exact maxima, which the group
@@ -311,7 +312,7 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           float2 v = ffma2(make_float2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), cs2, nm);
-          if ((i & 3) == 0) {
+          if (i == 0 && (RANK == 0 || (c & 1) == 0)) {
             v = exp2_fma2(v);
           } else {
             v.x = fast_exp2(v.x);

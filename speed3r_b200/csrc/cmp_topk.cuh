@@ -23,9 +23,10 @@
 //
 // Bound: instructions and their latency in the scan: a max tree and a vote per 16 columns of a warp, and for the chunks
 // with a hit (three in four at 250 views, one in three at 1000) a mask and a store.  The products take half of the time
-// that the tensor pipe alone would need.  S of a tile is two buffers of 64 columns, each taken into registers in one go, so
-// that the next products run while a half is scanned (16 columns at a time, S held for a whole tile: 1.05 instead of
-// 0.95 ms for 15750 x 15750, 16 heads).
+// that the tensor pipe alone would need.  S of a tile is two buffers of 64 columns, so that the next products run while a half is
+// scanned (16 columns at a time, S held for a whole tile: 1.05 instead of 0.95 ms for 15750 x 15750, 16 heads), each taken into
+// registers 32 columns at a time (all 64 at once spilled in the scan: both kernels 448 instead of 439 us for 6300 x 6300, 2140
+// instead of 2098 for 15750 x 15750).
 // RANK 1 sums exponentials relative to the bound, three in four of them needed where a block counts three columns, and
 // only blocks that reach it get their logarithm: bound by the exponentials' unit.
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-19 scan: R = 2 row tiles of
@@ -409,26 +410,24 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl.s_empty[t][b][h]);
       };
-      uint32_t xa[32], xb[32];
-      tmem_ld32(src, xa);
-      tmem_ld32(src + 32, xb);
-      tmem_ld_wait();
-      release();
-      if (left < 64) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          if (i >= left) xa[i] = 0xff800000u;   // -inf
-          if (32 + i >= left) xb[i] = 0xff800000u;
-        }
-      }
       auto go = [&](const uint32_t* x, int c) {
         if (RANK) scan_blocks(x, c);
         else scan(x, c);
       };
-      go(xa, col0);
-      go(xa + 16, col0 + 16);
-      go(xb, col0 + 32);
-      go(xb + 16, col0 + 48);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t x[32];
+        tmem_ld32(src + 32 * q, x);
+        tmem_ld_wait();
+        if (q == 1) release();
+        if (left < 64) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (32 * q + i >= left) x[i] = 0xff800000u;   // -inf
+        }
+        go(x, col0 + 32 * q);
+        go(x + 16, col0 + 32 * q + 16);
+      }
       return true;
     };
     if (split) {
