@@ -275,7 +275,7 @@ int s3r_sel_attn_bwd(const void* q, const void* k, const void* v, const int32_t*
  * with one rounding:
  *   dq[t] += sum over windows j containing t of dq_c[j] / q_kernel   (windows of q_kernel tokens every q_stride)
  *   dk[t], dv[t] likewise from dk_c, dv_c with k_kernel, k_stride
- * dq_c [B,H,(Tq-q_kernel)/q_stride+1,d], dk_c / dv_c [B,H,(Tk-k_kernel)/k_stride+1,d]; any of them may be NULL.
+ * dq_c [B,H,(Tq-q_kernel)/q_stride+1,d], dk_c / dv_c [B,H,(Tk-k_kernel)/k_stride+1,d], 4-byte aligned; any of them may be NULL.
  * Kernels and strides must be multiples of 16. */
 int s3r_sel_attn_bwd_pooled(const void* q, const void* k, const void* v, const int32_t* idx, const int32_t* offsets,
                             const int32_t* qids, const float* lse_s, const float* delta_s, const void* do_s, void* dq,

@@ -1049,6 +1049,8 @@ static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
                        reinterpret_cast<uintptr_t>(p.d_o) | reinterpret_cast<uintptr_t>(p.dq) |
                        reinterpret_cast<uintptr_t>(p.dk) | reinterpret_cast<uintptr_t>(p.dv);
   S3R_REQUIRE((al & 15) == 0, S3R_ERR_ALIGNMENT, "s3r_sel_attn_bwd: tensors must be 16-byte aligned");
+  const uintptr_t al_c = reinterpret_cast<uintptr_t>(p.dq_c) | reinterpret_cast<uintptr_t>(p.dk_c) | reinterpret_cast<uintptr_t>(p.dv_c);
+  S3R_REQUIRE((al_c & 3) == 0, S3R_ERR_ALIGNMENT, "s3r_sel_attn_bwd_pooled: gradients of the pooled branch must be 4-byte aligned");
   p.block_shift = p.block == 16 ? 0 : p.block == 32 ? 1 : 2;
   p.nqb = (p.Tq + p.block - 1) / p.block;
   p.nkb = (p.Tk + p.block - 1) / p.block;

@@ -43,17 +43,20 @@ struct S64Maps {
   CUtensorMap q, d_o, k, v;      // boxes of 64 rows
 };
 
-// acc += the pooled branch's gradient of token t: g_c[j] / kernel of every window j that contains it
+// acc += the pooled branch's gradient of token t: g_c[j] / kernel of every window j that contains it.  g_c begins at a multiple of 4
+// bytes; where that is one of 16, as from any allocation, its rows are read in a quarter of the loads.
 __device__ __forceinline__ void s64_add_pooled(float (&acc)[64], const __nv_bfloat16* g_c, int bh, int t, int kernel, int stride,
                                                int windows) {
   if (g_c == nullptr) return;
   const int hi = min(windows - 1, t / stride), lo = t + 1 <= kernel ? 0 : (t - kernel) / stride + 1;
   const float inv = 1.0f / static_cast<float>(kernel);
+  const bool vec = (reinterpret_cast<uintptr_t>(g_c) & 15) == 0;
   for (int j = lo; j <= hi; ++j) {
-    const uint4* src = reinterpret_cast<const uint4*>(g_c + (static_cast<int64_t>(bh) * windows + j) * 64);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(g_c + (static_cast<int64_t>(bh) * windows + j) * 64);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint4 v = __ldg(src + i);
+      const uint4 v = vec ? __ldg(reinterpret_cast<const uint4*>(src) + i)
+                          : make_uint4(__ldg(src + 4 * i), __ldg(src + 4 * i + 1), __ldg(src + 4 * i + 2), __ldg(src + 4 * i + 3));
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {

@@ -301,18 +301,19 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q, const Tensor& k, con
   const int64_t B = q.size(0), H = q.size(1), Tq = q.size(2), d = q.size(3), Tk = k.size(2), K = idx.size(-1);
   c10::cuda::CUDAGuard guard(q.device());
   const Tensor do_s = aligned(do_s_);
+  const Tensor pooled[3] = {dq_c ? aligned(*dq_c) : Tensor(), dq_c ? aligned(*dk_c) : Tensor(), dq_c ? aligned(*dv_c) : Tensor()};
   auto [offsets, qids] = inverse ? *inverse : csr(idx, (Tk + block - 1) / block, false);
   Tensor dq = fresh_like(q), dk = fresh_like(k), dv = fresh_like(v);
   const bool fused = dq_c != nullptr && block % 16 == 0 && kernel % 16 == 0 && stride % 16 == 0;
-  auto ptr = [&](const Tensor* t) -> const void* { return fused ? t->data_ptr() : nullptr; };
+  auto ptr = [&](int i) -> const void* { return fused ? pooled[i].data_ptr() : nullptr; };
   check(s3r_sel_attn_bwd_pooled(q.data_ptr(), k.data_ptr(), v.data_ptr(), i32(idx), i32(offsets), i32(qids), f32(lse), f32(delta),
-                                do_s.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ptr(dq_c), ptr(dk_c), ptr(dv_c),
+                                do_s.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ptr(0), ptr(1), ptr(2),
                                 fused ? block : 16, fused ? block : 16, fused ? kernel : 16, fused ? stride : 16, B, H, Tq, Tk,
                                 d, block, K, scale, stream()), "s3r_sel_attn_bwd");
   if (dq_c != nullptr && !fused) {
-    check(s3r_pool_bwd(dq_c->data_ptr(), dq.data_ptr(), H * Tq * d, Tq * d, d, B, H, Tq, d, block, block, 1, stream()), "s3r_pool_bwd");
-    check(s3r_pool_bwd(dk_c->data_ptr(), dk.data_ptr(), H * Tk * d, Tk * d, d, B, H, Tk, d, kernel, stride, 1, stream()), "s3r_pool_bwd");
-    check(s3r_pool_bwd(dv_c->data_ptr(), dv.data_ptr(), H * Tk * d, Tk * d, d, B, H, Tk, d, kernel, stride, 1, stream()), "s3r_pool_bwd");
+    check(s3r_pool_bwd(pooled[0].data_ptr(), dq.data_ptr(), H * Tq * d, Tq * d, d, B, H, Tq, d, block, block, 1, stream()), "s3r_pool_bwd");
+    check(s3r_pool_bwd(pooled[1].data_ptr(), dk.data_ptr(), H * Tk * d, Tk * d, d, B, H, Tk, d, kernel, stride, 1, stream()), "s3r_pool_bwd");
+    check(s3r_pool_bwd(pooled[2].data_ptr(), dv.data_ptr(), H * Tk * d, Tk * d, d, B, H, Tk, d, kernel, stride, 1, stream()), "s3r_pool_bwd");
   }
   return {dq, dk, dv};
 }

@@ -98,6 +98,12 @@ def test_argument_errors_are_reported_without_a_gpu(lib):
         a = [p + 2 * (i == j) for j in range(6)]                   # dy, gate, o_c, o_s, do_s, do_c
         rc = lib.s3r_merge_bwd(a[0], a[1], 64, 32, 2, a[2], a[3], a[4], p, a[5], p, 1, 1, 16, 64, 16, None)
         assert rc == -3 and "aligned" in _lib.last_error()
+    # gradients of the pooled branch are read in words of 4 bytes
+    for block in (16, 32, 64):
+        for i in range(3):
+            rc = lib.s3r_sel_attn_bwd_pooled(*[p] * 12, *[p + 2 * (i == j) for j in range(3)], block, block, 16, 16, 1, 1, 64, 64, 64, block,
+                                             1, 0.125, None)
+            assert rc == -3 and "pooled" in _lib.last_error()
     # merge arguments must come together
     rc = lib.s3r_sel_attn_fwd(p, p, p, 1, 0, p, p, None, p, 0, 0, 0, None, None, 1, 1, 64, 64, 64, 16, 8, 0.125, None)
     assert rc == -4

@@ -889,6 +889,35 @@ def test_ops_take_gradients_that_begin_anywhere():
         assert all(torch.equal(a, b) for a, b in zip(got, want)), what
 
 
+@pytest.mark.parametrize("block,kernel,stride", [(16, 16, 16), (32, 32, 32), (64, 32, 16), (64, 64, 64), (64, 24, 8)])
+def test_pooled_gradients_that_begin_anywhere(block, kernel, stride):
+    """The pooled branch's gradients as views that begin at any element (the operator), at any multiple of 4 bytes (the library)."""
+    from speed3r_b200 import _lib, ops
+    B, H, T, K = 1, 2, 64 * 5 + 17, 3
+    nb, nw = -(-T // block), (T - kernel) // stride + 1
+    q, k, v, do = (randn(s, B, H, T, 64).to(DEV, torch.bfloat16) for s in range(4))
+    idx = table(5, B, H, nb, nb, K).to(DEV)
+    o, lse, _ = ops._sel_fwd(q, k, v, idx, None, None, block, 0.125, True, True, 1)
+    delta = (o.float() * do.float()).sum(-1)
+    pooled = [randn(6 + i, B, H, n, 64).to(DEV, torch.bfloat16) for i, n in enumerate((T // block, nw, nw))]
+    def moved(t, by):
+        m = torch.empty(t.numel() + by, device=DEV, dtype=t.dtype)[by:].view(t.shape)
+        return m.copy_(t)
+    call = lambda g: ops._ops().sel_attn_bwd_pooled(q, k, v, idx, lse, delta, do, *g, block, kernel, stride, 0.125)
+    want = call(pooled)
+    for by in (1, 2, 4, 8):
+        assert all(torch.equal(a, b) for a, b in zip(call([moved(t, by) for t in pooled]), want)), by
+    if kernel % 16 or stride % 16:
+        return
+    off, qids = ops.build_key_csr(idx, nb)
+    for by in (2, 4, 6):
+        g, got = [moved(t, by) for t in pooled], [torch.empty_like(t) for t in want]
+        _lib.check(_lib.load().s3r_sel_attn_bwd_pooled(*(t.data_ptr() for t in (q, k, v, idx, off, qids, lse, delta, do, *got, *g)), block,
+                                                       block, kernel, stride, B, H, T, T, 64, block, K, 0.125,
+                                                       torch.cuda.current_stream().cuda_stream), "s3r_sel_attn_bwd_pooled")
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), by
+
+
 def test_module_with_an_output_that_is_not_whole_vectors():
     """A projection to 100 channels: the sum of its bias gradient's rows cannot be read in vectors of eight."""
     m, x, pos = module_and_input(0)
