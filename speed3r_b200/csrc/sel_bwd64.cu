@@ -251,25 +251,27 @@ __device__ __forceinline__ void sel_bwd64_cta(const S64Maps& m, const SelBwdPara
       const int t = e * 64 + (r & 63);
       const bool in = e >= 0 && t < p.Tq;
       const int64_t at = static_cast<int64_t>(bh) * p.Tq + (in ? t : 0);
-      l = in ? __ldg(p.lse + at) * -1.4426950408889634f : -INFINITY;       // P exactly 0
+      l = in ? __ldg(p.lse + at) * -1.4426950408889634f : -INFINITY;
       d = in ? -__ldg(p.delta + at) : 0.f;
+      return in;
     };
     float nl = 0.f, nd = 0.f;
     int e2 = -1;
+    bool nlive = true;
     if (MODE == 0) {
-      stat(entry(0), nl, nd);
+      nlive = stat(entry(0), nl, nd);
       e2 = entry(1);
     }
     bool ok = true;
 #pragma unroll 1
     for (int j = 0; j < steps; ++j) {
       const float lse = nl, delta = nd;
+      // this row's query (dQ: key) exists
+      const bool live = MODE == 0 ? nlive : 2 * j + upper < cnt && list[2 * j + upper] + (r & 63) < p.Tk;
       if (MODE == 0) {
-        stat(e2, nl, nd);
+        nlive = stat(e2, nl, nd);
         e2 = entry(j + 2);
       }
-      // dQ: this row's key exists
-      const bool live = MODE == 0 || (2 * j + upper < cnt && list[2 * j + upper] + (r & 63) < p.Tk);
       ok = mbar_wait_warp(&ctl.s_full, j & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
@@ -300,9 +302,15 @@ __device__ __forceinline__ void sel_bwd64_cta(const S64Maps& m, const SelBwdPara
             x.y = fast_exp2(x.y);
             if (MODE == 0) pk[h * 16 + i + u] = pack_bf16(x.x, x.y);
             x = fmul2(x, fadd2(make_float2(__uint_as_float(dp[2 * (i + u)]), __uint_as_float(dp[2 * (i + u) + 1])), d[u]));
-            dk[h * 16 + i + u] = live ? pack_bf16(x.x, x.y) : 0u;
+            dk[h * 16 + i + u] = MODE == 0 || live ? pack_bf16(x.x, x.y) : 0u;
           }
         }
+      }
+      // dK/dV: rows of queries past the end, and of the half that a list of odd length leaves empty.  Their scores are products of
+      // zeros, which are NaN, not zero, with a key or value that is not finite.
+      if (MODE == 0 && !live) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pk[i] = dk[i] = 0u;
       }
       // the products of the step before must have read P and dS
       if (j > 0) {

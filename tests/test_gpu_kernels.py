@@ -286,6 +286,29 @@ def test_sel_bwd64_lists(Tq, Tk, K):
         assert wrong[0][0, 0, 0].isnan().all() and torch.equal(wrong[0][0, 0, 1:], grads[0][0, 0, 1:])
 
 
+@pytest.mark.parametrize("block", [16, 64])
+@pytest.mark.parametrize("Tq", [64, 64 * 2, 64 * 3, 64 * 3 - 16, 64 * 6 - 32])
+def test_sel_bwd_keys_that_are_minus_infinity(block, Tq):
+    """A key whose scores are all minus infinity has no weight: dK and dV there are those of a key far below all others, whether its
+    list of query blocks is of odd or even length, and whether or not the last of them is cut short."""
+    from speed3r_b200 import ops
+    B, H, Tk = 1, 2, 64 * 3
+    q, do = bf16_round(randn(100, B, H, Tq, 64), randn(101, B, H, Tq, 64))
+    k, v = bf16_round(randn(102, B, H, Tk, 64), randn(103, B, H, Tk, 64))
+    q[..., 5] = q[..., 5].abs() + 0.5
+    idx = torch.arange(Tk // block, dtype=torch.int32).expand(B, H, -(-Tq // block), -1).contiguous()
+    k[:, :, 3, 5] = -1e5
+    k[:, :, 77, 5] = -1e5
+    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    R.sel_attn(*ref, idx, block)[0].backward(do)
+    k[k[..., 5] == -1e5, 5] = -float("inf")
+    got = [t.to(DEV, torch.bfloat16).requires_grad_(True) for t in (q, k, v)]
+    grads = torch.autograd.grad(ops.topk_blocksparse_attention(*got, idx.to(DEV), block), got, do.to(DEV, torch.bfloat16))
+    for n, a, b in zip("kv", grads[1:], ref[1:]):
+        assert_bf16_close(a, b.grad, f"d{n}")
+        assert (a[:, :, [3, 77]] == 0).all(), f"d{n}"
+
+
 # ------------------------------------------------------------------ the op as one autograd node
 @pytest.mark.parametrize("block,kernel,stride,topk", [(16, 16, 16, 8), (64, 32, 16, 4), (16, 8, 4, 8), (32, 32, 32, 4)])
 def test_op_node_gradients_match_separate_nodes(block, kernel, stride, topk):
