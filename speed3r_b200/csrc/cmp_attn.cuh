@@ -65,7 +65,7 @@ struct AtCfg {
 };
 
 struct AtCtl {
-  uint64_t q_full, o_full;
+  uint64_t q_full, o_full, drained;
   uint64_t k_full[3], k_empty[3], v_full[3], v_empty[3];
   uint64_t s_full[2], s_free[2], p_full[2], pv_done[2];
   uint32_t tmem_base;
@@ -103,6 +103,7 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
     ctl.again = 0;
     mbar_init(&ctl.q_full, 1);
     mbar_init(&ctl.o_full, 1);
+    mbar_init(&ctl.drained, 1);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(&ctl.k_full[s], 1);
       mbar_init(&ctl.k_empty[s], 1);
@@ -233,11 +234,11 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
           s = sn;
           ph = phn;
         }
-        if (leader) umma_commit(&ctl.o_full);
+        if (leader) umma_commit(ok ? &ctl.o_full : &ctl.drained);           // who waits for results gets none from a CTA that gave up
         __syncwarp();
         if (!ok) {
           volatile uint32_t dummy = 0;
-          mbar_wait(&ctl.o_full, pass & 1, &dummy);       // let issued MMAs drain before tensor memory is freed
+          mbar_wait(&ctl.drained, 0, &dummy);             // let issued MMAs drain before tensor memory is freed
         }
       } while (another_pass(pass++));
     } else {

@@ -48,7 +48,7 @@ constexpr int kCbSmemBytes = kCbOffStat + kCbStages * 128 * 4 + 1024;
 constexpr uint32_t kCbColBuf = 128, kCbColDP = 64, kCbColAcc = 256, kCbColAcc1 = 64;
 
 struct CbCtl {
-  uint64_t x_full, o_full;
+  uint64_t x_full, o_full, drained;
   uint64_t y_full[kCbStages], y_empty[kCbStages], st_full[kCbStages];
   uint64_t s_full[2], dp_full[2], p_full[2], ds_full[2];
   uint32_t tmem_base;
@@ -82,6 +82,7 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
     ctl.abort_flag = 0;
     mbar_init(&ctl.x_full, MODE == 0 ? 1 : 16);
     mbar_init(&ctl.o_full, 1);
+    mbar_init(&ctl.drained, 1);
     for (int s = 0; s < kCbStages; ++s) {
       mbar_init(&ctl.y_full[s], 1);
       mbar_init(&ctl.y_empty[s], 1);
@@ -236,11 +237,11 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
           __syncwarp();
         }
       }
-      if (leader) umma_commit(&ctl.o_full);
+      if (leader) umma_commit(ok ? &ctl.o_full : &ctl.drained);      // who waits for results gets none from a CTA that gave up
       __syncwarp();
       if (!ok) {
         volatile uint32_t dummy = 0;
-        mbar_wait(&ctl.o_full, 0, &dummy);        // let issued MMAs drain before tensor memory is freed
+        mbar_wait(&ctl.drained, 0, &dummy);       // let issued MMAs drain before tensor memory is freed
       }
     }
   } else if (warp == 3) {

@@ -40,7 +40,7 @@ constexpr int kSbgThreads = 256;
 constexpr uint32_t kSbgColO = 128, kSbgColP = 192;
 
 struct SbgCtl {
-  uint64_t q_full, o_full;
+  uint64_t q_full, o_full, drained;
   uint64_t k_full[kSbgStages], k_empty[kSbgStages], v_full[kSbgStages], v_empty[kSbgStages];
   uint64_t s_full, s_free, p_full, pv_done;
   uint32_t tmem_base, abort_flag;
@@ -110,6 +110,7 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     ctl.abort_flag = 0;
     mbar_init(&ctl.q_full, 1);
     mbar_init(&ctl.o_full, 1);
+    mbar_init(&ctl.drained, 1);
     for (int s = 0; s < kSbgStages; ++s) {
       mbar_init(&ctl.k_full[s], 1);
       mbar_init(&ctl.k_empty[s], 1);
@@ -241,11 +242,11 @@ sel_big_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         s = sn;
         ph = phn;
       }
-      if (leader) umma_commit(&ctl.o_full);
+      if (leader) umma_commit(ok ? &ctl.o_full : &ctl.drained);            // who waits for results gets none from a CTA that gave up
       __syncwarp();
       if (!ok) {
         volatile uint32_t dummy = 0;
-        mbar_wait(&ctl.o_full, 0, &dummy);              // let issued MMAs drain before tensor memory is freed
+        mbar_wait(&ctl.drained, 0, &dummy);             // let issued MMAs drain before tensor memory is freed
       }
     }
   } else {

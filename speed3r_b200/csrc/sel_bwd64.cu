@@ -32,7 +32,7 @@ constexpr int kS64Threads = 256;
 constexpr uint32_t kS64ColDP = 64, kS64ColAcc = 128;
 
 struct S64Ctl {
-  uint64_t x_full, o_full;
+  uint64_t x_full, o_full, drained;
   uint64_t y_full[kS64Stages], y_empty[kS64Stages];
   uint64_t s_full, s_free, g_full, g_free;
   uint32_t tmem_base, abort_flag;
@@ -87,6 +87,7 @@ __device__ __forceinline__ void sel_bwd64_cta(const S64Maps& m, const SelBwdPara
     ctl.abort_flag = 0;
     mbar_init(&ctl.x_full, 1);
     mbar_init(&ctl.o_full, 1);
+    mbar_init(&ctl.drained, 1);
     for (int s = 0; s < kS64Stages; ++s) {
       mbar_init(&ctl.y_full[s], 1);
       mbar_init(&ctl.y_empty[s], 1);
@@ -231,11 +232,11 @@ __device__ __forceinline__ void sel_bwd64_cta(const S64Maps& m, const SelBwdPara
         if (leader) second(s, j > 0 ? 1u : 0u);
         __syncwarp();
       }
-      if (leader) umma_commit(&ctl.o_full);
+      if (leader) umma_commit(ok ? &ctl.o_full : &ctl.drained);            // who waits for results gets none from a CTA that gave up
       __syncwarp();
       if (!ok) {
         volatile uint32_t dummy = 0;
-        mbar_wait(&ctl.o_full, 0, &dummy);              // let issued MMAs drain before tensor memory is freed
+        mbar_wait(&ctl.drained, 0, &dummy);             // let issued MMAs drain before tensor memory is freed
       }
     }
   } else {

@@ -38,6 +38,17 @@ def test_next_kernel_starts_after_tensor_memory_is_allocated(path, at):
     assert 0 <= barrier < launch, "griddep_launch() before the barrier behind tcgen05.alloc"
 
 
+@pytest.mark.parametrize("path", sorted({p.values[0] for p in kernels_with_tensor_memory()}), ids=os.path.basename)
+def test_draining_after_a_wait_that_gave_up_signals_no_result(path):
+    """The issuing warp commits once more after a wait that gave up, to see its products drained.  The barrier of that commit is not one
+    that tells other warps their results are there: they may have got past their own waits, and would store what is not finished."""
+    src = code(path)
+    committed = set(re.findall(r"umma_commit\([^;]*?&ctl\.(\w+)", src)) | set(re.findall(r"umma_commit\([^;]*:\s*&ctl\.(\w+)", src))
+    drains = set(re.findall(r"\bmbar_wait\(&ctl\.(\w+)[^;]*&dummy\)", src)) & committed
+    waited = set(re.findall(r"mbar_wait_warp\(&ctl\.(\w+)[^;]*?abort_flag\)", src))
+    assert drains and not drains & waited, f"{os.path.basename(path)}: {drains & waited}"
+
+
 def test_polynomial_exponential_is_as_exact_as_stated():
     """2^f on [-1/2, 1/2] with the coefficients of exp2_fma2, in 64 bits and with every step rounded to fp32."""
     import numpy as np
