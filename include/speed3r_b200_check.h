@@ -40,6 +40,10 @@ int s3r_check_wait_gives_up(uint64_t limit_ns, uint64_t* waited_ns, void* stream
  * read): bit 0 b's tile in front of a's, bit 1 one tile serves as both, bit 2 two copies. */
 int s3r_check_pair_order(uint64_t a, uint64_t b);
 
+/* Whether the selection backward takes blocks of 64 with its tcgen05 kernel (1) or with the one for all block sizes (0): `bh`
+ * heads of `nqb` query blocks with `topk` entries each and `nkb` key blocks (host arithmetic). */
+int s3r_check_sel_bwd64_pays(int64_t bh, int64_t nqb, int64_t nkb, int64_t topk);
+
 /* This library's copies of the two helpers of speed3r_b200.h. */
 int s3r_last_error(char* buf, int n);
 int s3r_device_status(uint32_t* status_host, int clear);

@@ -58,6 +58,7 @@ CHECK_SIGNATURES = {
     "s3r_check_sel_attn_fwd": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _p]),
     "s3r_check_wait_gives_up": (_i, [C.c_uint64, _p, _p]),
     "s3r_check_pair_order": (_i, [C.c_uint64, C.c_uint64]),
+    "s3r_check_sel_bwd64_pays": (_i, [_i64, _i64, _i64, _i64]),
     "s3r_last_error": (_i, [C.c_char_p, _i]),
     "s3r_device_status": (_i, [C.POINTER(C.c_uint32), _i]),
 }

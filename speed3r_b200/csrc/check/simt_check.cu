@@ -2,7 +2,7 @@
 // the bf16 inputs, exact expf/logf).  They are slow and exist only so that tests can cross-check
 // the tensor-core kernels on the device at sizes a CPU check cannot reach.  No product path
 // calls them.  The file also holds the probe of the bounded wait (a wait that is made to run out).
-#include "../common.cuh"
+#include "../sel_common.cuh"
 
 namespace s3r {
 
@@ -168,6 +168,10 @@ extern "C" int s3r_check_sel_attn_fwd(const void* q, const void* k, const void* 
       idx, static_cast<__nv_bfloat16*>(o_s), lse_s, Tq, Tk, block, topk, scale);
   S3R_CUDA(cudaGetLastError());
   return 0;
+}
+
+extern "C" int s3r_check_sel_bwd64_pays(int64_t bh, int64_t nqb, int64_t nkb, int64_t topk) {
+  return sel_bwd64_pays(bh, nqb, nkb, topk);
 }
 
 extern "C" int s3r_check_pair_order(uint64_t a, uint64_t b) {

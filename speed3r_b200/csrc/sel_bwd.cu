@@ -1056,8 +1056,8 @@ static int launch_sel_bwd(SelBwdParams& p, int d, cudaStream_t st) {
   p.nkb = (p.Tk + p.block - 1) / p.block;
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_sel_attn_bwd: could not resolve the device status word");
-  if (p.block == 64) return sel_bwd64(p, st);          // 1.8 times as fast there; blocks of 32: see sel_bwd64.cu
   const int64_t bh = static_cast<int64_t>(p.B) * p.H;
+  if (p.block == 64 && sel_bwd64_pays(bh, p.nqb, p.nkb, p.topk)) return sel_bwd64(p, st);
   const int64_t tq = bh * ((p.Tq + 15) / 16), tk = bh * ((p.Tk + 15) / 16);
   S3R_REQUIRE(tq + tk < (1ll << 31), S3R_ERR_TOO_LARGE, "s3r_sel_attn_bwd: grid too large");
   PairMap mkv, mqdo;

@@ -9,7 +9,7 @@
 //        [dS_a | dS_b]^T [K_a | K_b]            (M=128, N=128, K=64): dQ is the sum of its diagonal blocks
 // The two blocks beside the diagonal are not read: an M=64 product takes as long as an M=128 one.  The softmax scale is applied
 // once, to the accumulators; the pooled branch's gradient is added in the store.
-// Blocks of 64 only.  The warps of sel_bwd.cu own 16 rows each, so that a block's four warps gather and read all of its tiles four
+// Blocks of 64 only, and there not where lists are next to empty (sel_bwd64_pays).  The warps of sel_bwd.cu own 16 rows each, so that a block's four warps gather and read all of its tiles four
 // times (2800 cycles of shared memory per pair of blocks and SM, 1860 of mma.sync); here it is 1220 of shared memory and 640 of
 // tensor pipe.  With blocks of 32 the same products would be a quarter instead of half useful.
 // 16 heads, top-16, both parts with the index: 8328 tokens 422 -> 229 us, 40 000 tokens 1812 -> 1027 us (random tables).

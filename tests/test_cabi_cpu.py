@@ -52,6 +52,17 @@ def test_tiles_of_tensors_far_apart_are_copied_one_by_one():
         assert order(base, base + gap) == 4 and order(base + gap, base) == 4
 
 
+def test_backward_of_short_lists_keeps_the_kernel_that_is_faster_there():
+    """Blocks of 64: lists of one or two entries on a full GPU, or of few queries over many keys, are not what tcgen05 pays for."""
+    from speed3r_b200 import _lib
+    pays = _lib.load_check().s3r_check_sel_bwd64_pays
+    for bh, nb, topk, want in ((1, 1, 1, 1), (16, 32, 1, 1), (12, 64, 1, 1), (16, 64, 1, 0), (16, 938, 1, 0), (2, 938, 2, 1), (16, 128, 2, 0),
+                               (16, 938, 2, 0), (16, 938, 3, 1), (1, 8, 8, 1), (16, 131, 16, 1), (16, 3938, 16, 1), (16, 1 << 20, 64, 1)):
+        assert pays(bh, nb, nb, topk) == want, (bh, nb, topk)
+    assert pays(16, 1, 938, 16) == 0 and pays(2, 1, 938, 4) == 0 and pays(2, 1, 938, 32) == 1
+    assert pays(16, 938, 16, 1) == 0 and pays(16, 938, 1, 1) == 1                  # one key block that every query block selects
+
+
 def test_argument_errors_are_reported_without_a_gpu(lib):
     from speed3r_b200 import _lib
     # NULL pointers

@@ -286,6 +286,23 @@ def test_sel_bwd64_lists(Tq, Tk, K):
         assert wrong[0][0, 0, 0].isnan().all() and torch.equal(wrong[0][0, 0, 1:], grads[0][0, 0, 1:])
 
 
+@pytest.mark.parametrize("Tq,Tk,K", [(64 * 130 - 9, 64 * 130 - 9, 1), (64 * 131, 64 * 130, 2), (64 * 2, 64 * 300 - 1, 16), (64 * 200, 64 * 50, 1)])
+def test_sel_bwd_short_lists_of_blocks_of_64(Tq, Tk, K):
+    """Lists too short, or too few of them, for the tcgen05 kernel: the kernel of the other block sizes, four tiles per block."""
+    from speed3r_b200 import _lib, ops
+    B, H, nq, nk = 1, 16, -(-Tq // 64), -(-Tk // 64)
+    assert not _lib.load_check().s3r_check_sel_bwd64_pays(H, nq, nk, K)
+    q, do = bf16_round(randn(104, B, H, Tq, 64), randn(105, B, H, Tq, 64))
+    k, v = bf16_round(randn(106, B, H, Tk, 64), randn(107, B, H, Tk, 64))
+    idx = table(108, B, H, nq, nk, K)
+    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    R.sel_attn(*ref, idx, 64)[0].backward(do)
+    got = [t.to(DEV, torch.bfloat16).requires_grad_(True) for t in (q, k, v)]
+    ops.topk_blocksparse_attention(*got, idx.to(DEV), 64).backward(do.to(DEV, torch.bfloat16))
+    for n, a, b in zip("qkv", got, ref):
+        assert_bf16_close(a.grad, b.grad, f"d{n} {Tq} {Tk} {K}")
+
+
 @pytest.mark.parametrize("block", [16, 64])
 @pytest.mark.parametrize("Tq", [64, 64 * 2, 64 * 3, 64 * 3 - 16, 64 * 6 - 32])
 def test_sel_bwd_keys_that_are_minus_infinity(block, Tq):
