@@ -17,9 +17,11 @@
 // needs more, and the pair's place - with a minimum and a maximum per exchange (sorting (key, column) as 64-bit words: 12 us
 // per CTA, most of the kernel up to 384 keys and 15 % of it at 6300).  Words of the same key - logits that are equal, or equal in
 // those bits: one row in several thousand, so that most launches have some - are put in order by their pairs afterwards, as
-// neighbours; only where the last of the 32 and one that was lost share a key is the row sorted again with the columns.  (All of a
-// warp's rows sorted again for any equal pair: this kernel 28 to 30 us instead of 17.5 for 2 x 384 x 384, 16 heads, 40 instead of 28
-// for 1024 x 1024; both kernels 466 instead of 454 for 6300 x 6300.)
+// neighbours.  A row is sorted again with the columns where the last of the 32 and one that was lost share a key, and where one pass
+// over the neighbours leaves a run of five or more out of order, which would take as many passes as it is long.  (All of a warp's rows
+// sorted again for any equal pair: this kernel 28 to 30 us instead of 17.5 for 2 x 384 x 384, 16 heads, 40 instead of 28 for
+// 1024 x 1024; both kernels 466 instead of 454 for 6300 x 6300.  Long runs pass by pass: 64 x 64 with all keys the same 84 us instead
+// of 39, 6300 x 6300 with every key there 16 times 666 instead of 620.)
 //
 // Bound: instructions and their latency in the scan: a max tree and a vote per 16 columns of a warp, and for the chunks
 // with a hit (three in four at 250 views, one in three at 1000) a mask and a store.  The products take half of the time
@@ -499,19 +501,17 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
 #pragma unroll
       for (int i = 0; i < 31; ++i) equal |= a[i + 1] != 0u && a[i] >> 7 == a[i + 1] >> 7 ? 1u << i : 0u;
       const uint2* other = buf + 4 * (kTkCap * 32);
-      if (__any_sync(0xffffffffu, cut_equal)) {
-        tk_exact(buf, cnt, other, static_cast<int>(tell[2 * 128]), words);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) a[i] = words[i * 128];
-      } else {
-        // neighbours of the same key change places until their pairs are in order
+      const bool exact = __any_sync(0xffffffffu, cut_equal);
+      bool moved = !exact && __any_sync(0xffffffffu, equal != 0u);
+      if (moved) {
+        // neighbours of the same key change places until their pairs are in order; once where five or more are in a row
         auto pair_of = [&](uint32_t w) {
           const int place = 127 - static_cast<int>(w & 127u);
           return tk_entry(place < kTkCap ? buf[place * 32] : other[(place - kTkCap) * 32]);
         };
-        bool moved = __any_sync(0xffffffffu, equal != 0u);
+        const bool run = __any_sync(0xffffffffu, (equal & (equal >> 1) & (equal >> 2) & (equal >> 3)) != 0u);
 #pragma unroll 1
-        while (moved) {
+        do {
           moved = false;
 #pragma unroll
           for (int i = 0; i < 31; ++i) {
@@ -525,7 +525,13 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
             }
           }
           moved = __any_sync(0xffffffffu, moved);
-        }
+        } while (moved && !run);
+      }
+      if (exact || moved) {
+        tk_exact(buf, cnt, other, static_cast<int>(tell[2 * 128]), words);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) a[i] = words[i * 128];
+      } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const int place = 127 - static_cast<int>(a[i] & 127u);
