@@ -255,19 +255,23 @@ def test_sel_bwd64_lists(Tq, Tk, K):
     """Blocks of 64: lists of odd and even length, of none and of more entries than a lane holds at once, repeated and skipped
     entries, first, last and cut-short blocks, as many queries as keys or not; values that are not finite stay with the rows
     that use them."""
-    from speed3r_b200 import ops
+    from speed3r_b200 import _lib, ops
     B, H = 2, 2
     nq, nk = -(-Tq // 64), -(-Tk // 64)
+    assert _lib.load_check().s3r_check_sel_bwd64_pays(B * H, nq, nk, K)
     q, do = bf16_round(randn(90, B, H, Tq, 64), randn(91, B, H, Tq, 64))
     k, v = bf16_round(randn(92, B, H, Tk, 64), randn(93, B, H, Tk, 64))
     idx = table(94, B, H, nq, nk, K)
     idx[:, 1, :, K // 2:] = -1                                           # skipped entries behind the first half
-    idx[:, :, 0, 0] = nk - 1                                             # the short block, and no list is empty
+    idx[:, :, 0, 0] = nk - 1                                             # the short block
     idx[1, 1, :, 0] = 0
     if nk > 2:
         idx[0, 0][idx[0, 0] == 1] = 0                                    # a block nobody selects
-    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
-    R.sel_attn(*ref, idx, 64)[0].backward(do)
+    ref, idx_ref, do_ref = [t.clone().requires_grad_(True) for t in (q, k, v)], idx.clone(), do.clone()
+    if nq > 1:
+        idx[1, 0, 1] = -1                                                # a list of none: as if nothing came back to its rows
+        idx_ref[1, 0, 1], do_ref[1, 0, 64:128] = 0, 0.0
+    R.sel_attn(*ref, idx_ref, 64)[0].backward(do_ref)
     got = [t.to(DEV, torch.bfloat16).requires_grad_(True) for t in (q, k, v)]
     o = ops.topk_blocksparse_attention(*got, idx.to(DEV), 64)
     grads = torch.autograd.grad(o, got, do.to(DEV, torch.bfloat16), retain_graph=True)
@@ -282,8 +286,46 @@ def test_sel_bwd64_lists(Tq, Tk, K):
         rows = used.repeat_interleave(64)[:Tk]
         for n, a, b in zip("kv", wrong[1:], grads[1:]):
             assert torch.equal(a[0, 0][~rows.to(DEV)], b[0, 0][~rows.to(DEV)]) and torch.equal(a[1], b[1]), n
-        assert a[0, 0][rows.to(DEV)].isnan().any(-1).all()
+            assert a[0, 0][rows.to(DEV)].isnan().any(-1).all(), n
         assert wrong[0][0, 0, 0].isnan().all() and torch.equal(wrong[0][0, 0, 1:], grads[0][0, 0, 1:])
+
+
+@pytest.mark.parametrize("block", [16, 32, 64])
+@pytest.mark.parametrize("which", ["q", "k", "v"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_sel_bwd_keeps_non_finite_values_to_the_rows_that_use_them(block, which, value):
+    """A query reaches its own row and the keys of its list; a key or value the query blocks that selected it and the keys of their
+    lists.  All other gradients are the same bits as without it (from the same forward: that of blocks of 32 and 64 rounds the rows beside
+    such rows otherwise)."""
+    from speed3r_b200 import ops
+    B, H, nb, K, at = 1, 2, 20, 3, 5 * block + 7
+    T = block * nb - 5
+    x = dict(zip("qkv", bf16_round(*(randn(110 + i, B, H, T, 64) for i in range(3)))))
+    do = randn(113, B, H, T, 64).to(DEV, torch.bfloat16)
+    idx = table(114, B, H, nb, nb, K)
+    idx[:, :, 5], idx[:, :, 6] = torch.tensor([5, 5, nb - 1]), torch.tensor([5, 0, -1])
+    users = torch.arange(nb) == 5                                        # query blocks that read the value, and their lists
+    if which != "q":
+        users = (idx[0, 0] == 5).any(-1)
+    listed = torch.zeros(nb, dtype=torch.bool)
+    listed[idx[0, 0][users][idx[0, 0][users] >= 0].long()] = True
+    rows, keys = (t.repeat_interleave(block)[:T] for t in (users, listed))
+    if which == "q":
+        rows = torch.arange(T) == at
+    idx = idx.to(DEV)
+    dev = lambda: [x[n].to(DEV, torch.bfloat16) for n in "qkv"]
+    forward = lambda: ops._sel_fwd(*dev(), idx, None, None, block, 0.125, True, True, 1)[:2]
+    backward = lambda o, lse: [g.cpu() for g in ops._ops().sel_attn_bwd(*dev(), idx, lse, (o.float() * do.float()).sum(-1), do, block, 0.125)]
+    o, lse = forward()
+    clean = backward(o, lse)
+    x[which] = x[which].clone()
+    x[which][0, 0, at, 9] = value
+    o_bad, lse_bad = forward()
+    o[0, 0, rows], lse[0, 0, rows] = o_bad[0, 0, rows], lse_bad[0, 0, rows]
+    bad = backward(o, lse)
+    for n, reached, a, b in zip("qkv", (rows, keys, keys), bad, clean):
+        assert torch.equal(a[0, 1], b[0, 1]) and torch.equal(a[0, 0][~reached], b[0, 0][~reached]), n
+    assert not bad[0][0, 0][rows].isfinite().all() and all(b.isfinite().all() for b in clean)
 
 
 @pytest.mark.parametrize("Tq,Tk,K", [(64 * 130 - 9, 64 * 130 - 9, 1), (64 * 131, 64 * 130, 2), (64 * 2, 64 * 300 - 1, 16), (64 * 200, 64 * 50, 1)])
@@ -496,8 +538,8 @@ def test_cmp_topk_of_equal_logits_takes_no_longer():
 # ------------------------------------------------------------------ selection backward
 @pytest.mark.parametrize("block,T,K", [(16, 16 * 500 + 9, 3), (16, 16 * 520, 9), (32, 32 * 270 - 1, 2), (64, 64 * 130 + 1, 5)])
 def test_sel_bwd_tasks_handed_over(block, T, K):
-    """More tasks than places on the GPU, so that warps take over others': lists of no entry, one, and several hundred (a key
-    block that every query block selects), an odd number of tiles, a short last block."""
+    """More tasks than places on the GPU, so that warps take over others' (blocks of 64, whose CTAs do not, beside them): lists of no
+    entry, one, and several hundred (a key block that every query block selects), an odd number of tiles, a short last block."""
     from speed3r_b200 import ops
     B, H, nb = 1, 4, -(-T // block)
     q, k, v, do = bf16_round(*(randn(75 + i, B, H, T, 64) for i in range(4)))
@@ -952,12 +994,14 @@ def test_ops_take_gradients_that_begin_anywhere():
 
 @pytest.mark.parametrize("block,kernel,stride", [(16, 16, 16), (32, 32, 32), (64, 32, 16), (64, 64, 64), (64, 24, 8)])
 def test_pooled_gradients_that_begin_anywhere(block, kernel, stride):
-    """The pooled branch's gradients as views that begin at any element (the operator), at any multiple of 4 bytes (the library)."""
+    """The pooled branch's gradients, with a short last block and a query block without a list, and as views that begin at any element
+    (the operator) or at any multiple of 4 bytes (the library)."""
     from speed3r_b200 import _lib, ops
     B, H, T, K = 1, 2, 64 * 5 + 17, 3
     nb, nw = -(-T // block), (T - kernel) // stride + 1
     q, k, v, do = (randn(s, B, H, T, 64).to(DEV, torch.bfloat16) for s in range(4))
     idx = table(5, B, H, nb, nb, K).to(DEV)
+    idx[:, :, 1] = -1
     o, lse, _ = ops._sel_fwd(q, k, v, idx, None, None, block, 0.125, True, True, 1)
     delta = (o.float() * do.float()).sum(-1)
     pooled = [randn(6 + i, B, H, n, 64).to(DEV, torch.bfloat16) for i, n in enumerate((T // block, nw, nw))]
@@ -966,6 +1010,14 @@ def test_pooled_gradients_that_begin_anywhere(block, kernel, stride):
         return m.copy_(t)
     call = lambda g: ops._ops().sel_attn_bwd_pooled(q, k, v, idx, lse, delta, do, *g, block, kernel, stride, 0.125)
     want = call(pooled)
+    alone = ops._ops().sel_attn_bwd(q, k, v, idx, lse, delta, do, block, 0.125)
+    for n, got, base, g, size, step in zip("qkv", want, alone, pooled, (block, kernel, kernel), (block, stride, stride)):
+        share = torch.zeros_like(base, dtype=torch.float)
+        for j in range(g.shape[2]):
+            share[:, :, j * step:j * step + size] += g[:, :, j:j + 1].float() / size
+        # two roundings to bf16, 2^-9 of what is rounded each, and sums of a few terms in fp32
+        assert ((got.float() - base.float() - share).abs() <= 2 ** -8 * (base.float().abs() + got.float().abs()) + 1e-6).all(), n
+    assert (alone[0][:, :, block:2 * block] == 0).all()
     for by in (1, 2, 4, 8):
         assert all(torch.equal(a, b) for a, b in zip(call([moved(t, by) for t in pooled]), want)), by
     if kernel % 16 or stride % 16:
