@@ -6,12 +6,11 @@
 // is written over the diagonal blocks of a zeroed tile, so that O += P V (K=128) adds the right keys to each row.  The
 // G - 1 unwanted blocks beside each wanted one are cheaper than mma.sync without them: 16 heads, top-16 blocks of 64 at 250
 // views 3.86 -> 2.51 ms, 64 views 1002 -> 585 us; top-32 blocks of 32, 60000 tokens 1073 -> 964 us.
-// Bound: latency, with no unit more than half busy.  Of a CTA's 18.5 us at 64500 tokens, top-16 (with fixed offsets, below), 2.4
-// pass until its first S is
-// there, 13 in 16 steps (0.8 us each beside another CTA, 80 KB of shared-memory traffic) and 3 at its end; 2.5 more until
-// the next CTA runs in its place.  The merge's operands are loaded before the last product is waited for (1.6 us less at the
-// end, 2 to 4 % of the whole).  Two threads per row instead of one changed nothing; several row tiles per CTA without a barrier
-// between them cost more registers and instructions than the starts they saved (574 -> 670 us).
+// Bound: latency, with no unit more than half busy.  A CTA takes its place for 19.8 us (64 512 tokens, top-16, 8064 CTAs in 538 us), of
+// which 16 steps of 1750 cycles beside another CTA (80 KB of shared-memory traffic each; below) are 14.5; the rest passes before its
+// first S, at its end and until the next CTA runs in its place.  The merge's operands are loaded before the last product is waited
+// for (1.6 us less at the end, 2 to 4 % of the whole).  Two threads per row instead of one changed nothing; several row tiles per CTA
+// without a barrier between them cost more registers and instructions than the starts they saved (574 -> 670 us).
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-7 softmax, thread = row.
 // Two CTAs per SM: their steps fill each other's waits.
 // The exponent offset of a row is its running maximum, step by step (O is rescaled in tensor memory with every step: among a

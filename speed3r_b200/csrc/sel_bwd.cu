@@ -426,16 +426,16 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
 // Both kernels: one warp = one CTA owns 16 rows (queries | keys) and meets tiles of 16 rows of the other side, two at
 // a time, out of a ring of two 8 KB stages; one TMA copy brings a tile of two tensors (K and V | Q and dO).
 // Fragments are loaded ahead of the products that use them.  Softmax scale: applied once, to the accumulators.
-// Bound: shared memory (a tile is written once and read as three | four 2 KB fragment sets: 10 | 12 KB of traffic per
-// 4 KB gathered, at 128 bytes per cycle) and, close behind, mma.sync (24 | 32 of 8 cycles per tile and sub-partition);
-// what is missing to either is latency that twelve warps per SM (registers, rings) do not cover.  In the dQ kernel the
+// Bound: latency that twelve warps per SM (registers, rings) do not cover, between shared memory (79 % busy: a tile is written once and
+// read as three | four 2 KB fragment sets, 10 | 12 KB of traffic per 4 KB gathered, at 128 bytes per cycle) and mma.sync (57 %: 24 |
+// 32 of 8 cycles per tile and sub-partition); busy at 100 views, top-32.  In the dQ kernel the
 // second tile's loads run under the first tile's exponentials (919 -> 638 us at 64 views, H = 16, top-32); the same
 // order in the dK/dV kernel needs more registers than it gains: with the tiles one after the other 1161 -> 937 us, with
 // eight or nine warps and the tiles overlapped 1110 us.
 // Packed pairs in the exponentials' arithmetic, an elected thread that asks for copies and a wait whose usual outcome is one vote:
 // both parts 1650 -> 1621 us at 64 views, 6350 -> 6255 at 250.  What an iteration asks for next - tokens of its copies, statistics -
-// is found at its start and nothing waits there for a load: 1621 -> 1596 and 6255 -> 6160.  Turning fragments in registers (movmatrix) instead of reading
-// them a second time: dQ the same (1627), dK/dV slower (1697), so that shared memory is not what is missing.
+// is found at its start and nothing waits there for a load: 1621 -> 1596 and 6255 -> 6160.  Turning fragments in registers (movmatrix)
+// instead of reading them a second time: dQ the same (1627), dK/dV slower (1697).
 constexpr int kSbStageBytes = 8192;
 constexpr int kSbSmem = 2 * kSbStageBytes + 1024;
 

@@ -11,9 +11,11 @@
 // once, to the accumulators; the pooled branch's gradient is added in the store.
 // Blocks of 64 only, and there not where lists are next to empty (sel_bwd64_pays).  The warps of sel_bwd.cu own 16 rows each, so that a block's four warps gather and read all of its tiles four
 // times (2800 cycles of shared memory per pair of blocks and SM, 1860 of mma.sync); here it is 1220 of shared memory and 640 of
-// tensor pipe.  With blocks of 32 the same products would be a quarter instead of half useful.
+// tensor pipe for a dK/dV and a dQ step.  With blocks of 32 the same products would be a quarter instead of half useful.
 // 16 heads, top-16, both parts with the index: 8328 tokens 422 -> 229 us, 40 000 tokens 1812 -> 1027 us (random tables).
-// Bound: what the products read of shared memory (176 KB per dK/dV step, 128 KB per dQ step, two CTAs per SM).  Two threads per row
+// Bound: the latency of a step's chain - copies, S and dP, P and dS, second product, 2250 cycles beside the SM's other CTA - with two
+// stages and two CTAs per SM.  No unit is half busy: shared memory 47 % (176 KB of copies, stores and reads per dK/dV step, 112 of them
+// read by the products; 128 and 80 per dQ step), tensor pipe 39 %, exponentials 31 %.  Two threads per row
 // instead of one changed nothing (230 and 1050 us), tasks handed on to running CTAs, with copies and first products ahead across
 // them, little (225 and 981 us).
 // Roles: warp 0 TMA producer, warp 1 tcgen05.mma issuer, warp 2 tensor-memory allocator, warps 4-7 P and dS.

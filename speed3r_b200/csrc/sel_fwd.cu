@@ -28,11 +28,12 @@ namespace s3r {
 //   * The thread that asks for copies is elected, so that the compiler knows it is one and coordinates need no loop over lanes
 //     (548 -> 533 us); the list's entries are read where they are used (read a pair ahead 548 -> 568 us).
 //   * CTAs of one warp: nothing is shared between query blocks, and a finished warp makes room at once.
-// Bound: the gather and shared memory (4 KB of a pair of blocks written and read again: 64 of 68 cycles per SM).  H = 16, top-32,
-// uniformly random blocks; before the last two points, and this kernel without its arithmetic, in brackets: 2048 tokens 26.2 us
-// (28.1, 21.5), 64 views 509 us = 16.6 TB/s gathered (548; 415, 20.4 TB/s), 100 views 791 (852, 648), 250 views 2.07 ms (2.16,
-// 1.66), 1000 views, where a head's 258 MB of keys and values miss L2, 13.9 ms = 9.5 TB/s (14.0; 13.6, 9.7 TB/s).  The op's own
-// tables favour some blocks (with independent inputs a tenth of them has a third of the picks): at 1000 views 11.2 ms.
+// Bound: the gather, then the latency of a pair's chain that twelve warps per SM do not cover, then the power limit.  H = 16,
+// top-32, uniformly random blocks, us at 1965 MHz - this kernel | its copies and waits alone | those and its fragment loads:
+// 2048 tokens 24.8 | 17.9 | 19.8, 64 views 486 = 17.4 TB/s gathered | 397 | 404, 100 views 775 | 625 | 632; so shared memory's reads
+// are 2 %.  In a long loop the clock falls under the power limit, to 1.75 GHz at 100 views (843 us), 1.6 at 250 (2.28 ms | 1.62 |
+// 1.65) and 1.3 at 1000, where a head's 258 MB of keys and values miss L2 (15.0 ms = 8.9 TB/s | 13.1 | 13.3).  The op's own tables
+// favour some blocks (with independent inputs a tenth of them has a third of the picks): at 1000 views 10.5 ms.
 // Slots of single blocks in a ring of three, which let 15 warps instead of 12 onto an SM, lost more to a second wait per pair
 // (64 views 592 us; 2048 tokens 25.2); refilling a slot before the products instead of after them changed nothing (lop3 of the
 // fragments or a proxy fence in front: 600 and 612 us).
