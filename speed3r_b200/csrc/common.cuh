@@ -204,6 +204,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Whether the phase is complete, without waiting for it.  Asking takes about a hundred cycles even where it is, so that a warp
+// with something else to issue asks before that and looks at the answer afterwards.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Per-warpgroup register re-partition (every warp of the group of four executes the same one).
 template <int N>
 __device__ __forceinline__ void reg_alloc() {
@@ -256,6 +269,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
                                                uint64_t limit_ns = 1000000000ull) {
   const bool ok = mbar_wait_limit(bar, parity, abort_flag, limit_ns);
   return __all_sync(0xffffffffu, ok);
+}
+
+// The rest of a wait that mbar_test began.  No vote: lanes may part where one of them gives up.
+__device__ __forceinline__ bool mbar_settle(bool done, uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  return done || mbar_wait(bar, parity, abort_flag);
 }
 
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -457,6 +475,43 @@ __device__ __forceinline__ void umma_ts_k4(uint32_t d_tmem, uint32_t a_tmem, uin
 // Arrive on an mbarrier once every tcgen05 operation issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
+}
+// The same for a warp that runs all of its loop converged: only the lane whose `lead` is set issues.  Without a branch around them
+// there is nothing to converge after, and operands stay warp-uniform.
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_ss_k4_by(uint32_t lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p, pt, l;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 pt, 0, 0;\n\tsetp.ne.b32 l, %7, 0;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "add.s64 a, %1, %5;\n\tadd.s64 b, %2, %6;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, pt;\n\t"
+      "add.s64 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, pt;\n\t"
+      "add.s64 a, a, %5;\n\tadd.s64 b, b, %6;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, pt;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accum), "n"(A_STEP), "n"(B_STEP), "r"(lead)
+      : "memory");
+}
+template <int B_STEP, int A_JUMP = 8>
+__device__ __forceinline__ void umma_ts_k4_by(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p, pt, l;\n\t.reg .b64 b;\n\t.reg .b32 a;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 pt, 0, 0;\n\tsetp.ne.b32 l, %7, 0;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "add.u32 a, %1, 8;\n\tadd.s64 b, %2, %5;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n\t"
+      "add.u32 a, a, %6;\n\tadd.s64 b, b, %5;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n\t"
+      "add.u32 a, a, 8;\n\tadd.s64 b, b, %5;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, pt;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "n"(B_STEP), "n"(A_JUMP), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_by(uint32_t lead, uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred l;\n\tsetp.ne.b32 l, %1, 0;\n\t"
+               "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lead)
                : "memory");
 }
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp receives lane (base_lane + i).

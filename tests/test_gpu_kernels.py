@@ -816,6 +816,40 @@ def test_cmp_backward_with_all_logits_far_below_zero(Nc):
         assert_bf16_close(a.grad, b.grad, name)
 
 
+@pytest.mark.parametrize("Nq, Nc", [(1, 128), (127, 129), (128, 1), (129, 256), (257, 641), (641, 257), (1409, 130)])
+def test_cmp_backward_tiles(Nq, Nc):
+    """Tiles of 128 rows on either side: one row, one short or long of a tile, one and several rounds of the ring of five."""
+    from speed3r_b200 import ops
+    B, H = 1, 2
+    q, k, v, do = bf16_round(randn(1, B, H, Nq, 64), randn(2, B, H, Nc, 64), randn(3, B, H, Nc, 64), randn(4, B, H, Nq, 64))
+    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    torch.softmax(ref[0] @ ref[1].transpose(-1, -2) * 0.125, -1).matmul(ref[2]).backward(do)
+    t = [x.to(DEV, torch.bfloat16).requires_grad_(True) for x in (q, k, v)]
+    ops.flash_attn_topk_func(*t, 1)[0].backward(do.to(DEV, torch.bfloat16))
+    for name, a, b in zip(("dq", "dk", "dv"), t, ref):
+        assert_bf16_close(a.grad, b.grad, name)
+
+
+@pytest.mark.parametrize("Nq", [64, 70, 128, 200])
+def test_cmp_backward_of_a_key_that_is_minus_infinity(Nq):
+    """A key that no query gives a weight has no gradient, whether the last tile of queries is whole or not: rows that do not exist
+    have no weight.  The other keys' gradients are what they are without it."""
+    from speed3r_b200 import ops
+    B, H, Nc, at = 1, 2, 96, 5
+    q, k, v, do = bf16_round(randn(1, B, H, Nq, 64), randn(2, B, H, Nc, 64), randn(3, B, H, Nc, 64), randn(4, B, H, Nq, 64))
+    q[..., 0] = q[..., 0].abs() + 0.5
+    k[:, :, at, 0] = float("-inf")
+    t = [x.to(DEV, torch.bfloat16).requires_grad_(True) for x in (q, k, v)]
+    ops.flash_attn_topk_func(*t, 8)[0].backward(do.to(DEV, torch.bfloat16))
+    rest = torch.arange(Nc) != at
+    ref = [x.clone().requires_grad_(True) for x in (q, k[:, :, rest], v[:, :, rest])]
+    torch.softmax(ref[0] @ ref[1].transpose(-1, -2) * 0.125, -1).matmul(ref[2]).backward(do)
+    for name, a, b in zip(("dk", "dv"), t[1:], ref[1:]):
+        g = a.grad.cpu()
+        assert (g[:, :, at] == 0).all(), name
+        assert_bf16_close(g[:, :, rest], b.grad, name)
+
+
 def test_prologue_of_blocks_whose_table_rows_do_not_fit_shared_memory():
     """Blocks of 6400 tokens: token rows as with blocks of 16, bit for bit, means as in fp32, and the backward."""
     import speed3r_b200
