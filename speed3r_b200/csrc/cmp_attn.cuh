@@ -84,8 +84,9 @@ struct AtParams {
   uint32_t* status;
 };
 
-// `cta`: which R * 128 rows
-template <int R, int RANK>
+// `cta`: which R * 128 rows.  FILL: the second kernel is a launch of its own, which starts early and waits for the bounds as they come:
+// a bound's place gets what it waits on (all bits set) before this CTA lets that kernel start.
+template <int R, int RANK, bool FILL>
 __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
                                              const CUtensorMap& map_ks, const CUtensorMap& map_vs, const AtParams& p, AtCtl& ctl,
                                              uint8_t* smem_raw, int cta) {
@@ -126,7 +127,7 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
   __syncthreads();
   tc_fence_after();
   griddep_wait();
-  griddep_launch();
+  if (!FILL) griddep_launch();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
@@ -242,6 +243,13 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
         }
       } while (another_pass(pass++));
     } else {
+      if (FILL && warp == 3) {                 // the bounds themselves are written behind another_pass
+        for (int i = lane; i < R * 128; i += 32)
+          if (q0 + i < p.Nq) p.bound[(static_cast<int64_t>(bh) * p.Nq + q0 + i) * p.topk] = __uint_as_float(~0u);
+        __threadfence();
+        __syncwarp();
+        griddep_launch();
+      }
       int pass = 0;
       while (another_pass(pass++)) {}
     }
@@ -416,8 +424,10 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
     if (ok && half == 0 && row < p.Nq) {
       float bound = INFINITY;
 #pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (i < p.topk) bound = fminf(bound, fmaxf(gm[i], other[(p.topk - 1 - i) * 128]));
+      for (int i = 0; i < 32; ++i) {
+        const float m = fmaxf(gm[i], other[max(p.topk - 1 - i, 0) * 128]);      // loaded in any case, so that no branch stands around it
+        bound = i < p.topk ? fminf(bound, m) : bound;
+      }
       // a sum's logarithm, less what its exponentials and the second kernel's scores can differ by: 2^-20 from the
       // exponentials, and roundings of the arguments, each below 2^-24 of their size.  The polynomial exponentials are 2^-126
       // for anything smaller: a sum in which two of those are more than 2^-21 bounds nothing.

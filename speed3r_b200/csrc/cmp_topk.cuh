@@ -170,8 +170,8 @@ __device__ __noinline__ void tk_exact(const uint2* la, int na, const uint2* lb, 
 }
 static_assert(kTkCap == 40, "tk_exact takes lists of up to 40, the packed words a place below 80");
 
-// Both kinds of CTA in one grid: a row's bound is there when its word is no longer what it was filled with (all bits set: a NaN
-// that no arithmetic returns).  For at most a second; called by whole warps.
+// A row's bound is there when its word is no longer what it was filled with (all bits set: a NaN that no arithmetic returns).  For
+// at most a second; called by whole warps.
 __device__ __forceinline__ bool wait_bound(const int32_t* word, bool mine, uint32_t& v, volatile uint32_t* abort_flag) {
   const uint64_t start = globaltimer_ns();
   while (true) {
@@ -187,8 +187,8 @@ __device__ __forceinline__ bool wait_bound(const int32_t* word, bool mine, uint3
   }
 }
 
-// `cta`: which R * 128 rows.  WAIT: in one grid with the CTAs that find the bounds.
-template <int R, int RANK, bool WAIT>
+// `cta`: which R * 128 rows.  ALONE: in a launch behind the kernel that finds the bounds, not in one grid with it.
+template <int R, int RANK, bool ALONE>
 __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUtensorMap& map_k, const TkParams& p, TkCtl& ctl,
                                              uint8_t* smem_raw, int cta) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -221,7 +221,10 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  griddep_wait();
+  // In a launch of its own this kernel starts once every CTA of the one before has filled its bounds' places, which those do when the
+  // pooled tensors are complete: copies and products begin at once, rows go on as their bounds come (waiting for that kernel's end
+  // instead took 1.5 us more), and that it has ended is waited for where the table is written.
+  if (!ALONE) griddep_wait();
   griddep_launch();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
@@ -298,8 +301,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     uint32_t base_key = 0;                       // every collected pair's key is at least this
     bool ok = true;
     uint32_t bound_word = 0;
-    if (WAIT) ok = wait_bound(out, row < p.Nq, bound_word, abort_flag);
-    else if (row < p.Nq) bound_word = static_cast<uint32_t>(*out);
+    ok = wait_bound(out, row < p.Nq, bound_word, abort_flag);
     if (ok && row < p.Nq) {
       const float bound = fmaxf(__uint_as_float(bound_word), -3.402823466e38f);
       base_key = sortable_key(bound == 0.f ? -0.f : bound);
@@ -451,8 +453,9 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     uint32_t a[32], e[kTkCap - 32];
     uint32_t top = 0;
     // keys above the bound's, plus one: an empty place is 0
+    // (loaded whether the place is filled or not: a choice between loads becomes a branch around each)
     auto word = [&](int i) {
-      const uint32_t d = i < cnt ? sortable_key(__uint_as_float(buf[i * 32].x)) - base_key + 1u : 0u;
+      const uint32_t k = sortable_key(__uint_as_float(buf[i * 32].x)) - base_key + 1u, d = i < cnt ? k : 0u;
       top = max(top, d);
       return d;
     };
@@ -486,6 +489,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
       for (int i = 0; i < 32; ++i) words[i * 128] = a[i];
       tell[1 * 128] = lost;
     }
+    if (ALONE) griddep_wait();
     meet();
     if (par == 0) {
       lost = max(lost, tell[1 * 128]);
@@ -534,8 +538,10 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const int place = 127 - static_cast<int>(a[i] & 127u);
-          a[i] = a[i] ? (place < kTkCap ? buf[place * 32].y : other[(place - kTkCap) * 32].y) : ~0u;
+          // one address and one load for either list and for empty places (place 127 -> 0)
+          const int place = a[i] ? 127 - static_cast<int>(a[i] & 127u) : 0;
+          const uint32_t col = buf[(place < kTkCap ? place : place + 3 * kTkCap) * 32].y;
+          a[i] = a[i] ? col : ~0u;
         }
       }
       if (ok && row < p.Nq) {

@@ -442,6 +442,24 @@ def test_cmp_one_and_two_row_tiles(heads):
     assert_bf16_close(o, ref, f"o_c {heads} heads")
 
 
+@pytest.mark.parametrize("heads, n", [(2, 130), (16, 128), (16, 1152), (12, 1500), (16, 2400)])
+def test_cmp_tables_of_calls_in_a_row(heads, n):
+    """The collection of a call's columns starts while its bounds are being found, and the next call while it runs: tables and outputs are
+    those of calls that have the GPU to themselves (one row tile per CTA, two, and both kinds in one grid)."""
+    from speed3r_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(n)
+    sets = [[torch.randn(1, heads, n, 64, device=DEV, generator=g).mul_(0.2 + 0.2 * i).bfloat16() for _ in range(3)] for i in range(6)]
+    alone = []
+    for x in sets:
+        torch.cuda.synchronize()
+        alone.append([t.clone() for t in ops.flash_attn_topk_func(*x, 32)])
+        torch.cuda.synchronize()
+    for _ in range(4):
+        for x, want in zip(sets, [list(ops.flash_attn_topk_func(*x, 32)) for x in sets]):
+            ref = alone[[a is x for a in sets].index(True)]
+            assert torch.equal(want[0], ref[0]) and torch.equal(want[1], ref[1])
+
+
 @pytest.mark.parametrize("period", [1, 16, 64])
 def test_cmp_table_when_the_bound_is_loose(period):
     """Keys that repeat with a period: the best logits fall into few of the 64 column groups, so that far more logits than
