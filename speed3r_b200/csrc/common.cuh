@@ -373,6 +373,12 @@ __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st
 __device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
 }
+// Appends a pair at `at` where `on` is not 0, and moves `at` by STEP bytes: predicated, where the compiler would branch.
+template <int STEP>
+__device__ __forceinline__ void sts64_append(uint32_t on, uint32_t& at, uint32_t x, uint32_t y) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p st.shared.v2.b32 [%0], {%2, %3};\n\t@p add.u32 %0, %0, %4;\n\t}"
+               : "+r"(at) : "r"(on), "r"(x), "r"(y), "n"(STEP) : "memory");
+}
 __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
