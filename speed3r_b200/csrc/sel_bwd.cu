@@ -361,42 +361,52 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
 #pragma unroll
     for (int i = 0; i < 4; ++i) { oc[2 * i] = bf16_lo(w[i]); oc[2 * i + 1] = bf16_hi(w[i]); acc[2 * i] = acc[2 * i + 1] = 0.f; }
   }
-  for (int t0 = 0; t0 < p.block; t0 += 4) {
-    const int t = m * p.block + t0 + sub;
-    const bool live = (t0 + sub < p.block) && (t < p.Tq);
-    float dyv[8] = {}, osv[8] = {}, g0 = 0.f, g1 = 0.f;
-    if (live) {
-      const uint4 a = *reinterpret_cast<const uint4*>(p.dy + ((static_cast<int64_t>(b) * p.Tq + t) * p.H + h) * 64 + c8 * 8);
-      const uint4 s = *reinterpret_cast<const uint4*>(p.o_s + (static_cast<int64_t>(bh) * p.Tq + t) * 64 + c8 * 8);
-      const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, sw[4] = {s.x, s.y, s.z, s.w};
+  for (int base = 0; base < p.block; base += 16) {
+    // 16 tokens' loads are under way before the first is used
+    uint4 a[4], s[4];
+    uint32_t gw[4];
+    bool live[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int in_block = base + 4 * u + sub, t = m * p.block + in_block;
+      live[u] = in_block < p.block && t < p.Tq;
+      const int tc = min(t, p.Tq - 1);                       // loaded in any case
+      a[u] = __ldg(reinterpret_cast<const uint4*>(p.dy + ((static_cast<int64_t>(b) * p.Tq + tc) * p.H + h) * 64 + c8 * 8));
+      s[u] = __ldg(reinterpret_cast<const uint4*>(p.o_s + (static_cast<int64_t>(bh) * p.Tq + tc) * 64 + c8 * 8));
+      gw[u] = __ldg(reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + tc * p.gst));
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = m * p.block + base + 4 * u + sub;
+      const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, sw[4] = {s[u].x, s[u].y, s[u].z, s[u].w};
+      float dyv[8], osv[8];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        dyv[2 * i] = bf16_lo(aw[i]); dyv[2 * i + 1] = bf16_hi(aw[i]);
+        dyv[2 * i] = live[u] ? bf16_lo(aw[i]) : 0.f; dyv[2 * i + 1] = live[u] ? bf16_hi(aw[i]) : 0.f;
         osv[2 * i] = bf16_lo(sw[i]); osv[2 * i + 1] = bf16_hi(sw[i]);
       }
-      const uint32_t gw = *reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + t * p.gst);
-      g0 = bf16_lo(gw); g1 = bf16_hi(gw);
-    }
-    float d0 = 0.f, d1 = 0.f;
+      const float g0 = live[u] ? bf16_lo(gw[u]) : 0.f, g1 = bf16_hi(gw[u]);
+      float d0 = 0.f, d1 = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      d0 += dyv[i] * oc[i];
-      d1 += dyv[i] * osv[i];
-      acc[i] += g0 * dyv[i];
-    }
+      for (int i = 0; i < 8; ++i) {
+        d0 += dyv[i] * oc[i];
+        d1 += dyv[i] * osv[i];
+        acc[i] += g0 * dyv[i];
+      }
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-      d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-      d1 += __shfl_xor_sync(0xffffffffu, d1, o);
-    }
-    if (live) {
-      uint4 out;
-      out.x = pack_bf16(g1 * dyv[0], g1 * dyv[1]); out.y = pack_bf16(g1 * dyv[2], g1 * dyv[3]);
-      out.z = pack_bf16(g1 * dyv[4], g1 * dyv[5]); out.w = pack_bf16(g1 * dyv[6], g1 * dyv[7]);
-      *reinterpret_cast<uint4*>(p.do_s + (static_cast<int64_t>(bh) * p.Tq + t) * 64 + c8 * 8) = out;
-      if (c8 == 0) {
-        *reinterpret_cast<float2*>(p.dgate + (static_cast<int64_t>(bh) * p.Tq + t) * 2) = make_float2(d0, d1);
-        p.delta_s[static_cast<int64_t>(bh) * p.Tq + t] = g1 * d1;
+      for (int o = 1; o < 8; o <<= 1) {
+        d0 += __shfl_xor_sync(0xffffffffu, d0, o);
+        d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+      }
+      if (live[u]) {
+        uint4 out;
+        out.x = pack_bf16(g1 * dyv[0], g1 * dyv[1]); out.y = pack_bf16(g1 * dyv[2], g1 * dyv[3]);
+        out.z = pack_bf16(g1 * dyv[4], g1 * dyv[5]); out.w = pack_bf16(g1 * dyv[6], g1 * dyv[7]);
+        *reinterpret_cast<uint4*>(p.do_s + (static_cast<int64_t>(bh) * p.Tq + t) * 64 + c8 * 8) = out;
+        if (c8 == 0) {
+          *reinterpret_cast<float2*>(p.dgate + (static_cast<int64_t>(bh) * p.Tq + t) * 2) = make_float2(d0, d1);
+          p.delta_s[static_cast<int64_t>(bh) * p.Tq + t] = g1 * d1;
+        }
       }
     }
   }
