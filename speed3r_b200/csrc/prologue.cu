@@ -95,18 +95,40 @@ __device__ __forceinline__ Vec8 lds_vec8(uint32_t a) {
 // LayerNorm over the 64 channels held by 8 lanes (8 each), fp32, two passes; the caller rounds to bf16.
 // `gmask` names the 8 lanes of the row: rows of one warp may belong to different tensors (q, k or v) and
 // take different paths, so every shuffle synchronises its own group only.
-__device__ __forceinline__ void ln_row(float2 (&x)[4], const float2 (&w)[4], const float2 (&b)[4], float eps, uint32_t gmask) {
-  const float2 s = fadd2(fadd2(x[0], x[1]), fadd2(x[2], x[3]));
-  const float mean = sum8(s.x + s.y, gmask) * (1.f / 64.f);
-  float2 v = make_float2(0.f, 0.f);
+// G rows side by side: the shuffles and the root of one are a chain, which the other's instructions fill.
+template <int G>
+__device__ __forceinline__ void ln_rows(float2 (&x)[G][4], const float2 (&w)[4], const float2 (&b)[4], float eps, uint32_t gmask) {
+  float m[G];
+  auto sums8 = [&]() {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    x[i] = fadd2(x[i], splat(-mean));
-    v = ffma2(x[i], x[i], v);
+    for (int d = 1; d < 8; d <<= 1)
+#pragma unroll
+      for (int u = 0; u < G; ++u) m[u] += __shfl_xor_sync(gmask, m[u], d);
+  };
+#pragma unroll
+  for (int u = 0; u < G; ++u) {
+    const float2 s = fadd2(fadd2(x[u][0], x[u][1]), fadd2(x[u][2], x[u][3]));
+    m[u] = s.x + s.y;
   }
-  const float rstd = rsqrtf(sum8(v.x + v.y, gmask) * (1.f / 64.f) + eps);
+  sums8();
 #pragma unroll
-  for (int i = 0; i < 4; ++i) x[i] = ffma2(fmul2(x[i], splat(rstd)), w[i], b[i]);   // rounded to bf16 when packed
+  for (int u = 0; u < G; ++u) {
+    const float mean = m[u] * (1.f / 64.f);
+    float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[u][i] = fadd2(x[u][i], splat(-mean));
+      v = ffma2(x[u][i], x[u][i], v);
+    }
+    m[u] = v.x + v.y;
+  }
+  sums8();
+#pragma unroll
+  for (int u = 0; u < G; ++u) {
+    const float rstd = rsqrtf(m[u] * (1.f / 64.f) + eps);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[u][i] = ffma2(fmul2(x[u][i], splat(rstd)), w[i], b[i]);   // rounded to bf16 when packed
+  }
 }
 
 // 2-D rotary embedding of a row held by 8 lanes, on packed bf16 pairs: lanes 0-3 hold the y half (32
@@ -122,25 +144,33 @@ __device__ __forceinline__ uint32_t bf2_add(uint32_t a, uint32_t b) {
   const __nv_bfloat162 r = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-__device__ __forceinline__ void rope_row(uint32_t (&xw)[4], const Vec8& c, const Vec8& s, int l8, uint32_t gmask) {
+template <int G>
+__device__ __forceinline__ void rope_rows(Vec8 (&o)[G], const Vec8 (&c)[G], const Vec8 (&s)[G], int l8, uint32_t gmask) {
   const uint32_t flip = (l8 & 2) == 0 ? 0x80008000u : 0u;
 #pragma unroll
-  for (int wd = 0; wd < 4; ++wd) {
-    const uint32_t other = __shfl_xor_sync(gmask, xw[wd], 2) ^ flip;
-    xw[wd] = bf2_add(bf2_mul(xw[wd], c.w[wd]), bf2_mul(other, s.w[wd]));
-  }
+  for (int wd = 0; wd < 4; ++wd)
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      const uint32_t other = __shfl_xor_sync(gmask, o[u].w[wd], 2) ^ flip;
+      o[u].w[wd] = bf2_add(bf2_mul(o[u].w[wd], c[u].w[wd]), bf2_mul(other, s[u].w[wd]));
+    }
 }
 
 // A CTA has up to 16 of the block's 3H rows (8 lanes each: four warps, one per scheduler).  A thread's share of 16 tokens is on
-// its way at once, 16 bytes a token in slots of its own in shared memory (cp.async; nobody else reads them, so there is no
-// barrier): 32 KB per CTA and six CTAs per SM keep 192 KB in flight.  16 heads, 252000 tokens: 628 us, 0.78 of the copy rate
-// (24 KB in flight, the next tokens' loads in registers: 759; four tokens ahead and the tables' rows found by every row: 908);
-// 24 rows per CTA 656 us, eight CTAs of 64 registers 804.
-constexpr int kProRows = 16, kProThreads = kProRows * 8, kProChunk = 16, kProCtas = 6, kProBwdCtas = 4;
+// its way at once, 16 bytes a token in slots of its own in shared memory (cp.async; nobody else reads them): 32 KB per CTA.
+// Bound: HBM on long sequences (0.8 of the copy rate), on short ones the chain of a token - two sums over eight lanes, a root, a
+// rotation - of which one after the other took 980 cycles with two or three warps per scheduler.  Four tokens go through it side by
+// side, with their table rows in shared memory, in four CTAs of 128 registers per SM (one by one in six of 80; two in five of 102 as
+// fast but for the short ones).  16 heads, one by one -> now: in the module at 2048 tokens 12.8 -> 8.8 us, 2 x 6144 37.9 -> 36.2,
+// 64 512 172.7 -> 162.3 (by itself, 1.8 GHz).  Earlier forms, 252 000 tokens: six CTAs 628 us, 24 KB in flight, the next tokens' loads
+// in registers 759, four tokens ahead and the tables' rows found by every row 908, 24 rows per CTA 656, eight CTAs of 64 registers 804.
+constexpr int kProRows = 16, kProThreads = kProRows * 8, kProChunk = 16, kProCtas = 4, kProBwdCtas = 4;
 constexpr int kProRingBytes = kProChunk * kProThreads * 16;
+constexpr int kProTabBytes = (kProChunk + 1) * 256;    // cos (y, x) and sin (y, x) of a chunk's tokens and of the block's mean, 64 bytes each
 
 template <bool LONG>
 __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(const PrologueParams p) {
+  constexpr int G = LONG ? 1 : 4;                      // tokens side by side
   extern __shared__ __align__(16) uint8_t smem[];      // [token of the chunk][thread] 16 bytes; [warp] rows of the tables
   griddep_wait();
   griddep_launch();
@@ -161,7 +191,8 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   const __nv_bfloat16* src = p.qkv + tok0 * p.tok_stride + g * 64 + l8 * 8;
   __nv_bfloat16* dst = out + (bh * p.N + n0) * 64 + l8 * 8;
   const uint32_t slots = smem_u32(smem) + threadIdx.x * 16;
-  int* rows = reinterpret_cast<int*>(smem + kProRingBytes) + (threadIdx.x >> 5) * 2 * (LONG ? 1 : p.block + 1);
+  const uint32_t tab = smem_u32(smem) + kProRingBytes;
+  int* rows = reinterpret_cast<int*>(smem + kProRingBytes + kProTabBytes) + (threadIdx.x >> 5) * 2 * (LONG ? 1 : p.block + 1);
   // two groups of loads per chunk: the first half is worked on while the second arrives
   auto fetch = [&](int t0) {
 #pragma unroll
@@ -172,69 +203,116 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
     cp_async_commit();
   };
   fetch(0);
-  if (p.pos != nullptr) block_rows<LONG>(rows, p.pos + tok0 * 2, p.block, p.tab_rows, p.status, lane);
-  if (!live) return;
+  // the gate's logits, as many as two per thread, are asked for here and used behind the rows' positions
+  const int gates = p.gate_in != nullptr && blockIdx.y == 0 ? p.block * p.H : 0;
+  auto gate_logits = [&](int i) { return __ldg(reinterpret_cast<const uint32_t*>(p.gate_in + (tok0 + i % p.block) * p.tok_stride) + i / p.block); };
+  uint32_t logits[2] = {0u, 0u};
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int i = threadIdx.x + u * kProThreads;
+    if (i < gates) logits[u] = gate_logits(i);
+  }
   float2 w[4], bias[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     w[i] = norm ? __ldg(reinterpret_cast<const float2*>(lw) + l8 * 4 + i) : splat(1.f);
     bias[i] = norm ? __ldg(reinterpret_cast<const float2*>(lb) + l8 * 4 + i) : splat(0.f);
   }
+  if (p.pos != nullptr) block_rows<LONG>(rows, p.pos + tok0 * 2, p.block, p.tab_rows, p.status, lane);
+  auto put_gate = [&](int i, uint32_t v) {
+    const float g0 = 1.f / (1.f + __expf(-bf16_lo(v))), g1 = 1.f / (1.f + __expf(-bf16_hi(v)));
+    p.gate[(static_cast<int64_t>(b) * p.H + i / p.block) * p.N + n0 + i % p.block] = pack_bf16(g0, g1);
+  };
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int i = threadIdx.x + u * kProThreads;
+    if (i < gates) put_gate(i, logits[u]);
+  }
+  for (int i = threadIdx.x + 2 * kProThreads; i < gates; i += kProThreads) put_gate(i, gate_logits(i));
+  // Table rows of a chunk's tokens to shared memory, for all rows of the CTA: asked for by every row as it came to a token, they
+  // were a trip to L2 per pair of tokens on a grid too small to fill it with others' work.
+  auto tables = [&](int t0) {
+    const int n = min(kProChunk, p.block - t0);
+    for (int i = threadIdx.x; i < 16 * (n + (t0 == 0)); i += kProThreads) {
+      const bool mean = i >= 16 * n;
+      const int row = rows[(mean ? 0 : 2 + 2 * (t0 + (i >> 4))) + ((i >> 2) & 1)];
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>((i & 8 ? p.sin_tab : p.cos_tab) + row * 32 + (i & 3) * 8));
+      sts128(tab + (mean ? kProChunk : i >> 4) * 256 + (i & 15) * 16, v.x, v.y, v.z, v.w);
+    }
+  };
   const int* my_row = rows + (l8 >> 2);                // y for lanes 0-3, x for 4-7
   const __nv_bfloat16 *cos_l = p.cos_tab + (l8 & 3) * 8, *sin_l = p.sin_tab + (l8 & 3) * 8;
-  auto row_of = [&](int t) { return LONG ? table_row(__ldg(p.pos + (tok0 + t) * 2 + (l8 >> 2)), p.tab_rows) : my_row[2 + 2 * t]; };
+  auto row_of = [&](int t) { return table_row(__ldg(p.pos + (tok0 + t) * 2 + (l8 >> 2)), p.tab_rows); };
 
   float2 acc[4] = {splat(0.f), splat(0.f), splat(0.f), splat(0.f)};
-  // one token of this row: accumulate the raw block sum, normalise, rotate, store
-  auto token = [&](int t, int slot) {
-    Vec8 c, s, o = lds_vec8(slots + slot * (kProThreads * 16));
-    if (rope) {
-      const int row = row_of(t) * 32;
-      c = ldg_vec8(cos_l + row);
-      s = ldg_vec8(sin_l + row);
-    }
-    float2 x[4];
-    unpack8(x, o);
+  // G tokens of this row: accumulate the raw block sum, normalise, rotate, store
+  auto tokens = [&](int t, int slot) {
+    Vec8 c[G], s[G], o[G];
+    float2 x[G][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i] = fadd2(acc[i], x[i]);
-    if (norm) {
-      ln_row(x, w, bias, p.eps, gmask);
-      o = pack8(x);
+    for (int u = 0; u < G; ++u) {
+      const int at = min(slot + u, kProChunk - 1);
+      o[u] = lds_vec8(slots + at * (kProThreads * 16));
+      if (rope && LONG) {
+        const int row = row_of(min(t + u, p.block - 1)) * 32;
+        c[u] = ldg_vec8(cos_l + row);
+        s[u] = ldg_vec8(sin_l + row);
+      } else if (rope) {
+        c[u] = lds_vec8(tab + at * 256 + l8 * 16);
+        s[u] = lds_vec8(tab + at * 256 + 128 + l8 * 16);
+      }
     }
-    if (rope) rope_row(o.w, c, s, l8, gmask);
-    *reinterpret_cast<Vec8*>(dst + t * 64) = o;
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      unpack8(x[u], o[u]);
+      if (t + u < p.block) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] = fadd2(acc[i], x[u][i]);
+      }
+    }
+    if (norm) {
+      ln_rows<G>(x, w, bias, p.eps, gmask);
+#pragma unroll
+      for (int u = 0; u < G; ++u) o[u] = pack8(x[u]);
+    }
+    if (rope) rope_rows<G>(o, c, s, l8, gmask);
+#pragma unroll
+    for (int u = 0; u < G; ++u)
+      if (t + u < p.block) *reinterpret_cast<Vec8*>(dst + (t + u) * 64) = o[u];
   };
   for (int t0 = 0; t0 < p.block; t0 += kProChunk) {
     const int n = min(kProChunk, p.block - t0);
-    cp_async_wait<1>();
-#pragma unroll 2
-    for (int i = 0; i < min(n, kProChunk / 2); ++i) token(t0 + i, i);
-    cp_async_wait<0>();
-#pragma unroll 2
-    for (int i = kProChunk / 2; i < n; ++i) token(t0 + i, i);
-    if (t0 + kProChunk < p.block) fetch(t0 + kProChunk);
+    if (!LONG && p.pos != nullptr) {
+      if (t0 > 0) __syncthreads();                     // the chunk before has been used
+      tables(t0);
+      __syncthreads();
+    }
+    if (live) {
+      cp_async_wait<1>();
+#pragma unroll 1
+      for (int i = 0; i < n; i += G) {
+        if (i == kProChunk / 2) cp_async_wait<0>();
+        tokens(t0 + i, i);
+      }
+      if (t0 + kProChunk < p.block) fetch(t0 + kProChunk);
+    }
   }
+  if (!live) return;
   // compression branch: mean of the raw rows, then the same norm and the rotary embedding at the block's
   // mean position
   const float inv = 1.f / static_cast<float>(p.block);
-  float2 x[4];
+  float2 x[1][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) x[i] = make_float2(bf16r(acc[i].x * inv), bf16r(acc[i].y * inv));
-  if (norm) ln_row(x, w, bias, p.eps, gmask);
-  Vec8 o = pack8(x);
+  for (int i = 0; i < 4; ++i) x[0][i] = make_float2(bf16r(acc[i].x * inv), bf16r(acc[i].y * inv));
+  if (norm) ln_rows<1>(x, w, bias, p.eps, gmask);
+  Vec8 o[1] = {pack8(x[0])};
   if (rope) {
     const int row = my_row[0] * 32;
-    rope_row(o.w, ldg_vec8(cos_l + row), ldg_vec8(sin_l + row), l8, gmask);
+    const Vec8 c[1] = {LONG ? ldg_vec8(cos_l + row) : lds_vec8(tab + kProChunk * 256 + l8 * 16)},
+               s[1] = {LONG ? ldg_vec8(sin_l + row) : lds_vec8(tab + kProChunk * 256 + 128 + l8 * 16)};
+    rope_rows<1>(o, c, s, l8, gmask);
   }
-  *reinterpret_cast<Vec8*>(out_c + (bh * p.Nc + j) * 64 + l8 * 8) = o;
-  if (p.gate_in != nullptr && blockIdx.y == 0) {
-    for (int i = threadIdx.x; i < p.block * p.H; i += min(kProThreads, 3 * p.H * 8)) {
-      const int t = i % p.block, hd = i / p.block;
-      const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(p.gate_in + (tok0 + t) * p.tok_stride) + hd);
-      const float g0 = 1.f / (1.f + __expf(-bf16_lo(v))), g1 = 1.f / (1.f + __expf(-bf16_hi(v)));
-      p.gate[(static_cast<int64_t>(b) * p.H + hd) * p.N + n0 + t] = pack_bf16(g0, g1);
-    }
-  }
+  *reinterpret_cast<Vec8*>(out_c + (bh * p.Nc + j) * 64 + l8 * 8) = o[0];
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -518,7 +596,7 @@ static int prologue_fwd(const void* qkv, int64_t tok_stride, const void* gate_in
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_qkv_prologue_fwd: could not resolve the device status word");
   bool lengthy;
-  const int smem = prologue_smem(kProRingBytes, block, &lengthy);
+  const int smem = prologue_smem(kProRingBytes + kProTabBytes, block, &lengthy);
   auto* kernel = lengthy ? prologue_fwd_kernel<true> : prologue_fwd_kernel<false>;
   S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
   return launch(kernel, dim3(static_cast<unsigned>(grid), prologue_parts(H)), kProThreads, smem,

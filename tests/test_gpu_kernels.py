@@ -624,6 +624,25 @@ def test_prologue_backward(B, H, Bs, blocks, norm, rope):
                 assert (a.grad.cpu() - r.grad).abs().max() <= 2e-3 * max(1.0, r.grad.abs().max().item())
 
 
+@pytest.mark.parametrize("Bs, blocks", [(1, 40), (3, 5), (16, 9), (18, 4), (35, 3)])
+@pytest.mark.parametrize("norm, rope", [(True, True), (False, True), (True, False)])
+def test_prologue_forward_blocks(Bs, blocks, norm, rope):
+    """Blocks that are no multiple of the four tokens a row takes side by side, nor of the 16 of a chunk; 21 rows, so that a CTA has some
+    that do not exist; tokens and means against fp32."""
+    import speed3r_b200
+    from speed3r_b200 import ops
+    B, H, N = 2, 7, Bs * blocks
+    qkv, = bf16_round(1.5 * randn(30, B, N, 3 * H * 64) + 0.3)
+    pos = torch.randint(0, 37, (B, N, 2), generator=torch.Generator().manual_seed(2)) if rope else None
+    cos, sin = speed3r_b200.RoPE2D(100.0)._cos_sin(32, 37, torch.device(DEV), torch.bfloat16)
+    wb = [(1 + 0.2 * randn(31 + i, 64), 0.1 * randn(33 + i, 64)) if norm else None for i in range(2)]
+    got = ops.qkv_prologue(qkv.to(DEV, torch.bfloat16), H, Bs, pos.to(DEV) if rope else None, cos if rope else None, sin if rope else None,
+                           *[(w[0].to(DEV), w[1].to(DEV), 1e-5) if norm else None for w in wb])
+    # positions of the means are truncated, and the means rounded to bf16 in front of the norm: two roundings of 2^-9 of values up to ~6
+    for name, a, b in zip(("q", "k", "v", "q_c", "k_c", "v_c"), got, _prologue_fp32(qkv, H, Bs, pos, cos, sin, *wb)):
+        assert_bf16_close(a, b, f"{name} {Bs}")
+
+
 def _prologue_fp32(qkv, H, Bs, pos, cos, sin, qn, kn):
     """Split, LayerNorm, rotary embedding and pooling in fp32 with the given (bf16) rotary tables."""
     B, N, d = qkv.shape[0], qkv.shape[1], 64
