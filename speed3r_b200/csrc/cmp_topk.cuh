@@ -438,10 +438,13 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     const int cnt = static_cast<int>(at - first) >> 8;
     const int r = quarter * 32 + lane;
     // Q and the K ring are idle once every scan warp is here (whatever happened): per row tile 32 words per row for sorted
-    // words and columns, and two per row for what its threads tell each other
+    // words and columns, and four per row for what its threads tell each other
     asm volatile("bar.sync 3, %0;" ::"n"(256 * R) : "memory");
-    uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (sbase - smem_u32(smem_raw))) + t * (35 * 128) + r;   // [place][row]
-    uint32_t* tell = words + 32 * 128;         // [list][row] largest key, [2][row] the second list's length
+    uint32_t* words = reinterpret_cast<uint32_t*>(smem_raw + (sbase - smem_u32(smem_raw))) + t * (36 * 128) + r;   // [place][row]
+    static_assert(R * 36 * 128 * 4 <= C::kOffBuf, "the lists behind Q and the K ring are still in use");
+    // [list][row] largest key (later [0]: whether the row's words are columns already), [2][row] the second list's length, [3][row] the
+    // largest word that it lost.  Between two meetings no word is both written and read: nothing else orders a row's two threads.
+    uint32_t* tell = words + 32 * 128;
     auto meet = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + t) : "memory"); };
     uint32_t a[32], e[kTkCap - 32];
     uint32_t top = 0;
@@ -480,12 +483,12 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     if (par == 1) {
 #pragma unroll
       for (int i = 0; i < 32; ++i) words[i * 128] = a[i];
-      tell[1 * 128] = lost;
+      tell[3 * 128] = lost;
     }
     if (ALONE) griddep_wait();
     meet();
     if (par == 0) {
-      lost = max(lost, tell[1 * 128]);
+      lost = max(lost, tell[3 * 128]);
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         const uint32_t o = words[(31 - i) * 128];

@@ -49,6 +49,29 @@ def test_draining_after_a_wait_that_gave_up_signals_no_result(path):
     assert drains and not drains & waited, f"{os.path.basename(path)}: {drains & waited}"
 
 
+def test_a_rows_two_threads_do_not_overwrite_what_they_tell_each_other():
+    """End of the collection: a row's two threads exchange words between meetings, the only thing that orders them.  A word that one of
+    them reads between two meetings is written in front of the first or behind the second."""
+    src = code(os.path.join(CSRC, "cmp_topk.cuh"))
+    src = src[src.index("uint32_t* tell = words"):]
+    src = src[src.index(";") + 1:]
+
+    def words_of(index):
+        if "par" in index:                     # either thread's own or the other's largest key
+            return {0, 1}
+        return {eval(index) // 128}
+
+    phases, seen = src.split("meet();"), set()
+    assert len(phases) == 4
+    for n, phase in enumerate(phases):
+        written, read = set(), set()
+        for m in re.finditer(r"\btell\[([^\]]*)\](\s*=(?!=))?", phase):
+            (written if m.group(2) else read).update(words_of(m.group(1)))
+        assert not written & read, f"words {written & read} between meetings {n} and {n + 1}"
+        assert read <= seen
+        seen |= written
+
+
 def test_polynomial_exponential_is_as_exact_as_stated():
     """2^f on [-1/2, 1/2] with the coefficients of exp2_fma2, in 64 bits and with every step rounded to fp32."""
     import numpy as np
