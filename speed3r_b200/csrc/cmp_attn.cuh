@@ -84,9 +84,8 @@ struct AtParams {
   uint32_t* status;
 };
 
-// `cta`: which R * 128 rows.  FILL: the second kernel is a launch of its own, which starts early and waits for the bounds as they come:
-// a bound's place gets what it waits on (all bits set) before this CTA lets that kernel start.
-template <int R, int RANK, bool FILL>
+// `cta`: which R * 128 rows
+template <int R, int RANK>
 __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
                                              const CUtensorMap& map_ks, const CUtensorMap& map_vs, const AtParams& p, AtCtl& ctl,
                                              uint8_t* smem_raw, int cta) {
@@ -127,7 +126,7 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
   __syncthreads();
   tc_fence_after();
   griddep_wait();
-  if (!FILL) griddep_launch();
+  griddep_launch();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
 
@@ -243,13 +242,6 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
         }
       } while (another_pass(pass++));
     } else {
-      if (FILL && warp == 3) {                 // the bounds themselves are written behind another_pass
-        for (int i = lane; i < R * 128; i += 32)
-          if (q0 + i < p.Nq) p.bound[(static_cast<int64_t>(bh) * p.Nq + q0 + i) * p.topk] = __uint_as_float(~0u);
-        __threadfence();
-        __syncwarp();
-        griddep_launch();
-      }
       int pass = 0;
       while (another_pass(pass++)) {}
     }

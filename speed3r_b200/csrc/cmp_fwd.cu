@@ -10,14 +10,14 @@ __global__ void __launch_bounds__(AtCfg<R>::kThreads, 1)
 cmp_attn_kernel(const __grid_constant__ CmpMaps m, const __grid_constant__ AtParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ AtCtl ctl;
-  cmp_attn_cta<R, RANK, true>(m.q, m.k, m.v, m.ks, m.vs, p, ctl, smem_raw, blockIdx.x);
+  cmp_attn_cta<R, RANK>(m.q, m.k, m.v, m.ks, m.vs, p, ctl, smem_raw, blockIdx.x);
 }
 template <int R, int RANK>
 __global__ void __launch_bounds__(TkCfg<R>::kThreads, 1)
 cmp_topk_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ TkParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ TkCtl ctl;
-  cmp_topk_cta<R, RANK, true>(map_q, map_k, p, ctl, smem_raw, blockIdx.x);
+  cmp_topk_cta<R, RANK, false>(map_q, map_k, p, ctl, smem_raw, blockIdx.x);
 }
 
 // Both in one grid, all of the attention's CTAs first.  With more row tiles than SMs the last wave of either leaves SMs idle
@@ -35,15 +35,13 @@ cmp_both_kernel(const __grid_constant__ CmpMaps m, const __grid_constant__ AtPar
     TkCtl topk;
   } ctl;
   if (static_cast<int>(blockIdx.x) < attn_ctas)
-    cmp_attn_cta<2, RANK, false>(m.q, m.k, m.v, m.ks, m.vs, pa, ctl.attn, smem_raw, blockIdx.x);
+    cmp_attn_cta<2, RANK>(m.q, m.k, m.v, m.ks, m.vs, pa, ctl.attn, smem_raw, blockIdx.x);
   else
-    cmp_topk_cta<2, RANK, false>(m.q, m.k, pt, ctl.topk, smem_raw, static_cast<int>(blockIdx.x) - attn_ctas);
+    cmp_topk_cta<2, RANK, true>(m.q, m.k, pt, ctl.topk, smem_raw, static_cast<int>(blockIdx.x) - attn_ctas);
 }
 static_assert(AtCfg<2>::kThreads == TkCfg<2>::kThreads && AtCfg<2>::kSmem <= TkCfg<2>::kSmem, "one launch shape for both kinds");
 
-// Two launches where all row tiles fit the GPU at once.  The second one's CTAs take the SMs that the first leaves idle while it runs, and
-// have their keys and first products when the bounds come.  Both kernels, 16 heads, the second waiting for the end of the first -> for
-// its bounds: 2 x 384 x 384 20.6 -> 20.1 us, 1024 x 1024 36.2 -> 34.6; the op at 2048 tokens 45.5 -> 44.2.
+// Two launches where all row tiles fit the GPU at once.
 template <int R, int RANK>
 static int launch_cmp_apart(const CmpMaps& m, const AtParams& a, const TkParams& t, int64_t ctas, cudaStream_t st) {
   S3R_CUDA(cudaFuncSetAttribute(cmp_attn_kernel<R, RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, AtCfg<R>::kSmem));

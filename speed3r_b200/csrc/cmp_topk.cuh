@@ -171,8 +171,8 @@ __device__ __noinline__ void tk_exact(const uint2* la, int na, const uint2* lb, 
 }
 static_assert(kTkCap == 40, "tk_exact takes lists of up to 40, the packed words a place below 80");
 
-// A row's bound is there when its word is no longer what it was filled with (all bits set: a NaN that no arithmetic returns).  For
-// at most a second; called by whole warps.
+// Both kinds of CTA in one grid: a row's bound is there when its word is no longer what it was filled with (all bits set: a NaN
+// that no arithmetic returns).  For at most a second; called by whole warps.
 __device__ __forceinline__ bool wait_bound(const int32_t* word, bool mine, uint32_t& v, volatile uint32_t* abort_flag) {
   const uint64_t start = globaltimer_ns();
   while (true) {
@@ -188,8 +188,8 @@ __device__ __forceinline__ bool wait_bound(const int32_t* word, bool mine, uint3
   }
 }
 
-// `cta`: which R * 128 rows.  ALONE: in a launch behind the kernel that finds the bounds, not in one grid with it.
-template <int R, int RANK, bool ALONE>
+// `cta`: which R * 128 rows.  WAIT: in one grid with the CTAs that find the bounds.
+template <int R, int RANK, bool WAIT>
 __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUtensorMap& map_k, const TkParams& p, TkCtl& ctl,
                                              uint8_t* smem_raw, int cta) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -222,10 +222,10 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // In a launch of its own this kernel starts once every CTA of the one before has filled its bounds' places, which those do when the
-  // pooled tensors are complete: copies and products begin at once, rows go on as their bounds come (waiting for that kernel's end
-  // instead took 1.5 us more), and that it has ended is waited for where the table is written.
-  if (!ALONE) griddep_wait();
+  // In a launch of its own this kernel could begin with its copies and products before the attention has ended, and wait for the bounds
+  // as they come, in places that the attention fills before it lets this launch start.  The op at 2048 tokens took 1.3 us less that way,
+  // but nothing documents what a grid sees of others in front of this wait, and a place's old content taken for a bound is a wrong table.
+  griddep_wait();
   griddep_launch();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
@@ -302,7 +302,8 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     uint32_t base_key = 0;                       // every collected pair's key is at least this
     bool ok = true;
     uint32_t bound_word = 0;
-    ok = wait_bound(out, row < p.Nq, bound_word, abort_flag);
+    if (WAIT) ok = wait_bound(out, row < p.Nq, bound_word, abort_flag);
+    else if (row < p.Nq) bound_word = static_cast<uint32_t>(*out);
     if (ok && row < p.Nq) {
       const float bound = fmaxf(__uint_as_float(bound_word), -3.402823466e38f);
       base_key = sortable_key(bound == 0.f ? -0.f : bound);
@@ -485,7 +486,6 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
       for (int i = 0; i < 32; ++i) words[i * 128] = a[i];
       tell[3 * 128] = lost;
     }
-    if (ALONE) griddep_wait();
     meet();
     if (par == 0) {
       lost = max(lost, tell[3 * 128]);

@@ -61,8 +61,7 @@ int sm_count();
 
 #ifdef __CUDACC__
 // Launch of a kernel whose CTAs may start while the kernel before it in the stream is still finishing (programmatic
-// stream serialisation).  Every thread of such a kernel calls griddep_wait() before its first access to global memory (the
-// collection of the table begins with what was complete before the kernel in front of it could start another);
+// stream serialisation).  Every thread of such a kernel calls griddep_wait() before its first access to global memory;
 // what comes before - barriers, tensor memory, index arithmetic - then overlaps the other kernel's last CTAs.  On a short
 // sequence a call is a chain of kernels of 3 to 25 us, whose starts and ends are a good part of it.
 template <typename... P, typename... A>

@@ -444,7 +444,7 @@ def test_cmp_one_and_two_row_tiles(heads):
 
 @pytest.mark.parametrize("heads, n", [(2, 130), (16, 128), (16, 1152), (12, 1500), (16, 2400)])
 def test_cmp_tables_of_calls_in_a_row(heads, n):
-    """The collection of a call's columns starts while its bounds are being found, and the next call while it runs: tables and outputs are
+    """A kernel's CTAs start while the one in front is still finishing, within a call and between calls: tables and outputs are
     those of calls that have the GPU to themselves (one row tile per CTA, two, and both kinds in one grid)."""
     from speed3r_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(n)
@@ -458,6 +458,42 @@ def test_cmp_tables_of_calls_in_a_row(heads, n):
         for x, want in zip(sets, [list(ops.flash_attn_topk_func(*x, 32)) for x in sets]):
             ref = alone[[a is x for a in sets].index(True)]
             assert torch.equal(want[0], ref[0]) and torch.equal(want[1], ref[1])
+
+
+@pytest.mark.parametrize("take", [0, 3])
+@pytest.mark.parametrize("heads, n", [(2, 130), (16, 128), (8, 600), (24, 700), (170, 130)])
+def test_cmp_tables_of_operands_just_written_over_stale_tables(heads, n, take):
+    """What a call reads is what the kernels directly in front of it wrote, and its bounds are this call's: the operands' buffers get
+    other values in front of every call, and the table words that, taken for a bound, would let no key through.  Columns and blocks; one
+    row tile per CTA, two, and both kinds in one grid."""
+    from speed3r_b200 import _lib
+    sets = [bf16_round(*((0.5 + 0.5 * i) * randn(10 * i + j, 1, heads, n, 64) for j in range(3))) for i in range(4)]
+    dev = [[t.to(DEV, torch.bfloat16) for t in x] for x in sets]
+    q, k, v, o = (torch.empty_like(dev[0][0]) for _ in range(4))
+    lse = torch.empty(1, heads, n, device=DEV)
+    idx = torch.empty(1, heads, n, 16, device=DEV, dtype=torch.int32)
+    got = [[torch.empty_like(idx), torch.empty_like(o)] for _ in sets]
+    torch.cuda.synchronize()
+    st = torch.cuda.current_stream().cuda_stream
+    args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), idx.data_ptr(), 1, heads, n, n, 64, 16, 0.125)
+    for i, (x, out) in enumerate(zip(dev, got)):
+        idx.fill_((0x7f000000, 0x7f800000)[i % 2])             # 2^127 and +inf as floats
+        for a, b in zip((v, k, q), x[::-1]):
+            a.copy_(b)
+        if take:
+            _lib.check(_lib.load().s3r_cmp_attn_blocktopk_fwd(*args, 4, take, st), "s3r_cmp_attn_blocktopk_fwd")
+        else:
+            _lib.check(_lib.load().s3r_cmp_attn_topk_fwd(*args, st), "s3r_cmp_attn_topk_fwd")
+        out[0].copy_(idx)
+        out[1].copy_(o)
+    assert _lib.device_status() == 0
+    for (q_, k_, v_), out in zip(sets, got):
+        ref, _, idx_ref = R.cmp_attn_topk(q_, k_, v_, 16, rank_group=(4, take) if take else None)
+        S = q_ @ k_.transpose(-1, -2)
+        # fp32 sums of 64 products of that size in another order
+        eps = max(1e-3, 64 * 2 ** -24 * S.abs().max().item())
+        assert_idx_match(out[0], idx_ref, R.block_rank_scores(S, 0.125, 4, take) if take else S, f"{heads} heads {n}", eps=eps)
+        assert_bf16_close(out[1], ref, f"o_c {heads} heads {n}")
 
 
 @pytest.mark.parametrize("period", [1, 16, 64])

@@ -38,6 +38,31 @@ def test_next_kernel_starts_after_tensor_memory_is_allocated(path, at):
     assert 0 <= barrier < launch, "griddep_launch() before the barrier behind tcgen05.alloc"
 
 
+def functions_that_order_launches():
+    found = []
+    for path in SOURCES:
+        if os.path.basename(path) == "common.cuh":
+            continue
+        for body in code(path).split("\n}"):
+            if "griddep_" in body:
+                name = re.findall(r"\b(\w+)\(", body[body.index("__device__" if "__device__" in body else "__global__"):])
+                name = [n for n in name if n != "__launch_bounds__"][0]
+                found.append(pytest.param(body, id=f"{os.path.basename(path)}:{name}"))
+    return found
+
+
+@pytest.mark.parametrize("body", functions_that_order_launches())
+def test_what_other_kernels_wrote_is_read_behind_the_wait_for_them(body):
+    """griddepcontrol.wait is all that makes the writes of the kernels in front visible: every thread goes through it, once, before it reads
+    global memory and before it lets the next kernel start."""
+    assert body.count("griddep_wait(") == 1 and body.count("griddep_launch(") == 1
+    wait = re.search(r"\n  griddep_wait\(\);", body)
+    assert wait, "the wait is not for every thread"
+    before = body[:wait.start()]
+    assert "griddep_launch(" not in before
+    assert not re.search(r"\b(tma_load|__ldg|ldg_|cp_async|wait_bound|ld\.(relaxed|acquire|global)|prefetch)", before)
+
+
 @pytest.mark.parametrize("path", sorted({p.values[0] for p in kernels_with_tensor_memory()}), ids=os.path.basename)
 def test_draining_after_a_wait_that_gave_up_signals_no_result(path):
     """The issuing warp commits once more after a wait that gave up, to see its products drained.  The barrier of that commit is not one
