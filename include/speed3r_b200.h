@@ -163,7 +163,8 @@ int s3r_cmp_attn_blocktopk_fwd(const void* q_c, const void* k_c, const void* v_c
  * _flash_attn_backward and its three kernels (flash_attention_topk.py:204-630).  No gradient
  * flows through idx (:665).
  *   delta [B,H,Nq] fp32 is scratch written by the call (sum_d o_c*do_c).
- *   dq_c [B,H,Nq,d], dk_c / dv_c [B,H,Nc,d] bf16 are overwritten. */
+ *   dq_c [B,H,Nq,d], dk_c / dv_c [B,H,Nc,d] bf16 are overwritten.
+ *   Any finite scale (the forward, which ranks raw logits for it, takes positive ones only). */
 int s3r_cmp_attn_bwd(const void* q_c, const void* k_c, const void* v_c, const void* o_c, const float* lse,
                      const void* do_c, float* delta, void* dq_c, void* dk_c, void* dv_c, int B, int H, int Nq,
                      int Nc, int d, float scale, void* stream);

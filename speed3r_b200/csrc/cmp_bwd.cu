@@ -333,20 +333,22 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
       tmem_ld16(t_s + 16, xb);
       tmem_ld_wait();
       if (MODE == 1) arrive(&ctl.p_full[i & 1]);
-      // streamed rows past the end: P and dS are 0, whatever the products with the zeros that stand for them are
+      // Streamed rows past the end.  dK/dV: P and dS are 0 for any scale, whatever the products with the zeros that stand for them are
+      // (0 x inf, where a key is infinite): S becomes 0, from which the row's lse of +inf makes P = 0, and dP becomes 0.
       const int left = i == ntiles - 1 ? p.n_str - i * 128 - cols : 32;
-      auto none_past = [&](uint32_t (&x)[16], int c, uint32_t value) {
+      auto none_past = [&](uint32_t (&x)[16], int c) {
 #pragma unroll
         for (int e = 0; e < 16; ++e)
-          if (16 * c + e >= left) x[e] = value;
+          if (16 * c + e >= left) x[e] = 0u;
       };
       if (MODE == 0 && left < 32) {
-        none_past(xa, 0, 0xff800000u);
-        none_past(xb, 1, 0xff800000u);
+        none_past(xa, 0);
+        none_past(xb, 1);
       }
       pass1(xa, 0);
       pass1(xb, 1);
-      // dQ: keys past the end have S = 0, whose P overflows where all of a row's logits are far below zero
+      // dQ: keys past the end have S = 0, whose P overflows where all of a row's logits are far below zero.  dS = P dP is 0 unless the
+      // row's dO is infinite, which makes all of its dQ NaN through the other keys.
       if (MODE == 1 && left < 32) {
 #pragma unroll
         for (int e = 0; e < 32; ++e)
@@ -362,8 +364,8 @@ __device__ __forceinline__ void cmp_bwd_cta(const CUtensorMap& map_x0, const CUt
       tmem_ld16(t_dp + 16, xb);
       tmem_ld_wait();
       if (MODE == 0 && left < 32) {
-        none_past(xa, 0, 0u);
-        none_past(xb, 1, 0u);
+        none_past(xa, 0);
+        none_past(xb, 1);
       }
       pass2(xa, 0);
       pass2(xb, 1);

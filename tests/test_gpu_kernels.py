@@ -903,6 +903,23 @@ def test_cmp_backward_tiles(Nq, Nc):
         assert_bf16_close(a.grad, b.grad, name)
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.125, 0.3])
+@pytest.mark.parametrize("Nq, Nc", [(1, 130), (127, 65), (128, 128), (200, 300)])
+def test_cmp_backward_of_any_scale(scale, Nq, Nc):
+    """The backward takes any softmax scale, 0 and negative ones too, whether the last tile of queries or keys is whole or not."""
+    from speed3r_b200 import ops
+    B, H = 1, 2
+    q, k, v, do = bf16_round(randn(1, B, H, Nq, 64), randn(2, B, H, Nc, 64), randn(3, B, H, Nc, 64), randn(4, B, H, Nq, 64))
+    ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    S = ref[0] @ ref[1].transpose(-1, -2) * scale
+    o = torch.softmax(S, -1) @ ref[2]
+    o.backward(do)
+    lse = torch.logsumexp(S.detach(), -1).to(DEV)
+    got = ops._ops().cmp_attn_bwd(*(t.to(DEV, torch.bfloat16) for t in (q, k, v, o.detach())), lse, do.to(DEV, torch.bfloat16), scale)
+    for name, a, b in zip(("dq", "dk", "dv"), got, ref):
+        assert_bf16_close(a, b.grad, f"{name} scale {scale}")
+
+
 @pytest.mark.parametrize("Nq", [64, 70, 128, 200])
 def test_cmp_backward_of_a_key_that_is_minus_infinity(Nq):
     """A key that no query gives a weight has no gradient, whether the last tile of queries is whole or not: rows that do not exist
