@@ -904,11 +904,11 @@ def test_cmp_backward_tiles(Nq, Nc):
 
 
 @pytest.mark.parametrize("scale", [0.0, -0.125, 0.3])
-@pytest.mark.parametrize("Nq, Nc", [(1, 130), (127, 65), (128, 128), (200, 300)])
-def test_cmp_backward_of_any_scale(scale, Nq, Nc):
+@pytest.mark.parametrize("H, Nq, Nc", [(2, 1, 130), (2, 127, 65), (2, 128, 128), (2, 200, 300), (64, 200, 150)])
+def test_cmp_backward_of_any_scale(scale, H, Nq, Nc):
     """The backward takes any softmax scale, 0 and negative ones too, whether the last tile of queries or keys is whole or not."""
     from speed3r_b200 import ops
-    B, H = 1, 2
+    B = 1
     q, k, v, do = bf16_round(randn(1, B, H, Nq, 64), randn(2, B, H, Nc, 64), randn(3, B, H, Nc, 64), randn(4, B, H, Nq, 64))
     ref = [t.clone().requires_grad_(True) for t in (q, k, v)]
     S = ref[0] @ ref[1].transpose(-1, -2) * scale
@@ -938,6 +938,30 @@ def test_cmp_backward_of_a_key_that_is_minus_infinity(Nq):
         g = a.grad.cpu()
         assert (g[:, :, at] == 0).all(), name
         assert_bf16_close(g[:, :, rest], b.grad, name)
+
+
+@pytest.mark.parametrize("H, Nq, Nc", [(64, 129, 256), (64, 256, 130), (64, 200, 200), (40, 150, 255), (32, 257, 384), (32, 500, 449), (48, 640, 577)])
+def test_cmp_backward_of_two_row_tiles(H, Nq, Nc):
+    """Grids of 256 own rows per CTA: a second row tile of one row, streamed tiles of 64 whole and not, one and several rounds of the ring
+    of six; one key that no query gives a weight."""
+    from speed3r_b200 import ops
+    B, at = 1, Nc - 1
+    q, k, v, do = bf16_round(randn(1, B, H, Nq, 64), randn(2, B, H, Nc, 64), randn(3, B, H, Nc, 64), randn(4, B, H, Nq, 64))
+    q[..., 0] = q[..., 0].abs() + 0.5
+    k[:, :, at, 0] = float("-inf")
+    t = [x.to(DEV, torch.bfloat16).requires_grad_(True) for x in (q, k, v)]
+    ops.flash_attn_topk_func(*t, 8)[0].backward(do.to(DEV, torch.bfloat16))
+    rest = torch.arange(Nc) != at
+    ref = [x.clone().requires_grad_(True) for x in (q, k[:, :, rest], v[:, :, rest])]
+    torch.softmax(ref[0] @ ref[1].transpose(-1, -2) * 0.125, -1).matmul(ref[2]).backward(do)
+    for name, a, b in zip(("dk", "dv"), t[1:], ref[1:]):
+        g = a.grad.cpu()
+        assert (g[:, :, at] == 0).all(), name
+        assert_bf16_close(g[:, :, rest], b.grad, name)
+    t = [x.to(DEV, torch.bfloat16).requires_grad_(True) for x in (q, k[:, :, rest].contiguous(), v[:, :, rest].contiguous())]
+    ops.flash_attn_topk_func(*t, 8)[0].backward(do.to(DEV, torch.bfloat16))
+    for name, a, b in zip(("dq", "dk", "dv"), t, ref):
+        assert_bf16_close(a.grad, b.grad, name)
 
 
 def test_prologue_of_blocks_whose_table_rows_do_not_fit_shared_memory():
