@@ -416,10 +416,8 @@ __device__ __forceinline__ void cmp_attn_cta(const CUtensorMap& map_q, const CUt
     if (ok && half == 0 && row < p.Nq) {
       float bound = INFINITY;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float m = fmaxf(gm[i], other[max(p.topk - 1 - i, 0) * 128]);      // loaded in any case, so that no branch stands around it
-        bound = i < p.topk ? fminf(bound, m) : bound;
-      }
+      for (int i = 0; i < 32; ++i)
+        if (i < p.topk) bound = fminf(bound, fmaxf(gm[i], other[(p.topk - 1 - i) * 128]));
       // a sum's logarithm, less what its exponentials and the second kernel's scores can differ by: 2^-20 from the
       // exponentials, and roundings of the arguments, each below 2^-24 of their size.  The polynomial exponentials are 2^-126
       // for anything smaller: a sum in which two of those are more than 2^-21 bounds nothing.

@@ -24,9 +24,11 @@
 // of 39, 6300 x 6300 with every key there 16 times 666 instead of 620.)
 //
 // Bound: instructions and their latency in the scan: a max tree and a vote per 16 columns of a warp, and for the chunks
-// with a hit (three in four at 250 views, one in three at 1000) a mask and a store.  Pairs are appended under a predicate, not in a
-// branch per column: both kernels, 16 heads, 4032 x 4032 207 -> 205 us, 6300 x 6300 426 -> 416, 15750 x 15750 2067 -> 2035.  The products take half of the time
-// that the tensor pipe alone would need.  S of a tile is two buffers of 64 columns, so that the next products run while a half is
+// with a hit (three in four at 250 views, one in three at 1000) a mask and a store.  A chunk's only pair is appended under a predicate,
+// not in a branch: both kernels, 16 heads, 4032 x 4032 206.5 -> 203.2 us, 6300 x 6300 446 -> 425; several pairs of a chunk as well for one
+// row tile (512 x 512 29.8 -> 29.5), but not for two, whose 16 warps cover the branches (1400 x 1400 55.1 with predicates, 54.6 with
+// branches, 6300 x 6300 426.0 and 425.2).  The products take half of the time that the tensor pipe alone would need.  S of a tile
+// is two buffers of 64 columns, so that the next products run while a half is
 // scanned (16 columns at a time, S held for a whole tile: 1.05 instead of 0.95 ms for 15750 x 15750, 16 heads), each taken into
 // registers 32 columns at a time (all 64 at once spilled in the scan: both kernels 448 instead of 439 us for 6300 x 6300, 2140
 // instead of 2098 for 15750 x 15750).
@@ -333,7 +335,14 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
         sts64_append<256>(mask, at, __float_as_uint(m), static_cast<uint32_t>(col0 - 16 + __clz(mask)));
       } else if (!__any_sync(0xffffffffu, at + 256 * __popc(mask) > end)) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) sts64_append<256>(mask & (0x8000u >> i), at, x[i], static_cast<uint32_t>(col0 + i));
+        for (int i = 0; i < 16; ++i) {
+          if (R == 1) {
+            sts64_append<256>(mask & (0x8000u >> i), at, x[i], static_cast<uint32_t>(col0 + i));
+          } else if (mask & (0x8000u >> i)) {
+            sts64(at, x[i], static_cast<uint32_t>(col0 + i));
+            at += 256;
+          }
+        }
       } else {
         TkChunk ch;
 #pragma unroll
@@ -450,9 +459,8 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     uint32_t a[32], e[kTkCap - 32];
     uint32_t top = 0;
     // keys above the bound's, plus one: an empty place is 0
-    // (loaded whether the place is filled or not: a choice between loads becomes a branch around each)
     auto word = [&](int i) {
-      const uint32_t k = sortable_key(__uint_as_float(buf[i * 32].x)) - base_key + 1u, d = i < cnt ? k : 0u;
+      const uint32_t d = i < cnt ? sortable_key(__uint_as_float(buf[i * 32].x)) - base_key + 1u : 0u;
       top = max(top, d);
       return d;
     };
