@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restr
 }
 
 // ------------------------------------------------------------------------------------------------
-// backward of the gated merge: one warp per (b,h,query block); 8 lanes per token, 4 tokens a pass
+// backward of the gated merge: one warp per (b,h,query block); 8 lanes per token, 4 U tokens a pass
 // ------------------------------------------------------------------------------------------------
 struct MergeBwdParams {
   const __nv_bfloat16* dy;
@@ -344,6 +344,13 @@ struct MergeBwdParams {
   int B, H, Tq, block, nqb;
 };
 
+// Bound: HBM and the latency of a pass.  U = 4 has 16 tokens' loads under way before the first is used, in 80 registers: 16 heads,
+// blocks of 16, U = 1 -> 4: 2 x 6144 tokens 15.0 -> 14.1 us, 64 512 93.8 -> 88.6, 252 000 353 -> 337 (0.76 of the copy rate).  A pass whose
+// tokens do not all exist costs as much as a whole one, and fewer warps fit: 64 512 tokens in blocks of 1 540 and 895 us, 4 148 and 234,
+// 8 110 and 141, 12 98 and 105, 15 98.7 and 92.5, 17 101 and 109, 24 90 and 93, 32 86.5 and 80.1, 33 91.1 and 90.6, 100 94.8 and 79.8.
+static bool merge_bwd_whole_passes(int block) { return block > 32 || block % 16 == 0 || block % 16 == 15; }
+
+template <int U>
 __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) {
   griddep_wait();
   griddep_launch();
@@ -361,22 +368,25 @@ __global__ void __launch_bounds__(256) merge_bwd_kernel(const MergeBwdParams p) 
 #pragma unroll
     for (int i = 0; i < 4; ++i) { oc[2 * i] = bf16_lo(w[i]); oc[2 * i + 1] = bf16_hi(w[i]); acc[2 * i] = acc[2 * i + 1] = 0.f; }
   }
-  for (int base = 0; base < p.block; base += 16) {
-    // 16 tokens' loads are under way before the first is used
-    uint4 a[4], s[4];
-    uint32_t gw[4];
-    bool live[4];
+  for (int base = 0; base < p.block; base += 4 * U) {
+    uint4 a[U], s[U];
+    uint32_t gw[U];
+    bool live[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int in_block = base + 4 * u + sub, t = m * p.block + in_block;
       live[u] = in_block < p.block && t < p.Tq;
-      const int tc = min(t, p.Tq - 1);                       // loaded in any case
-      a[u] = __ldg(reinterpret_cast<const uint4*>(p.dy + ((static_cast<int64_t>(b) * p.Tq + tc) * p.H + h) * 64 + c8 * 8));
-      s[u] = __ldg(reinterpret_cast<const uint4*>(p.o_s + (static_cast<int64_t>(bh) * p.Tq + tc) * 64 + c8 * 8));
-      gw[u] = __ldg(reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + tc * p.gst));
+      a[u] = s[u] = make_uint4(0u, 0u, 0u, 0u);
+      gw[u] = 0u;
+      if (U > 1 || live[u]) {                                // several: loaded in any case, without a branch around each
+        const int tc = min(t, p.Tq - 1);
+        a[u] = __ldg(reinterpret_cast<const uint4*>(p.dy + ((static_cast<int64_t>(b) * p.Tq + tc) * p.H + h) * 64 + c8 * 8));
+        s[u] = __ldg(reinterpret_cast<const uint4*>(p.o_s + (static_cast<int64_t>(bh) * p.Tq + tc) * 64 + c8 * 8));
+        gw[u] = __ldg(reinterpret_cast<const uint32_t*>(p.gate + b * p.gsb + h * p.gsh + tc * p.gst));
+      }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < U; ++u) {
       const int t = m * p.block + base + 4 * u + sub;
       const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, sw[4] = {s[u].x, s[u].y, s[u].z, s[u].w};
       float dyv[8], osv[8];
@@ -1037,7 +1047,7 @@ extern "C" int s3r_merge_bwd_deltas(const void* dy, const void* gate, int64_t ga
   p.B = B; p.H = H; p.Tq = Tq; p.block = block;
   p.nqb = (Tq + block - 1) / block;
   const int64_t warps = static_cast<int64_t>(B) * H * p.nqb;
-  return launch(merge_bwd_kernel, static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), p);
+  return launch(merge_bwd_whole_passes(block) ? merge_bwd_kernel<4> : merge_bwd_kernel<1>, static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" int s3r_merge_bwd(const void* dy, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,

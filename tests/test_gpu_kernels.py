@@ -679,6 +679,25 @@ def test_prologue_forward_blocks(Bs, blocks, norm, rope):
         assert_bf16_close(a, b, f"{name} {Bs}")
 
 
+@pytest.mark.parametrize("block", [1, 3, 4, 12, 15, 16, 17, 24, 31, 32, 33, 47, 48])
+def test_merge_backward_blocks(block):
+    """Blocks of one pass and of several, of 4 tokens and of 16, whole and not, with a last block cut short."""
+    from speed3r_b200 import ops
+    B, H, T = 2, 3, 5 * block + max(1, block // 3)
+    nb = -(-T // block)
+    dy, o_s, o_c, gate = bf16_round(randn(1, B, T, H * 64), randn(2, B, H, T, 64), randn(3, B, H, nb, 64), torch.sigmoid(randn(4, B, H, T, 2)))
+    do_s, dgate, do_c, delta = ops._ops().merge_bwd(*(t.to(DEV, torch.bfloat16) for t in (dy, gate, o_c, o_s)), block)
+    g, of = dy.view(B, T, H, 64).transpose(1, 2), o_c.repeat_interleave(block, 2)[:, :, :T]
+    dg = torch.stack(((g * of).sum(-1), (g * o_s).sum(-1)), -1)
+    c = torch.zeros(B, H, nb * block, 64)
+    c[:, :, :T] = gate[..., :1] * g
+    # fp32 sums of 64 products up to 2^4 each, in another order
+    assert (dgate.cpu() - dg).abs().max() <= 64 * 2 ** -24 * 64 * 16
+    assert (delta.cpu() - gate[..., 1] * dg[..., 1]).abs().max() <= 64 * 2 ** -24 * 64 * 16
+    assert_bf16_close(do_s, gate[..., 1:] * g, f"do_s block {block}")
+    assert_bf16_close(do_c, c.view(B, H, nb, block, 64).sum(3), f"do_c block {block}")
+
+
 def _prologue_fp32(qkv, H, Bs, pos, cos, sin, qn, kn):
     """Split, LayerNorm, rotary embedding and pooling in fp32 with the given (bf16) rotary tables."""
     B, N, d = qkv.shape[0], qkv.shape[1], 64
