@@ -159,18 +159,24 @@ __device__ __forceinline__ void rope_rows(Vec8 (&o)[G], const Vec8 (&c)[G], cons
 // A CTA has up to 16 of the block's 3H rows (8 lanes each: four warps, one per scheduler).  A thread's share of 16 tokens is on
 // its way at once, 16 bytes a token in slots of its own in shared memory (cp.async; nobody else reads them): 32 KB per CTA.
 // Bound: HBM on long sequences (0.8 of the copy rate), on short ones the chain of a token - two sums over eight lanes, a root, a
-// rotation - of which one after the other took 980 cycles with two or three warps per scheduler.  Four tokens go through it side by
-// side, with their table rows in shared memory, in four CTAs of 128 registers per SM (one by one in six of 80; two in five of 102 as
-// fast but for the short ones).  16 heads, one by one -> now: in the module at 2048 tokens 12.8 -> 8.8 us, 2 x 6144 37.9 -> 36.2,
-// 64 512 172.7 -> 162.3 (by itself, 1.8 GHz).  Earlier forms, 252 000 tokens: six CTAs 628 us, 24 KB in flight, the next tokens' loads
-// in registers 759, four tokens ahead and the tables' rows found by every row 908, 24 rows per CTA 656, eight CTAs of 64 registers 804.
-constexpr int kProRows = 16, kProThreads = kProRows * 8, kProChunk = 16, kProCtas = 4, kProBwdCtas = 4;
+// rotation - of which one after the other takes 980 cycles with two or three warps per scheduler.  Three forms:
+// kProSide: four tokens go through it side by side, with their table rows in shared memory, in four CTAs of 128 registers per SM (two
+//   in five of 102 as fast but for the short ones).
+// kProOne: one by one, in six CTAs of 80 registers.  For blocks that fill no four or no chunk (prologue_side_by_side).
+// kProLong: blocks whose rows of the tables do not fit shared memory; four side by side, each looking its row up.
+// 16 heads, blocks of 16, one by one -> side by side: 2048 tokens 13.3 -> 10.7 us, 6144 18.6 -> 18.2, 64 512 183.7 -> 176.7, 252 000
+// 697 -> 671.  One block of 6400 tokens, by itself or not, one by one -> four: 3.9 -> 2.7 ms.  Earlier forms, 252 000 tokens: six CTAs
+// 628 us (without the gate), 24 KB in flight, the next tokens' loads in registers 759, four tokens ahead and the tables' rows found by
+// every row 908, 24 rows per CTA 656, eight CTAs of 64 registers 804.
+constexpr int kProRows = 16, kProThreads = kProRows * 8, kProChunk = 16, kProCtas = 4, kProOneCtas = 6, kProBwdCtas = 4;
 constexpr int kProRingBytes = kProChunk * kProThreads * 16;
 constexpr int kProTabBytes = (kProChunk + 1) * 256;    // cos (y, x) and sin (y, x) of a chunk's tokens and of the block's mean, 64 bytes each
 
-template <bool LONG>
-__global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(const PrologueParams p) {
-  constexpr int G = LONG ? 1 : 4;                      // tokens side by side
+enum ProForm { kProSide, kProOne, kProLong };
+template <ProForm FORM>
+__global__ void __launch_bounds__(kProThreads, FORM == kProOne ? kProOneCtas : kProCtas) prologue_fwd_kernel(const PrologueParams p) {
+  constexpr bool LONG = FORM == kProLong, TAB = FORM == kProSide;
+  constexpr int G = FORM == kProOne ? 1 : 4;               // tokens side by side
   extern __shared__ __align__(16) uint8_t smem[];      // [token of the chunk][thread] 16 bytes; [warp] rows of the tables
   griddep_wait();
   griddep_launch();
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   __nv_bfloat16* dst = out + (bh * p.N + n0) * 64 + l8 * 8;
   const uint32_t slots = smem_u32(smem) + threadIdx.x * 16;
   const uint32_t tab = smem_u32(smem) + kProRingBytes;
-  int* rows = reinterpret_cast<int*>(smem + kProRingBytes + kProTabBytes) + (threadIdx.x >> 5) * 2 * (LONG ? 1 : p.block + 1);
+  int* rows = reinterpret_cast<int*>(smem + kProRingBytes + (TAB ? kProTabBytes : 0)) + (threadIdx.x >> 5) * 2 * (LONG ? 1 : p.block + 1);
   // two groups of loads per chunk: the first half is worked on while the second arrives
   auto fetch = [&](int t0) {
 #pragma unroll
@@ -242,7 +248,7 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   };
   const int* my_row = rows + (l8 >> 2);                // y for lanes 0-3, x for 4-7
   const __nv_bfloat16 *cos_l = p.cos_tab + (l8 & 3) * 8, *sin_l = p.sin_tab + (l8 & 3) * 8;
-  auto row_of = [&](int t) { return table_row(__ldg(p.pos + (tok0 + t) * 2 + (l8 >> 2)), p.tab_rows); };
+  auto row_of = [&](int t) { return LONG ? table_row(__ldg(p.pos + (tok0 + t) * 2 + (l8 >> 2)), p.tab_rows) : my_row[2 + 2 * t]; };
 
   float2 acc[4] = {splat(0.f), splat(0.f), splat(0.f), splat(0.f)};
   // G tokens of this row: accumulate the raw block sum, normalise, rotate, store
@@ -253,7 +259,7 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
     for (int u = 0; u < G; ++u) {
       const int at = min(slot + u, kProChunk - 1);
       o[u] = lds_vec8(slots + at * (kProThreads * 16));
-      if (rope && LONG) {
+      if (rope && !TAB) {
         const int row = row_of(min(t + u, p.block - 1)) * 32;
         c[u] = ldg_vec8(cos_l + row);
         s[u] = ldg_vec8(sin_l + row);
@@ -282,14 +288,14 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   };
   for (int t0 = 0; t0 < p.block; t0 += kProChunk) {
     const int n = min(kProChunk, p.block - t0);
-    if (!LONG && p.pos != nullptr) {
+    if (TAB && p.pos != nullptr) {
       if (t0 > 0) __syncthreads();                     // the chunk before has been used
       tables(t0);
       __syncthreads();
     }
     if (live) {
       cp_async_wait<1>();
-#pragma unroll 1
+#pragma unroll (FORM == kProOne ? 2 : 1)
       for (int i = 0; i < n; i += G) {
         if (i == kProChunk / 2) cp_async_wait<0>();
         tokens(t0 + i, i);
@@ -308,8 +314,8 @@ __global__ void __launch_bounds__(kProThreads, kProCtas) prologue_fwd_kernel(con
   Vec8 o[1] = {pack8(x[0])};
   if (rope) {
     const int row = my_row[0] * 32;
-    const Vec8 c[1] = {LONG ? ldg_vec8(cos_l + row) : lds_vec8(tab + kProChunk * 256 + l8 * 16)},
-               s[1] = {LONG ? ldg_vec8(sin_l + row) : lds_vec8(tab + kProChunk * 256 + 128 + l8 * 16)};
+    const Vec8 c[1] = {TAB ? lds_vec8(tab + kProChunk * 256 + l8 * 16) : ldg_vec8(cos_l + row)},
+               s[1] = {TAB ? lds_vec8(tab + kProChunk * 256 + 128 + l8 * 16) : ldg_vec8(sin_l + row)};
     rope_rows<1>(o, c, s, l8, gmask);
   }
   *reinterpret_cast<Vec8*>(out_c + (bh * p.Nc + j) * 64 + l8 * 8) = o[0];
@@ -541,6 +547,13 @@ static int prologue_smem(int ring, int block, bool* lengthy) {
   return *lengthy ? ring + static_cast<int>(warps * 2 * sizeof(int)) : static_cast<int>(all);
 }
 static int prologue_parts(int H) { return (3 * H + kProRows - 1) / kProRows; }
+// Whether the forward takes four tokens side by side.  What is left of a block beyond whole fours and whole chunks costs as much as they
+// do; where the GPU is not filled the shorter chain counts for more.  16 heads, one by one and side by side, us: 60 000 tokens in blocks of 1
+// 680 and 1130, 4 247 and 313, 8 182 and 213, 12 169 and 183, 17 173 and 191, 25 166 and 172, 28 162 and 161, 33 162 and 167 (20 000: 62 and
+// 59); of 15 by CTAs 450: 13.9 and 10.9, 720: 15.5 and 13.0, 999: 15.5 and 16.7.
+static bool prologue_side_by_side(int block, int64_t ctas) {
+  return block % 16 == 0 || block >= 28 || (block >= 14 && 2 * ctas <= 3 * kProCtas * sm_count());
+}
 // CTAs along the blocks: four per SM over all parts
 static int prologue_bwd_ctas(int B, int Nc, int H) {
   const int64_t n = static_cast<int64_t>(B) * Nc, parts = prologue_parts(H), cap = (kProBwdCtas * sm_count() + parts - 1) / parts;
@@ -595,9 +608,16 @@ static int prologue_fwd(const void* qkv, int64_t tok_stride, const void* gate_in
   p.B = B; p.H = H; p.N = N; p.Nc = Nc; p.block = block;
   p.status = device_status_ptr();
   S3R_REQUIRE(p.status != nullptr, S3R_ERR_DRIVER, "s3r_qkv_prologue_fwd: could not resolve the device status word");
-  bool lengthy;
-  const int smem = prologue_smem(kProRingBytes + kProTabBytes, block, &lengthy);
-  auto* kernel = lengthy ? prologue_fwd_kernel<true> : prologue_fwd_kernel<false>;
+  const int64_t ctas = grid * prologue_parts(H);
+  bool side = prologue_side_by_side(block, ctas), lengthy;
+  int smem = prologue_smem(kProRingBytes + (side ? kProTabBytes : 0), block, &lengthy);
+  if (side && lengthy) {
+    // 6104 to 6239 tokens' rows fit beside the slots alone, in one CTA per SM.  20 such blocks, 16 heads: one by one 3.2 ms, as long blocks
+    // 3.4, without a norm 2.6 and 3.0, but without positions 2.6 and 1.9, and 300 blocks of 4 heads 8.1 and 3.2
+    side = false;
+    if (pos != nullptr && ctas <= sm_count()) smem = prologue_smem(kProRingBytes, block, &lengthy);
+  }
+  auto* kernel = side ? prologue_fwd_kernel<kProSide> : lengthy ? prologue_fwd_kernel<kProLong> : prologue_fwd_kernel<kProOne>;
   S3R_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProMaxSmem));
   return launch(kernel, dim3(static_cast<unsigned>(grid), prologue_parts(H)), kProThreads, smem,
                 static_cast<cudaStream_t>(stream), p);

@@ -698,6 +698,59 @@ def test_merge_backward_blocks(block):
     assert_bf16_close(do_c, c.view(B, H, nb, block, 64).sum(3), f"do_c block {block}")
 
 
+@pytest.mark.parametrize("Bs, blocks", [(13, 5), (18, 300)])
+@pytest.mark.parametrize("norm, rope", [(True, True), (False, True), (True, False)])
+def test_prologue_forward_one_by_one(Bs, blocks, norm, rope):
+    """Blocks below a chunk, and of a chunk and a bit on a grid beyond the GPU."""
+    test_prologue_forward_blocks(Bs, blocks, norm, rope)
+
+
+@pytest.mark.parametrize("Bs", [6100, 6150, 6300, 6310])
+@pytest.mark.parametrize("norm, rope", [(True, True), (False, True), (True, False)])
+def test_prologue_forward_long_blocks(Bs, norm, rope):
+    """The longest blocks whose rows fit shared memory, beside the tables' and without them, and blocks whose rows do not, or have none:
+    tokens as with blocks of ten, bit for bit, means against fp32."""
+    import speed3r_b200
+    from speed3r_b200 import ops
+    B, H, N = 2, 3, Bs
+    qkv, = bf16_round(1.5 * randn(30, B, N, 3 * H * 64) + 0.3)
+    pos = torch.randint(0, 37, (B, N, 2), generator=torch.Generator().manual_seed(2)) if rope else None
+    cos, sin = speed3r_b200.RoPE2D(100.0)._cos_sin(32, 37, torch.device(DEV), torch.bfloat16)
+    wb = [(1 + 0.2 * randn(31 + i, 64), 0.1 * randn(33 + i, 64)) if norm else None for i in range(2)]
+    args = (pos.to(DEV) if rope else None, cos if rope else None, sin if rope else None,
+            *[(w[0].to(DEV), w[1].to(DEV), 1e-5) if norm else None for w in wb])
+    got, tens = (ops.qkv_prologue(qkv.to(DEV, torch.bfloat16), H, b, *args) for b in (Bs, 10))
+    assert all(torch.equal(a, b) for a, b in zip(got[:3], tens[:3]))
+    # The norm divides a block's mean, 0.3 and rounded to bf16 within 2^-11, by its spread of 1.5 / sqrt(Bs) = 0.019: 0.026, times weights
+    # up to 1.6 and, rotated, the sum of two; the sum's order may turn a rounding the other way, which doubles it
+    for name, a, b in zip(("q_c", "k_c", "v_c"), got[3:], _prologue_fp32(qkv, H, Bs, pos, cos, sin, *wb)[3:]):
+        err = (a.float().cpu() - b).abs()
+        assert err.max() <= (2 * 2 * 1.6 * 0.026 if norm and name != "v_c" else 2e-2) and err.mean() <= 0.03, f"{name} {Bs}: {err.max()}"
+
+
+@pytest.mark.parametrize("H, Bs, blocks", [(4, 3, 5), (12, 16, 4), (16, 16, 3), (20, 16, 5), (40, 16, 3), (8, 35, 3), (4, 100, 2), (20, 13, 3), (16, 6300, 1)])
+def test_prologue_forward_gates(H, Bs, blocks):
+    """The gate's logits: fewer pairs of a block than threads, exactly two per thread, a part of the second and more, in every form of the
+    kernel and with a part of the rows that is not whole; the other outputs are those of the projection without them."""
+    import speed3r_b200
+    from speed3r_b200 import _lib, ops
+    B, N, C = 2, Bs * blocks, 3 * H * 64
+    proj, = bf16_round(2 * randn(40 + H, B, N, C + 2 * H))
+    proj = proj.to(DEV, torch.bfloat16)
+    pos = torch.randint(0, 37, (B, N, 2), generator=torch.Generator().manual_seed(2)).to(DEV)
+    cos, sin = speed3r_b200.RoPE2D(100.0)._cos_sin(32, 37, torch.device(DEV), torch.bfloat16)
+    w = [t.to(DEV) for t in (1 + 0.2 * randn(3, 64), 0.1 * randn(4, 64), 1 + 0.2 * randn(5, 64), 0.1 * randn(6, 64))]
+    want = ops.qkv_prologue(proj[..., :C].contiguous(), H, Bs, pos, cos, sin, (w[0], w[1], 1e-5), (w[2], w[3], 1e-5))
+    got = [torch.full_like(t, float("nan")) for t in want] + [torch.full((B, H, N, 2), float("nan"), device=DEV, dtype=torch.bfloat16)]
+    _lib.check(_lib.load().s3r_qkv_gate_prologue_fwd(
+        proj.data_ptr(), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.shape[0], *(t.data_ptr() for t in w), 1e-5,
+        *(t.data_ptr() for t in got), B, H, N, 64, Bs, torch.cuda.current_stream().cuda_stream), "s3r_qkv_gate_prologue_fwd")
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    gate = torch.sigmoid(proj[..., C:].double()).view(B, N, H, 2).permute(0, 2, 1, 3)
+    # one rounding to bf16, whose 8 bits make half a unit of the last 2^-8 of the value at most, of fp32 values good to 2^-18
+    assert ((got[6].double() - gate).abs() <= (2 ** -8 + 2 ** -18) * gate).all()
+
+
 def _prologue_fp32(qkv, H, Bs, pos, cos, sin, qn, kn):
     """Split, LayerNorm, rotary embedding and pooling in fp32 with the given (bf16) rotary tables."""
     B, N, d = qkv.shape[0], qkv.shape[1], 64
