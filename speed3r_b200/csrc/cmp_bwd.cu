@@ -27,8 +27,8 @@
 // Bound: up to 2400 rows the chain of a tile (1845 cycles for dK/dV, 1460 for dQ, of which the exponentials' unit is busy 1024 and the
 // tensor pipe 1024 | 768), beyond that the power limit: the clock falls to 1.7 GHz.  Issuing a product blocks for as long as the pipe
 // takes for it (its queue holds one), so that all that the issuing warp does in between - waits that are over, address arithmetic, the
-// branch around an elected lane - is time in which the pipe idles.  Before (256 own rows, tiles of 64, one S: 1930 and 1410 cycles for
-// half as many columns of twice as many rows) that warp was what a period took.  With delta, 16 heads, us: 2400 x 2400 125 -> 107,
+// branch around an elected lane - is time in which the pipe idles.  With two row tiles (1930 and 1410 cycles for half as many columns
+// of twice as many rows) that warp is what a period takes.  Two row tiles throughout -> one, with delta, 16 heads, us: 2400 x 2400 125 -> 107,
 // 4032 x 4032 268 -> 259, 6300 x 6300 633 -> 615, 15750 x 15750 3689 -> 3605.  Tried: two streams of tiles of 64 with S twice in each
 // (6300: 670; asking ahead and without the branch 631), compute warps that ask for their barriers ahead too (637).
 // Both kinds of CTA are in one grid, dK/dV first: they do not depend on each other, and a small grid of one kind leaves

@@ -174,7 +174,9 @@ __device__ __noinline__ void tk_exact(const uint2* la, int na, const uint2* lb, 
 static_assert(kTkCap == 40, "tk_exact takes lists of up to 40, the packed words a place below 80");
 
 // Both kinds of CTA in one grid: a row's bound is there when its word is no longer what it was filled with (all bits set: a NaN
-// that no arithmetic returns).  For at most a second; called by whole warps.
+// that no arithmetic returns).  For at most a second, in which a CTA of the attention goes through some 2 x 10^8 keys; called by whole
+// warps.  Fill and grid are in stream order; the bound and the word that it replaces are one aligned word, so that nothing else has to be seen
+// with it.
 __device__ __forceinline__ bool wait_bound(const int32_t* word, bool mine, uint32_t& v, volatile uint32_t* abort_flag) {
   const uint64_t start = globaltimer_ns();
   while (true) {
@@ -225,7 +227,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
   __syncthreads();
   tc_fence_after();
   // In a launch of its own this kernel could begin with its copies and products before the attention has ended, and wait for the bounds
-  // as they come, in places that the attention fills before it lets this launch start.  The op at 2048 tokens took 1.3 us less that way,
+  // as they come, in places that the attention fills before it lets this launch start.  The op at 2048 tokens took 1.6 us less that way,
   // but nothing documents what a grid sees of others in front of this wait, and a place's old content taken for a bound is a wrong table.
   griddep_wait();
   griddep_launch();
@@ -546,7 +548,7 @@ __device__ __forceinline__ void cmp_topk_cta(const CUtensorMap& map_q, const CUt
     meet();
     // Words to columns, by both threads of a row, half of it each, in a loop: a CTA runs this code once, and what it takes is
     // the fetching of instructions (32 lookups and stores unrolled in one of the threads: 4400 to 8100 cycles; both kernels,
-    // 16 heads, 2 x 384 x 384 20.1 -> 19.7 us, the op at 2048 tokens 44.2 -> 43.7).
+    // 16 heads, 2 x 384 x 384 22.5 -> 22.0 us, 1024 x 1024 40.6 -> 39.9).
     if (ok && *abort_flag == 0u && row < p.Nq) {           // neither of the row's threads gave up
       const bool columns = tell[0] != 0u;
       const uint2* list = buf - par * 4 * (kTkCap * 32);
